@@ -188,6 +188,18 @@ int lbk_leaf_values(lbk_context* ctx, const double* leaf_value, const int32_t* l
  * (legateboost/models/tree.py:252-277, predict.cu:26-84).  pred is overwritten (zero + sum of
  * leaves in tree order, float64); the caller adds the model's initial prediction.
  */
+/* One tree of an ensemble whose arrays are on the device; node_off = the sum of max_nodes of the trees
+ * before it. */
+typedef struct lbk_tree_ref {
+  const double* leaf;
+  const int32_t* feature;
+  const double* split;
+  int32_t max_nodes;
+  int32_t node_off;
+} lbk_tree_ref;
+
+enum { LBK_RAW = 0, LBK_LOGISTIC = 1, LBK_SOFTMAX = 2 };
+
 typedef struct lbk_predict_args {
   const void* X;
   int32_t x_dtype;
@@ -204,6 +216,18 @@ typedef struct lbk_predict_args {
   int64_t ldp;
   void* stream;
   int32_t host_buffers;
+  /* Optional: the table of the trees as a device array that the caller keeps with the ensemble (device
+   * buffers only).  leaf_value, feature, split_value and max_nodes are then ignored, nothing is copied to
+   * the device and the call is asynchronous on `stream`; a fault that a kernel reports is returned by a
+   * later call on the context. */
+  const lbk_tree_ref* table;
+  int32_t table_max_nodes;    /* the largest max_nodes in the table */
+  int64_t table_total_nodes;  /* the sum of max_nodes */
+  /* Optional: device [n_outputs], added to every row's sums (the caller's initial prediction) */
+  const double* init;
+  /* LBK_RAW: pred holds the sums.  LBK_LOGISTIC (one output): two columns, 1 - p and p with p = 1 / (1 +
+   * exp(-sum)).  LBK_SOFTMAX: probabilities of the n_outputs classes. */
+  int32_t transform;
 } lbk_predict_args;
 
 int lbk_predict(lbk_context* ctx, const lbk_predict_args* args);

@@ -522,21 +522,36 @@ int lbk_predict(lbk_context* ctx, const lbk_predict_args* a)
     if (a->n_rows < 1) return;
     LBK_EXPECT(a->X && a->pred, "null argument");
     LBK_EXPECT(a->n_features >= 1 && a->n_outputs >= 1 && a->n_trees >= 0, "bad shape");
-    LBK_EXPECT(a->n_trees == 0 || (a->leaf_value && a->feature && a->split_value && a->max_nodes), "null tree arrays");
-    LBK_EXPECT(a->ldx >= a->n_features && a->ldp >= a->n_outputs, "Expected a dense row major store");
+    LBK_EXPECT(a->n_trees == 0 || a->table || (a->leaf_value && a->feature && a->split_value && a->max_nodes), "null tree arrays");
+    LBK_EXPECT(!a->table || (!a->host_buffers && a->table_max_nodes >= 1), "a table of trees is for device buffers");
+    LBK_EXPECT(a->transform == LBK_RAW || a->transform == LBK_SOFTMAX || (a->transform == LBK_LOGISTIC && a->n_outputs == 1),
+               "unknown transform");
+    const int columns = a->transform == LBK_LOGISTIC ? 2 : a->n_outputs;
+    LBK_EXPECT(a->ldx >= a->n_features && a->ldp >= columns, "Expected a dense row major store");
     cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
     lbk::Scratch s(ctx, stream);
-    const int F = a->n_features, K = a->n_outputs;
+    const int F = a->n_features, K = a->n_outputs, T = a->n_trees;
     const int64_t N = a->n_rows;
     const void* X   = a->X;
     double* pred    = a->pred;
     int64_t ldx = a->ldx, ldp = a->ldp;
-    std::vector<const double*> leaf(a->n_trees), split(a->n_trees);
-    std::vector<const int32_t*> feat(a->n_trees);
-    for (int t = 0; t < a->n_trees; ++t) {
-      leaf[t]  = a->leaf_value[t];
-      feat[t]  = a->feature[t];
-      split[t] = a->split_value[t];
+    const lbk_tree_ref* table = a->table;
+    int m_max                 = a->table_max_nodes;
+    int64_t total             = a->table_total_nodes;
+    std::vector<lbk_tree_ref> h;
+    if (table) {
+      lbk::ThrowReportedFault(ctx);
+    } else {
+      h.resize(T > 0 ? T : 1);
+      m_max = 1;
+      total = 0;
+      for (int t = 0; t < T; ++t) {
+        LBK_EXPECT(a->leaf_value[t] && a->feature[t] && a->split_value[t] && a->max_nodes[t] >= 1, "bad tree arrays");
+        LBK_EXPECT(total + a->max_nodes[t] < (int64_t{1} << 31), "ensemble too large");
+        h[t] = lbk_tree_ref{a->leaf_value[t], a->feature[t], a->split_value[t], a->max_nodes[t], static_cast<int32_t>(total)};
+        total += a->max_nodes[t];
+        m_max = std::max(m_max, a->max_nodes[t]);
+      }
     }
     const size_t esz = a->x_dtype == LBK_F32 ? 4 : 8;
     if (a->host_buffers) {
@@ -544,31 +559,36 @@ int lbk_predict(lbk_context* ctx, const lbk_predict_args* a)
       LBK_CUDA(cudaMemcpy2DAsync(dX, esz * F, X, esz * ldx, esz * F, N, cudaMemcpyHostToDevice, stream));
       X   = dX;
       ldx = F;
-      pred = s.alloc<double>(static_cast<size_t>(N) * K);
-      ldp  = K;
-      for (int t = 0; t < a->n_trees; ++t) {
-        const int m = a->max_nodes[t];
+      pred = s.alloc<double>(static_cast<size_t>(N) * columns);
+      ldp  = columns;
+      for (int t = 0; t < T; ++t) {
+        const int m = h[t].max_nodes;
         double* dl  = s.alloc<double>(static_cast<size_t>(m) * K);
         double* ds  = s.alloc<double>(m);
         int32_t* df = s.alloc<int32_t>(m);
-        LBK_CUDA(cudaMemcpyAsync(dl, leaf[t], sizeof(double) * m * K, cudaMemcpyHostToDevice, stream));
-        LBK_CUDA(cudaMemcpyAsync(ds, split[t], sizeof(double) * m, cudaMemcpyHostToDevice, stream));
-        LBK_CUDA(cudaMemcpyAsync(df, feat[t], sizeof(int32_t) * m, cudaMemcpyHostToDevice, stream));
-        leaf[t]  = dl;
-        split[t] = ds;
-        feat[t]  = df;
+        LBK_CUDA(cudaMemcpyAsync(dl, h[t].leaf, sizeof(double) * m * K, cudaMemcpyHostToDevice, stream));
+        LBK_CUDA(cudaMemcpyAsync(ds, h[t].split, sizeof(double) * m, cudaMemcpyHostToDevice, stream));
+        LBK_CUDA(cudaMemcpyAsync(df, h[t].feature, sizeof(int32_t) * m, cudaMemcpyHostToDevice, stream));
+        h[t].leaf    = dl;
+        h[t].split   = ds;
+        h[t].feature = df;
       }
     }
+    if (!table) {
+      lbk_tree_ref* d = s.alloc<lbk_tree_ref>(h.size());
+      if (T > 0) LBK_CUDA(cudaMemcpyAsync(d, h.data(), sizeof(lbk_tree_ref) * T, cudaMemcpyHostToDevice, stream));
+      table = d;  // (h is read before the call returns: it synchronises below)
+    }
     if (a->x_dtype == LBK_F32)
-      lbk::PredictLaunch<float>(ctx, s, static_cast<const float*>(X), ldx, N, F, K, a->n_trees, leaf.data(), feat.data(),
-                                split.data(), a->max_nodes, pred, ldp, stream);
+      lbk::PredictLaunch<float>(ctx, s, static_cast<const float*>(X), ldx, N, F, K, T, table, m_max, total, a->init,
+                                a->transform, pred, ldp, stream);
     else
-      lbk::PredictLaunch<double>(ctx, s, static_cast<const double*>(X), ldx, N, F, K, a->n_trees, leaf.data(),
-                                 feat.data(), split.data(), a->max_nodes, pred, ldp, stream);
+      lbk::PredictLaunch<double>(ctx, s, static_cast<const double*>(X), ldx, N, F, K, T, table, m_max, total, a->init,
+                                 a->transform, pred, ldp, stream);
     if (a->host_buffers)
-      LBK_CUDA(cudaMemcpy2DAsync(a->pred, sizeof(double) * a->ldp, pred, sizeof(double) * K, sizeof(double) * K, N,
+      LBK_CUDA(cudaMemcpy2DAsync(a->pred, sizeof(double) * a->ldp, pred, sizeof(double) * columns, sizeof(double) * columns, N,
                                  cudaMemcpyDeviceToHost, stream));
-    lbk::CheckDeviceStatus(ctx, stream);
+    if (!a->table) lbk::CheckDeviceStatus(ctx, stream);
   });
 }
 

@@ -164,18 +164,32 @@ std::pair<cudaEvent_t, cudaEvent_t> NextProfileEvents(lbk_context* ctx)
 
 void CheckDeviceStatus(lbk_context* ctx, cudaStream_t stream)
 {
-  int h = 0;
-  LBK_CUDA(cudaMemcpyAsync(&h, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, stream));
   LBK_CUDA(cudaStreamSynchronize(stream));
-  if (h != 0) {
-    LBK_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), stream));
-    throw Error(LBK_ERR_DEVICE, "a kernel reported fault code " + std::to_string(h));
-  }
+  ThrowReportedFault(ctx);
+}
+
+void ThrowReportedFault(lbk_context* ctx)
+{
+  volatile int* word = ctx->d_status;
+  const int h        = *word;
+  if (h == 0) return;
+  *word = 0;
+  throw Error(LBK_ERR_DEVICE, "a kernel reported fault code " + std::to_string(h));
 }
 
 // ABI boundary: exceptions never cross it.
 int Guard(lbk_context* ctx, const std::function<void()>& f)
 {
+  // the entry points make their context's device current; the caller's comes back on every way out
+  struct RestoreDevice {
+    int before = -1;
+    RestoreDevice() { cudaGetDevice(&before); }
+    ~RestoreDevice()
+    {
+      int now = -1;
+      if (before >= 0 && cudaGetDevice(&now) == cudaSuccess && now != before) cudaSetDevice(before);
+    }
+  } restore;
   try {
     f();
     return LBK_OK;
@@ -214,11 +228,15 @@ int lbk_context_create(int device, lbk_context** out)
       LBK_CUDA(cudaMemPoolCreate(&c->pool, &props));
       uint64_t keep = UINT64_MAX;  // keep freed scratch cached between calls
       LBK_CUDA(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep));
-      LBK_CUDA(cudaMalloc(&c->d_status, sizeof(int)));
-      LBK_CUDA(cudaMemset(c->d_status, 0, sizeof(int)));
+      // the status word lives in pinned host memory: kernels store a fault code straight into it, and
+      // the host reads it after a synchronisation without a copy
+      void* word = nullptr;
+      LBK_CUDA(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+      c->d_status  = static_cast<int*>(word);
+      *c->d_status = 0;
     } catch (...) {
       if (c->pool) cudaMemPoolDestroy(c->pool);
-      if (c->d_status) cudaFree(c->d_status);
+      if (c->d_status) cudaFreeHost(c->d_status);
       delete c;
       throw;
     }
@@ -233,7 +251,7 @@ void lbk_context_destroy(lbk_context* ctx)
   cudaDeviceSynchronize();
   lbk::DestroyExchange(ctx);
   if (ctx->owns_nccl && ctx->nccl_comm && nccl().CommDestroy) nccl().CommDestroy(ctx->nccl_comm);
-  if (ctx->d_status) cudaFree(ctx->d_status);
+  if (ctx->d_status) cudaFreeHost(ctx->d_status);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   for (auto& ev : ctx->prof_events) {
     cudaEventDestroy(ev.first);

@@ -10,6 +10,13 @@
 
 namespace lbk {
 
+// Stores a fault code into the context's status word (mapped host memory).
+__device__ inline void ReportFault(int* status, int code)
+{
+  *reinterpret_cast<volatile int*>(status) = code;
+  __threadfence_system();
+}
+
 // thrust::default_random_engine (minstd_rand): x <- 48271 x mod (2^31-1); a seed congruent to 0
 // becomes 1; the seed argument is first converted to the engine's 32-bit unsigned state type.
 struct MinStd {

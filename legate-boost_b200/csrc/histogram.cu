@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
   const unsigned hg_addr = static_cast<unsigned>(kHistBytes);
   // the staging area has to end before the histograms begin, and they inside what was asked for
   if (base + kWarps * kStageWords * 4 > hg_addr || hg_addr + 2u * kHistBytes > base + dyn_bytes) {
-    if (tid == 0 && p.status != nullptr) atomicExch(p.status, kFaultHistLayout);
+    if (tid == 0 && p.status != nullptr) ReportFault(p.status, kFaultHistLayout);
     return;
   }
   smem_t* stage_all = reinterpret_cast<smem_t*>(smem_raw);

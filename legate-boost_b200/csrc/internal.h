@@ -72,7 +72,7 @@ struct lbk_context {
   lbk_release_fn release_cb = nullptr;
   void* alloc_user          = nullptr;
   std::string err;
-  // device status word: 0 = ok, otherwise a kernel wrote a fault code
+  // status word in mapped host memory: 0 = ok, otherwise a kernel stored a fault code
   int* d_status = nullptr;
   // communicator
   int rank = 0, n_ranks = 1;
@@ -153,8 +153,10 @@ void ExchangeGatherAll(lbk_context* ctx, void* buf, void* dst, int n_seg, int B,
 // The event pair that brackets the next timed histogram launch (profile mode): the first that is
 // free, made on demand; when kMaxProfiledLaunches are in use the last one is used again.
 std::pair<cudaEvent_t, cudaEvent_t> NextProfileEvents(lbk_context* ctx);
-// Reads the device status word (synchronises the stream) and throws LBK_ERR_DEVICE if set.
+// Synchronises the stream, then throws LBK_ERR_DEVICE if a kernel stored a fault code.
 void CheckDeviceStatus(lbk_context* ctx, cudaStream_t stream);
+// The same without the synchronisation: what earlier, asynchronous calls have reported so far.
+void ThrowReportedFault(lbk_context* ctx);
 
 // Runs f, turning exceptions into a status code and an error text (the ABI boundary).
 int Guard(lbk_context* ctx, const std::function<void()>& f);
@@ -278,7 +280,7 @@ void InitRows(int32_t* row_index, int32_t* seg, int64_t n_rows, cudaStream_t str
 // predict.cu
 template <typename T>
 void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees,
-                   const double* const* leaf, const int32_t* const* feat, const double* const* split,
-                   const int32_t* max_nodes, double* pred, int64_t ldp, cudaStream_t stream);
+                   const lbk_tree_ref* d_trees /* device */, int m_max /* nodes of the largest tree */, int64_t total_nodes,
+                   const double* init, int transform, double* pred, int64_t ldp, cudaStream_t stream);
 
 }  // namespace lbk

@@ -50,13 +50,7 @@ struct NodeOf<float> {
   using type = Node8;
 };
 
-struct TreePtrs {
-  const double* leaf;
-  const int32_t* feature;
-  const double* split;
-  int max_nodes;
-  int node_off;  // offset of this tree's first node in the packed arrays
-};
+using TreePtrs = lbk_tree_ref;  // node_off: offset of the tree's first node in the packed arrays
 
 __device__ inline void MakeNode(Node8& n, double split, int foff)
 {
@@ -123,7 +117,7 @@ __device__ inline bool MbarWait(unsigned bar, unsigned parity, int* status)
     if (MbarTryWait(bar, parity)) return true;
     if (spin > 64) __nanosleep(256);
   }
-  atomicExch(status, kFaultPredictStaging);
+  ReportFault(status, kFaultPredictStaging);
   return false;
 }
 
@@ -195,13 +189,112 @@ __global__ void k_pack_complete(const TreePtrs* __restrict__ trees, int K, int F
   }
 }
 
+// ---- few rows ---------------------------------------------------------------------------------
+// What is added to the sums and what becomes of them: initial prediction, then probabilities.
+struct PredictOut {
+  double* pred;
+  int64_t ldp;
+  const double* init;  // [K] or null
+  int transform;       // LBK_RAW, LBK_LOGISTIC (two columns: 1 - p, p) or LBK_SOFTMAX
+};
+
+// The K raw predictions of one row -> its row of the output.  `raw` and the row may be the same.
+__device__ inline void FinishRow(const double* raw, int stride, int K, double* out, int transform)
+{
+  if (transform == LBK_RAW) {
+    for (int k = 0; k < K; ++k) out[k] = raw[k * stride];
+  } else if (transform == LBK_LOGISTIC) {
+    const double p = 1.0 / (1.0 + exp(-raw[0]));
+    out[0] = 1.0 - p;
+    out[1] = p;
+  } else {
+    double top = raw[0];
+    for (int k = 1; k < K; ++k) top = fmax(top, raw[k * stride]);
+    double sum = 0.0;
+    for (int k = 0; k < K; ++k) {
+      const double e = exp(raw[k * stride] - top);
+      out[k]         = e;
+      sum += e;
+    }
+    for (int k = 0; k < K; ++k) out[k] = out[k] / sum;
+  }
+}
+
+// One launch that walks the trees where they lie: a block takes `rows_per_block` rows, its threads take
+// (row, tree) pairs, trees in neighbouring lanes, and leave what each walk adds in shared memory; the
+// sums are then made in tree order, one thread per (row, output).  Bound by the latency of one walk
+// (two dependent loads per level from L2) plus the ordered sum, as long as there are few rows; nothing
+// is packed or staged, which for 16 rows and 100 trees of depth 6 takes longer than the walks.
+constexpr int kRowsThreads = 256;
+
+template <typename T>
+__global__ void __launch_bounds__(kRowsThreads)
+  k_predict_rows(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees, int rows_per_block,
+                 const TreePtrs* __restrict__ trees, PredictOut o)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  // [rows][trees] values (K == 1) or addresses of the leaves' values | [rows][K] sums | [rows][F] X
+  double* vals        = reinterpret_cast<double*>(smem_raw);
+  const double** adrs = reinterpret_cast<const double**>(smem_raw);
+  double* sums        = vals + static_cast<size_t>(rows_per_block) * n_trees;
+  T* xs               = reinterpret_cast<T*>(sums + static_cast<size_t>(rows_per_block) * K);
+  const int tid       = threadIdx.x;
+  const int64_t row0  = static_cast<int64_t>(blockIdx.x) * rows_per_block;
+  const int rows      = static_cast<int>(n_rows - row0 < rows_per_block ? n_rows - row0 : rows_per_block);
+  for (int i = tid; i < rows * F; i += kRowsThreads) {
+    const int r = i / F;
+    xs[i]       = X[(row0 + r) * ldx + (i - r * F)];
+  }
+  __syncthreads();
+  for (int i = tid; i < rows * n_trees; i += kRowsThreads) {
+    const int r      = i / n_trees, t = i - r * n_trees;
+    const TreePtrs p = trees[t];
+    const T* xr      = xs + r * F;
+    int pos          = 0;
+    for (int depth = 0; depth < 100; ++depth) {
+      const int f        = __ldg(p.feature + pos);
+      const double split = __ldg(p.split + pos);
+      if (f < 0 || f >= F || 2 * pos + 2 >= p.max_nodes) break;
+      pos = 2 * pos + 1 + (static_cast<double>(xr[f]) <= split ? 0 : 1);
+    }
+    if (K == 1) vals[i] = __ldg(p.leaf + pos);
+    else adrs[i] = p.leaf + static_cast<int64_t>(pos) * K;
+  }
+  __syncthreads();
+  for (int i = tid; i < rows * K; i += kRowsThreads) {
+    const int r = i / K, k = i - r * K;
+    double acc  = 0.0;
+    if (K == 1) {
+      const double* v = vals + static_cast<size_t>(r) * n_trees;
+#pragma unroll 8
+      for (int t = 0; t < n_trees; ++t) acc += v[t];
+    } else {
+      const double* const* v = adrs + static_cast<size_t>(r) * n_trees;
+#pragma unroll 8
+      for (int t = 0; t < n_trees; ++t) acc += __ldg(v[t] + k);
+    }
+    sums[i] = o.init ? o.init[k] + acc : acc;
+  }
+  __syncthreads();
+  for (int r = tid; r < rows; r += kRowsThreads) FinishRow(sums + r * K, 1, K, o.pred + (row0 + r) * o.ldp, o.transform);
+}
+
+// What is left to do after a kernel that wrote the raw sums.
+__global__ void __launch_bounds__(256) k_finish_rows(int64_t n_rows, int K, PredictOut o)
+{
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (row >= n_rows) return;
+  double* p = o.pred + row * o.ldp;
+  FinishRow(p, 1, K, p, o.transform);
+}
+
 // Tiled kernel.  Shared memory: X tile [F][RB] | accumulators [K][RB] (K > 1) |
 // NBUF x TG x slot, slot = NI nodes (+ NL leaf values when K == 1).
 template <typename T, int RB, int TG, bool kLeafShared>
 __global__ void __launch_bounds__(RB)
   k_predict_tiled(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees,
                   const typename NodeOf<T>::type* __restrict__ nodes_c, const double* __restrict__ leaves_c,
-                  double* __restrict__ pred, int64_t ldp, int S, int NI, int NL, int* __restrict__ status)
+                  PredictOut o, int S, int NI, int NL, int* __restrict__ status)
 {
   using NodeT = typename NodeOf<T>::type;
   __shared__ __align__(8) unsigned long long s_bar[2];
@@ -338,9 +431,12 @@ __global__ void __launch_bounds__(RB)
   if (tid < rows_here) {
     const int64_t row = row0 + tid;
     if (K == 1) {
-      pred[row * ldp] = acc0;
+      o.pred[row * o.ldp] = o.init ? o.init[0] + acc0 : acc0;
     } else {
-      for (int k = 0; k < K; ++k) pred[row * ldp + k] = accs[k * RB + tid];
+      for (int k = 0; k < K; ++k) {
+        const double v          = accs[k * RB + tid];
+        o.pred[row * o.ldp + k] = o.init ? o.init[k] + v : v;
+      }
     }
   }
 }
@@ -350,13 +446,14 @@ template <typename T>
 __global__ void __launch_bounds__(128)
   k_predict_global(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int K, int n_trees,
                    const TreePtrs* __restrict__ trees, const typename NodeOf<T>::type* __restrict__ nodes,
-                   const double* __restrict__ leaves, double* __restrict__ pred, int64_t ldp)
+                   const double* __restrict__ leaves, PredictOut o)
 {
   using NodeT       = typename NodeOf<T>::type;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (row >= n_rows) return;
   const T* xr = X + row * ldx;
-  for (int k = 0; k < K; ++k) pred[row * ldp + k] = 0.0;
+  double* pred = o.pred + row * o.ldp;
+  for (int k = 0; k < K; ++k) pred[k] = 0.0;
   for (int t = 0; t < n_trees; ++t) {
     const int off = trees[t].node_off;
     int pos       = 0;
@@ -366,8 +463,10 @@ __global__ void __launch_bounds__(128)
       pos = 2 * pos + 1 + (xr[n.foff] <= n.split ? 0 : 1);
     }
     const double* lf = leaves + static_cast<int64_t>(off + pos) * K;
-    for (int k = 0; k < K; ++k) pred[row * ldp + k] += lf[k];
+    for (int k = 0; k < K; ++k) pred[k] += lf[k];
   }
+  if (o.init)
+    for (int k = 0; k < K; ++k) pred[k] = o.init[k] + pred[k];
 }
 
 template <typename T>
@@ -382,15 +481,14 @@ size_t TiledSmem(int rb, int tg, int nbuf, int F, int K, int NI, int NL, bool le
 
 template <typename T, int RB, int TG, bool kLeafShared>
 void LaunchTiled(const T* X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees,
-                 const typename NodeOf<T>::type* nodes_c, const double* leaves_c, double* pred, int64_t ldp, int S,
-                 int NI, int NL, size_t smem, int* status, cudaStream_t stream)
+                 const typename NodeOf<T>::type* nodes_c, const double* leaves_c, const PredictOut& o, int S, int NI, int NL, size_t smem, int* status, cudaStream_t stream)
 {
   if (smem > 48 * 1024)
     LBK_CUDA(cudaFuncSetAttribute(k_predict_tiled<T, RB, TG, kLeafShared>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)));
   const unsigned grid = static_cast<unsigned>((n_rows + RB - 1) / RB);
-  k_predict_tiled<T, RB, TG, kLeafShared><<<grid, RB, smem, stream>>>(X, ldx, n_rows, F, K, n_trees, nodes_c, leaves_c, pred, ldp, S,
-                                                          NI, NL, status);
+  k_predict_tiled<T, RB, TG, kLeafShared><<<grid, RB, smem, stream>>>(X, ldx, n_rows, F, K, n_trees, nodes_c, leaves_c, o, S, NI, NL,
+                                                                      status);
   LBK_LAUNCH_CHECK();
 }
 
@@ -398,28 +496,32 @@ void LaunchTiled(const T* X, int64_t ldx, int64_t n_rows, int F, int K, int n_tr
 
 template <typename T>
 void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees,
-                   const double* const* leaf, const int32_t* const* feat, const double* const* split,
-                   const int32_t* max_nodes, double* pred, int64_t ldp, cudaStream_t stream)
+                   const lbk_tree_ref* d_trees, int m_max, int64_t total_nodes, const double* init, int transform,
+                   double* pred, int64_t ldp, cudaStream_t stream)
 {
   using NodeT = typename NodeOf<T>::type;
   if (n_rows < 1) return;  // an empty shard returns at once (reference: predict.cu:35)
-  if (n_trees == 0) {
-    LBK_CUDA(cudaMemset2DAsync(pred, sizeof(double) * ldp, 0, sizeof(double) * K, n_rows, stream));
-    return;
-  }
-  std::vector<TreePtrs> h(n_trees);
-  int64_t total_nodes = 0;
-  int m_max           = 1;
-  for (int t = 0; t < n_trees; ++t) {
-    LBK_EXPECT(leaf[t] && feat[t] && split[t] && max_nodes[t] >= 1, "bad tree arrays");
-    h[t].leaf      = leaf[t];
-    h[t].feature   = feat[t];
-    h[t].split     = split[t];
-    h[t].max_nodes = max_nodes[t];
-    LBK_EXPECT(total_nodes + max_nodes[t] < (int64_t{1} << 31), "ensemble too large");
-    h[t].node_off = static_cast<int>(total_nodes);
-    total_nodes += max_nodes[t];
-    m_max = max_nodes[t] > m_max ? max_nodes[t] : m_max;
+  const PredictOut o{pred, ldp, init, transform};
+  auto finish = [&]() {
+    if (transform == LBK_RAW) return;
+    k_finish_rows<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(n_rows, K, o);
+    LBK_LAUNCH_CHECK();
+  };
+  // Few rows: walk the trees in place.  The tiled kernel gives a block 256 rows and brings every tree
+  // into shared memory per block, so that it needs tens of thousands of rows to fill the chip.
+  {
+    constexpr int64_t kRowsMax = 8192;
+    int r = static_cast<int>((n_rows + 4 * ctx->sm_count - 1) / (4 * ctx->sm_count));
+    r     = r < 1 ? 1 : r > 8 ? 8 : r;
+    auto need = [&](int rows) { return static_cast<size_t>(rows) * ((n_trees + K) * sizeof(double) + F * sizeof(T)); };
+    if (n_trees == 0) r = 1;
+    while (r > 1 && need(r) > 48 * 1024) r /= 2;
+    if (n_trees == 0 || (n_rows <= kRowsMax && need(r) <= 48 * 1024)) {
+      const unsigned grid = static_cast<unsigned>((n_rows + r - 1) / r);
+      k_predict_rows<T><<<grid, kRowsThreads, need(r), stream>>>(X, ldx, n_rows, F, K, n_trees, r, d_trees, o);
+      LBK_LAUNCH_CHECK();
+      return;
+    }
   }
   // a walk through M heap-ordered nodes takes at most S = floor(log2(M)) steps
   int S = 0;
@@ -452,18 +554,15 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
     }
   }
 
-  TreePtrs* d_trees = s.alloc<TreePtrs>(n_trees);
-  LBK_CUDA(cudaMemcpyAsync(d_trees, h.data(), sizeof(TreePtrs) * n_trees, cudaMemcpyHostToDevice, stream));
-  LBK_CUDA(cudaStreamSynchronize(stream));  // h is a local; the copy must have read it
-
   if (rb == 0) {
     NodeT* nodes   = s.alloc<NodeT>(total_nodes);
     double* leaves = s.alloc<double>(total_nodes * K);
     k_pack_trees<NodeT><<<n_trees, 256, 0, stream>>>(d_trees, K, F, 1, nodes, leaves);
     LBK_LAUNCH_CHECK();
     const unsigned grid = static_cast<unsigned>((n_rows + 127) / 128);
-    k_predict_global<T><<<grid, 128, 0, stream>>>(X, ldx, n_rows, K, n_trees, d_trees, nodes, leaves, pred, ldp);
+    k_predict_global<T><<<grid, 128, 0, stream>>>(X, ldx, n_rows, K, n_trees, d_trees, nodes, leaves, o);
     LBK_LAUNCH_CHECK();
+    finish();
     return;
   }
   NodeT* nodes_c   = s.alloc<NodeT>(static_cast<size_t>(n_trees) * NI);
@@ -473,8 +572,9 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   LBK_LAUNCH_CHECK();
 #define LBK_PREDICT_CASE(RB_, TG_, LS_)                                                                             \
   if (rb == RB_ && tg == TG_ && leaf_shared == LS_) {                                                               \
-    LaunchTiled<T, RB_, TG_, LS_>(X, ldx, n_rows, F, K, n_trees, nodes_c, leaves_c, pred, ldp, S, NI, NL, smem,     \
+    LaunchTiled<T, RB_, TG_, LS_>(X, ldx, n_rows, F, K, n_trees, nodes_c, leaves_c, o, S, NI, NL, smem,             \
                                   ctx->d_status, stream);                                                           \
+    finish();                                                                                                       \
     return;                                                                                                         \
   }
 #define LBK_PREDICT_ROW(RB_)                                                                                        \
@@ -489,11 +589,9 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   throw Error(LBK_ERR_ARGUMENT, "predict: no kernel for the chosen tile");
 }
 
-template void PredictLaunch<float>(lbk_context*, Scratch&, const float*, int64_t, int64_t, int, int, int,
-                                   const double* const*, const int32_t* const*, const double* const*, const int32_t*,
-                                   double*, int64_t, cudaStream_t);
+template void PredictLaunch<float>(lbk_context*, Scratch&, const float*, int64_t, int64_t, int, int, int, const lbk_tree_ref*,
+                                   int, int64_t, const double*, int, double*, int64_t, cudaStream_t);
 template void PredictLaunch<double>(lbk_context*, Scratch&, const double*, int64_t, int64_t, int, int, int,
-                                    const double* const*, const int32_t* const*, const double* const*, const int32_t*,
-                                    double*, int64_t, cudaStream_t);
+                                    const lbk_tree_ref*, int, int64_t, const double*, int, double*, int64_t, cudaStream_t);
 
 }  // namespace lbk

@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import library as L
-from .tree import Sketch, Tree, _row_layout
+from .tree import _ARRAYS, Sketch, Tree, TreeTable, _row_layout
 
 
 def _all_sum(t: torch.Tensor) -> torch.Tensor:
@@ -174,12 +174,31 @@ class _LBBase:
         return self
 
     def predict_raw(self, X):
+        return self._predict(X, L.RAW)
+
+    def _predict(self, X, transform):
+        """Initial prediction plus the trees' sums, and what `transform` makes of them, in one call.  The
+        table of the trees' addresses is kept as long as models_ holds the same tensors."""
         if X.shape[1] != self.n_features_in_:
             raise ValueError("X.shape[1] = {} should be equal to {}".format(X.shape[1], self.n_features_in_))
-        pred = self.model_init_.repeat(X.shape[0], 1)
-        if self.models_:
-            pred += Tree.batch_predict(self.models_, X)
-        return pred
+        assert X.is_cuda, "X must be a CUDA tensor (no CPU fallback)"
+        init = self.model_init_
+        if init.dtype != torch.float64 or not init.is_contiguous() or init.device != X.device:
+            init = init.to(device=X.device, dtype=torch.float64).contiguous()
+        if not self.models_:
+            raw = init.repeat(X.shape[0], 1)
+            return raw if transform == L.RAW else self._probabilities(raw)
+        table = self.__dict__.get("_table")
+        if table is None or not table.matches(self.models_):
+            assert all(isinstance(m, Tree) for m in self.models_)
+            table = TreeTable(list(map(_ARRAYS, self.models_)))
+            self._table = table if table.reusable else None
+        return table.predict(X, init.shape[0], init=init, transform=transform)
+
+    def __getstate__(self):
+        state = dict(self.__dict__)
+        state.pop("_table", None)  # addresses of this process
+        return state
 
     def __iter__(self):
         return iter(self.models_)
@@ -206,11 +225,16 @@ class LBClassifier(_LBBase):
 
     _objective = _LogLoss
 
-    def predict_proba(self, X):
-        pred = self._obj.transform(self.predict_raw(X))
+    def _probabilities(self, raw):
+        pred = self._obj.transform(raw)
         if pred.shape[1] == 1:
             pred = torch.cat([1.0 - pred, pred], dim=1)
         return pred
+
+    def predict_proba(self, X):
+        if type(self._obj) is not _LogLoss:
+            return self._probabilities(self.predict_raw(X))
+        return self._predict(X, L.LOGISTIC if self.model_init_.shape[0] == 1 else L.SOFTMAX)
 
     def predict(self, X):
         return self.predict_proba(X).argmax(dim=1)

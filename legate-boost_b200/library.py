@@ -76,7 +76,12 @@ class PredictArgs(C.Structure):
         ("split_value", C.POINTER(C.c_void_p)), ("max_nodes", C.POINTER(C.c_int32)),
         ("pred", C.c_void_p), ("ldp", C.c_int64), ("stream", C.c_void_p),
         ("host_buffers", C.c_int32),
+        ("table", C.c_void_p), ("table_max_nodes", C.c_int32), ("table_total_nodes", C.c_int64),
+        ("init", C.c_void_p), ("transform", C.c_int32),
     ]
+
+
+RAW, LOGISTIC, SOFTMAX = 0, 1, 2
 
 
 class HistogramArgs(C.Structure):

@@ -10,6 +10,8 @@ rank passes its own contiguous block of rows and all ranks get the same tree.
 import copy
 import ctypes as C
 import warnings
+from itertools import chain
+from operator import attrgetter, is_
 from typing import Any, Callable, List, Sequence, Union
 
 import numpy as np
@@ -26,8 +28,8 @@ def _dtype_code(t: torch.Tensor) -> int:
     raise ValueError("X must be float32 or float64")
 
 
-def _stream_ptr():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream_ptr(device_index=None):
+    return C.c_void_p(torch.cuda.current_stream(device_index).cuda_stream)
 
 
 def _row_layout(n_local: int):
@@ -138,40 +140,75 @@ def build_tree_arrays(X, g, h, *, max_depth, split_samples, seed, l1=0.0, l2=1.0
     return out
 
 
+_ARRAYS = attrgetter("leaf_value", "feature", "split_value")
+
+
+class TreeTable:
+    """The arrays of an ensemble's trees as the device table ``lbk_predict`` walks
+    (``lbk_predict_args.table``): addresses, not contents, so a tree that is changed in place needs no
+    new table.  ``arrays``: (leaf_value, feature, split_value) per tree, on one CUDA device."""
+
+    def __init__(self, arrays):
+        self.source = list(chain.from_iterable(arrays))
+        device = self.source[1].device
+        keep, rows, total = [], np.empty((len(arrays), 4), dtype=np.int64), 0
+        self.max_nodes, self.n_outputs = 1, 1
+        for i, (lv, ft, sv) in enumerate(arrays):
+            lv = lv.to(torch.float64).contiguous()
+            ft, sv = ft.to(torch.int32).contiguous(), sv.to(torch.float64).contiguous()
+            if ft.device != device or lv.device != device or sv.device != device:
+                raise ValueError("the trees of an ensemble must be on one device")
+            keep += [lv, ft, sv]
+            M = ft.shape[0]
+            if M < 1 or total + M >= 2 ** 31:
+                raise ValueError("bad tree arrays" if M < 1 else "ensemble too large")
+            rows[i] = lv.data_ptr(), ft.data_ptr(), sv.data_ptr(), M | total << 32
+            total += M
+            self.max_nodes = max(self.max_nodes, M)
+            if i == 0:
+                self.n_outputs = lv.shape[1] if lv.dim() == 2 else 1
+        # converted copies would not follow later changes of the originals: such a table is not kept
+        self.reusable = all(map(is_, keep, self.source))
+        self.keep, self.total_nodes, self.n_trees = keep, total, len(arrays)
+        self.table = torch.from_numpy(rows).to(device)
+        self.device = device
+
+    def matches(self, models) -> bool:
+        """Whether these models still hold the very tensors the table was made from."""
+        return (self.reusable and len(models) == self.n_trees
+                and all(map(is_, chain.from_iterable(map(_ARRAYS, models)), self.source)))
+
+    def predict(self, X, n_outputs, init=None, transform=L.RAW, ctx=None):
+        """pred (N, columns) float64: ``init`` (n_outputs values, or None) plus the trees' sums, transformed."""
+        if X.stride(1) != 1 and X.shape[0] > 0:
+            X = X.contiguous()
+        N, F = X.shape
+        columns = 2 if transform == L.LOGISTIC else n_outputs
+        pred = torch.empty((N, columns), dtype=torch.float64, device=X.device)
+        if N == 0:
+            return pred
+        if X.device != self.device:
+            raise ValueError("X and the trees must be on one device")
+        ctx = ctx or L.context(X.device.index)
+        a = L.PredictArgs()
+        a.X, a.x_dtype, a.ldx, a.n_rows = X.data_ptr(), _dtype_code(X), X.stride(0), N
+        a.n_features, a.n_outputs, a.n_trees = F, n_outputs, self.n_trees
+        a.pred, a.ldp = pred.data_ptr(), columns
+        a.stream = _stream_ptr(X.device.index)
+        a.table, a.table_max_nodes, a.table_total_nodes = self.table.data_ptr(), self.max_nodes, self.total_nodes
+        a.init, a.transform = init.data_ptr() if init is not None else None, transform
+        ctx.check(ctx.lib.lbk_predict(ctx.handle, C.byref(a)))
+        return pred
+
+
 def predict_arrays(X, trees, n_outputs=None, ctx=None):
     """Run ``lbk_predict``.  ``trees`` is a sequence of (leaf_value, feature, split_value) CUDA
     tensors.  Returns pred (N, K) float64."""
     assert X.is_cuda, "X must be a CUDA tensor (no CPU fallback)"
-    if X.stride(1) != 1 and X.shape[0] > 0:
-        X = X.contiguous()
-    N, F = X.shape
-    T = len(trees)
-    keep = []
-    K = n_outputs
-    for lv, ft, sv in trees:
-        lv = lv.to(torch.float64).contiguous()
-        if lv.dim() == 1:
-            lv = lv[:, None]
-        keep.append((lv, ft.to(torch.int32).contiguous(), sv.to(torch.float64).contiguous()))
-        K = lv.shape[1] if K is None else K
-    pred = torch.empty((N, K), dtype=torch.float64, device=X.device)
-    if N == 0:
-        return pred
-    ctx = ctx or L.context(X.device.index)
-    a = L.PredictArgs()
-    a.X, a.x_dtype, a.ldx, a.n_rows = X.data_ptr(), _dtype_code(X), X.stride(0), N
-    a.n_features, a.n_outputs, a.n_trees = F, K, T
-    PP = C.c_void_p * max(T, 1)
-    lp, fp, sp = PP(), PP(), PP()
-    mn = (C.c_int32 * max(T, 1))()
-    for i, (lv, ft, sv) in enumerate(keep):
-        lp[i], fp[i], sp[i], mn[i] = lv.data_ptr(), ft.data_ptr(), sv.data_ptr(), ft.shape[0]
-    a.leaf_value, a.feature, a.split_value, a.max_nodes = lp, fp, sp, mn
-    a.pred, a.ldp = pred.data_ptr(), K
-    a.stream = _stream_ptr()
-    with torch.cuda.device(X.device):
-        ctx.check(ctx.lib.lbk_predict(ctx.handle, C.byref(a)))
-    return pred
+    if len(trees) == 0:
+        return torch.zeros((X.shape[0], n_outputs), dtype=torch.float64, device=X.device)
+    table = TreeTable(trees)
+    return table.predict(X, table.n_outputs if n_outputs is None else n_outputs, ctx=ctx)
 
 
 def onnx_tree_ensemble_attributes(feature, split_value, leaf_value):
@@ -371,8 +408,7 @@ class Tree(BaseModel):
     @staticmethod
     def batch_predict(models: Sequence["Tree"], X: torch.Tensor) -> torch.Tensor:
         assert all(isinstance(m, Tree) for m in models)
-        return predict_arrays(X, [(m.leaf_value, m.feature, m.split_value) for m in models],
-                              n_outputs=models[0].leaf_value.shape[1])
+        return predict_arrays(X, list(map(_ARRAYS, models)), n_outputs=models[0].leaf_value.shape[1])
 
     def __str__(self) -> str:
         leaf_value = self.leaf_value.cpu().numpy()
