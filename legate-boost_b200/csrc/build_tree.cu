@@ -6,9 +6,9 @@
 //   :826-845 outputs.
 // Differences in how, not in what: bins and quantised pairs are computed once per tree; rows are
 // kept grouped by node with a stable partition instead of a radix sort; only the nodes that are
-// built are held in the reduction buffer that crosses ranks; the whole level loop is enqueued
-// without host synchronisation (the only synchronisation of a call is the read-back of the
-// number of bins after the split proposals, which sizes the histograms).
+// built are held in the reduction buffer that crosses ranks; a level is three launches (histograms, scan
+// and split search, repartition), enqueued without host synchronisation (where the number of bins decides
+// the layout the call waits once, for that number).
 #include <algorithm>
 #include <cstring>
 
@@ -200,49 +200,127 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   }
 
   // Tree (reference: struct Tree, build_tree.cu:785-809)
+  const bool keep_sums = a.trace_node_sums != nullptr && !a.host_buffers;
   TreeArrays tree;
   tree.leaf_value  = leaf_value;
   tree.feature     = feature;
   tree.split_value = split_value;
   tree.gain        = gain;
-  tree.node_sums   = s.alloc<GPairI64>(static_cast<size_t>(M) * K);
   tree.split_bin   = s.alloc<int32_t>(M);
   tree.max_nodes   = M;
-  LBK_CUDA(cudaMemsetAsync(leaf_value, 0, sizeof(double) * M * K, stream));
-  LBK_CUDA(cudaMemsetAsync(feature, 0xFF, sizeof(int32_t) * M, stream));
-  LBK_CUDA(cudaMemsetAsync(split_value, 0, sizeof(double) * M, stream));
-  LBK_CUDA(cudaMemsetAsync(gain, 0, sizeof(double) * M, stream));
-  LBK_CUDA(cudaMemsetAsync(tree.node_sums, 0, sizeof(GPairI64) * M * K, stream));
-  unsigned int* split_arrived = s.alloc<unsigned int>(M);  // see BestSplit
-  LBK_CUDA(cudaMemsetAsync(split_arrived, 0, sizeof(unsigned int) * M, stream));
 
-  // split proposals -> B (one host synchronisation); with a sketch buffer they and the binned
-  // matrix live in the caller's buffer and may come from an earlier call
   const bool sketch_save = a.sketch_mode == LBK_SKETCH_SAVE, sketch_reuse = a.sketch_mode == LBK_SKETCH_REUSE;
-  const SketchLayout sk  = SketchLayoutOf(N, F, a.split_samples, sizeof(T));
+  const int S            = a.split_samples;
+  const SketchLayout sk  = SketchLayoutOf(N, F, S, sizeof(T));
   unsigned char* skb     = static_cast<unsigned char*>(a.sketch);
   const bool in_sketch   = sketch_save || sketch_reuse;
-  T* proposals     = in_sketch ? reinterpret_cast<T*>(skb + sk.proposals) : s.alloc<T>(static_cast<size_t>(F) * a.split_samples);
+  T* cuts          = in_sketch ? reinterpret_cast<T*>(skb + sk.proposals) : s.alloc<T>(static_cast<size_t>(F) * S);
   int32_t* row_ptr = in_sketch ? reinterpret_cast<int32_t*>(skb + sk.row_ptr) : s.alloc<int32_t>(F + 1);
-  ProposalInfo pi;
+
+  // Does the host have to know how many bins there are?  They decide the width of the bin ids (above 256
+  // samples), the batches of a level whose histograms are larger than the cache (the reference's rule,
+  // below), and the layout that a trace, a sketch or other ranks see.  Otherwise everything is laid out for
+  // the upper bound F x S, and nothing waits for the device before the end of the tree.
+  auto cache_depth = [&](int64_t bins, size_t& max_histogram_nodes) {
+    // histogram cache rule (reference: build_tree.cu:1000-1017); identical on every rank
+    max_histogram_nodes = std::max<size_t>(1, size_t{1000000000} / (static_cast<size_t>(K) * bins * sizeof(GPairI64)));
+    int d = 0;
+    while (static_cast<size_t>(LevelEnd(d + 1)) <= max_histogram_nodes && d <= D) d++;
+    return d;
+  };
+  const int64_t bins_bound   = static_cast<int64_t>(F) * S;
+  size_t max_histogram_nodes = 0;
+  const bool wait_for_bins   = in_sketch || a.trace_hist != nullptr || ctx->n_ranks > 1 || S > 256 ||
+                             cache_depth(bins_bound, max_histogram_nodes) < D - 1;
+
+  // words that have to be zero before the first level: node sums, arrival counters and partition cursors of
+  // the nodes, tickets and merge counters of the histogram launches
+  constexpr int kTickets = 256;
+  HistScratch hist_scratch;
+  HistScratchNeeds(ctx, F, K, S <= 256 ? 1 : 2, S, N, hist_scratch);
+  size_t words = 0;
+  auto reserve = [&](size_t bytes) {
+    const size_t at = words;
+    words += (bytes + 15) / 16 * 16;
+    return at;
+  };
+  const size_t o_sums    = reserve(keep_sums ? 0 : sizeof(GPairI64) * M * K);
+  const size_t o_arrived = reserve(sizeof(unsigned int) * M);
+  const size_t o_cursor  = reserve(sizeof(unsigned long long) * M);
+  const size_t o_ticket  = reserve(sizeof(unsigned int) * kTickets);
+  const size_t o_arrive  = reserve(sizeof(unsigned int) * hist_scratch.n_arrive);
+  const size_t o_abs     = reserve(2 * sizeof(int));
+  unsigned char* zeroed  = static_cast<unsigned char*>(s.alloc_bytes(words));
+  tree.node_sums = keep_sums ? reinterpret_cast<GPairI64*>(a.trace_node_sums) : reinterpret_cast<GPairI64*>(zeroed + o_sums);
+  unsigned int* split_arrived  = reinterpret_cast<unsigned int*>(zeroed + o_arrived);
+  unsigned long long* cursor   = reinterpret_cast<unsigned long long*>(zeroed + o_cursor);
+  int* max_abs                 = reinterpret_cast<int*>(zeroed + o_abs);
+  hist_scratch.tickets         = reinterpret_cast<unsigned int*>(zeroed + o_ticket);
+  hist_scratch.n_tickets       = kTickets;
+  hist_scratch.arrive          = reinterpret_cast<unsigned int*>(zeroed + o_arrive);
+
+  // segments of a level's nodes: begins, then ends
+  const size_t max_level_nodes = D > 0 ? (size_t{1} << (D - 1)) : 1;
+  int32_t* seg_a  = s.alloc<int32_t>(2 * max_level_nodes);
+  int32_t* seg_b  = s.alloc<int32_t>(2 * max_level_nodes);
+  QuantParams* qp = s.alloc<QuantParams>(1);
+  double* sums    = s.alloc<double>(2);
+  int32_t* info   = s.alloc<int32_t>(2);
   SketchHeader head{};
   if (sketch_reuse) {
     LBK_CUDA(cudaMemcpyAsync(&head, skb, sizeof(head), cudaMemcpyDeviceToHost, stream));
     LBK_CUDA(cudaStreamSynchronize(stream));
     LBK_EXPECT(head.magic == kSketchMagic, "the sketch buffer holds no saved sketch");
-    LBK_EXPECT(head.n_rows == N && head.n_features == F && head.split_samples == a.split_samples &&
+    LBK_EXPECT(head.n_rows == N && head.n_features == F && head.split_samples == S &&
                  head.elem_bytes == static_cast<int32_t>(sizeof(T)),
                "the sketch was saved for a matrix of another shape or type");
     LBK_EXPECT(D <= 1 || head.has_feature_major, "the sketch was saved without the feature-major copy");
+  }
+  // the root's histogram, where its size is known already
+  const bool root_zeroed = !wait_for_bins && D > 0;
+  GPairI64* cache        = nullptr;
+  if (root_zeroed)
+    cache = s.alloc<GPairI64>(static_cast<size_t>(LevelEnd(std::max(D - 2, 0))) * K * bins_bound);
+  {
+    PrologueArgs<T> pa{};
+    pa.X            = X;
+    pa.ldx          = ldx;
+    pa.row_offset   = a.row_offset;
+    pa.n_local      = N;
+    pa.F            = F;
+    pa.S            = S;
+    pa.seed         = a.seed;
+    pa.dataset_rows = a.dataset_rows;
+    pa.cuts         = cuts;
+    pa.counts       = sketch_reuse ? nullptr : s.alloc<int32_t>(F);
+    pa.g            = g;
+    pa.h            = h;
+    pa.ldg          = ldg;
+    pa.K            = K;
+    pa.n_elements   = N * K;
+    pa.tree         = tree;
+    pa.root_begin   = seg_a;
+    pa.root_end     = seg_a + max_level_nodes;
+    pa.zero[0]      = zeroed;
+    pa.zero_n16[0]  = static_cast<int64_t>(words / 16);
+    pa.zero[1]      = tree.node_sums;
+    pa.zero_n16[1]  = keep_sums ? static_cast<int64_t>(M) * K : 0;
+    pa.zero[2]      = cache;
+    pa.zero_n16[2]  = root_zeroed ? static_cast<int64_t>(K) * bins_bound : 0;
+    Prologue<T>(ctx, s, pa, row_ptr, info, ctx->h_info, sums, qp, stream);
+  }
+  ProposalInfo pi{static_cast<int>(std::min<int64_t>(bins_bound, INT32_MAX)), S};
+  if (sketch_reuse) {
     pi.total_bins           = head.total_bins;
     pi.max_bins_per_feature = head.max_bins_per_feature;
-  } else {
-    pi = SplitProposals<T>(ctx, s, X, ldx, a.row_offset, N, F, a.split_samples, a.seed, a.dataset_rows, proposals,
-                           row_ptr, stream);
+  } else if (wait_for_bins) {
+    LBK_CUDA(cudaStreamSynchronize(stream));
+    pi.total_bins           = ctx->h_info[0];
+    pi.max_bins_per_feature = ctx->h_info[1];
+    LBK_EXPECT(pi.total_bins >= F, "every feature must have at least one proposal");
   }
-  const int B = pi.total_bins;
-  if (a.out_total_bins) *a.out_total_bins = B;
-  LBK_EXPECT(B >= F, "every feature must have at least one proposal");
+  const int B = pi.total_bins;  // (an upper bound unless wait_for_bins)
+  const int* max_bins_ptr = wait_for_bins ? nullptr : info + 1;
 
   // binned matrix, once per tree
   const int bin_bytes = pi.max_bins_per_feature <= 256 ? 1 : 2;
@@ -254,13 +332,13 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
                           : D > 1   ? s.alloc_bytes(static_cast<size_t>(F) * pitch_t * bin_bytes + 16)
                                     : nullptr;
   if (!sketch_reuse)
-    BinMatrix<T>(X, ldx, N, F, proposals, row_ptr, bins, bins_t, pitch_t, bin_bytes, pi.max_bins_per_feature, stream);
+    BinMatrix<T>(X, ldx, N, F, cuts, S, row_ptr, bins, bins_t, pitch_t, bin_bytes, pi.max_bins_per_feature, stream);
   if (sketch_save) {
     head.magic                = kSketchMagic;
     head.total_bins           = pi.total_bins;
     head.max_bins_per_feature = pi.max_bins_per_feature;
     head.n_features           = F;
-    head.split_samples        = a.split_samples;
+    head.split_samples        = S;
     head.elem_bytes           = static_cast<int32_t>(sizeof(T));
     head.has_feature_major    = 1;
     head.n_rows               = N;
@@ -269,32 +347,26 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   }
 
   // quantised pairs and root sums
-  QuantParams* qp = s.alloc<QuantParams>(1);
-  int2* gpair     = s.alloc<int2>(static_cast<size_t>(N) * K);
-  int* max_abs    = s.alloc<int>(2);
-  Quantise(ctx, s, g, h, ldg, a.row_offset, N, K, a.seed, gpair, tree.node_sums, qp, max_abs, stream);
-  RootLeaf(tree, K, qp, a.l1_regularization, a.l2_regularization, stream);
+  int2* gpair = s.alloc<int2>(static_cast<size_t>(N) * K);
+  Quantise(ctx, g, h, ldg, a.row_offset, N, K, a.seed, gpair, tree.node_sums, qp, max_abs, stream);
 
-  // histogram cache rule (reference: build_tree.cu:1000-1017); identical on every rank
-  const size_t bytes_per_node      = static_cast<size_t>(K) * B * sizeof(GPairI64);
-  const size_t max_histogram_nodes = std::max<size_t>(1, size_t{1000000000} / bytes_per_node);
-  int cdepth                       = 0;
-  while (static_cast<size_t>(LevelEnd(cdepth + 1)) <= max_histogram_nodes && cdepth <= D) cdepth++;
-  // levels >= D are never evaluated; no need to hold them
+  const int cdepth = cache_depth(B, max_histogram_nodes);
+  // levels >= D are never evaluated; no need to hold them.  The last level's histograms are evaluated as
+  // they are scanned and not written, unless they are built in place or a trace wants them.
   const int cache_levels  = std::min(cdepth, std::max(D - 1, 0));
   const int cache_nodes   = LevelEnd(cache_levels);
   const int cache_end_ref = LevelEnd(cdepth);  // extent of the reference's cached histogram
   const int64_t max_batch = static_cast<int>(max_histogram_nodes);
   const size_t node_elems = static_cast<size_t>(K) * B;
-  GPairI64* cache         = s.alloc<GPairI64>(static_cast<size_t>(cache_nodes) * node_elems);
+  if (cache == nullptr) {
+    const bool last_held = a.trace_hist != nullptr || cache_levels < D - 1 || D <= 1;
+    cache = s.alloc<GPairI64>(static_cast<size_t>(last_held ? cache_nodes : LevelEnd(D - 2)) * node_elems);
+  }
 
-  // rows grouped by node, ping-pong
-  int32_t* rows_a = s.alloc<int32_t>(N);
-  int32_t* rows_b = s.alloc<int32_t>(N);
-  const size_t max_level_nodes = D > 0 ? (size_t{1} << (D - 1)) : 1;
-  int32_t* seg_a  = s.alloc<int32_t>(2 * max_level_nodes + 2);
-  int32_t* seg_b  = s.alloc<int32_t>(2 * max_level_nodes + 2);
-  InitRows(rows_a, seg_a, N, stream);
+  // rows grouped by node, ping-pong; the root's rows are in order and need no list
+  int32_t* rows_a = nullptr;
+  int32_t* rows_b = D > 1 ? s.alloc<int32_t>(N) : nullptr;
+  int32_t* rows_c = D > 2 ? s.alloc<int32_t>(N) : nullptr;
   // With few outputs the quantised pairs are kept in row_index order: at the root that is the order
   // they are in already, and every repartition moves them together with the row ids (8 K bytes read
   // and written per row and level, as streams), so that the histogram kernel reads the pairs of a
@@ -306,11 +378,21 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
 
   SplitParams sp{a.l1_regularization, a.l2_regularization, a.min_split_gain, fset};
 
-  // reduction buffer for the built nodes of a batch; grown on demand
-  GPairI64* built    = nullptr;
-  size_t built_nodes = 0;
+  // raw sums of the built nodes of a level, alternating so that a level can zero the next one's
+  GPairI64* built[2]    = {nullptr, nullptr};
+  size_t built_nodes[2] = {0, 0};
+  auto built_buffer = [&](int which, size_t nodes) {
+    if (built_nodes[which] < nodes) {
+      if (built[which]) s.free_one(built[which]);
+      built[which]       = s.alloc<GPairI64>(nodes * node_elems);
+      built_nodes[which] = nodes;
+    }
+    return built[which];
+  };
+  bool built_zeroed   = root_zeroed;
   GPairI64* fresh    = nullptr;  // histogram of a batch that lies outside the cache
   size_t fresh_nodes = 0;
+  if (hist_scratch.partial_bytes > 0 && N > 0) hist_scratch.partial = s.alloc_bytes(hist_scratch.partial_bytes);
   // the most recently replaced "cache" of the reference, to decide parent availability
   int ref_hist_begin = 0, ref_hist_end = cache_end_ref;
 
@@ -342,12 +424,15 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
         ref_hist_begin = nb;
         ref_hist_end   = ne;
       }
-      const bool parent_available = nb > 0 && ((nb - 1) / 2) >= ref_hist_begin && ((nb - 1) / 2) < ref_hist_end;
-      const bool in_cache         = ne <= cache_nodes;
+      // a parent's histogram is there only for the whole levels of the cache
+      const bool derive = nb > 0 && ((nb - 1) / 2) >= ref_hist_begin && ((nb - 1) / 2) < ref_hist_end;
+      const bool in_cache = ne <= cache_nodes;
+      // is this batch's histogram written out?  The level below reads it if it derives from it.
+      const bool write_hist = depth < D - 1 || a.trace_hist != nullptr;
       // where this batch's histograms live
-      GPairI64* level_hist;
+      GPairI64* level_hist = nullptr;
       if (in_cache) {
-        level_hist = cache + static_cast<size_t>(nb) * node_elems;
+        if (write_hist || !derive) level_hist = cache + static_cast<size_t>(nb) * node_elems;
       } else {
         if (fresh_nodes < static_cast<size_t>(n_nodes)) {
           if (fresh) s.free_one(fresh);
@@ -356,7 +441,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
         }
         level_hist = fresh;
       }
-      const int n_slots = (parent_available && nb > 0) ? n_nodes / 2 : n_nodes;
+      const int n_slots = derive ? n_nodes / 2 : n_nodes;
       // With several ranks the level is built into a buffer the other ranks' GPUs can read, and
       // every rank sums, scans and searches only the features it owns (see exchange.cu); where the
       // peers cannot be mapped the whole buffer is all-reduced and every rank does everything.
@@ -364,22 +449,9 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       const int f_begin = owned ? OwnedBegin(ctx->rank, ctx->n_ranks, F) : 0;
       const int f_end   = owned ? OwnedBegin(ctx->rank + 1, ctx->n_ranks, F) : F;
       // built buffer: when nothing is derived the level histogram itself is the target
-      GPairI64* target;
-      if (n_slots == n_nodes) {
-        target = level_hist;
-      } else {
-        if (built_nodes < static_cast<size_t>(n_slots)) {
-          if (built) s.free_one(built);
-          built       = s.alloc<GPairI64>(static_cast<size_t>(n_slots) * node_elems);
-          built_nodes = n_slots;
-        }
-        target = built;
+      GPairI64* target = derive ? built_buffer(depth & 1, n_slots) : level_hist;
+      if (a.trace_hist != nullptr && derive)  // (nodes that do not exist read as zeros in a trace)
         LBK_CUDA(cudaMemsetAsync(level_hist, 0, sizeof(GPairI64) * n_nodes * node_elems, stream));
-      }
-      // (the build zeroes the target where it needs it zeroed)
-
-      int32_t* slot_of_node = s.alloc<int32_t>(n_nodes);
-      PlanBuilt(tree.node_sums, K, nb, n_nodes, parent_available, slot_of_node, stream);
 
       HistLevel lv;
       lv.bins                 = bins;
@@ -389,38 +461,50 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       lv.K                    = K;
       lv.B                    = B;
       lv.max_bins_per_feature = pi.max_bins_per_feature;
+      lv.max_bins_ptr         = max_bins_ptr;
       lv.row_ptr              = row_ptr;
       lv.gpair                = stream_pairs ? pairs_a : gpair;
       lv.pairs_by_position    = stream_pairs;
       lv.gpair_f              = nullptr;
       lv.max_abs              = max_abs;
       lv.row_index            = rows_a;
-      lv.seg                  = seg_a;
+      lv.seg_begin            = seg_a + (nb - level_begin);
+      lv.seg_end              = seg_a + max_level_nodes + (nb - level_begin);
       lv.n_nodes              = n_nodes;
-      lv.seg_node_offset      = nb - level_begin;
-      lv.slot_of_node         = slot_of_node;
+      lv.node_sums            = derive ? tree.node_sums : nullptr;
+      lv.node_begin           = nb;
       lv.out                  = target;
       lv.float_mode           = false;
+      lv.scratch              = &hist_scratch;
       // build + sum over ranks (reference: :1107-1113 reduces the whole batch; only built nodes here)
       const GPairI64* summed = static_cast<const GPairI64*>(
-        BuildHistogramSummed(ctx, s, lv, n_slots, HistSum::kSumOwned, false, true, stream));
+        BuildHistogramSummed(ctx, s, lv, n_slots, HistSum::kSumOwned, false, !built_zeroed, stream));
 
-      const GPairI64* parent_hist = nullptr;
-      int parent_begin            = 0;
-      if (parent_available) {
-        parent_begin = LevelBegin(depth - 1);
-        parent_hist  = cache + static_cast<size_t>(parent_begin) * node_elems;
-      }
-      ScanLevel(summed, slot_of_node, level_hist, parent_hist, parent_begin, tree.node_sums, nb, n_nodes, K, f_begin,
-                f_end, B, row_ptr, parent_available, stream);
+      ScanSplitLevel sl;
+      sl.built        = summed;
+      sl.level_hist   = level_hist;
+      sl.parent_begin = derive ? LevelBegin(depth - 1) : 0;
+      sl.parent_hist  = derive ? cache + static_cast<size_t>(sl.parent_begin) * node_elems : nullptr;
+      // does the next level derive?  (the same rule as above, one level ahead)
+      const int next_begin = LevelBegin(depth + 1), next_end = LevelEnd(depth + 1);
+      const bool next_derives = depth + 1 < D && level_nodes * int64_t{2} <= max_batch && next_begin >= ref_hist_begin &&
+                                next_end <= ref_hist_end && (next_begin - 1) / 2 >= ref_hist_begin;
+      built_zeroed    = next_derives && batches.size() == 1 && ctx->n_ranks <= 1;
+      sl.next_built   = built_zeroed ? built_buffer((depth + 1) & 1, n_nodes) : nullptr;
+      sl.bin_stride   = B;
+      sl.node_begin   = nb;
+      sl.n_nodes      = n_nodes;
+      sl.K            = K;
+      sl.f_begin      = f_begin;
+      sl.f_end        = f_end;
+      sl.derive       = derive;
+      sl.write_hist   = write_hist;
+      ScanSplit<T>(ctx, s, sl, F, row_ptr, cuts, S, qp, sp, tree, split_arrived, owned, stream);
       if (a.trace_hist && nb < a.trace_nodes) {
         const int cnt = std::min(ne, a.trace_nodes) - nb;
         LBK_CUDA(cudaMemcpyAsync(a.trace_hist + static_cast<size_t>(nb) * node_elems * 2, level_hist,
                                  sizeof(GPairI64) * cnt * node_elems, cudaMemcpyDeviceToDevice, stream));
       }
-      BestSplit<T>(ctx, s, level_hist, nb, n_nodes, K, F, B, row_ptr, proposals, qp, sp, tree, split_arrived, f_begin,
-                   f_end, owned, stream);
-      s.free_one(slot_of_node);
     }
     if (depth < D - 1) {
       PartitionLevel pl;
@@ -429,9 +513,12 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       pl.bin_pitch     = pitch_t;
       pl.n_rows        = N;
       pl.row_index_in  = rows_a;
-      pl.seg_in        = seg_a;
+      pl.seg_begin     = seg_a;
+      pl.seg_end       = seg_a + max_level_nodes;
       pl.row_index_out = rows_b;
-      pl.seg_out       = seg_b;
+      pl.seg_begin_out = seg_b;
+      pl.seg_end_out   = seg_b + max_level_nodes;
+      pl.cursor        = cursor;
       pl.node_begin    = level_begin;
       pl.n_nodes       = level_nodes;
       pl.feature       = tree.feature;
@@ -442,13 +529,16 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
         pl.K         = K;
       }
       PartitionRows(ctx, s, pl, stream);
-      std::swap(rows_a, rows_b);
+      // the lists alternate; the root had none
+      int32_t* spare = depth == 0 ? rows_c : rows_a;
+      rows_a         = rows_b;
+      rows_b         = spare;
       std::swap(seg_a, seg_b);
       std::swap(pairs_a, pairs_b);
     }
   }
 
-  WriteHessian(tree.node_sums, qp, hessian, static_cast<int64_t>(M) * K, stream);
+  FinishTree(tree, qp, K, a.l1_regularization, a.l2_regularization, hessian, stream);
   if (a.out_leaf != nullptr && N > 0) {
     int32_t* d_leaf = a.host_buffers ? s.alloc<int32_t>(static_cast<size_t>(N)) : a.out_leaf;
     const int64_t pitch = static_cast<int64_t>((F + kGroup - 1) / kGroup) * kGroup;
@@ -457,8 +547,8 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     if (a.host_buffers)
       LBK_CUDA(cudaMemcpyAsync(a.out_leaf, d_leaf, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, stream));
   }
-  if (a.trace_node_sums)
-    LBK_CUDA(cudaMemcpyAsync(a.trace_node_sums, tree.node_sums, sizeof(GPairI64) * M * K, cudaMemcpyDeviceToDevice, stream));
+  if (a.trace_node_sums && !keep_sums)
+    LBK_CUDA(cudaMemcpyAsync(a.trace_node_sums, tree.node_sums, sizeof(GPairI64) * M * K, cudaMemcpyDefault, stream));
   if (a.host_buffers) {
     LBK_CUDA(cudaMemcpyAsync(a.leaf_value, leaf_value, sizeof(double) * M * K, cudaMemcpyDeviceToHost, stream));
     LBK_CUDA(cudaMemcpyAsync(a.feature, feature, sizeof(int32_t) * M, cudaMemcpyDeviceToHost, stream));
@@ -467,6 +557,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     LBK_CUDA(cudaMemcpyAsync(a.hessian, hessian, sizeof(double) * M * K, cudaMemcpyDeviceToHost, stream));
   }
   CheckDeviceStatus(ctx, stream);  // synchronises, as the reference's task does (:1356)
+  if (a.out_total_bins) *a.out_total_bins = sketch_reuse ? head.total_bins : ctx->h_info[0];
 }
 
 }  // namespace
@@ -630,11 +721,11 @@ int lbk_bin_matrix(lbk_context* ctx, const void* X, int x_dtype, int64_t ldx, in
     for (int f = 0; f < n_features; ++f) mb = std::max(mb, rp[f + 1] - rp[f]);
     LBK_EXPECT(bin_bytes == 2 || mb <= 256, "one-byte bins need <= 256 proposals per feature");
     if (x_dtype == LBK_F32)
-      lbk::BinMatrix<float>(static_cast<const float*>(X), ldx, n_rows, n_features, static_cast<const float*>(proposals),
+      lbk::BinMatrix<float>(static_cast<const float*>(X), ldx, n_rows, n_features, static_cast<const float*>(proposals), 0,
                             row_ptr, bins, nullptr, 0, bin_bytes, mb, stream);
     else
       lbk::BinMatrix<double>(static_cast<const double*>(X), ldx, n_rows, n_features,
-                             static_cast<const double*>(proposals), row_ptr, bins, nullptr, 0, bin_bytes, mb, stream);
+                             static_cast<const double*>(proposals), 0, row_ptr, bins, nullptr, 0, bin_bytes, mb, stream);
   });
 }
 
@@ -647,9 +738,20 @@ int lbk_quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg
     LBK_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     lbk::Scratch s(ctx, stream);
-    lbk::Quantise(ctx, s, g, h, ldg, row_offset, n_local_rows, n_outputs, seed, reinterpret_cast<int2*>(gpair),
-                  reinterpret_cast<lbk::GPairI64*>(root_sums), reinterpret_cast<lbk::QuantParams*>(scale),
-                  max_abs ? max_abs : s.alloc<int>(2), stream);
+    int* abs = max_abs ? max_abs : s.alloc<int>(2);
+    LBK_CUDA(cudaMemsetAsync(root_sums, 0, sizeof(lbk::GPairI64) * n_outputs, stream));
+    LBK_CUDA(cudaMemsetAsync(abs, 0, 2 * sizeof(int), stream));
+    lbk::PrologueArgs<float> pa{};
+    pa.g          = g;
+    pa.h          = h;
+    pa.ldg        = ldg;
+    pa.K          = n_outputs;
+    pa.n_elements = n_local_rows * n_outputs;
+    pa.S          = 1;
+    lbk::QuantParams* qp = reinterpret_cast<lbk::QuantParams*>(scale);
+    lbk::Prologue<float>(ctx, s, pa, nullptr, nullptr, nullptr, s.alloc<double>(2), qp, stream);
+    lbk::Quantise(ctx, g, h, ldg, row_offset, n_local_rows, n_outputs, seed, reinterpret_cast<int2*>(gpair),
+                  reinterpret_cast<lbk::GPairI64*>(root_sums), qp, abs, stream);
   });
 }
 
@@ -724,10 +826,9 @@ int lbk_histogram(lbk_context* ctx, const lbk_histogram_args* a)
     lv.max_abs              = a->host_buffers ? nullptr : reinterpret_cast<const int*>(a->max_abs);
     lv.pairs_by_position    = a->pairs_by_position != 0;
     lv.row_index            = row_index;
-    lv.seg                  = seg;
+    lv.seg_begin            = seg;
+    lv.seg_end              = seg + 1;
     lv.n_nodes              = a->n_nodes;
-    lv.seg_node_offset      = 0;
-    lv.slot_of_node         = nullptr;
     lv.out                  = hist;
     lv.float_mode           = a->mode == 1;
     if (a->all_reduce == 1) lbk::BuildHistogramSummed(ctx, s, lv, a->n_nodes, lbk::HistSum::kSumEverywhere, true, true, stream);

@@ -100,7 +100,25 @@ Scratch::~Scratch()
     if (p) ReleaseScratch(ctx_, p, stream_);
 }
 
+// Small buffers are cut from blocks of kSlab bytes (a stream-ordered allocation and its release cost the
+// host about a microsecond and a half, and a tree has dozens of small buffers); they live as long as the Scratch.
 void* Scratch::alloc_bytes(size_t bytes)
+{
+  constexpr size_t kSlab = size_t{1} << 20, kSmall = size_t{1} << 18;
+  if (bytes <= kSmall) {
+    const size_t need = (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+    if (slab_ == nullptr || slab_used_ + need > kSlab) {
+      slab_      = static_cast<char*>(AllocBlock(kSlab));
+      slab_used_ = 0;
+    }
+    void* p = slab_ + slab_used_;
+    slab_used_ += need;
+    return p;
+  }
+  return AllocBlock(bytes);
+}
+
+void* Scratch::AllocBlock(size_t bytes)
 {
   void* p = nullptr;
   if (ctx_->alloc_cb != nullptr) {
@@ -231,9 +249,10 @@ int lbk_context_create(int device, lbk_context** out)
       // the status word lives in pinned host memory: kernels store a fault code straight into it, and
       // the host reads it after a synchronisation without a copy
       void* word = nullptr;
-      LBK_CUDA(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+      LBK_CUDA(cudaHostAlloc(&word, 4 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
       c->d_status  = static_cast<int*>(word);
       *c->d_status = 0;
+      c->h_info    = static_cast<int32_t*>(word) + 2;
     } catch (...) {
       if (c->pool) cudaMemPoolDestroy(c->pool);
       if (c->d_status) cudaFreeHost(c->d_status);

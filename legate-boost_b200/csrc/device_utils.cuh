@@ -17,29 +17,38 @@ __device__ inline void ReportFault(int* status, int code)
   __threadfence_system();
 }
 
+// x mod (2^31 - 1) for x < 2^62: the two 31-bit halves add up to the same residue (2^31 is 1 modulo the
+// Mersenne prime), twice, and one subtraction is left.
+__host__ __device__ inline uint32_t ModMersenne31(unsigned long long x)
+{
+  x = (x & 2147483647ull) + (x >> 31);
+  uint32_t r = static_cast<uint32_t>(x & 2147483647ull) + static_cast<uint32_t>(x >> 31);
+  return r >= 2147483647u ? r - 2147483647u : r;
+}
+
 // thrust::default_random_engine (minstd_rand): x <- 48271 x mod (2^31-1); a seed congruent to 0
 // becomes 1; the seed argument is first converted to the engine's 32-bit unsigned state type.
 struct MinStd {
   uint32_t x;
   __host__ __device__ explicit MinStd(uint32_t s)
   {
-    uint32_t r = s % 2147483647u;
+    uint32_t r = ModMersenne31(s);
     x          = r == 0 ? 1u : r;
   }
   __host__ __device__ uint32_t next()
   {
-    x = static_cast<uint32_t>((48271ull * x) % 2147483647ull);
+    x = ModMersenne31(48271ull * x);
     return x;
   }
   __host__ __device__ void discard(unsigned long long z)
   {
     unsigned long long mult = 48271ull, mult_z = 1ull;
     while (z > 0) {
-      if (z & 1ull) mult_z = (mult_z * mult) % 2147483647ull;
+      if (z & 1ull) mult_z = ModMersenne31(mult_z * mult);
       z >>= 1;
-      mult = (mult * mult) % 2147483647ull;
+      mult = ModMersenne31(mult * mult);
     }
-    x = static_cast<uint32_t>((mult_z * x) % 2147483647ull);
+    x = ModMersenne31(mult_z * x);
   }
   // thrust::uniform_real_distribution<double>(a,b)
   __host__ __device__ double uniform_real(double a, double b)
@@ -47,6 +56,15 @@ struct MinStd {
     double r = static_cast<double>(next() - 1u);
     r /= 2147483646.0;
     return (r * (b - a)) + a;
+  }
+  // uniform_real(0, 1) < r, for 0 <= r < 1.  The quotient is only formed when the product with the rounded
+  // reciprocal (off by less than 4e-16) is too close to r to tell.
+  __device__ bool uniform_below(double r)
+  {
+    const double n = static_cast<double>(next() - 1u);
+    const double u = n * (1.0 / 2147483646.0);
+    if (fabs(u - r) > 1e-14) return u < r;
+    return n / 2147483646.0 < r;
   }
   // thrust::uniform_int_distribution<int64_t>(a,b): truncated real draw from [a, b+1)
   __host__ __device__ long long uniform_int(long long a, long long b)
@@ -89,10 +107,10 @@ __device__ inline int2 QuantisePair(double g, double h, const QuantParams& qp, l
   const double fh = floor(sh);
   const double rg = sg - fg;
   const double rh = sh - fh;
-  const double ug = eng.uniform_real(0.0, 1.0);
-  const double uh = eng.uniform_real(0.0, 1.0);
-  const long long qg = static_cast<long long>(fg + static_cast<double>(ug < rg));
-  const long long qh = static_cast<long long>(fh + static_cast<double>(uh < rh));
+  const bool up_g = eng.uniform_below(rg);
+  const bool up_h = eng.uniform_below(rh);
+  const long long qg = static_cast<long long>(fg + static_cast<double>(up_g));
+  const long long qh = static_cast<long long>(fh + static_cast<double>(up_h));
   return make_int2(static_cast<int>(qg), static_cast<int>(qh));
 }
 
@@ -155,6 +173,13 @@ __device__ inline GPairF64 LoadPairStreaming(const GPairF64* p)
 {
   const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
   return GPairF64{v.x, v.y};
+}
+
+// Which child of a split node is built, the other one being derived from the parent: the one with the
+// smaller quantised hessian of output 0, ties to the right (reference: build_tree.h:80-104).
+__device__ inline bool SmallerChildIsLeft(const GPairI64* node_sums, int K, int left_child)
+{
+  return node_sums[static_cast<int64_t>(left_child) * K].hess < node_sums[static_cast<int64_t>(left_child + 1) * K].hess;
 }
 
 }  // namespace lbk

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <functional>
 #include <stdexcept>
@@ -74,6 +75,7 @@ struct lbk_context {
   std::string err;
   // status word in mapped host memory: 0 = ok, otherwise a kernel stored a fault code
   int* d_status = nullptr;
+  int32_t* h_info = nullptr;  // mapped host memory [2], beside it: number of bins, bins of the largest feature
   // communicator
   int rank = 0, n_ranks = 1;
   void* nccl_comm     = nullptr;
@@ -103,12 +105,15 @@ class Scratch {
   {
     return static_cast<T*>(alloc_bytes(sizeof(T) * (n > 0 ? n : 1)));
   }
-  void free_one(void* p);
+  void free_one(void* p);  // (a small buffer stays until the end)
 
  private:
+  void* AllocBlock(size_t bytes);
   lbk_context* ctx_;
   cudaStream_t stream_;
   std::vector<void*> ptrs_;
+  char* slab_       = nullptr;
+  size_t slab_used_ = 0;
 };
 
 // In-place all-reduce over the context's communicator; no-op for a single rank.
@@ -162,44 +167,101 @@ void ThrowReportedFault(lbk_context* ctx);
 int Guard(lbk_context* ctx, const std::function<void()>& f);
 
 // ---- stage launchers (defined in the .cu files named in the comments) ------------------------
+struct TreeArrays {
+  double* leaf_value;
+  int32_t* feature;
+  double* split_value;
+  double* gain;
+  GPairI64* node_sums;
+  int32_t* split_bin;  // feature-relative bin of the chosen split, per node
+  int max_nodes;
+};
 // proposals.cu
 struct ProposalInfo {
   int total_bins;            // B
   int max_bins_per_feature;  // largest feature
 };
+// The first two launches of a tree: split proposals, |g| and |h| sums, cleared arrays (k_prologue), then
+// what follows from all features or all sums (k_prologue_finish).
+constexpr int kZeroRanges = 3;
+template <typename T>
+struct PrologueArgs {
+  const T* X;
+  int64_t ldx, row_offset, n_local;
+  int F, S, S_pad, seed;
+  int64_t dataset_rows;
+  const T* draft;    // set by Prologue: the sampled values where they were summed over ranks first
+  T* cuts;           // out [F][S]: sorted distinct samples, the last one +inf
+  int32_t* counts;   // out [F]; null: no proposals are drawn
+  const double* g;
+  const double* h;
+  int64_t ldg;
+  int K;
+  int64_t n_elements;      // rows x K
+  double *part_g, *part_h; // set by Prologue
+  TreeArrays tree;         // feature, split_value and gain are cleared (max_nodes may be 0)
+  int32_t *root_begin, *root_end;  // the root's segment: all local rows (may be null)
+  void* zero[kZeroRanges];        // 16-byte aligned ranges to zero ...
+  int64_t zero_n16[kZeroRanges];  // ... in units of 16 bytes
+  int64_t sort_blocks, sum_blocks;
+  int fill_blocks;
+};
+// info: device [2] = bins, bins of the largest feature; info_host: the same in mapped host memory (may be
+// null).  sums (may be null: none are made): device [2]; params: the scale from the sums, maximum over ranks.
+template <typename T>
+void Prologue(lbk_context* ctx, Scratch& s, PrologueArgs<T> p, int32_t* row_ptr, int32_t* info, int32_t* info_host,
+              double* sums, QuantParams* params, cudaStream_t stream);
 template <typename T>
 ProposalInfo SplitProposals(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_t row_offset,
                             int64_t n_local, int F, int S, int seed, int64_t dataset_rows, T* proposals,
                             int32_t* row_ptr, cudaStream_t stream);  // synchronises the stream
 template <typename T>
 // bins_t (optional): feature-major copy, bins_t[f * pitch_t + row], pitch_t a multiple of 32 >= n_rows
-void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposals, const int32_t* row_ptr,
+// cut_stride > 0: the proposals of feature f begin at f * cut_stride (0: at row_ptr[f])
+void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposals, int64_t cut_stride, const int32_t* row_ptr,
                void* bins, void* bins_t, int64_t pitch_t, int bin_bytes, int max_bins_per_feature,
                cudaStream_t stream);
-// quantise.cu
-void Quantise(lbk_context* ctx, Scratch& s, const double* g, const double* h, int64_t ldg, int64_t row_offset,
-              int64_t n_local, int K, int seed, int2* gpair, GPairI64* root_sums, QuantParams* params,
-              int* max_abs /* device [2] */, cudaStream_t stream);
+// quantise.cu.  root_sums and max_abs are zero before the call.
+void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, int64_t row_offset, int64_t n_local, int K,
+              int seed, int2* gpair, GPairI64* root_sums, const QuantParams* params, int* max_abs /* device [2] */,
+              cudaStream_t stream);
 // histogram.cu
+struct HistScratch {
+  unsigned int* arrive   = nullptr;  // [n_arrive], zero
+  int n_arrive           = 0;
+  unsigned int* tickets  = nullptr;  // one per launch, zero
+  int next_ticket        = 0;
+  int n_tickets          = 0;
+  void* partial          = nullptr;
+  size_t partial_bytes   = 0;
+};
+// What a tree with these shapes needs of it (n_arrive, partial_bytes).
+void HistScratchNeeds(lbk_context* ctx, int F, int K, int bin_bytes, int max_bins_per_feature, int64_t n_rows, HistScratch& need);
 struct HistLevel {
   const void* bins;
   int bin_bytes;
   int64_t n_rows;      // rows of the bin matrix (local rows)
   int F, K, B;
-  int max_bins_per_feature;
+  int max_bins_per_feature;          // an upper bound ...
+  const int* max_bins_ptr = nullptr; // ... and where the device knows the number itself (may be null)
   const int32_t* row_ptr;
   const int2* gpair;       // int path
   const float2* gpair_f;   // float path
   bool pairs_by_position = false;  // gpair / gpair_f are stored in row_index order: entry i belongs to row_index[i]
   const int* max_abs;      // device [2]: largest |grad|, |hess| of gpair (null: computed by the call)
-  const int32_t* row_index;
-  const int32_t* seg;      // [n_level_nodes+1] offsets for nodes node_begin.. of the level range
+  const int32_t* row_index;  // null: row i is at position i (the root)
+  const int32_t* seg_begin;  // rows of node j of the batch: row_index[seg_begin[j] .. seg_end[j])
+  const int32_t* seg_end;
   int n_nodes;             // nodes in this batch
-  int seg_node_offset;     // index into seg of the batch's first node
-  // built-node selection: slot_of_node[j] = slot in `out` for node j of the batch, or -1
-  const int32_t* slot_of_node;
+  // node_sums null: every node is built, node j into slot j of `out`.  Else the batch is made of pairs of
+  // siblings and only the smaller one is built (SmallerChildIsLeft), into slot j / 2.
+  const GPairI64* node_sums = nullptr;
+  int node_begin            = 0;
   void* out;               // [n_slots, K, B] pairs (int64 or double), already zeroed
   bool float_mode;
+  // scratch that a tree keeps for all its levels (null: the call makes its own): words that are zero
+  // before the call and again after it, a zero ticket of this level, slots for partial sums
+  HistScratch* scratch      = nullptr;
   // set by BuildHistogramSummed only: the histograms go into the owners' receive buffers (see
   // HistParams in histogram.cu)
   void* const* push_recv     = nullptr;
@@ -223,50 +285,47 @@ void* BuildHistogramSummed(lbk_context* ctx, Scratch& s, const HistLevel& lv, in
 void GroupRows(lbk_context* ctx, Scratch& s, const int32_t* node_of_row, int64_t n_rows, int node_begin,
                int n_nodes, int32_t* row_index, int32_t* seg, cudaStream_t stream);
 // split.cu
-struct TreeArrays {
-  double* leaf_value;
-  int32_t* feature;
-  double* split_value;
-  double* gain;
-  GPairI64* node_sums;
-  int32_t* split_bin;  // feature-relative bin of the chosen split, per node
-  int max_nodes;
-};
 struct SplitParams {
   double l1, l2, min_split_gain;
   const uint8_t* feature_set;
 };
-// Decide which nodes of the batch are built: slot_of_node[j] (>=0 built, -1 derived/none).
-void PlanBuilt(const GPairI64* node_sums, int K, int node_begin, int n_nodes, bool parent_available,
-               int32_t* slot_of_node, cudaStream_t stream);
-// Scan built histograms into the level histogram, derive siblings from the parent.
-// Only the features [f_begin, f_end) are scanned / derived (all of them on one rank; the owned ones
-// when the features are divided among the ranks).
-void ScanLevel(const GPairI64* built, const int32_t* slot_of_node, GPairI64* level_hist /* node_begin based */,
-               const GPairI64* parent_hist /* level above, may be null */, int parent_begin,
-               const GPairI64* node_sums, int node_begin, int n_nodes, int K, int f_begin, int f_end, int B,
-               const int32_t* row_ptr, bool parent_available, cudaStream_t stream);
-// arrived: one counter per tree node, zero before the first call of a tree.  The bins of the features
-// [f_begin, f_end) are evaluated; with exchange_records every rank's best candidate of every node
+// One level (or batch of one) after its histograms have been built.
+struct ScanSplitLevel {
+  const GPairI64* built;        // raw sums, [unit][K][bin_stride]; may be level_hist itself when nothing is derived
+  GPairI64* level_hist;         // [n_nodes][K][bin_stride]; only touched if write_hist
+  const GPairI64* parent_hist;  // histograms of the level above, its first node is parent_begin (derive only)
+  int parent_begin;
+  GPairI64* next_built;         // [n_nodes][K][bin_stride]: zeroed for the level below; may be null
+  int64_t bin_stride;
+  int node_begin, n_nodes, K;
+  int f_begin, f_end;           // the features scanned and searched (the owned ones with several ranks)
+  bool derive;                  // pairs of siblings, one of them built
+  bool write_hist;
+};
+// cuts: the split proposals, feature f's from f * cut_stride on.  arrived: one counter per tree node, zero
+// before the first call of a tree.  With exchange_records every rank's best candidate of every node
 // (and the sums left of it) is gathered on all ranks and the best of them becomes the tree - the same
 // total order as within a rank, so the tree is the one a single rank would grow.
 template <typename T>
-void BestSplit(lbk_context* ctx, Scratch& s, const GPairI64* level_hist, int node_begin, int n_nodes, int K, int F, int B,
-               const int32_t* row_ptr, const T* proposals, const QuantParams* qp, const SplitParams& sp,
-               TreeArrays tree, unsigned int* arrived, int f_begin, int f_end, bool exchange_records,
-               cudaStream_t stream);
-void RootLeaf(TreeArrays tree, int K, const QuantParams* qp, double l1, double l2, cudaStream_t stream);
-void WriteHessian(const GPairI64* node_sums, const QuantParams* qp, double* hessian, int64_t n, cudaStream_t stream);
+void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, const int32_t* row_ptr, const T* cuts,
+               int64_t cut_stride, const QuantParams* qp, const SplitParams& sp, const TreeArrays& tree,
+               unsigned int* arrived, bool exchange_records, cudaStream_t stream);
+// hessians and leaf values of all nodes from their sums
+void FinishTree(const TreeArrays& tree, const QuantParams* qp, int K, double l1, double l2, double* hessian,
+                cudaStream_t stream);
 // partition.cu
 struct PartitionLevel {
   const void* bins;   // feature-major copy of the bin ids: bins[f * bin_pitch + row]
   int bin_bytes;
   int64_t bin_pitch;  // elements per feature
   int64_t n_rows;
-  const int32_t* row_index_in;
-  const int32_t* seg_in;  // [n_nodes+1] for the level
+  const int32_t* row_index_in;  // null: row i is at position i (the root)
+  const int32_t* seg_begin;     // [n_nodes]
+  const int32_t* seg_end;
   int32_t* row_index_out;
-  int32_t* seg_out;       // [2*n_nodes+1] for the next level
+  int32_t* seg_begin_out;       // [2 * n_nodes], for the next level
+  int32_t* seg_end_out;
+  unsigned long long* cursor;   // one per tree node, zero before the first call of a tree
   int node_begin, n_nodes;
   const int32_t* feature;
   const int32_t* split_bin;
@@ -276,7 +335,6 @@ struct PartitionLevel {
   int K                = 0;
 };
 void PartitionRows(lbk_context* ctx, Scratch& s, const PartitionLevel& pl, cudaStream_t stream);
-void InitRows(int32_t* row_index, int32_t* seg, int64_t n_rows, cudaStream_t stream);
 // predict.cu
 template <typename T>
 void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees,

@@ -16,6 +16,7 @@
 #include "device_utils.cuh"
 #include <type_traits>
 
+#include "abs_sum.cuh"
 #include "internal.h"
 
 namespace lbk {
@@ -23,143 +24,238 @@ namespace {
 
 constexpr int kSortThreads = 256;
 
+// The value of feature f in the i-th sampled row of the data set; 0 if another rank holds the row.
 template <typename T>
-__global__ void k_gather_samples(const T* __restrict__ X, int64_t ldx, int64_t row_offset, int64_t n_local,
-                                 int F, int S, int seed, int64_t dataset_rows, T* __restrict__ draft)
+__device__ inline T SampledValue(const PrologueArgs<T>& p, int i, int f)
 {
-  // draft is feature-major [F][S]
-  const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (idx >= static_cast<int64_t>(F) * S) return;
-  const int i = static_cast<int>(idx / F);
-  const int f = static_cast<int>(idx % F);
-  MinStd eng(static_cast<uint32_t>(seed));
+  MinStd eng(static_cast<uint32_t>(p.seed));
   eng.discard(static_cast<unsigned long long>(i));
-  const long long row = eng.uniform_int(0, dataset_rows - 1);
-  const bool has      = row >= row_offset && row < row_offset + n_local;
-  draft[static_cast<int64_t>(f) * S + i] = has ? X[(row - row_offset) * ldx + f] : T(0);
+  const long long row = eng.uniform_int(0, p.dataset_rows - 1);
+  const bool has      = row >= p.row_offset && row < p.row_offset + p.n_local;
+  return has ? p.X[(row - p.row_offset) * p.ldx + f] : T(0);
 }
 
-// One block per feature: bitonic sort of the S samples in shared memory, then unique.
+// [F][S] sampled values, for the sum over ranks that comes before the sort
 template <typename T>
-__global__ void __launch_bounds__(kSortThreads)
-  k_sort_unique(const T* __restrict__ draft, int S, int S_pad, T* __restrict__ uniq, int32_t* __restrict__ counts)
+__global__ void k_gather_samples(const __grid_constant__ PrologueArgs<T> p, T* __restrict__ draft)
 {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* vals        = reinterpret_cast<T*>(smem_raw);
-  int* scan_tmp  = reinterpret_cast<int*>(vals + S_pad);
-  const int f    = blockIdx.x;
-  const int tid  = threadIdx.x;
-  for (int i = tid; i < S_pad; i += kSortThreads)
-    vals[i] = i < S ? draft[static_cast<int64_t>(f) * S + i] : static_cast<T>(INFINITY);
-  __syncthreads();
-  for (int k = 2; k <= S_pad; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = tid; i < S_pad; i += kSortThreads) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const T a = vals[i], b = vals[ixj];
-          const bool up = (i & k) == 0;
-          if (up ? (b < a) : (a < b)) {
-            vals[i]   = b;
-            vals[ixj] = a;
+  const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (idx >= static_cast<int64_t>(p.F) * p.S) return;
+  const int i = static_cast<int>(idx / p.F);
+  const int f = static_cast<int>(idx % p.F);
+  draft[static_cast<int64_t>(f) * p.S + i] = SampledValue(p, i, f);
+}
+
+// One block: the S samples of feature f sorted (bitonic), the distinct ones kept in cuts[f * S ..], the
+// last of them replaced by +inf.  Up to 256 samples a thread holds one of them and the 30 of the 36
+// exchange steps that stay inside a warp are shuffles.
+template <typename T>
+__device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals /* shared [S_pad] */, int* s_cnt /* shared [9] */)
+{
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int S = p.S, S_pad = p.S_pad;
+  auto sample = [&](int i) -> T {
+    if (i >= S) return static_cast<T>(INFINITY);
+    return p.draft != nullptr ? p.draft[static_cast<int64_t>(f) * S + i] : SampledValue(p, i, f);
+  };
+  if (S_pad <= kSortThreads) {
+    T v = sample(tid);
+    for (int k = 2; k <= S_pad; k <<= 1) {
+      const bool up = (tid & k) == 0;
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        T o;
+        if (j >= 32) {
+          __syncthreads();
+          if (tid < S_pad) vals[tid] = v;
+          __syncthreads();
+          o = tid < S_pad ? vals[tid ^ j] : v;
+        } else {
+          o = __shfl_xor_sync(0xffffffffu, v, j);
+        }
+        const bool lower = (tid & j) == 0;
+        if (lower == up ? o < v : v < o) v = o;
+      }
+    }
+    __syncthreads();
+    if (tid < S_pad) vals[tid] = v;
+    __syncthreads();
+  } else {
+    for (int i = tid; i < S_pad; i += kSortThreads) vals[i] = sample(i);
+    __syncthreads();
+    for (int k = 2; k <= S_pad; k <<= 1) {
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int i = tid; i < S_pad; i += kSortThreads) {
+          const int ixj = i ^ j;
+          if (ixj > i) {
+            const T a = vals[i], b = vals[ixj];
+            const bool up = (i & k) == 0;
+            if (up ? (b < a) : (a < b)) {
+              vals[i]   = b;
+              vals[ixj] = a;
+            }
           }
         }
+        __syncthreads();
       }
-      __syncthreads();
     }
   }
-  // unique over the first S sorted entries; each thread owns a contiguous run
-  const int per   = (S + kSortThreads - 1) / kSortThreads;
-  const int begin = min(tid * per, S), end = min(begin + per, S);
-  int local = 0;
-  for (int i = begin; i < end; ++i) local += (i == 0 || vals[i] != vals[i - 1]) ? 1 : 0;
-  scan_tmp[tid] = local;
-  __syncthreads();
-  // exclusive scan of 256 counts by a single warp (8 per lane)
-  if (tid < 32) {
-    int v[kSortThreads / 32];
-    int sum = 0;
-#pragma unroll
-    for (int j = 0; j < kSortThreads / 32; ++j) {
-      v[j] = scan_tmp[tid * (kSortThreads / 32) + j];
-      sum += v[j];
-    }
-    int incl = sum;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      int n = __shfl_up_sync(0xffffffffu, incl, off);
-      if (tid >= off) incl += n;
-    }
-    int run = incl - sum;
-#pragma unroll
-    for (int j = 0; j < kSortThreads / 32; ++j) {
-      scan_tmp[tid * (kSortThreads / 32) + j] = run;
-      run += v[j];
-    }
-    if (tid == 31) counts[f] = incl;
+  // unique over the first S sorted entries, 256 at a time
+  T* out     = p.cuts + static_cast<int64_t>(f) * S;
+  int before = 0;
+  for (int base = 0; base < S; base += kSortThreads) {
+    const int i      = base + tid;
+    const bool keep  = i < S && (i == 0 || vals[i] != vals[i - 1]);
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) s_cnt[warp] = __popc(m);
+    __syncthreads();
+    int pos = before;
+    for (int w = 0; w < warp; ++w) pos += s_cnt[w];
+    int total = before;
+    for (int w = 0; w < kSortThreads / 32; ++w) total += s_cnt[w];
+    pos += __popc(m & ((1u << lane) - 1u));
+    if (keep) out[pos] = vals[i];
+    before = total;
+    __syncthreads();
   }
-  __syncthreads();
-  int pos = scan_tmp[tid];
-  for (int i = begin; i < end; ++i) {
-    if (i == 0 || vals[i] != vals[i - 1]) uniq[static_cast<int64_t>(f) * S + pos++] = vals[i];
+  if (tid == 0) {
+    out[before - 1] = static_cast<T>(INFINITY);
+    p.counts[f]     = before;
   }
 }
 
-// row_ptr = exclusive scan of counts (single block)
-__global__ void k_scan_counts(const int32_t* __restrict__ counts, int F, int32_t* __restrict__ row_ptr,
-                              int32_t* __restrict__ max_bins)
+// Everything a tree needs that depends on no other step, one launch with three kinds of blocks: a block
+// per feature draws, sorts and prunes the split proposals; a block per 4096 elements sums |g| and |h|
+// (the canonical order of quantise.cu); the rest clear the tree's arrays and counters.
+template <typename T>
+__global__ void __launch_bounds__(kSortThreads)
+  k_prologue(const __grid_constant__ PrologueArgs<T> p)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_cnt[kSortThreads / 32 + 1];
+  __shared__ double s_sum[2 * kSumThreads / 32];
+  int b = blockIdx.x;
+  if (b < p.sort_blocks) {
+    SortUniqueBlock(p, b, reinterpret_cast<T*>(smem_raw), s_cnt);
+    return;
+  }
+  b -= p.sort_blocks;
+  if (b < p.sum_blocks) {
+    AbsSumBlock<true>(p.g, p.h, p.ldg, p.K, p.n_elements, b, threadIdx.x, s_sum, p.part_g + b, p.part_h + b);
+    return;
+  }
+  b -= p.sum_blocks;
+  const int64_t t = static_cast<int64_t>(b) * kSortThreads + threadIdx.x, n = static_cast<int64_t>(p.fill_blocks) * kSortThreads;
+  for (int z = 0; z < kZeroRanges; ++z)
+    for (int64_t i = t; i < p.zero_n16[z]; i += n) static_cast<uint4*>(p.zero[z])[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (t == 0 && p.root_begin != nullptr) {
+    *p.root_begin = 0;
+    *p.root_end   = static_cast<int32_t>(p.n_local);
+  }
+  for (int64_t i = t; i < p.tree.max_nodes; i += n) {
+    p.tree.feature[i]     = -1;
+    p.tree.split_value[i] = 0.0;
+    p.tree.gain[i]        = 0.0;
+  }
+}
+
+// Single block: row_ptr = exclusive scan of the counts, the number of bins and the largest feature (to the
+// device and, if info_host is given, to mapped host memory), the rest of the |g|, |h| sums and, if
+// `params` is given, the quantiser's scale from them.
+__global__ void __launch_bounds__(1024)
+  k_prologue_finish(const int32_t* __restrict__ counts, int F, int32_t* __restrict__ row_ptr, int32_t* __restrict__ info,
+                    int32_t* info_host, double* part_g, double* part_h, int64_t n_parts, double* sums,
+                    QuantParams* params)
 {
   __shared__ int warp_sums[32];
   __shared__ int carry_s;
   __shared__ int max_s;
+  __shared__ double s_sum[4 * 2 * kSumThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    carry_s = 0;
-    max_s   = 0;
-    row_ptr[0] = 0;
-  }
-  __syncthreads();
-  for (int base = 0; base < F; base += blockDim.x) {
-    const int i = base + tid;
-    const int c = i < F ? counts[i] : 0;
-    int incl    = c;
-    for (int off = 1; off < 32; off <<= 1) {
-      int n = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += n;
+  if (counts != nullptr) {
+    if (tid == 0) {
+      carry_s    = 0;
+      max_s      = 0;
+      row_ptr[0] = 0;
     }
-    if (lane == 31) warp_sums[warp] = incl;
-    atomicMax(&max_s, c);
     __syncthreads();
-    if (warp == 0) {
-      int w = lane < (blockDim.x >> 5) ? warp_sums[lane] : 0;
-      int wi = w;
+    for (int base = 0; base < F; base += blockDim.x) {
+      const int i = base + tid;
+      const int c = i < F ? counts[i] : 0;
+      int incl    = c;
       for (int off = 1; off < 32; off <<= 1) {
-        int n = __shfl_up_sync(0xffffffffu, wi, off);
-        if (lane >= off) wi += n;
+        int n = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += n;
       }
-      warp_sums[lane] = wi - w;  // exclusive
+      if (lane == 31) warp_sums[warp] = incl;
+      const int top = __reduce_max_sync(0xffffffffu, c);
+      if (lane == 0) atomicMax(&max_s, top);
+      __syncthreads();
+      if (warp == 0) {
+        int w  = warp_sums[lane];
+        int wi = w;
+        for (int off = 1; off < 32; off <<= 1) {
+          int n = __shfl_up_sync(0xffffffffu, wi, off);
+          if (lane >= off) wi += n;
+        }
+        warp_sums[lane] = wi - w;  // exclusive
+      }
+      __syncthreads();
+      const int total_before = carry_s + warp_sums[warp];
+      if (i < F) row_ptr[i + 1] = total_before + incl;
+      __syncthreads();
+      if (tid == blockDim.x - 1) carry_s = total_before + incl;
+      __syncthreads();
     }
-    __syncthreads();
-    const int total_before = carry_s + warp_sums[warp];
-    if (i < F) row_ptr[i + 1] = total_before + incl;
-    __syncthreads();
-    if (tid == blockDim.x - 1) carry_s = total_before + incl;
-    __syncthreads();
+    if (tid == 0) {
+      info[0] = carry_s;
+      info[1] = max_s;
+      if (info_host != nullptr) {
+        volatile int32_t* h = info_host;
+        h[0] = carry_s;
+        h[1] = max_s;
+      }
+    }
   }
-  if (tid == 0) *max_bins = max_s;
+  if (sums == nullptr) return;
+  // four groups of 256 threads, each sums 4096 values at a time in the canonical order; a level's results
+  // overwrite its inputs block by block (block b of four per turn writes entry b, all inputs up to then
+  // have been read)
+  int64_t n = n_parts;
+  while (n > 1) {
+    const int64_t blocks = (n + kSumBlock - 1) / kSumBlock;
+    for (int64_t b0 = 0; b0 < blocks; b0 += 4) {
+      const int q     = tid / kSumThreads;
+      const int64_t b = b0 + q;
+      double tg, th;
+      AbsSumPartial<false>(part_g, part_h, 0, 1, n, b, tid % kSumThreads, s_sum + q * 2 * kSumThreads / 32, tg, th);
+      __syncthreads();
+      if (tid % kSumThreads == 0 && b < blocks) {
+        part_g[b] = tg;
+        part_h[b] = th;
+      }
+      __syncthreads();
+    }
+    n = blocks;
+  }
+  if (tid == 0) {
+    sums[0] = n_parts > 0 ? part_g[0] : 0.0;
+    sums[1] = n_parts > 0 ? part_h[0] : 0.0;
+    if (params != nullptr) *params = MakeScale(sums[0], sums[1]);
+  }
+}
+
+__global__ void k_make_scale(const double* __restrict__ sums /* g,h */, QuantParams* __restrict__ qp)
+{
+  *qp = MakeScale(sums[0], sums[1]);
 }
 
 template <typename T>
-__global__ void k_write_proposals(const T* __restrict__ uniq, int S, const int32_t* __restrict__ row_ptr,
+__global__ void k_write_proposals(const T* __restrict__ cuts, int S, const int32_t* __restrict__ row_ptr,
                                   T* __restrict__ proposals)
 {
   const int f     = blockIdx.x;
   const int begin = row_ptr[f], end = row_ptr[f + 1];
-  for (int j = threadIdx.x; j < end - begin; j += blockDim.x) {
-    T v = uniq[static_cast<int64_t>(f) * S + j];
-    if (j == end - begin - 1) v = static_cast<T>(INFINITY);
-    proposals[begin + j] = v;
-  }
+  for (int j = threadIdx.x; j < end - begin; j += blockDim.x) proposals[begin + j] = cuts[static_cast<int64_t>(f) * S + j];
 }
 
 // Streaming global loads as volatile asm: they stay where they are written, ahead of the search
@@ -233,7 +329,7 @@ constexpr int kBinTilePitch = kBinTileRows + 8;  // bytes; 18 words: 8-byte stor
 template <typename T, typename BinT, int kLog2P, bool kCopyT>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
   k_bin_smem(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const T* __restrict__ proposals,
-             const int32_t* __restrict__ row_ptr, BinT* __restrict__ bins, BinT* __restrict__ bins_t, int64_t pitch_t)
+             int64_t cut_stride, const int32_t* __restrict__ row_ptr, BinT* __restrict__ bins, BinT* __restrict__ bins_t, int64_t pitch_t)
 {
   constexpr int P = 1 << kLog2P;
   constexpr bool kTile = kCopyT && sizeof(BinT) == 1;
@@ -247,7 +343,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
     T v = static_cast<T>(INFINITY);
     if (f < F) {
       const int b = row_ptr[f];
-      if (j < row_ptr[f + 1] - b) v = proposals[b + j];
+      if (j < row_ptr[f + 1] - b) v = proposals[(cut_stride > 0 ? f * cut_stride : b) + j];
     }
     sp[idx] = v;
   }
@@ -369,7 +465,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
 template <typename T, typename BinT>
 __global__ void __launch_bounds__(256)
   k_bin_global(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const T* __restrict__ proposals,
-               const int32_t* __restrict__ row_ptr, BinT* __restrict__ bins, BinT* __restrict__ bins_t, int64_t pitch_t)
+               int64_t cut_stride, const int32_t* __restrict__ row_ptr, BinT* __restrict__ bins, BinT* __restrict__ bins_t, int64_t pitch_t)
 {
   const int g    = blockIdx.y;
   const int f0   = g * kGroup;
@@ -381,7 +477,7 @@ __global__ void __launch_bounds__(256)
     begin = row_ptr[f];
     n     = row_ptr[f + 1] - begin;
   }
-  const T* p = proposals + begin;
+  const T* p = proposals + (cut_stride > 0 && active ? f * cut_stride : begin);
   const int64_t pitch = static_cast<int64_t>(gridDim.y) * kGroup;
   BinT* out  = bins + f0;
   const int64_t warps_total = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
@@ -413,41 +509,71 @@ int NextPow2(int v)
 }  // namespace
 
 template <typename T>
+void Prologue(lbk_context* ctx, Scratch& s, PrologueArgs<T> p, int32_t* row_ptr, int32_t* info, int32_t* info_host,
+              double* sums, QuantParams* params, cudaStream_t stream)
+{
+  p.S_pad       = NextPow2(p.S);
+  p.sort_blocks = p.F;
+  if (p.counts == nullptr) p.sort_blocks = 0;
+  p.sum_blocks = sums != nullptr ? (p.n_elements + kSumBlock - 1) / kSumBlock : 0;
+  p.part_g     = s.alloc<double>(static_cast<size_t>(p.sum_blocks) + 1);
+  p.part_h     = s.alloc<double>(static_cast<size_t>(p.sum_blocks) + 1);
+  if (ctx->n_ranks > 1 && p.sort_blocks > 0) {
+    // every rank fills in the sampled rows it holds; the sum over the ranks makes them complete
+    const int64_t FS = static_cast<int64_t>(p.F) * p.S;
+    T* draft         = s.alloc<T>(FS);
+    k_gather_samples<T><<<static_cast<unsigned>((FS + 255) / 256), 256, 0, stream>>>(p, draft);
+    LBK_LAUNCH_CHECK();
+    AllReduce(ctx, draft, static_cast<size_t>(FS), sizeof(T) == 4 ? LBK_F32 : LBK_F64, LBK_SUM, stream);
+    p.draft = draft;
+  }
+  int64_t fill = p.tree.max_nodes;
+  for (int z = 0; z < kZeroRanges; ++z) fill += p.zero_n16[z];
+  p.fill_blocks = static_cast<int>(std::min<int64_t>((fill + 4 * kSortThreads - 1) / (4 * kSortThreads), ctx->sm_count * 4));
+  const int64_t blocks = p.sort_blocks + p.sum_blocks + p.fill_blocks;
+  if (blocks > 0) {
+    k_prologue<T><<<static_cast<unsigned>(blocks), kSortThreads, sizeof(T) * p.S_pad, stream>>>(p);
+    LBK_LAUNCH_CHECK();
+  }
+  const bool one_rank = ctx->n_ranks <= 1;
+  k_prologue_finish<<<1, 1024, 0, stream>>>(p.counts, p.F, row_ptr, info, info_host, p.part_g, p.part_h, p.sum_blocks, sums,
+                                            one_rank ? params : nullptr);
+  LBK_LAUNCH_CHECK();
+  if (!one_rank && sums != nullptr) {
+    AllReduce(ctx, sums, 2, LBK_F64, LBK_MAX, stream);
+    k_make_scale<<<1, 1, 0, stream>>>(sums, params);
+    LBK_LAUNCH_CHECK();
+  }
+}
+
+template <typename T>
 ProposalInfo SplitProposals(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_t row_offset, int64_t n_local,
                    int F, int S, int seed, int64_t dataset_rows, T* proposals, int32_t* row_ptr,
                    cudaStream_t stream)
 {
-  const int64_t FS = static_cast<int64_t>(F) * S;
-  T* draft         = s.alloc<T>(FS);
-  T* uniq          = s.alloc<T>(FS);
-  int32_t* counts  = s.alloc<int32_t>(F + 1);
-  {
-    const int threads = 256;
-    const int64_t blocks = (FS + threads - 1) / threads;
-    k_gather_samples<T><<<static_cast<unsigned>(blocks), threads, 0, stream>>>(X, ldx, row_offset, n_local, F, S, seed,
-                                                                               dataset_rows, draft);
-    LBK_LAUNCH_CHECK();
-  }
-  AllReduce(ctx, draft, static_cast<size_t>(FS), sizeof(T) == 4 ? LBK_F32 : LBK_F64, LBK_SUM, stream);
-  const int S_pad   = NextPow2(S);
-  const size_t smem = sizeof(T) * S_pad + sizeof(int) * kSortThreads;
-  k_sort_unique<T><<<F, kSortThreads, smem, stream>>>(draft, S, S_pad, uniq, counts);
-  LBK_LAUNCH_CHECK();
-  k_scan_counts<<<1, 1024, 0, stream>>>(counts, F, row_ptr, counts + F);
-  LBK_LAUNCH_CHECK();
-  k_write_proposals<T><<<F, 128, 0, stream>>>(uniq, S, row_ptr, proposals);
+  PrologueArgs<T> p{};
+  p.X            = X;
+  p.ldx          = ldx;
+  p.row_offset   = row_offset;
+  p.n_local      = n_local;
+  p.F            = F;
+  p.S            = S;
+  p.seed         = seed;
+  p.dataset_rows = dataset_rows;
+  p.cuts         = s.alloc<T>(static_cast<size_t>(F) * S);
+  p.counts       = s.alloc<int32_t>(F);
+  int32_t* info  = s.alloc<int32_t>(2);
+  Prologue<T>(ctx, s, p, row_ptr, info, nullptr, nullptr, nullptr, stream);
+  k_write_proposals<T><<<F, 128, 0, stream>>>(p.cuts, S, row_ptr, proposals);
   LBK_LAUNCH_CHECK();
   int32_t h[2] = {0, 0};
-  LBK_CUDA(cudaMemcpyAsync(&h[0], row_ptr + F, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-  LBK_CUDA(cudaMemcpyAsync(&h[1], counts + F, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+  LBK_CUDA(cudaMemcpyAsync(h, info, sizeof(h), cudaMemcpyDeviceToHost, stream));
   LBK_CUDA(cudaStreamSynchronize(stream));
-  s.free_one(draft);
-  s.free_one(uniq);
   return ProposalInfo{h[0], h[1]};
 }
 
 template <typename T>
-void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposals, const int32_t* row_ptr,
+void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposals, int64_t cut_stride, const int32_t* row_ptr,
                void* bins, void* bins_t, int64_t pitch_t, int bin_bytes, int max_bins_per_feature, cudaStream_t stream)
 {
   if (n_rows <= 0) return;
@@ -479,7 +605,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       LBK_CUDA(cudaFuncSetAttribute(fn_, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))); \
     int per_sm_ = 0;                                                                                      \
     LBK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_, fn_, 256, smem));                    \
-    fn_<<<make_grid(per_sm_), 256, smem, stream>>>(X, ldx, n_rows, F, proposals, row_ptr,                 \
+    fn_<<<make_grid(per_sm_), 256, smem, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr,                 \
                                                    static_cast<BinT*>(bins), static_cast<BinT*>(bins_t), pitch_t); \
   } while (0)
 #define LBK_BIN_SMEM(BinT, L)                                                                             \
@@ -494,7 +620,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       else if (log2p == 8) LBK_BIN_SMEM(BinT, 8);                                                         \
       else LBK_BIN_SMEM(BinT, 9);                                                                         \
     } else {                                                                                              \
-      k_bin_global<T, BinT><<<make_grid(8), 256, 0, stream>>>(X, ldx, n_rows, F, proposals, row_ptr,     \
+      k_bin_global<T, BinT><<<make_grid(8), 256, 0, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr,     \
                                                        static_cast<BinT*>(bins), static_cast<BinT*>(bins_t), \
                                                        pitch_t);                                          \
     }                                                                                                     \
@@ -514,9 +640,13 @@ template ProposalInfo SplitProposals<float>(lbk_context*, Scratch&, const float*
                                    int64_t, float*, int32_t*, cudaStream_t);
 template ProposalInfo SplitProposals<double>(lbk_context*, Scratch&, const double*, int64_t, int64_t, int64_t, int, int, int,
                                     int64_t, double*, int32_t*, cudaStream_t);
-template void BinMatrix<float>(const float*, int64_t, int64_t, int, const float*, const int32_t*, void*, void*, int64_t,
+template void Prologue<float>(lbk_context*, Scratch&, PrologueArgs<float>, int32_t*, int32_t*, int32_t*, double*, QuantParams*,
+                              cudaStream_t);
+template void Prologue<double>(lbk_context*, Scratch&, PrologueArgs<double>, int32_t*, int32_t*, int32_t*, double*,
+                               QuantParams*, cudaStream_t);
+template void BinMatrix<float>(const float*, int64_t, int64_t, int, const float*, int64_t, const int32_t*, void*, void*, int64_t,
                                int, int, cudaStream_t);
-template void BinMatrix<double>(const double*, int64_t, int64_t, int, const double*, const int32_t*, void*, void*,
+template void BinMatrix<double>(const double*, int64_t, int64_t, int, const double*, int64_t, const int32_t*, void*, void*,
                                 int64_t, int, int, cudaStream_t);
 
 }  // namespace lbk

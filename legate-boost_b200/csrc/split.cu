@@ -1,9 +1,9 @@
-// Node selection, prefix scan with sibling subtraction, and split evaluation.
+// Prefix scan with sibling subtraction and split evaluation of a level, in one pass over its histograms.
 //
 // Reference behaviour restated here (src/models/tree/):
 //   SelectHistogramNode / ComputeHistogramBin  build_tree.h:80-104 - only the child with the
 //     smaller quantised hessian of output 0 is built (ties: the right child) when the parent's
-//     histogram is available;
+//     histogram is available (SmallerChildIsLeft, device_utils.cuh);
 //   scan_kernel        build_tree.cu:597-668 - inclusive prefix over the bins of each feature; the
 //     prefix replaces the bin value only if prefix.grad > 0 or prefix.hess > 0; then
 //     sibling = parent - node;
@@ -20,96 +20,10 @@
 namespace lbk {
 namespace {
 
-__global__ void k_plan_built(const GPairI64* __restrict__ node_sums, int K, int node_begin, int n_nodes,
-                             bool parent_available, int32_t* __restrict__ slot_of_node)
-{
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n_nodes) return;
-  const int node = node_begin + j;
-  int slot;
-  if (node == 0) {
-    slot = 0;
-  } else if (!parent_available) {
-    slot = j;
-  } else {
-    const int parent = (node - 1) / 2;
-    const int l = 2 * parent + 1, r = 2 * parent + 2;
-    const int hist_node =
-      (node_sums[static_cast<int64_t>(l) * K].hess < node_sums[static_cast<int64_t>(r) * K].hess) ? l : r;
-    slot = hist_node == node ? j / 2 : -1;
-  }
-  slot_of_node[j] = slot;
-}
-
-// One warp per (node, feature); blockIdx.y = output.
-__global__ void __launch_bounds__(256)
-  k_scan(const GPairI64* __restrict__ built, const int32_t* __restrict__ slot_of_node,
-         GPairI64* __restrict__ level_hist, const GPairI64* __restrict__ parent_hist, int parent_begin,
-         const GPairI64* __restrict__ node_sums, int node_begin, int n_nodes, int K, int f_begin, int n_features,
-         int B, const int32_t* __restrict__ row_ptr, bool parent_available)
-{
-  const int lane    = threadIdx.x & 31;
-  const int64_t wid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  if (wid >= static_cast<int64_t>(n_nodes) * n_features) return;
-  const int j    = static_cast<int>(wid / n_features);
-  const int f    = f_begin + static_cast<int>(wid % n_features);
-  const int k    = blockIdx.y;
-  const int node = node_begin + j;
-  const int slot = slot_of_node[j];
-  if (slot < 0) return;
-  const GPairI64* src = built + (static_cast<int64_t>(slot) * K + k) * B;
-  GPairI64* dst       = level_hist + (static_cast<int64_t>(j) * K + k) * B;
-  const int fb = row_ptr[f], fe = row_ptr[f + 1];
-  if (node_sums[static_cast<int64_t>(node) * K + k].hess <= 0) {
-    // not scanned: the raw values stay, no sibling is derived
-    if (src != dst)
-      for (int b = fb + lane; b < fe; b += 32) StorePair(dst + b, LoadPair(src + b));
-    return;
-  }
-  const bool derive = node != 0 && parent_available;
-  GPairI64* sib     = nullptr;
-  const GPairI64* par = nullptr;
-  if (derive) {
-    const int js = j ^ 1;  // a level starts at an odd heap index: j even = left child
-    sib          = level_hist + (static_cast<int64_t>(js) * K + k) * B;
-    par          = parent_hist + (static_cast<int64_t>((node - 1) / 2 - parent_begin) * K + k) * B;
-  }
-  long long agg_g = 0, agg_h = 0;
-  for (int base = fb; base < fe; base += 32) {
-    const int b     = base + lane;
-    const bool part = b < fe;
-    GPairI64 raw{0, 0};
-    if (part) raw = LoadPair(src + b);
-    long long sg = raw.grad, sh = raw.hess;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const long long ng = __shfl_up_sync(0xffffffffu, sg, off);
-      const long long nh = __shfl_up_sync(0xffffffffu, sh, off);
-      if (lane >= off) {
-        sg += ng;
-        sh += nh;
-      }
-    }
-    const long long tile_g = __shfl_sync(0xffffffffu, sg, 31);
-    const long long tile_h = __shfl_sync(0xffffffffu, sh, 31);
-    sg += agg_g;
-    sh += agg_h;
-    if (part) {
-      const GPairI64 v = (sg > 0 || sh > 0) ? GPairI64{sg, sh} : raw;
-      StorePair(dst + b, v);
-      if (derive) {
-        const GPairI64 pv = LoadPair(par + b);
-        StorePair(sib + b, GPairI64{pv.grad - v.grad, pv.hess - v.hess});
-      }
-    }
-    agg_g += tile_g;
-    agg_h += tile_h;
-  }
-}
-
 struct Cand {
   double gain;
   int bin;
+  int feature;
 };
 __device__ inline bool Better(const Cand& a, const Cand& b)
 {
@@ -121,49 +35,7 @@ __device__ inline bool Better(const Cand& a, const Cand& b)
   return a.bin < b.bin;
 }
 
-constexpr int kSplitThreads = 256;
-
-// Candidate of one slice of a node's bins, as it travels through global memory.
-struct SliceBest {
-  double gain;
-  int bin;
-  int pad;
-};
-
-// The winner of a node becomes the tree: feature, split value, gain, and the sums and leaf values
-// of the two children.  left_sums[k * left_stride] = the sums left of the winning bin, output k.
-template <typename T>
-__device__ inline void ApplyWinner(const Cand& nb, int node, int K, int F, const int32_t* __restrict__ row_ptr,
-                                   const T* __restrict__ proposals, const QuantParams& qp, double l1, double l2,
-                                   TreeArrays tree, const GPairI64* __restrict__ left_sums, int64_t left_stride, int tid,
-                                   int n_threads)
-{
-  if (!(nb.gain > 1e-5)) return;
-  GPairI64* node_sums = tree.node_sums;
-  int lo = 0, hi = F;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (row_ptr[mid] <= nb.bin) lo = mid; else hi = mid;
-  }
-  const int bf = lo;
-  const int l = 2 * node + 1, r = 2 * node + 2;
-  for (int k = tid; k < K; k += n_threads) {
-    const GPairI64 ns = LoadPair(node_sums + static_cast<int64_t>(node) * K + k);
-    const GPairI64 ls = LoadPair(left_sums + static_cast<int64_t>(k) * left_stride);
-    const GPairI64 rs{ns.grad - ls.grad, ns.hess - ls.hess};
-    StorePair(node_sums + static_cast<int64_t>(l) * K + k, ls);
-    StorePair(node_sums + static_cast<int64_t>(r) * K + k, rs);
-    const GPairF64 dl = Dequantise(ls, qp), dr = Dequantise(rs, qp);
-    tree.leaf_value[static_cast<int64_t>(l) * K + k] = CalculateLeafValue(dl.grad, dl.hess, l1, l2);
-    tree.leaf_value[static_cast<int64_t>(r) * K + k] = CalculateLeafValue(dr.grad, dr.hess, l1, l2);
-    if (k == 0) {
-      tree.feature[node]     = bf;
-      tree.split_value[node] = static_cast<double>(proposals[nb.bin]);
-      tree.gain[node]        = nb.gain;
-      tree.split_bin[node]   = nb.bin - row_ptr[bf];
-    }
-  }
-}
+constexpr int kSplitWarps = 8;  // most warps of a block
 
 // What a rank knows about its best split of a node when the features are divided among the ranks:
 // the candidate and the sums left of it; K pairs follow the header.
@@ -174,119 +46,359 @@ struct SplitRecordHeader {
 };
 __host__ __device__ inline size_t SplitRecordBytes(int K) { return sizeof(SplitRecordHeader) + sizeof(GPairI64) * K; }
 
-// grid = (nodes, slices): a block evaluates one slice of the node's bins (all of them when there is
-// one slice).  With several slices every block leaves its best candidate in `slice_best`, and the
-// block that arrives last (a counter per node, zeroed once per tree) picks the winner and writes
-// the tree.  Better() is a total order, so the winner does not depend on how the bins were cut.
-template <typename T>
-__global__ void __launch_bounds__(kSplitThreads)
-  k_best_split(const GPairI64* __restrict__ level_hist, int node_begin, int K, int F, int B,
-               const int32_t* __restrict__ row_ptr, const T* __restrict__ proposals,
-               const QuantParams* __restrict__ qp_ptr, double l1, double l2, double msg,
-               const uint8_t* __restrict__ feature_set, TreeArrays tree, SliceBest* __restrict__ slice_best,
-               unsigned int* __restrict__ arrived, int f_begin, int f_end, unsigned char* __restrict__ records)
+// The winner of a node becomes the tree: feature, split value, gain and the sums of the two children.
+// left_of(k) = the sums left of the winning bin, output k (called by one thread per k).
+template <typename T, typename LeftOf>
+__device__ inline void ApplyWinner(const Cand& nb, int node, int K, const int32_t* __restrict__ row_ptr,
+                                   const T* __restrict__ cuts, int64_t cut_stride, const TreeArrays& tree, LeftOf left_of,
+                                   int tid, int n_threads)
 {
-  const int j      = blockIdx.x;
-  const int slices = gridDim.y;
-  const int node   = node_begin + j;
+  if (!(nb.gain > 1e-5)) return;
   GPairI64* node_sums = tree.node_sums;
-  if (LoadPair(node_sums + static_cast<int64_t>(node) * K).hess <= 0) return;
-  const QuantParams qp = *qp_ptr;
-  const GPairI64* hist = level_hist + static_cast<int64_t>(j) * K * B;
-  __shared__ Cand s_c[kSplitThreads / 32];
-  __shared__ Cand s_best;
-  __shared__ bool s_last;
-  const int tid = threadIdx.x;
-  // the bins this rank evaluates (all of them unless the features are divided among the ranks)
-  const int bin_begin = row_ptr[f_begin], bin_end = row_ptr[f_end];
-  const int per = (bin_end - bin_begin + slices - 1) / slices;
-  const int b0  = bin_begin + blockIdx.y * per, b1 = min(bin_end, b0 + per);
-  Cand best{0.0, -1};
-  for (int b = b0 + tid; b < b1; b += kSplitThreads) {
-    if (feature_set) {
-      int lo = 0, hi = F;  // last f with row_ptr[f] <= b
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (row_ptr[mid] <= b) lo = mid; else hi = mid;
-      }
-      if (!feature_set[lo]) continue;
+  const int l = 2 * node + 1, r = 2 * node + 2;
+  for (int k = tid; k < K; k += n_threads) {
+    const GPairI64 ns = LoadPair(node_sums + static_cast<int64_t>(node) * K + k);
+    const GPairI64 ls = left_of(k);
+    StorePair(node_sums + static_cast<int64_t>(l) * K + k, ls);
+    StorePair(node_sums + static_cast<int64_t>(r) * K + k, GPairI64{ns.grad - ls.grad, ns.hess - ls.hess});
+    if (k == 0) {
+      const int b            = nb.bin - row_ptr[nb.feature];
+      tree.feature[node]     = nb.feature;
+      tree.split_value[node] = static_cast<double>(cuts[nb.feature * cut_stride + b]);
+      tree.gain[node]        = nb.gain;
+      tree.split_bin[node]   = b;
     }
-    double gain = 0;
-    for (int k = 0; k < K; ++k) {
-      const GPairI64 ns = LoadPair(node_sums + static_cast<int64_t>(node) * K + k);
-      const GPairI64 ls = LoadPair(hist + static_cast<int64_t>(k) * B + b);
-      const GPairI64 rs{ns.grad - ls.grad, ns.hess - ls.hess};
-      if (ls.hess <= 0 || rs.hess <= 0) {
-        gain = 0;
-        break;
-      }
-      gain += CalculateGain(Dequantise(ls, qp), Dequantise(rs, qp), Dequantise(ns, qp), l1, l2, msg);
-    }
-    const Cand c{gain, b};
-    if (gain > 0 && Better(c, best)) best = c;
   }
-  auto warp_best = [&]() {
+}
+
+template <typename T>
+struct ScanSplitParams {
+  ScanSplitLevel lv;
+  const int32_t* row_ptr;
+  const T* cuts;
+  int64_t cut_stride;
+  const QuantParams* qp;
+  SplitParams sp;
+  TreeArrays tree;
+  struct SliceBest* slice_best;  // [units][slices][2]
+  unsigned int* arrived;
+  unsigned char* records;
+};
+
+// The best candidate of one slice of a unit; with one output also the sums left of it.
+struct SliceBest {
+  Cand c;
+  GPairI64 left;
+};
+
+// What the gains of one output need of a node: its sums as whole numbers in float64 and its own gain.
+struct NodeTerms {
+  double g, h, gain;
+};
+
+// (double)v for |v| < 2^51, exact: adding 1.5 * 2^52 to the bit pattern of the integer makes a float64 whose
+// value is that constant plus v.  Two instructions of full rate instead of a conversion of a sixteenth of it.
+__device__ inline double WholeToDouble(long long v)
+{
+  return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
+}
+
+__device__ inline NodeTerms TermsOf(GPairI64 sum, const QuantParams& qp, double l1, double reg)
+{
+  NodeTerms t;
+  t.g    = WholeToDouble(sum.grad);
+  t.h    = WholeToDouble(sum.hess);
+  t.gain = LeafGain(GPairF64{t.g * qp.inv_g, t.h * qp.inv_h}, l1, reg);
+  return t;
+}
+
+// The gain of one output at one bin, added to `gain`; false if a side has no positive hessian (sums are
+// below 2^51, so their differences are exact in float64).
+__device__ inline bool AddGain(GPairI64 left, const NodeTerms& n, const QuantParams& qp, double l1, double reg, double msg,
+                               double& gain)
+{
+  const double lg = WholeToDouble(left.grad), lh = WholeToDouble(left.hess);
+  const double rg = n.g - lg, rh = n.h - lh;
+  if (lh <= 0.0 || rh <= 0.0) return false;
+  const double gl = LeafGain(GPairF64{lg * qp.inv_g, lh * qp.inv_h}, l1, reg);
+  const double gr = LeafGain(GPairF64{rg * qp.inv_g, rh * qp.inv_h}, l1, reg);
+  gain += (0.5 * (gl + gr - n.gain)) - msg;
+  return true;
+}
+
+// grid = (units, slices).  A unit is a pair of siblings of which one was built (derive) or a single
+// built node; a warp takes one feature at a time: it scans the built histogram, derives the sibling's
+// from the parent's, writes both for the level below (not on the last level: nobody reads them there)
+// and evaluates both nodes' gains while the sums are in registers, so that a level's histograms cross
+// the memory once.  The buffer of the nodes built on the next level is zeroed on the way.  With several
+// slices every block leaves its best candidates in `slice_best`, and the block of the unit that arrives
+// last (a counter per node, zeroed once per tree) picks the winners and writes the tree.  Better() is a
+// total order, so the winners do not depend on how the features were cut.
+//
+// What bounds it: on wide levels the issue slots (two float64 divisions per bin, output and node, and a
+// 64-bit scan), on the upper levels the latency of one chain load - scan - division - reduction - claim.
+// kRun bins per lane and turn: four with one output (few warps, long chains), two with several, where
+// the registers that this saves keep three blocks on an SM.
+template <typename T, bool kManyOutputs, bool kDerive, int kRun>
+__global__ void __launch_bounds__(kSplitWarps * 32, kManyOutputs ? 3 : 2)
+  k_scan_split(const __grid_constant__ ScanSplitParams<T> p)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];  // several outputs: terms [2][K], then [warps][K] carries
+  __shared__ SliceBest s_c[2][kSplitWarps];
+  __shared__ SliceBest s_best[2];
+  __shared__ bool s_last;
+  const ScanSplitLevel& lv = p.lv;
+  const int K = lv.K, unit = blockIdx.x, slices = gridDim.y;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
+  const int node0 = lv.node_begin + (kDerive ? 2 * unit : unit);
+  GPairI64* node_sums = p.tree.node_sums;
+  // everything the block needs first, asked for at once
+  const int parent_feature = node0 > 0 ? p.tree.feature[(node0 - 1) / 2] : 0;
+  const GPairI64 sum_0 = LoadPair(node_sums + static_cast<int64_t>(node0) * K);
+  const GPairI64 sum_1 = kDerive ? LoadPair(node_sums + static_cast<int64_t>(node0 + 1) * K) : GPairI64{0, 0};
+  const QuantParams qp = *p.qp;
+  int f  = lv.f_begin + blockIdx.y * n_warps + warp;
+  int fb = f < lv.f_end ? p.row_ptr[f] : 0, fe = f < lv.f_end ? p.row_ptr[f + 1] : 0;
+  if (parent_feature < 0) return;  // the parent did not split: no such node
+  // _a: the built node, _b: its sibling (SmallerChildIsLeft)
+  const bool left_built = !kDerive || sum_0.hess < sum_1.hess;
+  const int node_a = left_built ? node0 : node0 + 1, node_b = left_built ? node0 + 1 : node0;
+  const int ja = node_a - lv.node_begin, jb = node_b - lv.node_begin;
+  const GPairI64 sum_a = left_built ? sum_0 : sum_1, sum_b = left_built ? sum_1 : sum_0;
+  const bool eval_a = sum_a.hess > 0, eval_b = kDerive && sum_b.hess > 0;
+  const double l1 = p.sp.l1, reg = fmax(1e-5, p.sp.l2), msg = p.sp.min_split_gain;
+  const int64_t Bs    = lv.bin_stride;
+  const GPairI64* src = lv.built + static_cast<int64_t>(unit) * K * Bs;
+  GPairI64* dst_a     = lv.level_hist + static_cast<int64_t>(ja) * K * Bs;
+  GPairI64* dst_b     = lv.level_hist + static_cast<int64_t>(jb) * K * Bs;
+  GPairI64* next_a    = lv.next_built + static_cast<int64_t>(ja) * K * Bs;
+  GPairI64* next_b    = lv.next_built + static_cast<int64_t>(jb) * K * Bs;
+  const GPairI64* par = lv.parent_hist + static_cast<int64_t>((node0 - 1) / 2 - lv.parent_begin) * K * Bs;
+  NodeTerms* s_terms  = reinterpret_cast<NodeTerms*>(smem_raw);
+  GPairI64* s_carry   = reinterpret_cast<GPairI64*>(smem_raw + sizeof(NodeTerms) * 2 * ((K + 1) / 2 * 2)) + warp * K;
+  NodeTerms ta{}, tb{};
+  if (kManyOutputs) {
+    for (int i = tid; i < 2 * K; i += blockDim.x) {
+      const int k = i >> 1, node = (i & 1) ? node_b : node_a;
+      if (kDerive || !(i & 1)) s_terms[i] = TermsOf(LoadPair(node_sums + static_cast<int64_t>(node) * K + k), qp, l1, reg);
+    }
+    __syncthreads();
+  } else {
+    ta = TermsOf(sum_a, qp, l1, reg);
+    if (kDerive) tb = TermsOf(sum_b, qp, l1, reg);
+  }
+
+  Cand best_a{0.0, -1, -1}, best_b{0.0, -1, -1};
+  GPairI64 left_a{0, 0}, left_b{0, 0};
+  while (f < lv.f_end) {
+    const bool search = p.sp.feature_set == nullptr || p.sp.feature_set[f] != 0;
+    GPairI64 carry{0, 0};
+    if (kManyOutputs) {
+      __syncwarp();
+      for (int k = lane; k < K; k += 32) s_carry[k] = GPairI64{0, 0};
+      __syncwarp();
+    }
+    for (int base = fb; base < fe; base += 32 * kRun) {
+      double gain_a[kRun], gain_b[kRun];
+      GPairI64 va[kRun], vb[kRun];
+      unsigned in = 0;
+#pragma unroll
+      for (int i = 0; i < kRun; ++i) {
+        gain_a[i] = gain_b[i] = 0.0;
+        if (base + i * 32 + lane < fe) in |= 1u << i;
+      }
+      unsigned ok_a = eval_a && search ? in : 0u, ok_b = eval_b && search ? in : 0u;
+      for (int k = 0; k < (kManyOutputs ? K : 1); ++k) {
+        const int64_t ko = (kManyOutputs ? static_cast<int64_t>(k) * Bs : 0) + base + lane;
+        if (kManyOutputs) {
+          ta = s_terms[2 * k];
+          if (kDerive) tb = s_terms[2 * k + 1];
+        }
+        const bool scanned = ta.h > 0.0;  // else the raw values stay and no sibling is derived
+        long long sg[kRun], sh[kRun];
+#pragma unroll
+        for (int i = 0; i < kRun; ++i) {
+          va[i] = in & (1u << i) ? LoadPair(src + ko + i * 32) : GPairI64{0, 0};
+          if (kDerive) vb[i] = (in & (1u << i)) && scanned ? LoadPair(par + ko + i * 32) : GPairI64{0, 0};
+          sg[i] = va[i].grad;
+          sh[i] = va[i].hess;
+        }
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+          for (int i = 0; i < kRun; ++i) {
+            const long long ng = __shfl_up_sync(0xffffffffu, sg[i], off);
+            const long long nh = __shfl_up_sync(0xffffffffu, sh[i], off);
+            if (lane >= off) {
+              sg[i] += ng;
+              sh[i] += nh;
+            }
+          }
+        }
+        GPairI64 run = kManyOutputs ? s_carry[k] : carry;
+#pragma unroll
+        for (int i = 0; i < kRun; ++i) {
+          const long long tg = __shfl_sync(0xffffffffu, sg[i], 31), th = __shfl_sync(0xffffffffu, sh[i], 31);
+          sg[i] += run.grad;
+          sh[i] += run.hess;
+          run.grad += tg;
+          run.hess += th;
+        }
+        if (kManyOutputs) {
+          __syncwarp();
+          if (lane == 0) s_carry[k] = run;
+        } else {
+          carry = run;
+        }
+#pragma unroll
+        for (int i = 0; i < kRun; ++i) {
+          if (!(in & (1u << i))) continue;
+          if (scanned && (sg[i] > 0 || sh[i] > 0)) va[i] = GPairI64{sg[i], sh[i]};
+          if (kDerive) vb[i] = scanned ? GPairI64{vb[i].grad - va[i].grad, vb[i].hess - va[i].hess} : GPairI64{0, 0};
+          if (lv.write_hist) {
+            StorePair(dst_a + ko + i * 32, va[i]);
+            if (kDerive) StorePair(dst_b + ko + i * 32, vb[i]);
+          }
+          if (lv.next_built != nullptr) {
+            StorePair(next_a + ko + i * 32, GPairI64{0, 0});
+            if (kDerive) StorePair(next_b + ko + i * 32, GPairI64{0, 0});
+          }
+          if (ok_a & (1u << i))
+            if (!AddGain(va[i], ta, qp, l1, reg, msg, gain_a[i])) ok_a &= ~(1u << i);
+          if (kDerive && (ok_b & (1u << i)))
+            if (!AddGain(vb[i], tb, qp, l1, reg, msg, gain_b[i])) ok_b &= ~(1u << i);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kRun; ++i) {
+        const int b = base + i * 32 + lane;
+        if ((ok_a & (1u << i)) && gain_a[i] > 0) {
+          const Cand c{gain_a[i], b, f};
+          if (Better(c, best_a)) {
+            best_a = c;
+            if (!kManyOutputs) left_a = va[i];
+          }
+        }
+        if (kDerive && (ok_b & (1u << i)) && gain_b[i] > 0) {
+          const Cand c{gain_b[i], b, f};
+          if (Better(c, best_b)) {
+            best_b = c;
+            if (!kManyOutputs) left_b = vb[i];
+          }
+        }
+      }
+    }
+    f += slices * n_warps;
+    if (f < lv.f_end) {
+      fb = p.row_ptr[f];
+      fe = p.row_ptr[f + 1];
+    }
+  }
+  // the warp's best: the lane that holds it writes it down
+  auto warp_best = [&](const Cand& mine, const GPairI64& left, SliceBest* out) {
+    Cand best = mine;
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) {
       Cand o;
-      o.gain = __shfl_down_sync(0xffffffffu, best.gain, off);
-      o.bin  = __shfl_down_sync(0xffffffffu, best.bin, off);
+      o.gain    = __shfl_xor_sync(0xffffffffu, best.gain, off);
+      o.bin     = __shfl_xor_sync(0xffffffffu, best.bin, off);
+      o.feature = __shfl_xor_sync(0xffffffffu, best.feature, off);
       if (Better(o, best)) best = o;
     }
+    if (best.bin < 0 ? lane == 0 : mine.bin == best.bin) *out = SliceBest{best, left};
   };
   auto block_best = [&]() {
-    warp_best();
-    if ((tid & 31) == 0) s_c[tid >> 5] = best;
+    warp_best(best_a, left_a, &s_c[0][warp]);
+    if (kDerive) warp_best(best_b, left_b, &s_c[1][warp]);
     __syncthreads();
-    if (tid == 0) {
-      Cand w0 = s_c[0];
-      for (int w = 1; w < kSplitThreads / 32; ++w)
-        if (Better(s_c[w], w0)) w0 = s_c[w];
-      s_best = w0;
+    if (tid < (kDerive ? 2 : 1)) {
+      int at = 0;
+      for (int w = 1; w < n_warps; ++w)
+        if (Better(s_c[tid][w].c, s_c[tid][at].c)) at = w;
+      s_best[tid] = s_c[tid][at];
     }
     __syncthreads();
   };
   block_best();
   if (slices > 1) {
+    SliceBest* mine = p.slice_best + static_cast<int64_t>(unit) * slices * 2;
     if (tid == 0) {
-      SliceBest sb;
-      sb.gain = s_best.gain;
-      sb.bin  = s_best.bin;
-      sb.pad  = 0;
-      slice_best[static_cast<int64_t>(j) * slices + blockIdx.y] = sb;
+      mine[blockIdx.y * 2] = s_best[0];
+      if (kDerive) mine[blockIdx.y * 2 + 1] = s_best[1];
       __threadfence();
-      s_last = atomicAdd(arrived + node, 1u) == static_cast<unsigned>(slices - 1);
+      s_last = atomicAdd(p.arrived + node0, 1u) == static_cast<unsigned>(slices - 1);
     }
+    // (what the other threads wrote to the level's histogram is ordered before thread 0's fence by the
+    // barrier inside block_best)
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    best = Cand{0.0, -1};
-    for (int i = tid; i < slices; i += kSplitThreads) {
-      const volatile SliceBest* sb = slice_best + static_cast<int64_t>(j) * slices + i;
-      const Cand c{sb->gain, sb->bin};
-      if (Better(c, best)) best = c;
+    best_a = best_b = Cand{0.0, -1, -1};
+    for (int i = tid; i < slices; i += blockDim.x) {
+      const volatile SliceBest* a = mine + i * 2;
+      const Cand ca{a[0].c.gain, a[0].c.bin, a[0].c.feature};
+      if (Better(ca, best_a)) {
+        best_a = ca;
+        left_a = GPairI64{a[0].left.grad, a[0].left.hess};
+      }
+      if (kDerive) {
+        const Cand cb{a[1].c.gain, a[1].c.bin, a[1].c.feature};
+        if (Better(cb, best_b)) {
+          best_b = cb;
+          left_b = GPairI64{a[1].left.grad, a[1].left.hess};
+        }
+      }
     }
-    __syncthreads();
     block_best();
   }
-  const Cand nb = s_best;
-  if (records != nullptr) {
-    // leave the candidate and its left sums for the exchange among the ranks
-    unsigned char* rec = records + static_cast<size_t>(j) * SplitRecordBytes(K);
-    if (tid == 0) {
-      SplitRecordHeader h;
-      h.gain = nb.gain;
-      h.bin  = nb.bin;
-      h.pad  = 0;
-      *reinterpret_cast<SplitRecordHeader*>(rec) = h;
+
+  // The sums left of the winning bin: with one output they came along; else from the level's histogram
+  // where it was written, else scanned again from the raw sums (one feature), a warp per output.
+  for (int side = 0; side < (kDerive ? 2 : 1); ++side) {
+    if (!(side == 0 ? eval_a : eval_b)) continue;
+    const int node = side == 0 ? node_a : node_b;
+    const Cand nb  = s_best[side].c;
+    unsigned char* rec = p.records ? p.records + static_cast<size_t>(node - lv.node_begin) * SplitRecordBytes(K) : nullptr;
+    if (rec != nullptr && tid == 0) *reinterpret_cast<SplitRecordHeader*>(rec) = SplitRecordHeader{nb.gain, nb.bin, 0};
+    GPairI64* rec_sums = reinterpret_cast<GPairI64*>(rec + sizeof(SplitRecordHeader));
+    if (nb.bin < 0) {
+      if (rec != nullptr)
+        for (int k = tid; k < K; k += blockDim.x) StorePair(rec_sums + k, GPairI64{0, 0});
+      continue;
     }
-    GPairI64* ls = reinterpret_cast<GPairI64*>(rec + sizeof(SplitRecordHeader));
-    for (int k = tid; k < K; k += kSplitThreads)
-      StorePair(ls + k, nb.bin >= 0 ? LoadPair(hist + static_cast<int64_t>(k) * B + nb.bin) : GPairI64{0, 0});
-    return;
+    for (int k = warp; k < K; k += n_warps) {
+      const int64_t ko = static_cast<int64_t>(k) * Bs;
+      GPairI64 ls;
+      if (!kManyOutputs) {
+        ls = s_best[side].left;
+      } else if (lv.write_hist) {
+        ls = LoadPairStreaming((side == 0 ? dst_a : dst_b) + ko + nb.bin);
+      } else {
+        const bool scanned = s_terms[2 * k].h > 0.0;
+        const GPairI64 raw = LoadPair(src + ko + nb.bin);
+        GPairI64 pre{0, 0};
+        for (int b = p.row_ptr[nb.feature] + lane; b <= nb.bin; b += 32) {
+          const GPairI64 v = LoadPair(src + ko + b);
+          pre.grad += v.grad;
+          pre.hess += v.hess;
+        }
+        for (int off = 16; off >= 1; off >>= 1) {
+          pre.grad += __shfl_xor_sync(0xffffffffu, pre.grad, off);
+          pre.hess += __shfl_xor_sync(0xffffffffu, pre.hess, off);
+        }
+        ls = scanned && (pre.grad > 0 || pre.hess > 0) ? pre : raw;
+        if (side == 1) {
+          const GPairI64 pv = LoadPair(par + ko + nb.bin);
+          ls = scanned ? GPairI64{pv.grad - ls.grad, pv.hess - ls.hess} : GPairI64{0, 0};
+        }
+      }
+      if (rec != nullptr) {
+        if (lane == 0) StorePair(rec_sums + k, ls);
+      } else if (lane == 0) {
+        ApplyWinner<T>(nb, node, K, p.row_ptr, p.cuts, p.cut_stride, p.tree, [&](int) { return ls; }, k, K);
+      }
+    }
   }
-  ApplyWinner<T>(nb, node, K, F, row_ptr, proposals, qp, l1, l2, tree, nb.bin >= 0 ? hist + nb.bin : hist, B, tid,
-                 kSplitThreads);
 }
 
 // One block per node: the best of the ranks' candidates (the same total order as inside a rank, so
@@ -294,130 +406,121 @@ __global__ void __launch_bounds__(kSplitThreads)
 template <typename T>
 __global__ void __launch_bounds__(64)
   k_apply_records(const unsigned char* __restrict__ all_records, int n_ranks, int n_nodes, int node_begin, int K, int F,
-                  const int32_t* __restrict__ row_ptr, const T* __restrict__ proposals,
-                  const QuantParams* __restrict__ qp_ptr, double l1, double l2, TreeArrays tree)
+                  const int32_t* __restrict__ row_ptr, const T* __restrict__ cuts, int64_t cut_stride, TreeArrays tree)
 {
   const int j    = blockIdx.x;
   const int node = node_begin + j;
   if (LoadPair(tree.node_sums + static_cast<int64_t>(node) * K).hess <= 0) return;
   const size_t rb = SplitRecordBytes(K);
-  Cand best{0.0, -1};
+  Cand best{0.0, -1, -1};
   int best_rank = -1;
   for (int r = 0; r < n_ranks; ++r) {
     const SplitRecordHeader* h =
       reinterpret_cast<const SplitRecordHeader*>(all_records + (static_cast<size_t>(r) * n_nodes + j) * rb);
-    const Cand c{h->gain, h->bin};
+    const Cand c{h->gain, h->bin, -1};
     if (c.gain > 0 && c.bin >= 0 && Better(c, best)) {
       best      = c;
       best_rank = r;
     }
   }
   if (best_rank < 0) return;
+  int lo = 0, hi = F;  // the feature of the bin: the last one with row_ptr <= bin
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (row_ptr[mid] <= best.bin) lo = mid; else hi = mid;
+  }
+  best.feature = lo;
   const GPairI64* ls = reinterpret_cast<const GPairI64*>(
     all_records + (static_cast<size_t>(best_rank) * n_nodes + j) * rb + sizeof(SplitRecordHeader));
-  ApplyWinner<T>(best, node, K, F, row_ptr, proposals, *qp_ptr, l1, l2, tree, ls, 1, threadIdx.x, blockDim.x);
+  ApplyWinner<T>(best, node, K, row_ptr, cuts, cut_stride, tree, [&](int k) { return LoadPair(ls + k); }, threadIdx.x, blockDim.x);
 }
 
-__global__ void k_root_leaf(TreeArrays tree, int K, const QuantParams* __restrict__ qp_ptr, double l1, double l2)
-{
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= K) return;
-  const GPairF64 s   = Dequantise(tree.node_sums[k], *qp_ptr);
-  tree.leaf_value[k] = CalculateLeafValue(s.grad, s.hess, l1, l2);
-}
-
-__global__ void k_write_hessian(const GPairI64* __restrict__ node_sums, const QuantParams* __restrict__ qp_ptr,
-                                double* __restrict__ hessian, int64_t n)
+// hessian and leaf value of every node from its quantised sums; a node whose parent did not split keeps 0
+__global__ void __launch_bounds__(256)
+  k_finish_tree(TreeArrays tree, const QuantParams* __restrict__ qp_ptr, int K, int64_t n, double l1, double l2,
+                double* __restrict__ hessian)
 {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (i < n) hessian[i] = static_cast<double>(node_sums[i].hess) * qp_ptr->inv_h;
+  if (i >= n) return;
+  const int node   = static_cast<int>(i / K);
+  const GPairF64 s = Dequantise(tree.node_sums[i], *qp_ptr);
+  hessian[i]       = s.hess;
+  const bool here  = node == 0 || tree.feature[(node - 1) / 2] >= 0;
+  tree.leaf_value[i] = here ? CalculateLeafValue(s.grad, s.hess, l1, l2) : 0.0;
 }
 
 }  // namespace
 
-void PlanBuilt(const GPairI64* node_sums, int K, int node_begin, int n_nodes, bool parent_available,
-               int32_t* slot_of_node, cudaStream_t stream)
-{
-  k_plan_built<<<(n_nodes + 255) / 256, 256, 0, stream>>>(node_sums, K, node_begin, n_nodes, parent_available,
-                                                          slot_of_node);
-  LBK_LAUNCH_CHECK();
-}
-
-void ScanLevel(const GPairI64* built, const int32_t* slot_of_node, GPairI64* level_hist, const GPairI64* parent_hist,
-               int parent_begin, const GPairI64* node_sums, int node_begin, int n_nodes, int K, int f_begin, int f_end,
-               int B, const int32_t* row_ptr, bool parent_available, cudaStream_t stream)
-{
-  const int n_features = f_end - f_begin;
-  if (n_features <= 0 || n_nodes <= 0) return;
-  const int64_t warps  = static_cast<int64_t>(n_nodes) * n_features;
-  const int64_t blocks = (warps + 7) / 8;
-  dim3 grid(static_cast<unsigned>(blocks), K);
-  k_scan<<<grid, 256, 0, stream>>>(built, slot_of_node, level_hist, parent_hist, parent_begin, node_sums, node_begin,
-                                   n_nodes, K, f_begin, n_features, B, row_ptr, parent_available);
-  LBK_LAUNCH_CHECK();
-}
-
 template <typename T>
-void BestSplit(lbk_context* ctx, Scratch& s, const GPairI64* level_hist, int node_begin, int n_nodes, int K, int F, int B,
-               const int32_t* row_ptr, const T* proposals, const QuantParams* qp, const SplitParams& sp, TreeArrays tree,
-               unsigned int* arrived, int f_begin, int f_end, bool exchange_records, cudaStream_t stream)
+void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, const int32_t* row_ptr, const T* cuts,
+               int64_t cut_stride, const QuantParams* qp, const SplitParams& sp, const TreeArrays& tree,
+               unsigned int* arrived, bool exchange_records, cudaStream_t stream)
 {
-  const int sm_count = ctx->sm_count;
-  // the bins of the features [f_begin, f_end): row_ptr lives on the device, so the kernel gets the
-  // range through two small reads of its own; here only an upper bound of its length matters
-  const int n_bins_bound = exchange_records ? (B + ctx->n_ranks - 1) / ctx->n_ranks + 1 : B;
-  // enough blocks for two per SM, at least one thread per bin in a block's slice
-  int slices = (2 * sm_count + n_nodes - 1) / n_nodes;
-  const int most = (n_bins_bound + kSplitThreads - 1) / kSplitThreads;
+  const int n_features = lv.f_end - lv.f_begin;
+  const int units      = lv.derive ? lv.n_nodes / 2 : lv.n_nodes;
+  if (units <= 0) return;
+  // with several outputs a block keeps K terms of two nodes and every warp K running prefixes in shared
+  // memory: fewer warps for very many outputs
+  int warps = kSplitWarps;
+  auto need = [&](int w) {
+    return lv.K > 1 ? sizeof(NodeTerms) * 2 * ((lv.K + 1) / 2 * 2) + static_cast<size_t>(w) * lv.K * sizeof(GPairI64) : 0;
+  };
+  while (warps > 1 && need(warps) > 40 * 1024) warps /= 2;
+  const size_t smem = need(warps);
+  // one feature per warp until there are about eight blocks per SM, then several
+  int slices     = (n_features + warps - 1) / warps;
+  const int most = (8 * ctx->sm_count + units - 1) / units;
   if (slices > most) slices = most;
-  if (slices > kSplitThreads) slices = kSplitThreads;
   if (slices < 1) slices = 1;
-  SliceBest* slice_best = slices > 1 ? s.alloc<SliceBest>(static_cast<size_t>(n_nodes) * slices) : nullptr;
-  if (!exchange_records) {
-    k_best_split<T><<<dim3(n_nodes, slices), kSplitThreads, 0, stream>>>(
-      level_hist, node_begin, K, F, B, row_ptr, proposals, qp, sp.l1, sp.l2, sp.min_split_gain, sp.feature_set, tree,
-      slice_best, arrived, f_begin, f_end, nullptr);
-    LBK_LAUNCH_CHECK();
-    if (slice_best) s.free_one(slice_best);
-    return;
+  ScanSplitParams<T> p;
+  p.lv         = lv;
+  p.row_ptr    = row_ptr;
+  p.cuts       = cuts;
+  p.cut_stride = cut_stride;
+  p.qp         = qp;
+  p.sp         = sp;
+  p.tree       = tree;
+  p.slice_best = slices > 1 ? s.alloc<SliceBest>(static_cast<size_t>(units) * slices * 2) : nullptr;
+  p.arrived    = arrived;
+  p.records    = nullptr;
+  unsigned char *mine = nullptr, *all = nullptr;
+  const size_t rb = SplitRecordBytes(lv.K);
+  if (exchange_records) {
+    mine = s.alloc<unsigned char>(rb * lv.n_nodes);
+    all  = s.alloc<unsigned char>(rb * lv.n_nodes * ctx->n_ranks);
+    LBK_CUDA(cudaMemsetAsync(mine, 0, rb * lv.n_nodes, stream));
+    p.records = mine;
   }
-  // every rank searches its own features, then the candidates of all ranks meet on every rank
-  const size_t rb   = SplitRecordBytes(K);
-  const int R       = ctx->n_ranks;
-  unsigned char* mine = s.alloc<unsigned char>(rb * n_nodes);
-  unsigned char* all  = s.alloc<unsigned char>(rb * n_nodes * R);
-  LBK_CUDA(cudaMemsetAsync(mine, 0, rb * n_nodes, stream));
-  k_best_split<T><<<dim3(n_nodes, slices), kSplitThreads, 0, stream>>>(
-    level_hist, node_begin, K, F, B, row_ptr, proposals, qp, sp.l1, sp.l2, sp.min_split_gain, sp.feature_set, tree,
-    slice_best, arrived, f_begin, f_end, mine);
+  auto fn = lv.K > 1 ? (lv.derive ? k_scan_split<T, true, true, 2> : k_scan_split<T, true, false, 2>)
+                     : (lv.derive ? k_scan_split<T, false, true, 4> : k_scan_split<T, false, false, 4>);
+  if (smem > 48 * 1024)
+    LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  fn<<<dim3(units, slices), warps * 32, smem, stream>>>(p);
   LBK_LAUNCH_CHECK();
-  if (!AllGatherBytes(ctx, mine, all, rb * n_nodes, stream))
-    throw Error(LBK_ERR_COMM, "the split records need an NCCL communicator");
-  k_apply_records<T><<<n_nodes, 64, 0, stream>>>(all, R, n_nodes, node_begin, K, F, row_ptr, proposals, qp, sp.l1, sp.l2,
-                                                  tree);
-  LBK_LAUNCH_CHECK();
-  if (slice_best) s.free_one(slice_best);
-  s.free_one(mine);
-  s.free_one(all);
+  if (exchange_records) {
+    // every rank has searched its own features: the candidates of all ranks meet on every rank
+    if (!AllGatherBytes(ctx, mine, all, rb * lv.n_nodes, stream))
+      throw Error(LBK_ERR_COMM, "the split records need an NCCL communicator");
+    k_apply_records<T><<<lv.n_nodes, 64, 0, stream>>>(all, ctx->n_ranks, lv.n_nodes, lv.node_begin, lv.K, F, row_ptr, cuts,
+                                                      cut_stride, tree);
+    LBK_LAUNCH_CHECK();
+    s.free_one(mine);
+    s.free_one(all);
+  }
+  if (p.slice_best) s.free_one(p.slice_best);
 }
 
-void RootLeaf(TreeArrays tree, int K, const QuantParams* qp, double l1, double l2, cudaStream_t stream)
+void FinishTree(const TreeArrays& tree, const QuantParams* qp, int K, double l1, double l2, double* hessian,
+                cudaStream_t stream)
 {
-  k_root_leaf<<<(K + 127) / 128, 128, 0, stream>>>(tree, K, qp, l1, l2);
+  const int64_t n = static_cast<int64_t>(tree.max_nodes) * K;
+  k_finish_tree<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(tree, qp, K, n, l1, l2, hessian);
   LBK_LAUNCH_CHECK();
 }
 
-void WriteHessian(const GPairI64* node_sums, const QuantParams* qp, double* hessian, int64_t n, cudaStream_t stream)
-{
-  k_write_hessian<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(node_sums, qp, hessian, n);
-  LBK_LAUNCH_CHECK();
-}
-
-template void BestSplit<float>(lbk_context*, Scratch&, const GPairI64*, int, int, int, int, int, const int32_t*,
-                               const float*, const QuantParams*, const SplitParams&, TreeArrays, unsigned int*, int, int,
-                               bool, cudaStream_t);
-template void BestSplit<double>(lbk_context*, Scratch&, const GPairI64*, int, int, int, int, int, const int32_t*,
-                                const double*, const QuantParams*, const SplitParams&, TreeArrays, unsigned int*, int, int,
-                                bool, cudaStream_t);
+template void ScanSplit<float>(lbk_context*, Scratch&, const ScanSplitLevel&, int, const int32_t*, const float*, int64_t,
+                               const QuantParams*, const SplitParams&, const TreeArrays&, unsigned int*, bool, cudaStream_t);
+template void ScanSplit<double>(lbk_context*, Scratch&, const ScanSplitLevel&, int, const int32_t*, const double*, int64_t,
+                                const QuantParams*, const SplitParams&, const TreeArrays&, unsigned int*, bool, cudaStream_t);
 
 }  // namespace lbk

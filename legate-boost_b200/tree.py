@@ -73,7 +73,7 @@ class Sketch:
 
 def build_tree_arrays(X, g, h, *, max_depth, split_samples, seed, l1=0.0, l2=1.0, min_split_gain=0.0,
                       feature_set=None, row_offset=None, dataset_rows=None, trace_nodes=0, ctx=None,
-                      want_leaf=False, sketch=None):
+                      want_leaf=False, sketch=None, want_node_sums=True):
     """Run ``lbk_build_tree`` on device tensors.  Returns a dict with the five tree arrays (and the
     optional traces; with ``want_leaf`` also ``leaf``: the node every local row ends in).  With a
     ``Sketch`` the proposals and bins are saved in it or, if it holds those of this matrix, reused."""
@@ -116,8 +116,9 @@ def build_tree_arrays(X, g, h, *, max_depth, split_samples, seed, l1=0.0, l2=1.0
     a.stream = _stream_ptr()
     B = C.c_int32(0)
     a.out_total_bins = C.pointer(B)
-    out["node_sums"] = torch.zeros((M, K, 2), dtype=torch.int64, device=dev)
-    a.trace_node_sums = out["node_sums"].data_ptr()
+    if want_node_sums:
+        out["node_sums"] = torch.empty((M, K, 2), dtype=torch.int64, device=dev)
+        a.trace_node_sums = out["node_sums"].data_ptr()
     trace = None
     if trace_nodes > 0:
         trace = torch.zeros((trace_nodes, K, F * split_samples, 2), dtype=torch.int64, device=dev)
@@ -346,7 +347,7 @@ class Tree(BaseModel):
             X, g, h, max_depth=self.max_depth, split_samples=self.split_samples, seed=seed,
             l1=self.l1_regularization, l2=self.l2_regularization, min_split_gain=self.min_split_gain,
             feature_set=feature_set, want_leaf=True, row_offset=row_offset, dataset_rows=dataset_rows,
-            sketch=getattr(self, "sketch", None))
+            sketch=getattr(self, "sketch", None), want_node_sums=False)
         self.leaf_value = out["leaf_value"]
         self.feature = out["feature"]
         self.split_value = out["split_value"]
