@@ -173,6 +173,27 @@ enum { LBK_SKETCH_OFF = 0, LBK_SKETCH_SAVE = 1, LBK_SKETCH_REUSE = 2 };
 
 int lbk_build_tree(lbk_context* ctx, const lbk_build_tree_args* args);
 
+/* One boosting round: the weighted gradients of `pred` (what lbk_gradient computes), a tree on them
+ * (lbk_build_tree; tree.g, tree.h and tree.ldg are ignored, no host buffers, no histogram trace, no
+ * out_total_bins) and pred += the tree's leaf value of every row.  Asynchronous on tree.stream unless the
+ * number of bins decides the layout (more than 256 split samples, a sketch, several ranks, histograms
+ * beyond the cache: then it waits for that number); a fault that a kernel reports is returned by a later
+ * call on the context, at the latest by lbk_synchronize.  The buffers stay in use until the stream gets
+ * there.  No counterpart in the reference, whose driver launches one task per step
+ * (legateboost/legateboost.py:254-298). */
+typedef struct lbk_boost_round_args {
+  lbk_build_tree_args tree;
+  int32_t objective;      /* LBK_SQUARED_ERROR or LBK_LOG_LOSS */
+  const double* y;        /* as in lbk_gradient */
+  double* pred;           /* [n_local_rows, n_outputs], in and out */
+  double learning_rate;
+} lbk_boost_round_args;
+
+int lbk_boost_round(lbk_context* ctx, const lbk_boost_round_args* args);
+
+/* Waits for `stream` and returns what kernels of earlier calls have reported (LBK_ERR_DEVICE). */
+int lbk_synchronize(lbk_context* ctx, void* stream);
+
 /* Bytes of the sketch buffer for a matrix of this shape (0 for a bad shape). */
 size_t lbk_sketch_bytes(int64_t n_local_rows, int n_features, int split_samples, int x_dtype);
 

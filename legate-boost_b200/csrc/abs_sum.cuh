@@ -11,6 +11,31 @@ constexpr int kSumThreads = 256;
 constexpr int kSumItems   = 16;
 constexpr int kSumBlock   = kSumThreads * kSumItems;  // 4096
 
+// The second half of a block's sum: groups of 32 threads fold into s_sum (16 values per 256 threads), and,
+// after a barrier, one thread adds the 8 group sums left to right.
+__device__ inline void FoldAbsSums(double sg, double sh, int tid, double* s_sum)
+{
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) {
+    sg += __shfl_down_sync(0xffffffffu, sg, off);
+    sh += __shfl_down_sync(0xffffffffu, sh, off);
+  }
+  if ((tid & 31) == 0) {
+    s_sum[tid >> 5]                      = sg;
+    s_sum[kSumThreads / 32 + (tid >> 5)] = sh;
+  }
+}
+__device__ inline void JoinAbsSums(const double* s_sum, double& tg, double& th)
+{
+  tg = s_sum[0];
+  th = s_sum[kSumThreads / 32];
+#pragma unroll
+  for (int w = 1; w < kSumThreads / 32; ++w) {
+    tg += s_sum[w];
+    th += s_sum[kSumThreads / 32 + w];
+  }
+}
+
 // Sums of block `block`, returned to thread 0 of the 256 (`tid` = 0..255 within the group; all threads of the
 // CTA call it, several groups may do so at once).  kFirst: |g|, |h| of the strided [n / K, K] inputs, else the
 // partial sums themselves.  s_sum: shared, 16 values per group.
@@ -38,26 +63,10 @@ __device__ inline void AbsSumPartial(const double* g, const double* h, int64_t l
     sg += vg;
     sh += vh;
   }
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) {
-    sg += __shfl_down_sync(0xffffffffu, sg, off);
-    sh += __shfl_down_sync(0xffffffffu, sh, off);
-  }
-  if ((tid & 31) == 0) {
-    s_sum[tid >> 5]                    = sg;
-    s_sum[kSumThreads / 32 + (tid >> 5)] = sh;
-  }
+  FoldAbsSums(sg, sh, tid, s_sum);
   __syncthreads();
   tg = th = 0.0;
-  if (tid == 0) {
-    tg = s_sum[0];
-    th = s_sum[kSumThreads / 32];
-#pragma unroll
-    for (int w = 1; w < kSumThreads / 32; ++w) {
-      tg += s_sum[w];
-      th += s_sum[kSumThreads / 32 + w];
-    }
-  }
+  if (tid == 0) JoinAbsSums(s_sum, tg, th);
 }
 
 template <bool kFirst>

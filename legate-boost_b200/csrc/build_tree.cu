@@ -159,8 +159,22 @@ SketchLayout SketchLayoutOf(int64_t N, int F, int S, size_t elem_bytes)
   return l;
 }
 
+// pred[i] += table[leaf[i]]: the leaf values of a round's tree onto the current prediction
+__global__ void __launch_bounds__(256)
+  k_add_leaf_values(const double* __restrict__ table, const int32_t* __restrict__ leaf, int64_t n, int K,
+                    double* __restrict__ pred)
+{
+  const int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (e >= n * K) return;
+  const int64_t i = K == 1 ? e : e / K;
+  const int k     = static_cast<int>(e - i * K);
+  pred[e] += __ldg(table + static_cast<int64_t>(__ldg(leaf + i)) * K + k);
+}
+
+// `round`: a boosting round instead of a tree on given gradients (they are those of round->pred, which gets
+// the leaf values added); the call is then asynchronous.
 template <typename T>
-void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t stream)
+void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t stream, const lbk_boost_round_args* round)
 {
   const int F = a.n_features, K = a.n_outputs, D = a.max_depth;
   const int64_t N = a.n_local_rows;
@@ -198,8 +212,79 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     gain        = s.alloc<double>(M);
     feature     = s.alloc<int32_t>(M);
   }
+  auto copy_tree_back = [&]() {
+    LBK_CUDA(cudaMemcpyAsync(a.leaf_value, leaf_value, sizeof(double) * M * K, cudaMemcpyDeviceToHost, stream));
+    LBK_CUDA(cudaMemcpyAsync(a.feature, feature, sizeof(int32_t) * M, cudaMemcpyDeviceToHost, stream));
+    LBK_CUDA(cudaMemcpyAsync(a.split_value, split_value, sizeof(double) * M, cudaMemcpyDeviceToHost, stream));
+    LBK_CUDA(cudaMemcpyAsync(a.gain, gain, sizeof(double) * M, cudaMemcpyDeviceToHost, stream));
+    LBK_CUDA(cudaMemcpyAsync(a.hessian, hessian, sizeof(double) * M * K, cudaMemcpyDeviceToHost, stream));
+  };
 
   // Tree (reference: struct Tree, build_tree.cu:785-809)
+  if (ctx->n_ranks <= 1 && a.sketch_mode == LBK_SKETCH_OFF && a.trace_hist == nullptr &&
+      SmallTreeFits(ctx, N, F, K, D, a.split_samples, sizeof(T))) {
+    SmallTreeArgs<T> t{};
+    t.X            = X;
+    t.ldx          = ldx;
+    t.N            = N;
+    t.F            = F;
+    t.K            = K;
+    t.D            = D;
+    t.S            = a.split_samples;
+    t.seed         = a.seed;
+    t.row_offset   = a.row_offset;
+    t.dataset_rows = a.dataset_rows;
+    t.g            = g;
+    t.h            = h;
+    t.ldg          = ldg;
+    t.objective    = -1;
+    const bool fused = round != nullptr && (round->objective == LBK_SQUARED_ERROR || K == 1);
+    if (fused) {
+      t.objective = round->objective;
+      t.y         = round->y;
+      t.pred      = round->pred;
+      t.lr        = round->learning_rate;
+    } else if (round != nullptr) {
+      double* rg = s.alloc<double>(static_cast<size_t>(N) * K);
+      double* rh = s.alloc<double>(static_cast<size_t>(N) * K);
+      Gradient(round->objective, round->pred, round->y, N, K, round->learning_rate, rg, rh, stream);
+      t.g   = rg;
+      t.h   = rh;
+      t.ldg = K;
+    }
+    t.sp          = SplitParams{a.l1_regularization, a.l2_regularization, a.min_split_gain, fset};
+    const bool device_sums = a.trace_node_sums != nullptr && !a.host_buffers;
+    t.tree        = TreeArrays{leaf_value, feature, split_value, gain,
+                        device_sums ? reinterpret_cast<GPairI64*>(a.trace_node_sums) : s.alloc<GPairI64>(static_cast<size_t>(M) * K),
+                        nullptr, M};
+    t.hessian     = hessian;
+    int32_t* leaf = a.out_leaf != nullptr && !a.host_buffers ? a.out_leaf
+                    : a.out_leaf != nullptr || (round != nullptr && !fused) ? s.alloc<int32_t>(static_cast<size_t>(N)) : nullptr;
+    t.leaf        = leaf;
+    SmallTree<T>(ctx, s, t, stream);
+    if (round != nullptr && !fused) {
+      k_add_leaf_values<<<static_cast<unsigned>((N * K + 255) / 256), 256, 0, stream>>>(leaf_value, leaf, N, K, round->pred);
+      LBK_LAUNCH_CHECK();
+    }
+    if (a.trace_node_sums && !device_sums)
+      LBK_CUDA(cudaMemcpyAsync(a.trace_node_sums, t.tree.node_sums, sizeof(GPairI64) * M * K, cudaMemcpyDefault, stream));
+    if (a.host_buffers) {
+      if (a.out_leaf) LBK_CUDA(cudaMemcpyAsync(a.out_leaf, leaf, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, stream));
+      copy_tree_back();
+    }
+    if (round != nullptr) return;
+    CheckDeviceStatus(ctx, stream);
+    if (a.out_total_bins) *a.out_total_bins = ctx->h_info[0];
+    return;
+  }
+  if (round != nullptr) {
+    double* rg = s.alloc<double>(static_cast<size_t>(N) * K);
+    double* rh = s.alloc<double>(static_cast<size_t>(N) * K);
+    Gradient(round->objective, round->pred, round->y, N, K, round->learning_rate, rg, rh, stream);
+    g   = rg;
+    h   = rh;
+    ldg = K;
+  }
   const bool keep_sums = a.trace_node_sums != nullptr && !a.host_buffers;
   TreeArrays tree;
   tree.leaf_value  = leaf_value;
@@ -539,25 +624,42 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   }
 
   FinishTree(tree, qp, K, a.l1_regularization, a.l2_regularization, hessian, stream);
-  if (a.out_leaf != nullptr && N > 0) {
-    int32_t* d_leaf = a.host_buffers ? s.alloc<int32_t>(static_cast<size_t>(N)) : a.out_leaf;
+  if ((a.out_leaf != nullptr || round != nullptr) && N > 0) {
+    int32_t* d_leaf = a.out_leaf != nullptr && !a.host_buffers ? a.out_leaf : s.alloc<int32_t>(static_cast<size_t>(N));
     const int64_t pitch = static_cast<int64_t>((F + kGroup - 1) / kGroup) * kGroup;
     if (bin_bytes == 1) LeafOfRow<uint8_t>(ctx, bins, pitch, N, F, tree.feature, tree.split_bin, D, M, d_leaf, stream);
     else LeafOfRow<uint16_t>(ctx, bins, pitch, N, F, tree.feature, tree.split_bin, D, M, d_leaf, stream);
-    if (a.host_buffers)
+    if (a.host_buffers && a.out_leaf)
       LBK_CUDA(cudaMemcpyAsync(a.out_leaf, d_leaf, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, stream));
+    if (round != nullptr) {
+      k_add_leaf_values<<<static_cast<unsigned>((N * K + 255) / 256), 256, 0, stream>>>(leaf_value, d_leaf, N, K, round->pred);
+      LBK_LAUNCH_CHECK();
+    }
   }
   if (a.trace_node_sums && !keep_sums)
     LBK_CUDA(cudaMemcpyAsync(a.trace_node_sums, tree.node_sums, sizeof(GPairI64) * M * K, cudaMemcpyDefault, stream));
-  if (a.host_buffers) {
-    LBK_CUDA(cudaMemcpyAsync(a.leaf_value, leaf_value, sizeof(double) * M * K, cudaMemcpyDeviceToHost, stream));
-    LBK_CUDA(cudaMemcpyAsync(a.feature, feature, sizeof(int32_t) * M, cudaMemcpyDeviceToHost, stream));
-    LBK_CUDA(cudaMemcpyAsync(a.split_value, split_value, sizeof(double) * M, cudaMemcpyDeviceToHost, stream));
-    LBK_CUDA(cudaMemcpyAsync(a.gain, gain, sizeof(double) * M, cudaMemcpyDeviceToHost, stream));
-    LBK_CUDA(cudaMemcpyAsync(a.hessian, hessian, sizeof(double) * M * K, cudaMemcpyDeviceToHost, stream));
-  }
+  if (a.host_buffers) copy_tree_back();
+  if (round != nullptr) return;
   CheckDeviceStatus(ctx, stream);  // synchronises, as the reference's task does (:1356)
   if (a.out_total_bins) *a.out_total_bins = sketch_reuse ? head.total_bins : ctx->h_info[0];
+}
+
+void CheckTreeArgs(const lbk_build_tree_args& a)
+{
+  LBK_EXPECT(a.x_dtype == LBK_F32 || a.x_dtype == LBK_F64, "X must be float32 or float64");
+  LBK_EXPECT(a.n_features >= 1 && a.n_outputs >= 1, "need at least one feature and one output");
+  LBK_EXPECT(a.n_local_rows >= 0 && a.n_local_rows < (int64_t{1} << 31), "rows per rank must fit 31 bits");
+  LBK_EXPECT(a.dataset_rows >= 1, "dataset_rows must be positive");
+  LBK_EXPECT(a.max_depth >= 0 && a.max_depth <= 29, "max_depth out of range");
+  LBK_EXPECT(a.max_nodes == (1 << (a.max_depth + 1)) - 1, "max_nodes must be 2^(max_depth+1)-1");
+  LBK_EXPECT(a.split_samples >= 1 && a.split_samples <= 2048, "split_samples must be in [1, 2048]");
+  LBK_EXPECT(a.sketch_mode == LBK_SKETCH_OFF || a.sketch_mode == LBK_SKETCH_SAVE || a.sketch_mode == LBK_SKETCH_REUSE,
+             "unknown sketch mode");
+  LBK_EXPECT(a.sketch_mode == LBK_SKETCH_OFF || a.sketch != nullptr, "sketch mode without a sketch buffer");
+  LBK_EXPECT(a.n_local_rows == 0 || (a.X || a.sketch_mode == LBK_SKETCH_REUSE), "null input");
+  LBK_EXPECT(a.n_local_rows == 0 || a.ldx >= a.n_features, "Expected a dense row major store");
+  LBK_EXPECT(a.leaf_value && a.feature && a.split_value && a.gain && a.hessian, "null output");
+  LBK_EXPECT(a.row_offset >= 0 && a.row_offset + a.n_local_rows <= a.dataset_rows, "row range outside the data set");
 }
 
 }  // namespace
@@ -582,25 +684,42 @@ int lbk_build_tree(lbk_context* ctx, const lbk_build_tree_args* a)
   return lbk::Guard(ctx, [&] {
     LBK_EXPECT(ctx && a, "null argument");
     LBK_CUDA(cudaSetDevice(ctx->device));
-    LBK_EXPECT(a->x_dtype == LBK_F32 || a->x_dtype == LBK_F64, "X must be float32 or float64");
-    LBK_EXPECT(a->n_features >= 1 && a->n_outputs >= 1, "need at least one feature and one output");
-    LBK_EXPECT(a->n_local_rows >= 0 && a->n_local_rows < (int64_t{1} << 31), "rows per rank must fit 31 bits");
-    LBK_EXPECT(a->dataset_rows >= 1, "dataset_rows must be positive");
-    LBK_EXPECT(a->max_depth >= 0 && a->max_depth <= 29, "max_depth out of range");
-    LBK_EXPECT(a->max_nodes == (1 << (a->max_depth + 1)) - 1, "max_nodes must be 2^(max_depth+1)-1");
-    LBK_EXPECT(a->split_samples >= 1 && a->split_samples <= 2048, "split_samples must be in [1, 2048]");
-    LBK_EXPECT(a->sketch_mode == LBK_SKETCH_OFF || a->sketch_mode == LBK_SKETCH_SAVE || a->sketch_mode == LBK_SKETCH_REUSE,
-               "unknown sketch mode");
-    LBK_EXPECT(a->sketch_mode == LBK_SKETCH_OFF || a->sketch != nullptr, "sketch mode without a sketch buffer");
-    LBK_EXPECT(a->n_local_rows == 0 || ((a->X || a->sketch_mode == LBK_SKETCH_REUSE) && a->g && a->h), "null input");
-    LBK_EXPECT(a->n_local_rows == 0 || (a->ldx >= a->n_features && a->ldg >= a->n_outputs), "Expected a dense row major store");
-    LBK_EXPECT(a->leaf_value && a->feature && a->split_value && a->gain && a->hessian, "null output");
-    LBK_EXPECT(a->row_offset >= 0 && a->row_offset + a->n_local_rows <= a->dataset_rows, "row range outside the data set");
+    lbk::CheckTreeArgs(*a);
+    LBK_EXPECT(a->n_local_rows == 0 || (a->g && a->h), "null input");
+    LBK_EXPECT(a->n_local_rows == 0 || a->ldg >= a->n_outputs, "Expected a dense row major store");
     cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
     if (a->x_dtype == LBK_F32)
-      lbk::BuildTreeImpl<float>(ctx, *a, stream);
+      lbk::BuildTreeImpl<float>(ctx, *a, stream, nullptr);
     else
-      lbk::BuildTreeImpl<double>(ctx, *a, stream);
+      lbk::BuildTreeImpl<double>(ctx, *a, stream, nullptr);
+  });
+}
+
+int lbk_boost_round(lbk_context* ctx, const lbk_boost_round_args* r)
+{
+  return lbk::Guard(ctx, [&] {
+    LBK_EXPECT(ctx && r, "null argument");
+    LBK_CUDA(cudaSetDevice(ctx->device));
+    const lbk_build_tree_args& a = r->tree;
+    lbk::CheckTreeArgs(a);
+    LBK_EXPECT(r->objective == LBK_SQUARED_ERROR || r->objective == LBK_LOG_LOSS, "unknown objective");
+    LBK_EXPECT(!a.host_buffers && a.trace_hist == nullptr && a.out_total_bins == nullptr, "a round takes device buffers and no trace");
+    LBK_EXPECT(a.n_local_rows == 0 || (r->y && r->pred), "null input");
+    lbk::ThrowReportedFault(ctx);
+    cudaStream_t stream = static_cast<cudaStream_t>(a.stream);
+    if (a.x_dtype == LBK_F32)
+      lbk::BuildTreeImpl<float>(ctx, a, stream, r);
+    else
+      lbk::BuildTreeImpl<double>(ctx, a, stream, r);
+  });
+}
+
+int lbk_synchronize(lbk_context* ctx, void* stream)
+{
+  return lbk::Guard(ctx, [&] {
+    LBK_EXPECT(ctx != nullptr, "context is null");
+    LBK_CUDA(cudaSetDevice(ctx->device));
+    lbk::CheckDeviceStatus(ctx, static_cast<cudaStream_t>(stream));
   });
 }
 

@@ -109,7 +109,7 @@ void* Scratch::alloc_bytes(size_t bytes)
     const size_t need = (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
     if (slab_ == nullptr || slab_used_ + need > kSlab) {
       slab_      = static_cast<char*>(AllocBlock(kSlab));
-      slab_used_ = 0;
+      slab_used_ = 256;  // no small buffer has the address of the block, which free_one would give back
     }
     void* p = slab_ + slab_used_;
     slab_used_ += need;
@@ -192,6 +192,10 @@ void ThrowReportedFault(lbk_context* ctx)
   const int h        = *word;
   if (h == 0) return;
   *word = 0;
+  if (ctx->grid_barrier != nullptr) {  // the count may not be where the host believes it is
+    cudaFree(ctx->grid_barrier);
+    ctx->grid_barrier = nullptr;
+  }
   throw Error(LBK_ERR_DEVICE, "a kernel reported fault code " + std::to_string(h));
 }
 
@@ -270,6 +274,7 @@ void lbk_context_destroy(lbk_context* ctx)
   cudaDeviceSynchronize();
   lbk::DestroyExchange(ctx);
   if (ctx->owns_nccl && ctx->nccl_comm && nccl().CommDestroy) nccl().CommDestroy(ctx->nccl_comm);
+  if (ctx->grid_barrier) cudaFree(ctx->grid_barrier);
   if (ctx->d_status) cudaFreeHost(ctx->d_status);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   for (auto& ev : ctx->prof_events) {

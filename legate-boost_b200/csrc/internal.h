@@ -76,6 +76,10 @@ struct lbk_context {
   // status word in mapped host memory: 0 = ok, otherwise a kernel stored a fault code
   int* d_status = nullptr;
   int32_t* h_info = nullptr;  // mapped host memory [2], beside it: number of bins, bins of the largest feature
+  // grid barrier of the one-launch trees: a word that only counts up, and where it stands
+  unsigned int* grid_barrier     = nullptr;
+  unsigned int grid_barrier_base = 0;
+  bool small_tree_ready[2]       = {false, false};
   // communicator
   int rank = 0, n_ranks = 1;
   void* nccl_comm     = nullptr;
@@ -335,6 +339,34 @@ struct PartitionLevel {
   int K                = 0;
 };
 void PartitionRows(lbk_context* ctx, Scratch& s, const PartitionLevel& pl, cudaStream_t stream);
+// objective.cu
+void Gradient(int objective, const double* raw_pred, const double* y, int64_t n_rows, int n_outputs, double learning_rate,
+              double* g, double* h, cudaStream_t stream);
+// small_tree.cu: a whole tree in one launch, for matrices of at most kSmallMaxElements rows x outputs
+constexpr int64_t kSmallMaxElements = 16384;
+template <typename T>
+struct SmallTreeArgs {
+  const T* X;
+  int64_t ldx, N;
+  int F, K, D, S, seed;
+  int64_t row_offset, dataset_rows;
+  const double* g;
+  const double* h;
+  int64_t ldg;
+  // objective >= 0: the gradients are those of `pred` (squared error, or log loss with one output), and the
+  // tree's leaf values are added to it; g and h are not read
+  int objective;
+  const double* y;
+  double* pred;
+  double lr;
+  SplitParams sp;
+  TreeArrays tree;   // node_sums [max_nodes][K]; split_bin is not used
+  double* hessian;
+  int32_t* leaf;     // may be null
+};
+bool SmallTreeFits(lbk_context* ctx, int64_t N, int F, int K, int D, int S, size_t elem);
+template <typename T>
+void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStream_t stream);
 // predict.cu
 template <typename T>
 void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees,

@@ -8,8 +8,8 @@
 // multi-class softmax with the row maximum taken out, g = p - onehot(label), h = p (1 - p).
 // The reference runs them as a chain of array operations (about ten passes over N x K float64);
 // here a row is read once and its pairs are written once.
-#include "device_utils.cuh"
 #include "internal.h"
+#include "objective.cuh"
 
 namespace lbk {
 namespace {
@@ -22,8 +22,9 @@ __global__ void __launch_bounds__(256)
 {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
-  g[i] = (raw[i] - y[i]) * lr;
-  h[i] = 1.0;
+  const double2 v = GradientSquaredError(raw[i], y[i], lr);
+  g[i] = v.x;
+  h[i] = v.y;
 }
 
 __global__ void __launch_bounds__(256)
@@ -32,9 +33,9 @@ __global__ void __launch_bounds__(256)
 {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
-  const double p = 1.0 / (1.0 + exp(-raw[i]));
-  g[i]           = (p - y[i]) * lr;
-  h[i]           = fmax(p * (1.0 - p), 1e-8);
+  const double2 v = GradientLogistic(raw[i], y[i], lr);
+  g[i] = v.x;
+  h[i] = v.y;
 }
 
 // one thread per row; the exponentials of up to 32 classes stay in registers, more are recomputed
@@ -64,6 +65,23 @@ __global__ void __launch_bounds__(256)
 }
 
 }  // namespace
+
+void Gradient(int objective, const double* raw_pred, const double* y, int64_t n_rows, int n_outputs, double learning_rate,
+              double* g, double* h, cudaStream_t stream)
+{
+  if (n_rows == 0) return;
+  const int64_t n = n_rows * n_outputs;
+  if (objective == LBK_SQUARED_ERROR) {
+    k_gradient_squared_error<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(raw_pred, y, n, learning_rate, g, h);
+  } else if (n_outputs == 1) {
+    k_gradient_logloss_binary<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(raw_pred, y, n, learning_rate, g, h);
+  } else {
+    k_gradient_softmax<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(raw_pred, y, n_rows, n_outputs,
+                                                                                       learning_rate, g, h);
+  }
+  LBK_LAUNCH_CHECK();
+}
+
 }  // namespace lbk
 
 extern "C" int lbk_gradient(lbk_context* ctx, int objective, const double* raw_pred, const double* y, int64_t n_rows,
@@ -77,18 +95,6 @@ extern "C" int lbk_gradient(lbk_context* ctx, int objective, const double* raw_p
     if (n_rows == 0) return;
     LBK_EXPECT(raw_pred && y && g && h, "null argument");
     LBK_CUDA(cudaSetDevice(ctx->device));
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    const int64_t n     = n_rows * n_outputs;
-    if (objective == LBK_SQUARED_ERROR) {
-      k_gradient_squared_error<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(raw_pred, y, n, learning_rate,
-                                                                                          g, h);
-    } else if (n_outputs == 1) {
-      k_gradient_logloss_binary<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(raw_pred, y, n, learning_rate,
-                                                                                           g, h);
-    } else {
-      k_gradient_softmax<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(raw_pred, y, n_rows, n_outputs,
-                                                                                         learning_rate, g, h);
-    }
-    LBK_LAUNCH_CHECK();
+    Gradient(objective, raw_pred, y, n_rows, n_outputs, learning_rate, g, h, static_cast<cudaStream_t>(stream_));
   });
 }

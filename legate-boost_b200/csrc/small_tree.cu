@@ -1,0 +1,723 @@
+// A whole tree on a small matrix in one cooperative launch.
+//
+// With a few thousand rows every kernel of the general path (build_tree.cu) takes its fixed cost - launch,
+// dependent loads, a last block that everybody waits for - and a tree has more than a dozen of them.  Here the
+// features are divided among the blocks and the blocks meet at one grid barrier per level:
+//   * block (feature, part) draws, sorts and prunes the feature's proposals, bins its column and quantises a
+//     slice of the rows; the |g|, |h| sums (canonical order, abs_sum.cuh) are made by every block for itself;
+//   * every block keeps the node of every row in shared memory.  On a level it sums its feature's
+//     histograms of the built nodes in shared memory, scans them, derives the siblings from the parents'
+//     (kept in global memory, one region per feature) and leaves its best candidate of every node;
+//   * after the barrier every block picks the winners of the level by itself (same candidates, same total
+//     order, so all blocks agree) and moves the rows down, reading the winning features' bin ids.
+// No repartition, no list of rows, no merge of partial histograms.
+//
+// 32-bit shared-memory sums are exact here without a bound on the magnitudes: a quantised value is added as
+// its high and its low 16 bits, whose sums over at most 65536 rows fit 32 bits.
+//
+// What bounds it: the chain of latencies of a level - pass over the rows, scan, float64 divisions, barrier,
+// candidates, move: 8 - 9 us each, of which the barrier is one, and about 10 us for everything before the root.
+// A thread per bin: with a warp per node (four bins per lane) a level of 500 x 10 took 9 us longer, because a
+// lone warp gets an instruction in about five clocks.  500 x 10, depth 4: 49 us per tree (260 us of kernels in
+// 70 launches, 570 us of wall time before); 712 x 128, 3 classes, depth 8, 7 rounds: 9.15 -> 3.9 ms.
+
+#include "abs_sum.cuh"
+#include "internal.h"
+#include "objective.cuh"
+#include "split.cuh"
+
+namespace lbk {
+namespace {
+
+constexpr int kSmallThreads     = 512;
+constexpr int kSmallWarps       = kSmallThreads / 32;
+constexpr int kSmallBins        = 256;
+constexpr int kFaultGridBarrier = 51;  // status word: a block did not reach the barrier
+
+struct SmallCand {
+  double gain;
+  int bin;  // of the feature
+  int pad;
+};
+
+template <typename T>
+struct SmallParams {
+  const T* X;
+  int64_t ldx;
+  int N, F, K, D, S, S_pad, seed;
+  int parts, part_shift;  // blocks per feature: a power of two
+  int64_t row_offset, dataset_rows;
+  // gradients: given (objective < 0), or made from the current prediction
+  const double* g;
+  const double* h;
+  int64_t ldg;
+  int objective;
+  const double* y;
+  double* pred;  // objective >= 0: [N][K], the tree's leaf values are added at the end
+  double lr;
+  double l1, l2, msg;
+  const uint8_t* feature_set;
+  TreeArrays tree;
+  double* hessian;
+  int32_t* leaf;  // may be null
+  // scratch
+  T* cuts;             // [F][S]
+  int32_t* counts;     // [F]
+  uint8_t* bins_t;     // [F][pitch]
+  int pitch;
+  int2* pairs;         // [N][K]
+  GPairI64* root_part; // [blocks][K]
+  GPairI64* hist[2];   // levels alternate: [F][nodes of the level][K][256]
+  SmallCand* cand;     // [nodes of the level][F]
+  GPairI64* cand_left; // [nodes of the level][F][K]
+  int max_slots;       // histograms in shared memory at a time
+  unsigned int* barrier;
+  unsigned int barrier_base;
+  int* status;
+  int32_t* info_host;  // mapped host memory [2]: number of bins, bins of the largest feature
+};
+
+// All blocks of the (cooperative) grid; bounded: after about a second it gives up, reports and returns false
+// in every thread of the block.
+__device__ inline bool GridBarrier(unsigned int* word, unsigned int target, int* status, int* s_ok)
+{
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(word, 1u);
+    int ok = 0;
+    for (unsigned spin = 0; spin < (1u << 21); ++spin) {
+      unsigned int v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(word) : "memory");
+      if (static_cast<int>(v - target) >= 0) {
+        ok = 1;
+        break;
+      }
+    }
+    if (!ok) ReportFault(status, kFaultGridBarrier);
+    *s_ok = ok;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+template <typename T>
+__device__ inline double2 SmallGradient(const SmallParams<T>& p, int row, int k)
+{
+  if (p.objective < 0) return make_double2(p.g[row * p.ldg + k], p.h[row * p.ldg + k]);
+  const double raw = p.pred[static_cast<int64_t>(row) * p.K + k], y = p.y[static_cast<int64_t>(row) * p.K + k];
+  return p.objective == LBK_SQUARED_ERROR ? GradientSquaredError(raw, y, p.lr) : GradientLogistic(raw, y, p.lr);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSmallThreads, 1)
+  k_tree_small(const SmallParams<T> p)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_ok, s_cnt[kSmallWarps + 1];
+  __shared__ double s_sum[2][2 * kSumThreads / 32];
+  __shared__ QuantParams s_qp;
+  __shared__ GPairI64 s_tot[2][kSmallWarps / 2];
+  __shared__ Cand s_best[2][2][kSmallWarps / 2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int N = p.N, F = p.F, K = p.K, D = p.D, S = p.S;
+  const int n_blocks = gridDim.x, block = blockIdx.x;
+  const int part     = block % p.parts;            // of the feature's rows (binning) and node pairs (levels)
+  const int f_first = block / p.parts, f_step = n_blocks / p.parts;
+  const int n_sums  = max(1, (1 << max(D - 1, 0)) * K);  // node sums of a level
+  // shared memory: histograms | node sums of two levels | candidate gains (several outputs) | row_ptr | winners |
+  // node of every row
+  int* s_hist         = reinterpret_cast<int*>(smem_raw);  // [slot][4][256]: g high, g low, h high, h low
+  double* s_gain      = reinterpret_cast<double*>(s_hist + p.max_slots * 4 * kSmallBins);
+  GPairI64* s_nodes   = reinterpret_cast<GPairI64*>(s_gain + (K > 1 ? p.max_slots * 2 * kSmallBins : 0));
+  GPairI64* s_next    = s_nodes + n_sums;
+  int* s_rp           = reinterpret_cast<int*>(s_next + n_sums);  // [F + 1]
+  int* s_wfeat        = s_rp + F + 1;                             // [nodes of a level], -1: no split / no node
+  int* s_wbin         = s_wfeat + (1 << max(D - 1, 0));
+  T* s_cuts           = reinterpret_cast<T*>(s_hist);  // (before the levels) [256]
+  int* s_wnew         = s_wbin + (1 << max(D - 1, 0));            // (the next s_wfeat while it is made)
+  uint16_t* s_pos     = reinterpret_cast<uint16_t*>(s_wnew + (1 << max(D - 1, 0)));
+  unsigned int target = p.barrier_base;
+
+  // ---- proposals and bins of the block's features
+  for (int f = f_first; f < F; f += f_step) {
+    T v = static_cast<T>(INFINITY);
+    if (tid < S) {
+      MinStd eng(static_cast<uint32_t>(p.seed));
+      eng.discard(static_cast<unsigned long long>(tid));
+      const long long row = eng.uniform_int(0, p.dataset_rows - 1) - p.row_offset;
+      v = row >= 0 && row < N ? p.X[row * p.ldx + f] : T(0);
+    }
+    for (int k = 2; k <= p.S_pad; k <<= 1) {
+      const bool up = (tid & k) == 0;
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        T o;
+        if (j >= 32) {
+          __syncthreads();
+          if (tid < p.S_pad) s_cuts[tid] = v;
+          __syncthreads();
+          o = tid < p.S_pad ? s_cuts[tid ^ j] : v;
+        } else {
+          o = __shfl_xor_sync(0xffffffffu, v, j);
+        }
+        const bool lower = (tid & j) == 0;
+        if (lower == up ? o < v : v < o) v = o;
+      }
+    }
+    __syncthreads();
+    if (tid < p.S_pad) s_cuts[tid] = v;
+    __syncthreads();
+    const bool keep  = tid < S && (tid == 0 || v != s_cuts[tid - 1]);
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) s_cnt[warp] = __popc(m);
+    __syncthreads();
+    int pos = __popc(m & ((1u << lane) - 1u)), count = 0;
+    for (int w = 0; w < kSmallWarps; ++w) {
+      if (w < warp) pos += s_cnt[w];
+      count += s_cnt[w];
+    }
+    if (keep) s_cuts[pos] = pos == count - 1 ? static_cast<T>(INFINITY) : v;
+    __syncthreads();
+    if (part == 0) {
+      for (int i = tid; i < count; i += kSmallThreads) p.cuts[static_cast<int64_t>(f) * S + i] = s_cuts[i];
+      if (tid == 0) p.counts[f] = count;
+    }
+    // bin = first proposal >= x; the part's share of the rows
+    for (int row0 = part * kSmallThreads + tid; row0 < N; row0 += 4 * p.parts * kSmallThreads) {
+      T x[4];
+      int b[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = row0 + e * p.parts * kSmallThreads;
+        x[e]          = row < N ? p.X[row * p.ldx + f] : T(0);
+      }
+      for (int len = count; len > 1;) {
+        const int half = len >> 1;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (s_cuts[b[e] + half - 1] < x[e]) b[e] += half;
+        len -= half;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = row0 + e * p.parts * kSmallThreads;
+        if (row < N) p.bins_t[static_cast<int64_t>(f) * p.pitch + row] = static_cast<uint8_t>(b[e] + (s_cuts[b[e]] < x[e] ? 1 : 0));
+      }
+    }
+    __syncthreads();
+  }
+
+  // ---- the quantiser's scale: |g| and |h| sums of all rows
+  {
+    const int64_t n = static_cast<int64_t>(N) * K;
+    const int n_chunks = static_cast<int>((n + kSumBlock - 1) / kSumBlock);
+    const int grp = tid / kSumThreads, t = tid % kSumThreads;
+    double* s_part = reinterpret_cast<double*>(s_hist);  // [2][n_chunks]
+    for (int c0 = 0; c0 < n_chunks; c0 += 2) {
+      double sg = 0.0, sh = 0.0;
+#pragma unroll 4
+      for (int j = 0; j < kSumItems; ++j) {
+        const int64_t idx = static_cast<int64_t>(c0 + grp) * kSumBlock + j * kSumThreads + t;
+        double vg = 0.0, vh = 0.0;
+        if (idx < n) {
+          const int row    = static_cast<int>(K == 1 ? idx : idx / K);
+          const double2 gh = SmallGradient(p, row, static_cast<int>(idx - static_cast<int64_t>(row) * K));
+          vg               = fabs(gh.x);
+          vh               = fabs(gh.y);
+        }
+        sg += vg;
+        sh += vh;
+      }
+      FoldAbsSums(sg, sh, t, s_sum[grp]);
+      __syncthreads();
+      if (t == 0 && c0 + grp < n_chunks) {
+        double tg, th;
+        JoinAbsSums(s_sum[grp], tg, th);
+        s_part[c0 + grp]            = tg;
+        s_part[n_chunks + c0 + grp] = th;
+      }
+      __syncthreads();
+    }
+    // at most 4096 partial sums are left: one more step of the same order (none if there is one)
+    double tg = n_chunks > 0 ? s_part[0] : 0.0, th = n_chunks > 0 ? s_part[n_chunks] : 0.0;
+    if (n_chunks > 1) {
+      double sg = 0.0, sh = 0.0;
+      if (grp == 0) {
+        for (int j = 0; j < kSumItems; ++j) {
+          const int i = j * kSumThreads + t;
+          sg += i < n_chunks ? s_part[i] : 0.0;
+          sh += i < n_chunks ? s_part[n_chunks + i] : 0.0;
+        }
+      }
+      FoldAbsSums(sg, sh, t, s_sum[grp]);
+      __syncthreads();
+      if (tid == 0) JoinAbsSums(s_sum[0], tg, th);
+    }
+    if (tid == 0) s_qp = MakeScale(tg, th);
+    __syncthreads();
+  }
+  const QuantParams qp = s_qp;
+
+  // ---- quantised pairs of a slice of the rows, and the slice's sums
+  {
+    const int per = (N + n_blocks - 1) / n_blocks;
+    const int r0 = min(N, block * per), r1 = min(N, r0 + per);
+    long long* s_root = reinterpret_cast<long long*>(s_hist);  // [K][2]
+    for (int i = tid; i < 2 * K; i += kSmallThreads) s_root[i] = 0;
+    __syncthreads();
+    for (int i0 = r0 * K + warp * 32; i0 < r1 * K; i0 += kSmallThreads) {
+      const int i   = i0 + lane;
+      const int row = i / K, k = i - row * K;
+      long long qg = 0, qh = 0;
+      if (i < r1 * K) {
+        const double2 gh = SmallGradient(p, row, k);
+        const int2 q     = QuantisePair(gh.x, gh.y, qp, HashCombine(static_cast<long long>(p.seed), p.row_offset + row, k));
+        p.pairs[i]       = q;
+        qg               = q.x;
+        qh               = q.y;
+      }
+      if (K == 1) {  // (one address for all lanes: one pair of atomics per warp)
+        for (int off = 16; off >= 1; off >>= 1) {
+          qg += __shfl_down_sync(0xffffffffu, qg, off);
+          qh += __shfl_down_sync(0xffffffffu, qh, off);
+        }
+      }
+      if (K == 1 ? lane == 0 : i < r1 * K) {
+        atomicAdd(reinterpret_cast<unsigned long long*>(s_root + 2 * k), static_cast<unsigned long long>(qg));
+        atomicAdd(reinterpret_cast<unsigned long long*>(s_root + 2 * k + 1), static_cast<unsigned long long>(qh));
+      }
+    }
+    __syncthreads();
+    for (int k = tid; k < K; k += kSmallThreads)
+      p.root_part[static_cast<int64_t>(block) * K + k] = GPairI64{s_root[2 * k], s_root[2 * k + 1]};
+  }
+  // cleared outputs; the nodes that split are written over below, after the barrier
+  for (int i = block * kSmallThreads + tid; i < p.tree.max_nodes; i += n_blocks * kSmallThreads) {
+    p.tree.feature[i]     = -1;
+    p.tree.split_value[i] = 0.0;
+    p.tree.gain[i]        = 0.0;
+    for (int k = 0; k < K; ++k) p.tree.node_sums[static_cast<int64_t>(i) * K + k] = GPairI64{0, 0};
+  }
+  target += n_blocks;
+  if (!GridBarrier(p.barrier, target, p.status, &s_ok)) return;
+
+  // ---- root: sums, positions; where each feature's bins begin in the order of all bins
+  for (int k = warp; k < K; k += kSmallWarps) {
+    GPairI64 s{0, 0};
+    for (int b = lane; b < n_blocks; b += 32) {
+      const GPairI64 v = LoadPairStreaming(p.root_part + static_cast<int64_t>(b) * K + k);
+      s.grad += v.grad;
+      s.hess += v.hess;
+    }
+    for (int off = 16; off >= 1; off >>= 1) {
+      s.grad += __shfl_xor_sync(0xffffffffu, s.grad, off);
+      s.hess += __shfl_xor_sync(0xffffffffu, s.hess, off);
+    }
+    if (lane == 0) {
+      s_nodes[k] = s;
+      if (block == 0) p.tree.node_sums[k] = s;
+    }
+  }
+  for (int row = tid; row < N; row += kSmallThreads) s_pos[row] = 0;
+  {
+    // one warp scans the counts
+    if (warp == kSmallWarps - 1) {
+      int carry = 0;
+      for (int base = 0; base < F; base += 32) {
+        const int f = base + lane;
+        int incl    = f < F ? __ldcg(p.counts + f) : 0;
+        for (int off = 1; off < 32; off <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, incl, off);
+          if (lane >= off) incl += v;
+        }
+        if (f < F) s_rp[f + 1] = carry + incl;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) s_rp[0] = 0;
+      if (lane == 0 && block == 0) *static_cast<volatile int32_t*>(p.info_host) = carry;
+    }
+    if (tid == 0) s_wfeat[0] = 0;
+  }
+  __syncthreads();
+
+  const double l1 = p.l1, reg = fmax(1e-5, p.l2), msg = p.msg;
+  for (int depth = 0; depth < D; ++depth) {
+    const int begin = (1 << depth) - 1, nodes = 1 << depth;
+    const bool derive = depth > 0, write_hist = depth < D - 1;
+    const int units = derive ? nodes / 2 : 1;
+    // (s_wfeat still holds the winners of the level above: unit u exists if node u there was split)
+    for (int f = f_first; f < F; f += f_step) {
+      const bool search = p.feature_set == nullptr || p.feature_set[f] != 0;
+      const int nb      = s_rp[f + 1] - s_rp[f];
+      const uint8_t* bins = p.bins_t + static_cast<int64_t>(f) * p.pitch;
+      GPairI64* hist_f      = p.hist[depth & 1] + static_cast<int64_t>(f) * nodes * K * kSmallBins;
+      const GPairI64* par_f = p.hist[(depth & 1) ^ 1] + static_cast<int64_t>(f) * (nodes / 2) * K * kSmallBins;
+      // the part's units, max_slots at a time: unit = part + (c0 + slot) * parts
+      const int my_units = units > part ? (units - part + p.parts - 1) / p.parts : 0;
+      for (int c0 = 0; c0 < my_units; c0 += p.max_slots) {
+        const int slots = min(p.max_slots, my_units - c0);
+        for (int k = 0; k < K; ++k) {
+          for (int i = tid; i < slots * kSmallBins; i += kSmallThreads) reinterpret_cast<int4*>(s_hist)[i] = make_int4(0, 0, 0, 0);
+          if (k == 0 && K > 1)
+            for (int i = tid; i < slots * 2 * kSmallBins; i += kSmallThreads) s_gain[i] = 0.0;
+          __syncthreads();
+          // rows of the built nodes, four per thread at a time so that their loads overlap
+          for (int row0 = tid; row0 < N; row0 += 4 * kSmallThreads) {
+            int slot[4];
+            int2 q[4];
+            int bin[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int row = row0 + e * kSmallThreads;
+              const int j   = row < N ? static_cast<int>(s_pos[row]) - begin : -1;
+              const int u   = derive ? j >> 1 : 0;
+              slot[e]       = (u >> p.part_shift) - c0;
+              if (j < 0 || (u & (p.parts - 1)) != part || slot[e] < 0 || slot[e] >= slots) slot[e] = -1;
+              if (slot[e] >= 0 && derive) {
+                const bool left = s_nodes[static_cast<int64_t>(2 * u) * K].hess < s_nodes[static_cast<int64_t>(2 * u + 1) * K].hess;
+                if (left != ((j & 1) == 0)) slot[e] = -1;
+              }
+              if (slot[e] >= 0) {
+                q[e]   = p.pairs[static_cast<int64_t>(row) * K + k];
+                bin[e] = bins[row];
+              }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if (slot[e] < 0) continue;
+              int* dst = s_hist + slot[e] * 4 * kSmallBins + bin[e];
+              atomicAdd(dst, q[e].x >> 16);
+              atomicAdd(dst + kSmallBins, q[e].x & 0xffff);
+              atomicAdd(dst + 2 * kSmallBins, q[e].y >> 16);
+              atomicAdd(dst + 3 * kSmallBins, q[e].y & 0xffff);
+            }
+          }
+          __syncthreads();
+          // scan, sibling, gains: a thread per bin, two units at a time
+          for (int i0 = 0; i0 < slots; i0 += 2) {
+            const int grp = tid / kSmallBins, b = tid % kSmallBins, gw = warp % (kSmallWarps / 2);
+            const int i   = i0 + grp;
+            const int u   = part + (c0 + i) * p.parts;
+            const bool here = i < slots && (!derive || s_wfeat[u] >= 0);  // node u of the level above was split
+            const bool left = here && derive && s_nodes[static_cast<int64_t>(2 * u) * K].hess < s_nodes[static_cast<int64_t>(2 * u + 1) * K].hess;
+            const int ja    = here && derive ? 2 * u + (left ? 0 : 1) : 0, jb = here && derive ? 2 * u + (left ? 1 : 0) : 0;
+            const bool eval_a = here && search && s_nodes[static_cast<int64_t>(ja) * K].hess > 0;
+            const bool eval_b = here && search && derive && s_nodes[static_cast<int64_t>(jb) * K].hess > 0;
+            const GPairI64 sum_a = s_nodes[static_cast<int64_t>(ja) * K + k], sum_b = s_nodes[static_cast<int64_t>(jb) * K + k];
+            const bool scanned = sum_a.hess > 0, in = here && b < nb;
+            const int64_t at_a = (static_cast<int64_t>(ja) * K + k) * kSmallBins + b, at_b = (static_cast<int64_t>(jb) * K + k) * kSmallBins + b;
+            const int* hs      = s_hist + i * 4 * kSmallBins;
+            double* gains      = s_gain + i * 2 * kSmallBins;
+            GPairI64 va[1] = {{0, 0}}, vb[1] = {{0, 0}};
+            double ga[1] = {0.0}, gb[1] = {0.0};
+            if (in) {
+              if (derive && scanned) vb[0] = LoadPairStreaming(par_f + (static_cast<int64_t>(u) * K + k) * kSmallBins + b);
+              va[0].grad = static_cast<long long>(hs[b]) * 65536 + static_cast<unsigned>(hs[kSmallBins + b]);
+              va[0].hess = static_cast<long long>(hs[2 * kSmallBins + b]) * 65536 + static_cast<unsigned>(hs[3 * kSmallBins + b]);
+            }
+            long long sg = va[0].grad, sh = va[0].hess;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+              const long long ng = __shfl_up_sync(0xffffffffu, sg, off);
+              const long long nh = __shfl_up_sync(0xffffffffu, sh, off);
+              if (lane >= off) {
+                sg += ng;
+                sh += nh;
+              }
+            }
+            if (lane == 31) s_tot[grp][gw] = GPairI64{sg, sh};
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < kSmallWarps / 2 - 1; ++w) {
+              if (w < gw) {
+                const GPairI64 t = s_tot[grp][w];
+                sg += t.grad;
+                sh += t.hess;
+              }
+            }
+            if (in) {
+              if (scanned && (sg > 0 || sh > 0)) va[0] = GPairI64{sg, sh};
+              vb[0] = scanned && derive ? GPairI64{vb[0].grad - va[0].grad, vb[0].hess - va[0].hess} : GPairI64{0, 0};
+              if (write_hist || K > 1) {
+                StorePair(hist_f + at_a, va[0]);
+                if (derive) StorePair(hist_f + at_b, vb[0]);
+              }
+            }
+            unsigned ok_a = eval_a && in ? 1u : 0u, ok_b = eval_b && in ? 1u : 0u;
+            if (K > 1 && in) {  // the gains so far are in shared memory, -1e300 = a side without hessian
+              ga[0] = gains[b];
+              gb[0] = gains[kSmallBins + b];
+              if (ga[0] < -1e299) ok_a = 0u;
+              if (gb[0] < -1e299) ok_b = 0u;
+            }
+            if (__any_sync(0xffffffffu, ok_a)) ok_a = AddGains<1>(va, ok_a, TermsOf(sum_a, qp, l1, reg), qp, l1, reg, msg, ga);
+            if (__any_sync(0xffffffffu, ok_b)) ok_b = AddGains<1>(vb, ok_b, TermsOf(sum_b, qp, l1, reg), qp, l1, reg, msg, gb);
+            if (k < K - 1) {
+              if (in) {
+                gains[b]              = ok_a ? ga[0] : -1e300;
+                gains[kSmallBins + b] = ok_b ? gb[0] : -1e300;
+              }
+              __syncthreads();  // s_tot is written again
+              continue;
+            }
+            // the best bin of either node: of the warp, then of the unit's eight warps
+            const double gain_a = ok_a && ga[0] > 0 ? ga[0] : 0.0, gain_b = ok_b && gb[0] > 0 ? gb[0] : 0.0;
+            const int bin_a = WarpBest(gain_a, s_rp[f] + b), bin_b = derive ? WarpBest(gain_b, s_rp[f] + b) : -1;
+            if (bin_a < 0 ? lane == 0 : bin_a == s_rp[f] + b) s_best[grp][0][gw] = Cand{gain_a, bin_a, b};
+            if (bin_b < 0 ? lane == 0 : bin_b == s_rp[f] + b) s_best[grp][1][gw] = Cand{gain_b, bin_b, b};
+            __syncthreads();
+            if (here) {
+#pragma unroll
+              for (int side = 0; side < 2; ++side) {
+                if (side == 1 && !derive) continue;
+                Cand best = s_best[grp][side][0];
+#pragma unroll
+                for (int w = 1; w < kSmallWarps / 2; ++w)
+                  if (Better(s_best[grp][side][w], best)) best = s_best[grp][side][w];
+                const int j      = side == 0 ? ja : jb;
+                const int64_t at = static_cast<int64_t>(j) * F + f;
+                if (b == 0) p.cand[at] = SmallCand{best.gain, best.bin < 0 ? -1 : best.feature, 0};  // (feature: the bin of the feature)
+                if (K == 1) {
+                  if (best.bin >= 0 && b == best.feature) StorePair(p.cand_left + at, side == 0 ? va[0] : vb[0]);
+                } else if (best.bin >= 0) {
+                  // (written by threads of this block, before the barrier)
+                  for (int kk = b; kk < K; kk += kSmallBins)
+                    StorePair(p.cand_left + at * K + kk,
+                              LoadPairStreaming(hist_f + (static_cast<int64_t>(j) * K + kk) * kSmallBins + best.feature));
+                }
+              }
+            }
+          }
+          __syncthreads();
+        }
+      }
+    }
+    target += n_blocks;
+    if (!GridBarrier(p.barrier, target, p.status, &s_ok)) return;
+
+    // ---- winners of the level: a warp per node picks, the next node's candidates already on their way
+    const int words = derive ? nodes : 1;
+    auto exists = [&](int j) { return j < words && (!derive || s_wfeat[j >> 1] >= 0) && s_nodes[static_cast<int64_t>(j) * K].hess > 0; };
+    auto first_cand = [&](int j) {
+      return exists(j) && lane < F ? __ldcg(reinterpret_cast<const int4*>(p.cand + static_cast<int64_t>(j) * F + lane)) : make_int4(0, 0, -1, 0);
+    };
+    int4 ahead = first_cand(warp);
+    for (int j = warp; j < words; j += kSmallWarps) {
+      const bool here = exists(j);
+      Cand best{0.0, -1, -1};
+      int4 raw = ahead;
+      ahead    = first_cand(j + kSmallWarps);
+      if (here) {
+        for (int f = lane; f < F; f += 32) {
+          if (f >= 32) raw = __ldcg(reinterpret_cast<const int4*>(p.cand + static_cast<int64_t>(j) * F + f));
+          if (raw.z < 0) continue;
+          const Cand c{__hiloint2double(raw.y, raw.x), s_rp[f] + raw.z, f};
+          if (Better(c, best)) best = c;
+        }
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) {
+          Cand o;
+          o.gain    = __shfl_xor_sync(0xffffffffu, best.gain, off);
+          o.bin     = __shfl_xor_sync(0xffffffffu, best.bin, off);
+          o.feature = __shfl_xor_sync(0xffffffffu, best.feature, off);
+          if (Better(o, best)) best = o;
+        }
+      }
+      if (lane == 0) {
+        const bool split = best.gain > 1e-5;
+        const int b      = split ? best.bin - s_rp[best.feature] : -1;
+        s_wbin[j]        = b;
+        s_wnew[j]        = split ? best.feature : -1;
+        if (split && block == 0) {
+          p.tree.feature[begin + j]     = best.feature;
+          p.tree.split_value[begin + j] = static_cast<double>(p.cuts[static_cast<int64_t>(best.feature) * S + b]);
+          p.tree.gain[begin + j]        = best.gain;
+        }
+      }
+    }
+    __syncthreads();
+    // ... and the sums of their children
+    for (int i = tid; i < words * K; i += kSmallThreads) {
+      const int j = i / K, k = i - j * K, wf = s_wnew[j];
+      GPairI64 ls{0, 0}, rs{0, 0};
+      if (wf >= 0) {
+        ls                = LoadPairStreaming(p.cand_left + (static_cast<int64_t>(j) * F + wf) * K + k);
+        const GPairI64 ns = s_nodes[i];
+        rs                = GPairI64{ns.grad - ls.grad, ns.hess - ls.hess};
+        if (block == 0) {
+          const int node = begin + j;
+          StorePair(p.tree.node_sums + static_cast<int64_t>(2 * node + 1) * K + k, ls);
+          StorePair(p.tree.node_sums + static_cast<int64_t>(2 * node + 2) * K + k, rs);
+        }
+      }
+      if (depth < D - 1) {
+        s_next[static_cast<int64_t>(2 * j) * K + k]     = ls;
+        s_next[static_cast<int64_t>(2 * j + 1) * K + k] = rs;
+      }
+    }
+    for (int j = tid; j < words; j += kSmallThreads) s_wfeat[j] = s_wnew[j];
+    __syncthreads();
+    // ---- rows move down; a row whose node did not split stays where it is
+    for (int row0 = tid; row0 < N; row0 += 4 * kSmallThreads) {
+      int bin[4], j[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = row0 + e * kSmallThreads;
+        j[e]          = row < N ? static_cast<int>(s_pos[row]) - begin : -1;
+        const int wf  = j[e] >= 0 ? s_wfeat[j[e]] : -1;
+        if (wf < 0) j[e] = -1;
+        else bin[e] = p.bins_t[static_cast<int64_t>(wf) * p.pitch + row];
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (j[e] >= 0)
+          s_pos[row0 + e * kSmallThreads] = static_cast<uint16_t>(2 * (begin + j[e]) + 1 + (bin[e] > s_wbin[j[e]] ? 1 : 0));
+    }
+    GPairI64* t = s_nodes;
+    s_nodes     = s_next;
+    s_next      = t;
+    __syncthreads();
+  }
+
+  // ---- leaf values and hessians, the node of every row, the prediction
+  target += n_blocks;
+  if (!GridBarrier(p.barrier, target, p.status, &s_ok)) return;
+  for (int i = block * kSmallThreads + tid; i < p.tree.max_nodes * K; i += n_blocks * kSmallThreads) {
+    const int node   = i / K;
+    const GPairF64 s = Dequantise(LoadPairStreaming(p.tree.node_sums + i), qp);
+    p.hessian[i]     = s.hess;
+    const bool here  = node == 0 || __ldcg(p.tree.feature + (node - 1) / 2) >= 0;
+    p.tree.leaf_value[i] = here ? CalculateLeafValue(s.grad, s.hess, l1, p.l2) : 0.0;
+  }
+  const int per = (N + n_blocks - 1) / n_blocks;
+  const int r0 = min(N, block * per), r1 = min(N, r0 + per);
+  if (p.leaf != nullptr)
+    for (int row = r0 + tid; row < r1; row += kSmallThreads) p.leaf[row] = s_pos[row];
+  if (p.objective >= 0) {
+    for (int i = r0 * K + tid; i < r1 * K; i += kSmallThreads) {
+      const int row = i / K, k = i - row * K;
+      const GPairF64 s = Dequantise(LoadPairStreaming(p.tree.node_sums + static_cast<int64_t>(s_pos[row]) * K + k), qp);
+      p.pred[i] += CalculateLeafValue(s.grad, s.hess, l1, p.l2);
+    }
+  }
+}
+
+}  // namespace
+
+// The shapes this form takes, and how it is cut: nothing is launched.
+struct SmallPlan {
+  int blocks, parts, max_slots;
+  size_t smem;
+};
+
+static bool PlanSmall(lbk_context* ctx, int64_t N, int F, int K, int D, int S, size_t elem, SmallPlan& plan)
+{
+  (void)elem;
+  // One-byte bins; 16-bit node ids; the canonical sum's second step in one piece.  The bound on rows x outputs
+  // is where the general path catches up: a block passes over all rows on every level.
+  if (S > kSmallBins || D < 1 || D > 12 || N < 1 || N * K > kSmallMaxElements || F > 4 * ctx->sm_count) return false;
+  const int64_t level = int64_t{1} << (D - 1);
+  if (level * K > 1536) return false;
+  const int64_t hist_bytes = (K > 1 ? level * 3 / 2 + 1 : level) * F * K * kSmallBins * 16;
+  if (hist_bytes > (int64_t{256} << 20)) return false;
+  // several blocks per feature: they share its node pairs on the deeper levels and its rows for the binning
+  plan.parts  = static_cast<int>(std::min<int64_t>(std::max(1, ctx->sm_count / F), std::max<int64_t>({level / 2, N / 2048, 1})));
+  while (plan.parts & (plan.parts - 1)) plan.parts &= plan.parts - 1;  // a power of two
+  plan.blocks = F <= ctx->sm_count ? F * plan.parts : ctx->sm_count;
+  const size_t fixed = 2 * sizeof(GPairI64) * std::max<int64_t>(1, level * K) + sizeof(int) * (F + 1 + 3 * level) + 2 * N + 64;
+  const size_t slot  = 4 * kSmallBins * sizeof(int) + (K > 1 ? 2 * kSmallBins * sizeof(double) : 0);
+  const size_t room  = static_cast<size_t>(ctx->max_smem_optin) - 4096;
+  if (fixed + slot > room) return false;
+  const int64_t units = std::max<int64_t>(1, level / 2);
+  plan.max_slots      = static_cast<int>(std::min<int64_t>((units + plan.parts - 1) / plan.parts, (room - fixed) / slot));
+  plan.max_slots      = std::max(plan.max_slots, 1);
+  plan.smem           = fixed + plan.max_slots * slot;
+  // (the partial sums, the proposals and the root sums share the histograms' place)
+  const size_t early = std::max({size_t{2} * ((N * K + kSumBlock - 1) / kSumBlock) * 8, kSmallBins * size_t{8}, size_t{16} * K});
+  if (early > plan.max_slots * slot) return false;
+  return true;
+}
+
+bool SmallTreeFits(lbk_context* ctx, int64_t N, int F, int K, int D, int S, size_t elem)
+{
+  SmallPlan plan;
+  return PlanSmall(ctx, N, F, K, D, S, elem, plan);
+}
+
+template <typename T>
+void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStream_t stream)
+{
+  SmallPlan plan;
+  LBK_EXPECT(PlanSmall(ctx, a.N, a.F, a.K, a.D, a.S, sizeof(T), plan), "shape outside the small form");
+  const int N = static_cast<int>(a.N), F = a.F, K = a.K, D = a.D;
+  const int64_t level = int64_t{1} << (D - 1);
+  SmallParams<T> p{};
+  p.X = a.X;
+  p.ldx = a.ldx;
+  p.N = N;
+  p.F = F;
+  p.K = K;
+  p.D = D;
+  p.S = a.S;
+  p.S_pad = 1;
+  while (p.S_pad < a.S) p.S_pad *= 2;
+  p.seed = a.seed;
+  p.parts = plan.parts;
+  while ((2 << p.part_shift) <= p.parts) ++p.part_shift;
+  p.row_offset = a.row_offset;
+  p.dataset_rows = a.dataset_rows;
+  p.g = a.g;
+  p.h = a.h;
+  p.ldg = a.ldg;
+  p.objective = a.objective;
+  p.y = a.y;
+  p.pred = a.pred;
+  p.lr = a.lr;
+  p.l1 = a.sp.l1;
+  p.l2 = a.sp.l2;
+  p.msg = a.sp.min_split_gain;
+  p.feature_set = a.sp.feature_set;
+  p.tree = a.tree;
+  p.hessian = a.hessian;
+  p.leaf = a.leaf;
+  p.cuts = s.alloc<T>(static_cast<size_t>(F) * a.S);
+  p.counts = s.alloc<int32_t>(F);
+  p.pitch = (N + 31) / 32 * 32;
+  p.bins_t = s.alloc<uint8_t>(static_cast<size_t>(F) * p.pitch);
+  p.pairs = s.alloc<int2>(static_cast<size_t>(N) * K);
+  p.root_part = s.alloc<GPairI64>(static_cast<size_t>(plan.blocks) * K);
+  // level d's histograms are written for d < D - 1 (every level with several outputs: the left sums are read
+  // back from them)
+  const int64_t top = K > 1 ? level : std::max<int64_t>(level / 2, 1), below = std::max<int64_t>(top / 2, 1);
+  const int last    = K > 1 ? D - 1 : D - 2;  // the last level written
+  p.hist[last & 1]       = s.alloc<GPairI64>(static_cast<size_t>(F) * top * K * kSmallBins);
+  p.hist[(last & 1) ^ 1] = s.alloc<GPairI64>(static_cast<size_t>(F) * below * K * kSmallBins);
+  p.cand      = s.alloc<SmallCand>(static_cast<size_t>(level) * F);
+  p.cand_left = s.alloc<GPairI64>(static_cast<size_t>(level) * F * K);
+  p.max_slots = plan.max_slots;
+  p.status    = ctx->d_status;
+  p.info_host = ctx->h_info;
+  const unsigned phases = static_cast<unsigned>(D) + 2u;
+  if (ctx->grid_barrier == nullptr) {
+    LBK_CUDA(cudaMalloc(&ctx->grid_barrier, sizeof(unsigned int)));
+    LBK_CUDA(cudaMemsetAsync(ctx->grid_barrier, 0, sizeof(unsigned int), stream));
+    LBK_CUDA(cudaStreamSynchronize(stream));
+    ctx->grid_barrier_base = 0;
+  }
+  p.barrier      = ctx->grid_barrier;
+  p.barrier_base = ctx->grid_barrier_base;
+  auto fn = k_tree_small<T>;
+  if (!ctx->small_tree_ready[sizeof(T) == 8]) {
+    LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 2048));
+    ctx->small_tree_ready[sizeof(T) == 8] = true;
+  }
+  void* args[] = {&p};
+  LBK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(fn), dim3(plan.blocks), dim3(kSmallThreads), args,
+                                       plan.smem, stream));
+  ctx->grid_barrier_base += phases * static_cast<unsigned>(plan.blocks);
+}
+
+template void SmallTree<float>(lbk_context*, Scratch&, const SmallTreeArgs<float>&, cudaStream_t);
+template void SmallTree<double>(lbk_context*, Scratch&, const SmallTreeArgs<double>&, cudaStream_t);
+
+}  // namespace lbk

@@ -14,28 +14,14 @@
 //     comes from lower thread ids, so equal gains resolve to the largest (bin mod 512) and then
 //     the smallest bin.  That total order is applied here, independent of the reduction shape.
 // Compiled with -fmad=false.
-#include "device_utils.cuh"
 #include "internal.h"
+#include "split.cuh"
 
 namespace lbk {
 namespace {
 
-struct Cand {
-  double gain;
-  int bin;
-  int feature;
-};
-__device__ inline bool Better(const Cand& a, const Cand& b)
-{
-  if (a.gain > b.gain) return true;
-  if (a.gain < b.gain) return false;
-  if (a.bin < 0 || b.bin < 0) return b.bin < 0 && a.bin >= 0;
-  const int ta = a.bin & 511, tb = b.bin & 511;
-  if (ta != tb) return ta > tb;
-  return a.bin < b.bin;
-}
-
-constexpr int kSplitWarps = 8;  // most warps of a block
+constexpr int kSplitThreads = 256;
+constexpr int kSplitWarps   = kSplitThreads / 32;
 
 // What a rank knows about its best split of a node when the features are divided among the ranks:
 // the candidate and the sums left of it; K pairs follow the header.
@@ -91,65 +77,32 @@ struct SliceBest {
   GPairI64 left;
 };
 
-// What the gains of one output need of a node: its sums as whole numbers in float64 and its own gain.
-struct NodeTerms {
-  double g, h, gain;
-};
-
-// (double)v for |v| < 2^51, exact: adding 1.5 * 2^52 to the bit pattern of the integer makes a float64 whose
-// value is that constant plus v.  Two instructions of full rate instead of a conversion of a sixteenth of it.
-__device__ inline double WholeToDouble(long long v)
-{
-  return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
-}
-
-__device__ inline NodeTerms TermsOf(GPairI64 sum, const QuantParams& qp, double l1, double reg)
-{
-  NodeTerms t;
-  t.g    = WholeToDouble(sum.grad);
-  t.h    = WholeToDouble(sum.hess);
-  t.gain = LeafGain(GPairF64{t.g * qp.inv_g, t.h * qp.inv_h}, l1, reg);
-  return t;
-}
-
-// The gain of one output at one bin, added to `gain`; false if a side has no positive hessian (sums are
-// below 2^51, so their differences are exact in float64).
-__device__ inline bool AddGain(GPairI64 left, const NodeTerms& n, const QuantParams& qp, double l1, double reg, double msg,
-                               double& gain)
-{
-  const double lg = WholeToDouble(left.grad), lh = WholeToDouble(left.hess);
-  const double rg = n.g - lg, rh = n.h - lh;
-  if (lh <= 0.0 || rh <= 0.0) return false;
-  const double gl = LeafGain(GPairF64{lg * qp.inv_g, lh * qp.inv_h}, l1, reg);
-  const double gr = LeafGain(GPairF64{rg * qp.inv_g, rh * qp.inv_h}, l1, reg);
-  gain += (0.5 * (gl + gr - n.gain)) - msg;
-  return true;
-}
-
 // grid = (units, slices).  A unit is a pair of siblings of which one was built (derive) or a single
-// built node; a warp takes one feature at a time: it scans the built histogram, derives the sibling's
-// from the parent's, writes both for the level below (not on the last level: nobody reads them there)
-// and evaluates both nodes' gains while the sums are in registers, so that a level's histograms cross
-// the memory once.  The buffer of the nodes built on the next level is zeroed on the way.  With several
-// slices every block leaves its best candidates in `slice_best`, and the block of the unit that arrives
-// last (a counter per node, zeroed once per tree) picks the winners and writes the tree.  Better() is a
-// total order, so the winners do not depend on how the features were cut.
+// built node; a block takes one feature at a time, a thread one bin: it scans the built histogram, derives
+// the sibling's from the parent's, writes both for the level below (not on the last level: nobody reads
+// them there) and evaluates both nodes' gains while the sums are in registers, so that a level's histograms
+// cross the memory once.  The buffer of the nodes built on the next level is zeroed on the way.  With
+// several slices every block leaves its best candidates in `slice_best`, and the block of the unit that
+// arrives last (a counter per node, zeroed once per tree) picks the winners and writes the tree.  Better()
+// is a total order, so the winners do not depend on how the features were cut.
 //
 // What bounds it: on wide levels the issue slots (two float64 divisions per bin, output and node, and a
 // 64-bit scan), on the upper levels the latency of one chain load - scan - division - reduction - claim.
-// kRun bins per lane and turn: four with one output (few warps, long chains), two with several, where
-// the registers that this saves keep three blocks on an SM.
-template <typename T, bool kManyOutputs, bool kDerive, int kRun>
-__global__ void __launch_bounds__(kSplitWarps * 32, kManyOutputs ? 3 : 2)
+// A thread per bin and not a warp per feature (four bins per lane): a warp alone on its scheduler gets one
+// instruction in about five clocks, and a feature's 2600 of them were 9 us whatever the level held; and 60
+// registers instead of 128 keep 32 warps on an SM where the level is wide.
+template <typename T, bool kManyOutputs, bool kDerive>
+__global__ void __launch_bounds__(kSplitThreads, 4)
   k_scan_split(const __grid_constant__ ScanSplitParams<T> p)
 {
-  extern __shared__ __align__(16) unsigned char smem_raw[];  // several outputs: terms [2][K], then [warps][K] carries
+  extern __shared__ __align__(16) unsigned char smem_raw[];  // several outputs: terms [2][K]; then carries [K]
+  __shared__ GPairI64 s_tot[2][kSplitWarps];
   __shared__ SliceBest s_c[2][kSplitWarps];
   __shared__ SliceBest s_best[2];
   __shared__ bool s_last;
   const ScanSplitLevel& lv = p.lv;
   const int K = lv.K, unit = blockIdx.x, slices = gridDim.y;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int node0 = lv.node_begin + (kDerive ? 2 * unit : unit);
   GPairI64* node_sums = p.tree.node_sums;
   // everything the block needs first, asked for at once
@@ -157,7 +110,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32, kManyOutputs ? 3 : 2)
   const GPairI64 sum_0 = LoadPair(node_sums + static_cast<int64_t>(node0) * K);
   const GPairI64 sum_1 = kDerive ? LoadPair(node_sums + static_cast<int64_t>(node0 + 1) * K) : GPairI64{0, 0};
   const QuantParams qp = *p.qp;
-  int f  = lv.f_begin + blockIdx.y * n_warps + warp;
+  int f  = lv.f_begin + blockIdx.y;
   int fb = f < lv.f_end ? p.row_ptr[f] : 0, fe = f < lv.f_end ? p.row_ptr[f + 1] : 0;
   if (parent_feature < 0) return;  // the parent did not split: no such node
   // _a: the built node, _b: its sibling (SmallerChildIsLeft)
@@ -175,10 +128,10 @@ __global__ void __launch_bounds__(kSplitWarps * 32, kManyOutputs ? 3 : 2)
   GPairI64* next_b    = lv.next_built + static_cast<int64_t>(jb) * K * Bs;
   const GPairI64* par = lv.parent_hist + static_cast<int64_t>((node0 - 1) / 2 - lv.parent_begin) * K * Bs;
   NodeTerms* s_terms  = reinterpret_cast<NodeTerms*>(smem_raw);
-  GPairI64* s_carry   = reinterpret_cast<GPairI64*>(smem_raw + sizeof(NodeTerms) * 2 * ((K + 1) / 2 * 2)) + warp * K;
+  GPairI64* s_carry   = reinterpret_cast<GPairI64*>(smem_raw + (kManyOutputs ? sizeof(NodeTerms) * 2 * ((K + 1) / 2 * 2) : 0));
   NodeTerms ta{}, tb{};
   if (kManyOutputs) {
-    for (int i = tid; i < 2 * K; i += blockDim.x) {
+    for (int i = tid; i < 2 * K; i += kSplitThreads) {
       const int k = i >> 1, node = (i & 1) ? node_b : node_a;
       if (kDerive || !(i & 1)) s_terms[i] = TermsOf(LoadPair(node_sums + static_cast<int64_t>(node) * K + k), qp, l1, reg);
     }
@@ -190,122 +143,92 @@ __global__ void __launch_bounds__(kSplitWarps * 32, kManyOutputs ? 3 : 2)
 
   Cand best_a{0.0, -1, -1}, best_b{0.0, -1, -1};
   GPairI64 left_a{0, 0}, left_b{0, 0};
+  int turn = 0;
   while (f < lv.f_end) {
     const bool search = p.sp.feature_set == nullptr || p.sp.feature_set[f] != 0;
-    GPairI64 carry{0, 0};
-    if (kManyOutputs) {
-      __syncwarp();
-      for (int k = lane; k < K; k += 32) s_carry[k] = GPairI64{0, 0};
-      __syncwarp();
-    }
-    for (int base = fb; base < fe; base += 32 * kRun) {
-      double gain_a[kRun], gain_b[kRun];
-      GPairI64 va[kRun], vb[kRun];
-      unsigned in = 0;
-#pragma unroll
-      for (int i = 0; i < kRun; ++i) {
-        gain_a[i] = gain_b[i] = 0.0;
-        if (base + i * 32 + lane < fe) in |= 1u << i;
-      }
-      unsigned ok_a = eval_a && search ? in : 0u, ok_b = eval_b && search ? in : 0u;
+    for (int base = fb; base < fe; base += kSplitThreads) {
+      const bool in = base + tid < fe;
+      double gain_a[1] = {0.0}, gain_b[1] = {0.0};
+      GPairI64 va[1], vb[1] = {{0, 0}};
+      unsigned ok_a = eval_a && search && in ? 1u : 0u, ok_b = eval_b && search && in ? 1u : 0u;
       for (int k = 0; k < (kManyOutputs ? K : 1); ++k) {
-        const int64_t ko = (kManyOutputs ? static_cast<int64_t>(k) * Bs : 0) + base + lane;
+        const int64_t at = (kManyOutputs ? static_cast<int64_t>(k) * Bs : 0) + base + tid;
         if (kManyOutputs) {
           ta = s_terms[2 * k];
           if (kDerive) tb = s_terms[2 * k + 1];
         }
         const bool scanned = ta.h > 0.0;  // else the raw values stay and no sibling is derived
-        long long sg[kRun], sh[kRun];
-#pragma unroll
-        for (int i = 0; i < kRun; ++i) {
-          va[i] = in & (1u << i) ? LoadPair(src + ko + i * 32) : GPairI64{0, 0};
-          if (kDerive) vb[i] = (in & (1u << i)) && scanned ? LoadPair(par + ko + i * 32) : GPairI64{0, 0};
-          sg[i] = va[i].grad;
-          sh[i] = va[i].hess;
-        }
+        va[0] = in ? LoadPair(src + at) : GPairI64{0, 0};
+        if (kDerive) vb[0] = in && scanned ? LoadPair(par + at) : GPairI64{0, 0};
+        long long sg = va[0].grad, sh = va[0].hess;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-          for (int i = 0; i < kRun; ++i) {
-            const long long ng = __shfl_up_sync(0xffffffffu, sg[i], off);
-            const long long nh = __shfl_up_sync(0xffffffffu, sh[i], off);
-            if (lane >= off) {
-              sg[i] += ng;
-              sh[i] += nh;
-            }
+          const long long ng = __shfl_up_sync(0xffffffffu, sg, off);
+          const long long nh = __shfl_up_sync(0xffffffffu, sh, off);
+          if (lane >= off) {
+            sg += ng;
+            sh += nh;
           }
         }
-        GPairI64 run = kManyOutputs ? s_carry[k] : carry;
+        // the warps before this one (two buffers: one barrier per turn is enough)
+        const int buf = turn++ & 1;
+        if (lane == 31) s_tot[buf][warp] = GPairI64{sg, sh};
+        __syncthreads();
+        GPairI64 before{0, 0};
+        if (base > fb) before = s_carry[kManyOutputs ? k : 0];
 #pragma unroll
-        for (int i = 0; i < kRun; ++i) {
-          const long long tg = __shfl_sync(0xffffffffu, sg[i], 31), th = __shfl_sync(0xffffffffu, sh[i], 31);
-          sg[i] += run.grad;
-          sh[i] += run.hess;
-          run.grad += tg;
-          run.hess += th;
+        for (int w = 0; w < kSplitWarps - 1; ++w) {
+          if (w < warp) {
+            const GPairI64 t = s_tot[buf][w];
+            before.grad += t.grad;
+            before.hess += t.hess;
+          }
         }
-        if (kManyOutputs) {
-          __syncwarp();
-          if (lane == 0) s_carry[k] = run;
-        } else {
-          carry = run;
+        sg += before.grad;
+        sh += before.hess;
+        if (fe - base > kSplitThreads) {  // more bins than threads: the next turn starts from this one's total
+          __syncthreads();
+          if (tid == kSplitThreads - 1) s_carry[kManyOutputs ? k : 0] = GPairI64{sg, sh};
         }
-#pragma unroll
-        for (int i = 0; i < kRun; ++i) {
-          if (!(in & (1u << i))) continue;
-          if (scanned && (sg[i] > 0 || sh[i] > 0)) va[i] = GPairI64{sg[i], sh[i]};
-          if (kDerive) vb[i] = scanned ? GPairI64{vb[i].grad - va[i].grad, vb[i].hess - va[i].hess} : GPairI64{0, 0};
+        if (in) {
+          if (scanned && (sg > 0 || sh > 0)) va[0] = GPairI64{sg, sh};
+          if (kDerive) vb[0] = scanned ? GPairI64{vb[0].grad - va[0].grad, vb[0].hess - va[0].hess} : GPairI64{0, 0};
           if (lv.write_hist) {
-            StorePair(dst_a + ko + i * 32, va[i]);
-            if (kDerive) StorePair(dst_b + ko + i * 32, vb[i]);
+            StorePair(dst_a + at, va[0]);
+            if (kDerive) StorePair(dst_b + at, vb[0]);
           }
           if (lv.next_built != nullptr) {
-            StorePair(next_a + ko + i * 32, GPairI64{0, 0});
-            if (kDerive) StorePair(next_b + ko + i * 32, GPairI64{0, 0});
+            StorePair(next_a + at, GPairI64{0, 0});
+            if (kDerive) StorePair(next_b + at, GPairI64{0, 0});
           }
-          if (ok_a & (1u << i))
-            if (!AddGain(va[i], ta, qp, l1, reg, msg, gain_a[i])) ok_a &= ~(1u << i);
-          if (kDerive && (ok_b & (1u << i)))
-            if (!AddGain(vb[i], tb, qp, l1, reg, msg, gain_b[i])) ok_b &= ~(1u << i);
+        }
+        if (__any_sync(0xffffffffu, ok_a)) ok_a = AddGains<1>(va, ok_a, ta, qp, l1, reg, msg, gain_a);
+        if (kDerive && __any_sync(0xffffffffu, ok_b)) ok_b = AddGains<1>(vb, ok_b, tb, qp, l1, reg, msg, gain_b);
+      }
+      if (ok_a && gain_a[0] > 0) {
+        const Cand c{gain_a[0], base + tid, f};
+        if (Better(c, best_a)) {
+          best_a = c;
+          if (!kManyOutputs) left_a = va[0];
         }
       }
-#pragma unroll
-      for (int i = 0; i < kRun; ++i) {
-        const int b = base + i * 32 + lane;
-        if ((ok_a & (1u << i)) && gain_a[i] > 0) {
-          const Cand c{gain_a[i], b, f};
-          if (Better(c, best_a)) {
-            best_a = c;
-            if (!kManyOutputs) left_a = va[i];
-          }
-        }
-        if (kDerive && (ok_b & (1u << i)) && gain_b[i] > 0) {
-          const Cand c{gain_b[i], b, f};
-          if (Better(c, best_b)) {
-            best_b = c;
-            if (!kManyOutputs) left_b = vb[i];
-          }
+      if (kDerive && ok_b && gain_b[0] > 0) {
+        const Cand c{gain_b[0], base + tid, f};
+        if (Better(c, best_b)) {
+          best_b = c;
+          if (!kManyOutputs) left_b = vb[0];
         }
       }
     }
-    f += slices * n_warps;
-    if (f < lv.f_end) {
-      fb = p.row_ptr[f];
-      fe = p.row_ptr[f + 1];
-    }
+    f += slices;
+    if (f >= lv.f_end) break;
+    fb = p.row_ptr[f];
+    fe = p.row_ptr[f + 1];
   }
   // the warp's best: the lane that holds it writes it down
   auto warp_best = [&](const Cand& mine, const GPairI64& left, SliceBest* out) {
-    Cand best = mine;
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-      Cand o;
-      o.gain    = __shfl_xor_sync(0xffffffffu, best.gain, off);
-      o.bin     = __shfl_xor_sync(0xffffffffu, best.bin, off);
-      o.feature = __shfl_xor_sync(0xffffffffu, best.feature, off);
-      if (Better(o, best)) best = o;
-    }
-    if (best.bin < 0 ? lane == 0 : mine.bin == best.bin) *out = SliceBest{best, left};
+    const int bin = WarpBest(mine.bin >= 0 ? mine.gain : 0.0, mine.bin);
+    if (bin < 0 ? lane == 0 : mine.bin == bin) *out = SliceBest{bin < 0 ? Cand{0.0, -1, -1} : mine, left};
   };
   auto block_best = [&]() {
     warp_best(best_a, left_a, &s_c[0][warp]);
@@ -313,7 +236,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32, kManyOutputs ? 3 : 2)
     __syncthreads();
     if (tid < (kDerive ? 2 : 1)) {
       int at = 0;
-      for (int w = 1; w < n_warps; ++w)
+      for (int w = 1; w < kSplitWarps; ++w)
         if (Better(s_c[tid][w].c, s_c[tid][at].c)) at = w;
       s_best[tid] = s_c[tid][at];
     }
@@ -334,7 +257,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32, kManyOutputs ? 3 : 2)
     if (!s_last) return;
     __threadfence();
     best_a = best_b = Cand{0.0, -1, -1};
-    for (int i = tid; i < slices; i += blockDim.x) {
+    for (int i = tid; i < slices; i += kSplitThreads) {
       const volatile SliceBest* a = mine + i * 2;
       const Cand ca{a[0].c.gain, a[0].c.bin, a[0].c.feature};
       if (Better(ca, best_a)) {
@@ -363,10 +286,10 @@ __global__ void __launch_bounds__(kSplitWarps * 32, kManyOutputs ? 3 : 2)
     GPairI64* rec_sums = reinterpret_cast<GPairI64*>(rec + sizeof(SplitRecordHeader));
     if (nb.bin < 0) {
       if (rec != nullptr)
-        for (int k = tid; k < K; k += blockDim.x) StorePair(rec_sums + k, GPairI64{0, 0});
+        for (int k = tid; k < K; k += kSplitThreads) StorePair(rec_sums + k, GPairI64{0, 0});
       continue;
     }
-    for (int k = warp; k < K; k += n_warps) {
+    for (int k = warp; k < K; k += kSplitWarps) {
       const int64_t ko = static_cast<int64_t>(k) * Bs;
       GPairI64 ls;
       if (!kManyOutputs) {
@@ -459,19 +382,12 @@ void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, co
   const int n_features = lv.f_end - lv.f_begin;
   const int units      = lv.derive ? lv.n_nodes / 2 : lv.n_nodes;
   if (units <= 0) return;
-  // with several outputs a block keeps K terms of two nodes and every warp K running prefixes in shared
-  // memory: fewer warps for very many outputs
-  int warps = kSplitWarps;
-  auto need = [&](int w) {
-    return lv.K > 1 ? sizeof(NodeTerms) * 2 * ((lv.K + 1) / 2 * 2) + static_cast<size_t>(w) * lv.K * sizeof(GPairI64) : 0;
-  };
-  while (warps > 1 && need(warps) > 40 * 1024) warps /= 2;
-  const size_t smem = need(warps);
-  // one feature per warp until there are about eight blocks per SM, then several
-  int slices     = (n_features + warps - 1) / warps;
-  const int most = (8 * ctx->sm_count + units - 1) / units;
+  // with several outputs a block keeps K terms of two nodes and K running prefixes in shared memory
+  const size_t smem = (lv.K > 1 ? sizeof(NodeTerms) * 2 * ((lv.K + 1) / 2 * 2) : 0) + lv.K * sizeof(GPairI64);
+  // one feature per block until there are about sixteen blocks per SM, then several
+  int slices     = n_features > 0 ? n_features : 1;
+  const int most = (16 * ctx->sm_count + units - 1) / units;
   if (slices > most) slices = most;
-  if (slices < 1) slices = 1;
   ScanSplitParams<T> p;
   p.lv         = lv;
   p.row_ptr    = row_ptr;
@@ -491,11 +407,11 @@ void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, co
     LBK_CUDA(cudaMemsetAsync(mine, 0, rb * lv.n_nodes, stream));
     p.records = mine;
   }
-  auto fn = lv.K > 1 ? (lv.derive ? k_scan_split<T, true, true, 2> : k_scan_split<T, true, false, 2>)
-                     : (lv.derive ? k_scan_split<T, false, true, 4> : k_scan_split<T, false, false, 4>);
+  auto fn = lv.K > 1 ? (lv.derive ? k_scan_split<T, true, true> : k_scan_split<T, true, false>)
+                     : (lv.derive ? k_scan_split<T, false, true> : k_scan_split<T, false, false>);
   if (smem > 48 * 1024)
     LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  fn<<<dim3(units, slices), warps * 32, smem, stream>>>(p);
+  fn<<<dim3(units, slices), kSplitThreads, smem, stream>>>(p);
   LBK_LAUNCH_CHECK();
   if (exchange_records) {
     // every rank has searched its own features: the candidates of all ranks meet on every rank

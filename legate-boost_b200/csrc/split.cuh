@@ -1,0 +1,138 @@
+// Split candidates, their total order and the gain of a bin (reference behaviour: see split.cu).
+#pragma once
+#include "device_utils.cuh"
+
+namespace lbk {
+
+struct Cand {
+  double gain;
+  int bin;
+  int feature;
+};
+__device__ inline bool Better(const Cand& a, const Cand& b)
+{
+  if (a.gain > b.gain) return true;
+  if (a.gain < b.gain) return false;
+  if (a.bin < 0 || b.bin < 0) return b.bin < 0 && a.bin >= 0;
+  const int ta = a.bin & 511, tb = b.bin & 511;
+  if (ta != tb) return ta > tb;
+  return a.bin < b.bin;
+}
+
+// The largest of a warp's values (all not negative), in every lane: their bit patterns are ordered as the values.
+__device__ inline double WarpMax(double v)
+{
+  const unsigned hi = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(__double2hiint(v)));
+  const unsigned lo = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(__double2hiint(v)) == hi ? static_cast<unsigned>(__double2loint(v)) : 0u);
+  return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
+}
+
+// The bin of the warp's best candidate (a bin and a gain per lane, gain 0 = none), or -1.
+__device__ inline int WarpBest(double gain, int bin)
+{
+  const double top = WarpMax(gain);
+  if (top == 0.0) return -1;
+  const unsigned holders = __ballot_sync(0xffffffffu, gain == top);
+  Cand best{top, __shfl_sync(0xffffffffu, bin, __ffs(holders) - 1), 0};
+  for (unsigned rest = holders & (holders - 1u); rest != 0u; rest &= rest - 1u) {  // equal gains: the order of the bins decides
+    const Cand o{top, __shfl_sync(0xffffffffu, bin, __ffs(rest) - 1), 0};
+    if (Better(o, best)) best = o;
+  }
+  return best.bin;
+}
+
+// What the gains of one output need of a node: its sums as whole numbers in float64 and its own gain.
+struct NodeTerms {
+  double g, h, gain;
+};
+
+// (double)v for |v| < 2^51, exact: adding 1.5 * 2^52 to the bit pattern of the integer makes a float64 whose
+// value is that constant plus v.  Two instructions of full rate instead of a conversion of a sixteenth of it.
+__device__ inline double WholeToDouble(long long v)
+{
+  return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
+}
+
+__device__ inline NodeTerms TermsOf(GPairI64 sum, const QuantParams& qp, double l1, double reg)
+{
+  NodeTerms t;
+  t.g    = WholeToDouble(sum.grad);
+  t.h    = WholeToDouble(sum.hess);
+  t.gain = LeafGain(GPairF64{t.g * qp.inv_g, t.h * qp.inv_h}, l1, reg);
+  return t;
+}
+
+// a / b, correctly rounded, without a branch: the reciprocal approximation refined by Newton steps, and two
+// corrections of the quotient by its exact remainder (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990): a quotient within one unit in the last place
+// plus remainder times the correctly rounded reciprocal rounds to the exact quotient).  For the operands that
+// DivisionIsPlain accepts nothing on the way leaves the normal range.
+//
+// Why not the operator: its test for operands out of range is a branch per division, which keeps the compiler
+// from running the 16 divisions of a lane side by side, and one of them is a chain of a dozen dependent
+// float64 instructions.  A level of a 500 x 10 tree spent 8 of its 15 us there.
+__device__ inline double DividePlain(double a, double b)
+{
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(r) : "d"(b));
+  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
+  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
+  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
+  double q = a * r;
+  q        = __fma_rn(__fma_rn(-b, q, a), r, q);
+  return __fma_rn(__fma_rn(-b, q, a), r, q);
+}
+// b in [2^-500, 2^500), a zero or in the same range (both not negative)
+__device__ inline bool DivisionIsPlain(double a, double b)
+{
+  const unsigned ea = static_cast<unsigned>(__double2hiint(a)) - (523u << 20), eb = static_cast<unsigned>(__double2hiint(b)) - (523u << 20);
+  return eb < (1000u << 20) && (a == 0.0 || ea < (1000u << 20));
+}
+
+// LeafGain's numerator
+__device__ inline double LeafNumerator(double g, double l1)
+{
+  const double z = g > l1 ? g - l1 : g < -l1 ? g + l1 : 0.0;
+  return z * z;
+}
+
+// The gains of one output at kRun bins of a lane, added to gain[] where `ok` has the bin's bit; bits are cleared
+// where a side has no positive hessian (sums are below 2^51, so their differences are exact in float64).  All
+// lanes of a warp call it.
+template <int kRun>
+__device__ inline unsigned AddGains(const GPairI64 (&left)[kRun], unsigned ok, const NodeTerms& n, const QuantParams& qp,
+                                    double l1, double reg, double msg, double (&gain)[kRun])
+{
+  double na[kRun], da[kRun], nb[kRun], db[kRun];
+  bool plain = true;
+#pragma unroll
+  for (int i = 0; i < kRun; ++i) {
+    const double lg = WholeToDouble(left[i].grad), lh = WholeToDouble(left[i].hess);
+    const double rg = n.g - lg, rh = n.h - lh;
+    if (lh <= 0.0 || rh <= 0.0) ok &= ~(1u << i);
+    na[i] = LeafNumerator(lg * qp.inv_g, l1);
+    nb[i] = LeafNumerator(rg * qp.inv_g, l1);
+    da[i] = lh * qp.inv_h + reg;
+    db[i] = rh * qp.inv_h + reg;
+    plain = plain && (!(ok & (1u << i)) || (DivisionIsPlain(na[i], da[i]) && DivisionIsPlain(nb[i], db[i])));
+  }
+  if (__all_sync(0xffffffffu, plain)) {
+#pragma unroll
+    for (int i = 0; i < kRun; ++i) {
+      na[i] = DividePlain(na[i], da[i]);
+      nb[i] = DividePlain(nb[i], db[i]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < kRun; ++i) {
+      if (!(ok & (1u << i))) continue;
+      na[i] = na[i] / da[i];
+      nb[i] = nb[i] / db[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kRun; ++i) gain[i] += (0.5 * (na[i] + nb[i] - n.gain)) - msg;
+  return ok;
+}
+
+}  // namespace lbk

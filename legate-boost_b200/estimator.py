@@ -9,6 +9,7 @@ Objectives: squared error (objectives.py:119-147) and multi-class / binary log l
 models, update, sklearn plumbing) is outside the tree-building hot path and is not provided.
 Arrays are torch CUDA tensors; under ``torch.distributed`` each rank holds a block of rows.
 """
+import ctypes as C
 from copy import deepcopy
 from typing import List, Optional
 
@@ -16,15 +17,30 @@ import numpy as np
 import torch
 
 from . import library as L
-from .tree import _ARRAYS, Sketch, Tree, TreeTable, _row_layout
+from .tree import _ARRAYS, Sketch, Tree, TreeTable, _row_layout, _tensor_key
+
+
+def _several_ranks() -> bool:
+    import torch.distributed as dist
+
+    return dist.is_available() and dist.is_initialized() and dist.get_world_size() > 1
 
 
 def _all_sum(t: torch.Tensor) -> torch.Tensor:
     import torch.distributed as dist
 
-    if dist.is_available() and dist.is_initialized() and dist.get_world_size() > 1:
+    if _several_ranks():
         dist.all_reduce(t)
     return t
+
+
+def _copy_of(base: Tree) -> Tree:
+    """deepcopy of a base model, whose attributes are plain values as a rule."""
+    if all(type(v) in (int, float, str, bool, type(None)) for v in base.__dict__.values()):
+        tree = Tree.__new__(Tree)
+        tree.__dict__.update(base.__dict__)
+        return tree
+    return deepcopy(base)
 
 
 class _SquaredError:
@@ -39,7 +55,10 @@ class _SquaredError:
     def init(self, y, average):
         if not average:
             return torch.zeros(y.shape[1], dtype=torch.float64, device=y.device)
-        s = _all_sum(torch.cat([y.sum(dim=0), torch.tensor([float(y.shape[0])], dtype=torch.float64, device=y.device)]))
+        count = torch.full((1,), float(y.shape[0]), dtype=torch.float64, device=y.device)
+        if not _several_ranks():
+            return y.sum(dim=0) / count
+        s = _all_sum(torch.cat([y.sum(dim=0), count]))
         return s[:-1] / s[-1]
 
     def metric(self, y, pred):
@@ -155,6 +174,10 @@ class _LBBase:
         self.train_metric_: List[float] = []
         train_pred = self.model_init_.repeat(X.shape[0], 1)
         layout = _row_layout(X.shape[0])  # this rank's block of rows: the same for every tree
+        if self._rounds_in_library():
+            self._fit_rounds(X, y, train_pred, layout)
+            self._train_pred = train_pred
+            return self
         sketches = {}
         for i in range(self.n_estimators):
             g, h = self._weighted_gradient(y, train_pred)
@@ -172,6 +195,82 @@ class _LBBase:
                 print("[%d] train: %.6f" % (i, m))
         self._train_pred = train_pred
         return self
+
+    def _rounds_in_library(self) -> bool:
+        """Whether a round is one `lbk_boost_round` call: plain trees, an objective the library knows, nothing
+        to report per round."""
+        return (not self.verbose and self.n_estimators > 0 and type(self._obj) in (_SquaredError, _LogLoss)
+                and all(type(b) is Tree and not callable(b.feature_fraction) and b.max_depth >= 0 for b in self.base_models))
+
+    def _fit_rounds(self, X, y, train_pred, layout):
+        """The rounds of fit(), one library call each, queued without waiting for the device.  What the host
+        decides - seeds and feature samples, in the order in which Tree.fit draws them - is drawn before
+        the first round; the trees of up to 64 rounds share one allocation per array."""
+        N, F = X.shape
+        K = train_pred.shape[1]
+        dev, rs = X.device, self.random_state_
+        bases = [self.base_models[i % len(self.base_models)] for i in range(self.n_estimators)]
+        seeds, masks = [], np.ones((self.n_estimators, F), dtype=np.uint8)
+        for i, b in enumerate(bases):
+            seeds.append(int(rs.randint(0, 2**31)))
+            mask = b._sample_features(rs, F)
+            if mask is not None:
+                masks[i] = mask
+        masks = None if masks.all() else torch.from_numpy(masks).to(dev)
+        if X.stride(1) != 1 and N > 0:
+            X = X.contiguous()
+        y = y.contiguous()
+        ctx = L.init_distributed(dev.index)
+        lib, handle, stream = ctx.lib, ctx.handle, torch.cuda.current_stream(dev).cuda_stream
+        r = L.BoostRoundArgs()
+        a = r.tree
+        a.X, a.x_dtype, a.ldx = X.data_ptr(), L.LBK_F32 if X.dtype == torch.float32 else L.LBK_F64, X.stride(0) if N > 0 else F
+        a.row_offset, a.dataset_rows = layout
+        a.n_local_rows, a.n_features, a.n_outputs = N, F, K
+        a.stream = stream
+        r.objective, r.y, r.pred, r.learning_rate = self._obj.code, y.data_ptr(), train_pred.data_ptr(), float(self.learning_rate)
+        ref, sketches, models = C.byref(r), {}, []
+        n_bases = len(self.base_models)
+        at = 0
+        while at < self.n_estimators:
+            run = list(range(at, min(at + 64, self.n_estimators)))
+            at += len(run)
+            trees = {}
+            for b in range(min(n_bases, len(run))):
+                mine = [i for i in run if i % n_bases == (run[0] + b) % n_bases]
+                M, n = 2 ** (bases[mine[0]].max_depth + 1) - 1, len(mine)
+                f64 = dict(dtype=torch.float64, device=dev)
+                arrays = {
+                    "leaf_value": torch.empty((n, M, K), **f64), "feature": torch.empty((n, M), dtype=torch.int32, device=dev),
+                    "split_value": torch.empty((n, M), **f64), "gain": torch.empty((n, M), **f64),
+                    "hessian": torch.empty((n, M, K), **f64),
+                }
+                parts = {name: t.unbind(0) for name, t in arrays.items()}
+                for q, i in enumerate(mine):
+                    trees[i] = {name: p[q] for name, p in parts.items()}
+                    trees[i]["at"] = [t.data_ptr() + q * t.stride(0) * t.element_size() for t in arrays.values()]
+            for i in run:
+                base, mine = bases[i], trees[i]
+                where = mine.pop("at")
+                a.leaf_value, a.feature, a.split_value, a.gain, a.hessian = where
+                a.feature_set = None if masks is None else masks.data_ptr() + i * F
+                a.max_depth, a.max_nodes = base.max_depth, mine["feature"].shape[0]
+                a.split_samples, a.seed = base.split_samples, seeds[i]
+                a.l1_regularization, a.l2_regularization = base.l1_regularization, base.l2_regularization
+                a.min_split_gain = base.min_split_gain
+                sketch = None
+                if self.fixed_sketch:
+                    sketch = sketches.setdefault(i % n_bases, Sketch())
+                    a.sketch_mode = sketch.mode_for(X, base.split_samples, ctx)
+                    a.sketch = sketch.buffer.data_ptr()
+                ctx.check(lib.lbk_boost_round(handle, ref))
+                if sketch is not None:
+                    sketch.key = (_tensor_key(X), base.split_samples)
+                tree = _copy_of(base)
+                tree.__dict__.update(mine, random_state=rs, row_layout=layout, sketch=None, _fit_rows=None)
+                models.append(tree)
+        ctx.check(lib.lbk_synchronize(handle, stream))
+        self.models_ = models
 
     def predict_raw(self, X):
         return self._predict(X, L.RAW)

@@ -325,6 +325,14 @@ class Tree(BaseModel):
     def right_child(self, id):
         return id * 2 + 2
 
+    def _sample_features(self, random_state, n_features: int):
+        """The feature mask of one tree from ``feature_fraction`` (a number), or None for all features."""
+        if self.feature_fraction >= 1.0:
+            return None
+        mask = np.zeros(n_features, dtype=bool)
+        mask[random_state.choice(n_features, max(1, int(n_features * self.feature_fraction)), False)] = True
+        return mask
+
     def fit(self, X: torch.Tensor, g: torch.Tensor, h: torch.Tensor) -> "Tree":
         # order of draws from the shared RandomState: the seed first, then the feature sample
         # (reference: tree.py:125 and :149-155)
@@ -335,11 +343,9 @@ class Tree(BaseModel):
             feature_set = torch.as_tensor(feature_set)
             if tuple(feature_set.shape) != (X.shape[1],) or feature_set.dtype != torch.bool:
                 raise ValueError("feature_fraction must return a boolean array of shape (n_features,)")
-        elif self.feature_fraction < 1.0:
-            mask = np.zeros(X.shape[1], dtype=bool)
-            n_sampled = max(1, int(X.shape[1] * self.feature_fraction))
-            mask[self.random_state.choice(X.shape[1], n_sampled, False)] = True
-            feature_set = torch.from_numpy(mask)
+        else:
+            mask = self._sample_features(self.random_state, X.shape[1])
+            feature_set = None if mask is None else torch.from_numpy(mask)
         # A driver that fits many trees on the same row blocks can set `row_layout` = (row_offset,
         # dataset_rows) once; otherwise every fit asks the other ranks for their row counts.
         row_offset, dataset_rows = getattr(self, "row_layout", None) or (None, None)
@@ -442,6 +448,11 @@ class Tree(BaseModel):
         state = dict(self.__dict__)
         state.pop("_fit_rows", None)
         state.pop("sketch", None)
+        for name in ("leaf_value", "feature", "split_value", "gain", "hessian"):
+            # (the trees of one fit share their storage: a copy takes its own part only)
+            t = state.get(name)
+            if torch.is_tensor(t) and t.untyped_storage().nbytes() > t.numel() * t.element_size():
+                state[name] = t.clone()
         return state
 
     def to_onnx(self) -> Any:

@@ -806,3 +806,33 @@ def test_weighted_gradient_kernels_match_the_array_formulas(lb):
         assert np.allclose(g.cpu().numpy(), want_g * 0.3, rtol=1e-12, atol=1e-15)
         assert np.allclose(h.cpu().numpy(), np.maximum(p * (1 - p), 1e-8), rtol=1e-12)
         assert h.min().item() == 1e-8
+
+
+@pytest.mark.parametrize("N,F,D,S,classes,dtype", [
+    (1, 1, 1, 16, 0, np.float32), (500, 10, 4, 256, 0, np.float32),        # one launch per tree, gradients inside
+    (16384, 3, 7, 64, 0, np.float64), (4000, 200, 3, 100, 2, np.float32),  # the most rows; more features than SMs
+    (1500, 20, 5, 32, 5, np.float32),                                      # ... several outputs: gradients outside
+    (16385, 9, 6, 256, 0, np.float32), (20000, 33, 9, 256, 2, np.float32), # the general path
+    (3000, 40, 5, 400, 3, np.float64),                                     # ... two-byte bins
+])
+def test_rounds_in_the_library_match_rounds_from_python(lb, N, F, D, S, classes, dtype):
+    """fit() queues whole rounds (`lbk_boost_round`); the same rounds driven tree by tree (gradient, Tree.fit,
+    prediction of the leaf record) give the same bits: every step does the same arithmetic."""
+    rs = np.random.RandomState(N % 101 + F)
+    X = rs.normal(size=(N, F)).astype(dtype)
+    X[:, 0] = np.round(X[:, 0] * 2) / 2
+    X = dev(X)
+    y = dev(rs.normal(size=N)) + 2 * X[:, 0].double() if classes == 0 else dev(rs.randint(0, classes, size=N))
+    kw = dict(n_estimators=5, random_state=3, base_models=(
+        lb.Tree(max_depth=D, split_samples=S), lb.Tree(max_depth=max(D - 1, 0), split_samples=S, feature_fraction=0.6)))
+    kind = lb.LBClassifier if classes else lb.LBRegressor
+    a, b = kind(**kw), kind(**kw)
+    a._rounds_in_library = lambda: False
+    a.fit(X, y)
+    b.fit(X, y)
+    assert len(a) == len(b) == 5
+    for i in range(5):
+        for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
+            assert torch.equal(getattr(a[i], name), getattr(b[i], name)), (i, name)
+    assert torch.equal(a._train_pred, b._train_pred)
+    assert torch.equal(a.predict_raw(X[:50]), b.predict_raw(X[:50]))
