@@ -187,6 +187,7 @@ typedef struct lbk_boost_round_args {
   const double* y;        /* as in lbk_gradient */
   double* pred;           /* [n_local_rows, n_outputs], in and out */
   double learning_rate;
+  void* zeroed;           /* optional: a device word that is zero and that this call alone uses (saves clearing one) */
 } lbk_boost_round_args;
 
 int lbk_boost_round(lbk_context* ctx, const lbk_boost_round_args* args);

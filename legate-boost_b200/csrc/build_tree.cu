@@ -180,6 +180,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   const int64_t N = a.n_local_rows;
   const int M     = a.max_nodes;
   Scratch s(ctx, stream);
+  HostWords words(ctx);
 
   const T* X      = static_cast<const T*>(a.X);
   const double* g = a.g;
@@ -261,6 +262,12 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     int32_t* leaf = a.out_leaf != nullptr && !a.host_buffers ? a.out_leaf
                     : a.out_leaf != nullptr || (round != nullptr && !fused) ? s.alloc<int32_t>(static_cast<size_t>(N)) : nullptr;
     t.leaf        = leaf;
+    t.barrier     = round != nullptr ? static_cast<unsigned int*>(round->zeroed) : nullptr;
+    if (t.barrier == nullptr) {
+      t.barrier = s.alloc<unsigned int>(1);
+      LBK_CUDA(cudaMemsetAsync(t.barrier, 0, sizeof(unsigned int), stream));
+    }
+    t.info_host = a.out_total_bins != nullptr ? words.get() : nullptr;
     SmallTree<T>(ctx, s, t, stream);
     if (round != nullptr && !fused) {
       k_add_leaf_values<<<static_cast<unsigned>((N * K + 255) / 256), 256, 0, stream>>>(leaf_value, leaf, N, K, round->pred);
@@ -274,7 +281,8 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     }
     if (round != nullptr) return;
     CheckDeviceStatus(ctx, stream);
-    if (a.out_total_bins) *a.out_total_bins = ctx->h_info[0];
+    words.settled();
+    if (a.out_total_bins) *a.out_total_bins = words.get()[0];
     return;
   }
   if (round != nullptr) {
@@ -323,10 +331,10 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   constexpr int kTickets = 256;
   HistScratch hist_scratch;
   HistScratchNeeds(ctx, F, K, S <= 256 ? 1 : 2, S, N, hist_scratch);
-  size_t words = 0;
+  size_t zero_bytes = 0;
   auto reserve = [&](size_t bytes) {
-    const size_t at = words;
-    words += (bytes + 15) / 16 * 16;
+    const size_t at = zero_bytes;
+    zero_bytes += (bytes + 15) / 16 * 16;
     return at;
   };
   const size_t o_sums    = reserve(keep_sums ? 0 : sizeof(GPairI64) * M * K);
@@ -335,7 +343,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   const size_t o_ticket  = reserve(sizeof(unsigned int) * kTickets);
   const size_t o_arrive  = reserve(sizeof(unsigned int) * hist_scratch.n_arrive);
   const size_t o_abs     = reserve(2 * sizeof(int));
-  unsigned char* zeroed  = static_cast<unsigned char*>(s.alloc_bytes(words));
+  unsigned char* zeroed  = static_cast<unsigned char*>(s.alloc_bytes(zero_bytes));
   tree.node_sums = keep_sums ? reinterpret_cast<GPairI64*>(a.trace_node_sums) : reinterpret_cast<GPairI64*>(zeroed + o_sums);
   unsigned int* split_arrived  = reinterpret_cast<unsigned int*>(zeroed + o_arrived);
   unsigned long long* cursor   = reinterpret_cast<unsigned long long*>(zeroed + o_cursor);
@@ -387,12 +395,12 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     pa.root_begin   = seg_a;
     pa.root_end     = seg_a + max_level_nodes;
     pa.zero[0]      = zeroed;
-    pa.zero_n16[0]  = static_cast<int64_t>(words / 16);
+    pa.zero_n16[0]  = static_cast<int64_t>(zero_bytes / 16);
     pa.zero[1]      = tree.node_sums;
     pa.zero_n16[1]  = keep_sums ? static_cast<int64_t>(M) * K : 0;
     pa.zero[2]      = cache;
     pa.zero_n16[2]  = root_zeroed ? static_cast<int64_t>(K) * bins_bound : 0;
-    Prologue<T>(ctx, s, pa, row_ptr, info, ctx->h_info, sums, qp, stream);
+    Prologue<T>(ctx, s, pa, row_ptr, info, wait_for_bins || a.out_total_bins ? words.get() : nullptr, sums, qp, stream);
   }
   ProposalInfo pi{static_cast<int>(std::min<int64_t>(bins_bound, INT32_MAX)), S};
   if (sketch_reuse) {
@@ -400,8 +408,9 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     pi.max_bins_per_feature = head.max_bins_per_feature;
   } else if (wait_for_bins) {
     LBK_CUDA(cudaStreamSynchronize(stream));
-    pi.total_bins           = ctx->h_info[0];
-    pi.max_bins_per_feature = ctx->h_info[1];
+    pi.total_bins           = words.get()[0];
+    pi.max_bins_per_feature = words.get()[1];
+    words.settled();
     LBK_EXPECT(pi.total_bins >= F, "every feature must have at least one proposal");
   }
   const int B = pi.total_bins;  // (an upper bound unless wait_for_bins)
@@ -641,7 +650,8 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   if (a.host_buffers) copy_tree_back();
   if (round != nullptr) return;
   CheckDeviceStatus(ctx, stream);  // synchronises, as the reference's task does (:1356)
-  if (a.out_total_bins) *a.out_total_bins = sketch_reuse ? head.total_bins : ctx->h_info[0];
+  words.settled();
+  if (a.out_total_bins) *a.out_total_bins = sketch_reuse ? head.total_bins : words.get()[0];
 }
 
 void CheckTreeArgs(const lbk_build_tree_args& a)

@@ -145,6 +145,31 @@ void Scratch::free_one(void* p)
     }
 }
 
+int32_t* HostWords::get()
+{
+  if (words_ != nullptr) return words_;
+  std::lock_guard<std::mutex> lock(ctx_->words_mutex);
+  if (ctx_->words_free.empty()) {
+    constexpr int kPairs = 512, kApart = 16;  // (a pair has a 64-byte line of its own)
+    ctx_->words_free.reserve(ctx_->words_free.capacity() + kPairs);
+    ctx_->words_pages.reserve(ctx_->words_pages.size() + 1);
+    void* page = nullptr;
+    LBK_CUDA(cudaHostAlloc(&page, sizeof(int32_t) * kApart * kPairs, cudaHostAllocMapped | cudaHostAllocPortable));
+    ctx_->words_pages.push_back(page);
+    for (int i = kPairs - 1; i >= 0; --i) ctx_->words_free.push_back(static_cast<int32_t*>(page) + i * kApart);
+  }
+  words_ = ctx_->words_free.back();
+  ctx_->words_free.pop_back();
+  return words_;
+}
+
+HostWords::~HostWords()
+{
+  if (words_ == nullptr || !settled_) return;
+  std::lock_guard<std::mutex> lock(ctx_->words_mutex);
+  ctx_->words_free.push_back(words_);  // (has room: every pair was in the list once)
+}
+
 void AllReduce(lbk_context* ctx, void* buf, size_t count, lbk_dtype dtype, lbk_redop op, cudaStream_t stream)
 {
   if (ctx->n_ranks <= 1 || count == 0) return;
@@ -192,10 +217,6 @@ void ThrowReportedFault(lbk_context* ctx)
   const int h        = *word;
   if (h == 0) return;
   *word = 0;
-  if (ctx->grid_barrier != nullptr) {  // the count may not be where the host believes it is
-    cudaFree(ctx->grid_barrier);
-    ctx->grid_barrier = nullptr;
-  }
   throw Error(LBK_ERR_DEVICE, "a kernel reported fault code " + std::to_string(h));
 }
 
@@ -253,10 +274,9 @@ int lbk_context_create(int device, lbk_context** out)
       // the status word lives in pinned host memory: kernels store a fault code straight into it, and
       // the host reads it after a synchronisation without a copy
       void* word = nullptr;
-      LBK_CUDA(cudaHostAlloc(&word, 4 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+      LBK_CUDA(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
       c->d_status  = static_cast<int*>(word);
       *c->d_status = 0;
-      c->h_info    = static_cast<int32_t*>(word) + 2;
     } catch (...) {
       if (c->pool) cudaMemPoolDestroy(c->pool);
       if (c->d_status) cudaFreeHost(c->d_status);
@@ -274,7 +294,7 @@ void lbk_context_destroy(lbk_context* ctx)
   cudaDeviceSynchronize();
   lbk::DestroyExchange(ctx);
   if (ctx->owns_nccl && ctx->nccl_comm && nccl().CommDestroy) nccl().CommDestroy(ctx->nccl_comm);
-  if (ctx->grid_barrier) cudaFree(ctx->grid_barrier);
+  for (void* page : ctx->words_pages) cudaFreeHost(page);
   if (ctx->d_status) cudaFreeHost(ctx->d_status);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   for (auto& ev : ctx->prof_events) {

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <functional>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <utility>
@@ -75,11 +76,10 @@ struct lbk_context {
   std::string err;
   // status word in mapped host memory: 0 = ok, otherwise a kernel stored a fault code
   int* d_status = nullptr;
-  int32_t* h_info = nullptr;  // mapped host memory [2], beside it: number of bins, bins of the largest feature
-  // grid barrier of the one-launch trees: a word that only counts up, and where it stands
-  unsigned int* grid_barrier     = nullptr;
-  unsigned int grid_barrier_base = 0;
-  bool small_tree_ready[2]       = {false, false};
+  // pairs of words in mapped host memory that a call borrows for what its kernels tell the host (HostWords)
+  std::mutex words_mutex;
+  std::vector<void*> words_pages;
+  std::vector<int32_t*> words_free;
   // communicator
   int rank = 0, n_ranks = 1;
   void* nccl_comm     = nullptr;
@@ -118,6 +118,24 @@ class Scratch {
   std::vector<void*> ptrs_;
   char* slab_       = nullptr;
   size_t slab_used_ = 0;
+};
+
+// Two words of mapped host memory for one call: number of bins, bins of the largest feature.  Calls in progress
+// on several streams or threads must not see each other's; a pair goes back only once the call has waited for its
+// kernels (`settled`) - after an error a kernel may still write it, and it stays out of use.
+class HostWords {
+ public:
+  explicit HostWords(lbk_context* ctx) : ctx_(ctx) {}
+  ~HostWords();
+  HostWords(const HostWords&)            = delete;
+  HostWords& operator=(const HostWords&) = delete;
+  int32_t* get();  // borrowed on first use
+  void settled() { settled_ = true; }
+
+ private:
+  lbk_context* ctx_;
+  int32_t* words_ = nullptr;
+  bool settled_   = false;
 };
 
 // In-place all-reduce over the context's communicator; no-op for a single rank.
@@ -363,6 +381,8 @@ struct SmallTreeArgs {
   TreeArrays tree;   // node_sums [max_nodes][K]; split_bin is not used
   double* hessian;
   int32_t* leaf;     // may be null
+  unsigned int* barrier;  // device word, zero; this tree's alone
+  int32_t* info_host;     // mapped host word for the number of bins, or null
 };
 bool SmallTreeFits(lbk_context* ctx, int64_t N, int F, int K, int D, int S, size_t elem);
 template <typename T>

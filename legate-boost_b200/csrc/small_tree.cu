@@ -71,10 +71,9 @@ struct SmallParams {
   SmallCand* cand;     // [nodes of the level][F]
   GPairI64* cand_left; // [nodes of the level][F][K]
   int max_slots;       // histograms in shared memory at a time
-  unsigned int* barrier;
-  unsigned int barrier_base;
+  unsigned int* barrier;  // zero at the start
   int* status;
-  int32_t* info_host;  // mapped host memory [2]: number of bins, bins of the largest feature
+  int32_t* info_host;     // mapped host word for the number of bins, or null
 };
 
 // All blocks of the (cooperative) grid; bounded: after about a second it gives up, reports and returns false
@@ -137,7 +136,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   T* s_cuts           = reinterpret_cast<T*>(s_hist);  // (before the levels) [256]
   int* s_wnew         = s_wbin + (1 << max(D - 1, 0));            // (the next s_wfeat while it is made)
   uint16_t* s_pos     = reinterpret_cast<uint16_t*>(s_wnew + (1 << max(D - 1, 0)));
-  unsigned int target = p.barrier_base;
+  unsigned int target = 0;
 
   // ---- proposals and bins of the block's features
   for (int f = f_first; f < F; f += f_step) {
@@ -334,7 +333,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
         carry += __shfl_sync(0xffffffffu, incl, 31);
       }
       if (lane == 0) s_rp[0] = 0;
-      if (lane == 0 && block == 0) *static_cast<volatile int32_t*>(p.info_host) = carry;
+      if (lane == 0 && block == 0 && p.info_host != nullptr) *static_cast<volatile int32_t*>(p.info_host) = carry;
     }
     if (tid == 0) s_wfeat[0] = 0;
   }
@@ -696,25 +695,13 @@ void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStre
   p.cand_left = s.alloc<GPairI64>(static_cast<size_t>(level) * F * K);
   p.max_slots = plan.max_slots;
   p.status    = ctx->d_status;
-  p.info_host = ctx->h_info;
-  const unsigned phases = static_cast<unsigned>(D) + 2u;
-  if (ctx->grid_barrier == nullptr) {
-    LBK_CUDA(cudaMalloc(&ctx->grid_barrier, sizeof(unsigned int)));
-    LBK_CUDA(cudaMemsetAsync(ctx->grid_barrier, 0, sizeof(unsigned int), stream));
-    LBK_CUDA(cudaStreamSynchronize(stream));
-    ctx->grid_barrier_base = 0;
-  }
-  p.barrier      = ctx->grid_barrier;
-  p.barrier_base = ctx->grid_barrier_base;
+  p.info_host = a.info_host;
+  p.barrier   = a.barrier;
   auto fn = k_tree_small<T>;
-  if (!ctx->small_tree_ready[sizeof(T) == 8]) {
-    LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 2048));
-    ctx->small_tree_ready[sizeof(T) == 8] = true;
-  }
+  LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 2048));
   void* args[] = {&p};
   LBK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(fn), dim3(plan.blocks), dim3(kSmallThreads), args,
                                        plan.smem, stream));
-  ctx->grid_barrier_base += phases * static_cast<unsigned>(plan.blocks);
 }
 
 template void SmallTree<float>(lbk_context*, Scratch&, const SmallTreeArgs<float>&, cudaStream_t);

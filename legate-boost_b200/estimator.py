@@ -235,6 +235,7 @@ class _LBBase:
         while at < self.n_estimators:
             run = list(range(at, min(at + 64, self.n_estimators)))
             at += len(run)
+            zeroed = torch.zeros((len(run),), dtype=torch.int32, device=dev)
             trees = {}
             for b in range(min(n_bases, len(run))):
                 mine = [i for i in run if i % n_bases == (run[0] + b) % n_bases]
@@ -249,11 +250,12 @@ class _LBBase:
                 for q, i in enumerate(mine):
                     trees[i] = {name: p[q] for name, p in parts.items()}
                     trees[i]["at"] = [t.data_ptr() + q * t.stride(0) * t.element_size() for t in arrays.values()]
-            for i in run:
+            for j, i in enumerate(run):
                 base, mine = bases[i], trees[i]
                 where = mine.pop("at")
                 a.leaf_value, a.feature, a.split_value, a.gain, a.hessian = where
                 a.feature_set = None if masks is None else masks.data_ptr() + i * F
+                r.zeroed = zeroed.data_ptr() + 4 * j
                 a.max_depth, a.max_nodes = base.max_depth, mine["feature"].shape[0]
                 a.split_samples, a.seed = base.split_samples, seeds[i]
                 a.l1_regularization, a.l2_regularization = base.l1_regularization, base.l2_regularization
@@ -292,6 +294,10 @@ class _LBBase:
             assert all(isinstance(m, Tree) for m in self.models_)
             table = TreeTable(list(map(_ARRAYS, self.models_)))
             self._table = table if table.reusable else None
+        if table.n_outputs != init.shape[0]:  # (trees of the user's own with one column for all outputs)
+            raw = init.repeat(X.shape[0], 1)
+            raw += table.predict(X, table.n_outputs)
+            return raw if transform == L.RAW else self._probabilities(raw)
         return table.predict(X, init.shape[0], init=init, transform=transform)
 
     def __getstate__(self):

@@ -57,7 +57,7 @@ class BuildTreeArgs(C.Structure):
 class BoostRoundArgs(C.Structure):
     _fields_ = [
         ("tree", BuildTreeArgs), ("objective", C.c_int32), ("y", C.c_void_p), ("pred", C.c_void_p),
-        ("learning_rate", C.c_double),
+        ("learning_rate", C.c_double), ("zeroed", C.c_void_p),
     ]
 
 

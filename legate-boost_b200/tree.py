@@ -168,16 +168,22 @@ class TreeTable:
             self.max_nodes = max(self.max_nodes, M)
             if i == 0:
                 self.n_outputs = lv.shape[1] if lv.dim() == 2 else 1
+            if lv.numel() != M * self.n_outputs or sv.numel() != M:
+                raise ValueError("the trees of an ensemble must have arrays of one shape per node")
         # converted copies would not follow later changes of the originals: such a table is not kept
         self.reusable = all(map(is_, keep, self.source))
+        self.addresses = list(map(torch.Tensor.data_ptr, self.source))
         self.keep, self.total_nodes, self.n_trees = keep, total, len(arrays)
         self.table = torch.from_numpy(rows).to(device)
         self.device = device
 
     def matches(self, models) -> bool:
-        """Whether these models still hold the very tensors the table was made from."""
-        return (self.reusable and len(models) == self.n_trees
-                and all(map(is_, chain.from_iterable(map(_ARRAYS, models)), self.source)))
+        """Whether these models still hold the very tensors the table was made from, and these still lie
+        where they did (``t.data = ...`` or ``t.set_(...)`` moves a tensor)."""
+        if not self.reusable or len(models) != self.n_trees:
+            return False
+        arrays = list(chain.from_iterable(map(_ARRAYS, models)))
+        return all(map(is_, arrays, self.source)) and list(map(torch.Tensor.data_ptr, arrays)) == self.addresses
 
     def predict(self, X, n_outputs, init=None, transform=L.RAW, ctx=None):
         """pred (N, columns) float64: ``init`` (n_outputs values, or None) plus the trees' sums, transformed."""

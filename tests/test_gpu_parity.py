@@ -836,3 +836,69 @@ def test_rounds_in_the_library_match_rounds_from_python(lb, N, F, D, S, classes,
             assert torch.equal(getattr(a[i], name), getattr(b[i], name)), (i, name)
     assert torch.equal(a._train_pred, b._train_pred)
     assert torch.equal(a.predict_raw(X[:50]), b.predict_raw(X[:50]))
+
+
+def test_an_ensemble_predicts_what_its_trees_hold_now(lb):
+    """The device table of the trees' addresses follows every way to change a tree."""
+    from legateboost_b200.tree import predict_arrays
+
+    rs = np.random.RandomState(0)
+    X = dev(rs.normal(size=(300, 5)))
+    m = lb.LBRegressor(n_estimators=3, base_models=(lb.Tree(max_depth=3),), random_state=0).fit(X, dev(rs.normal(size=300)))
+
+    def check():
+        want = m.model_init_ + predict_arrays(X, [tree_tuple(t) for t in m])
+        assert torch.equal(m.predict_raw(X), want)
+
+    check()
+    m[0].leaf_value.mul_(2.0)
+    check()
+    m[1].leaf_value = m[1].leaf_value * 3.0
+    check()
+    m[2].leaf_value.data = m[2].leaf_value * 4.0  # the same tensor, other memory
+    check()
+    m[0].feature.set_(m[0].feature.clone())
+    check()
+    m.models_.append(m[0] * 0.5)
+    check()
+    m[3].leaf_value = m[3].leaf_value.repeat(1, 2)
+    with pytest.raises(ValueError):
+        m.predict_raw(X)
+
+
+def test_fits_on_several_threads_and_streams(lb):
+    """Calls in progress on one device share a context: what their kernels tell the host and where their blocks
+    meet belongs to one call."""
+    import threading
+
+    rs = np.random.RandomState(0)
+    jobs = []
+    for i, (N, F, S) in enumerate([(700, 6, 64), (30000, 12, 400), (900, 9, 256), (20000, 5, 600)]):
+        jobs.append((dev(rs.normal(size=(N, F))), dev(rs.normal(size=N)), S, i))
+
+    def fit(X, y, S, seed):
+        return lb.LBRegressor(n_estimators=4, base_models=(lb.Tree(max_depth=5, split_samples=S),), random_state=seed).fit(X, y)
+
+    want = [fit(*j) for j in jobs]
+    torch.cuda.synchronize()
+    got, errors = {}, []
+
+    def work(j):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(5):
+                    got[j[3]] = fit(*j)
+        except Exception as e:  # seen by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(j,)) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    for j, w in zip(jobs, want):
+        for a, b in zip(got[j[3]], w):
+            for name in ("feature", "split_value", "leaf_value", "hessian"):
+                assert torch.equal(getattr(a, name), getattr(b, name))
