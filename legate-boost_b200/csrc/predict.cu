@@ -5,24 +5,33 @@
 // feature[pos] != -1 (at most 100 steps), going left iff (double)x <= split_value[pos].
 //
 // Design for B200: ONE launch for the whole ensemble, everything a step of the walk touches lives
-// in shared memory.
+// in shared memory.  The load/store data pipe of the SM is what bounds it (one pass per clock; a 4-byte load of
+// a warp is one pass, an 8-byte load two, plus one per bank conflict), so the layouts save passes:
 //   * A block owns a tile of rows (one thread per row); every thread stages its own row,
 //     feature-major with a pitch of one element per thread, so thread t only ever touches bank
 //     t mod 32 whatever feature a tree asks for: the x lookups of a walk never conflict.  Every row
 //     of X is read from HBM exactly once (16-byte loads, the rest of a sector comes from L1).
-//   * The trees are first packed into one array of small nodes: for float32 X a node is 8 bytes
-//     (float split, int feature) - "x <= split" with x a float is the same test as
-//     "x <= the largest float not above split", so the split is rounded down once at packing time
-//     and the walk compares floats; for float64 X a node is 16 bytes.
+//   * The trees are first packed into records: the splits of the heap, then the feature ids of a node and its
+//     two children in one word (10 bits each), then (one output) the bottom level of leaf values.  Two
+//     levels of a walk are two split loads, one feature load and two x loads: 5 passes for float32, where
+//     {split, feature} nodes of 8 bytes took 6 and conflicted twice as often (24 passes per walk of depth 8
+//     against 34).  A walk keeps the shared-memory address of its node: a step is one addition for the
+//     left child and one more for the right one, whatever the level (with the position in the level and offsets per
+//     level a walk was 120 instructions, and those bound it).
+//   * For float32 X a split is a float - "x <= split" with x a float is the same test as "x <= the largest
+//     float not above split", so the split is rounded down once at packing time.
 //   * At packing time every tree is completed to the depth S of the deepest one: below a leaf
 //     the nodes become pass-through nodes (split = +inf) and the leaf's value is copied to the
-//     bottom level.  A walk is then exactly S steps of "load node, load x, compare, descend" with
-//     no leaf test, and only the bottom level of leaf values is kept.
-//   * Trees are brought into shared memory in groups of up to eight (bulk async copies, double buffered)
-//     together with their bottom-level leaf values; a thread walks the trees of a group as
-//     independent chains, which hides the shared-memory latency that one dependent chain exposes.
+//     bottom level.  A walk is then exactly S steps with no leaf test, and only the bottom level of leaf
+//     values is kept.
+//   * Trees are brought into shared memory in groups of up to eight by a producer warp (bulk async copies, two
+//     buffers, full and empty mbarriers): no warp waits for another one's walks.  A thread walks the trees
+//     of a group as independent chains, which hides the latency that one dependent chain exposes.
+//   * With several outputs the leaf values stay in global memory and a warp reads them together: its 32 x K
+//     sums are spread over the lanes, output innermost, so that a load covers the K values of three or more
+//     rows' leaves as whole pieces of lines.  (A lane reading its own row's K values cost 32 passes per value.)
 //   * Predictions are accumulated in float64 in tree order (bit-identical to the reference's
-//     tree-by-tree accumulation) and written once.
+//     tree-by-tree accumulation), transformed and written once.
 // A fallback kernel with the nodes in global memory covers shapes whose tile or trees do not fit.
 #include "device_utils.cuh"
 #include "internal.h"
@@ -121,16 +130,15 @@ __device__ inline bool MbarWait(unsigned bar, unsigned parity, int* status)
   return false;
 }
 
-__device__ inline void LdsNode(unsigned addr, float& split, int& foff)
+__device__ inline void MbarArrive(unsigned bar)
 {
-  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];\n" : "=f"(split), "=r"(foff) : "r"(addr));
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
-__device__ inline void LdsNode(unsigned addr, double& split, int& foff)
+__device__ inline unsigned LdsU32(unsigned addr)
 {
-  int pad;
-  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n"
-               : "=r"(reinterpret_cast<int2&>(split).x), "=r"(reinterpret_cast<int2&>(split).y), "=r"(foff), "=r"(pad)
-               : "r"(addr));
+  unsigned v;
+  asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(addr));
+  return v;
 }
 __device__ inline float LdsX(unsigned addr, float)
 {
@@ -151,40 +159,75 @@ __device__ inline double LdsF64(unsigned addr)
   return v;
 }
 
-// Completed-tree packing for the tiled kernel.  For tree t: nodes_c[t*NI + i], i < 2^S - 1, are the
-// internal levels of a complete tree of depth S; leaves_c[(t*NL + j)*K + k], j < 2^S, the values of
-// its bottom level.  A node whose children would fall outside the input arrays, or whose feature
-// id is outside [0, F), counts as a leaf, so a walk can never leave the arrays.
-template <typename NodeT>
-__global__ void k_pack_complete(const TreePtrs* __restrict__ trees, int K, int F, int xmul, int S, int NI, int NL,
-                                NodeT* __restrict__ nodes_c, double* __restrict__ leaves_c)
+__device__ inline void MakeSplit(float& s, double split) { s = __double2float_rd(split); }
+__device__ inline void MakeSplit(double& s, double split) { s = split; }
+
+// A completed tree of depth S as the tiled kernel reads it.  Nodes are counted from 1: those of level l are
+// [2^l, 2^(l + 1)), the children of i are 2 i and 2 i + 1.  Splits [2^S] of T; words with the feature ids of a
+// node and its children (used for the nodes of even levels); leaf values [2^S] (one output only).  The parts
+// are whole multiples of 16 bytes.
+struct TreeRecord {
+  int S;
+  int split_bytes, word_bytes, leaf_bytes, bytes;
+};
+constexpr int kIdBits     = 10;  // feature ids in a word: three of them
+constexpr int kMaxFeature = 1 << kIdBits;
+static TreeRecord RecordOf(int S, size_t elem, bool with_leaves)
 {
-  const TreePtrs t = trees[blockIdx.x];
-  const int M      = t.max_nodes;
-  const int total  = (2 << S) - 1;  // nodes of the complete tree
-  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+  auto up16 = [](int v) { return (v + 15) / 16 * 16; };
+  TreeRecord r;
+  r.S           = S;
+  r.split_bytes = up16((1 << S) * static_cast<int>(elem));
+  r.word_bytes  = up16((S > 0 ? 2 << ((S - 1) / 2 * 2) : 0) * 4);
+  r.leaf_bytes  = with_leaves ? up16((1 << S) * 8) : 0;
+  r.bytes       = r.split_bytes + r.word_bytes + r.leaf_bytes;
+  return r;
+}
+
+// One block packs one tree.  A node whose children would fall outside the input arrays, or whose feature
+// id is outside [0, F), counts as a leaf, so a walk can never leave the arrays.
+template <typename T>
+__global__ void k_pack_complete(const TreePtrs* __restrict__ trees, int K, int F, TreeRecord rec,
+                                unsigned char* __restrict__ records, double* __restrict__ leaves_c)
+{
+  const TreePtrs t   = trees[blockIdx.x];
+  const int M = t.max_nodes, S = rec.S;
+  unsigned char* out = records + static_cast<int64_t>(blockIdx.x) * rec.bytes;
+  T* splits          = reinterpret_cast<T*>(out);
+  unsigned* words    = reinterpret_cast<unsigned*>(out + rec.split_bytes);
+  double* leaves     = rec.leaf_bytes > 0 ? reinterpret_cast<double*>(out + rec.split_bytes + rec.word_bytes)
+                                          : leaves_c + (static_cast<int64_t>(blockIdx.x) << S) * K;
+  auto splits_here = [&](int a) {
+    if (a >= M || 2 * a + 2 >= M) return false;
+    const int f = t.feature[a];
+    return f >= 0 && f < F;
+  };
+  // first leaf on the path root -> i, or -1
+  auto cover_of = [&](int i) {
     const int L = 31 - __clz(i + 1);
-    int cover   = -1;  // first leaf on the path root -> i
     for (int l = 0; l <= L; ++l) {
-      const int a   = ((i + 1) >> (L - l)) - 1;
-      const int f   = a < M ? t.feature[a] : -1;
-      if (a >= M || f < 0 || f >= F || 2 * a + 2 >= M) {
-        cover = a;
-        break;
-      }
+      const int a = ((i + 1) >> (L - l)) - 1;
+      if (!splits_here(a)) return a;
     }
+    return -1;
+  };
+  const int total = (2 << S) - 1;  // nodes of the complete tree
+  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+    const int L = 31 - __clz(i + 1), cover = cover_of(i);
     if (L < S) {
-      NodeT n;
-      if (cover >= 0) {
-        MakeNode(n, static_cast<double>(INFINITY), 0);  // pass-through: always descends left
-      } else {
-        MakeNode(n, t.split[i], t.feature[i] * xmul);
+      // (a pass-through node sends a NaN to the right: the same leaf value is there)
+      MakeSplit(splits[i + 1], cover >= 0 ? static_cast<double>(INFINITY) : t.split[i]);
+      if ((L & 1) == 0) {
+        unsigned w = cover >= 0 ? 0u : static_cast<unsigned>(t.feature[i]);
+        if (cover < 0 && L + 1 < S) {
+          if (splits_here(2 * i + 1)) w |= static_cast<unsigned>(t.feature[2 * i + 1]) << kIdBits;
+          if (splits_here(2 * i + 2)) w |= static_cast<unsigned>(t.feature[2 * i + 2]) << (2 * kIdBits);
+        }
+        words[i + 1] = w;
       }
-      nodes_c[static_cast<int64_t>(blockIdx.x) * NI + i] = n;
     } else {
       const int j = i - ((1 << S) - 1);
-      for (int k = 0; k < K; ++k)
-        leaves_c[(static_cast<int64_t>(blockIdx.x) * NL + j) * K + k] = t.leaf[static_cast<int64_t>(cover) * K + k];
+      for (int k = 0; k < K; ++k) leaves[static_cast<int64_t>(j) * K + k] = t.leaf[static_cast<int64_t>(cover) * K + k];
     }
   }
 }
@@ -279,6 +322,236 @@ __global__ void __launch_bounds__(kRowsThreads)
   for (int r = tid; r < rows; r += kRowsThreads) FinishRow(sums + r * K, 1, K, o.pred + (row0 + r) * o.ldp, o.transform);
 }
 
+constexpr int kTileThreads = 512;  // of all blocks of an SM, producer warps included: 128 registers each
+
+template <typename T>
+struct TiledArgs {
+  const T* X;
+  int64_t ldx, n_rows;
+  int F, K, n_trees;
+  int rb;            // rows per block, a multiple of 32
+  int nbuf;          // group buffers: 2, or 1 if all trees are one group
+  unsigned x_bytes;  // of the X tile (and of what takes its place at the end)
+  const unsigned char* records;
+  TreeRecord rec;
+  const double* leaves_c;  // [tree][2^S][K] (several outputs)
+  PredictOut o;
+  int* status;
+};
+
+// Tiled kernel.  Shared memory: X tile [F][rb] | sums [K][rb] (KR < 0) | nbuf x TG records.
+// KR: outputs whose sums a warp holds in registers (at most KR of them); 0: one output, leaf values in the
+// records; -1: any number of outputs, sums in shared memory.
+// Measured against {split, feature} nodes, a block barrier per group, 256 rows per block and every lane reading
+// its own row's values: 10M x 100 float32, 500 trees of depth 8: 23.2 -> 19.5 ms; 1M x 64 float64, 100 trees: 1117 -> 803
+// us; 100003 x 100, 10 outputs, 50 trees: 224 -> 131 us.
+template <typename T, int TG, int KR>
+__global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledArgs<T> a)
+{
+  __shared__ __align__(8) unsigned long long s_bar[4];  // full[2], empty[2]
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int rb = a.rb, F = a.F, K = a.K, S = a.rec.S;
+  T* xs        = reinterpret_cast<T*>(smem_raw);
+  double* accs = reinterpret_cast<double*>(smem_raw + a.x_bytes);
+  const unsigned rec_bytes = a.rec.bytes, buf_bytes = TG * rec_bytes;
+  const unsigned tree0 = static_cast<unsigned>(__cvta_generic_to_shared(smem_raw)) + a.x_bytes + (KR < 0 ? 8u * K * rb : 0u);
+  const unsigned full0 = static_cast<unsigned>(__cvta_generic_to_shared(&s_bar[0])), empty0 = full0 + 16;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * rb;
+  const int n_groups = (a.n_trees + TG - 1) / TG;
+  if (tid == 0) {
+    for (int b = 0; b < 2; ++b) {
+      MbarInit(full0 + 8 * b, 1);
+      MbarInit(empty0 + 8 * b, rb / 32);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  __syncthreads();
+
+  if (warp == rb / 32) {  // the producer: brings group after group into the buffer that every warp is done with
+    if (lane == 0) {
+      int g   = 0;
+      bool ok = true;
+      for (; g < n_groups && ok; ++g) {
+        const int b = a.nbuf == 2 ? g & 1 : 0;
+        if (g >= 2) ok = MbarWait(empty0 + 8 * b, ((g >> 1) - 1) & 1, a.status);
+        if (!ok) break;
+        const unsigned bytes = min(TG, a.n_trees - g * TG) * rec_bytes;
+        MbarExpectTx(full0 + 8 * b, bytes);
+        BulkCopy(tree0 + b * buf_bytes, a.records + static_cast<int64_t>(g) * buf_bytes, bytes, full0 + 8 * b);
+      }
+      // nothing is in flight when the block ends, whatever the other warps waited for
+      for (int h = max(g - 2, 0); h < g; ++h) MbarWait(full0 + 8 * (a.nbuf == 2 ? h & 1 : 0), (h >> 1) & 1, a.status);
+    }
+    __syncthreads();
+    return;
+  }
+
+  // Every thread copies its own row into its own column of the tile and reads nothing else of it.  16-byte loads
+  // when the rows allow it; the sectors of a row are reused from L1 by the following loads of the same thread.
+  if (row0 + tid < a.n_rows) {
+    const T* xr     = a.X + (row0 + tid) * a.ldx;
+    constexpr int V = 16 / sizeof(T);
+    int f           = 0;
+    if ((reinterpret_cast<uintptr_t>(a.X) & 15) == 0 && a.ldx % V == 0) {
+#pragma unroll 8
+      for (; f + V <= F; f += V) {
+        const int4 v = *reinterpret_cast<const int4*>(xr + f);
+#pragma unroll
+        for (int i = 0; i < V; ++i) xs[(f + i) * rb + tid] = reinterpret_cast<const T*>(&v)[i];
+      }
+    }
+    for (; f < F; ++f) xs[f * rb + tid] = xr[f];
+  } else {
+    // the walks of the missing rows are made too (any value leads to some leaf) and not written
+    for (int f = 0; f < F; ++f) xs[f * rb + tid] = T(0);
+  }
+  if (KR < 0)
+    for (int k = 0; k < K; ++k) accs[k * rb + tid] = 0.0;
+
+  // KR > 0: the warp's sums are numbered output innermost, lane l holds l, l + 32, ...
+  constexpr int kSums = KR > 0 ? KR : 1;
+  double acc[kSums];
+  int which[kSums];  // of each: lane (row of the warp) + 32 x output
+#pragma unroll
+  for (int i = 0; i < kSums; ++i) {
+    acc[i] = 0.0;
+    const int r = KR > 0 ? (lane + 32 * i) / K : 0;
+    which[i]    = KR > 0 && i < K ? r + 32 * (lane + 32 * i - r * K) : 0;  // (what is beyond K is read and dropped)
+  }
+
+  // The walk works on 32-bit shared addresses; at[j] is that of the split of tree j's current node.
+  constexpr unsigned kT    = sizeof(T);
+  const unsigned xcol_s    = static_cast<unsigned>(__cvta_generic_to_shared(xs + tid));
+  const unsigned pitch     = static_cast<unsigned>(rb * sizeof(T));
+  const unsigned word_off  = a.rec.split_bytes;
+  const unsigned leaf_off  = a.rec.split_bytes + a.rec.word_bytes - (8u << S);
+  constexpr unsigned kMask = kMaxFeature - 1;
+  for (int g = 0; g < n_groups; ++g) {
+    const int b = a.nbuf == 2 ? g & 1 : 0;
+    if (!__all_sync(0xffffffffu, MbarWait(full0 + 8 * b, (g >> 1) & 1, a.status) ? 1 : 0)) break;
+    const int nt = min(TG, a.n_trees - g * TG);
+    unsigned at[TG], base[TG];
+#pragma unroll
+    for (int j = 0; j < TG; ++j) {
+      base[j] = tree0 + b * buf_bytes + j * rec_bytes;
+      at[j]   = base[j] + kT;
+    }
+    // Two levels of all walks at a time: first every split and word, then every x, then the compares, so that
+    // the loads of the independent walks are in flight together (the loads are volatile and keep
+    // their order).  `here(j)` is always true but in the last group.
+    auto walk = [&](auto here) {
+      T split[TG], x[TG];
+      unsigned w[TG];
+      auto first_loads = [&]() {
+#pragma unroll
+        for (int j = 0; j < TG; ++j)
+          if (here(j)) {
+            w[j]     = LdsU32(kT == 4 ? at[j] + word_off : base[j] + word_off + ((at[j] - base[j]) >> 1));
+            split[j] = LdsX(at[j], T());
+          }
+      };
+      auto x_loads = [&]() {
+#pragma unroll
+        for (int j = 0; j < TG; ++j)
+          if (here(j)) x[j] = LdsX(xcol_s + (w[j] & kMask) * pitch, T());
+      };
+      auto descend = [&](int j) {
+        const bool left = x[j] <= split[j];
+        at[j]           = at[j] + at[j] - base[j];
+        if (!left) at[j] += kT;
+        return left;
+      };
+      int l = 0;
+#pragma unroll 1
+      for (; l + 1 < S; l += 2) {
+        first_loads();
+        x_loads();
+#pragma unroll
+        for (int j = 0; j < TG; ++j)
+          if (here(j)) {
+            w[j] >>= descend(j) ? kIdBits : 2 * kIdBits;
+            split[j] = LdsX(at[j], T());
+          }
+        x_loads();
+#pragma unroll
+        for (int j = 0; j < TG; ++j)
+          if (here(j)) descend(j);
+      }
+      if (l < S) {
+        first_loads();
+        x_loads();
+#pragma unroll
+        for (int j = 0; j < TG; ++j)
+          if (here(j)) descend(j);
+      }
+      if (KR == 0) {
+        double v[TG];
+#pragma unroll
+        for (int j = 0; j < TG; ++j)
+          if (here(j)) v[j] = LdsF64(base[j] + leaf_off + (at[j] - base[j]) * (8u / kT));
+#pragma unroll
+        for (int j = 0; j < TG; ++j)
+          if (here(j)) acc[0] += v[j];
+      }
+    };
+    if (nt == TG) walk([](int) { return true; });
+    else walk([&](int j) { return j < nt; });
+    __syncwarp();
+    if (lane == 0) MbarArrive(empty0 + 8 * b);  // this warp is done with the buffer
+    if (KR != 0) {
+      const int64_t tree_values = static_cast<int64_t>(K) << S;
+      const double* lf          = a.leaves_c + g * TG * tree_values;
+      auto add = [&](auto here) {
+#pragma unroll
+        for (int j = 0; j < TG; ++j) {
+          if (!here(j)) continue;
+          const int v = (static_cast<int>((at[j] - base[j]) / kT) - (1 << S)) * K;  // the row's first value
+          if (KR > 0) {
+#pragma unroll
+            for (int i = 0; i < kSums; ++i) acc[i] += __ldg(lf + __shfl_sync(0xffffffffu, v, which[i] & 31) + (which[i] >> 5));
+          } else {
+            for (int k = 0; k < K; ++k) accs[k * rb + tid] += lf[v + k];
+          }
+          lf += tree_values;
+        }
+      };
+      if (nt == TG) add([](int) { return true; });
+      else add([&](int j) { return j < nt; });
+    }
+  }
+
+  const PredictOut& o = a.o;
+  const int64_t row   = row0 + tid;
+  if (KR == 0) {
+    const double raw = o.init ? o.init[0] + acc[0] : acc[0];
+    if (row < a.n_rows) FinishRow(&raw, 1, 1, o.pred + row * o.ldp, o.transform);
+  } else if (KR < 0) {
+    if (o.init)
+      for (int k = 0; k < K; ++k) accs[k * rb + tid] = o.init[k] + accs[k * rb + tid];
+    if (row < a.n_rows) FinishRow(accs + tid, rb, K, o.pred + row * o.ldp, o.transform);
+  } else {
+    double* rows = reinterpret_cast<double*>(smem_raw) + static_cast<int64_t>(warp) * 32 * K;  // of the warp, [32][K]
+    if (o.transform != LBK_RAW) {
+      asm volatile("bar.sync 1, %0;\n" ::"r"(rb) : "memory");  // the walks are done: the rows take the place of X
+#pragma unroll
+      for (int i = 0; i < kSums; ++i)
+        if (i < K) rows[lane + 32 * i] = o.init ? o.init[which[i] >> 5] + acc[i] : acc[i];
+      __syncwarp();
+      FinishRow(rows + lane * K, 1, K, rows + lane * K, o.transform);
+      __syncwarp();
+    }
+#pragma unroll
+    for (int i = 0; i < kSums; ++i) {
+      const int64_t r = row0 + warp * 32 + (which[i] & 31);
+      if (i < K && r < a.n_rows)
+        o.pred[r * o.ldp + (which[i] >> 5)] = o.transform != LBK_RAW ? rows[lane + 32 * i] : o.init ? o.init[which[i] >> 5] + acc[i] : acc[i];
+    }
+  }
+  __syncthreads();  // (the producer's copies)
+}
+
 // What is left to do after a kernel that wrote the raw sums.
 __global__ void __launch_bounds__(256) k_finish_rows(int64_t n_rows, int K, PredictOut o)
 {
@@ -286,159 +559,6 @@ __global__ void __launch_bounds__(256) k_finish_rows(int64_t n_rows, int K, Pred
   if (row >= n_rows) return;
   double* p = o.pred + row * o.ldp;
   FinishRow(p, 1, K, p, o.transform);
-}
-
-// Tiled kernel.  Shared memory: X tile [F][RB] | accumulators [K][RB] (K > 1) |
-// NBUF x TG x slot, slot = NI nodes (+ NL leaf values when K == 1).
-template <typename T, int RB, int TG, bool kLeafShared>
-__global__ void __launch_bounds__(RB)
-  k_predict_tiled(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees,
-                  const typename NodeOf<T>::type* __restrict__ nodes_c, const double* __restrict__ leaves_c,
-                  PredictOut o, int S, int NI, int NL, int* __restrict__ status)
-{
-  using NodeT = typename NodeOf<T>::type;
-  __shared__ __align__(8) unsigned long long s_bar[2];
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* xs = reinterpret_cast<T*>(smem_raw);
-  size_t off = (sizeof(T) * static_cast<size_t>(F) * RB + 15) / 16 * 16;
-  double* accs = reinterpret_cast<double*>(smem_raw + off);
-  off += K > 1 ? sizeof(double) * static_cast<size_t>(K) * RB : 0;
-  // a group buffer: the nodes of its TG trees, then (K == 1) their bottom-level values
-  const unsigned node_bytes = static_cast<unsigned>(NI * sizeof(NodeT));
-  const unsigned leaf_bytes = kLeafShared ? static_cast<unsigned>(NL * sizeof(double)) : 0u;
-  const unsigned buf_bytes  = TG * (node_bytes + leaf_bytes);
-  unsigned char* tree_s     = smem_raw + off;
-
-  const int tid       = threadIdx.x;
-  const int64_t row0  = static_cast<int64_t>(blockIdx.x) * RB;
-  const int rows_here = static_cast<int>((n_rows - row0) < RB ? (n_rows - row0) : RB);
-  const unsigned tree0 = static_cast<unsigned>(__cvta_generic_to_shared(tree_s));
-  const unsigned bar0  = static_cast<unsigned>(__cvta_generic_to_shared(&s_bar[0]));
-  const int n_groups   = (n_trees + TG - 1) / TG;
-  if (tid == 0) {
-    MbarInit(bar0, 1);
-    MbarInit(bar0 + 8, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncthreads();
-
-  // group of trees -> shared memory: two bulk copies (the trees of a group are neighbours in the
-  // packed arrays), issued by one thread
-  auto stage_group = [&](int group, int buf) {
-    if (tid != 0) return;
-    const int t0       = group * TG;
-    const unsigned nt  = static_cast<unsigned>(min(TG, n_trees - t0));
-    const unsigned bar = bar0 + 8u * buf;
-    const unsigned dst = tree0 + static_cast<unsigned>(buf) * buf_bytes;
-    MbarExpectTx(bar, nt * (node_bytes + leaf_bytes));
-    BulkCopy(dst, nodes_c + static_cast<int64_t>(t0) * NI, nt * node_bytes, bar);
-    if (kLeafShared) BulkCopy(dst + TG * node_bytes, leaves_c + static_cast<int64_t>(t0) * NL, nt * leaf_bytes, bar);
-  };
-  stage_group(0, 0);
-
-  // Stage the X tile: every thread copies its own row, feature-major with a pitch of RB elements,
-  // so that thread t only ever touches bank t mod 32 (x 2 for float64) - on the way in and in every
-  // step of every walk, whatever features the trees ask for.  16-byte loads when the rows allow it;
-  // the sectors of a row are reused from L1 by the following loads of the same thread.
-  if (tid < rows_here) {
-    const T* xr     = X + (row0 + tid) * ldx;
-    constexpr int V = 16 / sizeof(T);
-    int f           = 0;
-    if ((reinterpret_cast<uintptr_t>(X) & 15) == 0 && ldx % V == 0) {
-#pragma unroll 4
-      for (; f + V <= F; f += V) {
-        const int4 v = *reinterpret_cast<const int4*>(xr + f);
-#pragma unroll
-        for (int i = 0; i < V; ++i) xs[(f + i) * RB + tid] = reinterpret_cast<const T*>(&v)[i];
-      }
-    }
-    for (; f < F; ++f) xs[f * RB + tid] = xr[f];
-  }
-  if (K > 1)
-    for (int k = 0; k < K; ++k) accs[k * RB + tid] = 0.0;
-
-  // The walk works on 32-bit shared addresses.  `p8` is the heap index of the current node times 8
-  // (times sizeof(NodeT)/8 it is the node's byte offset); after S steps it points into the bottom
-  // level, whose values start at heap index 2^S - 1.
-  constexpr unsigned kNodeShift = sizeof(NodeT) == 16 ? 1 : 0;
-  const unsigned xcol_s   = static_cast<unsigned>(__cvta_generic_to_shared(xs + tid));
-  const unsigned leaf_adj = TG * node_bytes - 8u * ((1u << S) - 1u);  // from a bottom-level p8 to the value, tree 0
-  const bool one_buffer   = n_groups == 1;
-  double acc0             = 0.0;
-  __syncthreads();  // the X tile is in place
-  for (int g = 0; g < n_groups; ++g) {
-    const int buf = one_buffer ? 0 : (g & 1);
-    // buffer `buf` is filled for the (g / 2)-th time (every time when there is one buffer)
-    const unsigned parity = one_buffer ? (g & 1) : ((g >> 1) & 1);
-    // group g has landed - or every thread of the block gives up together
-    if (!__syncthreads_and(MbarWait(bar0 + 8u * buf, parity, status) ? 1 : 0)) break;
-    if (g + 1 < n_groups && !one_buffer) stage_group(g + 1, buf ^ 1);
-    const unsigned gbase = tree0 + static_cast<unsigned>(buf) * buf_bytes;
-    const int nt         = min(TG, n_trees - g * TG);
-    if (tid < rows_here) {
-      unsigned p8[TG];
-#pragma unroll
-      for (int j = 0; j < TG; ++j) p8[j] = 0;
-      if (nt == TG) {
-        // a step of all TG walks: first every node load, then every x load, then the compares, so
-        // that the loads of the independent walks are in flight together (the loads are volatile
-        // and keep their order: interleaved per walk they would run one after the other)
-        for (int step = 0; step < S; ++step) {
-          T split[TG];
-          int foff[TG];
-          T x[TG];
-#pragma unroll
-          for (int j = 0; j < TG; ++j) LdsNode(gbase + j * node_bytes + (p8[j] << kNodeShift), split[j], foff[j]);
-#pragma unroll
-          for (int j = 0; j < TG; ++j) x[j] = LdsX(xcol_s + foff[j], T());
-#pragma unroll
-          for (int j = 0; j < TG; ++j) p8[j] = 2 * p8[j] + (x[j] <= split[j] ? 8u : 16u);
-        }
-      } else {
-        // (the last, partial group: the same unrolled steps under a predicate, so that p8 stays in
-        // registers)
-        for (int step = 0; step < S; ++step) {
-          T split[TG];
-          int foff[TG];
-          T x[TG];
-#pragma unroll
-          for (int j = 0; j < TG; ++j)
-            if (j < nt) LdsNode(gbase + j * node_bytes + (p8[j] << kNodeShift), split[j], foff[j]);
-#pragma unroll
-          for (int j = 0; j < TG; ++j)
-            if (j < nt) x[j] = LdsX(xcol_s + foff[j], T());
-#pragma unroll
-          for (int j = 0; j < TG; ++j)
-            if (j < nt) p8[j] = 2 * p8[j] + (x[j] <= split[j] ? 8u : 16u);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < TG; ++j) {
-        if (j < nt) {
-          if (kLeafShared) {
-            acc0 += LdsF64(gbase + j * leaf_bytes + leaf_adj + p8[j]);
-          } else {
-            const int64_t lj = static_cast<int64_t>(g * TG + j) * NL + ((p8[j] >> 3) - ((1u << S) - 1u));
-            const double* lf = leaves_c + lj * K;
-            for (int k = 0; k < K; ++k) accs[k * RB + tid] += lf[k];
-          }
-        }
-      }
-    }
-    __syncthreads();  // everyone is done with buffer `buf` before it is refilled
-    if (g + 1 < n_groups && one_buffer) stage_group(g + 1, 0);
-  }
-  if (tid < rows_here) {
-    const int64_t row = row0 + tid;
-    if (K == 1) {
-      o.pred[row * o.ldp] = o.init ? o.init[0] + acc0 : acc0;
-    } else {
-      for (int k = 0; k < K; ++k) {
-        const double v          = accs[k * RB + tid];
-        o.pred[row * o.ldp + k] = o.init ? o.init[k] + v : v;
-      }
-    }
-  }
 }
 
 // Fallback: original (uncompleted) trees, nodes and leaves in global memory, X read directly.
@@ -469,27 +589,76 @@ __global__ void __launch_bounds__(128)
     for (int k = 0; k < K; ++k) pred[k] = o.init[k] + pred[k];
 }
 
+// How the tiled kernel is cut.  rb == 0: the shape does not fit.
+struct TilePlan {
+  int rb = 0, tg = 0, nbuf = 0;
+  unsigned x_bytes = 0;
+  size_t smem      = 0;
+  TreeRecord rec{};
+};
+constexpr int kRegisterSums = 16;  // outputs whose sums a warp keeps in registers
+
+// The pipe is kept busy by the walks in flight: warps x trees per group.  That product is made as large as shared
+// memory allows, over groups of 8, 4, 2 or 1 trees and 1 to 4 blocks per SM, up to kTileThreads; equal products go to
+// more blocks, of which one stages its rows while another walks.  The rows are then spread evenly over the
+// waves that this takes, so that the last one is not nearly empty.
 template <typename T>
-size_t TiledSmem(int rb, int tg, int nbuf, int F, int K, int NI, int NL, bool leaf_shared)
+TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, int S, int transform)
 {
-  using NodeT = typename NodeOf<T>::type;
-  const size_t x_bytes    = (sizeof(T) * static_cast<size_t>(F) * rb + 15) / 16 * 16;
-  const size_t a_bytes    = K > 1 ? sizeof(double) * static_cast<size_t>(K) * rb : 0;
-  const size_t slot_bytes = static_cast<size_t>(NI) * sizeof(NodeT) + (leaf_shared ? static_cast<size_t>(NL) * sizeof(double) : 0);
-  return x_bytes + a_bytes + static_cast<size_t>(nbuf) * tg * slot_bytes;
+  TilePlan best;
+  int best_score = 0, best_res = 1;
+  const size_t row_bytes = sizeof(T) * static_cast<size_t>(F) + (K > kRegisterSums ? 8 * static_cast<size_t>(K) : 0);
+  // (the finished rows of a few outputs take the place of X)
+  const size_t x_row = K > 1 && K <= kRegisterSums && transform != LBK_RAW ? std::max<size_t>(sizeof(T) * F, 8 * static_cast<size_t>(K)) : sizeof(T) * static_cast<size_t>(F);
+  const size_t per_row = std::max(row_bytes, x_row);
+  for (int tg = 8; tg >= 1; tg /= 2) {
+    if (tg > n_trees && tg > 1) continue;  // no wider than the ensemble
+    const TreeRecord rec = RecordOf(S, sizeof(T), K == 1);
+    const int nbuf       = n_trees > tg ? 2 : 1;
+    const size_t trees   = static_cast<size_t>(nbuf) * tg * rec.bytes;
+    for (int res = 1; res <= 4; ++res) {
+      const size_t room = res == 1 ? static_cast<size_t>(ctx->max_smem_optin) - 256 : (static_cast<size_t>(ctx->max_smem_optin) + 1024) / res - 1024 - 256;
+      if (trees + 32 * per_row > room) continue;
+      const int rb    = static_cast<int>(std::min<size_t>((room - trees) / per_row, kTileThreads / res - 32) / 32 * 32);
+      const int score = res * rb / 32 * tg;
+      if (score < best_score || (score == best_score && tg < best.tg)) continue;
+      best_score   = score;
+      best_res     = res;
+      best.rb      = rb;
+      best.tg      = tg;
+      best.nbuf    = nbuf;
+      best.rec     = rec;
+    }
+  }
+  if (best.rb == 0) return best;
+  const int64_t slots = static_cast<int64_t>(ctx->sm_count) * best_res;
+  const int64_t waves = (n_rows + best.rb * slots - 1) / (best.rb * slots);
+  best.rb             = static_cast<int>(((n_rows + waves * slots - 1) / (waves * slots) + 31) / 32 * 32);
+  best.x_bytes        = static_cast<unsigned>((x_row * best.rb + 15) / 16 * 16);
+  best.smem = best.x_bytes + (K > kRegisterSums ? 8 * static_cast<size_t>(K) * best.rb : 0) + static_cast<size_t>(best.nbuf) * best.tg * best.rec.bytes;
+  return best;
 }
 
-template <typename T, int RB, int TG, bool kLeafShared>
-void LaunchTiled(const T* X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees,
-                 const typename NodeOf<T>::type* nodes_c, const double* leaves_c, const PredictOut& o, int S, int NI, int NL, size_t smem, int* status, cudaStream_t stream)
+template <typename T, int TG, int KR>
+void LaunchTiledAs(const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
-  if (smem > 48 * 1024)
-    LBK_CUDA(cudaFuncSetAttribute(k_predict_tiled<T, RB, TG, kLeafShared>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
-  const unsigned grid = static_cast<unsigned>((n_rows + RB - 1) / RB);
-  k_predict_tiled<T, RB, TG, kLeafShared><<<grid, RB, smem, stream>>>(X, ldx, n_rows, F, K, n_trees, nodes_c, leaves_c, o, S, NI, NL,
-                                                                      status);
+  if (plan.smem > 48 * 1024)
+    LBK_CUDA(cudaFuncSetAttribute(k_predict_tiled<T, TG, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.smem)));
+  const unsigned grid = static_cast<unsigned>((a.n_rows + a.rb - 1) / a.rb);
+  k_predict_tiled<T, TG, KR><<<grid, a.rb + 32, plan.smem, stream>>>(a);
   LBK_LAUNCH_CHECK();
+}
+
+template <typename T, int TG>
+void LaunchTiled(const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
+{
+  if (a.K == 1) LaunchTiledAs<T, TG, 0>(a, plan, stream);
+  else if (a.K <= 2) LaunchTiledAs<T, TG, 2>(a, plan, stream);
+  else if (a.K <= 4) LaunchTiledAs<T, TG, 4>(a, plan, stream);
+  else if (a.K <= 8) LaunchTiledAs<T, TG, 8>(a, plan, stream);
+  else if (a.K <= 12) LaunchTiledAs<T, TG, 12>(a, plan, stream);
+  else if (a.K <= kRegisterSums) LaunchTiledAs<T, TG, kRegisterSums>(a, plan, stream);
+  else LaunchTiledAs<T, TG, -1>(a, plan, stream);
 }
 
 }  // namespace
@@ -526,35 +695,8 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   // a walk through M heap-ordered nodes takes at most S = floor(log2(M)) steps
   int S = 0;
   while ((2 << S) <= m_max) ++S;
-  const int NI = (1 << S) > 2 ? (1 << S) : 2;  // internal nodes 2^S - 1, padded to a 16-byte multiple
-  const int NL = NI;                           // bottom level 2^S values, same padding
-
-  // tile shape: rows per block RB, trees per group TG, one or two group buffers.  (Measured at 5 M x
-  // 100, 500 trees of depth 8: groups of 8 trees 14.8 ms; groups of 16 with the bottom-level values
-  // left in global memory 29.8 ms; groups of 4 27.3 ms.)
-  const size_t budget = static_cast<size_t>(ctx->max_smem_optin) - 1024;
-  int rb = 0, tg = 0;
-  const bool leaf_shared = K == 1;
-  size_t smem = 0;
-  if (S <= 14) {
-    const int rbs[4] = {256, 128, 64, 32};
-    const int tgs[4] = {8, 4, 2, 1};
-    for (int ri = 0; ri < 4 && rb == 0; ++ri) {
-      if (static_cast<int64_t>(F) * rbs[ri] * static_cast<int64_t>(sizeof(T)) >= (int64_t{1} << 30)) continue;
-      for (int ti = 0; ti < 4 && rb == 0; ++ti) {
-        if (tgs[ti] > n_trees && tgs[ti] > 1) continue;  // no wider than the ensemble
-        const int nbuf = n_trees > tgs[ti] ? 2 : 1;
-        const size_t need = TiledSmem<T>(rbs[ri], tgs[ti], nbuf, F, K, NI, NL, leaf_shared);
-        if (need <= budget) {
-          rb   = rbs[ri];
-          tg   = tgs[ti];
-          smem = need;
-        }
-      }
-    }
-  }
-
-  if (rb == 0) {
+  const TilePlan plan = S <= 14 && F <= kMaxFeature ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
+  if (plan.rb == 0) {
     NodeT* nodes   = s.alloc<NodeT>(total_nodes);
     double* leaves = s.alloc<double>(total_nodes * K);
     k_pack_trees<NodeT><<<n_trees, 256, 0, stream>>>(d_trees, K, F, 1, nodes, leaves);
@@ -565,28 +707,17 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
     finish();
     return;
   }
-  NodeT* nodes_c   = s.alloc<NodeT>(static_cast<size_t>(n_trees) * NI);
-  double* leaves_c = s.alloc<double>(static_cast<size_t>(n_trees) * NL * K);
-  k_pack_complete<NodeT><<<n_trees, 256, 0, stream>>>(d_trees, K, F, rb * static_cast<int>(sizeof(T)), S, NI, NL,
-                                                      nodes_c, leaves_c);
+  unsigned char* records = static_cast<unsigned char*>(s.alloc_bytes(static_cast<size_t>(n_trees) * plan.rec.bytes));
+  double* leaves_c       = K == 1 ? nullptr : s.alloc<double>((static_cast<size_t>(n_trees) << S) * K);
+  k_pack_complete<T><<<n_trees, 256, 0, stream>>>(d_trees, K, F, plan.rec, records, leaves_c);
   LBK_LAUNCH_CHECK();
-#define LBK_PREDICT_CASE(RB_, TG_, LS_)                                                                             \
-  if (rb == RB_ && tg == TG_ && leaf_shared == LS_) {                                                               \
-    LaunchTiled<T, RB_, TG_, LS_>(X, ldx, n_rows, F, K, n_trees, nodes_c, leaves_c, o, S, NI, NL, smem,             \
-                                  ctx->d_status, stream);                                                           \
-    finish();                                                                                                       \
-    return;                                                                                                         \
+  const TiledArgs<T> a{X, ldx, n_rows, F, K, n_trees, plan.rb, plan.nbuf, plan.x_bytes, records, plan.rec, leaves_c, o, ctx->d_status};
+  switch (plan.tg) {
+    case 8: LaunchTiled<T, 8>(a, plan, stream); break;
+    case 4: LaunchTiled<T, 4>(a, plan, stream); break;
+    case 2: LaunchTiled<T, 2>(a, plan, stream); break;
+    default: LaunchTiled<T, 1>(a, plan, stream); break;
   }
-#define LBK_PREDICT_ROW(RB_)                                                                                        \
-  LBK_PREDICT_CASE(RB_, 8, true) LBK_PREDICT_CASE(RB_, 4, true) LBK_PREDICT_CASE(RB_, 2, true) LBK_PREDICT_CASE(RB_, 1, true) \
-  LBK_PREDICT_CASE(RB_, 8, false) LBK_PREDICT_CASE(RB_, 4, false) LBK_PREDICT_CASE(RB_, 2, false) LBK_PREDICT_CASE(RB_, 1, false)
-  LBK_PREDICT_ROW(256)
-  LBK_PREDICT_ROW(128)
-  LBK_PREDICT_ROW(64)
-  LBK_PREDICT_ROW(32)
-#undef LBK_PREDICT_ROW
-#undef LBK_PREDICT_CASE
-  throw Error(LBK_ERR_ARGUMENT, "predict: no kernel for the chosen tile");
 }
 
 template void PredictLaunch<float>(lbk_context*, Scratch&, const float*, int64_t, int64_t, int, int, int, const lbk_tree_ref*,

@@ -838,6 +838,58 @@ def test_rounds_in_the_library_match_rounds_from_python(lb, N, F, D, S, classes,
     assert torch.equal(a.predict_raw(X[:50]), b.predict_raw(X[:50]))
 
 
+def random_trees(rs, F, K, T, D):
+    M = 2 ** (D + 1) - 1
+    trees = []
+    for _ in range(T):
+        feat = rs.randint(0, F, size=M).astype(np.int32)
+        feat[2 ** D - 1:] = -1
+        feat[rs.random(M) < 0.1] = -1
+        trees.append((rs.normal(size=(M, K)), feat, rs.normal(size=M)))
+    return trees
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("N,F,K,T,D", [
+    (8193, 1, 1, 1, 0), (8200, 7, 1, 8, 1), (20011, 100, 1, 17, 8),   # one group, whole groups, a last group of one
+    (9001, 5, 1, 3, 10), (9001, 40, 1, 30, 13), (8193, 3, 2, 9, 14),  # narrower groups and blocks for deep trees
+    (8193, 1024, 1, 5, 3), (8193, 1025, 2, 5, 3),                     # the last feature id of a packed word; beyond it
+    (8193, 12, 2, 9, 6), (30001, 20, 4, 8, 7), (8193, 3, 5, 16, 5), (8193, 9, 8, 10, 5),  # sums in registers
+    (8193, 4, 16, 3, 4), (8193, 4, 17, 11, 4),                        # ... the most of them; in shared memory
+])
+def test_predict_of_many_rows_is_bit_exact(lb, oracle, dtype, N, F, K, T, D):
+    """More rows than the one-launch form takes: trees in groups in shared memory, for rows that start on 16 bytes
+    and rows that do not, with values that compare false with everything."""
+    from legateboost_b200.tree import predict_arrays
+
+    rs = np.random.RandomState(N % 97 + F + K + T + D)
+    X = rs.normal(size=(N, F)).astype(dtype)
+    X[rs.random((N, F)) < 0.01] = np.nan
+    X[rs.random((N, F)) < 0.01] = np.inf
+    X[rs.random((N, F)) < 0.01] = -np.inf
+    trees = random_trees(rs, F, K, T, D)
+    d_trees = [tuple(map(dev, t)) for t in trees]
+    want = oracle.predict(X, trees)
+    assert np.array_equal(predict_arrays(dev(X), d_trees).cpu().numpy(), want)
+    wide = torch.zeros((N, F + 2), dtype=torch.from_numpy(X).dtype, device="cuda")
+    wide[:, 1:F + 1] = dev(X)
+    assert np.array_equal(predict_arrays(wide[:, 1:F + 1], d_trees).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("N,classes,F", [(50, 2, 4), (9000, 2, 4), (50, 3, 4), (9000, 3, 4), (9000, 10, 3), (9000, 20, 4)])
+def test_probabilities_are_those_of_the_raw_predictions(lb, N, classes, F):
+    rs = np.random.RandomState(classes)
+    X = dev(rs.normal(size=(N, F)))
+    m = lb.LBClassifier(n_estimators=4, base_models=(lb.Tree(max_depth=3, split_samples=32),), random_state=0)
+    m.fit(X, dev(np.arange(N) % classes))
+    raw = m.predict_raw(X)
+    p = torch.sigmoid(raw) if classes == 2 else torch.softmax(raw, dim=1)
+    if classes == 2:
+        p = torch.cat([1.0 - p, p], dim=1)
+    # exp, a sum of `classes` terms and a division: a few units in the last place
+    assert torch.allclose(m.predict_proba(X), p, rtol=(classes + 8) * 2.3e-16, atol=2.3e-16)
+
+
 def test_an_ensemble_predicts_what_its_trees_hold_now(lb):
     """The device table of the trees' addresses follows every way to change a tree."""
     from legateboost_b200.tree import predict_arrays
