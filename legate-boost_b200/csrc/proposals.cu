@@ -461,7 +461,83 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
   if (turn < n) do_turn(std::true_type());
 }
 
-// Global-memory variant for features with more proposals than shared memory holds.
+// Two-byte ids, more proposals than k_bin_smem's table of 32 features holds: a table of as many features
+// (16, 8 or 4) as fill 64 KB, three blocks per SM.  A lane has one feature and eight consecutive rows, which leave as
+// one 16-byte store of the feature-major copy; the 32 / kFeatures row groups of a warp may meet in a bank
+// (a probe is 1 to 2.5 passes), which costs less than the probes going to L2: 300003 x 37 float64,
+// 512 proposals: 70 us against 425 of k_bin_global.  Filling the table takes 8 (float64) to 15 us (float32), so that
+// small float32 matrices stay with k_bin_global (10000 x 37, 1024 proposals: 20 us here, 13 there; 100000 x 37: 35
+// and 64; float64: 14 and 18; 39 and 77).
+constexpr int kWideTableBytes = 64 * 1024;
+
+template <typename T, int kLog2P, bool kCopyT>
+__global__ void __launch_bounds__(256, 3)
+  k_bin_wide(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const T* __restrict__ proposals, int64_t cut_stride,
+             const int32_t* __restrict__ row_ptr, int pitch, uint16_t* __restrict__ bins, uint16_t* __restrict__ bins_t, int64_t pitch_t)
+{
+  constexpr int P         = 1 << kLog2P;
+  constexpr int kFeatures = kWideTableBytes / (P * static_cast<int>(sizeof(T)));
+  constexpr int U         = 8;
+  constexpr int kTurn     = 32 / kFeatures * U;  // rows of a warp
+  constexpr unsigned kPitch = kFeatures * sizeof(T);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* sp        = reinterpret_cast<T*>(smem_raw);
+  const int f0 = blockIdx.y * kFeatures;
+  if (f0 >= F) {  // padding columns
+    const int64_t all = n_rows * kFeatures;
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < all; i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+      bins[i / kFeatures * pitch + f0 + i % kFeatures] = 0;
+    return;
+  }
+  for (int idx = threadIdx.x; idx < P * kFeatures; idx += blockDim.x) {
+    const int j = idx / kFeatures, f = f0 + idx % kFeatures;
+    T v = static_cast<T>(INFINITY);
+    if (f < F) {
+      const int b = row_ptr[f];
+      if (j < row_ptr[f + 1] - b) v = proposals[(cut_stride > 0 ? f * cut_stride : b) + j];
+    }
+    sp[idx] = v;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, f = f0 + lane % kFeatures;
+  // lanes beyond the last feature read the last feature's values; their column is all +inf, their ids are 0
+  const bool active    = f < F;
+  const unsigned col_s = static_cast<unsigned>(__cvta_generic_to_shared(sp + lane % kFeatures));
+  const T* xcol        = X + (active ? f : F - 1);
+  const int n          = static_cast<int>(n_rows);
+  const int hop        = static_cast<int>(gridDim.x) * (blockDim.x >> 5) * kTurn;
+  int base             = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kTurn + lane / kFeatures * U;
+  T xn[U];
+  auto load_rows = [&](int first) {
+    const T* src = xcol + static_cast<int64_t>(first) * ldx;
+#pragma unroll
+    for (int u = 0; u < U; ++u) xn[u] = first + u < n ? LdgStream(src + u * ldx) : static_cast<T>(-INFINITY);
+  };
+  load_rows(base);
+  for (; base < n; base += hop) {
+    T x[U];
+    unsigned pos[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      x[u]   = xn[u];
+      pos[u] = col_s;
+    }
+    if (base + hop < n) load_rows(base + hop);
+    SearchLevels<T, U, kLog2P - 1, kPitch>::run(pos, x);
+    unsigned id[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) id[u] = (pos[u] - col_s) / kPitch;
+    uint16_t* out = bins + static_cast<int64_t>(base) * pitch + f;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (base + u < n) out[static_cast<int64_t>(u) * pitch] = static_cast<uint16_t>(id[u]);
+    if (kCopyT && active)  // (the copy's rows are padded to 32; ids beyond the last row are 0)
+      *reinterpret_cast<uint4*>(bins_t + static_cast<int64_t>(f) * pitch_t + base) =
+        make_uint4(id[0] | (id[1] << 16), id[2] | (id[3] << 16), id[4] | (id[5] << 16), id[6] | (id[7] << 16));
+  }
+}
+
+// Global-memory variant: more proposals than any table here holds, or too few rows to pay for filling one.
 template <typename T, typename BinT>
 __global__ void __launch_bounds__(256)
   k_bin_global(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const T* __restrict__ proposals,
@@ -498,6 +574,10 @@ __global__ void __launch_bounds__(256)
     if (bins_t != nullptr && active) bins_t[static_cast<int64_t>(f) * pitch_t + row] = static_cast<BinT>(bin);
   }
 }
+
+// k_bin_wide pays for filling its table from this many cells on
+template <typename T>
+constexpr int64_t kWideMinCells = sizeof(T) == 8 ? 0 : int64_t{1} << 20;
 
 int NextPow2(int v)
 {
@@ -625,7 +705,27 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
                                                        pitch_t);                                          \
     }                                                                                                     \
   } while (0)
-  if (bin_bytes == 1) {
+  if (bin_bytes == 2 && !use_smem && need <= 2048 && n_rows * F >= kWideMinCells<T>) {
+    auto wide = [&](auto log2p_, auto copy_) {
+      constexpr int L    = decltype(log2p_)::value;
+      constexpr bool CT  = decltype(copy_)::value;
+      constexpr int kFeatures = kWideTableBytes / ((1 << L) * static_cast<int>(sizeof(T)));
+      auto fn = k_bin_wide<T, L, CT>;
+      LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideTableBytes));
+      dim3 grid = make_grid(3);  // (resident blocks, spread over the tables that hold features)
+      grid.x    = std::max<unsigned>(1u, grid.x * G / ((F + kFeatures - 1) / kFeatures));
+      grid.y    = G * kGroup / kFeatures;
+      fn<<<grid, 256, kWideTableBytes, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, G * kGroup,
+                                                 static_cast<uint16_t*>(bins), static_cast<uint16_t*>(bins_t), pitch_t);
+    };
+    auto by_copy = [&](auto log2p_) {
+      if (bins_t != nullptr) wide(log2p_, std::true_type());
+      else wide(log2p_, std::false_type());
+    };
+    if (need <= 512 && sizeof(T) == 8) by_copy(std::integral_constant<int, sizeof(T) == 8 ? 9 : 10>());
+    else if (need <= 1024) by_copy(std::integral_constant<int, 10>());
+    else by_copy(std::integral_constant<int, 11>());
+  } else if (bin_bytes == 1) {
     LBK_BIN_LAUNCH(uint8_t);
   } else {
     LBK_BIN_LAUNCH(uint16_t);

@@ -954,3 +954,28 @@ def test_fits_on_several_threads_and_streams(lb):
         for a, b in zip(got[j[3]], w):
             for name in ("feature", "split_value", "leaf_value", "hessian"):
                 assert torch.equal(getattr(a, name), getattr(b, name))
+
+
+@pytest.mark.parametrize("dtype,N,F,S", [
+    (np.float64, 1, 1, 512), (np.float64, 1003, 37, 512), (np.float64, 4099, 33, 1024), (np.float64, 2051, 5, 2048),
+    (np.float32, 1048583, 1, 1024), (np.float32, 40009, 27, 1000), (np.float32, 131075, 9, 2048), (np.float32, 500, 9, 2048),
+])
+def test_two_byte_bin_ids_count_the_proposals_below(lb, dtype, N, F, S):
+    """The id of a value is the number of proposals below it (0 for a NaN); the padding columns are zero."""
+    from legateboost_b200 import stages
+
+    rs = np.random.RandomState(F)
+    X = rs.normal(size=(N, F)).astype(dtype)
+    X[rs.random((N, F)) < 0.01] = np.inf
+    X[rs.random((N, F)) < 0.01] = -np.inf
+    sample = dev(rs.normal(size=(4000, F)).astype(dtype))
+    proposals, row_ptr = stages.split_proposals(sample, S, 3)
+    p, rp = proposals.cpu().numpy(), row_ptr.cpu().numpy()
+    X[: min(N, 300)] = p[rp[:-1]]  # values that are proposals
+    X[rs.random((N, F)) < 0.01] = np.nan
+    got = stages.bin_matrix(dev(X), proposals, row_ptr, 2).cpu().numpy()
+    assert not got[:, F:].any()
+    for f in range(F):
+        x = X[:, f]
+        want = np.where(np.isnan(x), 0, np.searchsorted(p[rp[f]:rp[f + 1]], x, side="left"))
+        assert np.array_equal(got[:, f], want), f
