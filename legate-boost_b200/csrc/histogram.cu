@@ -980,13 +980,17 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
 // is zeroed as it is read.
 //
 // Measured (B200, kernel time per level): 500 x 10 float32, 256 bins: 13 -> 9.5 us; 200k x 50: 24 -> 23 us;
-// 300k x 37, 512 bins (64-bit global atomics before): 267 -> 36 us.
+// 300k x 37, 512 bins (64-bit global atomics before): 267 -> 29 us.
 constexpr int kTileFeatures = 8;
 constexpr int kTileMinRows  = 1024;
 constexpr int kTileItemsPerSm = 1;
+// (one block's worth of pieces per SM: more threads only help where the histograms take longer to zero and flush;
+// 200k x 50, 256 bins: 23.5 us per level with 256 threads, 24.4 with 1024; 300k x 37, 512 bins: 35 and 29)
+constexpr int kTileThreads     = 256;
+constexpr int kTileWideThreads = 1024;
 
 template <typename BinT, int kBins, int kThreads>
-__global__ void __launch_bounds__(kThreads, kBins <= 512 ? 1536 / kThreads : 1)
+__global__ void __launch_bounds__(kThreads, 1536 / kThreads)
   k_hist_tile(const HistParams p)
 {
   using A = Acc<false>;
@@ -1179,13 +1183,13 @@ HistLaunch PickHistKernel(int bin_bytes, int mb, bool float_mode, RowOrder order
     h.smem_path    = false;
     h.width        = 1;
     const int bins = mb <= 256 ? 256 : mb <= 512 ? 512 : mb <= 1024 ? 1024 : 2048;
-    h.threads      = bins == 2048 ? 1024 : bins == 1024 ? 512 : 256;
+    h.threads      = bins <= 256 ? kTileThreads : kTileWideThreads;
     h.smem         = static_cast<size_t>(bins) * kTileFeatures * 8;
-    if (bin_bytes == 1) h.fn = k_hist_tile<uint8_t, 256, 256>;
-    else if (bins == 256) h.fn = k_hist_tile<uint16_t, 256, 256>;
-    else if (bins == 512) h.fn = k_hist_tile<uint16_t, 512, 256>;
-    else if (bins == 1024) h.fn = k_hist_tile<uint16_t, 1024, 512>;
-    else h.fn = k_hist_tile<uint16_t, 2048, 1024>;
+    if (bin_bytes == 1) h.fn = k_hist_tile<uint8_t, 256, kTileThreads>;
+    else if (bins == 256) h.fn = k_hist_tile<uint16_t, 256, kTileThreads>;
+    else if (bins == 512) h.fn = k_hist_tile<uint16_t, 512, kTileWideThreads>;
+    else if (bins == 1024) h.fn = k_hist_tile<uint16_t, 1024, kTileWideThreads>;
+    else h.fn = k_hist_tile<uint16_t, 2048, kTileWideThreads>;
   } else if (h.smem_path) {
     h.smem = HistSmemBytes(h.width);
     h.fn = h.width == 2 ? (float_mode ? SmemKernel<true, 2>(order) : SmemKernel<false, 2>(order))
