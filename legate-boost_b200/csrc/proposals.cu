@@ -461,6 +461,179 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
   if (turn < n) do_turn(std::true_type());
 }
 
+// One-byte ids of float32 values, up to 256 proposals per feature: the search starts from a table lookup.
+//
+// k_bin_smem is bound by its issue slots and the load/store pipe (72 % each): five instructions for the two
+// levels in registers and three more and a pass for each of the other six.  Here a value is first mapped to one of
+// 512 buckets by t = rint(clamp(x s + b)), of which a table holds the number of proposals in the buckets below; since
+// the map never decreases, those are below x and the proposals of the buckets above are not, and what is left to
+// search are the proposals of x's own bucket.  s and b spread the buckets evenly from the fifth proposal to the
+// fifth from the end (beyond them lie four proposals and any outliers).  A block looks how many proposals share a
+// bucket in its features at worst and takes three steps of the search (up to 7: uniform and normal columns), four (up
+// to 15) or, where the values crowd together more, the whole search without the table.  A NaN ends in bucket 0 and
+// fails every comparison: id 0, as in the other kernels.
+//
+// Blocks of 16 warps share the proposals (34 KB) and the buckets (16 KB); two fit an SM with 64 registers a
+// thread.  The bucket table is [bucket][lane] bytes: a lookup is two passes, four lanes share a word's column.
+// 10M x 64: 1047 -> 841 us, 1M x 100: 285 -> 217 us; 200k x 50 stays at 42 us, filling the tables and two turns of a warp.
+constexpr int kBuckets    = 512;
+constexpr int kLutThreads = 512;
+constexpr int kLutRows    = 256 + 16;  // of the table: the last steps may look beyond the last proposal
+constexpr size_t kLutSmem = sizeof(float) * kGroup * kLutRows + kBuckets * kGroup + (kLutThreads / 32) * kGroup * kBinTilePitch;
+
+template <bool kCopyT>
+__global__ void __launch_bounds__(kLutThreads, 2)
+  k_bin_lut(const float* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const float* __restrict__ proposals,
+            int64_t cut_stride, const int32_t* __restrict__ row_ptr, uint8_t* __restrict__ bins, uint8_t* __restrict__ bins_t, int64_t pitch_t)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_n[kGroup];
+  __shared__ float2 s_map[kGroup];
+  float* sp          = reinterpret_cast<float*>(smem_raw);
+  unsigned char* lut = smem_raw + sizeof(float) * kGroup * kLutRows;
+  const int f0   = blockIdx.y * kGroup;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kLutThreads / 32;
+  if (threadIdx.x < kGroup) s_n[threadIdx.x] = f0 + threadIdx.x < F ? row_ptr[f0 + threadIdx.x + 1] - row_ptr[f0 + threadIdx.x] : 0;
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < kLutRows * kGroup; idx += kLutThreads) {
+    const int j = idx >> 5, f = f0 + (idx & 31);
+    sp[idx]     = j < s_n[idx & 31] ? proposals[(cut_stride > 0 ? f * cut_stride : row_ptr[f]) + j] : INFINITY;
+  }
+  __syncthreads();
+  if (threadIdx.x < kGroup) {
+    const int n = s_n[threadIdx.x], end = n >= 32 ? 4 : 0;
+    float s = 0.0f, b = 0.0f;
+    if (n >= 3) {  // (the last proposal is +inf)
+      const float lo = sp[end * kGroup + threadIdx.x], hi = sp[(n - 2 - end) * kGroup + threadIdx.x];
+      s = (kBuckets - 3) / (hi - lo);
+      b = 1.0f - lo * s;
+      if (!(s > 0.0f) || !(s < INFINITY) || !(fabsf(b) < INFINITY)) s = b = 0.0f;  // all in one bucket
+    }
+    s_map[threadIdx.x] = make_float2(s, b);
+  }
+  __syncthreads();
+  const float2 map = s_map[lane];
+  // the bucket of x plus the bits of 2^23
+  auto bucket_bits = [&](float x) {
+    return __float_as_uint(fminf(fmaxf(__fmaf_rn(x, map.x, map.y), 0.0f), static_cast<float>(kBuckets - 1)) + 8388608.0f);
+  };
+  int crowd = 0;  // 1: more than 7 of a feature's proposals share a bucket, 2: more than 15, or they are not in order
+  {
+    auto at_of  = [&](int j) { return static_cast<int>(bucket_bits(sp[j * kGroup + lane]) & (kBuckets - 1)); };
+    const int n = s_n[lane];
+    for (int j = warp; j < n; j += kWarps) {
+      const int at = at_of(j);
+      for (int k = j > 0 ? at_of(j - 1) + 1 : 0; k <= at; ++k) lut[k * kGroup + lane] = static_cast<unsigned char>(j);
+      if (j == n - 1)  // (+inf is in the last bucket, unless all are in the first)
+        for (int k = at + 1; k < kBuckets; ++k) lut[k * kGroup + lane] = 0;
+      // the table is only right for proposals in order that end in +inf (a NaN among the samples is neither)
+      const float v = sp[j * kGroup + lane];
+      if (j == n - 1 ? v != INFINITY : !(v < sp[(j + 1) * kGroup + lane])) crowd |= 2;
+      if (j >= 7 && at_of(j - 7) == at) crowd |= 1;
+      if (j >= 15 && at_of(j - 15) == at) crowd |= 2;
+    }
+    if (n == 0)
+      for (int k = warp; k < kBuckets; k += kWarps) lut[k * kGroup + lane] = 0;
+  }
+  const int most = __syncthreads_or(crowd & 2) ? 2 : __syncthreads_or(crowd & 1) ? 1 : 0;
+  // Lanes beyond the last feature read the last feature's values (in bounds); their column of the
+  // table is all +inf, so their ids are 0.
+  const bool active = f0 + lane < F;
+  constexpr unsigned kPitch = kGroup * sizeof(float);
+  const unsigned col_s  = static_cast<unsigned>(__cvta_generic_to_shared(sp + lane));
+  const unsigned lut_s  = static_cast<unsigned>(__cvta_generic_to_shared(lut + lane)) - 0x4b000000u * kGroup;  // (the bits of 2^23)
+  const unsigned tile_s = static_cast<unsigned>(__cvta_generic_to_shared(lut + kBuckets * kGroup + warp * (kGroup * kBinTilePitch)));
+  const int pitch   = static_cast<int>(gridDim.y) * kGroup;
+  constexpr int U   = 8;  // rows per warp in flight
+  const int n       = static_cast<int>(n_rows);
+  const int ld      = static_cast<int>(ldx);
+  constexpr int kSubs = kBinTileRows / U;
+  constexpr int kTurn = kBinTileRows;
+  const int hop     = static_cast<int>(gridDim.x) * kWarps * kTurn;  // rows from one turn of a warp to the next
+  int turn          = (blockIdx.x * kWarps + warp) * kTurn;
+  const float* xcol = X + (active ? f0 + lane : F - 1);
+  uint8_t* ocol     = bins + f0 + lane;
+  // the values of the warp's next eight rows are loaded while the current eight are searched
+  auto load_rows = [&](int first, float (&x)[U]) {
+    const float* src = xcol + static_cast<int64_t>(first) * ld;
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = LdgStream(src + static_cast<int64_t>(u) * ld);
+  };
+  auto load_rows_checked = [&](int first, float (&x)[U]) {
+    const float* src = xcol + static_cast<int64_t>(first) * ld;
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = first + u < n ? LdgStream(src + static_cast<int64_t>(u) * ld) : -INFINITY;
+  };
+  float xn[U];
+  if (turn < n) load_rows_checked(turn, xn);
+  // one turn; checked: the turn may reach beyond the last row; levels: steps of the search, 8 = without the buckets
+  auto do_turn = [&](auto checked, auto levels) {
+    constexpr bool kChecked = decltype(checked)::value;
+    constexpr int kLevels   = decltype(levels)::value;
+#pragma unroll 2
+    for (int sub = 0; sub < kSubs; ++sub) {
+      const int base = turn + sub * U;
+      float x[U];
+      unsigned pos[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[u] = xn[u];
+      {
+        const int nb = sub + 1 < kSubs ? base + U : turn + hop;
+        if (sub + 1 < kSubs && !kChecked) load_rows(nb, xn);
+        else if (nb < n) load_rows_checked(nb, xn);
+      }
+      if (kLevels == 8) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) pos[u] = col_s;
+      } else {
+        unsigned first[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          asm volatile("ld.shared.u8 %0, [%1];\n" : "=r"(first[u]) : "r"(lut_s + bucket_bits(x[u]) * kGroup));
+#pragma unroll
+        for (int u = 0; u < U; ++u) pos[u] = col_s + first[u] * kPitch;
+      }
+      SearchLevels<float, U, kLevels - 1, kPitch>::run(pos, x);
+      unsigned id[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) id[u] = (pos[u] - col_s) / kPitch;
+      uint8_t* orow = ocol + static_cast<int64_t>(base) * pitch;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (!kChecked || base + u < n) orow[u * pitch] = static_cast<uint8_t>(id[u]);
+      if (kCopyT) {
+        const unsigned lo = id[0] | (id[1] << 8) | (id[2] << 16) | (id[3] << 24);
+        const unsigned hi = id[4] | (id[5] << 8) | (id[6] << 16) | (id[7] << 24);
+        asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(tile_s + lane * kBinTilePitch + sub * U), "r"(lo), "r"(hi)
+                     : "memory");
+      }
+    }
+    if (kCopyT) {
+      // the tile leaves feature by feature, as in k_bin_smem
+      __syncwarp();
+      const int w    = lane & 15;
+      const bool in  = turn + 4 * w < pitch_t;
+#pragma unroll 4
+      for (int i = 0; i < kGroup / 2; ++i) {
+        const int fl = 2 * i + (lane >> 4);
+        unsigned v;
+        asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(tile_s + fl * kBinTilePitch + 4 * w));
+        if (in && f0 + fl < F)
+          *reinterpret_cast<unsigned*>(bins_t + static_cast<int64_t>(f0 + fl) * pitch_t + turn + 4 * w) = v;
+      }
+      __syncwarp();
+    }
+  };
+  auto all_turns = [&](auto levels) {
+    for (; turn + kTurn <= n; turn += hop) do_turn(std::false_type(), levels);
+    if (turn < n) do_turn(std::true_type(), levels);
+  };
+  if (most == 0) all_turns(std::integral_constant<int, 3>());
+  else if (most == 1) all_turns(std::integral_constant<int, 4>());
+  else all_turns(std::integral_constant<int, 8>());
+}
+
 // Two-byte ids, more proposals than k_bin_smem's table of 32 features holds: a table of as many features
 // (16, 8 or 4) as fill 64 KB, three blocks per SM.  A lane has one feature and eight consecutive rows, which leave as
 // one 16-byte store of the feature-major copy; the 32 / kFeatures row groups of a warp may meet in a bank
@@ -705,6 +878,19 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
                                                        pitch_t);                                          \
     }                                                                                                     \
   } while (0)
+  if constexpr (sizeof(T) == 4) {
+    if (bin_bytes == 1 && log2p == 8) {
+      auto fn = bins_t != nullptr ? k_bin_lut<true> : k_bin_lut<false>;
+      LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLutSmem)));
+      constexpr int64_t kRows = kLutThreads / 32 * kBinTileRows;  // of a block's first turn
+      dim3 grid = make_grid(2);
+      grid.x    = static_cast<unsigned>(std::min<int64_t>(grid.x, (n_rows + kRows - 1) / kRows));
+      fn<<<grid, kLutThreads, kLutSmem, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, static_cast<uint8_t*>(bins),
+                                                  static_cast<uint8_t*>(bins_t), pitch_t);
+      LBK_LAUNCH_CHECK();
+      return;
+    }
+  }
   if (bin_bytes == 2 && !use_smem && need <= 2048 && n_rows * F >= kWideMinCells<T>) {
     auto wide = [&](auto log2p_, auto copy_) {
       constexpr int L    = decltype(log2p_)::value;

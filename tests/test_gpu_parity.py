@@ -979,3 +979,38 @@ def test_two_byte_bin_ids_count_the_proposals_below(lb, dtype, N, F, S):
         x = X[:, f]
         want = np.where(np.isnan(x), 0, np.searchsorted(p[rp[f]:rp[f + 1]], x, side="left"))
         assert np.array_equal(got[:, f], want), f
+
+
+@pytest.mark.parametrize("N,F,S", [(1, 1, 256), (63, 3, 100), (1025, 33, 256), (40007, 64, 256), (5000, 9, 65)])
+@pytest.mark.parametrize("kind", ["uniform", "normal", "lognormal", "crowded", "few", "outliers", "negative_infinity", "nan"])
+def test_one_byte_bin_ids_count_the_proposals_below(lb, kind, N, F, S):
+    """Whatever the distribution: columns for which the search starts from the bucket table, with three steps or four,
+    and columns whose proposals crowd in few buckets or are not in order."""
+    from legateboost_b200 import stages
+
+    rs = np.random.RandomState(N % 89 + S)
+    make = {
+        "uniform": lambda n: rs.random((n, F)), "normal": lambda n: rs.normal(size=(n, F)),
+        "lognormal": lambda n: np.exp(1.5 * rs.normal(size=(n, F))), "crowded": lambda n: np.exp(8 * rs.normal(size=(n, F))),
+        "few": lambda n: np.round(4 * rs.normal(size=(n, F))), "outliers": lambda n: rs.normal(size=(n, F)) * np.where(rs.random((n, F)) < 0.005, 1e30, 1),
+        "negative_infinity": lambda n: np.where(rs.random((n, F)) < 0.01, -np.inf, rs.normal(size=(n, F))),
+        "nan": lambda n: np.where(rs.random((n, F)) < 0.01, np.nan, rs.normal(size=(n, F))),
+    }[kind]
+    proposals, row_ptr = stages.split_proposals(dev(make(3000).astype(np.float32)), S, 3)
+    p, rp = proposals.cpu().numpy(), row_ptr.cpu().numpy()
+    X = make(N).astype(np.float32)
+    X[rs.random((N, F)) < 0.02] = np.inf
+    X[rs.random((N, F)) < 0.02] = -np.inf
+    for i in range(min(N, 200)):  # the proposals themselves and their neighbours
+        at = rp[:-1] + i % np.diff(rp)
+        X[i] = p[at] if i % 3 == 0 else np.nextafter(p[at], np.float32(np.inf if i % 3 == 1 else -np.inf))
+    X[rs.random((N, F)) < 0.02] = np.nan
+    got = stages.bin_matrix(dev(X), proposals, row_ptr, 1).cpu().numpy()
+    assert not got[:, F:].any()
+    for f in range(F):
+        table = np.full(256, np.inf, dtype=np.float32)
+        table[: rp[f + 1] - rp[f]] = p[rp[f]:rp[f + 1]]
+        want = np.zeros(N, dtype=np.int64)
+        for step in (128, 64, 32, 16, 8, 4, 2, 1):  # (also for a table with a NaN in it, where the order of probes matters)
+            want += np.where(table[want + step - 1] < X[:, f], step, 0)
+        assert np.array_equal(got[:, f], want), f
