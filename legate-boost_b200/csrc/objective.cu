@@ -14,8 +14,6 @@
 namespace lbk {
 namespace {
 
-constexpr int kMaxClassesInRegisters = 32;
-
 __global__ void __launch_bounds__(256)
   k_gradient_squared_error(const double* __restrict__ raw, const double* __restrict__ y, int64_t n, double lr,
                            double* __restrict__ g, double* __restrict__ h)
@@ -38,27 +36,66 @@ __global__ void __launch_bounds__(256)
   h[i] = v.y;
 }
 
-// one thread per row; the exponentials of up to 32 classes stay in registers, more are recomputed
-__global__ void __launch_bounds__(256)
-  k_gradient_softmax(const double* __restrict__ raw, const double* __restrict__ label, int64_t n_rows, int K, double lr,
+// A block takes `rows` rows: they come in and their gradients go out as whole lines, through shared memory, and
+// one thread per row makes the exponentials and their sum there.  Bound by HBM (24 bytes per value); a thread that
+// reads and writes its own row of K values touches a line per value: 1M x 10: 172 us, here 71 us.
+// Shared memory: exponentials [rows][K | 1] (an odd pitch), sums [rows], classes [rows].
+constexpr int kSoftmaxThreads = 256;
+size_t SoftmaxRowBytes(int K) { return sizeof(double) * ((K | 1) + 1) + sizeof(int); }
+
+__global__ void __launch_bounds__(kSoftmaxThreads)
+  k_gradient_softmax(const double* __restrict__ raw, const double* __restrict__ label, int64_t n_rows, int K, int rows, double lr,
                      double* __restrict__ g, double* __restrict__ h)
+{
+  extern __shared__ double s_e[];
+  const int pitch    = K | 1;
+  double* s_div      = s_e + rows * pitch;
+  int* s_cls         = reinterpret_cast<int*>(s_div + rows);
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * rows;
+  const int here     = static_cast<int>(n_rows - row0 < rows ? n_rows - row0 : rows);
+  const int64_t at0  = row0 * K;
+  for (int i = threadIdx.x; i < here * K; i += kSoftmaxThreads) {
+    const int row = i / K;
+    s_e[row * pitch + i - row * K] = raw[at0 + i];
+  }
+  __syncthreads();
+  for (int row = threadIdx.x; row < here; row += kSoftmaxThreads) {
+    double* e = s_e + row * pitch;
+    double s  = e[0];
+    for (int k = 1; k < K; ++k) s = fmax(s, e[k]);
+    double div = 0.0;
+    for (int k = 0; k < K; ++k) {
+      const double v = exp(e[k] - s);
+      e[k]           = v;
+      div += v;
+    }
+    s_div[row] = div;
+    s_cls[row] = static_cast<int>(label[row0 + row]);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < here * K; i += kSoftmaxThreads) {
+    const int row  = i / K, k = i - row * K;
+    const double p = s_e[row * pitch + k] / s_div[row];
+    g[at0 + i]     = (k == s_cls[row] ? p - 1.0 : p) * lr;
+    h[at0 + i]     = fmax(p * (1.0 - p), 1e-8);
+  }
+}
+
+// more classes than shared memory takes 32 rows of: one thread per row
+__global__ void __launch_bounds__(256)
+  k_gradient_softmax_wide(const double* __restrict__ raw, const double* __restrict__ label, int64_t n_rows, int K, double lr,
+                          double* __restrict__ g, double* __restrict__ h)
 {
   const int64_t row = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (row >= n_rows) return;
   const double* r = raw + row * K;
   double s        = r[0];
   for (int k = 1; k < K; ++k) s = fmax(s, r[k]);
-  double e[kMaxClassesInRegisters];
   double div = 0.0;
-  for (int k = 0; k < K; ++k) {
-    const double v = exp(r[k] - s);
-    if (k < kMaxClassesInRegisters) e[k] = v;
-    div += v;
-  }
+  for (int k = 0; k < K; ++k) div += exp(r[k] - s);
   const int cls = static_cast<int>(label[row]);
   for (int k = 0; k < K; ++k) {
-    const double v = k < kMaxClassesInRegisters ? e[k] : exp(r[k] - s);
-    const double p = v / div;
+    const double p = exp(r[k] - s) / div;
     g[row * K + k] = (k == cls ? p - 1.0 : p) * lr;
     h[row * K + k] = fmax(p * (1.0 - p), 1e-8);
   }
@@ -76,8 +113,13 @@ void Gradient(int objective, const double* raw_pred, const double* y, int64_t n_
   } else if (n_outputs == 1) {
     k_gradient_logloss_binary<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(raw_pred, y, n, learning_rate, g, h);
   } else {
-    k_gradient_softmax<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(raw_pred, y, n_rows, n_outputs,
-                                                                                       learning_rate, g, h);
+    const int rows = static_cast<int>(std::min<size_t>(kSoftmaxThreads, 48 * 1024 / SoftmaxRowBytes(n_outputs)) / 32 * 32);
+    if (rows > 0)
+      k_gradient_softmax<<<static_cast<unsigned>((n_rows + rows - 1) / rows), kSoftmaxThreads, rows * SoftmaxRowBytes(n_outputs), stream>>>(
+        raw_pred, y, n_rows, n_outputs, rows, learning_rate, g, h);
+    else
+      k_gradient_softmax_wide<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(raw_pred, y, n_rows, n_outputs,
+                                                                                             learning_rate, g, h);
   }
   LBK_LAUNCH_CHECK();
 }

@@ -1014,3 +1014,22 @@ def test_one_byte_bin_ids_count_the_proposals_below(lb, kind, N, F, S):
         for step in (128, 64, 32, 16, 8, 4, 2, 1):  # (also for a table with a NaN in it, where the order of probes matters)
             want += np.where(table[want + step - 1] < X[:, f], step, 0)
         assert np.array_equal(got[:, f], want), f
+
+
+@pytest.mark.parametrize("N,K", [(1, 3), (255, 23), (257, 24), (1000, 186), (70, 187), (70, 300)])
+def test_softmax_gradients_of_whole_and_partial_tiles(lb, N, K):
+    """The tiled kernel (256 rows down to 32 per block) and the one for more classes than it takes."""
+    from legateboost_b200 import estimator as E
+
+    rs = np.random.RandomState(K)
+    est = lb.LBRegressor(learning_rate=0.3)
+    est._obj = E._LogLoss()
+    raw, y = rs.normal(size=(N, K)) * 5, rs.randint(0, K, size=(N, 1)).astype(np.float64)
+    g, h = est._weighted_gradient(dev(y), dev(raw))
+    e = np.exp(raw - raw.max(axis=1, keepdims=True))
+    p = e / e.sum(axis=1, keepdims=True)
+    want_g = p.copy()
+    want_g[np.arange(N), y[:, 0].astype(int)] -= 1.0
+    tol = (K + 8) * 2.3e-16  # exp, K additions, a division, a product
+    assert np.allclose(g.cpu().numpy(), want_g * 0.3, rtol=tol, atol=tol)
+    assert np.allclose(h.cpu().numpy(), np.maximum(p * (1 - p), 1e-8), rtol=tol, atol=tol)
