@@ -178,6 +178,28 @@ __device__ inline int ChunkRowsOf(long long total, int nonempty_nodes, int GK, i
   return static_cast<int>(ch < (1ll << 30) ? ch : (1ll << 30));
 }
 
+// The same for k_hist_tile with copies, whose pieces should fill the SMs once (or a whole number of times: 154 pieces
+// on 148 SMs take as long as 296): pieces of ch rows are fewer than total / ch + nodes, so that w x SMs pieces are
+// kept by ch = total / (w x SMs / GK - nodes); of the turns w the one whose rows (and fixed cost, about as much as
+// kTileFixedRows rows) come to the least.  Nodes no longer than ch stay whole.
+constexpr int kTileFixedRows = 1500;
+__device__ inline int TileChunkRows(long long total, int nodes, int largest, int GK, int sms, int min_chunk)
+{
+  long long best = 1ll << 30, best_cost = 1ll << 60;
+  for (int w = 1; w <= 4; ++w) {
+    const long long pieces = static_cast<long long>(w) * sms / GK;
+    if (pieces < nodes) continue;
+    long long ch = pieces > nodes ? (total + pieces - nodes - 1) / (pieces - nodes) : largest;
+    ch           = min(max(ch, static_cast<long long>(min_chunk)), static_cast<long long>(max(largest, min_chunk)));
+    const long long cost = w * (ch + kTileFixedRows);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best      = ch;
+    }
+  }
+  return static_cast<int>(best);
+}
+
 // Single block: how the rows of the built nodes are handed to the resident blocks on this level.
 //
 // A unit of work is (rows, group set, output), GK = group sets x outputs per row.
@@ -194,28 +216,33 @@ __device__ inline int ChunkRowsOf(long long total, int nonempty_nodes, int GK, i
 // resident blocks, else equal chunks of about total / resident rows whose sums are added to the
 // histogram with 64-bit atomics; blocks draw (chunk, group set, output) tickets from a counter.
 __global__ void __launch_bounds__(1024)
-  k_hist_plan(const __grid_constant__ HistParams p, int GK, int resident, int min_chunk, int32_t* __restrict__ chunk_off,
+  k_hist_plan(const __grid_constant__ HistParams p, int GK, int resident, int min_chunk, bool whole_turns, int32_t* __restrict__ chunk_off,
               int32_t* __restrict__ wpre, int32_t* __restrict__ plan)
 {
   __shared__ long long red[32];
   __shared__ long long wsum[32];
   __shared__ long long carry;
   __shared__ long long total_s;
-  __shared__ int ch_s, nodes_s;
+  __shared__ int ch_s, nodes_s, largest_s;
   const int n_nodes = p.n_nodes;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
   auto rows_of = [&](int j) -> int { return BuiltRows(p, j); };
   for (int i = tid; i < p.n_arrive; i += blockDim.x) p.arrive[i] = 0u;
   long long rows = 0, nonempty = 0;
+  int largest = 0;
+  if (tid == 0) largest_s = 0;
   for (int j = tid; j < n_nodes; j += blockDim.x) {
     const int r = rows_of(j);
     rows += r;
     nonempty += r > 0;
+    largest = max(largest, r);
   }
   rows += nonempty << 40;
   for (int off = 16; off >= 1; off >>= 1) rows += __shfl_down_sync(0xffffffffu, rows, off);
   if (lane == 0) red[warp] = rows;
   __syncthreads();
+  largest = __reduce_max_sync(0xffffffffu, largest);
+  if (lane == 0) atomicMax(&largest_s, largest);
   if (tid == 0) {
     long long total = 0;
     for (int w = 0; w < n_warps; ++w) total += red[w];
@@ -270,14 +297,14 @@ __global__ void __launch_bounds__(1024)
 
   // tickets
   if (tid == 0) {
-    ch_s = ChunkRowsOf(total, nodes_s, GK, resident, min_chunk);
+    ch_s = whole_turns ? TileChunkRows(total, nodes_s, largest_s, GK, resident, min_chunk) : ChunkRowsOf(total, nodes_s, GK, resident, min_chunk);
   }
   __syncthreads();
   const int ch = ch_s;
   scan_nodes(
     [&](int j) -> long long {
       const int r = rows_of(j);
-      return r > 0 ? (r + ch - 1) / ch : 0;
+      return r > 0 ? (r - 1) / ch + 1 : 0;
     },
     [&](int j, long long incl) { chunk_off[j + 1] = static_cast<int>(incl); });
   if (tid == 0) {
@@ -297,7 +324,7 @@ struct PlanView {
   const int32_t* off;  // [n_nodes + 1]: built rows before each node (ranges) or chunks before each node (tickets)
   int rows_safe, range_rows, ranges, total_chunks;
 };
-template <int kThreads>
+template <int kThreads, bool kWholeTurns = false>
 __device__ inline PlanView PlanInside(const HistParams& p, int GK, int resident, int min_chunk, bool ranges_too,
                                       int32_t* s_off /* [kPlanNodes + 1] */, int* s_tmp /* [kThreads / 32] */)
 {
@@ -355,9 +382,22 @@ __device__ inline PlanView PlanInside(const HistParams& p, int GK, int resident,
   if (ranges_too) RangesOf(p, total, GK, resident, v.range_rows, v.ranges);
   v.total_chunks = 0;
   if (v.range_rows == 0) {
-    const int ch = ChunkRowsOf(total, nonempty, GK, resident, min_chunk);
+    int ch;
+    if (kWholeTurns) {
+      int largest = 0;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) c[i] = c[i] > 0 ? (c[i] + ch - 1) / ch : 0;
+      for (int i = 0; i < kPer; ++i) largest = max(largest, c[i]);
+      largest = __reduce_max_sync(0xffffffffu, largest);
+      if (lane == 0) s_tmp[warp] = largest;
+      __syncthreads();
+      for (int w = 0; w < kThreads / 32; ++w) largest = max(largest, s_tmp[w]);
+      __syncthreads();
+      ch = TileChunkRows(total, nonempty, largest, GK, resident, min_chunk);
+    } else {
+      ch = ChunkRowsOf(total, nonempty, GK, resident, min_chunk);
+    }
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) c[i] = c[i] > 0 ? (c[i] - 1) / ch + 1 : 0;
     scan();
     v.total_chunks = s_off[n];
   }
@@ -972,29 +1012,30 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
 // k_hist_smem keeps 128 KB of histograms per block: clearing, turning and merging them costs 10 - 15 us per
 // launch however few rows there are, and cutting a level into the pieces that fill the chip multiplies
 // the 64-bit atomics of the merge.  Here a unit is (piece of a node, eight features, output) with
-// kBins x 8 x 8 bytes of histograms (16 KB for 256 bins), several blocks per SM; a level is cut into fewer
-// pieces of rows because the feature groups fill the chip too.  A lane owns a row: one 8-byte (16-byte for
-// two-byte bins) load brings its eight bin ids, in step j of eight it handles feature (j xor lane % 8),
-// so that the 32 lanes of a warp spread over all banks (two lanes meet on average once per step).
+// kBins x 8 x 8 bytes of histograms (16 KB for 256 bins), once or four times; a level is cut into fewer pieces of
+// rows because the feature groups fill the chip too (with four copies one piece per SM, TileChunkRows; two cost more
+// atomics than they give, 200k x 50: 111 -> 132 us per tree).  A lane owns a row: one 8-byte (16-byte for
+// two-byte bins) load brings its eight bin ids, in step j of eight it handles feature (j xor lane % 8).
 // Piece sums go out with plain stores if the node is one piece, else with 64-bit atomics; the histogram
 // is zeroed as it is read.
 //
-// Measured (B200, kernel time per level): 500 x 10 float32, 256 bins: 13 -> 9.5 us; 200k x 50: 24 -> 23 us;
-// 300k x 37, 512 bins (64-bit global atomics before): 267 -> 29 us.
+// Measured (B200, kernel time per level): 200k x 50, 256 bins: 23.3 us with one copy and 256 threads, 16.3 with four
+// copies, pieces that fill the SMs once and 512 threads (256 threads: 25.3, 1024: 16.9); 300k x 37, 512 bins, 1024
+// threads: 29 -> 22.7 us (64-bit global atomics at first: 267).
 constexpr int kTileFeatures = 8;
 constexpr int kTileMinRows  = 1024;
 constexpr int kTileItemsPerSm = 1;
-// (one block's worth of pieces per SM: more threads only help where the histograms take longer to zero and flush;
-// 200k x 50, 256 bins: 23.5 us per level with 256 threads, 24.4 with 1024; 300k x 37, 512 bins: 35 and 29)
-constexpr int kTileThreads     = 256;
-constexpr int kTileWideThreads = 1024;
 
-template <typename BinT, int kBins, int kThreads>
-__global__ void __launch_bounds__(kThreads, 1536 / kThreads)
+// kCopies: 1, or 4 copies of the histograms, one per eight lanes of a warp: the 32 lanes then update 32 different
+// banks, where with one copy four lanes share eight banks and a reduction is three passes on average; but all copies
+// are read and cleared for every piece.
+template <typename BinT, int kBins, int kThreads, int kCopies>
+__global__ void __launch_bounds__(kThreads, kThreads == 256 ? 6 : 1)
   k_hist_tile(const HistParams p)
 {
   using A = Acc<false>;
-  extern __shared__ __align__(128) int s_hist[];  // [2][kBins][8]
+  constexpr int kRow = kTileFeatures * kCopies;  // words of a bin
+  extern __shared__ __align__(128) int s_hist[];  // [2][kBins][copies][8]
   __shared__ int32_t s_off[kPlanNodes + 1];
   __shared__ int s_tmp[32];
   __shared__ GPairI64* s_base[kTileFeatures];
@@ -1004,19 +1045,20 @@ __global__ void __launch_bounds__(kThreads, 1536 / kThreads)
   const int FG  = (p.F + kTileFeatures - 1) / kTileFeatures, Q = FG * p.K;
   PlanView pv;
   if (p.plan == nullptr) {
-    pv = PlanInside<kThreads>(p, Q, p.tile_items, kTileMinRows, false, s_off, s_tmp);
+    pv = PlanInside<kThreads, kCopies != 1>(p, Q, p.tile_items, kTileMinRows, false, s_off, s_tmp);
   } else {
     pv.rows_safe    = p.plan[3];
     pv.total_chunks = p.plan[1];
     pv.off          = p.chunk_off;
   }
   const int mb        = p.mb_ptr != nullptr ? min(p.mb, *p.mb_ptr) : p.mb;
-  const int words     = mb * kTileFeatures;
+  const int words     = mb * kTileFeatures;  // of a histogram, copies added up
   const int64_t pitch = static_cast<int64_t>(p.G) * kGroup;
   const int2* gpair   = static_cast<const int2*>(p.gpair);
   const bool by_pos   = p.pairs_by_position != 0 || p.row_index == nullptr;
-  for (int i = tid; i < words; i += kThreads) s_hist[i] = s_hist[kBins * kTileFeatures + i] = 0;
-  const unsigned lane_word = SmemAddr(s_hist) + (lane & 7) * 4;
+  for (int i = tid; i < mb * kRow / 4; i += kThreads)
+    reinterpret_cast<int4*>(s_hist)[i] = reinterpret_cast<int4*>(s_hist + kBins * kRow)[i] = make_int4(0, 0, 0, 0);
+  const unsigned lane_word = SmemAddr(s_hist) + (lane & (kRow - 1)) * 4;
   const unsigned swap = lane & 7, bsel = swap & 3;
   // one-byte ids: step j reads byte j of the pair of words permuted by `swap`; two-byte ids likewise
   const unsigned perm = bsel == 0 ? 0x3210u : bsel == 1 ? 0x2301u : bsel == 2 ? 0x1032u : 0x0123u;
@@ -1093,9 +1135,9 @@ __global__ void __launch_bounds__(kThreads, 1536 / kThreads)
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const unsigned addr = (lane_word ^ (4u * j)) + bin[j] * (kTileFeatures * 4);
+        const unsigned addr = (lane_word ^ (4u * j)) + bin[j] * (kRow * 4);
         A::red_shared(addr, x.v.x);
-        A::template red_shared_at<kBins * kTileFeatures * 4>(addr, x.v.y);
+        A::template red_shared_at<kBins * kRow * 4>(addr, x.v.y);
       }
     };
     bool atomics = pc.pieces > 1;
@@ -1123,10 +1165,16 @@ __global__ void __launch_bounds__(kThreads, 1536 / kThreads)
       }
       __syncthreads();
       for (int i = tid; i < words; i += kThreads) {
-        const int g = s_hist[i], h = s_hist[kBins * kTileFeatures + i];
+        const int f = i & 7, bin = i >> 3;
+        int g = 0, h = 0;
+#pragma unroll
+        for (int c = 0; c < kCopies; ++c) {  // (neighbouring bins begin with different copies: other banks)
+          int* at = s_hist + bin * kRow + ((c + bin) & (kCopies - 1)) * kTileFeatures + f;
+          g += at[0];
+          h += at[kBins * kRow];
+          at[0] = at[kBins * kRow] = 0;
+        }
         if ((g | h) != 0) {
-          s_hist[i] = s_hist[kBins * kTileFeatures + i] = 0;
-          const int f = i & 7, bin = i >> 3;
           if (bin < s_nb[f]) {
             if (atomics) A::add_global(s_base[f] + bin, g, h);
             else A::store_global(s_base[f] + bin, g, h);
@@ -1151,12 +1199,23 @@ struct HistLaunch {
   int width;  // feature groups per unit of work
   bool smem_path;  // k_hist_smem
   bool tile;       // k_hist_tile
+  int copies = 1;  // of its histograms
 };
 
-// Matrices of up to this many cells (rows x features x outputs) take the tile form with one-byte bins: there
-// its smaller fixed cost pays for a reduction rate that is 2.6 times lower (1M x 100 x 10 outputs: 912 us per
-// level against 355 us).
-constexpr int64_t kTileMaxCells = 1 << 24;
+// Which one-byte matrices take the tile form: its fixed cost is smaller, and its gathers take more passes per update
+// (eight bin bytes per line instead of 64).  Up to kTileMaxCellsFew cells (rows x features x outputs), and with one
+// output, one rank (the atomics of a node's pieces would cross NVLink) and few units of (node, eight features) up
+// to kTileMaxCells.  Kernel time per tree of depth 7, tile form and k_hist_smem: 300k x 64: 136 and 235 us, 600k x 64:
+// 211 and 315, 400k x 128: 296 and 380, 2M x 20: 290 and 296, 1.2M x 64: 424 and 408; ten outputs, 60k x 50: 274 and
+// 264, 100k x 100: 608 and 479.  A unit's histograms are read and cleared whatever they hold: 200k x 200, 256
+// nodes: 281 us and 197, 32 nodes: 76 and 65; hence also not many units with rows in them: 60k x 256, 8 nodes: 51 and
+// 43, 64 nodes: 70 and 54 (but 15k x 256, 64 nodes, 234 rows each: 47 and 47; 30k x 200, 256 nodes: 127 and 251).
+//
+// Four copies pay where a level is cut into about one piece per SM (no more units than SMs) and has something to
+// add: 200k x 40, one node: 33 -> 24 us; 30k x 40, 32 nodes (160 units) would be 19 -> 23 us, 30k x 200, 256 nodes 127
+// -> 215, 5k x 40, one node 17.2 -> 18.7.
+constexpr int64_t kCopiesMinCells = 1 << 20;
+constexpr int64_t kTileMaxCells = 3 << 24, kTileMaxCellsFew = 1 << 24, kTileMaxCellsMany = 1 << 23;
 
 RowOrder OrderOf(const HistParams& p)
 {
@@ -1170,12 +1229,16 @@ void (*SmemKernel(RowOrder order))(HistParams)
                               : order == kPairsByPosition ? k_hist_smem<kFloat, W, kPairsByPosition> : k_hist_smem<kFloat, W, kRowsInOrder>;
 }
 
-HistLaunch PickHistKernel(int bin_bytes, int mb, bool float_mode, RowOrder order, int F, int K, int64_t n_rows, int sm_count)
+HistLaunch PickHistKernel(int bin_bytes, int mb, bool float_mode, RowOrder order, int F, int K, int64_t n_rows, int n_nodes, bool derive, int sm_count, int ranks)
 {
   const int n_groups = (F + kGroup - 1) / kGroup;
+  const int n_slots   = derive ? n_nodes / 2 : n_nodes;
+  const int64_t cells = n_rows * F * K, units = static_cast<int64_t>(n_slots) * ((F + kTileFeatures - 1) / kTileFeatures) * K;
+  const bool many     = units > sm_count && (derive ? cells / 2 : cells) >= kTileMaxCellsMany && n_rows >= int64_t{512} * n_nodes;
   HistLaunch h;
   h.smem_path = bin_bytes == 1 && mb <= kSmemBins;
-  h.tile      = !float_mode && mb <= 2048 && (bin_bytes == 2 || (h.smem_path && n_rows * F * K <= kTileMaxCells));
+  h.tile      = !float_mode && mb <= 2048 && (bin_bytes == 2 || (h.smem_path && ((cells <= kTileMaxCellsFew && !many) ||
+                                                   (K == 1 && ranks <= 1 && cells <= kTileMaxCells && units <= 2 * sm_count))));
   h.width     = h.smem_path && n_groups >= 2 ? 2 : 1;
   h.threads   = kHistThreads * h.width;
   h.smem      = 0;
@@ -1183,13 +1246,14 @@ HistLaunch PickHistKernel(int bin_bytes, int mb, bool float_mode, RowOrder order
     h.smem_path    = false;
     h.width        = 1;
     const int bins = mb <= 256 ? 256 : mb <= 512 ? 512 : mb <= 1024 ? 1024 : 2048;
-    h.threads      = bins <= 256 ? kTileThreads : kTileWideThreads;
-    h.smem         = static_cast<size_t>(bins) * kTileFeatures * 8;
-    if (bin_bytes == 1) h.fn = k_hist_tile<uint8_t, 256, kTileThreads>;
-    else if (bins == 256) h.fn = k_hist_tile<uint16_t, 256, kTileThreads>;
-    else if (bins == 512) h.fn = k_hist_tile<uint16_t, 512, kTileWideThreads>;
-    else if (bins == 1024) h.fn = k_hist_tile<uint16_t, 1024, kTileWideThreads>;
-    else h.fn = k_hist_tile<uint16_t, 2048, kTileWideThreads>;
+    h.copies  = bins <= 512 && cells >= kCopiesMinCells && (units <= sm_count || (bin_bytes == 1 && cells > kTileMaxCellsFew)) ? 4 : 1;
+    h.threads = bins > 256 ? 1024 : h.copies == 4 ? 512 : 256;
+    h.smem    = static_cast<size_t>(bins) * kTileFeatures * h.copies * 8;
+    if (bin_bytes == 1) h.fn = h.copies == 4 ? k_hist_tile<uint8_t, 256, 512, 4> : k_hist_tile<uint8_t, 256, 256, 1>;
+    else if (bins == 256) h.fn = h.copies == 4 ? k_hist_tile<uint16_t, 256, 512, 4> : k_hist_tile<uint16_t, 256, 256, 1>;
+    else if (bins == 512) h.fn = h.copies == 4 ? k_hist_tile<uint16_t, 512, 1024, 4> : k_hist_tile<uint16_t, 512, 1024, 1>;
+    else if (bins == 1024) h.fn = k_hist_tile<uint16_t, 1024, 1024, 1>;
+    else h.fn = k_hist_tile<uint16_t, 2048, 1024, 1>;
   } else if (h.smem_path) {
     h.smem = HistSmemBytes(h.width);
     h.fn = h.width == 2 ? (float_mode ? SmemKernel<true, 2>(order) : SmemKernel<false, 2>(order))
@@ -1291,8 +1355,11 @@ __global__ void k_group_scatter(const int32_t* __restrict__ node_of_row, int64_t
 
 void HistScratchNeeds(lbk_context* ctx, int F, int K, int bin_bytes, int mb, int64_t n_rows, HistScratch& need)
 {
-  const HistLaunch hl = PickHistKernel(bin_bytes, mb, false, kPairsByPosition, F, K, n_rows, ctx->sm_count);
-  need.n_arrive       = hl.smem_path ? kTreeFanIn * hl.grid : 0;
+  // what k_hist_smem needs, where some level may take it
+  if (bin_bytes != 1 || mb > kSmemBins || n_rows * F * K < kTileMaxCellsMany) return;
+  constexpr int64_t kManyRows = int64_t{1} << 36;  // (beyond every bound of the tile form)
+  const HistLaunch hl = PickHistKernel(bin_bytes, mb, false, kPairsByPosition, F, K, kManyRows, 1, false, ctx->sm_count, ctx->n_ranks);
+  need.n_arrive       = kTreeFanIn * hl.grid;
   need.partial_bytes  = static_cast<size_t>(need.n_arrive) * mb * kGroup * hl.width * 8;
 }
 
@@ -1324,7 +1391,7 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
   p.push_len         = lv.push_len;
   p.mb               = lv.max_bins_per_feature;
   p.mb_ptr           = lv.max_bins_ptr;
-  const HistLaunch hl = PickHistKernel(lv.bin_bytes, p.mb, lv.float_mode, OrderOf(p), p.F, p.K, lv.n_rows, ctx->sm_count);
+  const HistLaunch hl = PickHistKernel(lv.bin_bytes, p.mb, lv.float_mode, OrderOf(p), p.F, p.K, lv.n_rows, p.n_nodes, p.node_sums != nullptr, ctx->sm_count, ctx->n_ranks);
 
   const int* max_abs = lv.max_abs;
   if (!lv.float_mode && max_abs == nullptr) {
@@ -1373,7 +1440,7 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
     int32_t* wpre      = hl.smem_path ? s.alloc<int32_t>(static_cast<size_t>(lv.n_nodes) + 1) : nullptr;
     int32_t* plan      = s.alloc<int32_t>(8);
     p.ticket           = reinterpret_cast<unsigned int*>(plan + 2);
-    k_hist_plan<<<1, 1024, 0, stream>>>(p, units, hl.tile ? p.tile_items : hl.grid, hl.tile ? kTileMinRows : kMinChunk, chunk_off, wpre, plan);
+    k_hist_plan<<<1, 1024, 0, stream>>>(p, units, hl.tile ? p.tile_items : hl.grid, hl.tile ? kTileMinRows : kMinChunk, hl.copies != 1, chunk_off, wpre, plan);
     LBK_LAUNCH_CHECK();
     p.chunk_off = chunk_off;
     p.wpre      = wpre;
@@ -1593,7 +1660,7 @@ extern "C" int lbk_histogram_noalloc(int device, const lbk_histogram_args* a)
     p.mb                 = mb;
     p.mb_ptr             = nullptr;
     p.pairs_by_position  = a->pairs_by_position != 0 ? 1 : 0;
-    const HistLaunch hl  = PickHistKernel(a->bin_bytes, mb, float_mode, OrderOf(p), F, K, a->n_rows, sm_count);
+    const HistLaunch hl  = PickHistKernel(a->bin_bytes, mb, float_mode, OrderOf(p), F, K, a->n_rows, a->n_nodes, false, sm_count, 1);
 
     // the array keeps what the previous call left: clear the words that accumulate
     LBK_CUDA(cudaMemsetAsync(plan, 0, sizeof(int32_t) * 12, stream));
@@ -1622,7 +1689,7 @@ extern "C" int lbk_histogram_noalloc(int device, const lbk_histogram_args* a)
     p.n_arrive          = 0;
     p.tile_items        = sm_count * kTileItemsPerSm;
     const int units     = (hl.tile ? (F + kTileFeatures - 1) / kTileFeatures : (p.G + hl.width - 1) / hl.width) * K;
-    k_hist_plan<<<1, 1024, 0, stream>>>(p, units, hl.tile ? p.tile_items : hl.grid, hl.tile ? kTileMinRows : kMinChunk, chunk_off, nullptr, plan);
+    k_hist_plan<<<1, 1024, 0, stream>>>(p, units, hl.tile ? p.tile_items : hl.grid, hl.tile ? kTileMinRows : kMinChunk, hl.copies != 1, chunk_off, nullptr, plan);
     LBK_LAUNCH_CHECK();
     hl.fn<<<hl.grid, hl.threads, hl.smem, stream>>>(p);
     LBK_LAUNCH_CHECK();

@@ -1033,3 +1033,33 @@ def test_softmax_gradients_of_whole_and_partial_tiles(lb, N, K):
     tol = (K + 8) * 2.3e-16  # exp, K additions, a division, a product
     assert np.allclose(g.cpu().numpy(), want_g * 0.3, rtol=tol, atol=tol)
     assert np.allclose(h.cpu().numpy(), np.maximum(p * (1 - p), 1e-8), rtol=tol, atol=tol)
+
+
+@pytest.mark.parametrize("N,F,K,bins,nodes", [
+    (131072, 8, 1, 256, 1), (65537, 17, 1, 256, 40), (65537, 17, 1, 256, 60),  # from 2^20 cells on; units around the SMs
+    (70001, 9, 2, 256, 5), (131072, 7, 1, 256, 3),                             # several outputs; fewer cells
+    (40009, 30, 1, 512, 7), (40009, 30, 1, 300, 64), (40009, 27, 1, 1024, 7),  # two-byte ids
+    (300007, 60, 1, 256, 9), (300007, 60, 1, 256, 64),                         # more cells: few units, many units
+    (60013, 150, 1, 200, 8),                                                   # many units with rows in them
+])
+@pytest.mark.parametrize("largest", [1 << 12, 1 << 26])
+def test_histograms_of_moderate_matrices(lb, N, F, K, bins, nodes, largest):
+    """The forms for up to 3 * 2^24 cells: one copy of the histograms or four, nodes of very different sizes, magnitudes
+    for which a block has to empty its 32-bit sums after 31 rows (64-bit atomics) or not before the end."""
+    from legateboost_b200 import stages
+
+    rs = np.random.RandomState(N % 97 + F)
+    ids = rs.randint(0, bins, size=(N, F))
+    ids[:, 0] = np.minimum(ids[:, 0], 2)  # a crowded column
+    dt = np.uint8 if bins <= 256 else np.int16
+    node = np.minimum(rs.geometric(0.4, size=N) - 1, nodes - 1).astype(np.int32) if nodes < 50 else rs.randint(0, nodes, size=N).astype(np.int32)
+    q = rs.randint(-largest, largest, size=(N, K, 2)).astype(np.int32)
+    row_ptr = (np.arange(F + 1) * bins).astype(np.int32)
+    d_node = dev(node)
+    row_index, seg = stages.group_rows(d_node, 0, nodes)
+    hist = stages.histogram(stages.to_padded_rows(dev(ids.astype(dt))), dev(row_ptr), dev(q), row_index, seg, F, mode=0)
+    want = torch.zeros((nodes * F * bins, K, 2), dtype=torch.int64, device="cuda")
+    for f in range(F):
+        want.index_add_(0, (d_node.long() * F + f) * bins + dev(ids[:, f]).long(), dev(q).long())
+    want = want.view(nodes, F * bins, K, 2).permute(0, 2, 1, 3)
+    assert torch.equal(hist, want)
