@@ -642,8 +642,8 @@ TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, i
 template <typename T, int TG, int KR>
 void LaunchTiledAs(const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
-  if (plan.smem > 48 * 1024)
-    LBK_CUDA(cudaFuncSetAttribute(k_predict_tiled<T, TG, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.smem)));
+  // (whatever the size: the limit without it is for the static and the dynamic part together)
+  LBK_CUDA(cudaFuncSetAttribute(k_predict_tiled<T, TG, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.smem)));
   const unsigned grid = static_cast<unsigned>((a.n_rows + a.rb - 1) / a.rb);
   k_predict_tiled<T, TG, KR><<<grid, a.rb + 32, plan.smem, stream>>>(a);
   LBK_LAUNCH_CHECK();

@@ -856,6 +856,7 @@ def random_trees(rs, F, K, T, D):
     (8193, 1024, 1, 5, 3), (8193, 1025, 2, 5, 3),                     # the last feature id of a packed word; beyond it
     (8193, 12, 2, 9, 6), (30001, 20, 4, 8, 7), (8193, 3, 5, 16, 5), (8193, 9, 8, 10, 5),  # sums in registers
     (8193, 4, 16, 3, 4), (8193, 4, 17, 11, 4),                        # ... the most of them; in shared memory
+    (8193, 60, 1, 16, 6), (8193, 136, 1, 16, 6),                      # 48 KB of dynamic shared memory to the byte (f64, f32)
 ])
 def test_predict_of_many_rows_is_bit_exact(lb, oracle, dtype, N, F, K, T, D):
     """More rows than the one-launch form takes: trees in groups in shared memory, for rows that start on 16 bytes
