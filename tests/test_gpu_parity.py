@@ -1064,3 +1064,18 @@ def test_histograms_of_moderate_matrices(lb, N, F, K, bins, nodes, largest):
         want.index_add_(0, (d_node.long() * F + f) * bins + dev(ids[:, f]).long(), dev(q).long())
     want = want.view(nodes, F * bins, K, 2).permute(0, 2, 1, 3)
     assert torch.equal(hist, want)
+
+
+@pytest.mark.parametrize("K", [700, 740, 768, 3072])
+def test_many_outputs_at_the_edge_of_default_shared_memory(lb, oracle, K):
+    """The per-output tables of the quantiser and of the split search grow past what a launch may use without asking."""
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.RandomState(K)
+    N, D = (40, 2) if K < 3000 else (40, 0)  # (the most outputs that the quantiser takes)
+    X = rs.normal(size=(N, 1)).astype(np.float32)
+    g, h = rs.normal(size=(N, K)), rs.random((N, K)) + 0.1
+    t = build_tree_arrays(dev(X), dev(g), dev(h), max_depth=D, split_samples=8, seed=1, row_offset=0, dataset_rows=N)
+    want = oracle.build_tree(X, g, h, max_depth=D, split_samples=8, seed=1, mode="Q")
+    for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
+        assert np.array_equal(t[name].cpu().numpy(), getattr(want, name)), name
