@@ -695,7 +695,13 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   // a walk through M heap-ordered nodes takes at most S = floor(log2(M)) steps
   int S = 0;
   while ((2 << S) <= m_max) ++S;
-  const TilePlan plan = S <= 14 && F <= kMaxFeature ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
+  // Rows of more than kTileMaxRowBytes leave room for fewer than 64 beside the trees, and two warps per SM do not hide the
+  // walks' latency: nodes and rows are then read through the caches (200k rows, 100 trees of depth 6, tile and that, us:
+  // float32 512 features 425 and 583, 700: 668 and 489, 1000: 1500 and 510; float64 250: 416 and 513, 350: 667 and
+  // 538, 512: 1520 and 629; 100k rows, depth 9, float64 350: 843 and 845).
+  constexpr size_t kTileMaxRowBytes = 2560;
+  static_assert(kTileMaxRowBytes / sizeof(T) <= kMaxFeature, "feature ids must fit a word's fields");
+  const TilePlan plan = S <= 14 && F * sizeof(T) <= kTileMaxRowBytes ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
   if (plan.rb == 0) {
     NodeT* nodes   = s.alloc<NodeT>(total_nodes);
     double* leaves = s.alloc<double>(total_nodes * K);
