@@ -12,6 +12,15 @@
 //     order, so all blocks agree) and moves the rows down, reading the winning features' bin ids.
 // No repartition, no list of rows, no merge of partial histograms.
 //
+// What one block writes and another reads is ordered by the barriers alone.  Written once, before the first of them:
+// cuts, counts, bins_t, pairs, root_part, the cleared tree and outputs.  Written on every level:
+//   * cand, cand_left: before the barrier of level d, read after it; two regions by the parity of the level
+//     (small_layout.h), so that level d is overwritten on level d + 2, behind the barrier of level d + 1, which no
+//     block reaches before it has read level d;
+//   * hist: before the barrier of level d, read on level d + 1 before its barrier; two buffers, overwritten on level
+//     d + 2, behind that barrier;
+//   * the nodes of the tree: by block 0 only, each once; read by all behind the last barrier.
+//
 // 32-bit shared-memory sums are exact here without a bound on the magnitudes: a quantised value is added as
 // its high and its low 16 bits, whose sums over at most 65536 rows fit 32 bits.
 //
@@ -24,6 +33,7 @@
 #include "abs_sum.cuh"
 #include "internal.h"
 #include "objective.cuh"
+#include "small_layout.h"
 #include "split.cuh"
 
 namespace lbk {
@@ -68,8 +78,8 @@ struct SmallParams {
   int2* pairs;         // [N][K]
   GPairI64* root_part; // [blocks][K]
   GPairI64* hist[2];   // levels alternate: [F][nodes of the level][K][256]
-  SmallCand* cand;     // [nodes of the level][F]
-  GPairI64* cand_left; // [nodes of the level][F][K]
+  SmallCand* cand;     // levels alternate (SmallCandBegin): [nodes of the level][F]
+  GPairI64* cand_left; // likewise, [nodes of the level][F][K]
   int max_slots;       // histograms in shared memory at a time
   unsigned int* barrier;  // zero at the start
   int* status;
@@ -344,6 +354,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     const int begin = (1 << depth) - 1, nodes = 1 << depth;
     const bool derive = depth > 0, write_hist = depth < D - 1;
     const int units = derive ? nodes / 2 : 1;
+    SmallCand* cand     = p.cand + static_cast<int64_t>(SmallCandBegin(depth, D)) * F;
+    GPairI64* cand_left = p.cand_left + static_cast<int64_t>(SmallCandBegin(depth, D)) * F * K;
     // (s_wfeat still holds the winners of the level above: unit u exists if node u there was split)
     for (int f = f_first; f < F; f += f_step) {
       const bool search = p.feature_set == nullptr || p.feature_set[f] != 0;
@@ -475,13 +487,13 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                   if (Better(s_best[grp][side][w], best)) best = s_best[grp][side][w];
                 const int j      = side == 0 ? ja : jb;
                 const int64_t at = static_cast<int64_t>(j) * F + f;
-                if (b == 0) p.cand[at] = SmallCand{best.gain, best.bin < 0 ? -1 : best.feature, 0};  // (feature: the bin of the feature)
+                if (b == 0) cand[at] = SmallCand{best.gain, best.bin < 0 ? -1 : best.feature, 0};  // (feature: the bin of the feature)
                 if (K == 1) {
-                  if (best.bin >= 0 && b == best.feature) StorePair(p.cand_left + at, side == 0 ? va[0] : vb[0]);
+                  if (best.bin >= 0 && b == best.feature) StorePair(cand_left + at, side == 0 ? va[0] : vb[0]);
                 } else if (best.bin >= 0) {
                   // (written by threads of this block, before the barrier)
                   for (int kk = b; kk < K; kk += kSmallBins)
-                    StorePair(p.cand_left + at * K + kk,
+                    StorePair(cand_left + at * K + kk,
                               LoadPairStreaming(hist_f + (static_cast<int64_t>(j) * K + kk) * kSmallBins + best.feature));
                 }
               }
@@ -498,7 +510,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     const int words = derive ? nodes : 1;
     auto exists = [&](int j) { return j < words && (!derive || s_wfeat[j >> 1] >= 0) && s_nodes[static_cast<int64_t>(j) * K].hess > 0; };
     auto first_cand = [&](int j) {
-      return exists(j) && lane < F ? __ldcg(reinterpret_cast<const int4*>(p.cand + static_cast<int64_t>(j) * F + lane)) : make_int4(0, 0, -1, 0);
+      return exists(j) && lane < F ? __ldcg(reinterpret_cast<const int4*>(cand + static_cast<int64_t>(j) * F + lane)) : make_int4(0, 0, -1, 0);
     };
     int4 ahead = first_cand(warp);
     for (int j = warp; j < words; j += kSmallWarps) {
@@ -508,7 +520,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       ahead    = first_cand(j + kSmallWarps);
       if (here) {
         for (int f = lane; f < F; f += 32) {
-          if (f >= 32) raw = __ldcg(reinterpret_cast<const int4*>(p.cand + static_cast<int64_t>(j) * F + f));
+          if (f >= 32) raw = __ldcg(reinterpret_cast<const int4*>(cand + static_cast<int64_t>(j) * F + f));
           if (raw.z < 0) continue;
           const Cand c{__hiloint2double(raw.y, raw.x), s_rp[f] + raw.z, f};
           if (Better(c, best)) best = c;
@@ -540,7 +552,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       const int j = i / K, k = i - j * K, wf = s_wnew[j];
       GPairI64 ls{0, 0}, rs{0, 0};
       if (wf >= 0) {
-        ls                = LoadPairStreaming(p.cand_left + (static_cast<int64_t>(j) * F + wf) * K + k);
+        ls                = LoadPairStreaming(cand_left + (static_cast<int64_t>(j) * F + wf) * K + k);
         const GPairI64 ns = s_nodes[i];
         rs                = GPairI64{ns.grad - ls.grad, ns.hess - ls.hess};
         if (block == 0) {
@@ -691,8 +703,8 @@ void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStre
   const int last    = K > 1 ? D - 1 : D - 2;  // the last level written
   p.hist[last & 1]       = s.alloc<GPairI64>(static_cast<size_t>(F) * top * K * kSmallBins);
   p.hist[(last & 1) ^ 1] = s.alloc<GPairI64>(static_cast<size_t>(F) * below * K * kSmallBins);
-  p.cand      = s.alloc<SmallCand>(static_cast<size_t>(level) * F);
-  p.cand_left = s.alloc<GPairI64>(static_cast<size_t>(level) * F * K);
+  p.cand      = s.alloc<SmallCand>(static_cast<size_t>(SmallCandNodes(D)) * F);
+  p.cand_left = s.alloc<GPairI64>(static_cast<size_t>(SmallCandNodes(D)) * F * K);
   p.max_slots = plan.max_slots;
   p.status    = ctx->d_status;
   p.info_host = a.info_host;

@@ -1080,3 +1080,19 @@ def test_many_outputs_at_the_edge_of_default_shared_memory(lb, oracle, K):
     want = oracle.build_tree(X, g, h, max_depth=D, split_samples=8, seed=1, mode="Q")
     for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
         assert np.array_equal(t[name].cpu().numpy(), getattr(want, name)), name
+
+
+@pytest.mark.parametrize("N,F,K,D", [(40, 300, 1, 8), (500, 10, 1, 6), (2000, 3, 3, 7), (16384, 2, 1, 5)])
+def test_one_launch_trees_are_the_same_every_time(lb, oracle, N, F, K, D):
+    """The blocks of the one-launch tree pick every level's winners for themselves and must agree, whichever of them is
+    ahead: one feature or several per block, several blocks per feature."""
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.RandomState(N)
+    X, g, h = rs.normal(size=(N, F)).astype(np.float32), rs.normal(size=(N, K)), rs.random((N, K)) + 0.1
+    want = oracle.build_tree(X, g, h, max_depth=D, split_samples=64, seed=9, mode="Q")
+    d = [dev(a) for a in (X, g, h)]
+    for i in range(50):
+        t = build_tree_arrays(*d, max_depth=D, split_samples=64, seed=9, row_offset=0, dataset_rows=N)
+        for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
+            assert np.array_equal(t[name].cpu().numpy(), getattr(want, name)), (i, name)
