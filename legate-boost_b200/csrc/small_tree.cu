@@ -300,13 +300,19 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     for (int k = tid; k < K; k += kSmallThreads)
       p.root_part[static_cast<int64_t>(block) * K + k] = GPairI64{s_root[2 * k], s_root[2 * k + 1]};
   }
-  // cleared outputs; the nodes that split are written over below, after the barrier
+  // cleared outputs; the nodes that split are written over below, after the barrier.  The values and the rows' nodes
+  // too: if a barrier gives up, the kernels that are queued behind this one still find nodes of the tree, with value 0.
   for (int i = block * kSmallThreads + tid; i < p.tree.max_nodes; i += n_blocks * kSmallThreads) {
     p.tree.feature[i]     = -1;
     p.tree.split_value[i] = 0.0;
     p.tree.gain[i]        = 0.0;
-    for (int k = 0; k < K; ++k) p.tree.node_sums[static_cast<int64_t>(i) * K + k] = GPairI64{0, 0};
+    for (int k = 0; k < K; ++k) {
+      p.tree.node_sums[static_cast<int64_t>(i) * K + k]  = GPairI64{0, 0};
+      p.tree.leaf_value[static_cast<int64_t>(i) * K + k] = p.hessian[static_cast<int64_t>(i) * K + k] = 0.0;
+    }
   }
+  if (p.leaf != nullptr)
+    for (int row = block * kSmallThreads + tid; row < N; row += n_blocks * kSmallThreads) p.leaf[row] = 0;
   target += n_blocks;
   if (!GridBarrier(p.barrier, target, p.status, &s_ok)) return;
 

@@ -1096,3 +1096,41 @@ def test_one_launch_trees_are_the_same_every_time(lb, oracle, N, F, K, D):
         t = build_tree_arrays(*d, max_depth=D, split_samples=64, seed=9, row_offset=0, dataset_rows=N)
         for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
             assert np.array_equal(t[name].cpu().numpy(), getattr(want, name)), (i, name)
+
+
+def test_round_after_a_barrier_that_gave_up(lb):
+    """The barrier word of a one-launch tree starts below what its blocks can count up to, so that the bounded wait runs
+    out (about a second): the fault is reported, and what is queued behind the tree finds no rows' nodes or values that
+    were never written (softmax: the leaf values are added by a kernel of its own)."""
+    import ctypes as C
+
+    L = lb.library
+    rs = np.random.RandomState(0)
+    N, F, K, D = 300, 4, 3, 3
+    M = 2 ** (D + 1) - 1
+    X, y, pred = dev(rs.normal(size=(N, F)).astype(np.float32)), dev(rs.randint(0, K, size=N).astype(np.float64)), dev(rs.normal(size=(N, K)))
+    before = pred.clone()
+    tree = dict(leaf_value=torch.full((M, K), 7.0, dtype=torch.float64, device="cuda"), feature=torch.full((M,), 3, dtype=torch.int32, device="cuda"))
+    for name, shape in (("split_value", M), ("gain", M), ("hessian", M * K)):
+        tree[name] = torch.full((shape,), 7.0, dtype=torch.float64, device="cuda")
+    word = torch.full((1,), -2 ** 30, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ctx = L.context()
+    r = L.BoostRoundArgs()
+    a = r.tree
+    a.X, a.x_dtype, a.ldx = X.data_ptr(), L.LBK_F32, F
+    a.n_local_rows, a.dataset_rows, a.n_features, a.n_outputs = N, N, F, K
+    a.max_depth, a.max_nodes, a.split_samples, a.seed, a.l2_regularization = D, M, 16, 1, 1.0
+    for name, t in tree.items():
+        setattr(a, name, t.data_ptr())
+    a.stream = torch.cuda.current_stream().cuda_stream
+    r.objective, r.y, r.pred, r.learning_rate, r.zeroed = 1, y.data_ptr(), pred.data_ptr(), 0.5, word.data_ptr()
+    ctx.check(ctx.lib.lbk_boost_round(ctx.handle, C.byref(r)))
+    with pytest.raises(L.LbkError, match="fault code 51"):
+        ctx.check(ctx.lib.lbk_synchronize(ctx.handle, a.stream))
+    assert torch.equal(pred, before)
+    assert (tree["feature"] == -1).all() and not tree["leaf_value"].any() and not tree["hessian"].any()
+    word.zero_()
+    ctx.check(ctx.lib.lbk_boost_round(ctx.handle, C.byref(r)))
+    ctx.check(ctx.lib.lbk_synchronize(ctx.handle, a.stream))
+    assert not torch.equal(pred, before) and (tree["feature"][0] >= 0)
