@@ -1,6 +1,7 @@
 // Split candidates, their total order and the gain of a bin (reference behaviour: see split.cu).
 #pragma once
 #include "device_utils.cuh"
+#include "division.cuh"
 
 namespace lbk {
 
@@ -60,33 +61,6 @@ __device__ inline NodeTerms TermsOf(GPairI64 sum, const QuantParams& qp, double 
   t.h    = WholeToDouble(sum.hess);
   t.gain = LeafGain(GPairF64{t.g * qp.inv_g, t.h * qp.inv_h}, l1, reg);
   return t;
-}
-
-// a / b, correctly rounded, without a branch: the reciprocal approximation refined by Newton steps, and two
-// corrections of the quotient by its exact remainder (P. Markstein, "Computation of elementary functions on the
-// IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990): a quotient within one unit in the last place
-// plus remainder times the correctly rounded reciprocal rounds to the exact quotient).  For the operands that
-// DivisionIsPlain accepts nothing on the way leaves the normal range.
-//
-// Why not the operator: its test for operands out of range is a branch per division, which keeps the compiler
-// from running the 16 divisions of a lane side by side, and one of them is a chain of a dozen dependent
-// float64 instructions.  A level of a 500 x 10 tree spent 8 of its 15 us there.
-__device__ inline double DividePlain(double a, double b)
-{
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(r) : "d"(b));
-  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
-  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
-  r = __fma_rn(r, __fma_rn(-b, r, 1.0), r);
-  double q = a * r;
-  q        = __fma_rn(__fma_rn(-b, q, a), r, q);
-  return __fma_rn(__fma_rn(-b, q, a), r, q);
-}
-// b in [2^-500, 2^500), a zero or in the same range (both not negative)
-__device__ inline bool DivisionIsPlain(double a, double b)
-{
-  const unsigned ea = static_cast<unsigned>(__double2hiint(a)) - (523u << 20), eb = static_cast<unsigned>(__double2hiint(b)) - (523u << 20);
-  return eb < (1000u << 20) && (a == 0.0 || ea < (1000u << 20));
 }
 
 // LeafGain's numerator
