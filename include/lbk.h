@@ -11,8 +11,11 @@
  *   - data pointers are DEVICE pointers unless the struct's `host_buffers` field is non-zero,
  *     in which case they are host pointers and the library stages the copies itself on `stream`;
  *   - every call returns 0 on success or a negative lbk_status; lbk_last_error() gives the text;
- *   - a context belongs to one device and one host thread at a time; different contexts may be
- *     used concurrently from different threads (one per GPU, as the runtime calls task variants);
+ *   - a context belongs to one device.  Without a communicator, calls may be in progress on it from several
+ *     host threads and streams at a time; two things are then shared: lbk_last_error may hold another
+ *     call's text, and a fault that a kernel reports is returned by whichever call looks next.  One
+ *     thread at a time for everything else: calls with a communicator, lbk_context_set_allocator,
+ *     lbk_context_trim, lbk_profile_*, lbk_selftest_*;
  *   - there is no CPU fallback: every entry point fails with LBK_ERR_CUDA when no device is
  *     usable.
  */

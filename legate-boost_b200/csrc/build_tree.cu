@@ -106,8 +106,7 @@ void LeafOfRow(lbk_context* ctx, const void* bins, int64_t pitch, int64_t N, int
   if (pitch_bytes <= kLeafMaxPitch && M <= kLeafMaxNodes && F < 65535 && aligned) {
     const size_t smem = (static_cast<size_t>(M) * 4 + 15) / 16 * 16 + static_cast<size_t>(kLeafWarps) * 32 * (pitch_bytes + 4);
     auto fn           = k_leaf_of_row_tiled<BinT>;
-    if (smem > 48 * 1024)
-      LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    if (smem > 48 * 1024) AllowSharedMemory(ctx, fn, 1024);
     int per_sm = 0;
     LBK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLeafWarps * 32, smem));
     const int64_t chunks = (N + 31) / 32;

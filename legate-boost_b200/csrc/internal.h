@@ -188,6 +188,15 @@ void ThrowReportedFault(lbk_context* ctx);
 // Runs f, turning exceptions into a status code and an error text (the ABI boundary).
 int Guard(lbk_context* ctx, const std::function<void()>& f);
 
+// Lets launches of `fn` ask for up to the device's limit of dynamic shared memory, less `static_bytes`, a bound of what the
+// kernel declares itself.  The limit belongs to the function and not to a launch: one constant per function,
+// or a call on another thread could lower it between this call's setting and its launch.
+template <typename Fn>
+inline void AllowSharedMemory(const lbk_context* ctx, Fn fn, int static_bytes)
+{
+  LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - static_bytes));
+}
+
 // ---- stage launchers (defined in the .cu files named in the comments) ------------------------
 struct TreeArrays {
   double* leaf_value;

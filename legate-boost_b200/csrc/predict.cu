@@ -596,7 +596,8 @@ struct TilePlan {
   size_t smem      = 0;
   TreeRecord rec{};
 };
-constexpr int kRegisterSums = 16;  // outputs whose sums a warp keeps in registers
+constexpr int kRegisterSums    = 16;   // outputs whose sums a warp keeps in registers
+constexpr int kTileStaticBytes = 256;  // (a bound of what the kernel declares)
 
 // The pipe is kept busy by the walks in flight: warps x trees per group.  That product is made as large as shared
 // memory allows, over groups of 8, 4, 2 or 1 trees and 1 to 4 blocks per SM, up to kTileThreads; equal products go to
@@ -617,7 +618,8 @@ TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, i
     const int nbuf       = n_trees > tg ? 2 : 1;
     const size_t trees   = static_cast<size_t>(nbuf) * tg * rec.bytes;
     for (int res = 1; res <= 4; ++res) {
-      const size_t room = res == 1 ? static_cast<size_t>(ctx->max_smem_optin) - 256 : (static_cast<size_t>(ctx->max_smem_optin) + 1024) / res - 1024 - 256;
+      const size_t room = res == 1 ? static_cast<size_t>(ctx->max_smem_optin) - kTileStaticBytes
+                                    : (static_cast<size_t>(ctx->max_smem_optin) + 1024) / res - 1024 - kTileStaticBytes;
       if (trees + 32 * per_row > room) continue;
       const int rb    = static_cast<int>(std::min<size_t>((room - trees) / per_row, kTileThreads / res - 32) / 32 * 32);
       const int score = res * rb / 32 * tg;
@@ -640,25 +642,25 @@ TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, i
 }
 
 template <typename T, int TG, int KR>
-void LaunchTiledAs(const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
+void LaunchTiledAs(lbk_context* ctx, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
   // (whatever the size: the limit without it is for the static and the dynamic part together)
-  LBK_CUDA(cudaFuncSetAttribute(k_predict_tiled<T, TG, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.smem)));
+  AllowSharedMemory(ctx, k_predict_tiled<T, TG, KR>, kTileStaticBytes);
   const unsigned grid = static_cast<unsigned>((a.n_rows + a.rb - 1) / a.rb);
   k_predict_tiled<T, TG, KR><<<grid, a.rb + 32, plan.smem, stream>>>(a);
   LBK_LAUNCH_CHECK();
 }
 
 template <typename T, int TG>
-void LaunchTiled(const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
+void LaunchTiled(lbk_context* ctx, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
-  if (a.K == 1) LaunchTiledAs<T, TG, 0>(a, plan, stream);
-  else if (a.K <= 2) LaunchTiledAs<T, TG, 2>(a, plan, stream);
-  else if (a.K <= 4) LaunchTiledAs<T, TG, 4>(a, plan, stream);
-  else if (a.K <= 8) LaunchTiledAs<T, TG, 8>(a, plan, stream);
-  else if (a.K <= 12) LaunchTiledAs<T, TG, 12>(a, plan, stream);
-  else if (a.K <= kRegisterSums) LaunchTiledAs<T, TG, kRegisterSums>(a, plan, stream);
-  else LaunchTiledAs<T, TG, -1>(a, plan, stream);
+  if (a.K == 1) LaunchTiledAs<T, TG, 0>(ctx, a, plan, stream);
+  else if (a.K <= 2) LaunchTiledAs<T, TG, 2>(ctx, a, plan, stream);
+  else if (a.K <= 4) LaunchTiledAs<T, TG, 4>(ctx, a, plan, stream);
+  else if (a.K <= 8) LaunchTiledAs<T, TG, 8>(ctx, a, plan, stream);
+  else if (a.K <= 12) LaunchTiledAs<T, TG, 12>(ctx, a, plan, stream);
+  else if (a.K <= kRegisterSums) LaunchTiledAs<T, TG, kRegisterSums>(ctx, a, plan, stream);
+  else LaunchTiledAs<T, TG, -1>(ctx, a, plan, stream);
 }
 
 }  // namespace
@@ -719,10 +721,10 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   LBK_LAUNCH_CHECK();
   const TiledArgs<T> a{X, ldx, n_rows, F, K, n_trees, plan.rb, plan.nbuf, plan.x_bytes, records, plan.rec, leaves_c, o, ctx->d_status};
   switch (plan.tg) {
-    case 8: LaunchTiled<T, 8>(a, plan, stream); break;
-    case 4: LaunchTiled<T, 4>(a, plan, stream); break;
-    case 2: LaunchTiled<T, 2>(a, plan, stream); break;
-    default: LaunchTiled<T, 1>(a, plan, stream); break;
+    case 8: LaunchTiled<T, 8>(ctx, a, plan, stream); break;
+    case 4: LaunchTiled<T, 4>(ctx, a, plan, stream); break;
+    case 2: LaunchTiled<T, 2>(ctx, a, plan, stream); break;
+    default: LaunchTiled<T, 1>(ctx, a, plan, stream); break;
   }
 }
 

@@ -95,8 +95,7 @@ void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, i
     if (blocks * 256 < K) blocks = (K + 255) / 256;  // a thread keeps one output: at least K threads
     const size_t smem = sizeof(unsigned long long) * 2 * K;
     LBK_EXPECT(smem <= 48 * 1024, "too many outputs for the quantiser's block sums");
-    if (smem > 40 * 1024)  // (the limit without it counts the static part too)
-      LBK_CUDA(cudaFuncSetAttribute(k_quantise, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    if (smem > 40 * 1024) AllowSharedMemory(ctx, k_quantise, 1024);  // (the limit without it counts the static part too)
     k_quantise<<<static_cast<unsigned>(blocks), 256, smem, stream>>>(g, h, ldg, row_offset, n_local, K,
                                                                   static_cast<long long>(seed), params, gpair, root_sums, max_abs);
     LBK_LAUNCH_CHECK();

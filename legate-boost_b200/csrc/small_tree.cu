@@ -716,7 +716,7 @@ void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStre
   p.info_host = a.info_host;
   p.barrier   = a.barrier;
   auto fn = k_tree_small<T>;
-  LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 2048));
+  AllowSharedMemory(ctx, fn, 2048);
   void* args[] = {&p};
   LBK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(fn), dim3(plan.blocks), dim3(kSmallThreads), args,
                                        plan.smem, stream));

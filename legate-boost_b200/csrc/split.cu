@@ -425,8 +425,7 @@ void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, co
   }
   auto fn = lv.K > 1 ? (lv.derive ? k_scan_split<T, true, true> : k_scan_split<T, true, false>)
                      : (lv.derive ? k_scan_split<T, false, true> : k_scan_split<T, false, false>);
-  if (smem > 40 * 1024)  // (the limit without it counts the static part too)
-    LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  if (smem > 40 * 1024) AllowSharedMemory(ctx, fn, 2048);  // (the limit without it counts the static part too)
   fn<<<dim3(units, slices), kSplitThreads, smem, stream>>>(p);
   LBK_LAUNCH_CHECK();
   if (exchange_records) {

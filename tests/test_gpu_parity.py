@@ -1134,3 +1134,35 @@ def test_round_after_a_barrier_that_gave_up(lb):
     ctx.check(ctx.lib.lbk_boost_round(ctx.handle, C.byref(r)))
     ctx.check(ctx.lib.lbk_synchronize(ctx.handle, a.stream))
     assert not torch.equal(pred, before) and (tree["feature"][0] >= 0)
+
+
+def test_predictions_on_several_threads(lb, oracle):
+    """Tiles of different sizes of the same kernel, launched from several threads on one context: the limit of shared
+    memory that a function may ask for is the same for all of them."""
+    import threading
+
+    from legateboost_b200.tree import predict_arrays
+
+    rs = np.random.RandomState(2)
+    jobs = []
+    for F, T, D in ((3, 1, 2), (100, 40, 8), (300, 9, 4), (20, 16, 10)):
+        X, trees = rs.normal(size=(8200, F)).astype(np.float32), random_trees(rs, F, 1, T, D)
+        jobs.append((dev(X), [tuple(map(dev, t)) for t in trees], oracle.predict(X, trees)))
+    errors = []
+
+    def work(X, trees, want):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(40):
+                    got = predict_arrays(X, trees)
+                assert np.array_equal(got.cpu().numpy(), want)
+        except Exception as e:  # seen by the main thread
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
