@@ -51,7 +51,8 @@ int lbk_version(void);
  * (legate::create_buffer scratch, context.get_task_stream(), context.communicator(0)). */
 int lbk_context_create(int device, lbk_context** out);
 void lbk_context_destroy(lbk_context* ctx);
-/* Text of the last error on this context (or of the last context-less call on this thread). */
+/* Text of the last error on this context (or of the last context-less call on this thread); valid until the calling
+ * thread's next call of this function. */
 const char* lbk_last_error(const lbk_context* ctx);
 /* Release cached scratch memory back to the driver. */
 int lbk_context_trim(lbk_context* ctx);

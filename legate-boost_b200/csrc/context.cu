@@ -233,14 +233,22 @@ int Guard(lbk_context* ctx, const std::function<void()>& f)
       if (before >= 0 && cudaGetDevice(&now) == cudaSuccess && now != before) cudaSetDevice(before);
     }
   } restore;
+  auto keep = [&](const char* what) {
+    if (ctx == nullptr) {
+      tls_error = what;
+    } else {
+      std::lock_guard<std::mutex> lock(ctx->err_mutex);
+      ctx->err = what;
+    }
+  };
   try {
     f();
     return LBK_OK;
   } catch (const Error& e) {
-    (ctx ? ctx->err : tls_error) = e.what();
+    keep(e.what());
     return e.code;
   } catch (const std::exception& e) {
-    (ctx ? ctx->err : tls_error) = e.what();
+    keep(e.what());
     return LBK_ERR_ARGUMENT;
   }
 }
@@ -304,7 +312,15 @@ void lbk_context_destroy(lbk_context* ctx)
   delete ctx;
 }
 
-const char* lbk_last_error(const lbk_context* ctx) { return ctx ? ctx->err.c_str() : tls_error.c_str(); }
+const char* lbk_last_error(const lbk_context* ctx)
+{
+  if (ctx == nullptr) return tls_error.c_str();
+  // a copy of the calling thread's own: another thread's failing call may replace the context's text at any time
+  static thread_local std::string copy;
+  std::lock_guard<std::mutex> lock(ctx->err_mutex);
+  copy = ctx->err;
+  return copy.c_str();
+}
 
 int lbk_context_trim(lbk_context* ctx)
 {

@@ -73,7 +73,8 @@ struct lbk_context {
   lbk_alloc_fn alloc_cb     = nullptr;
   lbk_release_fn release_cb = nullptr;
   void* alloc_user          = nullptr;
-  std::string err;
+  mutable std::mutex err_mutex;
+  std::string err;  // of the last call that failed, whatever its thread
   // status word in mapped host memory: 0 = ok, otherwise a kernel stored a fault code
   int* d_status = nullptr;
   // pairs of words in mapped host memory that a call borrows for what its kernels tell the host (HostWords)

@@ -1166,3 +1166,31 @@ def test_predictions_on_several_threads(lb, oracle):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_error_texts_of_calls_on_several_threads(lb):
+    """A text that is being read is not replaced by another thread's failing call: every thread reads one of the texts
+    that were written, whole."""
+    import ctypes as C
+    import threading
+
+    ctx = lb.library.context()
+    seen = set()
+
+    def fail(dtype, n):
+        a = lb.library.PredictArgs()
+        a.x_dtype, a.n_rows, a.X, a.pred = dtype, 1, 16, 16  # (refused before anything is read)
+        for _ in range(n):
+            assert ctx.lib.lbk_predict(ctx.handle, C.byref(a)) != 0
+            seen.add(ctx.lib.lbk_last_error(ctx.handle))
+
+    fail(9, 1)
+    fail(0, 1)
+    texts = set(seen)
+    assert len(texts) == 2
+    threads = [threading.Thread(target=fail, args=(d, 2000)) for d in (9, 0, 9, 0)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert seen == texts
