@@ -76,6 +76,9 @@ typedef void (*lbk_release_fn)(void* user, void* ptr, void* stream);
 int lbk_context_set_allocator(lbk_context* ctx, lbk_alloc_fn alloc, lbk_release_fn release, void* user);
 /* Bytes the context's own pool holds at the moment (reserved from the driver, in use or cached). */
 int lbk_context_pool_bytes(lbk_context* ctx, size_t* reserved);
+/* Pairs of words in pinned host memory that are out with calls: 0 when no call is in progress, unless a call failed
+ * while its kernels were queued (they may still write its pair, which then stays out of use). */
+int lbk_context_lent_words(lbk_context* ctx, int* pairs);
 
 /* Communicator (reference: the ncclComm_t* the runtime hands to the task, cpp_utils.cuh:100-134).
  * Either create one from an id that rank 0 made and every rank received out of band ... */

@@ -399,7 +399,9 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     pa.zero_n16[1]  = keep_sums ? static_cast<int64_t>(M) * K : 0;
     pa.zero[2]      = cache;
     pa.zero_n16[2]  = root_zeroed ? static_cast<int64_t>(K) * bins_bound : 0;
-    Prologue<T>(ctx, s, pa, row_ptr, info, wait_for_bins || a.out_total_bins ? words.get() : nullptr, sums, qp, stream);
+    // (a sketch that is reused knows its bins: no kernel counts any and no words are borrowed for them)
+    int32_t* info_host = !sketch_reuse && (wait_for_bins || a.out_total_bins) ? words.get() : nullptr;
+    Prologue<T>(ctx, s, pa, row_ptr, info, info_host, sums, qp, stream);
   }
   ProposalInfo pi{static_cast<int>(std::min<int64_t>(bins_bound, INT32_MAX)), S};
   if (sketch_reuse) {

@@ -160,6 +160,7 @@ int32_t* HostWords::get()
   }
   words_ = ctx_->words_free.back();
   ctx_->words_free.pop_back();
+  ctx_->words_lent++;
   return words_;
 }
 
@@ -168,6 +169,7 @@ HostWords::~HostWords()
   if (words_ == nullptr || !settled_) return;
   std::lock_guard<std::mutex> lock(ctx_->words_mutex);
   ctx_->words_free.push_back(words_);  // (has room: every pair was in the list once)
+  ctx_->words_lent--;
 }
 
 void AllReduce(lbk_context* ctx, void* buf, size_t count, lbk_dtype dtype, lbk_redop op, cudaStream_t stream)
@@ -351,6 +353,15 @@ int lbk_context_pool_bytes(lbk_context* ctx, size_t* reserved)
     uint64_t v = 0;
     LBK_CUDA(cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &v));
     *reserved = static_cast<size_t>(v);
+  });
+}
+
+int lbk_context_lent_words(lbk_context* ctx, int* pairs)
+{
+  return lbk::Guard(ctx, [&] {
+    LBK_EXPECT(ctx && pairs, "null argument");
+    std::lock_guard<std::mutex> lock(ctx->words_mutex);
+    *pairs = ctx->words_lent;
   });
 }
 

@@ -81,6 +81,7 @@ struct lbk_context {
   std::mutex words_mutex;
   std::vector<void*> words_pages;
   std::vector<int32_t*> words_free;
+  int words_lent = 0;
   // communicator
   int rank = 0, n_ranks = 1;
   void* nccl_comm     = nullptr;

@@ -1194,3 +1194,25 @@ def test_error_texts_of_calls_on_several_threads(lb):
     for t in threads:
         t.join()
     assert seen == texts
+
+
+@pytest.mark.parametrize("N,S", [(20000, 64), (20000, 400), (500, 64)])
+@pytest.mark.parametrize("fixed_sketch", [False, True])
+def test_calls_give_back_the_words_they_borrow(lb, N, S, fixed_sketch):
+    import ctypes as C
+
+    from legateboost_b200.tree import build_tree_arrays
+
+    ctx = lb.library.context()
+
+    def lent():
+        v = C.c_int(-1)
+        ctx.check(ctx.lib.lbk_context_lent_words(ctx.handle, C.byref(v)))
+        return v.value
+
+    before = lent()  # (what a call that failed kept)
+    rs = np.random.RandomState(0)
+    X, y = dev(rs.normal(size=(N, 5)).astype(np.float32)), dev(rs.normal(size=N))
+    lb.LBRegressor(n_estimators=7, base_models=(lb.Tree(max_depth=3, split_samples=S),), random_state=0, fixed_sketch=fixed_sketch).fit(X, y)
+    build_tree_arrays(X, y[:, None], torch.ones_like(y)[:, None], max_depth=3, split_samples=S, seed=1, row_offset=0, dataset_rows=N)
+    assert lent() == before
