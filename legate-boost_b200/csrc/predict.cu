@@ -552,6 +552,14 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
   __syncthreads();  // (the producer's copies)
 }
 
+// The raw sums of an ensemble without trees; nothing of X is read.
+__global__ void __launch_bounds__(256) k_predict_nothing(int64_t n_rows, int K, PredictOut o)
+{
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (row >= n_rows) return;
+  for (int k = 0; k < K; ++k) o.pred[row * o.ldp + k] = o.init ? o.init[k] : 0.0;
+}
+
 // What is left to do after a kernel that wrote the raw sums.
 __global__ void __launch_bounds__(256) k_finish_rows(int64_t n_rows, int K, PredictOut o)
 {
@@ -678,16 +686,21 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
     k_finish_rows<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(n_rows, K, o);
     LBK_LAUNCH_CHECK();
   };
-  // Few rows: walk the trees in place.  The tiled kernel gives a block 256 rows and brings every tree
-  // into shared memory per block, so that it needs tens of thousands of rows to fill the chip.
+  if (n_trees == 0) {
+    k_predict_nothing<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(n_rows, K, o);
+    LBK_LAUNCH_CHECK();
+    finish();
+    return;
+  }
+  // Few rows: walk the trees in place.  The tiled kernel brings every tree into shared memory per block (of up to
+  // 480 rows), so that it needs tens of thousands of rows to fill the chip.
   {
     constexpr int64_t kRowsMax = 8192;
     int r = static_cast<int>((n_rows + 4 * ctx->sm_count - 1) / (4 * ctx->sm_count));
     r     = r < 1 ? 1 : r > 8 ? 8 : r;
     auto need = [&](int rows) { return static_cast<size_t>(rows) * ((n_trees + K) * sizeof(double) + F * sizeof(T)); };
-    if (n_trees == 0) r = 1;
     while (r > 1 && need(r) > 48 * 1024) r /= 2;
-    if (n_trees == 0 || (n_rows <= kRowsMax && need(r) <= 48 * 1024)) {
+    if (n_rows <= kRowsMax && need(r) <= 48 * 1024) {
       const unsigned grid = static_cast<unsigned>((n_rows + r - 1) / r);
       k_predict_rows<T><<<grid, kRowsThreads, need(r), stream>>>(X, ldx, n_rows, F, K, n_trees, r, d_trees, o);
       LBK_LAUNCH_CHECK();

@@ -1216,3 +1216,28 @@ def test_calls_give_back_the_words_they_borrow(lb, N, S, fixed_sketch):
     lb.LBRegressor(n_estimators=7, base_models=(lb.Tree(max_depth=3, split_samples=S),), random_state=0, fixed_sketch=fixed_sketch).fit(X, y)
     build_tree_arrays(X, y[:, None], torch.ones_like(y)[:, None], max_depth=3, split_samples=S, seed=1, row_offset=0, dataset_rows=N)
     assert lent() == before
+
+
+@pytest.mark.parametrize("K,transform", [(1, "RAW"), (3, "RAW"), (1, "LOGISTIC"), (3, "SOFTMAX")])
+@pytest.mark.parametrize("with_init", [False, True])
+def test_an_ensemble_without_trees_takes_rows_of_any_width(lb, K, transform, with_init):
+    """Through the C ABI: every row is the initial prediction (or 0), transformed; X is not read, so that its width does
+    not matter."""
+    import ctypes as C
+
+    L = lb.library
+    N, F, columns = 9000, 20000, 2 if transform == "LOGISTIC" else K
+    X = torch.full((1, F), float("nan"), dtype=torch.float64, device="cuda")  # (a row stands for all of them)
+    init = dev(np.linspace(-1.0, 2.0, K))
+    pred = torch.full((N, columns + 1), 7.0, dtype=torch.float64, device="cuda")
+    a = L.PredictArgs()
+    a.X, a.x_dtype, a.ldx, a.n_rows, a.n_features, a.n_outputs = X.data_ptr(), L.LBK_F64, F, N, F, K
+    a.pred, a.ldp, a.transform = pred.data_ptr(), columns + 1, getattr(L, transform)
+    a.init = init.data_ptr() if with_init else None
+    a.stream = torch.cuda.current_stream().cuda_stream
+    ctx = L.context()
+    ctx.check(ctx.lib.lbk_predict(ctx.handle, C.byref(a)))
+    raw = init if with_init else torch.zeros_like(init)
+    want = raw if transform == "RAW" else torch.softmax(raw, 0) if transform == "SOFTMAX" else torch.stack([1 - torch.sigmoid(raw[0]), torch.sigmoid(raw[0])])
+    assert torch.allclose(pred[:, :columns], want.expand(N, columns), rtol=1e-15 * (K + 8), atol=0)
+    assert (pred[:, columns] == 7.0).all()
