@@ -220,6 +220,10 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     LBK_CUDA(cudaMemcpyAsync(a.hessian, hessian, sizeof(double) * M * K, cudaMemcpyDeviceToHost, stream));
   };
 
+  // The kernels work on node sums in the caller's own array where they can: device memory that their 16-byte accesses may
+  // go to.  Else the sums are copied there at the end.
+  const bool keep_sums = a.trace_node_sums != nullptr && !a.host_buffers && (reinterpret_cast<uintptr_t>(a.trace_node_sums) & 15) == 0;
+
   // Tree (reference: struct Tree, build_tree.cu:785-809)
   if (ctx->n_ranks <= 1 && a.sketch_mode == LBK_SKETCH_OFF && a.trace_hist == nullptr &&
       SmallTreeFits(ctx, N, F, K, D, a.split_samples, sizeof(T))) {
@@ -253,9 +257,8 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       t.ldg = K;
     }
     t.sp          = SplitParams{a.l1_regularization, a.l2_regularization, a.min_split_gain, fset};
-    const bool device_sums = a.trace_node_sums != nullptr && !a.host_buffers;
     t.tree        = TreeArrays{leaf_value, feature, split_value, gain,
-                        device_sums ? reinterpret_cast<GPairI64*>(a.trace_node_sums) : s.alloc<GPairI64>(static_cast<size_t>(M) * K),
+                        keep_sums ? reinterpret_cast<GPairI64*>(a.trace_node_sums) : s.alloc<GPairI64>(static_cast<size_t>(M) * K),
                         nullptr, M};
     t.hessian     = hessian;
     int32_t* leaf = a.out_leaf != nullptr && !a.host_buffers ? a.out_leaf
@@ -272,7 +275,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       k_add_leaf_values<<<static_cast<unsigned>((N * K + 255) / 256), 256, 0, stream>>>(leaf_value, leaf, N, K, round->pred);
       LBK_LAUNCH_CHECK();
     }
-    if (a.trace_node_sums && !device_sums)
+    if (a.trace_node_sums && !keep_sums)
       LBK_CUDA(cudaMemcpyAsync(a.trace_node_sums, t.tree.node_sums, sizeof(GPairI64) * M * K, cudaMemcpyDefault, stream));
     if (a.host_buffers) {
       if (a.out_leaf) LBK_CUDA(cudaMemcpyAsync(a.out_leaf, leaf, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, stream));
@@ -292,7 +295,6 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     h   = rh;
     ldg = K;
   }
-  const bool keep_sums = a.trace_node_sums != nullptr && !a.host_buffers;
   TreeArrays tree;
   tree.leaf_value  = leaf_value;
   tree.feature     = feature;

@@ -1241,3 +1241,32 @@ def test_an_ensemble_without_trees_takes_rows_of_any_width(lb, K, transform, wit
     want = raw if transform == "RAW" else torch.softmax(raw, 0) if transform == "SOFTMAX" else torch.stack([1 - torch.sigmoid(raw[0]), torch.sigmoid(raw[0])])
     assert torch.allclose(pred[:, :columns], want.expand(N, columns), rtol=1e-15 * (K + 8), atol=0)
     assert (pred[:, columns] == 7.0).all()
+
+
+@pytest.mark.parametrize("N", [500, 30000])
+def test_node_sums_go_to_any_array_of_64_bit_numbers(lb, N):
+    """The kernels' own 16-byte accesses must not reach an array that is aligned to 8 bytes only."""
+    import ctypes as C
+
+    from legateboost_b200.tree import build_tree_arrays
+
+    L = lb.library
+    rs = np.random.RandomState(1)
+    F, K, D = 6, 2, 4
+    M = 2 ** (D + 1) - 1
+    X, g, h = dev(rs.normal(size=(N, F)).astype(np.float32)), dev(rs.normal(size=(N, K))), dev(rs.random((N, K)) + 0.1)
+    want = build_tree_arrays(X, g, h, max_depth=D, split_samples=32, seed=4, row_offset=0, dataset_rows=N)
+    sums = torch.full((M * K * 2 + 2,), -5, dtype=torch.int64, device="cuda")
+    assert sums.data_ptr() % 16 == 0
+    out = [torch.empty((M * K,), dtype=torch.float64, device="cuda") for _ in range(4)] + [torch.empty((M,), dtype=torch.int32, device="cuda")]
+    a = L.BuildTreeArgs()
+    a.X, a.x_dtype, a.ldx, a.g, a.h, a.ldg = X.data_ptr(), L.LBK_F32, F, g.data_ptr(), h.data_ptr(), K
+    a.n_local_rows, a.dataset_rows, a.n_features, a.n_outputs = N, N, F, K
+    a.max_depth, a.max_nodes, a.split_samples, a.seed, a.l2_regularization = D, M, 32, 4, 1.0
+    a.leaf_value, a.split_value, a.gain, a.hessian, a.feature = (t.data_ptr() for t in out)
+    a.stream = torch.cuda.current_stream().cuda_stream
+    a.trace_node_sums = sums.data_ptr() + 8
+    ctx = L.context()
+    ctx.check(ctx.lib.lbk_build_tree(ctx.handle, C.byref(a)))
+    assert torch.equal(sums[1:-1].view(M, K, 2), want["node_sums"])
+    assert sums[0] == -5 and sums[-1] == -5
