@@ -222,7 +222,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
 
   // The kernels work on node sums in the caller's own array where they can: device memory that their 16-byte accesses may
   // go to.  Else the sums are copied there at the end.
-  const bool keep_sums = a.trace_node_sums != nullptr && !a.host_buffers && (reinterpret_cast<uintptr_t>(a.trace_node_sums) & 15) == 0;
+  const bool keep_sums = a.trace_node_sums != nullptr && !a.host_buffers && Aligned16(a.trace_node_sums);
 
   // Tree (reference: struct Tree, build_tree.cu:785-809)
   if (ctx->n_ranks <= 1 && a.sketch_mode == LBK_SKETCH_OFF && a.trace_hist == nullptr &&

@@ -1211,6 +1211,9 @@ struct HistLaunch {
 // nodes: 281 us and 197, 32 nodes: 76 and 65; hence also not many units with rows in them: 60k x 256, 8 nodes: 51 and
 // 43, 64 nodes: 70 and 54 (but 15k x 256, 64 nodes, 234 rows each: 47 and 47; 30k x 200, 256 nodes: 127 and 251).
 //
+// Its wide accesses need the bins and the histograms on 16-byte boundaries (`aligned`); arrays that are not go to the
+// kernels that take them as they are.
+//
 // Four copies pay where a level is cut into about one piece per SM (no more units than SMs) and has something to
 // add: 200k x 40, one node: 33 -> 24 us; 30k x 40, 32 nodes (160 units) would be 19 -> 23 us, 30k x 200, 256 nodes 127
 // -> 215, 5k x 40, one node 17.2 -> 18.7.
@@ -1229,7 +1232,7 @@ void (*SmemKernel(RowOrder order))(HistParams)
                               : order == kPairsByPosition ? k_hist_smem<kFloat, W, kPairsByPosition> : k_hist_smem<kFloat, W, kRowsInOrder>;
 }
 
-HistLaunch PickHistKernel(int bin_bytes, int mb, bool float_mode, RowOrder order, int F, int K, int64_t n_rows, int n_nodes, bool derive, int sm_count, int ranks)
+HistLaunch PickHistKernel(int bin_bytes, int mb, bool float_mode, RowOrder order, int F, int K, int64_t n_rows, int n_nodes, bool derive, int sm_count, int ranks, bool aligned)
 {
   const int n_groups = (F + kGroup - 1) / kGroup;
   const int n_slots   = derive ? n_nodes / 2 : n_nodes;
@@ -1237,7 +1240,7 @@ HistLaunch PickHistKernel(int bin_bytes, int mb, bool float_mode, RowOrder order
   const bool many     = units > sm_count && (derive ? cells / 2 : cells) >= kTileMaxCellsMany && n_rows >= int64_t{512} * n_nodes;
   HistLaunch h;
   h.smem_path = bin_bytes == 1 && mb <= kSmemBins;
-  h.tile      = !float_mode && mb <= 2048 && (bin_bytes == 2 || (h.smem_path && ((cells <= kTileMaxCellsFew && !many) ||
+  h.tile      = !float_mode && aligned && mb <= 2048 && (bin_bytes == 2 || (h.smem_path && ((cells <= kTileMaxCellsFew && !many) ||
                                                    (K == 1 && ranks <= 1 && cells <= kTileMaxCells && units <= 2 * sm_count))));
   h.width     = h.smem_path && n_groups >= 2 ? 2 : 1;
   h.threads   = kHistThreads * h.width;
@@ -1358,7 +1361,7 @@ void HistScratchNeeds(lbk_context* ctx, int F, int K, int bin_bytes, int mb, int
   // what k_hist_smem needs, where some level may take it
   if (bin_bytes != 1 || mb > kSmemBins || n_rows * F * K < kTileMaxCellsMany) return;
   constexpr int64_t kManyRows = int64_t{1} << 36;  // (beyond every bound of the tile form)
-  const HistLaunch hl = PickHistKernel(bin_bytes, mb, false, kPairsByPosition, F, K, kManyRows, 1, false, ctx->sm_count, ctx->n_ranks);
+  const HistLaunch hl = PickHistKernel(bin_bytes, mb, false, kPairsByPosition, F, K, kManyRows, 1, false, ctx->sm_count, ctx->n_ranks, true);
   need.n_arrive       = kTreeFanIn * hl.grid;
   need.partial_bytes  = static_cast<size_t>(need.n_arrive) * mb * kGroup * hl.width * 8;
 }
@@ -1391,7 +1394,8 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
   p.push_len         = lv.push_len;
   p.mb               = lv.max_bins_per_feature;
   p.mb_ptr           = lv.max_bins_ptr;
-  const HistLaunch hl = PickHistKernel(lv.bin_bytes, p.mb, lv.float_mode, OrderOf(p), p.F, p.K, lv.n_rows, p.n_nodes, p.node_sums != nullptr, ctx->sm_count, ctx->n_ranks);
+  const HistLaunch hl = PickHistKernel(lv.bin_bytes, p.mb, lv.float_mode, OrderOf(p), p.F, p.K, lv.n_rows, p.n_nodes, p.node_sums != nullptr, ctx->sm_count, ctx->n_ranks,
+                                       Aligned16(p.bins) && Aligned16(p.out));
 
   const int* max_abs = lv.max_abs;
   if (!lv.float_mode && max_abs == nullptr) {
@@ -1660,7 +1664,8 @@ extern "C" int lbk_histogram_noalloc(int device, const lbk_histogram_args* a)
     p.mb                 = mb;
     p.mb_ptr             = nullptr;
     p.pairs_by_position  = a->pairs_by_position != 0 ? 1 : 0;
-    const HistLaunch hl  = PickHistKernel(a->bin_bytes, mb, float_mode, OrderOf(p), F, K, a->n_rows, a->n_nodes, false, sm_count, 1);
+    const HistLaunch hl  = PickHistKernel(a->bin_bytes, mb, float_mode, OrderOf(p), F, K, a->n_rows, a->n_nodes, false, sm_count, 1,
+                                          Aligned16(p.bins) && Aligned16(p.out));
 
     // the array keeps what the previous call left: clear the words that accumulate
     LBK_CUDA(cudaMemsetAsync(plan, 0, sizeof(int32_t) * 12, stream));

@@ -57,6 +57,8 @@ inline int LevelEnd(int level) { return (1 << (level + 1)) - 1; }
 
 constexpr int kGroup = 32;  // features per feature group (one lane per feature)
 
+inline bool Aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 }  // namespace lbk
 
 namespace lbk {

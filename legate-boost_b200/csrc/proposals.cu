@@ -891,7 +891,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       return;
     }
   }
-  if (bin_bytes == 2 && !use_smem && need <= 2048 && n_rows * F >= kWideMinCells<T>) {
+  if (bin_bytes == 2 && !use_smem && need <= 2048 && n_rows * F >= kWideMinCells<T> && Aligned16(bins_t)) {
     auto wide = [&](auto log2p_, auto copy_) {
       constexpr int L    = decltype(log2p_)::value;
       constexpr bool CT  = decltype(copy_)::value;

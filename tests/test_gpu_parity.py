@@ -1270,3 +1270,41 @@ def test_node_sums_go_to_any_array_of_64_bit_numbers(lb, N):
     ctx.check(ctx.lib.lbk_build_tree(ctx.handle, C.byref(a)))
     assert torch.equal(sums[1:-1].view(M, K, 2), want["node_sums"])
     assert sums[0] == -5 and sums[-1] == -5
+
+
+@pytest.mark.parametrize("N,nb", [(20000, 512), (20000, 1024), (3000, 300)])
+@pytest.mark.parametrize("allocating", [True, False])
+def test_two_byte_histograms_of_arrays_on_any_boundary(lb, N, nb, allocating):
+    """Two-byte bins that begin on 2 bytes and histograms that begin on 8: taken as they are."""
+    import ctypes as C
+
+    L = lb.library
+    rs = np.random.RandomState(nb)
+    F, nodes, Fp = 20, 5, 32
+    ids = np.zeros((N, Fp), dtype=np.int16)
+    ids[:, :F] = rs.randint(0, nb, size=(N, F))
+    from legateboost_b200 import stages
+
+    d_node = dev(rs.randint(0, nodes, size=N).astype(np.int32))
+    row_index, seg = stages.group_rows(d_node, 0, nodes)
+    q, row_ptr = dev(rs.randint(-4000, 4000, size=(N, 1, 2)).astype(np.int32)), dev((np.arange(F + 1) * nb).astype(np.int32))
+    want = torch.zeros((nodes * F * nb, 2), dtype=torch.int64, device="cuda")
+    for f in range(F):
+        want.index_add_(0, (d_node.long() * F + f) * nb + dev(ids[:, f].astype(np.int64)), q[:, 0].long())
+    for shift_bins in (0, 1):
+        for shift_hist in (0, 1):
+            bins = torch.zeros((N * Fp + 8,), dtype=torch.int16, device="cuda")
+            bins[shift_bins:N * Fp + shift_bins] = dev(ids.reshape(-1))
+            hist = torch.full((nodes * F * nb * 2 + 2,), -7, dtype=torch.int64, device="cuda")
+            a = L.HistogramArgs()
+            a.bins, a.bin_bytes, a.n_rows, a.n_features = bins.data_ptr() + 2 * shift_bins, 2, N, F
+            a.row_ptr, a.total_bins, a.gpair, a.n_outputs = row_ptr.data_ptr(), F * nb, q.data_ptr(), 1
+            a.row_index, a.seg, a.n_nodes, a.hist = row_index.data_ptr(), seg.data_ptr(), nodes, hist.data_ptr() + 8 * shift_hist
+            a.stream = torch.cuda.current_stream().cuda_stream
+            ctx = L.context()
+            if allocating:
+                ctx.check(ctx.lib.lbk_histogram(ctx.handle, C.byref(a)))
+            else:
+                assert ctx.lib.lbk_histogram_noalloc(0, C.byref(a)) == 0
+            assert torch.equal(hist[shift_hist:shift_hist + want.numel()], want.view(-1))
+            assert (hist[shift_hist + want.numel():] == -7).all() and (hist[:shift_hist] == -7).all()
