@@ -34,6 +34,11 @@ def _all_sum(t: torch.Tensor) -> torch.Tensor:
     return t
 
 
+def _is_own(model, name: str) -> bool:
+    """Whether a method is _LBBase's own, overridden neither in a subclass nor on the object."""
+    return getattr(getattr(model, name), "__func__", None) is _LBBase.__dict__[name]
+
+
 def _copy_of(base: Tree) -> Tree:
     """deepcopy of a base model, whose attributes are plain values as a rule."""
     if all(type(v) in (int, float, str, bool, type(None)) for v in base.__dict__.values()):
@@ -197,9 +202,10 @@ class _LBBase:
         return self
 
     def _rounds_in_library(self) -> bool:
-        """Whether a round is one `lbk_boost_round` call: plain trees, an objective the library knows, nothing
-        to report per round."""
+        """Whether a round is one `lbk_boost_round` call: plain trees, an objective the library knows, gradients
+        that nobody overrides (sample weights, say), nothing to report per round."""
         return (not self.verbose and self.n_estimators > 0 and type(self._obj) in (_SquaredError, _LogLoss)
+                and _is_own(self, "_weighted_gradient")
                 and all(type(b) is Tree and not callable(b.feature_fraction) and b.max_depth >= 0 for b in self.base_models))
 
     def _fit_rounds(self, X, y, train_pred, layout):
@@ -337,7 +343,7 @@ class LBClassifier(_LBBase):
         return pred
 
     def predict_proba(self, X):
-        if type(self._obj) is not _LogLoss:
+        if type(self._obj) is not _LogLoss or not _is_own(self, "predict_raw"):
             return self._probabilities(self.predict_raw(X))
         return self._predict(X, L.LOGISTIC if self.model_init_.shape[0] == 1 else L.SOFTMAX)
 
