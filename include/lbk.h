@@ -248,7 +248,7 @@ typedef struct lbk_predict_args {
   /* Optional: the table of the trees as a device array that the caller keeps with the ensemble (device
    * buffers only).  leaf_value, feature, split_value and max_nodes are then ignored, nothing is copied to
    * the device and the call is asynchronous on `stream`; a fault that a kernel reports is returned by a
-   * later call on the context. */
+   * later call on the context, and the predictions that it touched are NaN. */
   const lbk_tree_ref* table;
   int32_t table_max_nodes;    /* the largest max_nodes in the table */
   int64_t table_total_nodes;  /* the sum of max_nodes */

@@ -117,8 +117,9 @@ __device__ inline bool MbarTryWait(unsigned bar, unsigned parity)
     : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after about a second, reports through the context's status word and lets
-// the block finish (with wrong sums, which the host then refuses) instead of spinning for ever.
+// Bounded wait: gives up after about a second, reports through the context's status word and lets the block finish instead
+// of spinning for ever.  A call with a table of trees has returned by then, so the warp's sums become NaN: its
+// predictions are not taken for those of the trees that it did see.
 constexpr int kFaultPredictStaging = 21;
 __device__ inline bool MbarWait(unsigned bar, unsigned parity, int* status)
 {
@@ -428,7 +429,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
   const unsigned word_off  = a.rec.split_bytes;
   const unsigned leaf_off  = a.rec.split_bytes + a.rec.word_bytes - (8u << S);
   constexpr unsigned kMask = kMaxFeature - 1;
-  for (int g = 0; g < n_groups; ++g) {
+  int g = 0;
+  for (; g < n_groups; ++g) {
     const int b = a.nbuf == 2 ? g & 1 : 0;
     if (!__all_sync(0xffffffffu, MbarWait(full0 + 8 * b, (g >> 1) & 1, a.status) ? 1 : 0)) break;
     const int nt = min(TG, a.n_trees - g * TG);
@@ -522,6 +524,12 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
     }
   }
 
+  if (g < n_groups) {  // the trees did not come
+#pragma unroll
+    for (int i = 0; i < kSums; ++i) acc[i] = NAN;
+    if (KR < 0)
+      for (int k = 0; k < K; ++k) accs[k * rb + tid] = NAN;
+  }
   const PredictOut& o = a.o;
   const int64_t row   = row0 + tid;
   if (KR == 0) {
