@@ -10,7 +10,7 @@ rank passes its own contiguous block of rows and all ranks get the same tree.
 import copy
 import ctypes as C
 import warnings
-from itertools import chain
+from itertools import accumulate, chain
 from operator import attrgetter, is_
 from typing import Any, Callable, List, Sequence, Union
 
@@ -142,6 +142,7 @@ def build_tree_arrays(X, g, h, *, max_depth, split_samples, seed, l1=0.0, l2=1.0
 
 
 _ARRAYS = attrgetter("leaf_value", "feature", "split_value")
+_ARRAY_TYPES = (torch.float64, torch.int32, torch.float64)
 
 
 class TreeTable:
@@ -150,30 +151,31 @@ class TreeTable:
     new table.  ``arrays``: (leaf_value, feature, split_value) per tree, on one CUDA device."""
 
     def __init__(self, arrays):
+        # (few calls per tensor: an ensemble's first prediction waits for them)
         self.source = list(chain.from_iterable(arrays))
-        device = self.source[1].device
-        keep, rows, total = [], np.empty((len(arrays), 4), dtype=np.int64), 0
-        self.max_nodes, self.n_outputs = 1, 1
-        for i, (lv, ft, sv) in enumerate(arrays):
-            lv = lv.to(torch.float64).contiguous()
-            ft, sv = ft.to(torch.int32).contiguous(), sv.to(torch.float64).contiguous()
-            if ft.device != device or lv.device != device or sv.device != device:
-                raise ValueError("the trees of an ensemble must be on one device")
-            keep += [lv, ft, sv]
-            M = ft.shape[0]
-            if M < 1 or total + M >= 2 ** 31:
-                raise ValueError("bad tree arrays" if M < 1 else "ensemble too large")
-            rows[i] = lv.data_ptr(), ft.data_ptr(), sv.data_ptr(), M | total << 32
-            total += M
-            self.max_nodes = max(self.max_nodes, M)
-            if i == 0:
-                self.n_outputs = lv.shape[1] if lv.dim() == 2 else 1
-            if lv.numel() != M * self.n_outputs or sv.numel() != M:
-                raise ValueError("the trees of an ensemble must have arrays of one shape per node")
+        keep = list(self.source)
+        for i, t in enumerate(keep):
+            want = _ARRAY_TYPES[i % 3]
+            if t.dtype is not want or not t.is_contiguous():
+                keep[i] = t.to(want).contiguous()
+        device = keep[1].device
+        if len(set(map(torch.Tensor.get_device, keep))) > 1:
+            raise ValueError("the trees of an ensemble must be on one device")
+        first = keep[0]
+        self.n_outputs = first.shape[1] if first.dim() == 2 else 1
+        sizes = list(map(torch.Tensor.numel, keep))
+        nodes = sizes[1::3]
+        ends = list(accumulate(nodes))
+        if min(nodes) < 1 or ends[-1] >= 2 ** 31:
+            raise ValueError("bad tree arrays" if min(nodes) < 1 else "ensemble too large")
+        if sizes[0::3] != [m * self.n_outputs for m in nodes] or sizes[2::3] != nodes:
+            raise ValueError("the trees of an ensemble must have arrays of one shape per node")
         # converted copies would not follow later changes of the originals: such a table is not kept
         self.reusable = all(map(is_, keep, self.source))
         self.addresses = list(map(torch.Tensor.data_ptr, self.source))
-        self.keep, self.total_nodes, self.n_trees = keep, total, len(arrays)
+        at = self.addresses if self.reusable else list(map(torch.Tensor.data_ptr, keep))
+        rows = np.array((at[0::3], at[1::3], at[2::3], [m | (e - m) << 32 for m, e in zip(nodes, ends)]), dtype=np.int64).T.copy()
+        self.keep, self.total_nodes, self.max_nodes, self.n_trees = keep, ends[-1], max(nodes), len(nodes)
         self.table = torch.from_numpy(rows).to(device)
         self.device = device
 
