@@ -28,8 +28,8 @@ def _dtype_code(t: torch.Tensor) -> int:
     raise ValueError("X must be float32 or float64")
 
 
-def _stream_ptr(device_index=None):
-    return C.c_void_p(torch.cuda.current_stream(device_index).cuda_stream)
+def _stream_ptr():
+    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def _row_layout(n_local: int):
@@ -178,6 +178,7 @@ class TreeTable:
         self.keep, self.total_nodes, self.max_nodes, self.n_trees = keep, ends[-1], max(nodes), len(nodes)
         self.table = torch.from_numpy(rows).to(device)
         self.device = device
+        self._init, self._streams = None, set()
 
     def matches(self, models) -> bool:
         """Whether these models still hold the very tensors the table was made from, and these still lie
@@ -187,8 +188,27 @@ class TreeTable:
         arrays = list(chain.from_iterable(map(_ARRAYS, models)))
         return all(map(is_, arrays, self.source)) and list(map(torch.Tensor.data_ptr, arrays)) == self.addresses
 
-    def predict(self, X, n_outputs, init=None, transform=L.RAW, ctx=None):
-        """pred (N, columns) float64: ``init`` (n_outputs values, or None) plus the trees' sums, transformed."""
+    def _hold(self, X, init, stream):
+        """The call is queued, and what it reads may have been allocated on another stream: given up by its owner, it
+        must not be handed out there before the call has run.  A tensor has to be told of a stream once (views: the
+        tensor that they are views of)."""
+        X.record_stream(stream)
+        if init is not self._init:
+            self._init = init
+            self._streams.clear()
+        if stream.cuda_stream in self._streams:
+            return
+        held = {id(self.table): self.table}
+        for t in self.keep if init is None else self.keep + [init]:
+            owner = t if t._base is None else t._base
+            held[id(owner)] = owner
+        for t in held.values():
+            t.record_stream(stream)
+        self._streams.add(stream.cuda_stream)
+
+    def predict(self, X, n_outputs, init=None, transform=L.RAW, ctx=None, wait=False):
+        """pred (N, columns) float64: ``init`` (n_outputs values, or None) plus the trees' sums, transformed.  Queued on
+        the current stream, or, with ``wait``, made before the call returns."""
         if X.stride(1) != 1 and X.shape[0] > 0:
             X = X.contiguous()
         N, F = X.shape
@@ -203,21 +223,26 @@ class TreeTable:
         a.X, a.x_dtype, a.ldx, a.n_rows = X.data_ptr(), _dtype_code(X), X.stride(0), N
         a.n_features, a.n_outputs, a.n_trees = F, n_outputs, self.n_trees
         a.pred, a.ldp = pred.data_ptr(), columns
-        a.stream = _stream_ptr(X.device.index)
+        stream = torch.cuda.current_stream(X.device.index)
+        a.stream = stream.cuda_stream
         a.table, a.table_max_nodes, a.table_total_nodes = self.table.data_ptr(), self.max_nodes, self.total_nodes
         a.init, a.transform = init.data_ptr() if init is not None else None, transform
+        if not wait:
+            self._hold(X, init, stream)
         ctx.check(ctx.lib.lbk_predict(ctx.handle, C.byref(a)))
+        if wait:
+            ctx.check(ctx.lib.lbk_synchronize(ctx.handle, a.stream))
         return pred
 
 
 def predict_arrays(X, trees, n_outputs=None, ctx=None):
     """Run ``lbk_predict``.  ``trees`` is a sequence of (leaf_value, feature, split_value) CUDA
-    tensors.  Returns pred (N, K) float64."""
+    tensors.  Returns pred (N, K) float64, when it is made."""
     assert X.is_cuda, "X must be a CUDA tensor (no CPU fallback)"
     if len(trees) == 0:
         return torch.zeros((X.shape[0], n_outputs), dtype=torch.float64, device=X.device)
     table = TreeTable(trees)
-    return table.predict(X, table.n_outputs if n_outputs is None else n_outputs, ctx=ctx)
+    return table.predict(X, table.n_outputs if n_outputs is None else n_outputs, ctx=ctx, wait=True)
 
 
 def onnx_tree_ensemble_attributes(feature, split_value, leaf_value):

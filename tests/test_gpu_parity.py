@@ -1308,3 +1308,35 @@ def test_two_byte_histograms_of_arrays_on_any_boundary(lb, N, nb, allocating):
                 assert ctx.lib.lbk_histogram_noalloc(0, C.byref(a)) == 0
             assert torch.equal(hist[shift_hist:shift_hist + want.numel()], want.view(-1))
             assert (hist[shift_hist + want.numel():] == -7).all() and (hist[:shift_hist] == -7).all()
+
+
+@pytest.mark.parametrize("N", [100, 9000])
+def test_queued_predictions_outlive_the_model_and_the_rows(lb, N):
+    """A prediction is queued on a stream that is busy; its model and rows, made on another stream, are given up, and their
+    memory is asked for again there."""
+    rs = np.random.RandomState(N)
+    Xt, y = dev(rs.normal(size=(2000, 6))), dev(rs.normal(size=2000))
+    X = dev(rs.normal(size=(N, 6)))
+    busy = torch.cuda.Stream()
+    for K in (1, 3):
+        def model():
+            base = (lb.Tree(max_depth=4),)
+            if K == 1:
+                return lb.LBRegressor(n_estimators=5, base_models=base, random_state=0).fit(Xt, y)
+            return lb.LBClassifier(n_estimators=5, base_models=base, random_state=0).fit(Xt, y.argsort() % K)
+
+        m = model()
+        want = m.predict_raw(X)
+        for fresh in (False, True):
+            m, rows = model(), X.clone()
+            if not fresh:
+                m.predict_raw(rows)  # (the table is made on this stream)
+            torch.cuda.synchronize()
+            with torch.cuda.stream(busy):
+                torch.cuda._sleep(200_000_000)
+                got = m.predict_raw(rows)
+            del m, rows
+            junk = [torch.full((n,), float("nan"), dtype=torch.float64, device="cuda") for n in (4, 16, 64, 155, 465, 1000, N * 6) for _ in range(40)]
+            torch.cuda.synchronize()
+            del junk
+            assert torch.equal(got, want), (K, fresh)
