@@ -180,7 +180,12 @@ class _LBBase:
         train_pred = self.model_init_.repeat(X.shape[0], 1)
         layout = _row_layout(X.shape[0])  # this rank's block of rows: the same for every tree
         if self._rounds_in_library():
-            self._fit_rounds(X, y, train_pred, layout)
+            try:
+                self._fit_rounds(X, y, train_pred, layout)
+            except BaseException:
+                # the rounds before the one that failed are queued and read the caller's tensors
+                torch.cuda.current_stream(X.device).synchronize()
+                raise
             self._train_pred = train_pred
             return self
         sketches = {}

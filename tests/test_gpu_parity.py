@@ -1340,3 +1340,21 @@ def test_queued_predictions_outlive_the_model_and_the_rows(lb, N):
             torch.cuda.synchronize()
             del junk
             assert torch.equal(got, want), (K, fresh)
+
+
+def test_a_round_that_fails_waits_for_the_rounds_before_it(lb):
+    rs = np.random.RandomState(0)
+    X, y = dev(rs.normal(size=(500, 4))), dev(rs.normal(size=500))
+    bad = lb.Tree(max_depth=3)
+    bad.split_samples = 4096  # (refused by the library, on the host)
+    m = lb.LBRegressor(n_estimators=4, base_models=(lb.Tree(max_depth=3), bad), random_state=0)
+    lb.LBRegressor(n_estimators=1, base_models=(lb.Tree(max_depth=3),), random_state=0).fit(X, y)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(200_000_000)
+        with pytest.raises(lb.library.LbkError, match="split_samples"):
+            m.fit(X, y)
+        assert stream.query()
+    assert m.models_ == []
+    lb.LBRegressor(n_estimators=1, base_models=(lb.Tree(max_depth=3),), random_state=0).fit(X, y)
