@@ -605,7 +605,20 @@ __global__ void __launch_bounds__(128)
     for (int k = 0; k < K; ++k) pred[k] = o.init[k] + pred[k];
 }
 
-// How the tiled kernel is cut.  rb == 0: the shape does not fit.
+// How the tiled kernel is cut.  rb == 0: the shape does not fit, or fewer than kTileMinRows rows do on an SM (one output:
+// if they are of more than kTileOneWarpBytes).
+//
+// A single warp per SM does not hide the walks' latency; nodes and rows are then read through the caches
+// (k_predict_global), which is fast where the trees ask for few of the features and slow where they ask for all of
+// them, while the tile's time does not depend on that.  Microseconds, tile and caches, 200k rows, 100 fitted trees of
+// depth 6: two warps, float32, 700 features, splits on five of them 662 and 422, on all of them 664 and 2278 (30k rows:
+// 144 and 270, 147 and 345); 850 features 1112 and 432, 1112 and 2367; three classes, 700 features 672 and 348, 673
+// and 1227; float64, 350 features 660 and 457, 660 and 2294; 20 outputs, 50 trees on random features, 100k rows 1060
+// and 2123.  One warp: float32, 1000 features 1492 and 439, 1493 and 2418; three classes 1542 and 353, 1540 and 1285.  Shorter rows come to one warp
+// beside deep trees: float64, 300 features, ten classes, 15 trees of depth 9 1354 and 840; with one output they stay
+// (float32, 600 features, 30 trees of depth 9, splits on all of them 906 and 1010).
+constexpr int kTileMinRows         = 64;
+constexpr size_t kTileOneWarpBytes = 2560;
 struct TilePlan {
   int rb = 0, tg = 0, nbuf = 0;
   unsigned x_bytes = 0;
@@ -648,7 +661,7 @@ TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, i
       best.rec     = rec;
     }
   }
-  if (best.rb == 0) return best;
+  if (best.rb == 0 || (best_res * best.rb < kTileMinRows && (K > 1 || sizeof(T) * F > kTileOneWarpBytes))) return TilePlan{};
   const int64_t slots = static_cast<int64_t>(ctx->sm_count) * best_res;
   const int64_t waves = (n_rows + best.rb * slots - 1) / (best.rb * slots);
   best.rb             = static_cast<int>(((n_rows + waves * slots - 1) / (waves * slots) + 31) / 32 * 32);
@@ -718,13 +731,7 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   // a walk through M heap-ordered nodes takes at most S = floor(log2(M)) steps
   int S = 0;
   while ((2 << S) <= m_max) ++S;
-  // Rows of more than kTileMaxRowBytes leave room for fewer than 64 beside the trees, and two warps per SM do not hide the
-  // walks' latency: nodes and rows are then read through the caches (200k rows, 100 trees of depth 6, tile and that, us:
-  // float32 512 features 425 and 583, 700: 668 and 489, 1000: 1500 and 510; float64 250: 416 and 513, 350: 667 and
-  // 538, 512: 1520 and 629; 100k rows, depth 9, float64 350: 843 and 845).
-  constexpr size_t kTileMaxRowBytes = 2560;
-  static_assert(kTileMaxRowBytes / sizeof(T) <= kMaxFeature, "feature ids must fit a word's fields");
-  const TilePlan plan = S <= 14 && F * sizeof(T) <= kTileMaxRowBytes ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
+  const TilePlan plan = S <= 14 && F <= kMaxFeature ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
   if (plan.rb == 0) {
     NodeT* nodes   = s.alloc<NodeT>(total_nodes);
     double* leaves = s.alloc<double>(total_nodes * K);

@@ -853,8 +853,9 @@ def random_trees(rs, F, K, T, D):
 @pytest.mark.parametrize("N,F,K,T,D", [
     (8193, 1, 1, 1, 0), (8200, 7, 1, 8, 1), (20011, 100, 1, 17, 8),   # one group, whole groups, a last group of one
     (9001, 5, 1, 3, 10), (9001, 40, 1, 30, 13), (8193, 3, 2, 9, 14),  # narrower groups and blocks for deep trees
-    (8193, 320, 1, 5, 3), (8193, 640, 1, 5, 3), (8193, 641, 2, 5, 3), # the widest rows of a tile (f64, f32); wider
-    (8193, 1025, 1, 3, 9),
+    (8193, 425, 1, 17, 6), (8193, 426, 1, 17, 6),                     # the widest rows of a tile, and wider (f64)
+    (8193, 851, 1, 17, 6), (8193, 852, 1, 17, 6),                     # ... (f32)
+    (8193, 700, 3, 9, 6), (8193, 800, 20, 5, 3), (8193, 1025, 1, 3, 9),
     (8193, 12, 2, 9, 6), (30001, 20, 4, 8, 7), (8193, 3, 5, 16, 5), (8193, 9, 8, 10, 5),  # sums in registers
     (8193, 4, 16, 3, 4), (8193, 4, 17, 11, 4),                        # ... the most of them; in shared memory
     (8193, 60, 1, 16, 6), (8193, 136, 1, 16, 6),                      # 48 KB of dynamic shared memory to the byte (f64, f32)
