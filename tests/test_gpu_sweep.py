@@ -60,6 +60,39 @@ def test_random_trees_match_the_oracle(seed):
         assert torch.equal(got["leaf_value"][got["leaf"].long()], pred), what
 
 
+@pytest.mark.parametrize("N,F,K,S", [
+    (16385, 9, 1, 256), (16400, 1, 1, 16), (20000, 65, 1, 100),  # just more rows than the one-launch form takes
+    (8200, 13, 2, 200), (5500, 20, 3, 64), (3300, 33, 5, 256),   # ... rows x outputs; fewer and more outputs than pairs are moved of
+    (300, 640, 1, 32),                                           # ... more features
+])
+@pytest.mark.parametrize("D", [1, 2, 7, 10])
+@pytest.mark.parametrize("kind", ["plain", "ties", "hessians that quantise to 0", "mask"])
+def test_trees_of_the_general_path_match_the_oracle(N, F, K, S, D, kind):
+    """Nothing traced and at most 256 samples: the layout is made for the upper bound of bins, the last level's histograms
+    are not written and its left sums are scanned again."""
+    from legateboost_b200.tree import build_tree_arrays
+    from oracle import oracle as O
+
+    rs = np.random.RandomState(N + D)
+    X = rs.normal(size=(N, F)).astype(np.float32 if D % 2 else np.float64)
+    if kind == "ties":
+        X = np.round(X * 2) / 2
+    g, h = rs.normal(size=(N, K)), rs.random((N, K)) * (1e-4 if "hessians" in kind else 1.0)
+    if kind == "ties":
+        h[:] = 1.0
+    mask = None
+    if kind == "mask":
+        mask = rs.random(F) < 0.5
+        mask[rs.randint(F)] = True
+    kw = dict(l1=0.1, l2=0.5, min_split_gain=0.01) if kind == "mask" else {}
+    want = O.build_tree(X, g, h, max_depth=D, split_samples=S, seed=77, mode="Q", feature_set=mask, **kw)
+    got = build_tree_arrays(_dev(X), _dev(g), _dev(h), max_depth=D, split_samples=S, seed=77,
+                            feature_set=None if mask is None else torch.from_numpy(mask), row_offset=0, dataset_rows=N,
+                            want_node_sums=False, **kw)
+    for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
+        assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
+
+
 def _reference_histogram(bins, pairs, node, node_begin, n_nodes, F, nb, K, dtype):
     """[node][k][feature * nb + bin] sums of the pairs of the rows whose node lies in the level."""
     dev = bins.device
