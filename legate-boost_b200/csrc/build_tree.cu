@@ -226,7 +226,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
 
   // Tree (reference: struct Tree, build_tree.cu:785-809)
   if (ctx->n_ranks <= 1 && a.sketch_mode == LBK_SKETCH_OFF && a.trace_hist == nullptr &&
-      SmallTreeFits(ctx, N, F, K, D, a.split_samples, sizeof(T))) {
+      SmallTreeFits(ctx, N, F, K, D, a.split_samples)) {
     SmallTreeArgs<T> t{};
     t.X            = X;
     t.ldx          = ldx;

@@ -397,7 +397,7 @@ struct SmallTreeArgs {
   unsigned int* barrier;  // device word, zero; this tree's alone
   int32_t* info_host;     // mapped host word for the number of bins, or null
 };
-bool SmallTreeFits(lbk_context* ctx, int64_t N, int F, int K, int D, int S, size_t elem);
+bool SmallTreeFits(lbk_context* ctx, int64_t N, int F, int K, int D, int S);
 template <typename T>
 void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStream_t stream);
 // predict.cu

@@ -39,8 +39,7 @@
 namespace lbk {
 namespace {
 
-// `foff` = feature index times a caller-chosen multiplier (the byte pitch of the staged tile for
-// the tiled kernel, 1 for the fallback), or -1 for a leaf
+// Nodes of the fallback; `foff` = feature index, or -1 for a leaf
 struct Node8 {
   float split;
   int foff;
@@ -76,7 +75,7 @@ __device__ inline void MakeNode(Node16& n, double split, int foff)
 // A split node whose children would fall outside the arrays is treated as a leaf, so a walk can
 // never leave the tree whatever the input arrays hold.
 template <typename NodeT>
-__global__ void k_pack_trees(const TreePtrs* __restrict__ trees, int K, int F, int xmul, NodeT* __restrict__ nodes,
+__global__ void k_pack_trees(const TreePtrs* __restrict__ trees, int K, int F, NodeT* __restrict__ nodes,
                              double* __restrict__ leaves)
 {
   const TreePtrs t = trees[blockIdx.x];
@@ -84,7 +83,7 @@ __global__ void k_pack_trees(const TreePtrs* __restrict__ trees, int K, int F, i
     int f = t.feature[i];
     if (2 * i + 2 >= t.max_nodes || f < 0 || f >= F) f = -1;
     NodeT n;
-    MakeNode(n, t.split[i], f < 0 ? -1 : f * xmul);
+    MakeNode(n, t.split[i], f);
     nodes[t.node_off + i] = n;
   }
   for (int64_t i = threadIdx.x; i < static_cast<int64_t>(t.max_nodes) * K; i += blockDim.x)
@@ -735,7 +734,7 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   if (plan.rb == 0) {
     NodeT* nodes   = s.alloc<NodeT>(total_nodes);
     double* leaves = s.alloc<double>(total_nodes * K);
-    k_pack_trees<NodeT><<<n_trees, 256, 0, stream>>>(d_trees, K, F, 1, nodes, leaves);
+    k_pack_trees<NodeT><<<n_trees, 256, 0, stream>>>(d_trees, K, F, nodes, leaves);
     LBK_LAUNCH_CHECK();
     const unsigned grid = static_cast<unsigned>((n_rows + 127) / 128);
     k_predict_global<T><<<grid, 128, 0, stream>>>(X, ldx, n_rows, K, n_trees, d_trees, nodes, leaves, o);

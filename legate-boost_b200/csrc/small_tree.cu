@@ -425,14 +425,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
             const int64_t at_a = (static_cast<int64_t>(ja) * K + k) * kSmallBins + b, at_b = (static_cast<int64_t>(jb) * K + k) * kSmallBins + b;
             const int* hs      = s_hist + i * 4 * kSmallBins;
             double* gains      = s_gain + i * 2 * kSmallBins;
-            GPairI64 va[1] = {{0, 0}}, vb[1] = {{0, 0}};
-            double ga[1] = {0.0}, gb[1] = {0.0};
+            GPairI64 va{0, 0}, vb{0, 0};
+            double ga = 0.0, gb = 0.0;
             if (in) {
-              if (derive && scanned) vb[0] = LoadPairStreaming(par_f + (static_cast<int64_t>(u) * K + k) * kSmallBins + b);
-              va[0].grad = static_cast<long long>(hs[b]) * 65536 + static_cast<unsigned>(hs[kSmallBins + b]);
-              va[0].hess = static_cast<long long>(hs[2 * kSmallBins + b]) * 65536 + static_cast<unsigned>(hs[3 * kSmallBins + b]);
+              if (derive && scanned) vb = LoadPairStreaming(par_f + (static_cast<int64_t>(u) * K + k) * kSmallBins + b);
+              va.grad = static_cast<long long>(hs[b]) * 65536 + static_cast<unsigned>(hs[kSmallBins + b]);
+              va.hess = static_cast<long long>(hs[2 * kSmallBins + b]) * 65536 + static_cast<unsigned>(hs[3 * kSmallBins + b]);
             }
-            long long sg = va[0].grad, sh = va[0].hess;
+            long long sg = va.grad, sh = va.hess;
 #pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
               const long long ng = __shfl_up_sync(0xffffffffu, sg, off);
@@ -453,32 +453,32 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
               }
             }
             if (in) {
-              if (scanned && (sg > 0 || sh > 0)) va[0] = GPairI64{sg, sh};
-              vb[0] = scanned && derive ? GPairI64{vb[0].grad - va[0].grad, vb[0].hess - va[0].hess} : GPairI64{0, 0};
+              if (scanned && (sg > 0 || sh > 0)) va = GPairI64{sg, sh};
+              vb = scanned && derive ? GPairI64{vb.grad - va.grad, vb.hess - va.hess} : GPairI64{0, 0};
               if (write_hist || K > 1) {
-                StorePair(hist_f + at_a, va[0]);
-                if (derive) StorePair(hist_f + at_b, vb[0]);
+                StorePair(hist_f + at_a, va);
+                if (derive) StorePair(hist_f + at_b, vb);
               }
             }
             unsigned ok_a = eval_a && in ? 1u : 0u, ok_b = eval_b && in ? 1u : 0u;
             if (K > 1 && in) {  // the gains so far are in shared memory, -1e300 = a side without hessian
-              ga[0] = gains[b];
-              gb[0] = gains[kSmallBins + b];
-              if (ga[0] < -1e299) ok_a = 0u;
-              if (gb[0] < -1e299) ok_b = 0u;
+              ga = gains[b];
+              gb = gains[kSmallBins + b];
+              if (ga < -1e299) ok_a = 0u;
+              if (gb < -1e299) ok_b = 0u;
             }
-            if (__any_sync(0xffffffffu, ok_a)) ok_a = AddGains<1>(va, ok_a, TermsOf(sum_a, qp, l1, reg), qp, l1, reg, msg, ga);
-            if (__any_sync(0xffffffffu, ok_b)) ok_b = AddGains<1>(vb, ok_b, TermsOf(sum_b, qp, l1, reg), qp, l1, reg, msg, gb);
+            if (__any_sync(0xffffffffu, ok_a)) ok_a = AddGain(va, ok_a, TermsOf(sum_a, qp, l1, reg), qp, l1, reg, msg, ga);
+            if (__any_sync(0xffffffffu, ok_b)) ok_b = AddGain(vb, ok_b, TermsOf(sum_b, qp, l1, reg), qp, l1, reg, msg, gb);
             if (k < K - 1) {
               if (in) {
-                gains[b]              = ok_a ? ga[0] : -1e300;
-                gains[kSmallBins + b] = ok_b ? gb[0] : -1e300;
+                gains[b]              = ok_a ? ga : -1e300;
+                gains[kSmallBins + b] = ok_b ? gb : -1e300;
               }
               __syncthreads();  // s_tot is written again
               continue;
             }
             // the best bin of either node: of the warp, then of the unit's eight warps
-            const double gain_a = ok_a && ga[0] > 0 ? ga[0] : 0.0, gain_b = ok_b && gb[0] > 0 ? gb[0] : 0.0;
+            const double gain_a = ok_a && ga > 0 ? ga : 0.0, gain_b = ok_b && gb > 0 ? gb : 0.0;
             const int bin_a = WarpBest(gain_a, s_rp[f] + b), bin_b = derive ? WarpBest(gain_b, s_rp[f] + b) : -1;
             if (bin_a < 0 ? lane == 0 : bin_a == s_rp[f] + b) s_best[grp][0][gw] = Cand{gain_a, bin_a, b};
             if (bin_b < 0 ? lane == 0 : bin_b == s_rp[f] + b) s_best[grp][1][gw] = Cand{gain_b, bin_b, b};
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                 const int64_t at = static_cast<int64_t>(j) * F + f;
                 if (b == 0) cand[at] = SmallCand{best.gain, best.bin < 0 ? -1 : best.feature, 0};  // (feature: the bin of the feature)
                 if (K == 1) {
-                  if (best.bin >= 0 && b == best.feature) StorePair(cand_left + at, side == 0 ? va[0] : vb[0]);
+                  if (best.bin >= 0 && b == best.feature) StorePair(cand_left + at, side == 0 ? va : vb);
                 } else if (best.bin >= 0) {
                   // (written by threads of this block, before the barrier)
                   for (int kk = b; kk < K; kk += kSmallBins)
@@ -627,9 +627,8 @@ struct SmallPlan {
   size_t smem;
 };
 
-static bool PlanSmall(lbk_context* ctx, int64_t N, int F, int K, int D, int S, size_t elem, SmallPlan& plan)
+static bool PlanSmall(lbk_context* ctx, int64_t N, int F, int K, int D, int S, SmallPlan& plan)
 {
-  (void)elem;
   // One-byte bins; 16-bit node ids; the canonical sum's second step in one piece.  The bound on rows x outputs
   // is where the general path catches up: a block passes over all rows on every level.
   if (S > kSmallBins || D < 1 || D > 12 || N < 1 || N * K > kSmallMaxElements || F > 4 * ctx->sm_count) return false;
@@ -655,17 +654,17 @@ static bool PlanSmall(lbk_context* ctx, int64_t N, int F, int K, int D, int S, s
   return true;
 }
 
-bool SmallTreeFits(lbk_context* ctx, int64_t N, int F, int K, int D, int S, size_t elem)
+bool SmallTreeFits(lbk_context* ctx, int64_t N, int F, int K, int D, int S)
 {
   SmallPlan plan;
-  return PlanSmall(ctx, N, F, K, D, S, elem, plan);
+  return PlanSmall(ctx, N, F, K, D, S, plan);
 }
 
 template <typename T>
 void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStream_t stream)
 {
   SmallPlan plan;
-  LBK_EXPECT(PlanSmall(ctx, a.N, a.F, a.K, a.D, a.S, sizeof(T), plan), "shape outside the small form");
+  LBK_EXPECT(PlanSmall(ctx, a.N, a.F, a.K, a.D, a.S, plan), "shape outside the small form");
   const int N = static_cast<int>(a.N), F = a.F, K = a.K, D = a.D;
   const int64_t level = int64_t{1} << (D - 1);
   SmallParams<T> p{};

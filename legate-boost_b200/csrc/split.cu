@@ -148,8 +148,8 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs ? 3 : 4)
     const bool search = p.sp.feature_set == nullptr || p.sp.feature_set[f] != 0;
     for (int base = fb; base < fe; base += kSplitThreads) {
       const bool in = base + tid < fe;
-      double gain_a[1] = {0.0}, gain_b[1] = {0.0};
-      GPairI64 va[1], vb[1] = {{0, 0}};
+      double gain_a = 0.0, gain_b = 0.0;
+      GPairI64 va, vb{0, 0};
       unsigned ok_a = eval_a && search && in ? 1u : 0u, ok_b = eval_b && search && in ? 1u : 0u;
       // (several outputs: the next output's sums are on their way while this one's are scanned, for which 24 warps
       // an SM instead of 32 are the price: 1M x 100, 10 outputs, 128 nodes: 416 -> 386 us)
@@ -166,17 +166,17 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs ? 3 : 4)
         }
         const bool scanned = ta.h > 0.0;  // else the raw values stay and no sibling is derived
         if (kManyOutputs) {
-          va[0] = ahead_a;
-          if (kDerive) vb[0] = ahead_b;
+          va = ahead_a;
+          if (kDerive) vb = ahead_b;
           if (in && k + 1 < K) {
             ahead_a = LoadPair(src + at + Bs);
             if (kDerive) ahead_b = LoadPair(par + at + Bs);
           }
         } else {
-          va[0] = in ? LoadPair(src + at) : GPairI64{0, 0};
-          if (kDerive) vb[0] = in && scanned ? LoadPair(par + at) : GPairI64{0, 0};
+          va = in ? LoadPair(src + at) : GPairI64{0, 0};
+          if (kDerive) vb = in && scanned ? LoadPair(par + at) : GPairI64{0, 0};
         }
-        long long sg = va[0].grad, sh = va[0].hess;
+        long long sg = va.grad, sh = va.hess;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
           const long long ng = __shfl_up_sync(0xffffffffu, sg, off);
@@ -207,32 +207,32 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs ? 3 : 4)
           if (tid == kSplitThreads - 1) s_carry[kManyOutputs ? k : 0] = GPairI64{sg, sh};
         }
         if (in) {
-          if (scanned && (sg > 0 || sh > 0)) va[0] = GPairI64{sg, sh};
-          if (kDerive) vb[0] = scanned ? GPairI64{vb[0].grad - va[0].grad, vb[0].hess - va[0].hess} : GPairI64{0, 0};
+          if (scanned && (sg > 0 || sh > 0)) va = GPairI64{sg, sh};
+          if (kDerive) vb = scanned ? GPairI64{vb.grad - va.grad, vb.hess - va.hess} : GPairI64{0, 0};
           if (lv.write_hist) {
-            StorePair(dst_a + at, va[0]);
-            if (kDerive) StorePair(dst_b + at, vb[0]);
+            StorePair(dst_a + at, va);
+            if (kDerive) StorePair(dst_b + at, vb);
           }
           if (lv.next_built != nullptr) {
             StorePair(next_a + at, GPairI64{0, 0});
             if (kDerive) StorePair(next_b + at, GPairI64{0, 0});
           }
         }
-        if (__any_sync(0xffffffffu, ok_a)) ok_a = AddGains<1>(va, ok_a, ta, qp, l1, reg, msg, gain_a);
-        if (kDerive && __any_sync(0xffffffffu, ok_b)) ok_b = AddGains<1>(vb, ok_b, tb, qp, l1, reg, msg, gain_b);
+        if (__any_sync(0xffffffffu, ok_a)) ok_a = AddGain(va, ok_a, ta, qp, l1, reg, msg, gain_a);
+        if (kDerive && __any_sync(0xffffffffu, ok_b)) ok_b = AddGain(vb, ok_b, tb, qp, l1, reg, msg, gain_b);
       }
-      if (ok_a && gain_a[0] > 0) {
-        const Cand c{gain_a[0], base + tid, f};
+      if (ok_a && gain_a > 0) {
+        const Cand c{gain_a, base + tid, f};
         if (Better(c, best_a)) {
           best_a = c;
-          if (!kManyOutputs) left_a = va[0];
+          if (!kManyOutputs) left_a = va;
         }
       }
-      if (kDerive && ok_b && gain_b[0] > 0) {
-        const Cand c{gain_b[0], base + tid, f};
+      if (kDerive && ok_b && gain_b > 0) {
+        const Cand c{gain_b, base + tid, f};
         if (Better(c, best_b)) {
           best_b = c;
-          if (!kManyOutputs) left_b = vb[0];
+          if (!kManyOutputs) left_b = vb;
         }
       }
     }

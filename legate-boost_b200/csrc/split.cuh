@@ -70,42 +70,24 @@ __device__ inline double LeafNumerator(double g, double l1)
   return z * z;
 }
 
-// The gains of one output at kRun bins of a lane, added to gain[] where `ok` has the bin's bit; bits are cleared
-// where a side has no positive hessian (sums are below 2^51, so their differences are exact in float64).  All
-// lanes of a warp call it.
-template <int kRun>
-__device__ inline unsigned AddGains(const GPairI64 (&left)[kRun], unsigned ok, const NodeTerms& n, const QuantParams& qp,
-                                    double l1, double reg, double msg, double (&gain)[kRun])
+// The gain of one output at a lane's bin, added to `gain` where `ok`; returns whether both sides have a positive hessian
+// too (sums are below 2^51, so their differences are exact in float64).  All lanes of a warp call it.
+__device__ inline unsigned AddGain(const GPairI64& left, unsigned ok, const NodeTerms& n, const QuantParams& qp, double l1,
+                                   double reg, double msg, double& gain)
 {
-  double na[kRun], da[kRun], nb[kRun], db[kRun];
-  bool plain = true;
-#pragma unroll
-  for (int i = 0; i < kRun; ++i) {
-    const double lg = WholeToDouble(left[i].grad), lh = WholeToDouble(left[i].hess);
-    const double rg = n.g - lg, rh = n.h - lh;
-    if (lh <= 0.0 || rh <= 0.0) ok &= ~(1u << i);
-    na[i] = LeafNumerator(lg * qp.inv_g, l1);
-    nb[i] = LeafNumerator(rg * qp.inv_g, l1);
-    da[i] = lh * qp.inv_h + reg;
-    db[i] = rh * qp.inv_h + reg;
-    plain = plain && (!(ok & (1u << i)) || (DivisionIsPlain(na[i], da[i]) && DivisionIsPlain(nb[i], db[i])));
+  const double lg = WholeToDouble(left.grad), lh = WholeToDouble(left.hess);
+  const double rg = n.g - lg, rh = n.h - lh;
+  if (lh <= 0.0 || rh <= 0.0) ok = 0u;
+  double a = LeafNumerator(lg * qp.inv_g, l1), b = LeafNumerator(rg * qp.inv_g, l1);
+  const double da = lh * qp.inv_h + reg, db = rh * qp.inv_h + reg;
+  if (__all_sync(0xffffffffu, ok == 0u || (DivisionIsPlain(a, da) && DivisionIsPlain(b, db)))) {
+    a = DividePlain(a, da);
+    b = DividePlain(b, db);
+  } else if (ok != 0u) {
+    a = a / da;
+    b = b / db;
   }
-  if (__all_sync(0xffffffffu, plain)) {
-#pragma unroll
-    for (int i = 0; i < kRun; ++i) {
-      na[i] = DividePlain(na[i], da[i]);
-      nb[i] = DividePlain(nb[i], db[i]);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < kRun; ++i) {
-      if (!(ok & (1u << i))) continue;
-      na[i] = na[i] / da[i];
-      nb[i] = nb[i] / db[i];
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < kRun; ++i) gain[i] += (0.5 * (na[i] + nb[i] - n.gain)) - msg;
+  gain += (0.5 * (a + b - n.gain)) - msg;
   return ok;
 }
 
