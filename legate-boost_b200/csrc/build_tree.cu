@@ -5,7 +5,7 @@
 //   :1191-1258 batching of a level when its histograms exceed the cache, :1154-1187 root,
 //   :826-845 outputs.
 // Differences in how, not in what: bins and quantised pairs are computed once per tree; rows are
-// kept grouped by node with a stable partition instead of a radix sort; only the nodes that are
+// kept grouped by node with a two-way partition instead of a radix sort; only the nodes that are
 // built are held in the reduction buffer that crosses ranks; a level is three launches (histograms, scan
 // and split search, repartition), enqueued without host synchronisation (where the number of bins decides
 // the layout the call waits once, for that number).

@@ -29,7 +29,7 @@
 //   * matrices of moderate size, and bins of two bytes, are built by k_hist_tile: many small blocks with
 //     the histograms of eight features each;
 //   * a node built in one piece owns its output region and flushes with plain stores, turned in
-//     shared memory so that the bins of a feature leave as whole 128-byte lines; the pieces of a
+//     shared memory so that four bins of a feature leave as 64 contiguous bytes; the pieces of a
 //     node that reaches over a range boundary meet in a merge tree of arrival counters in which
 //     nobody waits (k_hist_smem); without scratch for the tree: 64-bit global atomics; chunks of
 //     <= 128 rows skip shared memory.
@@ -1210,6 +1210,8 @@ struct HistLaunch {
 // 264, 100k x 100: 608 and 479.  A unit's histograms are read and cleared whatever they hold: 200k x 200, 256
 // nodes: 281 us and 197, 32 nodes: 76 and 65; hence also not many units with rows in them: 60k x 256, 8 nodes: 51 and
 // 43, 64 nodes: 70 and 54 (but 15k x 256, 64 nodes, 234 rows each: 47 and 47; 30k x 200, 256 nodes: 127 and 251).
+// These points are all there is: the lines between them follow the points, not a model of the two kernels' costs, and a
+// shape far from all of them may lie on the wrong side.
 //
 // Its wide accesses need the bins and the histograms on 16-byte boundaries (`aligned`); arrays that are not go to the
 // kernels that take them as they are.
