@@ -117,16 +117,17 @@ __device__ inline bool MbarTryWait(unsigned bar, unsigned parity)
   return ok != 0;
 }
 // Bounded wait: gives up after about a second, reports through the context's status word and lets the block finish instead
-// of spinning for ever.  A call with a table of trees has returned by then, so the warp's sums become NaN: its
-// predictions are not taken for those of the trees that it did see.
+// of spinning for ever.  A call with a table of trees has returned by then, so the producer warp makes the
+// block's predictions NaN: they are not taken for those of the trees that it did see.
 constexpr int kFaultPredictStaging = 21;
-__device__ inline bool MbarWait(unsigned bar, unsigned parity, int* status)
+__device__ inline bool MbarWait(unsigned bar, unsigned parity, int* status, int* failed)
 {
   for (unsigned spin = 0; spin < (1u << 22); ++spin) {
     if (MbarTryWait(bar, parity)) return true;
     if (spin > 64) __nanosleep(256);
   }
   ReportFault(status, kFaultPredictStaging);
+  *failed = 1;
   return false;
 }
 
@@ -349,6 +350,7 @@ template <typename T, int TG, int KR>
 __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledArgs<T> a)
 {
   __shared__ __align__(8) unsigned long long s_bar[4];  // full[2], empty[2]
+  __shared__ int s_failed;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int rb = a.rb, F = a.F, K = a.K, S = a.rec.S;
   T* xs        = reinterpret_cast<T*>(smem_raw);
@@ -361,6 +363,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
   const int64_t row0 = static_cast<int64_t>(blockIdx.x) * rb;
   const int n_groups = (a.n_trees + TG - 1) / TG;
   if (tid == 0) {
+    s_failed = 0;
     for (int b = 0; b < 2; ++b) {
       MbarInit(full0 + 8 * b, 1);
       MbarInit(empty0 + 8 * b, rb / 32);
@@ -375,16 +378,21 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
       bool ok = true;
       for (; g < n_groups && ok; ++g) {
         const int b = a.nbuf == 2 ? g & 1 : 0;
-        if (g >= 2) ok = MbarWait(empty0 + 8 * b, ((g >> 1) - 1) & 1, a.status);
+        if (g >= 2) ok = MbarWait(empty0 + 8 * b, ((g >> 1) - 1) & 1, a.status, &s_failed);
         if (!ok) break;
         const unsigned bytes = min(TG, a.n_trees - g * TG) * rec_bytes;
         MbarExpectTx(full0 + 8 * b, bytes);
         BulkCopy(tree0 + b * buf_bytes, a.records + static_cast<int64_t>(g) * buf_bytes, bytes, full0 + 8 * b);
       }
       // nothing is in flight when the block ends, whatever the other warps waited for
-      for (int h = max(g - 2, 0); h < g; ++h) MbarWait(full0 + 8 * (a.nbuf == 2 ? h & 1 : 0), (h >> 1) & 1, a.status);
+      for (int h = max(g - 2, 0); h < g; ++h) MbarWait(full0 + 8 * (a.nbuf == 2 ? h & 1 : 0), (h >> 1) & 1, a.status, &s_failed);
     }
     __syncthreads();
+    if (s_failed != 0) {  // (the other warps have written what they have)
+      const int columns = a.o.transform == LBK_LOGISTIC ? 2 : K;
+      for (int64_t row = row0 + lane; row < row0 + rb && row < a.n_rows; row += 32)
+        for (int k = 0; k < columns; ++k) a.o.pred[row * a.o.ldp + k] = NAN;
+    }
     return;
   }
 
@@ -428,10 +436,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
   const unsigned word_off  = a.rec.split_bytes;
   const unsigned leaf_off  = a.rec.split_bytes + a.rec.word_bytes - (8u << S);
   constexpr unsigned kMask = kMaxFeature - 1;
-  int g = 0;
-  for (; g < n_groups; ++g) {
+  for (int g = 0; g < n_groups; ++g) {
     const int b = a.nbuf == 2 ? g & 1 : 0;
-    if (!__all_sync(0xffffffffu, MbarWait(full0 + 8 * b, (g >> 1) & 1, a.status) ? 1 : 0)) break;
+    if (!__all_sync(0xffffffffu, MbarWait(full0 + 8 * b, (g >> 1) & 1, a.status, &s_failed) ? 1 : 0)) break;
     const int nt = min(TG, a.n_trees - g * TG);
     unsigned at[TG], base[TG];
 #pragma unroll
@@ -523,12 +530,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
     }
   }
 
-  if (g < n_groups) {  // the trees did not come
-#pragma unroll
-    for (int i = 0; i < kSums; ++i) acc[i] = NAN;
-    if (KR < 0)
-      for (int k = 0; k < K; ++k) accs[k * rb + tid] = NAN;
-  }
   const PredictOut& o = a.o;
   const int64_t row   = row0 + tid;
   if (KR == 0) {
