@@ -30,9 +30,9 @@
 //     the histograms of eight features each;
 //   * a node built in one piece owns its output region and flushes with plain stores, turned in
 //     shared memory so that four bins of a feature leave as 64 contiguous bytes; the pieces of a
-//     node that reaches over a range boundary meet in a merge tree of arrival counters in which
-//     nobody waits (k_hist_smem); without scratch for the tree: 64-bit global atomics; chunks of
-//     <= 128 rows skip shared memory.
+//     node that reaches over a range boundary add to it with 64-bit atomics on whole sectors or, where the
+//     histograms go to other ranks' memory, meet in a merge tree of arrival counters in which nobody
+//     waits (k_hist_smem); chunks of <= 128 rows skip shared memory.
 #include <mutex>
 #include <string>
 
@@ -82,10 +82,11 @@ struct HistParams {
   const int32_t* plan;       // [0] rows per chunk, [1] total chunks, [3] rows between flushes, [4] rows per
                              // range (0 = tickets from the counter), [7] ranges
   int tile_items;            // k_hist_tile: units of work a level is cut into if its nodes alone are fewer
+  bool ranges;               // static ranges may be used
   long long slot_capacity;   // slots and counters of the merge trees
   int n_arrive;
   unsigned int* ticket;
-  unsigned int* arrive;      // counters of the merge trees (zero before the kernel and after it); may be null
+  unsigned int* arrive;      // counters of the merge trees (zero before the kernel and after it); null: no merge trees
   void* partial;             // partial-sum slots of the merge trees: [slot][2][mb * 32 W] of the
                              // accumulator type; may be null
   int pairs_by_position;     // 1: gpair is stored in row_index order (pair i belongs to row_index[i]): a stream
@@ -156,14 +157,16 @@ __global__ void k_max_abs(const int2* __restrict__ gpair, int64_t n, int* __rest
 __device__ inline void RangesOf(const HistParams& p, long long total, int GK, int resident, int& range_rows, int& ranges)
 {
   range_rows = ranges = 0;
-  if (p.arrive == nullptr || GK > resident) return;
+  if (!p.ranges || GK > resident) return;
   int n       = resident / GK;
   long long q = (total + n - 1) / n;
   q           = (q + kTileRows - 1) / kTileRows * kTileRows;
   if (q < 2 * kMinChunk) return;
-  n                     = static_cast<int>((total + q - 1) / q);
-  const long long slots = static_cast<long long>(kTreeFanIn) * (n - 1) * GK;
-  if (slots > p.slot_capacity || slots > p.n_arrive) return;
+  n = static_cast<int>((total + q - 1) / q);
+  if (p.partial != nullptr) {
+    const long long slots = static_cast<long long>(kTreeFanIn) * (n - 1) * GK;
+    if (slots > p.slot_capacity || slots > p.n_arrive) return;
+  }
   range_rows = static_cast<int>(q);
   ranges     = n;
 }
@@ -204,12 +207,12 @@ __device__ inline int TileChunkRows(long long total, int nodes, int largest, int
 //
 // A unit of work is (rows, group set, output), GK = group sets x outputs per row.
 //
-// Static ranges (needs `wpre`, the merge-tree counters and slots): the built rows of the level, laid
+// Static ranges (needs `wpre`): the built rows of the level, laid
 // end to end in node order, are cut into resident / GK equal ranges; block b takes range b / GK
 // for (group set, output) b % GK and walks through the nodes its range touches.  Every block gets the
 // same number of rows whatever the node sizes are (256 equal tickets on 148 blocks would otherwise
 // take two rounds, the second one partly empty).  A node that reaches over a range boundary is
-// built in pieces whose partial sums meet in a merge tree (see k_hist_smem).  Chosen when every
+// built in pieces (see k_hist_smem).  Chosen when every
 // range gets at least 2 * kMinChunk rows.
 //
 // Tickets (everything else): one chunk per node when there are at least as many non-empty nodes as
@@ -416,6 +419,10 @@ struct Acc<false> {
     atomicAdd(reinterpret_cast<unsigned long long*>(&dst->grad), static_cast<unsigned long long>(static_cast<long long>(g)));
     atomicAdd(reinterpret_cast<unsigned long long*>(&dst->hess), static_cast<unsigned long long>(static_cast<long long>(h)));
   }
+  __device__ static void add_word(out_t* dst, int word, int v)
+  {
+    atomicAdd(reinterpret_cast<unsigned long long*>(dst) + word, static_cast<unsigned long long>(static_cast<long long>(v)));
+  }
   __device__ static void store_global(out_t* dst, int g, int h)
   {
     *reinterpret_cast<longlong2*>(dst) = make_longlong2(g, h);
@@ -442,6 +449,7 @@ struct Acc<true> {
     atomicAdd(&dst->grad, static_cast<double>(g));
     atomicAdd(&dst->hess, static_cast<double>(h));
   }
+  __device__ static void add_word(out_t* dst, int word, float v) { atomicAdd(reinterpret_cast<double*>(dst) + word, static_cast<double>(v)); }
   __device__ static void store_global(out_t* dst, float g, float h)
   {
     *reinterpret_cast<double2*>(dst) = make_double2(g, h);
@@ -729,7 +737,14 @@ __device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, in
 // array, conflict free both ways) and writes, per word, the 4 bins of a feature as 64 contiguous
 // bytes of the output.
 //
-// Merge tree (static ranges): the P pieces of a node that reaches over range boundaries are summed
+// The pieces of a node that reaches over range boundaries add their sums to its histogram with 64-bit atomics. An
+// instruction of the warp covers 16 whole (grad, hess) pairs, so that every sector is touched once: 148 blocks adding 256 KB
+// each, all to the same region, take 10 us, as long as plain stores to regions of their own (15 with the two words
+// of a pair in two instructions).  The merge tree took 28 us for the 148 pieces of one node, mostly on few SMs, and
+// scratch for the pieces.  One node, 10M x 64: 240 -> 214 us; 8 nodes 270 -> 241, 128 nodes 277 -> 252; 10M x 128, 128 nodes
+// 470 -> 462; 1.25M x 64, one node 68 -> 46.
+//
+// Merge tree (static ranges, histograms of other ranks' features, where the atomics would cross NVLink): the P pieces of a node that reaches over range boundaries are summed
 // without waits.  A piece writes its 32-bit partial sums to its slot and adds one to the counter
 // of its group of four; the last one to arrive adds the others' slots to its own sums and goes on
 // as one member of the next level, until one block holds the node's total and writes the
@@ -859,12 +874,23 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
 #pragma unroll
             for (int i = 0; i < kFlushBins; ++i) {
               const smem_t hv = stage[b * 32 + ((kWordsPer * i + a + kWordsPer * b) & 31)];
-              const int f     = feature_of_word(half * 32 + kWordsPer * i + a);
-              const int bin   = bin0 + b;
-              if (bin < s_rp[f + 1] - s_rp[f] && A::nonzero(gv[i], hv)) {
-                if (atomics) A::add_global(s_base[f] + bin, gv[i], hv);
-                else A::store_global(s_base[f] + bin, gv[i], hv);
+              if (atomics) {
+                // the lanes of an instruction add to whole sectors: lane l the word l % 2 of the pair that lane
+                // l / 2 (or 16 + l / 2) holds
+#pragma unroll
+                for (int part = 0; part < 2; ++part) {
+                  const int from  = part * 16 + (lane >> 1);
+                  const smem_t vg = __shfl_sync(0xffffffffu, gv[i], from), vh = __shfl_sync(0xffffffffu, hv, from);
+                  const int f     = feature_of_word(half * 32 + kWordsPer * i + from / kFlushBins);
+                  const int bin   = bin0 + from % kFlushBins;
+                  const smem_t v  = (lane & 1) ? vh : vg;
+                  if (bin < s_rp[f + 1] - s_rp[f] && v != smem_t(0)) A::add_word(s_base[f] + bin, lane & 1, v);
+                }
+                continue;
               }
+              const int f   = feature_of_word(half * 32 + kWordsPer * i + a);
+              const int bin = bin0 + b;
+              if (bin < s_rp[f + 1] - s_rp[f] && A::nonzero(gv[i], hv)) A::store_global(s_base[f] + bin, gv[i], hv);
             }
           }
           __syncwarp();
@@ -1361,7 +1387,7 @@ __global__ void k_group_scatter(const int32_t* __restrict__ node_of_row, int64_t
 void HistScratchNeeds(lbk_context* ctx, int F, int K, int bin_bytes, int mb, int64_t n_rows, HistScratch& need)
 {
   // what k_hist_smem needs, where some level may take it
-  if (bin_bytes != 1 || mb > kSmemBins || n_rows * F * K < kTileMaxCellsMany) return;
+  if (ctx->n_ranks <= 1 || bin_bytes != 1 || mb > kSmemBins || n_rows * F * K < kTileMaxCellsMany) return;
   constexpr int64_t kManyRows = int64_t{1} << 36;  // (beyond every bound of the tile form)
   const HistLaunch hl = PickHistKernel(bin_bytes, mb, false, kPairsByPosition, F, K, kManyRows, 1, false, ctx->sm_count, ctx->n_ranks, true);
   need.n_arrive       = kTreeFanIn * hl.grid;
@@ -1413,11 +1439,11 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
   }
   p.max_abs = lv.float_mode ? nullptr : max_abs;
   p.tile_items = ctx->sm_count * kTileItemsPerSm;
-  // static ranges need slots and counters for the merge trees of the nodes that reach over a range
-  // boundary: kTreeFanIn per resident block covers every cut
+  // histograms that go to other ranks' memory: slots and counters for the merge trees of the nodes that reach over a
+  // range boundary, kTreeFanIn per resident block covers every cut
   HistScratch own;
   HistScratch* hs = lv.scratch;
-  const int need_arrive  = hl.smem_path ? kTreeFanIn * hl.grid : 0;
+  const int need_arrive  = hl.smem_path && p.push_recv != nullptr ? kTreeFanIn * hl.grid : 0;
   const size_t need_bytes = static_cast<size_t>(need_arrive) * p.mb * kGroup * hl.width * 8;
   const bool kept = hs != nullptr && hs->next_ticket < hs->n_tickets && hs->n_arrive >= need_arrive && hs->partial_bytes >= need_bytes;
   if (!kept) hs = &own;
@@ -1425,7 +1451,8 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
   p.partial = nullptr;
   p.slot_capacity = 0;
   p.n_arrive = 0;
-  if (hl.smem_path) {
+  p.ranges   = hl.smem_path;
+  if (need_arrive > 0) {
     p.n_arrive      = need_arrive;
     p.slot_capacity = need_arrive;
     if (!kept) {
@@ -1683,6 +1710,7 @@ extern "C" int lbk_histogram_noalloc(int device, const lbk_histogram_args* a)
     }
     // no merge-tree slots here (they would have to be allocated): nodes cut into chunks flush with atomics
     p.wpre      = nullptr;
+    p.ranges    = false;
     p.arrive    = nullptr;
     p.partial   = nullptr;
     p.status    = nullptr;
