@@ -465,49 +465,75 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
 //
 // k_bin_smem is bound by its issue slots and the load/store pipe (72 % each): five instructions for the two
 // levels in registers and three more and a pass for each of the other six.  Here a value is first mapped to one of
-// 512 buckets by t = rint(clamp(x s + b)), of which a table holds the number of proposals in the buckets below; since
+// 512 buckets, of which a table says where the search begins: at the number of proposals in the buckets below.  Since
 // the map never decreases, those are below x and the proposals of the buckets above are not, and what is left to
-// search are the proposals of x's own bucket.  s and b spread the buckets evenly from the fifth proposal to the
-// fifth from the end (beyond them lie four proposals and any outliers).  A block looks how many proposals share a
-// bucket in its features at worst and takes three steps of the search (up to 7: uniform and normal columns), four (up
-// to 15) or, where the values crowd together more, the whole search without the table.  A NaN ends in bucket 0 and
-// fails every comparison: id 0, as in the other kernels.
+// search are the proposals of x's own bucket.  The map spreads the buckets evenly from the fifth proposal to the
+// fifth from the end (beyond them lie four proposals and any outliers): t = x s + b, saturated to [0, 1], then
+// t 511 + 2^23 rounds to the bucket.  A block looks how many proposals share a bucket in its features at worst and
+// takes three steps of the search (up to 7: uniform and normal columns), four (up to 15) or, where the values crowd
+// together more, the whole search without the table.  A NaN ends in bucket 0 and fails every comparison: id 0, as
+// in the other kernels.
 //
-// Blocks of 16 warps share the proposals (34 KB) and the buckets (16 KB); two fit an SM with 64 registers a
-// thread.  The bucket table is [bucket][lane] bytes: a lookup is two passes, four lanes share a word's column.
-// 10M x 64: 1047 -> 841 us, 1M x 100: 285 -> 217 us; 200k x 50 stays at 42 us, filling the tables and two turns of a warp.
-constexpr int kBuckets    = 512;
-constexpr int kLutThreads = 512;
-constexpr int kLutRows    = 256 + 16;  // of the table: the last steps may look beyond the last proposal
-constexpr size_t kLutSmem = sizeof(float) * kGroup * kLutRows + kBuckets * kGroup + (kLutThreads / 32) * kGroup * kBinTilePitch;
+// Shared memory: rows of 256 bytes from the address 32768 on, row j = proposal j of the 32 features | what the
+// bucket j of each feature begins with, as the address of that proposal.  So a lookup and a probe are one pass
+// (bank = lane), the search goes on with what was looked up, and the id is byte 1 of the address it ends at, less 128.
+// A block of 32 warps has one such table; the warps' tiles for the feature-major copy lie before and behind it.  The
+// row-major ids leave as words of four features, turned among four lanes.
+//
+// Bound by HBM and the load/store pipe (about 56 passes and 190 instructions per 256 ids).  With a table of bytes (lookups of
+// three passes), one store per row and eight values ahead: 10M x 64, with the copy, 840 us; now 690 (3.84 GB, for which
+// the copy rate of HBM gives 587); 1M x 100: 221 -> 158; 200k x 50: 42 -> 24, where the fill of the table counts: a thread
+// per feature read the proposals 1 KB apart.  Eight values ahead instead of sixteen, with this layout: 827.
+constexpr int kBuckets         = 512;
+constexpr int kLutThreads      = 1024;
+constexpr int kLutWarps        = kLutThreads / 32;
+constexpr int kLutRows         = 256 + 16;  // of the table: the last steps may look beyond the last proposal
+constexpr unsigned kLutRow     = 2 * kGroup * sizeof(float);
+constexpr unsigned kLutAt      = 32768;     // an id is byte 1 of the address of its row, less 128
+constexpr int kLutTurn         = 32;        // rows of a warp's tile
+constexpr unsigned kLutTile    = kGroup * kLutTurn;
+constexpr int kLutTilesBefore  = 30;        // (1 KB is reserved, the kernel declares less than another)
+constexpr unsigned kLutTilesAt = kLutAt - kLutTilesBefore * kLutTile;
+constexpr unsigned kLutEnd     = kLutAt + kBuckets * kLutRow + (kLutWarps - kLutTilesBefore) * kLutTile;
+constexpr unsigned kLutStageAt = kLutAt + kLutRows * kLutRow;  // (the proposals are turned there before the buckets are made)
+static_assert(kLutTilesAt >= 2048 && kLutStageAt + kLutRows * (kGroup + 1) * 4 <= kLutEnd, "room around the table");
 
 template <bool kCopyT>
-__global__ void __launch_bounds__(kLutThreads, 2)
+__global__ void __launch_bounds__(kLutThreads, 1)
   k_bin_lut(const float* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const float* __restrict__ proposals,
             int64_t cut_stride, const int32_t* __restrict__ row_ptr, uint8_t* __restrict__ bins, uint8_t* __restrict__ bins_t, int64_t pitch_t)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_n[kGroup];
   __shared__ float2 s_map[kGroup];
-  float* sp          = reinterpret_cast<float*>(smem_raw);
-  unsigned char* lut = smem_raw + sizeof(float) * kGroup * kLutRows;
-  const int f0   = blockIdx.y * kGroup;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kWarps = kLutThreads / 32;
-  if (threadIdx.x < kGroup) s_n[threadIdx.x] = f0 + threadIdx.x < F ? row_ptr[f0 + threadIdx.x + 1] - row_ptr[f0 + threadIdx.x] : 0;
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < kLutRows * kGroup; idx += kLutThreads) {
-    const int j = idx >> 5, f = f0 + (idx & 31);
-    sp[idx]     = j < s_n[idx & 31] ? proposals[(cut_stride > 0 ? f * cut_stride : row_ptr[f]) + j] : INFINITY;
+  // (addresses of the shared window as offsets from where the dynamic part begins)
+  unsigned char* window = smem_raw - static_cast<unsigned>(__cvta_generic_to_shared(smem_raw));
+  auto row_of     = [&](int j) { return reinterpret_cast<float*>(window + kLutAt + j * kLutRow); };
+  const int f0    = blockIdx.y * kGroup;
+  const int lane  = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  {
+    // a warp reads the proposals of one feature
+    float* stage = reinterpret_cast<float*>(window + kLutStageAt);
+    const int f  = f0 + warp;
+    int begin = 0, n = 0;
+    if (f < F) {
+      begin = row_ptr[f];
+      n     = row_ptr[f + 1] - begin;
+    }
+    const float* src = proposals + (cut_stride > 0 ? f * cut_stride : begin);
+    for (int j = lane; j < kLutRows; j += 32) stage[j * (kGroup + 1) + warp] = j < n ? src[j] : INFINITY;
+    if (lane == 0) s_n[warp] = n;
+    __syncthreads();
+    for (int j = warp; j < kLutRows; j += kLutWarps) row_of(j)[lane] = stage[j * (kGroup + 1) + lane];
   }
   __syncthreads();
   if (threadIdx.x < kGroup) {
     const int n = s_n[threadIdx.x], end = n >= 32 ? 4 : 0;
     float s = 0.0f, b = 0.0f;
     if (n >= 3) {  // (the last proposal is +inf)
-      const float lo = sp[end * kGroup + threadIdx.x], hi = sp[(n - 2 - end) * kGroup + threadIdx.x];
-      s = (kBuckets - 3) / (hi - lo);
-      b = 1.0f - lo * s;
+      const float lo = row_of(end)[threadIdx.x], hi = row_of(n - 2 - end)[threadIdx.x];
+      s = (kBuckets - 3) / (hi - lo) / (kBuckets - 1);
+      b = 1.0f / (kBuckets - 1) - lo * s;
       if (!(s > 0.0f) || !(s < INFINITY) || !(fabsf(b) < INFINITY)) s = b = 0.0f;  // all in one bucket
     }
     s_map[threadIdx.x] = make_float2(s, b);
@@ -516,111 +542,117 @@ __global__ void __launch_bounds__(kLutThreads, 2)
   const float2 map = s_map[lane];
   // the bucket of x plus the bits of 2^23
   auto bucket_bits = [&](float x) {
-    return __float_as_uint(fminf(fmaxf(__fmaf_rn(x, map.x, map.y), 0.0f), static_cast<float>(kBuckets - 1)) + 8388608.0f);
+    float t;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;\n" : "=f"(t) : "f"(x), "f"(map.x), "f"(map.y));  // (NaN: 0)
+    return __float_as_uint(__fmaf_rn(t, static_cast<float>(kBuckets - 1), 8388608.0f));
   };
+  const unsigned col_s = kLutAt + lane * 4;
   int crowd = 0;  // 1: more than 7 of a feature's proposals share a bucket, 2: more than 15, or they are not in order
   {
-    auto at_of  = [&](int j) { return static_cast<int>(bucket_bits(sp[j * kGroup + lane]) & (kBuckets - 1)); };
+    auto at_of  = [&](int j) { return static_cast<int>(bucket_bits(row_of(j)[lane]) & (kBuckets - 1)); };
+    auto begins = [&](int k, int j) { reinterpret_cast<unsigned*>(row_of(k))[kGroup + lane] = col_s + j * kLutRow; };
     const int n = s_n[lane];
-    for (int j = warp; j < n; j += kWarps) {
+    for (int j = warp; j < n; j += kLutWarps) {
       const int at = at_of(j);
-      for (int k = j > 0 ? at_of(j - 1) + 1 : 0; k <= at; ++k) lut[k * kGroup + lane] = static_cast<unsigned char>(j);
+      for (int k = j > 0 ? at_of(j - 1) + 1 : 0; k <= at; ++k) begins(k, j);
       if (j == n - 1)  // (+inf is in the last bucket, unless all are in the first)
-        for (int k = at + 1; k < kBuckets; ++k) lut[k * kGroup + lane] = 0;
+        for (int k = at + 1; k < kBuckets; ++k) begins(k, 0);
       // the table is only right for proposals in order that end in +inf (a NaN among the samples is neither)
-      const float v = sp[j * kGroup + lane];
-      if (j == n - 1 ? v != INFINITY : !(v < sp[(j + 1) * kGroup + lane])) crowd |= 2;
+      const float v = row_of(j)[lane];
+      if (j == n - 1 ? v != INFINITY : !(v < row_of(j + 1)[lane])) crowd |= 2;
       if (j >= 7 && at_of(j - 7) == at) crowd |= 1;
       if (j >= 15 && at_of(j - 15) == at) crowd |= 2;
     }
     if (n == 0)
-      for (int k = warp; k < kBuckets; k += kWarps) lut[k * kGroup + lane] = 0;
+      for (int k = warp; k < kBuckets; k += kLutWarps) begins(k, 0);
   }
   const int most = __syncthreads_or(crowd & 2) ? 2 : __syncthreads_or(crowd & 1) ? 1 : 0;
   // Lanes beyond the last feature read the last feature's values (in bounds); their column of the
   // table is all +inf, so their ids are 0.
-  const bool active = f0 + lane < F;
-  constexpr unsigned kPitch = kGroup * sizeof(float);
-  const unsigned col_s  = static_cast<unsigned>(__cvta_generic_to_shared(sp + lane));
-  const unsigned lut_s  = static_cast<unsigned>(__cvta_generic_to_shared(lut + lane)) - 0x4b000000u * kGroup;  // (the bits of 2^23)
-  const unsigned tile_s = static_cast<unsigned>(__cvta_generic_to_shared(lut + kBuckets * kGroup + warp * (kGroup * kBinTilePitch)));
+  const bool active     = f0 + lane < F;
+  const unsigned lut_s  = col_s + kGroup * 4 - 0x4b000000u * kLutRow;  // (the bits of 2^23)
+  const unsigned tile_s = warp < kLutTilesBefore ? kLutTilesAt + warp * kLutTile : kLutAt + kBuckets * kLutRow + (warp - kLutTilesBefore) * kLutTile;
   const int pitch   = static_cast<int>(gridDim.y) * kGroup;
   constexpr int U   = 8;  // rows per warp in flight
   const int n       = static_cast<int>(n_rows);
   const int ld      = static_cast<int>(ldx);
-  constexpr int kSubs = kBinTileRows / U;
-  constexpr int kTurn = kBinTileRows;
-  const int hop     = static_cast<int>(gridDim.x) * kWarps * kTurn;  // rows from one turn of a warp to the next
-  int turn          = (blockIdx.x * kWarps + warp) * kTurn;
+  constexpr int kTurn = kLutTurn;
+  static_assert(kTurn == 4 * U, "four times eight rows");
+  const int hop     = static_cast<int>(gridDim.x) * kLutWarps * kTurn;  // rows from one turn of a warp to the next
+  int turn          = (warp * gridDim.x + blockIdx.x) * kTurn;  // (a small matrix is spread over the blocks)
   const float* xcol = X + (active ? f0 + lane : F - 1);
-  uint8_t* ocol     = bins + f0 + lane;
-  // the values of the warp's next eight rows are loaded while the current eight are searched
+  // the lane's word of the row-major ids: row lane % 4 of four, features lane / 4 * 4 and the next three
+  uint8_t* ocol     = bins + static_cast<int64_t>(lane & 3) * pitch + f0 + (lane & ~3);
+  const unsigned sel1 = (lane & 1) ? 0x3715u : 0x6240u, sel2 = (lane & 2) ? 0x3276u : 0x5410u;
+  // four ids of the lane's feature (one per row) -> the ids of four features in the lane's row
+  auto turned = [&](unsigned w) {
+    w = __byte_perm(w, __shfl_xor_sync(0xffffffffu, w, 1), sel1);
+    return __byte_perm(w, __shfl_xor_sync(0xffffffffu, w, 2), sel2);
+  };
+  // Sixteen rows of the warp are on their way or searched: the values of eight are asked for as soon as the eight rows
+  // sixteen before them have been.
   auto load_rows = [&](int first, float (&x)[U]) {
     const float* src = xcol + static_cast<int64_t>(first) * ld;
 #pragma unroll
-    for (int u = 0; u < U; ++u) x[u] = LdgStream(src + static_cast<int64_t>(u) * ld);
+    for (int u = 0; u < U; ++u, src += ld) x[u] = LdgStream(src);  // (a sum per row: eight offsets would take registers)
   };
   auto load_rows_checked = [&](int first, float (&x)[U]) {
     const float* src = xcol + static_cast<int64_t>(first) * ld;
 #pragma unroll
-    for (int u = 0; u < U; ++u) x[u] = first + u < n ? LdgStream(src + static_cast<int64_t>(u) * ld) : -INFINITY;
+    for (int u = 0; u < U; ++u, src += ld) x[u] = first + u < n ? LdgStream(src) : -INFINITY;
   };
-  float xn[U];
-  if (turn < n) load_rows_checked(turn, xn);
+  float xa[U], xb[U];
+  if (turn < n) {
+    load_rows_checked(turn, xa);
+    load_rows_checked(turn + U, xb);
+  }
+  const unsigned swap = lane >> 2;  // the words of a feature's 32 bytes are swapped so that the lanes' stores fall on distinct banks
   // one turn; checked: the turn may reach beyond the last row; levels: steps of the search, 8 = without the buckets
   auto do_turn = [&](auto checked, auto levels) {
     constexpr bool kChecked = decltype(checked)::value;
     constexpr int kLevels   = decltype(levels)::value;
-#pragma unroll 2
-    for (int sub = 0; sub < kSubs; ++sub) {
+    auto eight_rows = [&](int sub, float (&x)[U]) {
       const int base = turn + sub * U;
-      float x[U];
       unsigned pos[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) x[u] = xn[u];
-      {
-        const int nb = sub + 1 < kSubs ? base + U : turn + hop;
-        if (sub + 1 < kSubs && !kChecked) load_rows(nb, xn);
-        else if (nb < n) load_rows_checked(nb, xn);
-      }
       if (kLevels == 8) {
 #pragma unroll
         for (int u = 0; u < U; ++u) pos[u] = col_s;
       } else {
-        unsigned first[U];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          asm volatile("ld.shared.u8 %0, [%1];\n" : "=r"(first[u]) : "r"(lut_s + bucket_bits(x[u]) * kGroup));
-#pragma unroll
-        for (int u = 0; u < U; ++u) pos[u] = col_s + first[u] * kPitch;
+          asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(pos[u]) : "r"(lut_s + bucket_bits(x[u]) * kLutRow));
       }
-      SearchLevels<float, U, kLevels - 1, kPitch>::run(pos, x);
-      unsigned id[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) id[u] = (pos[u] - col_s) / kPitch;
+      SearchLevels<float, U, kLevels - 1, kLutRow>::run(pos, x);
+      if (sub < 2 && !kChecked) load_rows(base + 2 * U, x);
+      else if (sub < 2 || turn + hop < n) load_rows_checked(base + 2 * U + (sub < 2 ? 0 : hop - kTurn), x);
+      // byte 1 of each, less 128
+      const unsigned lo = __byte_perm(__byte_perm(pos[0], pos[1], 0x0051), __byte_perm(pos[2], pos[3], 0x0051), 0x5410) ^ 0x80808080u;
+      const unsigned hi = __byte_perm(__byte_perm(pos[4], pos[5], 0x0051), __byte_perm(pos[6], pos[7], 0x0051), 0x5410) ^ 0x80808080u;
       uint8_t* orow = ocol + static_cast<int64_t>(base) * pitch;
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (!kChecked || base + u < n) orow[u * pitch] = static_cast<uint8_t>(id[u]);
+      const unsigned first4 = turned(lo), last4 = turned(hi);
+      if (!kChecked || base + (lane & 3) < n) *reinterpret_cast<unsigned*>(orow) = first4;
+      if (!kChecked || base + 4 + (lane & 3) < n) *reinterpret_cast<unsigned*>(orow + 4 * pitch) = last4;
       if (kCopyT) {
-        const unsigned lo = id[0] | (id[1] << 8) | (id[2] << 16) | (id[3] << 24);
-        const unsigned hi = id[4] | (id[5] << 8) | (id[6] << 16) | (id[7] << 24);
-        asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(tile_s + lane * kBinTilePitch + sub * U), "r"(lo), "r"(hi)
-                     : "memory");
+        asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(tile_s + lane * kTurn + ((2 * sub) ^ swap) * 4), "r"(lo) : "memory");
+        asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(tile_s + lane * kTurn + ((2 * sub + 1) ^ swap) * 4), "r"(hi) : "memory");
       }
+    };
+#pragma unroll 1
+    for (int sub = 0; sub < 4; sub += 2) {
+      eight_rows(sub, xa);
+      eight_rows(sub + 1, xb);
     }
     if (kCopyT) {
-      // the tile leaves feature by feature, as in k_bin_smem
+      // the tile leaves feature by feature, four of them and the 32 bytes of each per store (rows up to the padded end
+      // of a feature's row of the copy; the ids of rows beyond the last one are 0)
       __syncwarp();
-      const int w    = lane & 15;
-      const bool in  = turn + 4 * w < pitch_t;
-#pragma unroll 4
-      for (int i = 0; i < kGroup / 2; ++i) {
-        const int fl = 2 * i + (lane >> 4);
+      uint8_t* dst = bins_t + static_cast<int64_t>(f0 + (lane >> 3)) * pitch_t + turn + 4 * (lane & 7);
+#pragma unroll
+      for (int i = 0; i < kGroup / 4; ++i) {
         unsigned v;
-        asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(tile_s + fl * kBinTilePitch + 4 * w));
-        if (in && f0 + fl < F)
-          *reinterpret_cast<unsigned*>(bins_t + static_cast<int64_t>(f0 + fl) * pitch_t + turn + 4 * w) = v;
+        asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(tile_s + (4 * i + (lane >> 3)) * kTurn + ((lane & 7) ^ i) * 4));
+        if (f0 + 4 * i + (lane >> 3) < F) *reinterpret_cast<unsigned*>(dst) = v;
+        dst += 4 * pitch_t;
       }
       __syncwarp();
     }
@@ -879,13 +911,11 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
     }                                                                                                     \
   } while (0)
   if constexpr (sizeof(T) == 4) {
-    if (bin_bytes == 1 && log2p == 8) {
+    // (words of four row-major ids: an array on an odd boundary is left to k_bin_smem)
+    if (bin_bytes == 1 && log2p == 8 && (reinterpret_cast<uintptr_t>(bins) & 3) == 0) {
       auto fn = bins_t != nullptr ? k_bin_lut<true> : k_bin_lut<false>;
-      LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLutSmem)));
-      constexpr int64_t kRows = kLutThreads / 32 * kBinTileRows;  // of a block's first turn
-      dim3 grid = make_grid(2);
-      grid.x    = static_cast<unsigned>(std::min<int64_t>(grid.x, (n_rows + kRows - 1) / kRows));
-      fn<<<grid, kLutThreads, kLutSmem, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, static_cast<uint8_t*>(bins),
+      LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLutEnd)));
+      fn<<<make_grid(1), kLutThreads, kLutEnd, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, static_cast<uint8_t*>(bins),
                                                   static_cast<uint8_t*>(bins_t), pitch_t);
       LBK_LAUNCH_CHECK();
       return;

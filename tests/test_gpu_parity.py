@@ -1019,6 +1019,29 @@ def test_one_byte_bin_ids_count_the_proposals_below(lb, kind, N, F, S):
         assert np.array_equal(got[:, f], want), f
 
 
+@pytest.mark.parametrize("offset", [0, 1, 2, 4])
+@pytest.mark.parametrize("N", [1, 31, 32, 33, 95, 4737])
+def test_one_byte_bin_ids_on_any_boundary(lb, N, offset):
+    """Whole and partial tiles of 32 rows; row-major ids that may leave as words of four, and ids that may not."""
+    from legateboost_b200 import library as L
+    from legateboost_b200 import stages
+    from legateboost_b200.tree import _stream_ptr
+
+    F, rs = 41, np.random.RandomState(N)
+    proposals, row_ptr = stages.split_proposals(dev(rs.random((2000, F)).astype(np.float32)), 256, 3)
+    p, rp = proposals.cpu().numpy(), row_ptr.cpu().numpy()
+    X, ctx = rs.random((N, F)).astype(np.float32), L.context(0)
+    dX = dev(X)
+    room = torch.full((offset + N * 64 + 64,), 255, dtype=torch.uint8, device="cuda")
+    ctx.check(ctx.lib.lbk_bin_matrix(ctx.handle, dX.data_ptr(), L.LBK_F32, F, N, F, proposals.data_ptr(), row_ptr.data_ptr(),
+                                     room.data_ptr() + offset, 1, _stream_ptr()))
+    got = room.cpu().numpy()
+    ids = got[offset:offset + N * 64].reshape(N, 64)
+    for f in range(F):
+        assert np.array_equal(ids[:, f], np.searchsorted(p[rp[f]:rp[f + 1]], X[:, f], side="left")), f
+    assert not ids[:, F:].any() and (got[:offset] == 255).all() and (got[offset + N * 64:] == 255).all()
+
+
 @pytest.mark.parametrize("N,K", [(1, 3), (255, 23), (257, 24), (1000, 186), (70, 187), (70, 300)])
 def test_softmax_gradients_of_whole_and_partial_tiles(lb, N, K):
     """The tiled kernel (256 rows down to 32 per block) and the one for more classes than it takes."""
