@@ -23,6 +23,7 @@ namespace {
 constexpr int kPartThreads   = 256;
 constexpr int kPartItems     = 8;
 constexpr int kPartTile      = kPartThreads * kPartItems;  // rows per chunk
+constexpr int kPartBlocks    = 4;    // per SM: as many as are resident
 constexpr int kPartPlanNodes = 1024;  // levels of up to this many nodes are planned inside the kernel
 
 __device__ inline int ChunksOf(const PartitionLevel& p, int j)
@@ -70,11 +71,15 @@ __global__ void __launch_bounds__(1024)
 }
 
 // Persistent blocks, a chunk at a time.  Bound by HBM: per row and level the row id, its pair and the
-// 32-byte sector of its bin in, row id and pair out.  kPlanInside: every block finds the chunks before
+// 32-byte sector of its bin in, row id and pair out.  Four blocks of 64 registers a thread are resident on an SM, and no
+// more are launched (six: the two that come later do their third of the chunks on a half-empty SM): 40M x 64, depth 8,
+// seven levels: 1.91 -> 1.60 ms, 10M: 454 -> 414 us; the second level 26 bytes per row at 5.0 TB/s.  512 threads with four rows
+// each: 1.70 ms; five blocks of 48 registers: 2.06 ms; the rows put in order in shared memory and written as
+// whole lines while the next chunk's are on their way: 1.77 ms.  kPlanInside: every block finds the chunks before
 // each node by itself (a scan of at most kPartPlanNodes counts once per block, about a microsecond,
 // instead of a launch of its own).
 template <typename BinT, bool kPlanInside>
-__global__ void __launch_bounds__(kPartThreads)
+__global__ void __launch_bounds__(kPartThreads, kPartBlocks)
   k_partition(const __grid_constant__ PartitionLevel p, const int32_t* __restrict__ chunk_off_global)
 {
   __shared__ int32_t s_off[kPlanInside ? kPartPlanNodes + 1 : 1];
@@ -221,7 +226,7 @@ void PartitionRows(lbk_context* ctx, Scratch& s, const PartitionLevel& pl, cudaS
   }
   // an upper bound of the number of chunks; no more blocks than are resident at once
   const int64_t max_chunks = pl.n_rows / kPartTile + std::min<int64_t>(pl.n_nodes, pl.n_rows) + 1;
-  const unsigned grid      = static_cast<unsigned>(std::min<int64_t>(max_chunks, static_cast<int64_t>(ctx->sm_count) * 6));
+  const unsigned grid      = static_cast<unsigned>(std::min<int64_t>(max_chunks, static_cast<int64_t>(ctx->sm_count) * kPartBlocks));
   const bool inside        = pl.n_nodes <= kPartPlanNodes;
   int32_t* chunk_off       = nullptr;
   if (!inside) {
