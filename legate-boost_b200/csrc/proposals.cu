@@ -480,10 +480,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
 // A block of 32 warps has one such table; the warps' tiles for the feature-major copy lie before and behind it.  The
 // row-major ids leave as words of four features, turned among four lanes.
 //
-// Bound by HBM and the load/store pipe (about 56 passes and 190 instructions per 256 ids).  With a table of bytes (lookups of
-// three passes), one store per row and eight values ahead: 10M x 64, with the copy, 840 us; now 690 (3.84 GB, for which
-// the copy rate of HBM gives 587); 1M x 100: 221 -> 158; 200k x 50: 42 -> 24, where the fill of the table counts: a thread
-// per feature read the proposals 1 KB apart.  Eight values ahead instead of sixteen, with this layout: 827.
+// The feature-major copy is 32 streams per block that lie n_rows bytes apart.  Four warps with neighbouring rows write
+// their tiles together, 128 bytes of a feature at a time: with 32 bytes per warp the 100M rows took 9430 us (and 5960
+// without the copy, of which that is 1 ms at the copy rate of HBM), with eight or sixteen warps 6940 and 8120 (they wait for each other;
+// 10M: 712 and 818).
+//
+// Bound by HBM and the load/store pipe (about 56 passes and 190 instructions per 256 ids).  Measured with the copy, before
+// (a table of bytes, whose lookups are three passes, a store per row, eight values ahead, a table filled by reads 1 KB apart)
+// and now: 100M x 64: 8430 -> 6960 us (the copy rate of HBM gives 5870), 10M x 64: 840 -> 696, 1M x 100: 221 -> 175,
+// 200k x 50: 42 -> 25.  Eight values ahead instead of sixteen, in this layout: 10M x 64 827 us.
 constexpr int kBuckets         = 512;
 constexpr int kLutThreads      = 1024;
 constexpr int kLutWarps        = kLutThreads / 32;
@@ -491,10 +496,11 @@ constexpr int kLutRows         = 256 + 16;  // of the table: the last steps may 
 constexpr unsigned kLutRow     = 2 * kGroup * sizeof(float);
 constexpr unsigned kLutAt      = 32768;     // an id is byte 1 of the address of its row, less 128
 constexpr int kLutTurn         = 32;        // rows of a warp's tile
-constexpr unsigned kLutTile    = kGroup * kLutTurn;
-constexpr int kLutTilesBefore  = 30;        // (1 KB is reserved, the kernel declares less than another)
+constexpr int kLutTeam         = 4;         // warps that write the feature-major copy of their rows together
+constexpr unsigned kLutTile    = kGroup * kLutTurn + 32;  // (the tiles of a team begin in different banks)
+constexpr int kLutTilesBefore  = 29;        // (1 KB is reserved, the kernel declares less than another)
 constexpr unsigned kLutTilesAt = kLutAt - kLutTilesBefore * kLutTile;
-constexpr unsigned kLutEnd     = kLutAt + kBuckets * kLutRow + (kLutWarps - kLutTilesBefore) * kLutTile;
+constexpr unsigned kLutEnd     = kLutAt + kBuckets * kLutRow + (kLutWarps - kLutTilesBefore / kLutTeam * kLutTeam) * kLutTile;
 constexpr unsigned kLutStageAt = kLutAt + kLutRows * kLutRow;  // (the proposals are turned there before the buckets are made)
 static_assert(kLutTilesAt >= 2048 && kLutStageAt + kLutRows * (kGroup + 1) * 4 <= kLutEnd, "room around the table");
 
@@ -571,7 +577,11 @@ __global__ void __launch_bounds__(kLutThreads, 1)
   // table is all +inf, so their ids are 0.
   const bool active     = f0 + lane < F;
   const unsigned lut_s  = col_s + kGroup * 4 - 0x4b000000u * kLutRow;  // (the bits of 2^23)
-  const unsigned tile_s = warp < kLutTilesBefore ? kLutTilesAt + warp * kLutTile : kLutAt + kBuckets * kLutRow + (warp - kLutTilesBefore) * kLutTile;
+  // (a team's tiles lie together: the teams that do not fit before the table come after it)
+  constexpr int kTeamsBefore = kLutTilesBefore / kLutTeam;
+  const unsigned tiles_s = warp / kLutTeam < kTeamsBefore ? kLutTilesAt + warp / kLutTeam * kLutTeam * kLutTile
+                                                         : kLutAt + kBuckets * kLutRow + (warp / kLutTeam - kTeamsBefore) * kLutTeam * kLutTile;
+  const unsigned tile_s = tiles_s + warp % kLutTeam * kLutTile, team_s = tiles_s + (lane >> 3) * kLutTile;
   const int pitch   = static_cast<int>(gridDim.y) * kGroup;
   constexpr int U   = 8;  // rows per warp in flight
   const int n       = static_cast<int>(n_rows);
@@ -579,7 +589,9 @@ __global__ void __launch_bounds__(kLutThreads, 1)
   constexpr int kTurn = kLutTurn;
   static_assert(kTurn == 4 * U, "four times eight rows");
   const int hop     = static_cast<int>(gridDim.x) * kLutWarps * kTurn;  // rows from one turn of a warp to the next
-  int turn          = (warp * gridDim.x + blockIdx.x) * kTurn;  // (a small matrix is spread over the blocks)
+  const int team    = warp / kLutTeam, mate = warp - team * kLutTeam;
+  // the rows of a team follow each other (and a small matrix is spread over the blocks)
+  int turn          = ((team * gridDim.x + blockIdx.x) * kLutTeam + mate) * kTurn;
   const float* xcol = X + (active ? f0 + lane : F - 1);
   // the lane's word of the row-major ids: row lane % 4 of four, features lane / 4 * 4 and the next three
   uint8_t* ocol     = bins + static_cast<int64_t>(lane & 3) * pitch + f0 + (lane & ~3);
@@ -602,10 +614,8 @@ __global__ void __launch_bounds__(kLutThreads, 1)
     for (int u = 0; u < U; ++u, src += ld) x[u] = first + u < n ? LdgStream(src) : -INFINITY;
   };
   float xa[U], xb[U];
-  if (turn < n) {
-    load_rows_checked(turn, xa);
-    load_rows_checked(turn + U, xb);
-  }
+  load_rows_checked(turn, xa);
+  load_rows_checked(turn + U, xb);
   const unsigned swap = lane >> 2;  // the words of a feature's 32 bytes are swapped so that the lanes' stores fall on distinct banks
   // one turn; checked: the turn may reach beyond the last row; levels: steps of the search, 8 = without the buckets
   auto do_turn = [&](auto checked, auto levels) {
@@ -643,23 +653,29 @@ __global__ void __launch_bounds__(kLutThreads, 1)
       eight_rows(sub + 1, xb);
     }
     if (kCopyT) {
-      // the tile leaves feature by feature, four of them and the 32 bytes of each per store (rows up to the padded end
-      // of a feature's row of the copy; the ids of rows beyond the last one are 0)
-      __syncwarp();
-      uint8_t* dst = bins_t + static_cast<int64_t>(f0 + (lane >> 3)) * pitch_t + turn + 4 * (lane & 7);
+      // The tiles of the team leave feature by feature, 128 bytes per store (the rows of a warp up to the padded end of a
+      // feature's row of the copy; the ids of rows beyond the last one are 0).
+      auto meet = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + team), "n"(kLutTeam * 32) : "memory"); };
+      meet();
+      const int row0 = turn - mate * kTurn + 4 * lane;
+      uint8_t* dst   = bins_t + static_cast<int64_t>(f0 + mate) * pitch_t + row0;
+#pragma unroll 4
+      for (int fl = mate; fl < kGroup; fl += kLutTeam) {
 #pragma unroll
-      for (int i = 0; i < kGroup / 4; ++i) {
-        unsigned v;
-        asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(tile_s + (4 * i + (lane >> 3)) * kTurn + ((lane & 7) ^ i) * 4));
-        if (f0 + 4 * i + (lane >> 3) < F) *reinterpret_cast<unsigned*>(dst) = v;
-        dst += 4 * pitch_t;
+        for (int piece = 0; piece < kLutTeam / 4; ++piece) {
+          unsigned v;
+          asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(team_s + piece * 4 * kLutTile + fl * kTurn + ((lane & 7) ^ (fl >> 2)) * 4));
+          if (f0 + fl < F && (!kChecked || row0 + piece * 128 < pitch_t)) *reinterpret_cast<unsigned*>(dst + piece * 128) = v;
+        }
+        dst += kLutTeam * pitch_t;
       }
-      __syncwarp();
+      meet();
     }
   };
+  // (every warp of a team takes the same turns; the last ones may have no rows for some of its warps)
   auto all_turns = [&](auto levels) {
-    for (; turn + kTurn <= n; turn += hop) do_turn(std::false_type(), levels);
-    if (turn < n) do_turn(std::true_type(), levels);
+    for (; turn + (kLutTeam - mate) * kTurn <= n; turn += hop) do_turn(std::false_type(), levels);
+    if (turn - mate * kTurn < n) do_turn(std::true_type(), levels);
   };
   if (most == 0) all_turns(std::integral_constant<int, 3>());
   else if (most == 1) all_turns(std::integral_constant<int, 4>());
