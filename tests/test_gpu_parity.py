@@ -75,6 +75,22 @@ def test_quantise(lb, oracle, N, K):
     assert np.array_equal(root.cpu().numpy(), want_q.sum(axis=0))
 
 
+@pytest.mark.parametrize("g,h", [
+    ([5.0], [0.25]), ([-5.0], [3.0]), ([0.0], [0.0]), ([-0.0, 0.0], [0.0, 1e-290]), ([1e-12, -1e12, 3.5], [1e-8, 1.0, 1e8]),
+    ([2.0 ** 30, -(2.0 ** 30)], [1.0, 1.0]), ([1.0, -1.0] * 700, [0.5] * 1400),
+])
+def test_quantise_whole_numbers_at_the_ends(lb, oracle, g, h):
+    """Values that are whole multiples of the scale, the largest magnitudes, zeros of both signs."""
+    from legateboost_b200 import stages
+
+    g, h = np.array(g)[:, None], np.array(h)[:, None]
+    for seed in (0, 7, 2 ** 31 - 1):
+        want_q, want_scale = oracle.quantise(g, h, seed=seed)
+        gp, _, scale = stages.quantise(dev(g), dev(h), seed=seed)
+        assert np.array_equal(gp.cpu().numpy().reshape(want_q.shape), want_q)
+        assert np.array_equal(scale.cpu().numpy(), want_scale)
+
+
 def test_quantise_row_offset(lb, oracle):
     # the quantised pair depends on the GLOBAL row id: a shard quantised on its own, with the
     # scale of its own |g| sum, must equal the oracle's shard
