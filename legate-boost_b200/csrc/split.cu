@@ -374,18 +374,16 @@ __global__ void __launch_bounds__(64)
   ApplyWinner<T>(best, node, K, row_ptr, cuts, cut_stride, tree, [&](int k) { return LoadPair(ls + k); }, threadIdx.x, blockDim.x);
 }
 
-// hessian and leaf value of every node from its quantised sums; a node whose parent did not split keeps 0
+// hessian and leaf value of every node from its quantised sums
 __global__ void __launch_bounds__(256)
   k_finish_tree(TreeArrays tree, const QuantParams* __restrict__ qp_ptr, int K, int64_t n, double l1, double l2,
                 double* __restrict__ hessian)
 {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
-  const int node   = static_cast<int>(i / K);
-  const GPairF64 s = Dequantise(tree.node_sums[i], *qp_ptr);
-  hessian[i]       = s.hess;
-  const bool here  = node == 0 || tree.feature[(node - 1) / 2] >= 0;
-  tree.leaf_value[i] = here ? CalculateLeafValue(s.grad, s.hess, l1, l2) : 0.0;
+  const double2 v    = FinishedNode(tree, *qp_ptr, K, i, l1, l2);
+  tree.leaf_value[i] = v.x;
+  hessian[i]         = v.y;
 }
 
 }  // namespace

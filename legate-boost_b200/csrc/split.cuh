@@ -91,4 +91,14 @@ __device__ inline unsigned AddGain(const GPairI64& left, unsigned ok, const Node
   return ok;
 }
 
+// Leaf value and hessian of entry i = node * K + output, from the node's quantised sums; the leaf value of a node whose
+// parent did not split is 0.
+__device__ inline double2 FinishedNode(const TreeArrays& tree, const QuantParams& qp, int K, int64_t i, double l1, double l2)
+{
+  const int node   = static_cast<int>(i / K);
+  const GPairF64 s = Dequantise(tree.node_sums[i], qp);
+  const bool here  = node == 0 || tree.feature[(node - 1) / 2] >= 0;
+  return make_double2(here ? CalculateLeafValue(s.grad, s.hess, l1, l2) : 0.0, s.hess);
+}
+
 }  // namespace lbk
