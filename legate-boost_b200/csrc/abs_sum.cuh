@@ -4,6 +4,7 @@
 // reduced the same way until one value is left.  The CPU oracle uses the same order.
 #pragma once
 #include "device_utils.cuh"
+#include "objective.cuh"
 
 namespace lbk {
 
@@ -40,8 +41,8 @@ __device__ inline void JoinAbsSums(const double* s_sum, double& tg, double& th)
 // CTA call it, several groups may do so at once).  kFirst: |g|, |h| of the strided [n / K, K] inputs, else the
 // partial sums themselves.  s_sum: shared, 16 values per group.
 template <bool kFirst>
-__device__ inline void AbsSumPartial(const double* g, const double* h, int64_t ldg, int K, int64_t n, int64_t block, int tid,
-                                     double* s_sum, double& tg, double& th)
+__device__ inline void AbsSumPartial(const double* g, const double* h, int64_t ldg, const GradientForm& form, int K, int64_t n,
+                                     int64_t block, int tid, double* s_sum, double& tg, double& th)
 {
   const int64_t base = block * kSumBlock;
   double sg = 0.0, sh = 0.0;
@@ -53,8 +54,9 @@ __device__ inline void AbsSumPartial(const double* g, const double* h, int64_t l
       if (kFirst) {
         const int64_t row = K == 1 ? idx : idx / K;
         const int k       = static_cast<int>(idx - row * K);
-        vg                = fabs(g[row * ldg + k]);
-        vh                = fabs(h[row * ldg + k]);
+        const double2 v   = GradientAt(g, h, row * ldg + k, form);
+        vg                = fabs(v.x);
+        vh                = fabs(v.y);
       } else {
         vg = g[idx];
         vh = h[idx];
@@ -70,11 +72,11 @@ __device__ inline void AbsSumPartial(const double* g, const double* h, int64_t l
 }
 
 template <bool kFirst>
-__device__ inline void AbsSumBlock(const double* g, const double* h, int64_t ldg, int K, int64_t n, int64_t block, int tid,
-                                   double* s_sum, double* out_g, double* out_h)
+__device__ inline void AbsSumBlock(const double* g, const double* h, int64_t ldg, const GradientForm& form, int K, int64_t n,
+                                   int64_t block, int tid, double* s_sum, double* out_g, double* out_h)
 {
   double tg, th;
-  AbsSumPartial<kFirst>(g, h, ldg, K, n, block, tid, s_sum, tg, th);
+  AbsSumPartial<kFirst>(g, h, ldg, form, K, n, block, tid, s_sum, tg, th);
   if (tid == 0) {
     *out_g = tg;
     *out_h = th;

@@ -334,7 +334,13 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     if (a.out_total_bins) *a.out_total_bins = words.get()[0];
     return;
   }
-  if (round != nullptr) {
+  GradientForm form;
+  if (round != nullptr && round->objective == LBK_SQUARED_ERROR) {
+    form = GradientForm{true, round->learning_rate};
+    g    = round->pred;
+    h    = round->y;
+    ldg  = K;
+  } else if (round != nullptr) {
     double* rg = s.alloc<double>(static_cast<size_t>(N) * K);
     double* rh = s.alloc<double>(static_cast<size_t>(N) * K);
     Gradient(round->objective, round->pred, round->y, N, K, round->learning_rate, rg, rh, stream);
@@ -437,6 +443,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     pa.g            = g;
     pa.h            = h;
     pa.ldg          = ldg;
+    pa.form         = form;
     pa.K            = K;
     pa.n_elements   = N * K;
     pa.tree         = tree;
@@ -492,7 +499,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
 
   // quantised pairs and root sums
   int2* gpair = s.alloc<int2>(static_cast<size_t>(N) * K);
-  Quantise(ctx, g, h, ldg, a.row_offset, N, K, a.seed, gpair, tree.node_sums, qp, max_abs, stream);
+  Quantise(ctx, g, h, ldg, form, a.row_offset, N, K, a.seed, gpair, tree.node_sums, qp, max_abs, stream);
 
   const int cdepth = cache_depth(B, max_histogram_nodes);
   // levels >= D are never evaluated; no need to hold them.  The last level's histograms are evaluated as
@@ -938,7 +945,7 @@ int lbk_quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg
     pa.S          = 1;
     lbk::QuantParams* qp = reinterpret_cast<lbk::QuantParams*>(scale);
     lbk::Prologue<float>(ctx, s, pa, nullptr, nullptr, nullptr, s.alloc<double>(2), qp, stream);
-    lbk::Quantise(ctx, g, h, ldg, row_offset, n_local_rows, n_outputs, seed, reinterpret_cast<int2*>(gpair),
+    lbk::Quantise(ctx, g, h, ldg, lbk::GradientForm{}, row_offset, n_local_rows, n_outputs, seed, reinterpret_cast<int2*>(gpair),
                   reinterpret_cast<lbk::GPairI64*>(root_sums), qp, abs, stream);
   });
 }

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kSortThreads)
   }
   b -= p.sort_blocks;
   if (b < p.sum_blocks) {
-    AbsSumBlock<true>(p.g, p.h, p.ldg, p.K, p.n_elements, b, threadIdx.x, s_sum, p.part_g + b, p.part_h + b);
+    AbsSumBlock<true>(p.g, p.h, p.ldg, p.form, p.K, p.n_elements, b, threadIdx.x, s_sum, p.part_g + b, p.part_h + b);
     return;
   }
   b -= p.sum_blocks;
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(1024)
       const int q     = tid / kSumThreads;
       const int64_t b = b0 + q;
       double tg, th;
-      AbsSumPartial<false>(part_g, part_h, 0, 1, n, b, tid % kSumThreads, s_sum + q * 2 * kSumThreads / 32, tg, th);
+      AbsSumPartial<false>(part_g, part_h, 0, GradientForm{}, 1, n, b, tid % kSumThreads, s_sum + q * 2 * kSumThreads / 32, tg, th);
       __syncthreads();
       if (tid % kSumThreads == 0 && b < blocks) {
         part_g[b] = tg;

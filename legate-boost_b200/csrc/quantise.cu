@@ -12,6 +12,7 @@
 // (The sums of |g| and |h|: abs_sum.cuh, made in the prologue of the tree.)
 #include "device_utils.cuh"
 #include "internal.h"
+#include "objective.cuh"
 
 namespace lbk {
 namespace {
@@ -23,8 +24,8 @@ namespace {
 // Bound by its instructions (the hash's multiplications, twelve float64 operations of half rate): 100M rows 615 us, of which
 // HBM asks for 370; with conversions between float64 and integers 804.
 __global__ void __launch_bounds__(256)
-  k_quantise(const double* __restrict__ g, const double* __restrict__ h, int64_t ldg, int64_t row_offset,
-             int64_t n_local, int K, long long seed, const QuantParams* __restrict__ qp_ptr,
+  k_quantise(const double* __restrict__ g, const double* __restrict__ h, int64_t ldg, const GradientForm form,
+             int64_t row_offset, int64_t n_local, int K, long long seed, const QuantParams* __restrict__ qp_ptr,
              int2* __restrict__ gpair, GPairI64* __restrict__ root_sums, int* __restrict__ max_abs)
 {
   extern __shared__ unsigned long long s_sum[];  // [K][2]
@@ -43,9 +44,8 @@ __global__ void __launch_bounds__(256)
     long long sg = 0, sh = 0;
 #pragma unroll 4
     for (int64_t row = t / K; row < n_local; row += rows_per_turn) {
-      const double gv = g[row * ldg + k];
-      const double hv = h[row * ldg + k];
-      const int2 q    = QuantisePair(gv, hv, qp, HashCombine(seed, row_offset + row, k));
+      const double2 v = GradientAt(g, h, row * ldg + k, form);
+      const int2 q    = QuantisePair(v.x, v.y, qp, HashCombine(seed, row_offset + row, k));
       gpair[row * K + k] = q;
       sg += q.x;
       sh += q.y;
@@ -88,8 +88,8 @@ __global__ void __launch_bounds__(256)
 
 }  // namespace
 
-void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, int64_t row_offset, int64_t n_local, int K,
-              int seed, int2* gpair, GPairI64* root_sums, const QuantParams* params, int* max_abs, cudaStream_t stream)
+void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, const GradientForm& form, int64_t row_offset,
+              int64_t n_local, int K, int seed, int2* gpair, GPairI64* root_sums, const QuantParams* params, int* max_abs, cudaStream_t stream)
 {
   if (n_local > 0) {
     int64_t blocks = (n_local * K + 511) / 512;  // (two elements per thread: fewer blocks at the common words)
@@ -99,7 +99,7 @@ void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, i
     const size_t smem = sizeof(unsigned long long) * 2 * K;
     LBK_EXPECT(smem <= 48 * 1024, "too many outputs for the quantiser's block sums");
     if (smem > 40 * 1024) AllowSharedMemory(ctx, k_quantise, 1024);  // (the limit without it counts the static part too)
-    k_quantise<<<static_cast<unsigned>(blocks), 256, smem, stream>>>(g, h, ldg, row_offset, n_local, K,
+    k_quantise<<<static_cast<unsigned>(blocks), 256, smem, stream>>>(g, h, ldg, form, row_offset, n_local, K,
                                                                   static_cast<long long>(seed), params, gpair, root_sums, max_abs);
     LBK_LAUNCH_CHECK();
   }
