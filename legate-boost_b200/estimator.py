@@ -39,13 +39,39 @@ def _is_own(model, name: str) -> bool:
     return getattr(getattr(model, name), "__func__", None) is _LBBase.__dict__[name]
 
 
-def _copy_of(base: Tree) -> Tree:
-    """deepcopy of a base model, whose attributes are plain values as a rule."""
-    if all(type(v) in (int, float, str, bool, type(None)) for v in base.__dict__.values()):
+def _is_own_sampling(base: Tree) -> bool:
+    """Whether a base model samples features as Tree does."""
+    return getattr(base._sample_features, "__func__", None) is Tree._sample_features
+
+
+def _is_plain(base: Tree) -> bool:
+    """Whether a base model's attributes are plain values, as they are as a rule."""
+    return all(type(v) in (int, float, str, bool, type(None)) for v in base.__dict__.values())
+
+
+def _copy_of(base: Tree, plain: bool) -> Tree:
+    """deepcopy of a base model."""
+    if plain:
         tree = Tree.__new__(Tree)
         tree.__dict__.update(base.__dict__)
         return tree
     return deepcopy(base)
+
+
+class _NoSeed(np.random.bit_generator.ISeedSequence):
+    """For a generator that is seeded right after it is made."""
+
+    def generate_state(self, n_words, dtype=np.uint32):
+        return np.zeros(n_words, dtype=dtype)
+
+
+def _random_state(seed) -> np.random.RandomState:
+    """RandomState(seed).  That one first seeds its generator from the system's entropy, which takes 100 of its 140 us."""
+    if type(seed) is not int:
+        return np.random.RandomState(seed)
+    state = np.random.RandomState(np.random.MT19937(_NoSeed()))
+    state.seed(seed)
+    return state
 
 
 class _SquaredError:
@@ -91,16 +117,24 @@ class _LogLoss:
         return e / e.sum(dim=1, keepdim=True)
 
     def init(self, y, average):
-        mx = torch.tensor([float(y.max()) if y.numel() else 0.0], dtype=torch.float64, device=y.device)
-        import torch.distributed as dist
+        lo = 0.0
+        if _several_ranks():
+            import torch.distributed as dist
 
-        if dist.is_available() and dist.is_initialized() and dist.get_world_size() > 1:
+            mx = torch.tensor([float(y.max()) if y.numel() else 0.0], dtype=torch.float64, device=y.device)
             dist.all_reduce(mx, op=dist.ReduceOp.MAX)
-        num_class = int(mx.item()) + 1
+            hi = mx.item()
+        else:
+            lo, hi = torch.stack(torch.aminmax(y)).tolist() if y.numel() else (0.0, 0.0)
+        num_class = int(hi) + 1
         n_targets = num_class if num_class > 2 else 1
         if not average:
             return torch.zeros(n_targets, dtype=torch.float64, device=y.device)
-        counts = _all_sum(torch.bincount(y.reshape(-1).to(torch.int64), minlength=num_class).to(torch.float64))
+        labels = y.reshape(-1).to(torch.int64)
+        if _several_ranks() or num_class > 16 or num_class * y.numel() > 1 << 26 or lo <= -1.0:
+            counts = _all_sum(torch.bincount(labels, minlength=num_class).to(torch.float64))
+        else:  # (bincount waits for the device twice more; it refuses negative labels)
+            counts = (labels[:, None] == torch.arange(num_class, device=y.device)).sum(dim=0, dtype=torch.float64)
         prob = counts / counts.sum()
         if n_targets == 1:
             return -torch.log(1.0 / prob[1:2] - 1.0)
@@ -173,11 +207,11 @@ class _LBBase:
         self.n_features_in_ = X.shape[1]
         self.models_: List[Tree] = []
         rs = self.random_state
-        self.random_state_ = rs if isinstance(rs, np.random.RandomState) else np.random.RandomState(rs)
+        self.random_state_ = rs if isinstance(rs, np.random.RandomState) else _random_state(rs)
         self._obj = self._objective()
         self.model_init_ = self._obj.init(y, self.init == "average")
         self.train_metric_: List[float] = []
-        train_pred = self.model_init_.repeat(X.shape[0], 1)
+        train_pred = self.model_init_.expand(X.shape[0], -1).clone(memory_format=torch.contiguous_format)
         layout = _row_layout(X.shape[0])  # this rank's block of rows: the same for every tree
         if self._rounds_in_library():
             try:
@@ -221,13 +255,17 @@ class _LBBase:
         K = train_pred.shape[1]
         dev, rs = X.device, self.random_state_
         bases = [self.base_models[i % len(self.base_models)] for i in range(self.n_estimators)]
-        seeds, masks = [], np.ones((self.n_estimators, F), dtype=np.uint8)
-        for i, b in enumerate(bases):
-            seeds.append(int(rs.randint(0, 2**31)))
-            mask = b._sample_features(rs, F)
-            if mask is not None:
-                masks[i] = mask
-        masks = None if masks.all() else torch.from_numpy(masks).to(dev)
+        masks = None
+        if type(rs) is np.random.RandomState and all(b.feature_fraction >= 1.0 and _is_own_sampling(b) for b in self.base_models):
+            seeds = rs.randint(0, 2**31, size=self.n_estimators).tolist()  # (the same draws as one by one)
+        else:
+            seeds, masks = [], np.ones((self.n_estimators, F), dtype=np.uint8)
+            for i, b in enumerate(bases):
+                seeds.append(int(rs.randint(0, 2**31)))
+                mask = b._sample_features(rs, F)
+                if mask is not None:
+                    masks[i] = mask
+            masks = None if masks.all() else torch.from_numpy(masks).to(dev)
         if X.stride(1) != 1 and N > 0:
             X = X.contiguous()
         y = y.contiguous()
@@ -240,34 +278,32 @@ class _LBBase:
         a.n_local_rows, a.n_features, a.n_outputs = N, F, K
         a.stream = stream
         r.objective, r.y, r.pred, r.learning_rate = self._obj.code, y.data_ptr(), train_pred.data_ptr(), float(self.learning_rate)
-        ref, sketches, models = C.byref(r), {}, []
+        ref, sketches, made = C.byref(r), {}, []
         n_bases = len(self.base_models)
         at = 0
         while at < self.n_estimators:
             run = list(range(at, min(at + 64, self.n_estimators)))
             at += len(run)
             zeroed = torch.zeros((len(run),), dtype=torch.int32, device=dev)
-            trees = {}
+            of_base = {}
             for b in range(min(n_bases, len(run))):
-                mine = [i for i in run if i % n_bases == (run[0] + b) % n_bases]
-                M, n = 2 ** (bases[mine[0]].max_depth + 1) - 1, len(mine)
+                first = run[b]
+                M, n = 2 ** (bases[first].max_depth + 1) - 1, (len(run) - b + n_bases - 1) // n_bases
                 f64 = dict(dtype=torch.float64, device=dev)
                 arrays = {
                     "leaf_value": torch.empty((n, M, K), **f64), "feature": torch.empty((n, M), dtype=torch.int32, device=dev),
                     "split_value": torch.empty((n, M), **f64), "gain": torch.empty((n, M), **f64),
                     "hessian": torch.empty((n, M, K), **f64),
                 }
-                parts = {name: t.unbind(0) for name, t in arrays.items()}
-                for q, i in enumerate(mine):
-                    trees[i] = {name: p[q] for name, p in parts.items()}
-                    trees[i]["at"] = [t.data_ptr() + q * t.stride(0) * t.element_size() for t in arrays.values()]
+                of_base[first % n_bases] = (arrays, [(t.data_ptr(), t.stride(0) * t.element_size()) for t in arrays.values()], M)
             for j, i in enumerate(run):
-                base, mine = bases[i], trees[i]
-                where = mine.pop("at")
-                a.leaf_value, a.feature, a.split_value, a.gain, a.hessian = where
+                base = bases[i]
+                _, where, M = of_base[i % n_bases]
+                q = j // n_bases  # which tree of its base model's this is
+                a.leaf_value, a.feature, a.split_value, a.gain, a.hessian = [p + q * step for p, step in where]
                 a.feature_set = None if masks is None else masks.data_ptr() + i * F
                 r.zeroed = zeroed.data_ptr() + 4 * j
-                a.max_depth, a.max_nodes = base.max_depth, mine["feature"].shape[0]
+                a.max_depth, a.max_nodes = base.max_depth, M
                 a.split_samples, a.seed = base.split_samples, seeds[i]
                 a.l1_regularization, a.l2_regularization = base.l1_regularization, base.l2_regularization
                 a.min_split_gain = base.min_split_gain
@@ -279,8 +315,15 @@ class _LBBase:
                 ctx.check(lib.lbk_boost_round(handle, ref))
                 if sketch is not None:
                     sketch.key = (_tensor_key(X), base.split_samples)
-                tree = _copy_of(base)
-                tree.__dict__.update(mine, random_state=rs, row_layout=layout, sketch=None, _fit_rows=None)
+            made.append((run, of_base, zeroed))
+        # (the trees' objects are made while the rounds run)
+        models, plain = [], [_is_plain(b) for b in self.base_models]
+        for run, of_base, _ in made:
+            parts = {b: {name: t.unbind(0) for name, t in arrays.items()} for b, (arrays, _, _) in of_base.items()}
+            for j, i in enumerate(run):
+                tree = _copy_of(bases[i], plain[i % n_bases])
+                tree.__dict__.update({name: p[j // n_bases] for name, p in parts[i % n_bases].items()},
+                                     random_state=rs, row_layout=layout, sketch=None, _fit_rows=None)
                 models.append(tree)
         ctx.check(lib.lbk_synchronize(handle, stream))
         self.models_ = models

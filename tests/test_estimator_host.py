@@ -1,0 +1,52 @@
+"""What an estimator draws and counts on the host is what the plain calls give, on the CPU."""
+import pickle
+
+import numpy as np
+import pytest
+import torch
+
+import legateboost_b200 as lb
+from legateboost_b200 import estimator as E
+
+
+@pytest.mark.parametrize("seed", [0, 1, 12345, 2 ** 31 - 1, 2 ** 32 - 1])
+def test_random_state_is_numpys(seed):
+    mine, want = E._random_state(seed), np.random.RandomState(seed)
+    for a, b in zip(mine.get_state(), want.get_state()):
+        assert np.array_equal(a, b)
+    # seeds of a whole fit at once are those drawn one by one, and leave the generator where those do
+    assert mine.randint(0, 2 ** 31, size=1000).tolist() == [int(want.randint(0, 2 ** 31)) for _ in range(1000)]
+    assert mine.randint(0, 1000) == want.randint(0, 1000)
+    assert pickle.loads(pickle.dumps(mine)).randint(0, 2 ** 31) == want.randint(0, 2 ** 31)
+
+
+def test_random_state_refuses_what_numpy_refuses():
+    for bad in (-1, 2 ** 32, 1.5, "1"):
+        with pytest.raises((ValueError, TypeError)) as want:
+            np.random.RandomState(bad)
+        with pytest.raises(want.type):
+            E._random_state(bad)
+    assert isinstance(E._random_state(None), np.random.RandomState)
+    assert E._random_state(np.int64(3)).randint(0, 100) == np.random.RandomState(3).randint(0, 100)
+
+
+@pytest.mark.parametrize("labels", [[0, 1], [1, 1], [0, 0], [0, 2, 1, 1], list(range(16)), list(range(40)), [3], [0.9, 1.2, 2.0], [-0.5, 1]])
+def test_initial_log_odds_are_those_of_the_counts(labels):
+    y = torch.tensor(labels, dtype=torch.float64)[:, None].repeat(3, 1)
+    n = int(y.max()) + 1
+    counts = torch.bincount(y.reshape(-1).to(torch.int64), minlength=n).to(torch.float64)
+    prob = counts / counts.sum()
+    want = torch.log(prob) if n > 2 else -torch.log(1.0 / prob[1:2] - 1.0)
+    assert torch.equal(E._LogLoss().init(y, True), want)
+
+
+def test_negative_labels_are_refused():
+    with pytest.raises(RuntimeError):
+        E._LogLoss().init(torch.tensor([[0.0], [-1.0], [1.0]], dtype=torch.float64), True)
+
+
+def test_feature_samples_of_ones_own_are_drawn_tree_by_tree():
+    base = lb.Tree(max_depth=3)
+    assert E._is_own_sampling(base)
+    base._sample_features = lambda rs, n: None
+    assert not E._is_own_sampling(base)
