@@ -217,6 +217,9 @@ __global__ void __launch_bounds__(256)
   pred[e] += __ldg(table + static_cast<int64_t>(__ldg(leaf + i)) * K + k);
 }
 
+// Rows x features x outputs above which a tree of more than 256 samples waits for the number of bins (BuildTreeImpl).
+constexpr int64_t kWidthMattersCells = int64_t{1} << 24;
+
 // `round`: a boosting round instead of a tree on given gradients (they are those of round->pred, which gets
 // the leaf values added); the call is then asynchronous.
 template <typename T>
@@ -365,7 +368,8 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   int32_t* row_ptr = in_sketch ? reinterpret_cast<int32_t*>(skb + sk.row_ptr) : s.alloc<int32_t>(F + 1);
 
   // Does the host have to know how many bins there are?  They decide the width of the bin ids (above 256
-  // samples), the batches of a level whose histograms are larger than the cache (the reference's rule,
+  // samples, where the matrix is large enough for that to matter: up to 2^24 cells both widths are built by the same
+  // kernels, and waiting cost 300k x 37 float64, 512 samples, 15 us per tree), the batches of a level whose histograms are larger than the cache (the reference's rule,
   // below), and the layout that a trace, a sketch or other ranks see.  Otherwise everything is laid out for
   // the upper bound F x S, and nothing waits for the device before the end of the tree.
   auto cache_depth = [&](int64_t bins, size_t& max_histogram_nodes) {
@@ -377,7 +381,8 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   };
   const int64_t bins_bound   = static_cast<int64_t>(F) * S;
   size_t max_histogram_nodes = 0;
-  const bool wait_for_bins   = in_sketch || a.trace_hist != nullptr || ctx->n_ranks > 1 || S > 256 ||
+  const bool wait_for_bins   = in_sketch || a.trace_hist != nullptr || ctx->n_ranks > 1 ||
+                             (S > 256 && N * F * K > kWidthMattersCells) ||
                              cache_depth(bins_bound, max_histogram_nodes) < D - 1;
 
   // words that have to be zero before the first level: node sums, arrival counters and partition cursors of

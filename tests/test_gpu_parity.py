@@ -1398,3 +1398,35 @@ def test_a_round_that_fails_waits_for_the_rounds_before_it(lb):
         assert stream.query()
     assert m.models_ == []
     lb.LBRegressor(n_estimators=1, base_models=(lb.Tree(max_depth=3),), random_state=0).fit(X, y)
+
+
+@pytest.mark.parametrize("distinct", [3, 200, 10 ** 6])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_fine_bins_without_waiting_for_their_number(lb, oracle, dtype, distinct):
+    """More than 256 samples on a matrix so small that the width of the bin ids does not wait for the number of bins, whether
+    one byte would have done or not; rounds and trees grow what the oracle grows."""
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.RandomState(distinct % 97)
+    N, F, D = 21001, 7, 5
+    X = np.round(rs.random((N, F)) * distinct).astype(dtype)
+    g, h = rs.normal(size=(N, 1)), rs.random((N, 1)) + 0.1
+    want = oracle.build_tree(X, g, h, max_depth=D, split_samples=700, seed=11, mode="Q")
+    got = build_tree_arrays(dev(X), dev(g), dev(h), max_depth=D, split_samples=700, seed=11, row_offset=0, dataset_rows=N)
+    for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
+        assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
+
+
+@pytest.mark.parametrize("N,F,K,depth", [(17001, 5, 1, 3), (20011, 9, 1, 9), (17003, 6, 1, 10), (6007, 40, 3, 7), (5801, 300, 3, 4), (5801, 33, 10, 7)])
+def test_rounds_add_the_leaf_values_where_the_leaves_are_found(lb, N, F, K, depth):
+    """Leaf tables made by every block and read from memory (more than 1024 values), rows too wide for the tiled walk: the
+    kept predictions are those of the trees."""
+    rs = np.random.RandomState(depth)
+    X = dev(rs.normal(size=(N, F)).astype(np.float32))
+    y = dev(rs.normal(size=N)) if K == 1 else dev(rs.randint(0, K, size=N).astype(np.float64))
+    make = lb.LBRegressor if K == 1 else lb.LBClassifier
+    m = make(n_estimators=3, base_models=(lb.Tree(max_depth=depth),), random_state=5).fit(X, y)
+    want = m.model_init_.repeat(N, 1)
+    for t in m:
+        want += lb.Tree.batch_predict([t], X)
+    assert torch.equal(m._train_pred, want)
