@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
 // without the copy, of which that is 1 ms at the copy rate of HBM), with eight or sixteen warps 6940 and 8120 (they wait for each other;
 // 10M: 712 and 818).
 //
-// Bound by HBM and the load/store pipe (about 56 passes and 190 instructions per 256 ids).  Measured with the copy, before
+// Bound by the issue slots and the load/store pipe (262 instructions and about 62 passes per 256 ids), close to HBM.  Measured with the copy, before
 // (a table of bytes, whose lookups are three passes, a store per row, eight values ahead, a table filled by reads 1 KB apart)
 // and now: 100M x 64: 8430 -> 6960 us (the copy rate of HBM gives 5870), 10M x 64: 840 -> 696, 1M x 100: 221 -> 175,
 // 200k x 50: 42 -> 25.  Eight values ahead instead of sixteen, in this layout: 10M x 64 827 us.
