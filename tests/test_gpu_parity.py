@@ -1430,3 +1430,20 @@ def test_rounds_add_the_leaf_values_where_the_leaves_are_found(lb, N, F, K, dept
     for t in m:
         want += lb.Tree.batch_predict([t], X)
     assert torch.equal(m._train_pred, want)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("F,width,offset", [(1, 1, 0), (2, 3, 1), (3, 7, 2), (4, 4, 0), (5, 9, 3), (7, 7, 0), (8, 13, 1), (33, 40, 3), (75, 75, 0)])
+def test_predict_rows_on_any_boundary(lb, oracle, dtype, F, width, offset):
+    """Rows that begin and end on any value of a 16-byte vector: columns of a wider matrix, odd numbers of columns."""
+    rs = np.random.RandomState(F * 7 + offset)
+    N, D = 8193 + 37, 5
+    M = 2 ** (D + 1) - 1
+    wide = rs.normal(size=(N, width)).astype(dtype)
+    X = wide[:, offset:offset + F]
+    trees = []
+    for _ in range(9):
+        feature = np.where(np.arange(M) < 2 ** D - 1, rs.randint(0, F, size=M), -1).astype(np.int32)
+        trees.append((rs.normal(size=(M, 1)), feature, rs.normal(size=M) * 0.5))
+    got = lb.tree.predict_arrays(dev(wide)[:, offset:offset + F], [tuple(dev(a) for a in t) for t in trees])
+    assert np.array_equal(got.cpu().numpy(), oracle.predict(np.ascontiguousarray(X), trees))
