@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "abs_sum.cuh"
+#include "bin_grid.h"
 #include "internal.h"
 
 namespace lbk {
@@ -873,6 +874,9 @@ ProposalInfo SplitProposals(lbk_context* ctx, Scratch& s, const T* X, int64_t ld
   return ProposalInfo{h[0], h[1]};
 }
 
+// Rows that take a block as long as filling its table: about 10 us.
+constexpr int64_t kLutFillRows = 2048, kSmemFillRows = 512;
+
 template <typename T>
 void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposals, int64_t cut_stride, const int32_t* row_ptr,
                void* bins, void* bins_t, int64_t pitch_t, int bin_bytes, int max_bins_per_feature, cudaStream_t stream)
@@ -887,18 +891,15 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
   const size_t table    = sizeof(T) * static_cast<size_t>(kGroup) * (size_t{1} << log2p);
   const size_t smem     = table + (bins_t != nullptr && bin_bytes == 1 ? size_t{8} * kGroup * kBinTilePitch : 0);
   const bool use_smem   = need <= 512 && table <= 96 * 1024;
-  // a block fills its table once and then walks the rows with a grid stride: the grid is what is
-  // resident at once (from the occupancy calculator), spread over the feature groups
-  auto make_grid = [&](int blocks_per_sm) {
+  // a block fills its table once and then walks the rows with a grid stride: whole waves of what is resident at once
+  // (from the occupancy calculator), spread over the tables (bin_grid.h)
+  auto blocks_of = [&](int64_t tables, int blocks_per_sm, int64_t fill_rows) {
     int sms = 148;
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int64_t blocks_x = (static_cast<int64_t>(sms) * (blocks_per_sm > 0 ? blocks_per_sm : 1) + G - 1) / G;
-    const int64_t most = (n_rows + 63) / 64;
-    if (blocks_x > most) blocks_x = most;
-    if (blocks_x < 1) blocks_x = 1;
-    return dim3(static_cast<unsigned>(blocks_x), G);
+    return static_cast<unsigned>(BinGridBlocks(n_rows, tables, static_cast<int64_t>(sms) * (blocks_per_sm > 0 ? blocks_per_sm : 1), fill_rows));
   };
+  auto make_grid = [&](int blocks_per_sm, int64_t fill_rows) { return dim3(blocks_of(G, blocks_per_sm, fill_rows), G); };
 #define LBK_BIN_SMEM2(BinT, L, CT)                                                                        \
   do {                                                                                                    \
     auto fn_ = k_bin_smem<T, BinT, L, CT>;                                                                \
@@ -906,7 +907,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       LBK_CUDA(cudaFuncSetAttribute(fn_, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))); \
     int per_sm_ = 0;                                                                                      \
     LBK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_, fn_, 256, smem));                    \
-    fn_<<<make_grid(per_sm_), 256, smem, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr,                 \
+    fn_<<<make_grid(per_sm_, kSmemFillRows), 256, smem, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr,                 \
                                                    static_cast<BinT*>(bins), static_cast<BinT*>(bins_t), pitch_t); \
   } while (0)
 #define LBK_BIN_SMEM(BinT, L)                                                                             \
@@ -921,7 +922,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       else if (log2p == 8) LBK_BIN_SMEM(BinT, 8);                                                         \
       else LBK_BIN_SMEM(BinT, 9);                                                                         \
     } else {                                                                                              \
-      k_bin_global<T, BinT><<<make_grid(8), 256, 0, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr,     \
+      k_bin_global<T, BinT><<<make_grid(8, 0), 256, 0, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr,     \
                                                        static_cast<BinT*>(bins), static_cast<BinT*>(bins_t), \
                                                        pitch_t);                                          \
     }                                                                                                     \
@@ -931,7 +932,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
     if (bin_bytes == 1 && log2p == 8 && (reinterpret_cast<uintptr_t>(bins) & 3) == 0) {
       auto fn = bins_t != nullptr ? k_bin_lut<true> : k_bin_lut<false>;
       LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLutEnd)));
-      fn<<<make_grid(1), kLutThreads, kLutEnd, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, static_cast<uint8_t*>(bins),
+      fn<<<make_grid(1, kLutFillRows), kLutThreads, kLutEnd, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, static_cast<uint8_t*>(bins),
                                                   static_cast<uint8_t*>(bins_t), pitch_t);
       LBK_LAUNCH_CHECK();
       return;
@@ -944,9 +945,8 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       constexpr int kFeatures = kWideTableBytes / ((1 << L) * static_cast<int>(sizeof(T)));
       auto fn = k_bin_wide<T, L, CT>;
       LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideTableBytes));
-      dim3 grid = make_grid(3);  // (resident blocks, spread over the tables that hold features)
-      grid.x    = std::max<unsigned>(1u, grid.x * G / ((F + kFeatures - 1) / kFeatures));
-      grid.y    = G * kGroup / kFeatures;
+      // (three blocks per SM, spread over the tables that hold features)
+      const dim3 grid(blocks_of((F + kFeatures - 1) / kFeatures, 3, kSmemFillRows), G * kGroup / kFeatures);
       fn<<<grid, 256, kWideTableBytes, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, G * kGroup,
                                                  static_cast<uint16_t*>(bins), static_cast<uint16_t*>(bins_t), pitch_t);
     };

@@ -1058,6 +1058,32 @@ def test_one_byte_bin_ids_on_any_boundary(lb, N, offset):
     assert not ids[:, F:].any() and (got[:offset] == 255).all() and (got[offset + N * 64:] == 255).all()
 
 
+@pytest.mark.parametrize("N,F", [
+    (2 * 75776 + 1, 64), (3 * 75776, 33),                       # two tables: 75776 rows a turn of all blocks; a last team of one row
+    (2 * 50176 + 97, 75), (5 * 29696 + 31, 160), (40007, 250),  # three, five and eight tables, which do not divide the SMs
+])
+def test_one_byte_bin_ids_of_several_turns(lb, oracle, N, F):
+    """Rows that take every warp through its turns twice and more, row-major and in the feature-major copy that the rows
+    are repartitioned by (a wrong id there is a row in a wrong node)."""
+    from legateboost_b200 import stages
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.RandomState(F)
+    X = rs.random((N, F)).astype(np.float32)
+    dX = dev(X)
+    proposals, row_ptr = stages.split_proposals(dX, 256, 3)
+    p, rp = proposals.cpu().numpy(), row_ptr.cpu().numpy()
+    got = stages.bin_matrix(dX, proposals, row_ptr, 1).cpu().numpy()
+    assert not got[:, F:].any()
+    for f in range(F):
+        assert np.array_equal(got[:, f], np.searchsorted(p[rp[f]:rp[f + 1]], X[:, f], side="left")), f
+    g, h = rs.normal(size=(N, 1)) + np.sin(6 * X[:, :1]), np.ones((N, 1))
+    want = oracle.build_tree(X, g, h, max_depth=3, split_samples=256, seed=5, mode="Q")
+    tree = build_tree_arrays(dX, dev(g), dev(h), max_depth=3, split_samples=256, seed=5, row_offset=0, dataset_rows=N)
+    for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
+        assert np.array_equal(tree[name].cpu().numpy(), getattr(want, name)), name
+
+
 @pytest.mark.parametrize("N,K", [(1, 3), (255, 23), (257, 24), (1000, 186), (70, 187), (70, 300)])
 def test_softmax_gradients_of_whole_and_partial_tiles(lb, N, K):
     """The tiled kernel (256 rows down to 32 per block) and the one for more classes than it takes."""
