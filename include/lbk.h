@@ -386,6 +386,10 @@ typedef struct lbk_histogram_args {
 
 int lbk_histogram(lbk_context* ctx, const lbk_histogram_args* args);
 
+/* The same result the way a rank with peers makes it: the pieces of a node that several blocks build meet in merge trees
+ * (histogram.cu) instead of adding to the histogram with atomics.  A check of that path on one GPU. */
+int lbk_selftest_histogram(lbk_context* ctx, const lbk_histogram_args* args);
+
 /* The same histogram build for callers that cannot allocate device memory at the time of the
  * call: a task running under a runtime that has already handed out the whole memory budget (a
  * cudaMalloc there fails, or takes memory the runtime believes it owns), or a process whose device

@@ -955,7 +955,7 @@ int lbk_quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg
   });
 }
 
-int lbk_histogram(lbk_context* ctx, const lbk_histogram_args* a)
+static int StageHistogram(lbk_context* ctx, const lbk_histogram_args* a, bool merge_tree)
 {
   return lbk::Guard(ctx, [&] {
     LBK_EXPECT(ctx && a, "null argument");
@@ -1075,3 +1075,7 @@ int lbk_leaf_values(lbk_context* ctx, const double* leaf_value, const int32_t* l
 }
 
 }  // extern "C"
+    lv.merge_tree           = merge_tree;
+int lbk_histogram(lbk_context* ctx, const lbk_histogram_args* a) { return StageHistogram(ctx, a, false); }
+int lbk_selftest_histogram(lbk_context* ctx, const lbk_histogram_args* a) { return StageHistogram(ctx, a, true); }
+

@@ -746,8 +746,8 @@ __device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, in
 // scratch for the pieces.  One node, 10M x 64: 240 -> 214 us; 8 nodes 270 -> 241, 128 nodes 277 -> 252; 10M x 128, 128 nodes
 // 470 -> 462; 1.25M x 64, one node 68 -> 46.
 //
-// Merge tree (static ranges, histograms of other ranks' features, where the atomics would cross NVLink): the P pieces of a node that reaches over range boundaries are summed
-// without waits.  A piece writes its 32-bit partial sums to its slot and adds one to the counter
+// Merge tree (static ranges, histograms of other ranks' features, where the atomics would cross NVLink): the P pieces of a
+// node that reaches over range boundaries are summed without waits.  A piece writes its 32-bit partial sums to its slot and adds one to the counter
 // of its group of four; the last one to arrive adds the others' slots to its own sums and goes on
 // as one member of the next level, until one block holds the node's total and writes the
 // histogram.  Nobody waits for anybody: whoever arrives first leaves.
@@ -1455,7 +1455,7 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
   // range boundary, kTreeFanIn per resident block covers every cut
   HistScratch own;
   HistScratch* hs = lv.scratch;
-  const int need_arrive  = hl.smem_path && p.push_recv != nullptr ? kTreeFanIn * hl.grid : 0;
+  const int need_arrive  = hl.smem_path && (p.push_recv != nullptr || lv.merge_tree) ? kTreeFanIn * hl.grid : 0;
   const size_t need_bytes = static_cast<size_t>(need_arrive) * p.mb * kGroup * hl.width * 8;
   const bool kept = hs != nullptr && hs->next_ticket < hs->n_tickets && hs->n_arrive >= need_arrive && hs->partial_bytes >= need_bytes;
   if (!kept) hs = &own;

@@ -309,6 +309,7 @@ struct HistLevel {
   void* const* push_recv     = nullptr;
   long long push_slot_pairs = 0;
   int push_len              = 0;
+  bool merge_tree           = false;  // pieces of a node meet in a merge tree although the histograms are local (lbk_selftest_histogram)
 };
 void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStream_t stream);
 // BuildHistogram followed by the sum over ranks of the n_slots histograms.

@@ -82,11 +82,12 @@ def group_rows(node_of_row, node_begin, n_nodes, ctx=None):
 
 
 def histogram(bins, row_ptr, gpair, row_index, seg, n_features, mode=0, hist=None, ctx=None, host=False,
-              max_abs=None, all_reduce=False, max_bins=0, total_bins=None, pairs_by_position=False):
+              max_abs=None, all_reduce=False, max_bins=0, total_bins=None, pairs_by_position=False, merge_tree=False):
     """Histogram [n_nodes, K, B, 2] (int64 for mode 0, float64 for mode 1) of node-grouped rows.
 
     ``host=True`` takes CPU tensors and lets the library do the copies (the end-to-end path).
-    ``pairs_by_position``: gpair[i] belongs to row_index[i] (the pairs were moved with the row ids)."""
+    ``pairs_by_position``: gpair[i] belongs to row_index[i] (the pairs were moved with the row ids).
+    ``merge_tree``: through ``lbk_selftest_histogram``, the way a rank with peers sums the pieces of a node."""
     dev = bins.device
     ctx = ctx or L.context(None if host else dev.index)
     N = bins.shape[0]
@@ -112,5 +113,5 @@ def histogram(bins, row_ptr, gpair, row_index, seg, n_features, mode=0, hist=Non
     a.all_reduce = int(all_reduce)  # False / True, or 2 = only the owned features are summed
     a.max_bins = int(max_bins)
     a.pairs_by_position = 1 if pairs_by_position else 0
-    ctx.check(ctx.lib.lbk_histogram(ctx.handle, C.byref(a)))
+    ctx.check((ctx.lib.lbk_selftest_histogram if merge_tree else ctx.lib.lbk_histogram)(ctx.handle, C.byref(a)))
     return hist

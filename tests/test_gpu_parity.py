@@ -696,19 +696,21 @@ def test_full_size_histogram_exact(lb):
     assert torch.equal(stages.histogram(bins, row_ptr, gpair, row_index, seg, bench.HIST_FEATURES, mode=0), hist)
 
 
+@pytest.mark.parametrize("merge_tree", [False, True])
 @pytest.mark.parametrize("N,F,K,weights,mode,qmax", [
-    (1_500_000, 64, 1, [0.80, 0.0, 0.15, 0.05], 0, 300),    # one node in about 120 pieces: a deep merge tree
-    (1_500_000, 64, 1, [0.80, 0.0, 0.15, 0.05], 0, 5000),   # ... too many rows for 32-bit sums: the tree is climbed
-                                                            # two levels, the rest are 64-bit atomics
-    (1_500_000, 64, 1, [0.80, 0.0, 0.15, 0.05], 0, 40000),  # ... one level only
-    (1_500_000, 64, 1, [0.80, 0.0, 0.15, 0.05], 0, 400000), # ... a single piece is already too long: no tree
+    (1_500_000, 64, 1, [0.80, 0.0, 0.15, 0.05], 0, 300),    # one node in about 120 pieces (a deep merge tree)
+    (1_500_000, 64, 1, [0.80, 0.0, 0.15, 0.05], 0, 5000),   # ... too many rows for 32-bit sums (the tree is climbed
+                                                            # two levels, the rest are 64-bit atomics)
+    (1_500_000, 64, 1, [0.80, 0.0, 0.15, 0.05], 0, 40000),  # ... (one level only)
+    (1_500_000, 64, 1, [0.80, 0.0, 0.15, 0.05], 0, 400000), # ... a piece is flushed several times (no tree)
     (1_500_000, 96, 3, [0.3, 0.3, 0.2, 0.1, 0.1], 0, 300),  # three groups: the second group set is half empty
     (2_000_000, 32, 2, [1.0] * 37, 0, 300),                 # one group per unit (two blocks per SM)
     (1_500_000, 128, 1, [0.55, 0.45], 1, 0),                # float pairs through the same ranges
 ])
-def test_histogram_static_ranges(lb, oracle, N, F, K, weights, mode, qmax):
-    """Enough rows for the planner to hand out equal static ranges: nodes reach over range
-    boundaries and their pieces meet in the merge tree; sums stay exact (floats within 1e-5)."""
+def test_histogram_static_ranges(lb, oracle, N, F, K, weights, mode, qmax, merge_tree):
+    """Enough rows for the planner to hand out equal static ranges: nodes reach over range boundaries and their pieces
+    add to their histograms with atomics or, as on a rank with peers, meet in merge trees; sums stay exact (floats
+    within 1e-5)."""
     from legateboost_b200 import stages
 
     rng = np.random.default_rng(N + F)
@@ -722,10 +724,10 @@ def test_histogram_static_ranges(lb, oracle, N, F, K, weights, mode, qmax):
         q = rng.integers(-qmax, qmax, size=(N, K, 2), dtype=np.int32)
         q[:, :, 1] = np.abs(q[:, :, 1])
         want = oracle.histogram_q(bins, row_ptr, q, node, n_nodes - 1, 2 * n_nodes - 1)
-        got = stages.histogram(stages.to_padded_rows(dev(bins)), dev(row_ptr), dev(q), row_index, seg, F, mode=0)
+        got = stages.histogram(stages.to_padded_rows(dev(bins)), dev(row_ptr), dev(q), row_index, seg, F, mode=0, merge_tree=merge_tree)
         assert np.array_equal(got.cpu().numpy(), want)
         got = stages.histogram(stages.to_padded_rows(dev(bins)), dev(row_ptr), _by_position(dev(q), row_index), row_index,
-                               seg, F, mode=0, pairs_by_position=True, max_abs=_max_abs(q))
+                               seg, F, mode=0, pairs_by_position=True, max_abs=_max_abs(q), merge_tree=merge_tree)
         assert np.array_equal(got.cpu().numpy(), want)
     else:
         gh = np.stack([rng.normal(size=(N, K)), np.ones((N, K))], axis=2).astype(np.float32)
@@ -733,7 +735,7 @@ def test_histogram_static_ranges(lb, oracle, N, F, K, weights, mode, qmax):
         for by_pos in (False, True):
             pairs = _by_position(dev(gh), row_index) if by_pos else dev(gh)
             got = stages.histogram(stages.to_padded_rows(dev(bins)), dev(row_ptr), pairs, row_index, seg, F, mode=1,
-                                   pairs_by_position=by_pos)
+                                   pairs_by_position=by_pos, merge_tree=merge_tree)
             err = np.abs(got.cpu().numpy() - want).max()
             assert err <= 1e-5 * np.abs(want).max()
 

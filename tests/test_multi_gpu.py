@@ -146,7 +146,8 @@ def _hist_worker(rank, world, port, q):
     for empty_last in (False, True):
         for mode in (0, 1):
             empty = empty_last and rank == world - 1
-            N = 1 if empty else 150000 + 1000 * rank
+            # 74 ranges of more than 4096 rows, of which one node takes about 45: ranges, and a merge tree of several levels
+            N = 1 if empty else 400000 + 1000 * rank
             F, nb, n_nodes = 128, 256, 128
             bins = torch.randint(0, nb, (N, F), dtype=torch.uint8, device=dev, generator=gen)
             row_ptr = torch.arange(F + 1, dtype=torch.int32, device=dev) * nb
@@ -155,6 +156,7 @@ def _hist_worker(rank, world, port, q):
             else:
                 pairs = torch.randn((N, 1, 2), dtype=torch.float32, device=dev, generator=gen)
             node = torch.randint(0, n_nodes, (N,), dtype=torch.int32, device=dev, generator=gen) + (n_nodes - 1)
+            node[torch.rand((N,), device=dev, generator=gen) < 0.6] = n_nodes + 2
             if empty:
                 node[:] = 5 * n_nodes  # its one row belongs to no node of the level: nothing to build
             row_index, seg = stages.group_rows(node, n_nodes - 1, n_nodes)
