@@ -1031,6 +1031,7 @@ static int StageHistogram(lbk_context* ctx, const lbk_histogram_args* a, bool me
     lv.n_nodes              = a->n_nodes;
     lv.out                  = hist;
     lv.float_mode           = a->mode == 1;
+    lv.merge_tree           = merge_tree;
     if (a->all_reduce == 1) lbk::BuildHistogramSummed(ctx, s, lv, a->n_nodes, lbk::HistSum::kSumEverywhere, true, true, stream);
     else if (a->all_reduce == 2) lbk::BuildHistogramSummed(ctx, s, lv, a->n_nodes, lbk::HistSum::kSumOwned, true, true, stream);
     else lbk::BuildHistogram(ctx, s, lv, stream);
@@ -1042,6 +1043,9 @@ static int StageHistogram(lbk_context* ctx, const lbk_histogram_args* a, bool me
     }
   });
 }
+
+int lbk_histogram(lbk_context* ctx, const lbk_histogram_args* a) { return StageHistogram(ctx, a, false); }
+int lbk_selftest_histogram(lbk_context* ctx, const lbk_histogram_args* a) { return StageHistogram(ctx, a, true); }
 
 int lbk_group_rows(lbk_context* ctx, const int32_t* node_of_row, int64_t n_rows, int node_begin, int n_nodes,
                    int32_t* row_index, int32_t* seg, void* stream_)
@@ -1075,7 +1079,3 @@ int lbk_leaf_values(lbk_context* ctx, const double* leaf_value, const int32_t* l
 }
 
 }  // extern "C"
-    lv.merge_tree           = merge_tree;
-int lbk_histogram(lbk_context* ctx, const lbk_histogram_args* a) { return StageHistogram(ctx, a, false); }
-int lbk_selftest_histogram(lbk_context* ctx, const lbk_histogram_args* a) { return StageHistogram(ctx, a, true); }
-
