@@ -217,8 +217,10 @@ __global__ void __launch_bounds__(256)
   pred[e] += __ldg(table + static_cast<int64_t>(__ldg(leaf + i)) * K + k);
 }
 
-// Rows x features x outputs above which a tree of more than 256 samples waits for the number of bins (BuildTreeImpl).
-constexpr int64_t kWidthMattersCells = int64_t{1} << 24;
+// Rows x features x outputs up to which a tree of more than 256 samples has the memory of two-byte ids, 32 MB for either
+// matrix, before it knows whether one byte will do (BuildTreeImpl); above, nothing is laid out before the bins are counted.
+constexpr int64_t kWidthLaterCells = int64_t{1} << 24;
+constexpr int64_t kHistogramCacheBytes = 1000000000;  // (reference: build_tree.cu:1000-1017)
 
 // `round`: a boosting round instead of a tree on given gradients (they are those of round->pred, which gets
 // the leaf values added); the call is then asynchronous.
@@ -367,14 +369,19 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   T* cuts          = in_sketch ? reinterpret_cast<T*>(skb + sk.proposals) : s.alloc<T>(static_cast<size_t>(F) * S);
   int32_t* row_ptr = in_sketch ? reinterpret_cast<int32_t*>(skb + sk.row_ptr) : s.alloc<int32_t>(F + 1);
 
-  // Does the host have to know how many bins there are?  They decide the width of the bin ids (above 256
-  // samples, where the matrix is large enough for that to matter: up to 2^24 cells both widths are built by the same
-  // kernels, and waiting cost 300k x 37 float64, 512 samples, 15 us per tree), the batches of a level whose histograms are larger than the cache (the reference's rule,
-  // below), and the layout that a trace, a sketch or other ranks see.  Otherwise everything is laid out for
-  // the upper bound F x S, and nothing waits for the device before the end of the tree.
+  // Does the host have to know how many bins there are before anything is laid out?  They decide the batches of a level
+  // whose histograms are larger than the cache (the reference's rule, below), the layout that a trace, a sketch or other
+  // ranks see and, above 256 samples, the memory for the ids of a large matrix or for a root of more than the cache.
+  // Otherwise everything is laid out for the upper bound F x S, and up to 256 samples nothing waits for the device before
+  // the end of the tree.  Above them the width of the ids is still open: the host polls for the largest feature's number of
+  // bins, which the device has before it has summed |g| and quantised the pairs, so that it does not run dry (to wait
+  // for the stream and then lay out and queue everything costs 15 us per tree of 300k x 37 float64, this nothing).
+  // Three rounds of depth 6, two-byte ids whatever the columns hold and the width they ask for: columns of 50 values,
+  // 300k x 37 float64, 512 samples 1068 and 964 us, 2048 samples 1500 and 1123; 100k x 64 1155 and 1039 (2048), 921 and 879
+  // (300); 8k x 500 1265 and 1190 (300); 10^6 values, 300k x 37 1242 and 1244, 100k x 64 1043 and 1042, 5k x 20 884 and 882.
   auto cache_depth = [&](int64_t bins, size_t& max_histogram_nodes) {
     // histogram cache rule (reference: build_tree.cu:1000-1017); identical on every rank
-    max_histogram_nodes = std::max<size_t>(1, size_t{1000000000} / (static_cast<size_t>(K) * bins * sizeof(GPairI64)));
+    max_histogram_nodes = std::max<size_t>(1, static_cast<size_t>(kHistogramCacheBytes) / (static_cast<size_t>(K) * bins * sizeof(GPairI64)));
     int d = 0;
     while (static_cast<size_t>(LevelEnd(d + 1)) <= max_histogram_nodes && d <= D) d++;
     return d;
@@ -382,8 +389,9 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   const int64_t bins_bound   = static_cast<int64_t>(F) * S;
   size_t max_histogram_nodes = 0;
   const bool wait_for_bins   = in_sketch || a.trace_hist != nullptr || ctx->n_ranks > 1 ||
-                             (S > 256 && N * F * K > kWidthMattersCells) ||
+                             (S > 256 && (N * F * K > kWidthLaterCells || bins_bound * K > kHistogramCacheBytes / static_cast<int64_t>(sizeof(GPairI64)))) ||
                              cache_depth(bins_bound, max_histogram_nodes) < D - 1;
+  const bool wait_for_width  = S > 256 && !wait_for_bins;
 
   // words that have to be zero before the first level: node sums, arrival counters and partition cursors of
   // the nodes, tickets and merge counters of the histogram launches
@@ -461,7 +469,8 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     pa.zero[2]      = cache;
     pa.zero_n16[2]  = root_zeroed ? static_cast<int64_t>(K) * bins_bound : 0;
     // (a sketch that is reused knows its bins: no kernel counts any and no words are borrowed for them)
-    int32_t* info_host = !sketch_reuse && (wait_for_bins || a.out_total_bins) ? words.get() : nullptr;
+    int32_t* info_host = !sketch_reuse && (wait_for_bins || wait_for_width || a.out_total_bins) ? words.get() : nullptr;
+    if (wait_for_width) words.expect();
     Prologue<T>(ctx, s, pa, row_ptr, info, info_host, sums, qp, stream);
   }
   ProposalInfo pi{static_cast<int>(std::min<int64_t>(bins_bound, INT32_MAX)), S};
@@ -476,17 +485,30 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     LBK_EXPECT(pi.total_bins >= F, "every feature must have at least one proposal");
   }
   const int B = pi.total_bins;  // (an upper bound unless wait_for_bins)
-  const int* max_bins_ptr = wait_for_bins ? nullptr : info + 1;
+  const int* max_bins_ptr = wait_for_bins || wait_for_width ? nullptr : info + 1;
 
   // binned matrix, once per tree
-  const int bin_bytes = pi.max_bins_per_feature <= 256 ? 1 : 2;
-  void* bins          = in_sketch ? static_cast<void*>(skb + sk.bins) : s.alloc_bytes(lbk_bin_matrix_bytes(N, F, bin_bytes));
+  const int bin_bytes_bound = pi.max_bins_per_feature <= 256 ? 1 : 2;
+  void* bins = in_sketch ? static_cast<void*>(skb + sk.bins) : s.alloc_bytes(lbk_bin_matrix_bytes(N, F, bin_bytes_bound));
   // feature-major copy for the repartition (no copy for a stump: nothing is repartitioned; a saved
   // sketch always has it, later trees may be deeper)
   const int64_t pitch_t = (N + 31) / 32 * 32;
   void* bins_t          = in_sketch ? static_cast<void*>(skb + sk.bins_t)
-                          : D > 1   ? s.alloc_bytes(static_cast<size_t>(F) * pitch_t * bin_bytes + 16)
+                          : D > 1   ? s.alloc_bytes(static_cast<size_t>(F) * pitch_t * bin_bytes_bound + 16)
                                     : nullptr;
+
+  // quantised pairs and root sums
+  int2* gpair   = s.alloc<int2>(static_cast<size_t>(N) * K);
+  auto quantise = [&]() {
+    Quantise(ctx, g, h, ldg, form, a.row_offset, N, K, a.seed, gpair, tree.node_sums, qp, max_abs, stream);
+  };
+  if (wait_for_width) {
+    quantise();
+    words.await(stream);
+    pi.max_bins_per_feature = words.get()[1];
+    LBK_EXPECT(words.get()[0] >= F, "every feature must have at least one proposal");
+  }
+  const int bin_bytes = pi.max_bins_per_feature <= 256 ? 1 : 2;
   if (!sketch_reuse)
     BinMatrix<T>(X, ldx, N, F, cuts, S, row_ptr, bins, bins_t, pitch_t, bin_bytes, pi.max_bins_per_feature, stream);
   if (sketch_save) {
@@ -502,9 +524,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     LBK_CUDA(cudaStreamSynchronize(stream));  // `head` is on this frame
   }
 
-  // quantised pairs and root sums
-  int2* gpair = s.alloc<int2>(static_cast<size_t>(N) * K);
-  Quantise(ctx, g, h, ldg, form, a.row_offset, N, K, a.seed, gpair, tree.node_sums, qp, max_abs, stream);
+  if (!wait_for_width) quantise();
 
   const int cdepth = cache_depth(B, max_histogram_nodes);
   // levels >= D are never evaluated; no need to hold them.  The last level's histograms are evaluated as

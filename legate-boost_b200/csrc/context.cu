@@ -164,6 +164,25 @@ int32_t* HostWords::get()
   return words_;
 }
 
+void HostWords::expect() { *reinterpret_cast<volatile int64_t*>(get()) = -1; }
+
+void HostWords::await(cudaStream_t stream)
+{
+  const volatile int64_t* both = reinterpret_cast<const volatile int64_t*>(get());
+  for (unsigned spin = 1; *both == -1; ++spin) {
+    if ((spin & 0xffff) != 0) continue;
+    // (now and then: does what is queued still run?)
+    const cudaError_t e = cudaStreamQuery(stream);
+    if (e == cudaErrorNotReady) {
+      cudaGetLastError();
+      continue;
+    }
+    LBK_CUDA(e);
+    LBK_EXPECT(*both != -1, "the number of bins has not been written");
+  }
+  settled();
+}
+
 HostWords::~HostWords()
 {
   if (words_ == nullptr || !settled_) return;

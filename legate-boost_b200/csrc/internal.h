@@ -135,6 +135,10 @@ class HostWords {
   HostWords& operator=(const HostWords&) = delete;
   int32_t* get();  // borrowed on first use
   void settled() { settled_ = true; }
+  // Before the kernel that writes the words (both with one store) is queued; and, afterwards, the wait for that store,
+  // which does not wait for what the kernel does besides.
+  void expect();
+  void await(cudaStream_t stream);
 
  private:
   lbk_context* ctx_;

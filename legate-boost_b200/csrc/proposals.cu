@@ -210,11 +210,9 @@ __global__ void __launch_bounds__(1024)
     if (tid == 0) {
       info[0] = carry_s;
       info[1] = max_s;
-      if (info_host != nullptr) {
-        volatile int32_t* h = info_host;
-        h[0] = carry_s;
-        h[1] = max_s;
-      }
+      // (one store of 8 bytes: a host that polls sees both or neither)
+      if (info_host != nullptr)
+        *reinterpret_cast<volatile unsigned long long*>(info_host) = static_cast<unsigned>(carry_s) | static_cast<unsigned long long>(max_s) << 32;
     }
   }
   if (sums == nullptr) return;

@@ -1264,7 +1264,7 @@ def test_error_texts_of_calls_on_several_threads(lb):
     assert seen == texts
 
 
-@pytest.mark.parametrize("N,S", [(20000, 64), (20000, 400), (500, 64)])
+@pytest.mark.parametrize("N,S", [(20000, 64), (20000, 400), (3_400_000, 400), (500, 64)])  # (400: a wait for the width, for the layout)
 @pytest.mark.parametrize("fixed_sketch", [False, True])
 def test_calls_give_back_the_words_they_borrow(lb, N, S, fixed_sketch):
     import ctypes as C
@@ -1428,15 +1428,16 @@ def test_a_round_that_fails_waits_for_the_rounds_before_it(lb):
     lb.LBRegressor(n_estimators=1, base_models=(lb.Tree(max_depth=3),), random_state=0).fit(X, y)
 
 
-@pytest.mark.parametrize("distinct", [3, 200, 10 ** 6])
-@pytest.mark.parametrize("dtype", [np.float32, np.float64])
-def test_fine_bins_without_waiting_for_their_number(lb, oracle, dtype, distinct):
-    """More than 256 samples on a matrix so small that the width of the bin ids does not wait for the number of bins, whether
-    one byte would have done or not; rounds and trees grow what the oracle grows."""
+@pytest.mark.parametrize("N,F,dtype,distinct", [(21001, 7, dtype, distinct) for dtype in (np.float32, np.float64) for distinct in (3, 200, 10 ** 6)] +
+                         [(130_001, 37, dtype, distinct) for dtype in (np.float32, np.float64) for distinct in (3, 300, 10 ** 6)] +
+                         [(230_001, 75, np.float32, 50), (230_001, 75, np.float32, 10 ** 6)])
+def test_fine_bins_of_one_byte_and_of_two(lb, oracle, N, F, dtype, distinct):
+    """More than 256 samples, columns whose values ask for ids of one byte and of two: matrices whose ids wait for the
+    number of bins, and (above 2^24 cells) one whose whole layout does."""
     from legateboost_b200.tree import build_tree_arrays
 
     rs = np.random.RandomState(distinct % 97)
-    N, F, D = 21001, 7, 5
+    D = 5
     X = np.round(rs.random((N, F)) * distinct).astype(dtype)
     g, h = rs.normal(size=(N, 1)), rs.random((N, 1)) + 0.1
     want = oracle.build_tree(X, g, h, max_depth=D, split_samples=700, seed=11, mode="Q")
