@@ -36,6 +36,8 @@ constexpr int kLeafMaxPitch = 256;
 constexpr int kLeafMaxNodes = 8192;
 constexpr int kLeafWarps    = 8;
 constexpr int kLeafTable    = 1024;  // leaf values (nodes x outputs) that every block makes for itself
+constexpr int kLeafOutputs  = 24;    // up to so many a round adds where it finds the leaves
+constexpr int kLeafAhead    = 4;     // of several outputs: values of a lane on their way
 
 struct LeafRound {
   double* pred;      // [n_rows][K]
@@ -46,12 +48,14 @@ struct LeafRound {
   double* hessian;
 };
 
-template <typename BinT, bool kRound>
-__global__ void __launch_bounds__(kLeafWarps * 32)
+// kForm: 0 no round, 1 a round of one output, 2 of several
+template <typename BinT, int kForm>
+__global__ void __launch_bounds__(kLeafWarps * 32, kForm == 0 ? 6 : 5)
   k_leaf_of_row_tiled(const BinT* __restrict__ bins, int pitch_bytes, int64_t n_rows, const int32_t* __restrict__ feature,
                       const int32_t* __restrict__ split_bin, int max_depth, int n_nodes, int32_t* __restrict__ leaf,
                       const __grid_constant__ LeafRound rnd)
 {
+  constexpr bool kRound = kForm != 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned* s_node = reinterpret_cast<unsigned*>(smem_raw);
   __shared__ double s_value[kRound ? kLeafTable : 1];
@@ -85,7 +89,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32)
     const uint4* src   = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(bins) + row0 * pitch_bytes);
     const int n_vec    = rows * vec_per_row;
     double before = 0.0;  // (one output: on its way while the row is copied and walked)
-    if (kRound && rnd.K == 1 && lane < rows) before = rnd.pred[row0 + lane];
+    if (kForm == 1 && lane < rows) before = rnd.pred[row0 + lane];
     __syncwarp();  // the previous chunk's walks are done with the tile
     for (int v = lane; v < n_vec; v += 32) {
       const uint4 w = __ldcs(src + v);
@@ -107,14 +111,28 @@ __global__ void __launch_bounds__(kLeafWarps * 32)
         node = 2 * node + 1 + (static_cast<unsigned>(b[(nd >> 16) - 1]) > (nd & 0xffffu) ? 1 : 0);
       }
       if (leaf != nullptr) leaf[row0 + lane] = node;
-      if (kRound && rnd.K == 1) rnd.pred[row0 + lane] = before + value[node];
+      if (kForm == 1) rnd.pred[row0 + lane] = before + value[node];
     }
-    if (kRound && rnd.K > 1) {
-      double* p = rnd.pred + row0 * rnd.K;
-      for (int e0 = 0; e0 < rows * rnd.K; e0 += 32) {
-        const int e = e0 + lane, r = e / rnd.K;
-        const int nd = __shfl_sync(0xffffffffu, node, min(r, 31));
-        if (e < rows * rnd.K) p[e] += value[static_cast<int64_t>(nd) * rnd.K + (e - r * rnd.K)];
+    if (kForm == 2) {
+      // the lanes over the warp's rows x outputs, kLeafAhead of a lane's at a time: the loads of one after the other's
+      // store would wait for memory each (depth 7, 16 outputs: 20k x 20 17.7 us, now 11.2, 200k x 30 31.0 and 17.6; ten outputs,
+      // 1M x 100 65.5 and 55.6)
+      double* p   = rnd.pred + row0 * rnd.K;
+      const int n = rows * rnd.K;
+      for (int e0 = lane; e0 - lane < n; e0 += 32 * kLeafAhead) {
+        double sum[kLeafAhead], add[kLeafAhead];
+#pragma unroll
+        for (int u = 0; u < kLeafAhead; ++u)
+          if (e0 + 32 * u < n) sum[u] = p[e0 + 32 * u];
+#pragma unroll
+        for (int u = 0; u < kLeafAhead; ++u) {
+          const int e = e0 + 32 * u, r = e / rnd.K;
+          const int nd = __shfl_sync(0xffffffffu, node, min(r, 31));
+          if (e < n) add[u] = value[static_cast<int64_t>(nd) * rnd.K + (e - r * rnd.K)];
+        }
+#pragma unroll
+        for (int u = 0; u < kLeafAhead; ++u)
+          if (e0 + 32 * u < n) p[e0 + 32 * u] = sum[u] + add[u];
       }
     }
   }
@@ -151,7 +169,7 @@ void LeafOfRow(lbk_context* ctx, const void* bins, int64_t pitch, int64_t N, int
   const int64_t pitch_bytes = pitch * static_cast<int64_t>(sizeof(BinT));
   if (LeafTiled(bins, pitch_bytes, F, M)) {
     const size_t smem = (static_cast<size_t>(M) * 4 + 15) / 16 * 16 + static_cast<size_t>(kLeafWarps) * 32 * (pitch_bytes + 4);
-    auto fn           = rnd != nullptr ? k_leaf_of_row_tiled<BinT, true> : k_leaf_of_row_tiled<BinT, false>;
+    auto fn           = rnd == nullptr ? k_leaf_of_row_tiled<BinT, 0> : rnd->K == 1 ? k_leaf_of_row_tiled<BinT, 1> : k_leaf_of_row_tiled<BinT, 2>;
     if (smem > 36 * 1024) AllowSharedMemory(ctx, fn, 12 * 1024);  // (the limit without it counts the static part too)
     int per_sm = 0;
     LBK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLeafWarps * 32, smem));
@@ -715,7 +733,10 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   }
 
   const int64_t pitch  = static_cast<int64_t>((F + kGroup - 1) / kGroup) * kGroup;
-  const bool add_here  = round != nullptr && N > 0 && LeafTiled(bins, pitch * bin_bytes, F, M);  // by the kernel that finds the leaves
+  // By the kernel that finds the leaves.  A warp adds the outputs of 32 rows: of many outputs and few rows too little is in
+  // flight.  Depth 7, this and the three kernels: 5k x 60, 16 outputs 11.7 and 12.5 us, 40 outputs 17.2 and 12.6, 100 outputs
+  // 62 and 14 (with one value of a lane on its way); 200k x 30, 16 outputs 17.6 and 25.4, 40 outputs 27.8 and 43.5.
+  const bool add_here  = round != nullptr && N > 0 && K <= kLeafOutputs && LeafTiled(bins, pitch * bin_bytes, F, M);
   const bool make_here = add_here && static_cast<int64_t>(M) * K <= kLeafTable;
   if (!make_here) FinishTree(tree, qp, K, a.l1_regularization, a.l2_regularization, hessian, stream);
   if ((a.out_leaf != nullptr || round != nullptr) && N > 0) {

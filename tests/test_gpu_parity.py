@@ -1446,14 +1446,31 @@ def test_fine_bins_of_one_byte_and_of_two(lb, oracle, N, F, dtype, distinct):
         assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
 
 
-@pytest.mark.parametrize("N,F,K,depth", [(17001, 5, 1, 3), (20011, 9, 1, 9), (17003, 6, 1, 10), (6007, 40, 3, 7), (5801, 300, 3, 4), (5801, 33, 10, 7)])
+@pytest.mark.parametrize("N,F,K", [(30011, 9, 1), (30011, 9, 2), (20003, 40, 3)])
+@pytest.mark.parametrize("S", [256, 700])
+def test_squared_error_rounds_are_trees_on_their_gradients(lb, N, F, K, S):
+    """Rounds read predictions and labels, of one target or several, where trees driven one by one are given (g, h)."""
+    rs = np.random.RandomState(K)
+    X, y = dev(rs.normal(size=(N, F)).astype(np.float32)), dev(rs.normal(size=(N, K)))
+    make = lambda: lb.LBRegressor(n_estimators=3, base_models=(lb.Tree(max_depth=5, split_samples=S),), random_state=5, learning_rate=0.3)
+    one_by_one = make()
+    one_by_one._weighted_gradient = lambda *a: lb.LBRegressor._weighted_gradient(one_by_one, *a)  # (gradients of one's own are asked for)
+    want, got = one_by_one.fit(X, y), make().fit(X, y)
+    for a, b in zip(want, got):
+        for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
+            assert torch.equal(getattr(a, name), getattr(b, name)), name
+    assert torch.equal(want._train_pred, got._train_pred)
+
+
+@pytest.mark.parametrize("N,F,K,depth", [(17001, 5, 1, 3), (20011, 9, 1, 9), (17003, 6, 1, 10), (6007, 40, 3, 7), (5801, 300, 3, 4), (5801, 33, 10, 7),
+                                         (20011, 4, 2, 4), (5801, 9, 24, 3), (5801, 9, 24, 6), (5801, 9, 30, 4)])
 def test_rounds_add_the_leaf_values_where_the_leaves_are_found(lb, N, F, K, depth):
     """Leaf tables made by every block and read from memory (more than 1024 values), rows too wide for the tiled walk: the
     kept predictions are those of the trees."""
     rs = np.random.RandomState(depth)
     X = dev(rs.normal(size=(N, F)).astype(np.float32))
-    y = dev(rs.normal(size=N)) if K == 1 else dev(rs.randint(0, K, size=N).astype(np.float64))
-    make = lb.LBRegressor if K == 1 else lb.LBClassifier
+    y = dev(rs.normal(size=(N, K))) if K <= 2 else dev(rs.randint(0, K, size=N).astype(np.float64))
+    make = lb.LBRegressor if K <= 2 else lb.LBClassifier
     m = make(n_estimators=3, base_models=(lb.Tree(max_depth=depth),), random_state=5).fit(X, y)
     want = m.model_init_.repeat(N, 1)
     for t in m:
