@@ -528,7 +528,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   }
   const int bin_bytes = pi.max_bins_per_feature <= 256 ? 1 : 2;
   if (!sketch_reuse)
-    BinMatrix<T>(X, ldx, N, F, cuts, S, row_ptr, bins, bins_t, pitch_t, bin_bytes, pi.max_bins_per_feature, stream);
+    BinMatrix<T>(X, ldx, N, F, cuts, S, row_ptr, bins, bins_t, pitch_t, bin_bytes, pi.max_bins_per_feature, ctx->d_status, stream);
   if (sketch_save) {
     head.magic                = kSketchMagic;
     head.total_bins           = pi.total_bins;
@@ -963,10 +963,11 @@ int lbk_bin_matrix(lbk_context* ctx, const void* X, int x_dtype, int64_t ldx, in
     LBK_EXPECT(bin_bytes == 2 || mb <= 256, "one-byte bins need <= 256 proposals per feature");
     if (x_dtype == LBK_F32)
       lbk::BinMatrix<float>(static_cast<const float*>(X), ldx, n_rows, n_features, static_cast<const float*>(proposals), 0,
-                            row_ptr, bins, nullptr, 0, bin_bytes, mb, stream);
+                            row_ptr, bins, nullptr, 0, bin_bytes, mb, ctx->d_status, stream);
     else
       lbk::BinMatrix<double>(static_cast<const double*>(X), ldx, n_rows, n_features,
-                             static_cast<const double*>(proposals), 0, row_ptr, bins, nullptr, 0, bin_bytes, mb, stream);
+                             static_cast<const double*>(proposals), 0, row_ptr, bins, nullptr, 0, bin_bytes, mb,
+                             ctx->d_status, stream);
   });
 }
 

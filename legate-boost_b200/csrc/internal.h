@@ -265,7 +265,7 @@ template <typename T>
 // bins_t (optional): feature-major copy, bins_t[f * pitch_t + row], pitch_t a multiple of 32 >= n_rows
 // cut_stride > 0: the proposals of feature f begin at f * cut_stride (0: at row_ptr[f])
 void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposals, int64_t cut_stride, const int32_t* row_ptr,
-               void* bins, void* bins_t, int64_t pitch_t, int bin_bytes, int max_bins_per_feature,
+               void* bins, void* bins_t, int64_t pitch_t, int bin_bytes, int max_bins_per_feature, int* status,
                cudaStream_t stream);
 // quantise.cu.  root_sums and max_abs are zero before the call.
 void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, const GradientForm& form, int64_t row_offset,

@@ -488,6 +488,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
 // (a table of bytes, whose lookups are three passes, a store per row, eight values ahead, a table filled by reads 1 KB apart)
 // and now: 100M x 64: 8430 -> 6960 us (the copy rate of HBM gives 5870), 10M x 64: 840 -> 696, 1M x 100: 221 -> 175,
 // 200k x 50: 42 -> 25.  Eight values ahead instead of sixteen, in this layout: 10M x 64 827 us.
+constexpr int kFaultBinLayout  = 32;  // status word: shared memory is not laid out as the kernel's addresses need it
 constexpr int kBuckets         = 512;
 constexpr int kLutThreads      = 1024;
 constexpr int kLutWarps        = kLutThreads / 32;
@@ -506,13 +507,21 @@ static_assert(kLutTilesAt >= 2048 && kLutStageAt + kLutRows * (kGroup + 1) * 4 <
 template <bool kCopyT>
 __global__ void __launch_bounds__(kLutThreads, 1)
   k_bin_lut(const float* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const float* __restrict__ proposals,
-            int64_t cut_stride, const int32_t* __restrict__ row_ptr, uint8_t* __restrict__ bins, uint8_t* __restrict__ bins_t, int64_t pitch_t)
+            int64_t cut_stride, const int32_t* __restrict__ row_ptr, uint8_t* __restrict__ bins, uint8_t* __restrict__ bins_t, int64_t pitch_t,
+            int* __restrict__ status)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_n[kGroup];
   __shared__ float2 s_map[kGroup];
   // (addresses of the shared window as offsets from where the dynamic part begins)
-  unsigned char* window = smem_raw - static_cast<unsigned>(__cvta_generic_to_shared(smem_raw));
+  const unsigned dynamic_at = static_cast<unsigned>(__cvta_generic_to_shared(smem_raw));
+  unsigned dynamic_bytes;
+  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynamic_bytes));
+  if (dynamic_at > kLutTilesAt || kLutEnd > dynamic_at + dynamic_bytes) {  // (not what the constants above were made for)
+    if (threadIdx.x == 0 && status != nullptr) ReportFault(status, kFaultBinLayout);
+    return;
+  }
+  unsigned char* window = smem_raw - dynamic_at;
   auto row_of     = [&](int j) { return reinterpret_cast<float*>(window + kLutAt + j * kLutRow); };
   const int f0    = blockIdx.y * kGroup;
   const int lane  = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -877,7 +886,8 @@ constexpr int64_t kLutFillRows = 2048, kSmemFillRows = 512;
 
 template <typename T>
 void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposals, int64_t cut_stride, const int32_t* row_ptr,
-               void* bins, void* bins_t, int64_t pitch_t, int bin_bytes, int max_bins_per_feature, cudaStream_t stream)
+               void* bins, void* bins_t, int64_t pitch_t, int bin_bytes, int max_bins_per_feature, int* status,
+               cudaStream_t stream)
 {
   if (n_rows <= 0) return;
   LBK_EXPECT(n_rows <= 2000000000ll && ldx <= (1 << 27), "bin_matrix: at most 2e9 rows per rank and a row pitch of 2^27 elements");
@@ -931,7 +941,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       auto fn = bins_t != nullptr ? k_bin_lut<true> : k_bin_lut<false>;
       LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLutEnd)));
       fn<<<make_grid(1, kLutFillRows), kLutThreads, kLutEnd, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, static_cast<uint8_t*>(bins),
-                                                  static_cast<uint8_t*>(bins_t), pitch_t);
+                                                  static_cast<uint8_t*>(bins_t), pitch_t, status);
       LBK_LAUNCH_CHECK();
       return;
     }
@@ -975,8 +985,8 @@ template void Prologue<float>(lbk_context*, Scratch&, PrologueArgs<float>, int32
 template void Prologue<double>(lbk_context*, Scratch&, PrologueArgs<double>, int32_t*, int32_t*, int32_t*, double*,
                                QuantParams*, cudaStream_t);
 template void BinMatrix<float>(const float*, int64_t, int64_t, int, const float*, int64_t, const int32_t*, void*, void*, int64_t,
-                               int, int, cudaStream_t);
+                               int, int, int*, cudaStream_t);
 template void BinMatrix<double>(const double*, int64_t, int64_t, int, const double*, int64_t, const int32_t*, void*, void*,
-                                int64_t, int, int, cudaStream_t);
+                                int64_t, int, int, int*, cudaStream_t);
 
 }  // namespace lbk
