@@ -30,8 +30,9 @@ namespace {
 // memory too, feature + 1 and split bin packed into one word.
 //
 // In a boosting round the same kernel makes the tree's leaf values and hessians (every block its own table, where there
-// are few enough; the first one writes them out) and adds the leaf values to the prediction, which took two launches more
-// and the leaf record's way through memory: per round 200k x 50, depth 6: 9.2 -> 5.9 us; 10M x 64, depth 8: 182 -> 149.
+// are few enough; the first one writes them out) and adds the leaf values to the prediction (up to kLeafOutputs outputs),
+// which took two launches more and the leaf record's way through memory: per round 200k x 50, depth 6: 9.2 -> 5.9 us; 10M x 64,
+// depth 8: 182 -> 149.
 constexpr int kLeafMaxPitch = 256;
 constexpr int kLeafMaxNodes = 8192;
 constexpr int kLeafWarps    = 8;
@@ -407,7 +408,8 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   const int64_t bins_bound   = static_cast<int64_t>(F) * S;
   size_t max_histogram_nodes = 0;
   const bool wait_for_bins   = in_sketch || a.trace_hist != nullptr || ctx->n_ranks > 1 ||
-                             (S > 256 && (N * F * K > kWidthLaterCells || bins_bound * K > kHistogramCacheBytes / static_cast<int64_t>(sizeof(GPairI64)))) ||
+                             (S > 256 && (N * F * K > kWidthLaterCells ||
+                                          bins_bound * K > kHistogramCacheBytes / static_cast<int64_t>(sizeof(GPairI64)))) ||
                              cache_depth(bins_bound, max_histogram_nodes) < D - 1;
   const bool wait_for_width  = S > 256 && !wait_for_bins;
 

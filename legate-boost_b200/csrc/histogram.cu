@@ -747,10 +747,10 @@ __device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, in
 // 470 -> 462; 1.25M x 64, one node 68 -> 46.
 //
 // Merge tree (static ranges, histograms of other ranks' features, where the atomics would cross NVLink): the P pieces of a
-// node that reaches over range boundaries are summed without waits.  A piece writes its 32-bit partial sums to its slot and adds one to the counter
-// of its group of four; the last one to arrive adds the others' slots to its own sums and goes on
-// as one member of the next level, until one block holds the node's total and writes the
-// histogram.  Nobody waits for anybody: whoever arrives first leaves.
+// node that reaches over range boundaries are summed without waits.  A piece writes its 32-bit partial sums to its slot and
+// adds one to the counter of its group of four; the last one to arrive adds the others' slots to its own sums and goes on
+// as one member of the next level, until one block holds the node's total and writes the histogram.  Nobody waits for
+// anybody: whoever arrives first leaves.  (lbk_selftest_histogram takes it with local histograms.)
 template <bool kFloat, int W, RowOrder kOrder>
 __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
   k_hist_smem(const HistParams p)

@@ -481,12 +481,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
 //
 // The feature-major copy is 32 streams per block that lie n_rows bytes apart.  Four warps with neighbouring rows write
 // their tiles together, 128 bytes of a feature at a time: with 32 bytes per warp the 100M rows took 9430 us (and 5960
-// without the copy, of which that is 1 ms at the copy rate of HBM), with eight or sixteen warps 6940 and 8120 (they wait for each other;
-// 10M: 712 and 818).
+// without the copy, of which that is 1 ms at the copy rate of HBM), with eight or sixteen warps 6940 and 8120 (they wait for
+// each other; 10M: 712 and 818).  Of 1M x 100, whose copy stays in L2, a warp by itself takes 158 instead of 175.
 //
-// Bound by the issue slots and the load/store pipe (262 instructions and about 62 passes per 256 ids), close to HBM.  Measured with the copy, before
-// (a table of bytes, whose lookups are three passes, a store per row, eight values ahead, a table filled by reads 1 KB apart)
-// and now: 100M x 64: 8430 -> 6960 us (the copy rate of HBM gives 5870), 10M x 64: 840 -> 696, 1M x 100: 221 -> 175,
+// Bound by the issue slots and the load/store pipe (262 instructions and about 62 passes per 256 ids), close to HBM.
+// Measured with the copy, before (a table of bytes, whose lookups are three passes, a store per row, eight values ahead, a
+// table filled by reads 1 KB apart) and now: 100M x 64: 8430 -> 6960 us (the copy rate of HBM gives 5870), 10M x 64: 840 -> 696, 1M x 100: 221 -> 175,
 // 200k x 50: 42 -> 25.  Eight values ahead instead of sixteen, in this layout: 10M x 64 827 us.
 constexpr int kFaultBinLayout  = 32;  // status word: shared memory is not laid out as the kernel's addresses need it
 constexpr int kBuckets         = 512;
