@@ -398,6 +398,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   // Three rounds of depth 6, two-byte ids whatever the columns hold and the width they ask for: columns of 50 values,
   // 300k x 37 float64, 512 samples 1068 and 964 us, 2048 samples 1500 and 1123; 100k x 64 1155 and 1039 (2048), 921 and 879
   // (300); 8k x 500 1265 and 1190 (300); 10^6 values, 300k x 37 1242 and 1244, 100k x 64 1043 and 1042, 5k x 20 884 and 882.
+  // (Trees of few rows are bound by the host: two rounds of 1.4k x 48, 512 samples, all values distinct 667 and 677.)
   auto cache_depth = [&](int64_t bins, size_t& max_histogram_nodes) {
     // histogram cache rule (reference: build_tree.cu:1000-1017); identical on every rank
     max_histogram_nodes = std::max<size_t>(1, static_cast<size_t>(kHistogramCacheBytes) / (static_cast<size_t>(K) * bins * sizeof(GPairI64)));
