@@ -75,6 +75,7 @@ struct HistParams {
   const GPairI64* node_sums;   // null: every node is built; else the smaller child of every pair
   int node_begin;
   int n_nodes;
+  const int* build_all;        // not null and not 0 there: every node is built although node_sums is given
   const int* max_abs;          // largest |grad|, |hess| of the pairs (null for float pairs)
   // the plan, where it was made by k_hist_plan (plan == null: the kernel plans for itself)
   const int32_t* chunk_off;  // [n_nodes+1] chunks before each node (tickets drawn from a counter)
@@ -101,16 +102,18 @@ struct HistParams {
   int push_len;              // pairs per segment in a receive buffer (bound of the owned bins)
 };
 
+__device__ inline bool OneOfTwo(const HistParams& p) { return p.node_sums != nullptr && (p.build_all == nullptr || *p.build_all == 0); }
+
 // Rows of node j of the batch that have to be summed: 0 for the sibling that is derived.
 __device__ inline int BuiltRows(const HistParams& p, int j)
 {
   const int rows = p.seg_end[j] - p.seg_begin[j];
   if (rows <= 0) return 0;
-  if (p.node_sums == nullptr) return rows;
+  if (!OneOfTwo(p)) return rows;
   const bool left = SmallerChildIsLeft(p.node_sums, p.K, p.node_begin + (j & ~1));
   return left == ((j & 1) == 0) ? rows : 0;
 }
-__device__ inline int SlotOf(const HistParams& p, int j) { return p.node_sums != nullptr ? j >> 1 : j; }
+__device__ inline int SlotOf(const HistParams& p, int j) { return OneOfTwo(p) ? j >> 1 : j; }
 __device__ inline int RowsSafe(const int* max_abs)
 {
   return max_abs ? 2147483647 / max(1, max(max_abs[0], max_abs[1])) : 2147483647;
@@ -1423,6 +1426,7 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
   p.seg_end      = lv.seg_end;
   p.node_sums    = lv.node_sums;
   p.node_begin   = lv.node_begin;
+  p.build_all    = lv.build_all;
   p.n_nodes      = lv.n_nodes;
   p.status       = ctx->d_status;
   p.pairs_by_position = lv.pairs_by_position ? 1 : 0;
@@ -1697,6 +1701,7 @@ extern "C" int lbk_histogram_noalloc(int device, const lbk_histogram_args* a)
     p.seg_end      = a->seg + 1;
     p.node_sums    = nullptr;
     p.node_begin   = 0;
+    p.build_all    = nullptr;
     p.n_nodes      = a->n_nodes;
     p.chunk_off    = chunk_off;
     p.plan         = plan;

@@ -267,10 +267,11 @@ template <typename T>
 void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposals, int64_t cut_stride, const int32_t* row_ptr,
                void* bins, void* bins_t, int64_t pitch_t, int bin_bytes, int max_bins_per_feature, int* status,
                cudaStream_t stream);
-// quantise.cu.  root_sums and max_abs are zero before the call.
+// quantise.cu.  root_sums, max_abs and hess_below_one (may be null; 1 if some quantised hessian is below one) are zero before
+// the call.
 void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, const GradientForm& form, int64_t row_offset,
               int64_t n_local, int K, int seed, int2* gpair, GPairI64* root_sums, const QuantParams* params, int* max_abs /* device [2] */,
-              cudaStream_t stream);
+              int* hess_below_one, cudaStream_t stream);
 // histogram.cu
 struct HistScratch {
   unsigned int* arrive   = nullptr;  // [n_arrive], zero
@@ -303,6 +304,7 @@ struct HistLevel {
   // siblings and only the smaller one is built (SmallerChildIsLeft), into slot j / 2.
   const GPairI64* node_sums = nullptr;
   int node_begin            = 0;
+  const int* build_all      = nullptr;  // device word: where it is not 0 every node is built although node_sums is given
   void* out;               // [n_slots, K, B] pairs (int64 or double), already zeroed
   bool float_mode;
   // scratch that a tree keeps for all its levels (null: the call makes its own): words that are zero
@@ -348,6 +350,7 @@ struct ScanSplitLevel {
   int f_begin, f_end;           // the features scanned and searched (the owned ones with several ranks)
   bool derive;                  // pairs of siblings, one of them built
   bool write_hist;
+  const int* build_all = nullptr;  // device word (HistLevel): the call does nothing where it says the other of `derive`
 };
 // cuts: the split proposals, feature f's from f * cut_stride on.  arrived: one counter per tree node, zero
 // before the first call of a tree.  With exchange_records every rank's best candidate of every node

@@ -26,7 +26,8 @@ namespace {
 __global__ void __launch_bounds__(256)
   k_quantise(const double* __restrict__ g, const double* __restrict__ h, int64_t ldg, const GradientForm form,
              int64_t row_offset, int64_t n_local, int K, long long seed, const QuantParams* __restrict__ qp_ptr,
-             int2* __restrict__ gpair, GPairI64* __restrict__ root_sums, int* __restrict__ max_abs)
+             int2* __restrict__ gpair, GPairI64* __restrict__ root_sums, int* __restrict__ max_abs,
+             int* __restrict__ hess_below_one)
 {
   extern __shared__ unsigned long long s_sum[];  // [K][2]
   __shared__ int s_max[2];
@@ -38,7 +39,7 @@ __global__ void __launch_bounds__(256)
   const int64_t threads = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t rows_per_turn = threads / K;  // >= 1: the launcher gives at least K threads
   const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + tid;
-  int mg = 0, mh = 0;
+  int mg = 0, mh = 0, lowest = INT32_MAX;
   if (t < rows_per_turn * K) {
     const int k = static_cast<int>(t % K);
     long long sg = 0, sh = 0;
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(256)
       sh += q.y;
       mg = max(mg, q.x == INT32_MIN ? INT32_MAX : abs(q.x));
       mh = max(mh, q.y == INT32_MIN ? INT32_MAX : abs(q.y));
+      lowest = min(lowest, q.y);
     }
     if (K == 1) {
       // every lane holds the same output: one pair of shared-memory atomics per warp
@@ -67,7 +69,7 @@ __global__ void __launch_bounds__(256)
       atomicAdd(&s_sum[2 * k + 1], static_cast<unsigned long long>(sh));
     }
   }
-  __syncthreads();
+  if (__syncthreads_or(lowest < 1) != 0 && tid == 0 && hess_below_one != nullptr) *hess_below_one = 1;
   for (int i = tid; i < 2 * K; i += blockDim.x) {
     unsigned long long* dst = reinterpret_cast<unsigned long long*>(root_sums) + i;  // grad, hess of k = i / 2
     if (s_sum[i] != 0ull) atomicAdd(dst, s_sum[i]);
@@ -89,7 +91,8 @@ __global__ void __launch_bounds__(256)
 }  // namespace
 
 void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, const GradientForm& form, int64_t row_offset,
-              int64_t n_local, int K, int seed, int2* gpair, GPairI64* root_sums, const QuantParams* params, int* max_abs, cudaStream_t stream)
+              int64_t n_local, int K, int seed, int2* gpair, GPairI64* root_sums, const QuantParams* params, int* max_abs, int* hess_below_one,
+              cudaStream_t stream)
 {
   if (n_local > 0) {
     int64_t blocks = (n_local * K + 511) / 512;  // (two elements per thread: fewer blocks at the common words)
@@ -100,7 +103,8 @@ void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, c
     LBK_EXPECT(smem <= 48 * 1024, "too many outputs for the quantiser's block sums");
     if (smem > 40 * 1024) AllowSharedMemory(ctx, k_quantise, 1024);  // (the limit without it counts the static part too)
     k_quantise<<<static_cast<unsigned>(blocks), 256, smem, stream>>>(g, h, ldg, form, row_offset, n_local, K,
-                                                                  static_cast<long long>(seed), params, gpair, root_sums, max_abs);
+                                                                  static_cast<long long>(seed), params, gpair, root_sums, max_abs,
+                                                                  hess_below_one);
     LBK_LAUNCH_CHECK();
   }
   AllReduce(ctx, root_sums, static_cast<size_t>(2) * K, LBK_I64, LBK_SUM, stream);

@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs ? 3 : 4)
   __shared__ SliceBest s_best[2];
   __shared__ bool s_last;
   const ScanSplitLevel& lv = p.lv;
+  if (lv.build_all != nullptr && (*lv.build_all != 0) == kDerive) return;
   const int K = lv.K, unit = blockIdx.x, slices = gridDim.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int node0 = lv.node_begin + (kDerive ? 2 * unit : unit);

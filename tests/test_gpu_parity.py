@@ -453,6 +453,26 @@ def test_build_tree_level_batching(lb, oracle):
     assert np.array_equal(got["leaf_value"].cpu().numpy(), want.leaf_value)
 
 
+@pytest.mark.parametrize("zeros", [False, True])
+@pytest.mark.parametrize("N,F,K,D", [(2500, 600, 2, 8), (2500, 600, 2, 10), (700, 1000, 1, 9)])
+def test_levels_outside_the_cache(lb, oracle, N, F, K, D, zeros):
+    """Levels that the reference builds node by node: derived where every quantised hessian is at least one (in one batch,
+    in two, and below a level that was not kept), built where some are 0, which a derived node would show."""
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.RandomState(N + F + D)
+    X = rs.random((N, F)).astype(np.float32)
+    X[:, 0] = np.round(X[:, 0] * 5) / 5
+    g = rs.normal(size=(N, K))
+    h = rs.random((N, K)) + 0.1
+    if zeros:
+        h[rs.random(N) < 0.3] = 0.0
+    want = oracle.build_tree(X, g, h, max_depth=D, split_samples=256, seed=5, mode="Q")
+    got = build_tree_arrays(dev(X), dev(g), dev(h), max_depth=D, split_samples=256, seed=5, row_offset=0, dataset_rows=N)
+    for name in ("feature", "split_value", "node_sums", "gain", "hessian", "leaf_value"):
+        assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
+
+
 def test_golden_trees_on_gpu(lb, oracle):
     """The committed golden inputs: the GPU (quantised) tree must predict within 1e-4 of... itself
     via the oracle's Mode Q, and stay close to the reference CPU tree's training loss."""
