@@ -420,5 +420,10 @@ template <typename T>
 void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees,
                    const lbk_tree_ref* d_trees /* device */, int m_max /* nodes of the largest tree */, int64_t total_nodes,
                    const double* init, int transform, double* pred, int64_t ldp, cudaStream_t stream);
+// predict_ranked.cu: one output, more rows and trees than k_predict_tiled is better for.  False: the shape does not fit,
+// nothing was done.
+template <typename T>
+bool PredictRanked(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_t n_rows, int F, int n_trees, const lbk_tree_ref* d_trees, int S,
+                   int64_t total_nodes, const double* init, int transform, double* pred, int64_t ldp, cudaStream_t stream);
 
 }  // namespace lbk

@@ -33,8 +33,7 @@
 //   * Predictions are accumulated in float64 in tree order (bit-identical to the reference's
 //     tree-by-tree accumulation), transformed and written once.
 // A fallback kernel with the nodes in global memory covers shapes whose tile or trees do not fit.
-#include "device_utils.cuh"
-#include "internal.h"
+#include "predict.cuh"
 
 namespace lbk {
 namespace {
@@ -57,8 +56,6 @@ template <>
 struct NodeOf<float> {
   using type = Node8;
 };
-
-using TreePtrs = lbk_tree_ref;  // node_off: offset of the tree's first node in the packed arrays
 
 __device__ inline void MakeNode(Node8& n, double split, int foff)
 {
@@ -89,79 +86,6 @@ __global__ void k_pack_trees(const TreePtrs* __restrict__ trees, int K, int F, N
   for (int64_t i = threadIdx.x; i < static_cast<int64_t>(t.max_nodes) * K; i += blockDim.x)
     leaves[static_cast<int64_t>(t.node_off) * K + i] = t.leaf[i];
 }
-
-// Bulk asynchronous copy global -> shared (the copy engine moves whole lines; nothing passes
-// through the load/store pipe), completion counted in bytes on an mbarrier; a plain copy into this block only.
-__device__ inline void MbarInit(unsigned bar, unsigned count)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ inline void MbarExpectTx(unsigned bar, unsigned bytes)
-{
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ inline void BulkCopy(unsigned smem_dst, const void* gsrc, unsigned bytes, unsigned bar)
-{
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(smem_dst),
-               "l"(gsrc), "r"(bytes), "r"(bar)
-               : "memory");
-}
-__device__ inline bool MbarTryWait(unsigned bar, unsigned parity)
-{
-  unsigned ok;
-  asm volatile(
-    "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-    : "=r"(ok)
-    : "r"(bar), "r"(parity)
-    : "memory");
-  return ok != 0;
-}
-// Bounded wait: gives up after about a second, reports through the context's status word and lets the block finish instead
-// of spinning for ever.  A call with a table of trees has returned by then, so the producer warp makes the
-// block's predictions NaN: they are not taken for those of the trees that it did see.
-constexpr int kFaultPredictStaging = 21;
-__device__ inline bool MbarWait(unsigned bar, unsigned parity, int* status, int* failed)
-{
-  for (unsigned spin = 0; spin < (1u << 22); ++spin) {
-    if (MbarTryWait(bar, parity)) return true;
-    if (spin > 64) __nanosleep(256);
-  }
-  ReportFault(status, kFaultPredictStaging);
-  *failed = 1;
-  return false;
-}
-
-__device__ inline void MbarArrive(unsigned bar)
-{
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
-__device__ inline unsigned LdsU32(unsigned addr)
-{
-  unsigned v;
-  asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(addr));
-  return v;
-}
-__device__ inline float LdsX(unsigned addr, float)
-{
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(v) : "r"(addr));
-  return v;
-}
-__device__ inline double LdsX(unsigned addr, double)
-{
-  double v;
-  asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(v) : "r"(addr));
-  return v;
-}
-__device__ inline double LdsF64(unsigned addr)
-{
-  double v;
-  asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(v) : "r"(addr));
-  return v;
-}
-
-__device__ inline void MakeSplit(float& s, double split) { s = __double2float_rd(split); }
-__device__ inline void MakeSplit(double& s, double split) { s = split; }
 
 // A completed tree of depth S as the tiled kernel reads it.  Nodes are counted from 1: those of level l are
 // [2^l, 2^(l + 1)), the children of i are 2 i and 2 i + 1.  Splits [2^S] of T; words with the feature ids of a
@@ -234,36 +158,6 @@ __global__ void k_pack_complete(const TreePtrs* __restrict__ trees, int K, int F
 }
 
 // ---- few rows ---------------------------------------------------------------------------------
-// What is added to the sums and what becomes of them: initial prediction, then probabilities.
-struct PredictOut {
-  double* pred;
-  int64_t ldp;
-  const double* init;  // [K] or null
-  int transform;       // LBK_RAW, LBK_LOGISTIC (two columns: 1 - p, p) or LBK_SOFTMAX
-};
-
-// The K raw predictions of one row -> its row of the output.  `raw` and the row may be the same.
-__device__ inline void FinishRow(const double* raw, int stride, int K, double* out, int transform)
-{
-  if (transform == LBK_RAW) {
-    for (int k = 0; k < K; ++k) out[k] = raw[k * stride];
-  } else if (transform == LBK_LOGISTIC) {
-    const double p = 1.0 / (1.0 + exp(-raw[0]));
-    out[0] = 1.0 - p;
-    out[1] = p;
-  } else {
-    double top = raw[0];
-    for (int k = 1; k < K; ++k) top = fmax(top, raw[k * stride]);
-    double sum = 0.0;
-    for (int k = 0; k < K; ++k) {
-      const double e = exp(raw[k * stride] - top);
-      out[k]         = e;
-      sum += e;
-    }
-    for (int k = 0; k < K; ++k) out[k] = out[k] / sum;
-  }
-}
-
 // One launch that walks the trees where they lie: a block takes `rows_per_block` rows, its threads take
 // (row, tree) pairs, trees in neighbouring lanes, and leave what each walk adds in shared memory; the
 // sums are then made in tree order, one thread per (row, output).  Bound by the latency of one walk
@@ -714,6 +608,27 @@ void LaunchTiled(lbk_context* ctx, const TiledArgs<T>& a, const TilePlan& plan, 
   else LaunchTiledAs<T, TG, -1>(ctx, a, plan, stream);
 }
 
+// One output: is it worth finding the ranks of X first (predict_ranked.cu)?
+//
+// What it gives a million rows and tree, and what it costs them for the ranks, in microseconds; what is left pays for the
+// launches that make the tables (40 to 50) and the sorting of a feature's splits (40 per thousand).  Fitted to both
+// paths over 4 to 150 trees of depth 4 to 10 on 8 to 200 features, random splits.  A million rows, tiled and ranked: float32,
+// 100 features, 150 trees of depth 8 873 and 726 us (10M rows, 500 fitted trees: 19.3 and 13.5 ms), 25 trees of depth 4 202 and
+// 324, 64 features, 150 trees of depth 8 622 and 626; float64, 100 features, 150 trees of depth 8 1334 and 830, 10 of depth 4
+// 394 and 380, 30 features, 10 trees of depth 6 135 and 165.  Twenty thousand rows: 20 to 60 and 45 to 130.
+//
+// Not where one feature might have more splits than there are ranks and the average is not far from that either: the rows
+// would be walked through the caches.
+template <typename T>
+bool RankedPays(int64_t n_rows, int F, int K, int n_trees, int S)
+{
+  if (K != 1 || S < 3) return false;
+  const double millions = static_cast<double>(n_rows) * 1e-6, splits = static_cast<double>(n_trees) * ((1 << S) - 1);
+  if (splits > 32764.0 && splits > 8192.0 * F) return false;
+  const double gain = sizeof(T) == 4 ? n_trees * (0.2 * S - 0.6) - 0.7 * F : n_trees * (0.7 * S - 2.3) + 0.3 * F;
+  return millions * gain > (sizeof(T) == 4 ? 40.0 : 50.0) + 0.04 * splits / F;
+}
+
 }  // namespace
 
 template <typename T>
@@ -753,6 +668,9 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   // a walk through M heap-ordered nodes takes at most S = floor(log2(M)) steps
   int S = 0;
   while ((2 << S) <= m_max) ++S;
+  if (RankedPays<T>(n_rows, F, K, n_trees, S) &&
+      PredictRanked<T>(ctx, s, X, ldx, n_rows, F, n_trees, d_trees, S, total_nodes, init, transform, pred, ldp, stream))
+    return;
   const TilePlan plan = S <= 14 && F <= kMaxFeature ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
   if (plan.rb == 0) {
     NodeT* nodes   = s.alloc<NodeT>(total_nodes);

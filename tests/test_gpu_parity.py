@@ -453,6 +453,69 @@ def test_build_tree_level_batching(lb, oracle):
     assert np.array_equal(got["leaf_value"].cpu().numpy(), want.leaf_value)
 
 
+def _random_trees(rs, T, D, features, odd=False):
+    """Trees of depth <= D on the given features, splits around U(0, 1); with `odd` infinite and NaN ones too."""
+    trees = []
+    for _ in range(T):
+        M = 2 ** (D + 1) - 1
+        f = np.full(M, -1, np.int32)
+        f[: M // 2] = rs.choice(features, size=M // 2)
+        f[1: M // 2][rs.random(M // 2 - 1) < 0.1] = -1
+        for i in range(1, M // 2):
+            if f[(i - 1) // 2] < 0:
+                f[i] = -1
+        v = rs.random(M)
+        if odd:
+            at = rs.random(M)
+            v[at < 0.02], v[(at > 0.02) & (at < 0.03)], v[(at > 0.03) & (at < 0.04)] = np.inf, -np.inf, np.nan
+            v[at > 0.9] = np.round(v[at > 0.9] * 4) / 4
+        trees.append((dev(rs.normal(size=(M, 1))), dev(f), dev(v)))
+    return trees
+
+
+@pytest.mark.parametrize("N,F,T,D,dt,used,what", [
+    (1_000_001, 100, 130, 8, np.float32, None, "odd"),     # a last group of four features, a ragged last tile
+    (1_200_003, 33, 200, 5, np.float32, None, "odd"),    # a last group of one feature; several pieces of rows
+    (300_000, 64, 64, 8, np.float64, None, "odd"),
+    (1_200_001, 9, 70, 10, np.float64, None, "odd"),       # tables of a group in several turns
+    (4_000_000, 1, 60, 4, np.float64, None, ""),         # one feature
+    (300_000, 150, 50, 11, np.float64, None, ""),        # one tree per group
+    (400_000, 20, 100, 8, np.float64, [3], ""),          # all splits on one feature: sorted in chunks, no room for the table
+    (300_000, 20, 150, 8, np.float64, [3], "logistic"),  # ... more of them than there are ranks
+])
+def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what):
+    """Large ensembles of one output are walked on ranks (RankedPays says so for all of these); a few rows at a time, where
+    the trees are walked where they lie, give the same bits."""
+    from legateboost_b200 import library as L
+    from legateboost_b200.tree import TreeTable
+
+    rs = np.random.RandomState(N % 1000 + F)
+    X = rs.random((N, F)).astype(dt)
+    X[:, 0] = np.round(X[:, 0] * 4) / 4
+    if what == "odd":
+        for value in (np.nan, np.inf, -np.inf):
+            X[rs.randint(N, size=3000), rs.randint(F, size=3000)] = value
+        X[-40:] = np.nan
+    trees = _random_trees(rs, T, D, np.arange(F) if used is None else used, what == "odd")
+    table, transform = TreeTable(trees), L.LOGISTIC if what == "logistic" else L.RAW
+    init = dev(np.array([0.25])) if what else None
+    dX = dev(X)
+    got = table.predict(dX, 1, init=init, transform=transform, wait=True)
+    picks = [np.arange(5000), np.arange(N - 5000, N), np.sort(rs.choice(N, 8000, replace=False))]
+    for rows in picks:
+        rows = dev(rows)
+        few = table.predict(dX[rows].contiguous(), 1, init=init, transform=transform, wait=True)
+        assert torch.equal(got[rows], few)
+    if what == "":
+        few = picks[0][:500]
+        want = oracle.predict(X[few], [tuple(a.cpu().numpy() for a in t) for t in trees])
+        assert np.array_equal(got[few].cpu().numpy(), want)
+    # rows that lie apart in memory
+    wide = torch.zeros((N, F + 3), dtype=dX.dtype, device="cuda")
+    wide[:, 1: F + 1] = dX
+    assert torch.equal(table.predict(wide[:, 1: F + 1], 1, init=init, transform=transform, wait=True), got)
+
+
 @pytest.mark.parametrize("zeros", [False, True])
 @pytest.mark.parametrize("N,F,K,D", [(2500, 600, 2, 8), (2500, 600, 2, 10), (700, 1000, 1, 9)])
 def test_levels_outside_the_cache(lb, oracle, N, F, K, D, zeros):
