@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "abs_sum.cuh"
+#include "count_sort.cuh"
 #include "bin_grid.h"
 #include "internal.h"
 
@@ -47,11 +48,17 @@ __global__ void k_gather_samples(const __grid_constant__ PrologueArgs<T> p, T* _
   draft[static_cast<int64_t>(f) * p.S + i] = SampledValue(p, i, f);
 }
 
-// One block: the S samples of feature f sorted (bitonic), the distinct ones kept in cuts[f * S ..], the
-// last of them replaced by +inf.  Up to 256 samples a thread holds one of them and the 30 of the 36
-// exchange steps that stay inside a warp are shuffles.
+// Samples of a feature that are sorted by counting, beyond them by a bitonic network; and the shared memory of either.
+constexpr int kCountMax = 512;
 template <typename T>
-__device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals /* shared [S_pad] */, int* s_cnt /* shared [9] */)
+__host__ __device__ constexpr size_t SortSmem(int S_pad)
+{
+  return S_pad <= kCountMax ? (2 * sizeof(T) + sizeof(int)) * (S_pad < 4 ? 4 : S_pad) : sizeof(T) * S_pad;
+}
+
+// One block: the S samples of feature f sorted, the distinct ones kept in cuts[f * S ..], the last of them replaced by +inf.
+template <typename T>
+__device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals /* shared, SortSmem */, int* s_cnt /* shared [9] */)
 {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int S = p.S, S_pad = p.S_pad;
@@ -59,26 +66,36 @@ __device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals 
     if (i >= S) return static_cast<T>(INFINITY);
     return p.draft != nullptr ? p.draft[static_cast<int64_t>(f) * S + i] : SampledValue(p, i, f);
   };
-  if (S_pad <= kSortThreads) {
-    T v = sample(tid);
-    for (int k = 2; k <= S_pad; k <<= 1) {
-      const bool up = (tid & k) == 0;
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        T o;
-        if (j >= 32) {
-          __syncthreads();
-          if (tid < S_pad) vals[tid] = v;
-          __syncthreads();
-          o = tid < S_pad ? vals[tid ^ j] : v;
-        } else {
-          o = __shfl_xor_sync(0xffffffffu, v, j);
-        }
-        const bool lower = (tid & j) == 0;
-        if (lower == up ? o < v : v < o) v = o;
+  const int P     = S_pad < 4 ? 4 : S_pad;  // (whole 16-byte words)
+  T* sorted       = vals;
+  const int* mark = nullptr;  // counted: where there is a value
+  if (S_pad <= kCountMax) {
+    constexpr int kPer = kCountMax / kSortThreads;
+    sorted    = vals + P;
+    int* here = reinterpret_cast<int*>(sorted + P);
+    mark      = here;
+    T mine[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int i = tid + u * kSortThreads;
+      mine[u]     = sample(i);
+      if (mine[u] != mine[u]) mine[u] = static_cast<T>(INFINITY);
+      if (i < P) {
+        vals[i] = mine[u];
+        here[i] = 0;
       }
     }
     __syncthreads();
-    if (tid < S_pad) vals[tid] = v;
+    int below[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      below[u] = u == 0 || P > kSortThreads ? CountBelow(vals, P / static_cast<int>(16 / sizeof(T)), mine[u]) : 0;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      if (tid + u * kSortThreads < S) {
+        sorted[below[u]] = mine[u];
+        here[below[u]]   = 1;
+      }
     __syncthreads();
   } else {
     for (int i = tid; i < S_pad; i += kSortThreads) vals[i] = sample(i);
@@ -105,7 +122,7 @@ __device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals 
   int before = 0;
   for (int base = 0; base < S; base += kSortThreads) {
     const int i      = base + tid;
-    const bool keep  = i < S && (i == 0 || vals[i] != vals[i - 1]);
+    const bool keep  = i < S && (mark != nullptr ? mark[i] != 0 : i == 0 || vals[i] != vals[i - 1]);
     const unsigned m = __ballot_sync(0xffffffffu, keep);
     if (lane == 0) s_cnt[warp] = __popc(m);
     __syncthreads();
@@ -114,7 +131,7 @@ __device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals 
     int total = before;
     for (int w = 0; w < kSortThreads / 32; ++w) total += s_cnt[w];
     pos += __popc(m & ((1u << lane) - 1u));
-    if (keep) out[pos] = vals[i];
+    if (keep) out[pos] = sorted[i];
     before = total;
     __syncthreads();
   }
@@ -841,7 +858,7 @@ void Prologue(lbk_context* ctx, Scratch& s, PrologueArgs<T> p, int32_t* row_ptr,
   p.fill_blocks = static_cast<int>(std::min<int64_t>((fill + 4 * kSortThreads - 1) / (4 * kSortThreads), ctx->sm_count * 4));
   const int64_t blocks = p.sort_blocks + p.sum_blocks + p.fill_blocks;
   if (blocks > 0) {
-    k_prologue<T><<<static_cast<unsigned>(blocks), kSortThreads, sizeof(T) * p.S_pad, stream>>>(p);
+    k_prologue<T><<<static_cast<unsigned>(blocks), kSortThreads, SortSmem<T>(p.S_pad), stream>>>(p);
     LBK_LAUNCH_CHECK();
   }
   const bool one_rank = ctx->n_ranks <= 1;

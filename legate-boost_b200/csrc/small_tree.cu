@@ -24,13 +24,17 @@
 // 32-bit shared-memory sums are exact here without a bound on the magnitudes: a quantised value is added as
 // its high and its low 16 bits, whose sums over at most 65536 rows fit 32 bits.
 //
-// What bounds it: the chain of latencies of a level - pass over the rows, scan, float64 divisions, barrier,
-// candidates, move: 8 - 9 us each, of which the barrier is one, and about 10 us for everything before the root.
-// A thread per bin: with a warp per node (four bins per lane) a level of 500 x 10 took 9 us longer, because a
-// lone warp gets an instruction in about five clocks.  500 x 10, depth 4: 49 us per tree (260 us of kernels in
-// 70 launches, 570 us of wall time before); 712 x 128, 3 classes, depth 8, 7 rounds: 9.15 -> 3.9 ms.
+// What bounds it: the chain of latencies of a level - pass over the rows 1.2 us, scan, float64 divisions and candidates 2.5,
+// barrier 1 to 2, winners and move 1.5 - and about 8 us for everything before the root.  Where a block has one or two pairs of
+// nodes a thread takes a bin; with a warp per node (four bins per lane) a level of 500 x 10 took 9 us longer, because a lone
+// warp gets an instruction in about five clocks.  Deeper levels have a warp per pair: the chain, most of it waiting, came
+// once for every two pairs before.  500 x 10, depth 4: 39 us per tree (260 us of kernels in 70 launches before
+// there was this form).  Five rounds, a thread per bin on all levels, proposals sorted by a bitonic network (3.3 us), the four
+// divisions of a pair of nodes one after the other, and this: 500 x 10, depth 4: 482 -> 433 us; 2000 x 30, depth 8 1122 -> 851;
+// 4000 x 64, depth 10 4211 -> 2392; 15000 x 100, depth 8 2872 -> 1965.
 
 #include "abs_sum.cuh"
+#include "count_sort.cuh"
 #include "internal.h"
 #include "objective.cuh"
 #include "small_layout.h"
@@ -44,17 +48,18 @@ constexpr int kSmallWarps       = kSmallThreads / 32;
 constexpr int kSmallBins        = 256;
 constexpr int kFaultGridBarrier = 51;  // status word: a block did not reach the barrier
 
-struct SmallCand {
+struct alignas(16) SmallCand {
   double gain;
   int bin;  // of the feature
   int pad;
+  GPairI64 left;  // the sums left of it (one output)
 };
 
 template <typename T>
 struct SmallParams {
   const T* X;
   int64_t ldx;
-  int N, F, K, D, S, S_pad, seed;
+  int N, F, K, D, S, seed;
   int parts, part_shift;  // blocks per feature: a power of two
   int64_t row_offset, dataset_rows;
   // gradients: given (objective < 0), or made from the current prediction
@@ -79,7 +84,7 @@ struct SmallParams {
   GPairI64* root_part; // [blocks][K]
   GPairI64* hist[2];   // levels alternate: [F][nodes of the level][K][256]
   SmallCand* cand;     // levels alternate (SmallCandBegin): [nodes of the level][F]
-  GPairI64* cand_left; // likewise, [nodes of the level][F][K]
+  GPairI64* cand_left; // several outputs: likewise, [nodes of the level][F][K]
   int max_slots;       // histograms in shared memory at a time
   unsigned int* barrier;  // zero at the start
   int* status;
@@ -127,20 +132,21 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   __shared__ double s_sum[2][2 * kSumThreads / 32];
   __shared__ QuantParams s_qp;
   __shared__ GPairI64 s_tot[2][kSmallWarps / 2];
-  __shared__ Cand s_best[2][2][kSmallWarps / 2];
+  __shared__ SmallCand s_best[2][2][kSmallWarps / 2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int N = p.N, F = p.F, K = p.K, D = p.D, S = p.S;
   const int n_blocks = gridDim.x, block = blockIdx.x;
   const int part     = block % p.parts;            // of the feature's rows (binning) and node pairs (levels)
   const int f_first = block / p.parts, f_step = n_blocks / p.parts;
   const int n_sums  = max(1, (1 << max(D - 1, 0)) * K);  // node sums of a level
-  // shared memory: histograms | node sums of two levels | candidate gains (several outputs) | row_ptr | winners |
+  // shared memory: histograms | candidate gains (several outputs) | node sums of two levels, terms | row_ptr | winners |
   // node of every row
   int* s_hist         = reinterpret_cast<int*>(smem_raw);  // [slot][4][256]: g high, g low, h high, h low
   double* s_gain      = reinterpret_cast<double*>(s_hist + p.max_slots * 4 * kSmallBins);
   GPairI64* s_nodes   = reinterpret_cast<GPairI64*>(s_gain + (K > 1 ? p.max_slots * 2 * kSmallBins : 0));
   GPairI64* s_next    = s_nodes + n_sums;
-  int* s_rp           = reinterpret_cast<int*>(s_next + n_sums);  // [F + 1]
+  NodeTerms* s_terms  = reinterpret_cast<NodeTerms*>(s_next + n_sums);  // of the level's nodes
+  int* s_rp           = reinterpret_cast<int*>(s_terms + n_sums);       // [F + 1]
   int* s_wfeat        = s_rp + F + 1;                             // [nodes of a level], -1: no split / no node
   int* s_wbin         = s_wfeat + (1 << max(D - 1, 0));
   T* s_cuts           = reinterpret_cast<T*>(s_hist);  // (before the levels) [256]
@@ -157,28 +163,31 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       const long long row = eng.uniform_int(0, p.dataset_rows - 1) - p.row_offset;
       v = row >= 0 && row < N ? p.X[row * p.ldx + f] : T(0);
     }
-    for (int k = 2; k <= p.S_pad; k <<= 1) {
-      const bool up = (tid & k) == 0;
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        T o;
-        if (j >= 32) {
-          __syncthreads();
-          if (tid < p.S_pad) s_cuts[tid] = v;
-          __syncthreads();
-          o = tid < p.S_pad ? s_cuts[tid ^ j] : v;
-        } else {
-          o = __shfl_xor_sync(0xffffffffu, v, j);
-        }
-        const bool lower = (tid & j) == 0;
-        if (lower == up ? o < v : v < o) v = o;
+    // sorted by counting, two threads per value
+    __syncthreads();
+    T* s_sorted = s_cuts + kSmallBins;                              // [256]
+    int* s_mark = reinterpret_cast<int*>(s_sorted + kSmallBins);    // [256]
+    if (tid < kSmallBins) {
+      s_cuts[tid] = v == v ? v : static_cast<T>(INFINITY);
+      s_mark[tid] = 0;
+    }
+    __syncthreads();
+    {
+      const T mine     = s_cuts[tid >> 1];
+      constexpr int kPer = 16 / sizeof(T);
+      const int n_vec  = (S + 2 * kPer - 1) / (2 * kPer);  // 16-byte words of a half
+      int below        = CountBelow(s_cuts + (tid & 1) * n_vec * kPer, n_vec, mine);
+      below += __shfl_xor_sync(0xffffffffu, below, 1);
+      if ((tid & 1) == 0 && (tid >> 1) < S) {
+        s_sorted[below] = mine;
+        s_mark[below]   = 1;
       }
     }
     __syncthreads();
-    if (tid < p.S_pad) s_cuts[tid] = v;
-    __syncthreads();
-    const bool keep  = tid < S && (tid == 0 || v != s_cuts[tid - 1]);
+    const bool keep  = tid < S && s_mark[tid] != 0;
     const unsigned m = __ballot_sync(0xffffffffu, keep);
     if (lane == 0) s_cnt[warp] = __popc(m);
+    if (keep) v = s_sorted[tid];
     __syncthreads();
     int pos = __popc(m & ((1u << lane) - 1u)), count = 0;
     for (int w = 0; w < kSmallWarps; ++w) {
@@ -362,6 +371,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     const int units = derive ? nodes / 2 : 1;
     SmallCand* cand     = p.cand + static_cast<int64_t>(SmallCandBegin(depth, D)) * F;
     GPairI64* cand_left = p.cand_left + static_cast<int64_t>(SmallCandBegin(depth, D)) * F * K;
+    // (read behind the next barrier of the block)
+    for (int i = tid; i < nodes * K; i += kSmallThreads) s_terms[i] = TermsOf(s_nodes[i], qp, l1, reg);
     // (s_wfeat still holds the winners of the level above: unit u exists if node u there was split)
     for (int f = f_first; f < F; f += f_step) {
       const bool search = p.feature_set == nullptr || p.feature_set[f] != 0;
@@ -410,25 +421,44 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
             }
           }
           __syncthreads();
-          // scan, sibling, gains: a thread per bin, two units at a time
-          for (int i0 = 0; i0 < slots; i0 += 2) {
+          // What a unit's scan needs of it.  _a: the built node, _b: its sibling.
+          struct Unit {
+            bool here, scanned, eval_a, eval_b;
+            int ja, jb, u;
+          };
+          auto unit_of = [&](int i) {
+            Unit n;
+            n.u             = part + (c0 + i) * p.parts;
+            n.here          = i < slots && (!derive || s_wfeat[n.u] >= 0);  // node u of the level above was split
+            const bool left = n.here && derive && s_nodes[static_cast<int64_t>(2 * n.u) * K].hess < s_nodes[static_cast<int64_t>(2 * n.u + 1) * K].hess;
+            n.ja            = n.here && derive ? 2 * n.u + (left ? 0 : 1) : 0;
+            n.jb            = n.here && derive ? 2 * n.u + (left ? 1 : 0) : 0;
+            n.eval_a        = n.here && search && s_nodes[static_cast<int64_t>(n.ja) * K].hess > 0;
+            n.eval_b        = n.here && search && derive && s_nodes[static_cast<int64_t>(n.jb) * K].hess > 0;
+            n.scanned       = s_nodes[static_cast<int64_t>(n.ja) * K + k].hess > 0;
+            return n;
+          };
+          // The candidate of node j, by the lanes of a warp: `best` is the same in all of them.
+          auto write_cand = [&](int j, const SmallCand& best) {
+            const int64_t at = static_cast<int64_t>(j) * F + f;
+            if (lane == 0) cand[at] = best;
+            if (K > 1 && best.bin >= 0)  // (written by threads of this block, before the barrier)
+              for (int kk = lane; kk < K; kk += 32)
+                StorePair(cand_left + at * K + kk, LoadPairStreaming(hist_f + (static_cast<int64_t>(j) * K + kk) * kSmallBins + best.bin));
+          };
+          if (slots <= 2) {
+            // a thread per bin, both units at a time
             const int grp = tid / kSmallBins, b = tid % kSmallBins, gw = warp % (kSmallWarps / 2);
-            const int i   = i0 + grp;
-            const int u   = part + (c0 + i) * p.parts;
-            const bool here = i < slots && (!derive || s_wfeat[u] >= 0);  // node u of the level above was split
-            const bool left = here && derive && s_nodes[static_cast<int64_t>(2 * u) * K].hess < s_nodes[static_cast<int64_t>(2 * u + 1) * K].hess;
-            const int ja    = here && derive ? 2 * u + (left ? 0 : 1) : 0, jb = here && derive ? 2 * u + (left ? 1 : 0) : 0;
-            const bool eval_a = here && search && s_nodes[static_cast<int64_t>(ja) * K].hess > 0;
-            const bool eval_b = here && search && derive && s_nodes[static_cast<int64_t>(jb) * K].hess > 0;
-            const GPairI64 sum_a = s_nodes[static_cast<int64_t>(ja) * K + k], sum_b = s_nodes[static_cast<int64_t>(jb) * K + k];
-            const bool scanned = sum_a.hess > 0, in = here && b < nb;
-            const int64_t at_a = (static_cast<int64_t>(ja) * K + k) * kSmallBins + b, at_b = (static_cast<int64_t>(jb) * K + k) * kSmallBins + b;
+            const int i   = grp;
+            const Unit n  = unit_of(i);
+            const bool in = n.here && b < nb;
+            const int64_t at_a = (static_cast<int64_t>(n.ja) * K + k) * kSmallBins + b, at_b = (static_cast<int64_t>(n.jb) * K + k) * kSmallBins + b;
             const int* hs      = s_hist + i * 4 * kSmallBins;
             double* gains      = s_gain + i * 2 * kSmallBins;
             GPairI64 va{0, 0}, vb{0, 0};
             double ga = 0.0, gb = 0.0;
             if (in) {
-              if (derive && scanned) vb = LoadPairStreaming(par_f + (static_cast<int64_t>(u) * K + k) * kSmallBins + b);
+              if (derive && n.scanned) vb = LoadPairStreaming(par_f + (static_cast<int64_t>(n.u) * K + k) * kSmallBins + b);
               va.grad = static_cast<long long>(hs[b]) * 65536 + static_cast<unsigned>(hs[kSmallBins + b]);
               va.hess = static_cast<long long>(hs[2 * kSmallBins + b]) * 65536 + static_cast<unsigned>(hs[3 * kSmallBins + b]);
             }
@@ -453,55 +483,131 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
               }
             }
             if (in) {
-              if (scanned && (sg > 0 || sh > 0)) va = GPairI64{sg, sh};
-              vb = scanned && derive ? GPairI64{vb.grad - va.grad, vb.hess - va.hess} : GPairI64{0, 0};
+              if (n.scanned && (sg > 0 || sh > 0)) va = GPairI64{sg, sh};
+              vb = n.scanned && derive ? GPairI64{vb.grad - va.grad, vb.hess - va.hess} : GPairI64{0, 0};
               if (write_hist || K > 1) {
                 StorePair(hist_f + at_a, va);
                 if (derive) StorePair(hist_f + at_b, vb);
               }
             }
-            unsigned ok_a = eval_a && in ? 1u : 0u, ok_b = eval_b && in ? 1u : 0u;
+            unsigned ok_a = n.eval_a && in ? 1u : 0u, ok_b = n.eval_b && in ? 1u : 0u;
             if (K > 1 && in) {  // the gains so far are in shared memory, -1e300 = a side without hessian
               ga = gains[b];
               gb = gains[kSmallBins + b];
               if (ga < -1e299) ok_a = 0u;
               if (gb < -1e299) ok_b = 0u;
             }
-            if (__any_sync(0xffffffffu, ok_a)) ok_a = AddGain(va, ok_a, TermsOf(sum_a, qp, l1, reg), qp, l1, reg, msg, ga);
-            if (__any_sync(0xffffffffu, ok_b)) ok_b = AddGain(vb, ok_b, TermsOf(sum_b, qp, l1, reg), qp, l1, reg, msg, gb);
+            if (__any_sync(0xffffffffu, ok_a | ok_b))
+              AddGains(va, ok_a, s_terms[static_cast<int64_t>(n.ja) * K + k], ga, vb, ok_b, s_terms[static_cast<int64_t>(n.jb) * K + k], gb, qp, l1, reg, msg);
             if (k < K - 1) {
               if (in) {
                 gains[b]              = ok_a ? ga : -1e300;
                 gains[kSmallBins + b] = ok_b ? gb : -1e300;
               }
-              __syncthreads();  // s_tot is written again
-              continue;
+            } else {
+              // the best bin of either node: of the warp, then of the unit's eight warps
+              const double gain_a = ok_a && ga > 0 ? ga : 0.0, gain_b = ok_b && gb > 0 ? gb : 0.0;
+              const int bin_a = WarpBest(gain_a, s_rp[f] + b), bin_b = derive ? WarpBest(gain_b, s_rp[f] + b) : -1;
+              if (bin_a < 0 ? lane == 0 : bin_a == s_rp[f] + b) s_best[grp][0][gw] = SmallCand{gain_a, bin_a < 0 ? -1 : b, 0, va};
+              if (bin_b < 0 ? lane == 0 : bin_b == s_rp[f] + b) s_best[grp][1][gw] = SmallCand{gain_b, bin_b < 0 ? -1 : b, 0, vb};
+              __syncthreads();
+              if (n.here && gw < (derive ? 2 : 1)) {  // a warp per node
+                const SmallCand mine = s_best[grp][gw][lane % (kSmallWarps / 2)];
+                const int best       = WarpBest(lane < kSmallWarps / 2 && mine.bin >= 0 ? mine.gain : 0.0, s_rp[f] + mine.bin);
+                const int from       = best < 0 ? 0 : (best - s_rp[f]) / 32;  // the warp that has the bin
+                write_cand(gw == 0 ? n.ja : n.jb, s_best[grp][gw][from]);
+              }
             }
-            // the best bin of either node: of the warp, then of the unit's eight warps
-            const double gain_a = ok_a && ga > 0 ? ga : 0.0, gain_b = ok_b && gb > 0 ? gb : 0.0;
-            const int bin_a = WarpBest(gain_a, s_rp[f] + b), bin_b = derive ? WarpBest(gain_b, s_rp[f] + b) : -1;
-            if (bin_a < 0 ? lane == 0 : bin_a == s_rp[f] + b) s_best[grp][0][gw] = Cand{gain_a, bin_a, b};
-            if (bin_b < 0 ? lane == 0 : bin_b == s_rp[f] + b) s_best[grp][1][gw] = Cand{gain_b, bin_b, b};
-            __syncthreads();
-            if (here) {
+          } else {
+            // A warp per unit.  The four words of the bins become their prefix sums where they lie (at most sums of all rows, which
+            // fit 32 bits): a lane adds up eight neighbouring bins; then the lanes take the bins 32 at a time.
+            for (int i = warp; i < slots; i += kSmallWarps) {
+              const Unit n = unit_of(i);
+              if (!n.here) continue;
+              int* hs = s_hist + i * 4 * kSmallBins;
+#pragma unroll
+              for (int word = 0; word < 4; ++word) {
+                int4* at = reinterpret_cast<int4*>(hs + word * kSmallBins) + 2 * lane;
+                int4 x = at[0], y = at[1];
+                x.y += x.x;
+                x.z += x.y;
+                x.w += x.z;
+                y.x += x.w;
+                y.y += y.x;
+                y.z += y.y;
+                y.w += y.z;
+                int incl = y.w;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                  const int v = __shfl_up_sync(0xffffffffu, incl, off);
+                  if (lane >= off) incl += v;
+                }
+                const int before = incl - y.w;
+                at[0]     = make_int4(x.x + before, x.y + before, x.z + before, x.w + before);
+                at[1]     = make_int4(y.x + before, y.y + before, y.z + before, y.w + before);
+              }
+              __syncwarp();
+              const NodeTerms ta = s_terms[static_cast<int64_t>(n.ja) * K + k], tb = s_terms[static_cast<int64_t>(n.jb) * K + k];
+              double* gains      = s_gain + i * 2 * kSmallBins;
+              auto prefix        = [&](int b) {
+                return GPairI64{static_cast<long long>(hs[b]) * 65536 + static_cast<unsigned>(hs[kSmallBins + b]),
+                                static_cast<long long>(hs[2 * kSmallBins + b]) * 65536 + static_cast<unsigned>(hs[3 * kSmallBins + b])};
+              };
+              SmallCand best_a{0.0, -1, 0, GPairI64{0, 0}}, best_b = best_a;
+              auto parent_of = [&](int b) {
+                return derive && n.scanned && b < nb ? LoadPairStreaming(par_f + (static_cast<int64_t>(n.u) * K + k) * kSmallBins + b) : GPairI64{0, 0};
+              };
+              GPairI64 ahead = parent_of(lane);
+              for (int b0 = 0; b0 < nb; b0 += 32) {
+                const int b   = b0 + lane;
+                const bool in = b < nb;
+                GPairI64 va = prefix(b), vb = ahead;
+                ahead = parent_of(b + 32);
+                if (!(n.scanned && (va.grad > 0 || va.hess > 0)) && b > 0) {  // the bin itself
+                  const GPairI64 before = prefix(b - 1);
+                  va = GPairI64{va.grad - before.grad, va.hess - before.hess};
+                }
+                vb = n.scanned && derive ? GPairI64{vb.grad - va.grad, vb.hess - va.hess} : GPairI64{0, 0};
+                if (in && (write_hist || K > 1)) {
+                  StorePair(hist_f + (static_cast<int64_t>(n.ja) * K + k) * kSmallBins + b, va);
+                  if (derive) StorePair(hist_f + (static_cast<int64_t>(n.jb) * K + k) * kSmallBins + b, vb);
+                }
+                unsigned ok_a = n.eval_a && in ? 1u : 0u, ok_b = n.eval_b && in ? 1u : 0u;
+                double ga = 0.0, gb = 0.0;
+                if (K > 1) {
+                  ga = gains[b];
+                  gb = gains[kSmallBins + b];
+                  if (ga < -1e299) ok_a = 0u;
+                  if (gb < -1e299) ok_b = 0u;
+                }
+                if (__any_sync(0xffffffffu, ok_a | ok_b)) AddGains(va, ok_a, ta, ga, vb, ok_b, tb, gb, qp, l1, reg, msg);
+                if (k < K - 1) {
+                  if (in) {
+                    gains[b]              = ok_a ? ga : -1e300;
+                    gains[kSmallBins + b] = ok_b ? gb : -1e300;
+                  }
+                  continue;
+                }
+                auto better = [&](double gain, const SmallCand& best) {
+                  return gain > 0 && Better(Cand{gain, s_rp[f] + b, f}, Cand{best.gain, best.bin < 0 ? -1 : s_rp[f] + best.bin, f});
+                };
+                if (ok_a && better(ga, best_a)) best_a = SmallCand{ga, b, 0, va};
+                if (ok_b && better(gb, best_b)) best_b = SmallCand{gb, b, 0, vb};
+              }
+              if (k < K - 1) continue;
+              __syncwarp();  // (the level's histogram is read again with several outputs)
 #pragma unroll
               for (int side = 0; side < 2; ++side) {
                 if (side == 1 && !derive) continue;
-                Cand best = s_best[grp][side][0];
-#pragma unroll
-                for (int w = 1; w < kSmallWarps / 2; ++w)
-                  if (Better(s_best[grp][side][w], best)) best = s_best[grp][side][w];
-                const int j      = side == 0 ? ja : jb;
-                const int64_t at = static_cast<int64_t>(j) * F + f;
-                if (b == 0) cand[at] = SmallCand{best.gain, best.bin < 0 ? -1 : best.feature, 0};  // (feature: the bin of the feature)
-                if (K == 1) {
-                  if (best.bin >= 0 && b == best.feature) StorePair(cand_left + at, side == 0 ? va : vb);
-                } else if (best.bin >= 0) {
-                  // (written by threads of this block, before the barrier)
-                  for (int kk = b; kk < K; kk += kSmallBins)
-                    StorePair(cand_left + at * K + kk,
-                              LoadPairStreaming(hist_f + (static_cast<int64_t>(j) * K + kk) * kSmallBins + best.feature));
-                }
+                SmallCand best  = side == 0 ? best_a : best_b;
+                const int bin   = WarpBest(best.bin >= 0 ? best.gain : 0.0, s_rp[f] + best.bin);
+                const unsigned holder = __ballot_sync(0xffffffffu, bin >= 0 && best.bin >= 0 && s_rp[f] + best.bin == bin);
+                const int from        = holder != 0u ? __ffs(holder) - 1 : 0;
+                best.gain      = bin < 0 ? 0.0 : __shfl_sync(0xffffffffu, best.gain, from);
+                best.left.grad = __shfl_sync(0xffffffffu, best.left.grad, from);
+                best.left.hess = __shfl_sync(0xffffffffu, best.left.hess, from);
+                best.bin       = bin < 0 ? -1 : bin - s_rp[f];
+                write_cand(side == 0 ? n.ja : n.jb, best);
               }
             }
           }
@@ -515,51 +621,23 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     // ---- winners of the level: a warp per node picks, the next node's candidates already on their way
     const int words = derive ? nodes : 1;
     auto exists = [&](int j) { return j < words && (!derive || s_wfeat[j >> 1] >= 0) && s_nodes[static_cast<int64_t>(j) * K].hess > 0; };
-    auto first_cand = [&](int j) {
-      return exists(j) && lane < F ? __ldcg(reinterpret_cast<const int4*>(cand + static_cast<int64_t>(j) * F + lane)) : make_int4(0, 0, -1, 0);
+    auto cand_of = [&](int j, int f) {
+      SmallCand c{0.0, -1, 0, GPairI64{0, 0}};
+      if (exists(j) && f < F) {
+        const int4* at = reinterpret_cast<const int4*>(cand + static_cast<int64_t>(j) * F + f);
+        const int4 raw = __ldcg(at);
+        if (K == 1) c.left = LoadPairStreaming(reinterpret_cast<const GPairI64*>(at + 1));
+        c.gain = __hiloint2double(raw.y, raw.x);
+        c.bin  = raw.z;
+      }
+      return c;
     };
-    int4 ahead = first_cand(warp);
-    for (int j = warp; j < words; j += kSmallWarps) {
-      const bool here = exists(j);
-      Cand best{0.0, -1, -1};
-      int4 raw = ahead;
-      ahead    = first_cand(j + kSmallWarps);
-      if (here) {
-        for (int f = lane; f < F; f += 32) {
-          if (f >= 32) raw = __ldcg(reinterpret_cast<const int4*>(cand + static_cast<int64_t>(j) * F + f));
-          if (raw.z < 0) continue;
-          const Cand c{__hiloint2double(raw.y, raw.x), s_rp[f] + raw.z, f};
-          if (Better(c, best)) best = c;
-        }
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) {
-          Cand o;
-          o.gain    = __shfl_xor_sync(0xffffffffu, best.gain, off);
-          o.bin     = __shfl_xor_sync(0xffffffffu, best.bin, off);
-          o.feature = __shfl_xor_sync(0xffffffffu, best.feature, off);
-          if (Better(o, best)) best = o;
-        }
-      }
-      if (lane == 0) {
-        const bool split = best.gain > 1e-5;
-        const int b      = split ? best.bin - s_rp[best.feature] : -1;
-        s_wbin[j]        = b;
-        s_wnew[j]        = split ? best.feature : -1;
-        if (split && block == 0) {
-          p.tree.feature[begin + j]     = best.feature;
-          p.tree.split_value[begin + j] = static_cast<double>(p.cuts[static_cast<int64_t>(best.feature) * S + b]);
-          p.tree.gain[begin + j]        = best.gain;
-        }
-      }
-    }
-    __syncthreads();
-    // ... and the sums of their children
-    for (int i = tid; i < words * K; i += kSmallThreads) {
-      const int j = i / K, k = i - j * K, wf = s_wnew[j];
+    // the sums of the children of node j
+    auto set_children = [&](int j, int k, bool split, const GPairI64& left) {
       GPairI64 ls{0, 0}, rs{0, 0};
-      if (wf >= 0) {
-        ls                = LoadPairStreaming(cand_left + (static_cast<int64_t>(j) * F + wf) * K + k);
-        const GPairI64 ns = s_nodes[i];
+      if (split) {
+        const GPairI64 ns = s_nodes[static_cast<int64_t>(j) * K + k];
+        ls                = left;
         rs                = GPairI64{ns.grad - ls.grad, ns.hess - ls.hess};
         if (block == 0) {
           const int node = begin + j;
@@ -570,6 +648,41 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       if (depth < D - 1) {
         s_next[static_cast<int64_t>(2 * j) * K + k]     = ls;
         s_next[static_cast<int64_t>(2 * j + 1) * K + k] = rs;
+      }
+    };
+    SmallCand ahead = cand_of(warp, lane);
+    for (int j = warp; j < words; j += kSmallWarps) {
+      SmallCand mine = ahead;
+      int feature    = lane;
+      ahead          = cand_of(j + kSmallWarps, lane);
+      for (int f = lane + 32; f < F; f += 32) {
+        const SmallCand c = cand_of(j, f);
+        if (c.bin >= 0 && (mine.bin < 0 || Better(Cand{c.gain, s_rp[f] + c.bin, f}, Cand{mine.gain, s_rp[feature] + mine.bin, feature}))) {
+          mine    = c;
+          feature = f;
+        }
+      }
+      const int own = mine.bin >= 0 ? s_rp[feature] + mine.bin : -1;
+      const int bin = WarpBest(mine.bin >= 0 ? mine.gain : 0.0, own);
+      const unsigned holder = __ballot_sync(0xffffffffu, bin >= 0 && own == bin);
+      const int from        = holder != 0u ? __ffs(holder) - 1 : 0;
+      const bool split      = bin >= 0 && __shfl_sync(0xffffffffu, mine.gain, from) > 1e-5;
+      if (lane == from) {
+        s_wbin[j] = split ? mine.bin : -1;
+        s_wnew[j] = split ? feature : -1;
+        if (K == 1) set_children(j, 0, split, mine.left);
+        if (split && block == 0) {
+          p.tree.feature[begin + j]     = feature;
+          p.tree.split_value[begin + j] = static_cast<double>(p.cuts[static_cast<int64_t>(feature) * S + mine.bin]);
+          p.tree.gain[begin + j]        = mine.gain;
+        }
+      }
+    }
+    __syncthreads();
+    if (K > 1) {
+      for (int i = tid; i < words * K; i += kSmallThreads) {
+        const int j = i / K, k = i - j * K, wf = s_wnew[j];
+        set_children(j, k, wf >= 0, wf >= 0 ? LoadPairStreaming(cand_left + (static_cast<int64_t>(j) * F + wf) * K + k) : GPairI64{0, 0});
       }
     }
     for (int j = tid; j < words; j += kSmallThreads) s_wfeat[j] = s_wnew[j];
@@ -640,14 +753,16 @@ static bool PlanSmall(lbk_context* ctx, int64_t N, int F, int K, int D, int S, S
   plan.parts  = static_cast<int>(std::min<int64_t>(std::max(1, ctx->sm_count / F), std::max<int64_t>({level / 2, N / 2048, 1})));
   while (plan.parts & (plan.parts - 1)) plan.parts &= plan.parts - 1;  // a power of two
   plan.blocks = F <= ctx->sm_count ? F * plan.parts : ctx->sm_count;
-  const size_t fixed = 2 * sizeof(GPairI64) * std::max<int64_t>(1, level * K) + sizeof(int) * (F + 1 + 3 * level) + 2 * N + 64;
+  const size_t fixed = (2 * sizeof(GPairI64) + sizeof(NodeTerms)) * std::max<int64_t>(1, level * K) + sizeof(int) * (F + 1 + 3 * level) + 2 * N + 64;
   const size_t slot  = 4 * kSmallBins * sizeof(int) + (K > 1 ? 2 * kSmallBins * sizeof(double) : 0);
   const size_t room  = static_cast<size_t>(ctx->max_smem_optin) - 4096;
   if (fixed + slot > room) return false;
   const int64_t units = std::max<int64_t>(1, level / 2);
   plan.max_slots      = static_cast<int>(std::min<int64_t>((units + plan.parts - 1) / plan.parts, (room - fixed) / slot));
   plan.max_slots      = std::max(plan.max_slots, 1);
-  plan.smem           = fixed + plan.max_slots * slot;
+  if (plan.max_slots > kSmallWarps) plan.max_slots = plan.max_slots / kSmallWarps * kSmallWarps;  // (a warp per unit: whole turns)
+  // (the proposals, three arrays of kSmallBins, begin where the histograms do and may reach beyond them)
+  plan.smem = std::max(fixed + plan.max_slots * slot, kSmallBins * size_t{2 * 8 + 4});
   // (the partial sums, the proposals and the root sums share the histograms' place)
   const size_t early = std::max({size_t{2} * ((N * K + kSumBlock - 1) / kSumBlock) * 8, kSmallBins * size_t{8}, size_t{16} * K});
   if (early > plan.max_slots * slot) return false;
@@ -675,8 +790,6 @@ void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStre
   p.K = K;
   p.D = D;
   p.S = a.S;
-  p.S_pad = 1;
-  while (p.S_pad < a.S) p.S_pad *= 2;
   p.seed = a.seed;
   p.parts = plan.parts;
   while ((2 << p.part_shift) <= p.parts) ++p.part_shift;
@@ -709,7 +822,7 @@ void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStre
   p.hist[last & 1]       = s.alloc<GPairI64>(static_cast<size_t>(F) * top * K * kSmallBins);
   p.hist[(last & 1) ^ 1] = s.alloc<GPairI64>(static_cast<size_t>(F) * below * K * kSmallBins);
   p.cand      = s.alloc<SmallCand>(static_cast<size_t>(SmallCandNodes(D)) * F);
-  p.cand_left = s.alloc<GPairI64>(static_cast<size_t>(SmallCandNodes(D)) * F * K);
+  p.cand_left = K > 1 ? s.alloc<GPairI64>(static_cast<size_t>(SmallCandNodes(D)) * F * K) : nullptr;
   p.max_slots = plan.max_slots;
   p.status    = ctx->d_status;
   p.info_host = a.info_host;

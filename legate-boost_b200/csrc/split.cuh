@@ -91,6 +91,38 @@ __device__ inline unsigned AddGain(const GPairI64& left, unsigned ok, const Node
   return ok;
 }
 
+// The same for a node and its sibling: the four divisions of a lane are under way together (one after the other's vote they
+// take twice as long, and a lone chain is what small levels wait for).
+__device__ inline void AddGains(const GPairI64& left_a, unsigned& ok_a, const NodeTerms& a, double& gain_a, const GPairI64& left_b, unsigned& ok_b,
+                                const NodeTerms& b, double& gain_b, const QuantParams& qp, double l1, double reg, double msg)
+{
+  const double alg = WholeToDouble(left_a.grad), alh = WholeToDouble(left_a.hess), arg = a.g - alg, arh = a.h - alh;
+  const double blg = WholeToDouble(left_b.grad), blh = WholeToDouble(left_b.hess), brg = b.g - blg, brh = b.h - blh;
+  if (alh <= 0.0 || arh <= 0.0) ok_a = 0u;
+  if (blh <= 0.0 || brh <= 0.0) ok_b = 0u;
+  double n0 = LeafNumerator(alg * qp.inv_g, l1), n1 = LeafNumerator(arg * qp.inv_g, l1);
+  double n2 = LeafNumerator(blg * qp.inv_g, l1), n3 = LeafNumerator(brg * qp.inv_g, l1);
+  const double d0 = alh * qp.inv_h + reg, d1 = arh * qp.inv_h + reg, d2 = blh * qp.inv_h + reg, d3 = brh * qp.inv_h + reg;
+  if (__all_sync(0xffffffffu, (ok_a == 0u || (DivisionIsPlain(n0, d0) && DivisionIsPlain(n1, d1))) &&
+                                (ok_b == 0u || (DivisionIsPlain(n2, d2) && DivisionIsPlain(n3, d3))))) {
+    n0 = DividePlain(n0, d0);
+    n1 = DividePlain(n1, d1);
+    n2 = DividePlain(n2, d2);
+    n3 = DividePlain(n3, d3);
+  } else {
+    if (ok_a != 0u) {
+      n0 = n0 / d0;
+      n1 = n1 / d1;
+    }
+    if (ok_b != 0u) {
+      n2 = n2 / d2;
+      n3 = n3 / d3;
+    }
+  }
+  gain_a += (0.5 * (n0 + n1 - a.gain)) - msg;
+  gain_b += (0.5 * (n2 + n3 - b.gain)) - msg;
+}
+
 // Leaf value and hessian of entry i = node * K + output, from the node's quantised sums; the leaf value of a node whose
 // parent did not split is 0.
 __device__ inline double2 FinishedNode(const TreeArrays& tree, const QuantParams& qp, int K, int64_t i, double l1, double l2)
