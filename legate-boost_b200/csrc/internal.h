@@ -388,8 +388,8 @@ void PartitionRows(lbk_context* ctx, Scratch& s, const PartitionLevel& pl, cudaS
 // objective.cu
 void Gradient(int objective, const double* raw_pred, const double* y, int64_t n_rows, int n_outputs, double learning_rate,
               double* g, double* h, cudaStream_t stream);
-// small_tree.cu: a whole tree in one launch, for matrices of at most kSmallMaxElements rows x outputs
-constexpr int64_t kSmallMaxElements = 16384;
+// small_tree.cu: a whole tree in one launch, for matrices of at most kSmallMaxRows rows
+constexpr int64_t kSmallMaxRows = 32768;
 template <typename T>
 struct SmallTreeArgs {
   const T* X;

@@ -115,15 +115,19 @@ __device__ inline bool GridBarrier(unsigned int* word, unsigned int target, int*
   return *s_ok != 0;
 }
 
-template <typename T>
+// What a tree is grown on, as far as it is one output: less code, which every launch of this kernel fetches anew.
+enum SmallForm { kGiven, kSquaredError, kAnyForm };
+
+template <SmallForm kForm, typename T>
 __device__ inline double2 SmallGradient(const SmallParams<T>& p, int row, int k)
 {
-  if (p.objective < 0) return make_double2(p.g[row * p.ldg + k], p.h[row * p.ldg + k]);
+  if (kForm == kSquaredError) return GradientSquaredError(p.pred[row], p.y[row], p.lr);
+  if (kForm == kGiven || p.objective < 0) return make_double2(p.g[row * p.ldg + k], p.h[row * p.ldg + k]);
   const double raw = p.pred[static_cast<int64_t>(row) * p.K + k], y = p.y[static_cast<int64_t>(row) * p.K + k];
   return p.objective == LBK_SQUARED_ERROR ? GradientSquaredError(raw, y, p.lr) : GradientLogistic(raw, y, p.lr);
 }
 
-template <typename T>
+template <typename T, bool kMany, SmallForm kForm>
 __global__ void __launch_bounds__(kSmallThreads, 1)
   k_tree_small(const SmallParams<T> p)
 {
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   __shared__ GPairI64 s_tot[2][kSmallWarps / 2];
   __shared__ SmallCand s_best[2][2][kSmallWarps / 2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int N = p.N, F = p.F, K = p.K, D = p.D, S = p.S;
+  const int N = p.N, F = p.F, K = kMany ? p.K : 1, D = p.D, S = p.S;
   const int n_blocks = gridDim.x, block = blockIdx.x;
   const int part     = block % p.parts;            // of the feature's rows (binning) and node pairs (levels)
   const int f_first = block / p.parts, f_step = n_blocks / p.parts;
@@ -239,7 +243,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
         double vg = 0.0, vh = 0.0;
         if (idx < n) {
           const int row    = static_cast<int>(K == 1 ? idx : idx / K);
-          const double2 gh = SmallGradient(p, row, static_cast<int>(idx - static_cast<int64_t>(row) * K));
+          const double2 gh = SmallGradient<kForm>(p, row, static_cast<int>(idx - static_cast<int64_t>(row) * K));
           vg               = fabs(gh.x);
           vh               = fabs(gh.y);
         }
@@ -288,7 +292,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       const int row = i / K, k = i - row * K;
       long long qg = 0, qh = 0;
       if (i < r1 * K) {
-        const double2 gh = SmallGradient(p, row, k);
+        const double2 gh = SmallGradient<kForm>(p, row, k);
         const int2 q     = QuantisePair(gh.x, gh.y, qp, HashCombine(static_cast<long long>(p.seed), p.row_offset + row, k));
         p.pairs[i]       = q;
         qg               = q.x;
@@ -723,7 +727,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   const int r0 = min(N, block * per), r1 = min(N, r0 + per);
   if (p.leaf != nullptr)
     for (int row = r0 + tid; row < r1; row += kSmallThreads) p.leaf[row] = s_pos[row];
-  if (p.objective >= 0) {
+  if (kForm != kGiven && p.objective >= 0) {
     for (int i = r0 * K + tid; i < r1 * K; i += kSmallThreads) {
       const int row = i / K, k = i - row * K;
       const GPairF64 s = Dequantise(LoadPairStreaming(p.tree.node_sums + static_cast<int64_t>(s_pos[row]) * K + k), qp);
@@ -740,11 +744,33 @@ struct SmallPlan {
   size_t smem;
 };
 
+// Is this form faster than the general path?  A block passes over all rows for every feature, output and chunk of pairs of
+// nodes that it has, and takes the pairs in turns; the general path pays for launches, whatever they do, and a little for
+// bins and rows.  Fitted to 318 shapes of both (microseconds for three rounds; what the histograms' memory costs is the same
+// on either side): all but seven of those more than 4 % apart are told right, and these are at most 12 % apart.  General and small:
+// 20k rows x 60, depth 6 1.16, 28k x 60 0.99; 16k x 100, depth 8 1.13, depth 10 0.78; 10k x 300, depth 6 1.00, depth 8 0.84; three
+// classes, 8k x 100, depth 6 1.03, 1333 x 300 0.78; ten classes, 1000 x 20, depth 4 1.14, 400 x 300 0.65.
+static bool SmallPays(const SmallPlan& plan, int64_t N, int F, int K, int D)
+{
+  int64_t passes = 0, turns = 0;
+  auto turns_of  = [](int64_t slots) { return slots > 2 ? (slots + kSmallWarps - 1) / kSmallWarps : int64_t{1}; };
+  for (int d = 0; d < D; ++d) {
+    const int64_t units = d == 0 ? 1 : int64_t{1} << (d - 1), mine = (units + plan.parts - 1) / plan.parts;
+    const int64_t whole = mine / plan.max_slots, rest = mine - whole * plan.max_slots;
+    passes += whole + (rest > 0 ? 1 : 0);
+    turns += whole * turns_of(plan.max_slots) + (rest > 0 ? turns_of(rest) : 0);
+  }
+  const int abreast  = plan.blocks / plan.parts;  // features that are worked on at a time
+  const double each  = static_cast<double>((F + abreast - 1) / abreast) * K;
+  const double small = each * (2.4e-3 * static_cast<double>(passes * N) + 20.0 * static_cast<double>(turns) - 9.0 * D);
+  const double general = D * (72.0 + 5.0 * K + (K > 1 ? 7.0 : 0.0) + 3.4e-6 * static_cast<double>(N) * F * K);
+  return small <= general;
+}
+
 static bool PlanSmall(lbk_context* ctx, int64_t N, int F, int K, int D, int S, SmallPlan& plan)
 {
-  // One-byte bins; 16-bit node ids; the canonical sum's second step in one piece.  The bound on rows x outputs
-  // is where the general path catches up: a block passes over all rows on every level.
-  if (S > kSmallBins || D < 1 || D > 12 || N < 1 || N * K > kSmallMaxElements || F > 4 * ctx->sm_count) return false;
+  // One-byte bins; 16-bit node ids; the canonical sum's second step in one piece; the range that SmallPays was measured over.
+  if (S > kSmallBins || D < 1 || D > 12 || N < 1 || N > kSmallMaxRows || N * K > 2 * kSmallMaxRows || F > 4 * ctx->sm_count) return false;
   const int64_t level = int64_t{1} << (D - 1);
   if (level * K > 1536) return false;
   const int64_t hist_bytes = (K > 1 ? level * 3 / 2 + 1 : level) * F * K * kSmallBins * 16;
@@ -766,7 +792,7 @@ static bool PlanSmall(lbk_context* ctx, int64_t N, int F, int K, int D, int S, S
   // (the partial sums, the proposals and the root sums share the histograms' place)
   const size_t early = std::max({size_t{2} * ((N * K + kSumBlock - 1) / kSumBlock) * 8, kSmallBins * size_t{8}, size_t{16} * K});
   if (early > plan.max_slots * slot) return false;
-  return true;
+  return SmallPays(plan, N, F, K, D);
 }
 
 bool SmallTreeFits(lbk_context* ctx, int64_t N, int F, int K, int D, int S)
@@ -827,7 +853,10 @@ void SmallTree(lbk_context* ctx, Scratch& s, const SmallTreeArgs<T>& a, cudaStre
   p.status    = ctx->d_status;
   p.info_host = a.info_host;
   p.barrier   = a.barrier;
-  auto fn = k_tree_small<T>;
+  auto fn = K > 1                                ? k_tree_small<T, true, kAnyForm>
+            : a.objective < 0                     ? k_tree_small<T, false, kGiven>
+            : a.objective == LBK_SQUARED_ERROR    ? k_tree_small<T, false, kSquaredError>
+                                                  : k_tree_small<T, false, kAnyForm>;
   AllowSharedMemory(ctx, fn, 2048);
   void* args[] = {&p};
   LBK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(fn), dim3(plan.blocks), dim3(kSmallThreads), args,

@@ -1233,6 +1233,19 @@ def test_many_outputs_at_the_edge_of_default_shared_memory(lb, oracle, K):
         assert np.array_equal(t[name].cpu().numpy(), getattr(want, name)), name
 
 
+@pytest.mark.parametrize("N,F,K,D,dt", [
+    (26_001, 20, 1, 6, np.float32), (32_768, 4, 1, 3, np.float64), (32_769, 4, 1, 3, np.float64),  # many rows; one too many
+    (3_000, 64, 1, 9, np.float32), (900, 145, 1, 9, np.float64),  # a warp per pair of nodes, in whole and broken turns
+    (300, 12, 1, 11, np.float32), (2_000, 18, 3, 8, np.float32), (700, 9, 10, 5, np.float64),
+    (400, 300, 10, 4, np.float32), (12_000, 300, 1, 8, np.float32),  # few rows, but the general path is faster
+])
+def test_trees_around_the_one_launch_rule(lb, oracle, N, F, K, D, dt):
+    for small in (False, True):  # (hessians that quantise to 0: raw bins stay in the scan)
+        _, want, got = _run_tree_case(lb, oracle, (N, F, K, D, 256, dt, {}), seed=D, hess_small=small)
+        for name in ("feature", "split_value", "node_sums", "gain", "hessian", "leaf_value"):
+            assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
+
+
 @pytest.mark.parametrize("N,F,K,D", [(40, 300, 1, 8), (500, 10, 1, 6), (2000, 3, 3, 7), (16384, 2, 1, 5)])
 def test_one_launch_trees_are_the_same_every_time(lb, oracle, N, F, K, D):
     """The blocks of the one-launch tree pick every level's winners for themselves and must agree, whichever of them is
