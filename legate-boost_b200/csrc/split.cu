@@ -23,6 +23,18 @@ namespace {
 constexpr int kSplitThreads = 256;
 constexpr int kSplitWarps   = kSplitThreads / 32;
 
+// A warp takes a feature (kWide) where there are so many units x features that no warp is alone on its scheduler: no
+// barrier, and no totals of eight warps to add up, per output and 256 bins.  Microseconds with a block per feature and with
+// a warp: one output, 400 features, 8 units 36 and 27, 128 units 272 and 259; 64 features, 32 units 29 and 24, 16 units 17.7 and 20; 20
+// features, 128 units 36.7 and 27.7, 32 units 15.7 and 20.4; three outputs, 100 features, 32 units 79 and 66, 16 units 46 and
+// 48; ten outputs, 64 units 296 and 287, 32 units 167 and 177.
+constexpr int kWideOutputs = 64;  // (what a block has room for)
+__host__ inline bool ScanIsWide(int64_t units, int n_features, int K)
+{
+  const int64_t least = K <= 1 ? 1500 : K < 6 ? 1000 * K : 6000;
+  return K <= kWideOutputs && units * n_features >= least;
+}
+
 // What a rank knows about its best split of a node when the features are divided among the ranks:
 // the candidate and the sums left of it; K pairs follow the header.
 struct SplitRecordHeader {
@@ -91,8 +103,8 @@ struct SliceBest {
 // A thread per bin and not a warp per feature (four bins per lane): a warp alone on its scheduler gets one
 // instruction in about five clocks, and a feature's 2600 of them were 9 us whatever the level held; and 60
 // registers instead of 128 keep 32 warps on an SM where the level is wide.
-template <typename T, bool kManyOutputs, bool kDerive>
-__global__ void __launch_bounds__(kSplitThreads, kManyOutputs ? 3 : 4)
+template <typename T, bool kManyOutputs, bool kDerive, bool kWide>
+__global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
   k_scan_split(const __grid_constant__ ScanSplitParams<T> p)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];  // several outputs: terms [2][K]; then carries [K]
@@ -111,7 +123,8 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs ? 3 : 4)
   const GPairI64 sum_0 = LoadPair(node_sums + static_cast<int64_t>(node0) * K);
   const GPairI64 sum_1 = kDerive ? LoadPair(node_sums + static_cast<int64_t>(node0 + 1) * K) : GPairI64{0, 0};
   const QuantParams qp = *p.qp;
-  int f  = lv.f_begin + blockIdx.y;
+  const int f_step = kWide ? kSplitWarps * slices : slices;
+  int f  = lv.f_begin + (kWide ? kSplitWarps * blockIdx.y + warp : blockIdx.y);
   int fb = f < lv.f_end ? p.row_ptr[f] : 0, fe = f < lv.f_end ? p.row_ptr[f + 1] : 0;
   if (parent_feature < 0) return;  // the parent did not split: no such node
   // _a: the built node, _b: its sibling (SmallerChildIsLeft)
@@ -145,7 +158,89 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs ? 3 : 4)
   Cand best_a{0.0, -1, -1}, best_b{0.0, -1, -1};
   GPairI64 left_a{0, 0}, left_b{0, 0};
   int turn = 0;
-  while (f < lv.f_end) {
+  auto keep_best = [&](unsigned ok, double gain, int bin, const GPairI64& v, Cand& best, GPairI64& left) {
+    if (ok && gain > 0) {
+      const Cand c{gain, bin, f};
+      if (Better(c, best)) {
+        best = c;
+        if (!kManyOutputs) left = v;
+      }
+    }
+  };
+  while (kWide && f < lv.f_end) {
+    const bool search = p.sp.feature_set == nullptr || p.sp.feature_set[f] != 0;
+    GPairI64* carry = s_carry + (kManyOutputs ? warp * K : 0);  // (several outputs: sums of the bins before)
+    GPairI64 before{0, 0};
+    for (int base = fb; base < fe; base += 32) {
+      const bool in = base + lane < fe;
+      double gain_a = 0.0, gain_b = 0.0;
+      GPairI64 va, vb{0, 0};
+      unsigned ok_a = eval_a && search && in ? 1u : 0u, ok_b = eval_b && search && in ? 1u : 0u;
+      GPairI64 ahead_a{0, 0}, ahead_b{0, 0};
+      if (in) {
+        ahead_a = LoadPair(src + base + lane);
+        if (kDerive) ahead_b = LoadPair(par + base + lane);
+      }
+      if (kManyOutputs) __syncwarp();
+      for (int k = 0; k < (kManyOutputs ? K : 1); ++k) {
+        const int64_t at = (kManyOutputs ? static_cast<int64_t>(k) * Bs : 0) + base + lane;
+        if (kManyOutputs) {
+          ta = s_terms[2 * k];
+          if (kDerive) tb = s_terms[2 * k + 1];
+          before = base > fb ? carry[k] : GPairI64{0, 0};
+        }
+        const bool scanned = ta.h > 0.0;
+        va = ahead_a;
+        if (kDerive) vb = ahead_b;
+        if (kManyOutputs && in && k + 1 < K) {
+          ahead_a = LoadPair(src + at + Bs);
+          if (kDerive) ahead_b = LoadPair(par + at + Bs);
+        }
+        long long sg = va.grad, sh = va.hess;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const long long ng = __shfl_up_sync(0xffffffffu, sg, off);
+          const long long nh = __shfl_up_sync(0xffffffffu, sh, off);
+          if (lane >= off) {
+            sg += ng;
+            sh += nh;
+          }
+        }
+        sg += before.grad;
+        sh += before.hess;
+        if (kManyOutputs) {
+          __syncwarp();
+          if (lane == 31) carry[k] = GPairI64{sg, sh};
+        } else {
+          before = GPairI64{__shfl_sync(0xffffffffu, sg, 31), __shfl_sync(0xffffffffu, sh, 31)};
+        }
+        if (in) {
+          if (scanned && (sg > 0 || sh > 0)) va = GPairI64{sg, sh};
+          if (kDerive) vb = scanned ? GPairI64{vb.grad - va.grad, vb.hess - va.hess} : GPairI64{0, 0};
+          if (lv.write_hist) {
+            StorePair(dst_a + at, va);
+            if (kDerive) StorePair(dst_b + at, vb);
+          }
+          if (lv.next_built != nullptr) {
+            StorePair(next_a + at, GPairI64{0, 0});
+            if (kDerive) StorePair(next_b + at, GPairI64{0, 0});
+          }
+        }
+        if (kDerive) {
+          if (__any_sync(0xffffffffu, ok_a | ok_b)) AddGains(va, ok_a, ta, gain_a, vb, ok_b, tb, gain_b, qp, l1, reg, msg);
+        } else if (__any_sync(0xffffffffu, ok_a)) {
+          ok_a = AddGain(va, ok_a, ta, qp, l1, reg, msg, gain_a);
+        }
+      }
+      keep_best(ok_a, gain_a, base + lane, va, best_a, left_a);
+      if (kDerive) keep_best(ok_b, gain_b, base + lane, vb, best_b, left_b);
+    }
+    f += f_step;
+    if (f >= lv.f_end) break;
+    fb = p.row_ptr[f];
+    fe = p.row_ptr[f + 1];
+  }
+  while (!kWide && f < lv.f_end) {
     const bool search = p.sp.feature_set == nullptr || p.sp.feature_set[f] != 0;
     for (int base = fb; base < fe; base += kSplitThreads) {
       const bool in = base + tid < fe;
@@ -219,25 +314,16 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs ? 3 : 4)
             if (kDerive) StorePair(next_b + at, GPairI64{0, 0});
           }
         }
-        if (__any_sync(0xffffffffu, ok_a)) ok_a = AddGain(va, ok_a, ta, qp, l1, reg, msg, gain_a);
-        if (kDerive && __any_sync(0xffffffffu, ok_b)) ok_b = AddGain(vb, ok_b, tb, qp, l1, reg, msg, gain_b);
-      }
-      if (ok_a && gain_a > 0) {
-        const Cand c{gain_a, base + tid, f};
-        if (Better(c, best_a)) {
-          best_a = c;
-          if (!kManyOutputs) left_a = va;
+        if (kDerive) {
+          if (__any_sync(0xffffffffu, ok_a | ok_b)) AddGains(va, ok_a, ta, gain_a, vb, ok_b, tb, gain_b, qp, l1, reg, msg);
+        } else if (__any_sync(0xffffffffu, ok_a)) {
+          ok_a = AddGain(va, ok_a, ta, qp, l1, reg, msg, gain_a);
         }
       }
-      if (kDerive && ok_b && gain_b > 0) {
-        const Cand c{gain_b, base + tid, f};
-        if (Better(c, best_b)) {
-          best_b = c;
-          if (!kManyOutputs) left_b = vb;
-        }
-      }
+      keep_best(ok_a, gain_a, base + tid, va, best_a, left_a);
+      if (kDerive) keep_best(ok_b, gain_b, base + tid, vb, best_b, left_b);
     }
-    f += slices;
+    f += f_step;
     if (f >= lv.f_end) break;
     fb = p.row_ptr[f];
     fe = p.row_ptr[f + 1];
@@ -397,10 +483,11 @@ void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, co
   const int n_features = lv.f_end - lv.f_begin;
   const int units      = lv.derive ? lv.n_nodes / 2 : lv.n_nodes;
   if (units <= 0) return;
-  // with several outputs a block keeps K terms of two nodes and K running prefixes in shared memory
-  const size_t smem = (lv.K > 1 ? sizeof(NodeTerms) * 2 * ((lv.K + 1) / 2 * 2) : 0) + lv.K * sizeof(GPairI64);
-  // one feature per block until there are about sixteen blocks per SM, then several
-  int slices     = n_features > 0 ? n_features : 1;
+  const bool wide = ScanIsWide(units, n_features, lv.K);
+  // with several outputs a block keeps K terms of two nodes and K running prefixes (of every warp) in shared memory
+  const size_t smem = (lv.K > 1 ? sizeof(NodeTerms) * 2 * ((lv.K + 1) / 2 * 2) : 0) + lv.K * sizeof(GPairI64) * (wide ? kSplitWarps : 1);
+  // one feature per block (warp) until there are about sixteen blocks per SM, then several
+  int slices     = n_features > 0 ? (wide ? (n_features + kSplitWarps - 1) / kSplitWarps : n_features) : 1;
   const int most = (16 * ctx->sm_count + units - 1) / units;
   if (slices > most) slices = most;
   ScanSplitParams<T> p;
@@ -422,8 +509,10 @@ void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, co
     LBK_CUDA(cudaMemsetAsync(mine, 0, rb * lv.n_nodes, stream));
     p.records = mine;
   }
-  auto fn = lv.K > 1 ? (lv.derive ? k_scan_split<T, true, true> : k_scan_split<T, true, false>)
-                     : (lv.derive ? k_scan_split<T, false, true> : k_scan_split<T, false, false>);
+  auto fn = lv.K > 1 ? (lv.derive ? (wide ? k_scan_split<T, true, true, true> : k_scan_split<T, true, true, false>)
+                                  : (wide ? k_scan_split<T, true, false, true> : k_scan_split<T, true, false, false>))
+                     : (lv.derive ? (wide ? k_scan_split<T, false, true, true> : k_scan_split<T, false, true, false>)
+                                  : (wide ? k_scan_split<T, false, false, true> : k_scan_split<T, false, false, false>));
   if (smem > 40 * 1024) AllowSharedMemory(ctx, fn, 2048);  // (the limit without it counts the static part too)
   fn<<<dim3(units, slices), kSplitThreads, smem, stream>>>(p);
   LBK_LAUNCH_CHECK();

@@ -1233,6 +1233,18 @@ def test_many_outputs_at_the_edge_of_default_shared_memory(lb, oracle, K):
         assert np.array_equal(t[name].cpu().numpy(), getattr(want, name)), name
 
 
+@pytest.mark.parametrize("N,F,K,D,S,dt", [
+    (40_000, 30, 1, 8, 256, np.float32), (40_000, 33, 1, 8, 100, np.float64),  # a warp per feature on the last levels
+    (9_000, 60, 1, 7, 700, np.float32), (20_000, 101, 3, 7, 256, np.float32), (4_000, 130, 10, 7, 256, np.float32),
+    (33_000, 49, 2, 8, 31, np.float32),
+])
+def test_wide_levels(lb, oracle, N, F, K, D, S, dt):
+    for small in (False, True):
+        _, want, got = _run_tree_case(lb, oracle, (N, F, K, D, S, dt, {"mask": small}), seed=D, hess_small=small)
+        for name in ("feature", "split_value", "node_sums", "gain", "hessian", "leaf_value"):
+            assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
+
+
 @pytest.mark.parametrize("N,F,K,D,dt", [
     (26_001, 20, 1, 6, np.float32), (32_768, 4, 1, 3, np.float64), (32_769, 4, 1, 3, np.float64),  # many rows; one too many
     (3_000, 64, 1, 9, np.float32), (900, 145, 1, 9, np.float64),  # a warp per pair of nodes, in whole and broken turns
