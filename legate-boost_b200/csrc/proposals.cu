@@ -323,6 +323,87 @@ struct SearchLevels<T, U, -1, kPitch> {
   __device__ static void run(unsigned (&)[U], const T (&)[U]) {}
 };
 
+// Where the search for x begins, as in k_bin_lut: x falls into one of P buckets by a map that never decreases, and a table says
+// how many proposals lie in the buckets below.  The map goes through float32 whatever T is (rounding does not decrease either), is
+// spread from the fifth proposal to the fifth from the end, and sends a NaN on the way to bucket 0.
+struct StartMap {
+  float lo, scale;
+};
+template <int P>
+__device__ inline int StartBucket(float x, const StartMap& m)
+{
+  const int b = __float2int_rz((x - m.lo) * m.scale);
+  return b < 0 ? 0 : b < P ? b : P - 1;
+}
+constexpr int kStartSpare = 16;  // rows of the table behind the proposals, +inf: the last steps may look beyond the last one
+
+// Fills the table of a block, sp[P + kStartSpare][kFeatures], with the proposals of the features from f0 on.
+template <typename T, int kFeatures, int kRows>
+__device__ inline void FillProposals(T* sp, int* s_begin, int* s_n, const T* proposals, int64_t cut_stride, const int32_t* row_ptr, int f0, int F)
+{
+  if (threadIdx.x < kFeatures) {
+    const int f = f0 + static_cast<int>(threadIdx.x), b = f < F ? row_ptr[f] : 0;
+    s_begin[threadIdx.x] = cut_stride > 0 ? 0 : b;
+    s_n[threadIdx.x]     = f < F ? row_ptr[f + 1] - b : 0;
+  }
+  __syncthreads();
+#pragma unroll 8
+  for (int idx = threadIdx.x; idx < kRows * kFeatures; idx += blockDim.x) {
+    const int j = idx / kFeatures, fl = idx % kFeatures;
+    sp[idx]     = j < s_n[fl] ? proposals[(cut_stride > 0 ? (f0 + fl) * cut_stride : s_begin[fl]) + j] : static_cast<T>(INFINITY);
+  }
+  __syncthreads();
+}
+
+// starts [P][kFeatures] and the maps, by kThreads threads; returns how many steps of a search from there are enough for every
+// feature of the block: 3 (no more than 7 proposals share a bucket), 4 (15), or 0: the whole search, without the table
+// (they crowd together more, or are not in order with +inf at the end).
+template <typename T, int kFeatures, int P, int kThreads>
+__device__ inline int MakeStarts(const T* sp, uint16_t* starts, const int* s_n, StartMap* s_map)
+{
+  if (threadIdx.x < kFeatures) {
+    const int fl = threadIdx.x, n = s_n[fl], end = n >= 32 ? 4 : 0;
+    StartMap m{0.0f, 0.0f};
+    if (n >= 3) {  // (the last proposal is +inf)
+      m.lo    = static_cast<float>(sp[end * kFeatures + fl]);
+      m.scale = static_cast<float>(P) / (static_cast<float>(sp[(n - 2 - end) * kFeatures + fl]) - m.lo);
+      if (!(m.scale > 0.0f) || !(m.scale < INFINITY) || !(fabsf(m.lo) < INFINITY)) m.lo = m.scale = 0.0f;  // all in one bucket
+    }
+    s_map[fl] = m;
+  }
+  __syncthreads();
+  // a thread has kOwn neighbouring proposals (and then buckets) of one feature
+  constexpr int kOwn = P * kFeatures / kThreads;
+  const int fl = threadIdx.x % kFeatures, n = s_n[fl], j0 = threadIdx.x / kFeatures * kOwn;
+  const StartMap m = s_map[fl];
+  auto at_of  = [&](int i) { return StartBucket<P>(static_cast<float>(sp[i * kFeatures + fl]), m); };
+  int crowd   = 0;
+  int before  = j0 > 0 && j0 < n ? at_of(j0 - 1) : -1;
+#pragma unroll 4
+  for (int i = 0; i < kOwn; ++i) {
+    const int j = j0 + i;
+    if (j < n) {
+      const int at = at_of(j);
+      const T v = sp[j * kFeatures + fl], next = sp[(j + 1) * kFeatures + fl];
+      for (int k = before + 1; k <= at; ++k) starts[k * kFeatures + fl] = static_cast<uint16_t>(j);
+      if (j == n - 1 ? v != static_cast<T>(INFINITY) : !(v < next)) crowd = 2;
+      if (j == n - 1)  // (+inf is in the last bucket, unless all are in the first)
+        for (int k = at + 1; k < P; ++k) starts[k * kFeatures + fl] = static_cast<uint16_t>(n);
+      before = at;
+    }
+  }
+  if (n == 0)
+    for (int i = 0; i < kOwn; ++i) starts[(j0 + i) * kFeatures + fl] = 0;
+  if (__syncthreads_or(crowd)) return 0;
+#pragma unroll 4
+  for (int i = 0; i < kOwn; ++i) {
+    const int b = j0 + i, first = starts[b * kFeatures + fl], next = b + 1 < P ? starts[(b + 1) * kFeatures + fl] : n;
+    crowd = max(crowd, next - first);
+  }
+  if (!__syncthreads_or(crowd > 7)) return 3;
+  return !__syncthreads_or(crowd > 15) ? 4 : 0;
+}
+
 // One warp per row, one lane per feature of the group.
 //
 // Shared-memory variant: the proposals of the group are kept transposed and padded, sp[j][lane] =
@@ -711,76 +792,93 @@ __global__ void __launch_bounds__(kLutThreads, 1)
 // (16, 8 or 4) as fill 64 KB, three blocks per SM.  A lane has one feature and eight consecutive rows, which leave as
 // one 16-byte store of the feature-major copy; the 32 / kFeatures row groups of a warp may meet in a bank
 // (a probe is 1 to 2.5 passes), which costs less than the probes going to L2: 300003 x 37 float64,
-// 512 proposals: 70 us against 425 of k_bin_global.  Filling the table takes 8 (float64) to 15 us (float32), so that
-// small float32 matrices stay with k_bin_global (10000 x 37, 1024 proposals: 20 us here, 13 there; 100000 x 37: 35
-// and 64; float64: 14 and 18; 39 and 77).
+// 512 proposals: 70 us with the copy against 425 of k_bin_global.  Small float32 matrices stay with k_bin_global.
+//
+// With enough rows the search begins from a table of starts and takes three or four steps instead of nine to eleven.  (Two
+// blocks and their tables stay within 196 KB: the next larger share of the SM leaves an L1 of 28 KB, which is less than
+// the rows on their way: 2M x 64 float32, 2048 proposals: 540 and 660 us.)  Before (three blocks of 256 threads, the whole
+// search, a table filled by one load after the other) and now: 300003 x 37 float64, 512 proposals 57.6 -> 51 us (exponential
+// columns, which crowd together: 57.3 -> 62), 2048 proposals 152 -> 97; 2M x 64, 512 proposals 342 -> 259; float32, 1024 proposals
+// 366 -> 306, 2048 704 -> 540; 10000 x 37 float64 14.2 -> 11.8.
 constexpr int kWideTableBytes = 64 * 1024;
+constexpr int kWideThreads    = 512;
+constexpr int kStartMinRows   = 2500;  // of a block, from which the table of starts (4 us) pays
+template <typename T, int kLog2P>
+struct WideTable {
+  static constexpr int P         = 1 << kLog2P;
+  static constexpr int kFeatures = kWideTableBytes / (P * static_cast<int>(sizeof(T)));
+  static constexpr size_t kSmem  = (P + kStartSpare) * kFeatures * sizeof(T) + P * kFeatures * sizeof(uint16_t);
+};
 
 template <typename T, int kLog2P, bool kCopyT>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(kWideThreads, 2)
   k_bin_wide(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const T* __restrict__ proposals, int64_t cut_stride,
              const int32_t* __restrict__ row_ptr, int pitch, uint16_t* __restrict__ bins, uint16_t* __restrict__ bins_t, int64_t pitch_t)
 {
-  constexpr int P         = 1 << kLog2P;
-  constexpr int kFeatures = kWideTableBytes / (P * static_cast<int>(sizeof(T)));
+  using Table             = WideTable<T, kLog2P>;
+  constexpr int P         = Table::P;
+  constexpr int kFeatures = Table::kFeatures;
   constexpr int U         = 8;
   constexpr int kTurn     = 32 / kFeatures * U;  // rows of a warp
   constexpr unsigned kPitch = kFeatures * sizeof(T);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sp        = reinterpret_cast<T*>(smem_raw);
-  const int f0 = blockIdx.y * kFeatures;
+  __shared__ int s_begin[kFeatures], s_n[kFeatures];
+  __shared__ StartMap s_map[kFeatures];
+  T* sp            = reinterpret_cast<T*>(smem_raw);
+  uint16_t* starts = reinterpret_cast<uint16_t*>(sp + (P + kStartSpare) * kFeatures);
+  const int f0     = blockIdx.y * kFeatures;
   if (f0 >= F) {  // padding columns
     const int64_t all = n_rows * kFeatures;
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < all; i += static_cast<int64_t>(gridDim.x) * blockDim.x)
       bins[i / kFeatures * pitch + f0 + i % kFeatures] = 0;
     return;
   }
-  for (int idx = threadIdx.x; idx < P * kFeatures; idx += blockDim.x) {
-    const int j = idx / kFeatures, f = f0 + idx % kFeatures;
-    T v = static_cast<T>(INFINITY);
-    if (f < F) {
-      const int b = row_ptr[f];
-      if (j < row_ptr[f + 1] - b) v = proposals[(cut_stride > 0 ? f * cut_stride : b) + j];
-    }
-    sp[idx] = v;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, f = f0 + lane % kFeatures;
+  FillProposals<T, kFeatures, P + kStartSpare>(sp, s_begin, s_n, proposals, cut_stride, row_ptr, f0, F);
+  const int steps = n_rows >= static_cast<int64_t>(gridDim.x) * kStartMinRows ? MakeStarts<T, kFeatures, P, kWideThreads>(sp, starts, s_n, s_map) : 0;
+  const int lane = threadIdx.x & 31, fl = lane % kFeatures, f = f0 + fl;
   // lanes beyond the last feature read the last feature's values; their column is all +inf, their ids are 0
   const bool active    = f < F;
-  const unsigned col_s = static_cast<unsigned>(__cvta_generic_to_shared(sp + lane % kFeatures));
+  const unsigned col_s = static_cast<unsigned>(__cvta_generic_to_shared(sp + fl));
+  const StartMap map   = steps != 0 ? s_map[fl] : StartMap{};
   const T* xcol        = X + (active ? f : F - 1);
   const int n          = static_cast<int>(n_rows);
   const int hop        = static_cast<int>(gridDim.x) * (blockDim.x >> 5) * kTurn;
-  int base             = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kTurn + lane / kFeatures * U;
-  T xn[U];
-  auto load_rows = [&](int first) {
-    const T* src = xcol + static_cast<int64_t>(first) * ldx;
+  auto all_rows = [&](auto levels) {
+    constexpr int kLevels = decltype(levels)::value;  // 0: the whole search
+    int base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kTurn + lane / kFeatures * U;
+    T xn[U];
+    auto load_rows = [&](int first) {
+      const T* src = xcol + static_cast<int64_t>(first) * ldx;
 #pragma unroll
-    for (int u = 0; u < U; ++u) xn[u] = first + u < n ? LdgStream(src + u * ldx) : static_cast<T>(-INFINITY);
-  };
-  load_rows(base);
-  for (; base < n; base += hop) {
-    T x[U];
-    unsigned pos[U];
+      for (int u = 0; u < U; ++u, src += ldx) xn[u] = first + u < n ? LdgStream(src) : static_cast<T>(-INFINITY);
+    };
+    load_rows(base);
+    for (; base < n; base += hop) {
+      T x[U];
+      unsigned pos[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      x[u]   = xn[u];
-      pos[u] = col_s;
+      for (int u = 0; u < U; ++u) {
+        x[u]   = xn[u];
+        pos[u] = col_s;
+        if (kLevels != 0) pos[u] += starts[StartBucket<P>(static_cast<float>(x[u]), map) * kFeatures + fl] * kPitch;
+      }
+      if (base + hop < n) load_rows(base + hop);
+      SearchLevels<T, U, (kLevels != 0 ? kLevels : kLog2P) - 1, kPitch>::run(pos, x);
+      unsigned id[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) id[u] = (pos[u] - col_s) / kPitch;
+      uint16_t* out = bins + static_cast<int64_t>(base) * pitch + f;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (base + u < n) out[static_cast<int64_t>(u) * pitch] = static_cast<uint16_t>(id[u]);
+      if (kCopyT && active)  // (the copy's rows are padded to 32; ids beyond the last row are 0)
+        *reinterpret_cast<uint4*>(bins_t + static_cast<int64_t>(f) * pitch_t + base) =
+          make_uint4(id[0] | (id[1] << 16), id[2] | (id[3] << 16), id[4] | (id[5] << 16), id[6] | (id[7] << 16));
     }
-    if (base + hop < n) load_rows(base + hop);
-    SearchLevels<T, U, kLog2P - 1, kPitch>::run(pos, x);
-    unsigned id[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) id[u] = (pos[u] - col_s) / kPitch;
-    uint16_t* out = bins + static_cast<int64_t>(base) * pitch + f;
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (base + u < n) out[static_cast<int64_t>(u) * pitch] = static_cast<uint16_t>(id[u]);
-    if (kCopyT && active)  // (the copy's rows are padded to 32; ids beyond the last row are 0)
-      *reinterpret_cast<uint4*>(bins_t + static_cast<int64_t>(f) * pitch_t + base) =
-        make_uint4(id[0] | (id[1] << 16), id[2] | (id[3] << 16), id[4] | (id[5] << 16), id[6] | (id[7] << 16));
-  }
+  };
+  if (steps == 3) all_rows(std::integral_constant<int, 3>());
+  else if (steps == 4) all_rows(std::integral_constant<int, 4>());
+  else all_rows(std::integral_constant<int, 0>());
 }
 
 // Global-memory variant: more proposals than any table here holds, or too few rows to pay for filling one.
@@ -967,12 +1065,13 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
     auto wide = [&](auto log2p_, auto copy_) {
       constexpr int L    = decltype(log2p_)::value;
       constexpr bool CT  = decltype(copy_)::value;
-      constexpr int kFeatures = kWideTableBytes / ((1 << L) * static_cast<int>(sizeof(T)));
+      using Table = WideTable<T, L>;
+      constexpr int kFeatures = Table::kFeatures;
       auto fn = k_bin_wide<T, L, CT>;
-      LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideTableBytes));
-      // (three blocks per SM, spread over the tables that hold features)
-      const dim3 grid(blocks_of((F + kFeatures - 1) / kFeatures, 3, kSmemFillRows), G * kGroup / kFeatures);
-      fn<<<grid, 256, kWideTableBytes, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, G * kGroup,
+      LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Table::kSmem)));
+      // (two blocks per SM, spread over the tables that hold features)
+      const dim3 grid(blocks_of((F + kFeatures - 1) / kFeatures, 2, kSmemFillRows), G * kGroup / kFeatures);
+      fn<<<grid, kWideThreads, Table::kSmem, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, G * kGroup,
                                                  static_cast<uint16_t*>(bins), static_cast<uint16_t*>(bins_t), pitch_t);
     };
     auto by_copy = [&](auto log2p_) {

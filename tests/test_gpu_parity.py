@@ -1169,6 +1169,40 @@ def test_one_byte_bin_ids_of_several_turns(lb, oracle, N, F):
         assert np.array_equal(tree[name].cpu().numpy(), getattr(want, name)), name
 
 
+@pytest.mark.parametrize("N,F,S,dt", [
+    (250_003, 40, 512, np.float64), (80_001, 39, 2048, np.float64), (250_003, 40, 1000, np.float32), (150_001, 37, 2048, np.float32),
+    (30_000, 40, 512, np.float64),  # too few rows for a table of starts
+])
+@pytest.mark.parametrize("spread", ["even", "crowded"])
+def test_two_byte_bin_ids_of_many_rows(lb, oracle, N, F, S, dt, spread):
+    """Searches that begin from a table, of three and four steps, and whole ones where proposals crowd together."""
+    from legateboost_b200 import stages
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.RandomState(F + S)
+    X = rs.random((N, F)).astype(dt)
+    if spread == "crowded":
+        X[:, 1::3] = np.exp(4 * rs.normal(size=X[:, 1::3].shape)).astype(dt)
+        X[:, 2::3] = np.round(X[:, 2::3] * 700) / 700
+        X[:, 3] = 7.0
+        X[rs.randint(N, size=20), 4] = 1e30
+    proposals, row_ptr = stages.split_proposals(dev(X), S, 3)
+    p, rp = proposals.cpu().numpy(), row_ptr.cpu().numpy()
+    Z = X.copy()
+    for value in (np.nan, np.inf, -np.inf, 0.0):
+        Z[rs.randint(N, size=500), rs.randint(F, size=500)] = value
+    got = stages.bin_matrix(dev(Z), proposals, row_ptr, 2).cpu().numpy().view(np.uint16)
+    assert not got[:, F:].any()
+    for f in range(F):
+        want = np.where(np.isnan(Z[:, f]), 0, np.searchsorted(p[rp[f]:rp[f + 1]], Z[:, f], side="left"))
+        assert np.array_equal(got[:, f], want), f
+    g, h = rs.normal(size=(N, 1)) + np.sin(6 * X[:, :1]), np.ones((N, 1))  # (the feature-major copy)
+    want = oracle.build_tree(X, g, h, max_depth=2, split_samples=S, seed=5, mode="Q")
+    tree = build_tree_arrays(dev(X), dev(g), dev(h), max_depth=2, split_samples=S, seed=5, row_offset=0, dataset_rows=N)
+    for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
+        assert np.array_equal(tree[name].cpu().numpy(), getattr(want, name)), name
+
+
 @pytest.mark.parametrize("N,K", [(1, 3), (255, 23), (257, 24), (1000, 186), (70, 187), (70, 300)])
 def test_softmax_gradients_of_whole_and_partial_tiles(lb, N, K):
     """The tiled kernel (256 rows down to 32 per block) and the one for more classes than it takes."""
