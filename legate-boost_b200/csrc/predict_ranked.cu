@@ -714,16 +714,35 @@ bool PredictRanked(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   const int64_t wave    = tile * ctx->sm_count;
   const int64_t waves   = std::max<int64_t>(1, static_cast<int64_t>(kRankBytes / (static_cast<size_t>(wave) * F * 2)));
   const int64_t piece   = std::min(waves * wave, (n_rows + tile - 1) / tile * tile);
-  int* words            = s.alloc<int>(2 * static_cast<size_t>(F) + 1);  // counts, cursors, too many
-  int* off              = s.alloc<int>(static_cast<size_t>(F) + 1);
-  T* lists              = s.alloc<T>(static_cast<size_t>(total_nodes));
-  T* cuts               = s.alloc<T>(static_cast<size_t>(total_nodes));
-  unsigned* lut         = s.alloc<unsigned>(static_cast<size_t>(total_nodes));
-  RankTable* tables     = s.alloc<RankTable>(F);
-  unsigned char* records = static_cast<unsigned char*>(s.alloc_bytes(static_cast<size_t>(n_trees) * RankRecordBytes(S)));
-  unsigned* ranks        = s.alloc<unsigned>(static_cast<size_t>(piece / 2) * F);
+  // one piece of scratch, so that a call which has no room for it is left as it was: it takes the other path
+  size_t bytes = 0;
+  auto reserve = [&](size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  };
+  const size_t nodes = static_cast<size_t>(total_nodes), words_bytes = sizeof(int) * (2 * static_cast<size_t>(F) + 1);
+  const size_t o_words = reserve(words_bytes), o_off = reserve(sizeof(int) * (static_cast<size_t>(F) + 1));
+  const size_t o_lists = reserve(nodes * sizeof(T)), o_cuts = reserve(nodes * sizeof(T)), o_lut = reserve(nodes * sizeof(unsigned));
+  const size_t o_tables = reserve(sizeof(RankTable) * F), o_records = reserve(static_cast<size_t>(n_trees) * RankRecordBytes(S));
+  const size_t o_ranks  = reserve(static_cast<size_t>(piece / 2) * F * sizeof(unsigned));
+  unsigned char* room   = nullptr;
+  try {
+    room = static_cast<unsigned char*>(s.alloc_bytes(bytes));
+  } catch (const Error& e) {
+    if (e.code != LBK_ERR_ALLOC) throw;
+    return false;
+  }
+  int* words             = reinterpret_cast<int*>(room + o_words);  // counts, cursors, too many
   int* too_many          = words + 2 * F;
-  LBK_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * (2 * static_cast<size_t>(F) + 1), stream));
+  int* off               = reinterpret_cast<int*>(room + o_off);
+  T* lists               = reinterpret_cast<T*>(room + o_lists);
+  T* cuts                = reinterpret_cast<T*>(room + o_cuts);
+  unsigned* lut          = reinterpret_cast<unsigned*>(room + o_lut);
+  RankTable* tables      = reinterpret_cast<RankTable*>(room + o_tables);
+  unsigned char* records = room + o_records;
+  unsigned* ranks        = reinterpret_cast<unsigned*>(room + o_ranks);
+  LBK_CUDA(cudaMemsetAsync(words, 0, words_bytes, stream));
   k_rank_count<T><<<n_trees, 256, 0, stream>>>(d_trees, F, words);
   LBK_LAUNCH_CHECK();
   k_rank_scatter<T><<<n_trees, 256, 0, stream>>>(d_trees, F, words, words + F, off, lists);

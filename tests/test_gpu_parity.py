@@ -516,6 +516,37 @@ def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what):
     assert torch.equal(table.predict(wide[:, 1: F + 1], 1, init=init, transform=transform, wait=True), got)
 
 
+def test_predict_without_room_for_ranks(lb):
+    """A caller's allocator that has no 64 MB gets the predictions by the path that needs less."""
+    from legateboost_b200.tree import TreeTable
+
+    rs = np.random.RandomState(1)
+    X, table = dev(rs.random((500_000, 64))), TreeTable(_random_trees(rs, 64, 8, np.arange(64)))
+    want = table.predict(X, 1, wait=True)
+    ctx = lb.library.context(X.device.index)
+    held, refused = {}, []
+
+    def alloc(user, nbytes, stream):
+        if nbytes > 20_000_000:
+            refused.append(nbytes)
+            return None
+        t = torch.empty(int(nbytes), dtype=torch.uint8, device="cuda")
+        held[t.data_ptr()] = t
+        return t.data_ptr()
+
+    def release(user, ptr, stream):
+        held.pop(ptr, None)
+
+    cbs = lb.library.ALLOC_FN(alloc), lb.library.RELEASE_FN(release)
+    ctx.check(ctx.lib.lbk_context_set_allocator(ctx.handle, cbs[0], cbs[1], None))
+    try:
+        got = table.predict(X, 1, wait=True)
+        torch.cuda.synchronize()
+    finally:
+        ctx.use_torch_allocator(False)
+    assert len(refused) == 1 and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("zeros", [False, True])
 @pytest.mark.parametrize("N,F,K,D", [(2500, 600, 2, 8), (2500, 600, 2, 10), (700, 1000, 1, 9)])
 def test_levels_outside_the_cache(lb, oracle, N, F, K, D, zeros):
