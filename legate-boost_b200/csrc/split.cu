@@ -99,10 +99,12 @@ struct SliceBest {
 // is a total order, so the winners do not depend on how the features were cut.
 //
 // What bounds it: on wide levels the issue slots (two float64 divisions per bin, output and node, and a
-// 64-bit scan), on the upper levels the latency of one chain load - scan - division - reduction - claim.
-// A thread per bin and not a warp per feature (four bins per lane): a warp alone on its scheduler gets one
-// instruction in about five clocks, and a feature's 2600 of them were 9 us whatever the level held; and 60
-// registers instead of 128 keep 32 warps on an SM where the level is wide.
+// 64-bit scan), on the upper levels the latency of one chain load - scan - division - reduction - claim, whose loads are
+// asked for before anything is made of the nodes' sums and whose two winners are written by a warp each (200k x 50: 8.7
+// -> 8.2 us a level).  There a thread takes a bin and not a warp a feature: a warp alone on its scheduler gets one
+// instruction in about five clocks, and a feature's instructions were 9 us longer whatever the level held.  On wide levels
+// (ScanIsWide) a warp takes a feature, 32 bins at a time.  Four blocks an SM and not three: 64 features, 8 and 16 units 11.2 and 16.9
+// us instead of 12.8 and 18.4, for spills that cost the upper levels 0.3.
 template <typename T, bool kManyOutputs, bool kDerive, bool kWide>
 __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
   k_scan_split(const __grid_constant__ ScanSplitParams<T> p)
@@ -143,6 +145,13 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
   const GPairI64* par = lv.parent_hist + static_cast<int64_t>((node0 - 1) / 2 - lv.parent_begin) * K * Bs;
   NodeTerms* s_terms  = reinterpret_cast<NodeTerms*>(smem_raw);
   GPairI64* s_carry   = reinterpret_cast<GPairI64*>(smem_raw + (kManyOutputs ? sizeof(NodeTerms) * 2 * ((K + 1) / 2 * 2) : 0));
+  // one output: the first bins are on their way before the nodes' terms are made
+  GPairI64 first_a{0, 0}, first_b{0, 0};
+  if (!kManyOutputs && !kWide && fb + tid < fe) {
+    first_a = LoadPair(src + fb + tid);
+    if (kDerive) first_b = LoadPair(par + fb + tid);
+  }
+  bool first = !kManyOutputs && !kWide;
   NodeTerms ta{}, tb{};
   if (kManyOutputs) {
     for (int i = tid; i < 2 * K; i += kSplitThreads) {
@@ -269,8 +278,9 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
             if (kDerive) ahead_b = LoadPair(par + at + Bs);
           }
         } else {
-          va = in ? LoadPair(src + at) : GPairI64{0, 0};
-          if (kDerive) vb = in && scanned ? LoadPair(par + at) : GPairI64{0, 0};
+          va = first ? first_a : in ? LoadPair(src + at) : GPairI64{0, 0};
+          if (kDerive) vb = first ? first_b : in && scanned ? LoadPair(par + at) : GPairI64{0, 0};
+          first = false;
         }
         long long sg = va.grad, sh = va.hess;
 #pragma unroll
@@ -392,7 +402,8 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
         for (int k = tid; k < K; k += kSplitThreads) StorePair(rec_sums + k, GPairI64{0, 0});
       continue;
     }
-    for (int k = warp; k < K; k += kSplitWarps) {
+    // (one output: a warp per node, so that the loads of either node's winner are on their way together)
+    for (int k = kManyOutputs ? warp : warp == side ? 0 : K; k < K; k += kSplitWarps) {
       const int64_t ko = static_cast<int64_t>(k) * Bs;
       GPairI64 ls;
       if (!kManyOutputs) {
