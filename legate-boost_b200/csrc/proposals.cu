@@ -53,7 +53,7 @@ constexpr int kCountMax = 512;
 template <typename T>
 __host__ __device__ constexpr size_t SortSmem(int S_pad)
 {
-  return S_pad <= kCountMax ? (2 * sizeof(T) + sizeof(int)) * (S_pad < 4 ? 4 : S_pad) : sizeof(T) * S_pad;
+  return S_pad <= kCountMax ? (sizeof(T) + 1) * (S_pad < 4 ? 4 : S_pad) : sizeof(T) * S_pad;
 }
 
 // One block: the S samples of feature f sorted, the distinct ones kept in cuts[f * S ..], the last of them replaced by +inf.
@@ -67,13 +67,11 @@ __device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals 
     return p.draft != nullptr ? p.draft[static_cast<int64_t>(f) * S + i] : SampledValue(p, i, f);
   };
   const int P     = S_pad < 4 ? 4 : S_pad;  // (whole 16-byte words)
-  T* sorted       = vals;
-  const int* mark = nullptr;  // counted: where there is a value
+  const uint8_t* mark = nullptr;  // counted: where there is a value
   if (S_pad <= kCountMax) {
     constexpr int kPer = kCountMax / kSortThreads;
-    sorted    = vals + P;
-    int* here = reinterpret_cast<int*>(sorted + P);
-    mark      = here;
+    uint8_t* here = reinterpret_cast<uint8_t*>(vals + P);
+    mark          = here;
     T mine[kPer];
 #pragma unroll
     for (int u = 0; u < kPer; ++u) {
@@ -90,11 +88,12 @@ __device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals 
 #pragma unroll
     for (int u = 0; u < kPer; ++u)
       below[u] = u == 0 || P > kSortThreads ? CountBelow(vals, P / static_cast<int>(16 / sizeof(T)), mine[u]) : 0;
+    __syncthreads();  // (the places are those of the same array: the sum blocks of the launch want the rest of the SM as L1)
 #pragma unroll
     for (int u = 0; u < kPer; ++u)
       if (tid + u * kSortThreads < S) {
-        sorted[below[u]] = mine[u];
-        here[below[u]]   = 1;
+        vals[below[u]] = mine[u];
+        here[below[u]] = 1;
       }
     __syncthreads();
   } else {
@@ -131,7 +130,7 @@ __device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals 
     int total = before;
     for (int w = 0; w < kSortThreads / 32; ++w) total += s_cnt[w];
     pos += __popc(m & ((1u << lane) - 1u));
-    if (keep) out[pos] = sorted[i];
+    if (keep) out[pos] = vals[i];
     before = total;
     __syncthreads();
   }
