@@ -97,14 +97,14 @@ struct TreeRecord {
 };
 constexpr int kIdBits     = 10;  // feature ids in a word: three of them
 constexpr int kMaxFeature = 1 << kIdBits;
-static TreeRecord RecordOf(int S, size_t elem, bool with_leaves)
+static TreeRecord RecordOf(int S, size_t elem, int leaf_values /* of a leaf; 0: they are elsewhere */)
 {
   auto up16 = [](int v) { return (v + 15) / 16 * 16; };
   TreeRecord r;
   r.S           = S;
   r.split_bytes = up16((1 << S) * static_cast<int>(elem));
   r.word_bytes  = up16((S > 0 ? 2 << ((S - 1) / 2 * 2) : 0) * 4);
-  r.leaf_bytes  = with_leaves ? up16((1 << S) * 8) : 0;
+  r.leaf_bytes  = up16((1 << S) * 8 * leaf_values);
   r.bytes       = r.split_bytes + r.word_bytes + r.leaf_bytes;
   return r;
 }
@@ -240,7 +240,8 @@ struct TiledArgs {
 // Measured against {split, feature} nodes, a block barrier per group, 256 rows per block and every lane reading
 // its own row's values: 10M x 100 float32, 500 trees of depth 8: 23.2 -> 19.5 ms; 1M x 64 float64, 100 trees: 1117 -> 803
 // us; 100003 x 100, 10 outputs, 50 trees: 224 -> 131 us.
-template <typename T, int TG, int KR>
+// kStaged (KR > 0): the leaf values of several outputs are in the records too.
+template <typename T, int TG, int KR, bool kStaged>
 __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledArgs<T> a)
 {
   __shared__ __align__(8) unsigned long long s_bar[4];  // full[2], empty[2]
@@ -423,8 +424,26 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
     if (nt == TG) walk([](int) { return true; });
     else walk([&](int j) { return j < nt; });
     __syncwarp();
-    if (lane == 0) MbarArrive(empty0 + 8 * b);  // this warp is done with the buffer
-    if (KR != 0) {
+    if (!kStaged && lane == 0) MbarArrive(empty0 + 8 * b);  // this warp is done with the buffer
+    if constexpr (kStaged) {
+      const unsigned values = a.rec.split_bytes + a.rec.word_bytes;
+      auto add = [&](auto here) {
+#pragma unroll
+        for (int j = 0; j < TG; ++j) {
+          if (!here(j)) continue;
+          const unsigned v = base[j] + values + ((at[j] - base[j]) / kT - (1u << S)) * (8u * K);  // where the row's values are
+#pragma unroll
+          for (int i = 0; i < kSums; ++i) {
+            const double x = LdsF64(__shfl_sync(0xffffffffu, v, which[i] & 31) + 8u * (which[i] >> 5));
+            acc[i] += x;
+          }
+        }
+      };
+      if (nt == TG) add([](int) { return true; });
+      else add([&](int j) { return j < nt; });
+      __syncwarp();
+      if (lane == 0) MbarArrive(empty0 + 8 * b);
+    } else if (KR != 0) {
       const int64_t tree_values = static_cast<int64_t>(K) << S;
       const double* lf          = a.leaves_c + g * TG * tree_values;
       auto add = [&](auto here) {
@@ -539,60 +558,83 @@ struct TilePlan {
   int rb = 0, tg = 0, nbuf = 0;
   unsigned x_bytes = 0;
   size_t smem      = 0;
+  int64_t waves    = 0;
   TreeRecord rec{};
 };
 constexpr int kRegisterSums    = 16;   // outputs whose sums a warp keeps in registers
+constexpr int kStagedOutputs   = 6;    // from which leaf values may come with the records (PlanTile), ...
+constexpr int kStagedTrees     = 16;   // ... and trees: of fewer the rows are most of the work, which more blocks an SM overlap
 constexpr int kTileStaticBytes = 256;  // (a bound of what the kernel declares)
 
 // The pipe is kept busy by the walks in flight: warps x trees per group.  That product is made as large as shared
 // memory allows, over groups of 8, 4, 2 or 1 trees and 1 to 4 blocks per SM, up to kTileThreads; equal products go to
 // more blocks, of which one stages its rows while another walks.  The rows are then spread evenly over the
 // waves that this takes, so that the last one is not nearly empty.
+//
+// With six to kRegisterSums outputs the leaf values come with the records where a block reads them often enough: a
+// block of rb rows would gather rb x K of a tree's values from L2, sectors of 32 bytes for pieces of 8 K, and brings 2^S x K in
+// one piece instead.  100003 x 100, ten outputs, 50 trees of depth 8: the gathers' 500 MB were most of 124 us, now 107; depth 6,
+// 20000 rows 52 -> 31, 600000 rows of float64 818 -> 631; sixteen outputs, 100003 x 300 float64 658 -> 362.  Small tables stay
+// in L1 where rows come in many waves: depth 4, 600000 rows 401 and 460.
 template <typename T>
 TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, int S, int transform)
 {
-  TilePlan best;
-  int best_score = 0, best_res = 1;
   const size_t row_bytes = sizeof(T) * static_cast<size_t>(F) + (K > kRegisterSums ? 8 * static_cast<size_t>(K) : 0);
   // (the finished rows of a few outputs take the place of X)
   const size_t x_row = K > 1 && K <= kRegisterSums && transform != LBK_RAW ? std::max<size_t>(sizeof(T) * F, 8 * static_cast<size_t>(K)) : sizeof(T) * static_cast<size_t>(F);
   const size_t per_row = std::max(row_bytes, x_row);
-  for (int tg = 8; tg >= 1; tg /= 2) {
-    if (tg > n_trees && tg > 1) continue;  // no wider than the ensemble
-    const TreeRecord rec = RecordOf(S, sizeof(T), K == 1);
-    const int nbuf       = n_trees > tg ? 2 : 1;
-    const size_t trees   = static_cast<size_t>(nbuf) * tg * rec.bytes;
-    for (int res = 1; res <= 4; ++res) {
-      const size_t room = res == 1 ? static_cast<size_t>(ctx->max_smem_optin) - kTileStaticBytes
-                                    : (static_cast<size_t>(ctx->max_smem_optin) + 1024) / res - 1024 - kTileStaticBytes;
-      if (trees + 32 * per_row > room) continue;
-      const int rb    = static_cast<int>(std::min<size_t>((room - trees) / per_row, kTileThreads / res - 32) / 32 * 32);
-      const int score = res * rb / 32 * tg;
-      if (score < best_score || (score == best_score && tg < best.tg)) continue;
-      best_score   = score;
-      best_res     = res;
-      best.rb      = rb;
-      best.tg      = tg;
-      best.nbuf    = nbuf;
-      best.rec     = rec;
+  auto plan = [&](int leaf_values) {
+    TilePlan best;
+    int best_score = 0, best_res = 1;
+    for (int tg = 8; tg >= 1; tg /= 2) {
+      if (tg > n_trees && tg > 1) continue;  // no wider than the ensemble
+      const TreeRecord rec = RecordOf(S, sizeof(T), leaf_values);
+      const int nbuf       = n_trees > tg ? 2 : 1;
+      const size_t trees   = static_cast<size_t>(nbuf) * tg * rec.bytes;
+      for (int res = 1; res <= 4; ++res) {
+        const size_t room = res == 1 ? static_cast<size_t>(ctx->max_smem_optin) - kTileStaticBytes
+                                      : (static_cast<size_t>(ctx->max_smem_optin) + 1024) / res - 1024 - kTileStaticBytes;
+        if (trees + 32 * per_row > room) continue;
+        const int rb    = static_cast<int>(std::min<size_t>((room - trees) / per_row, kTileThreads / res - 32) / 32 * 32);
+        const int score = res * rb / 32 * tg;
+        // (with a table of leaf values per tree, more trees at a time are fewer rows: not for one more wave of them)
+        const int64_t waves = (n_rows + static_cast<int64_t>(rb) * res * ctx->sm_count - 1) / (static_cast<int64_t>(rb) * res * ctx->sm_count);
+        if (leaf_values > 1 && best_score > 0 && waves != best.waves ? waves > best.waves : score < best_score || (score == best_score && tg < best.tg)) continue;
+        best_score   = score;
+        best.waves   = waves;
+        best_res     = res;
+        best.rb      = rb;
+        best.tg      = tg;
+        best.nbuf    = nbuf;
+        best.rec     = rec;
+      }
     }
-  }
-  if (best.rb == 0 || (best_res * best.rb < kTileMinRows && (K > 1 || sizeof(T) * F > kTileOneWarpBytes))) return TilePlan{};
-  const int64_t slots = static_cast<int64_t>(ctx->sm_count) * best_res;
-  const int64_t waves = (n_rows + best.rb * slots - 1) / (best.rb * slots);
-  best.rb             = static_cast<int>(((n_rows + waves * slots - 1) / (waves * slots) + 31) / 32 * 32);
-  best.x_bytes        = static_cast<unsigned>((x_row * best.rb + 15) / 16 * 16);
-  best.smem = best.x_bytes + (K > kRegisterSums ? 8 * static_cast<size_t>(K) * best.rb : 0) + static_cast<size_t>(best.nbuf) * best.tg * best.rec.bytes;
-  return best;
+    if (best.rb == 0 || (best_res * best.rb < kTileMinRows && (K > 1 || sizeof(T) * F > kTileOneWarpBytes))) return TilePlan{};
+    const int64_t slots = static_cast<int64_t>(ctx->sm_count) * best_res;
+    const int64_t waves = (n_rows + best.rb * slots - 1) / (best.rb * slots);
+    best.rb             = static_cast<int>(((n_rows + waves * slots - 1) / (waves * slots) + 31) / 32 * 32);
+    best.x_bytes        = static_cast<unsigned>((x_row * best.rb + 15) / 16 * 16);
+    best.smem = best.x_bytes + (K > kRegisterSums ? 8 * static_cast<size_t>(K) * best.rb : 0) + static_cast<size_t>(best.nbuf) * best.tg * best.rec.bytes;
+    best.waves = waves;
+    return best;
+  };
+  if (K == 1) return plan(1);
+  const TilePlan apart = plan(0);
+  if (K < kStagedOutputs || K > kRegisterSums || n_trees < kStagedTrees || apart.rb == 0) return apart;
+  const TilePlan with = plan(K);
+  return with.rb >= (1 << S) && with.waves <= apart.waves && (S >= 5 || with.waves <= 4) ? with : apart;
 }
 
 template <typename T, int TG, int KR>
 void LaunchTiledAs(lbk_context* ctx, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
+  auto fn = k_predict_tiled<T, TG, KR, false>;
+  if constexpr (KR >= 8)
+    if (a.leaves_c == nullptr) fn = k_predict_tiled<T, TG, KR, true>;
   // (whatever the size: the limit without it is for the static and the dynamic part together)
-  AllowSharedMemory(ctx, k_predict_tiled<T, TG, KR>, kTileStaticBytes);
+  AllowSharedMemory(ctx, fn, kTileStaticBytes);
   const unsigned grid = static_cast<unsigned>((a.n_rows + a.rb - 1) / a.rb);
-  k_predict_tiled<T, TG, KR><<<grid, a.rb + 32, plan.smem, stream>>>(a);
+  fn<<<grid, a.rb + 32, plan.smem, stream>>>(a);
   LBK_LAUNCH_CHECK();
 }
 
@@ -684,7 +726,7 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
     return;
   }
   unsigned char* records = static_cast<unsigned char*>(s.alloc_bytes(static_cast<size_t>(n_trees) * plan.rec.bytes));
-  double* leaves_c       = K == 1 ? nullptr : s.alloc<double>((static_cast<size_t>(n_trees) << S) * K);
+  double* leaves_c       = plan.rec.leaf_bytes > 0 ? nullptr : s.alloc<double>((static_cast<size_t>(n_trees) << S) * K);
   k_pack_complete<T><<<n_trees, 256, 0, stream>>>(d_trees, K, F, plan.rec, records, leaves_c);
   LBK_LAUNCH_CHECK();
   const TiledArgs<T> a{X, ldx, n_rows, F, K, n_trees, plan.rb, plan.nbuf, plan.x_bytes, records, plan.rec, leaves_c, o, ctx->d_status};

@@ -516,6 +516,28 @@ def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what):
     assert torch.equal(table.predict(wide[:, 1: F + 1], 1, init=init, transform=transform, wait=True), got)
 
 
+@pytest.mark.parametrize("N,F,K,T,D,dt", [
+    (20_001, 10, 6, 16, 5, np.float32), (30_000, 33, 10, 50, 8, np.float32), (9_000, 65, 16, 17, 6, np.float64),
+    (12_345, 300, 10, 23, 6, np.float32), (20_000, 7, 12, 40, 3, np.float64), (9_999, 20, 10, 20, 9, np.float32),
+    (20_000, 10, 10, 15, 6, np.float32),  # too few trees for tables of leaf values
+])
+def test_predict_of_several_outputs_by_tables(lb, oracle, N, F, K, T, D, dt):
+    """Leaf values that come with the trees (and shapes around them): the bits of the walk in place, a few rows at a time."""
+    from legateboost_b200 import library as L
+    from legateboost_b200.tree import TreeTable
+
+    rs = np.random.RandomState(N + K)
+    X = dev(rs.random((N, F)).astype(dt))
+    trees = [(dev(rs.normal(size=(t[1].shape[0], K))),) + t[1:] for t in _random_trees(rs, T, D, np.arange(F))]
+    table, init = TreeTable(trees), dev(rs.normal(size=K))
+    for transform in (L.RAW, L.SOFTMAX):
+        got = table.predict(X, K, init=init, transform=transform, wait=True)
+        for rows in (slice(0, 4000), slice(N - 4000, N)):
+            assert torch.equal(got[rows], table.predict(X[rows], K, init=init, transform=transform, wait=True))
+    want = oracle.predict(X[:300].cpu().numpy(), [tuple(a.cpu().numpy() for a in t) for t in trees])
+    assert np.array_equal(table.predict(X, K, wait=True)[:300].cpu().numpy(), want)
+
+
 def test_predict_without_room_for_ranks(lb):
     """A caller's allocator that has no 64 MB gets the predictions by the path that needs less."""
     from legateboost_b200.tree import TreeTable
