@@ -571,16 +571,27 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   // finds out; where it is so, such a level is derived too, from the level above, which is kept up to kHeldHistogramBytes: half
   // of the rows are summed and half of the histograms read.  Level 7 of 1M x 100, ten classes: 808 -> 324 us for the
   // histograms and 391 -> 302 for scan and search; the launch that finds the other answer 4 us.
-  const bool hold = ctx->n_ranks <= 1 && a.trace_hist == nullptr && max_batch > 1;
+  bool hold = ctx->n_ranks <= 1 && a.trace_hist == nullptr && max_batch > 1;
+  const int reference_levels = cache_levels;
   while (hold && cache_levels < D - 1 && LevelEnd(cache_levels + 1) * static_cast<int64_t>(K) * B * static_cast<int64_t>(sizeof(GPairI64)) <= kHeldHistogramBytes)
     ++cache_levels;
-  const int cache_nodes   = LevelEnd(cache_levels);
   const int cache_end_ref = LevelEnd(cdepth);  // extent of the reference's cached histogram
   const size_t node_elems = static_cast<size_t>(K) * B;
   if (cache == nullptr) {
-    const bool last_held = a.trace_hist != nullptr || cache_levels < D - 1 || D <= 1;
-    cache = s.alloc<GPairI64>(static_cast<size_t>(last_held ? cache_nodes : LevelEnd(D - 2)) * node_elems);
+    auto allocate = [&]() {
+      const bool last_held = a.trace_hist != nullptr || cache_levels < D - 1 || D <= 1;
+      cache = s.alloc<GPairI64>(static_cast<size_t>(last_held ? LevelEnd(cache_levels) : LevelEnd(D - 2)) * node_elems);
+    };
+    try {
+      allocate();
+    } catch (const Error& e) {  // (no room for more than the reference keeps: nothing is derived beyond it)
+      if (e.code != LBK_ERR_ALLOC || !hold || cache_levels == reference_levels) throw;
+      hold         = false;
+      cache_levels = reference_levels;
+      allocate();
+    }
   }
+  const int cache_nodes = LevelEnd(cache_levels);
 
   // rows grouped by node, ping-pong; the root's rows are in order and need no list
   int32_t* rows_a = nullptr;

@@ -589,6 +589,40 @@ def test_levels_outside_the_cache(lb, oracle, N, F, K, D, zeros):
         assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
 
 
+def test_levels_outside_the_cache_without_room_for_more(lb):
+    """A caller's allocator that has room for the reference's cache only gets the tree that is built node by node there."""
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.RandomState(4)
+    X, g, h = dev(rs.random((700, 1000)).astype(np.float32)), dev(rs.normal(size=(700, 1))), dev(rs.random((700, 1)) + 0.1)
+    build = lambda: build_tree_arrays(X, g, h, max_depth=10, split_samples=256, seed=5, row_offset=0, dataset_rows=700)
+    want = build()
+    ctx = lb.library.context(X.device.index)
+    held, refused = {}, []
+
+    def alloc(user, nbytes, stream):
+        if nbytes > 1_000_000_000:
+            refused.append(nbytes)
+            return None
+        t = torch.empty(int(nbytes), dtype=torch.uint8, device="cuda")
+        held[t.data_ptr()] = t
+        return t.data_ptr()
+
+    def release(user, ptr, stream):
+        held.pop(ptr, None)
+
+    cbs = lb.library.ALLOC_FN(alloc), lb.library.RELEASE_FN(release)
+    ctx.check(ctx.lib.lbk_context_set_allocator(ctx.handle, cbs[0], cbs[1], None))
+    try:
+        got = build()
+        torch.cuda.synchronize()
+    finally:
+        ctx.use_torch_allocator(False)
+    assert len(refused) == 1
+    for name in ("feature", "split_value", "gain", "hessian", "leaf_value"):
+        assert torch.equal(got[name], want[name]), name
+
+
 def test_golden_trees_on_gpu(lb, oracle):
     """The committed golden inputs: the GPU (quantised) tree must predict within 1e-4 of... itself
     via the oracle's Mode Q, and stay close to the reference CPU tree's training loss."""
