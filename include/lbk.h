@@ -261,6 +261,13 @@ typedef struct lbk_predict_args {
 
 int lbk_predict(lbk_context* ctx, const lbk_predict_args* args);
 
+/* How lbk_predict would be made for more than 8192 rows, for tests of its paths.  out [8]: half the rows per block of the
+ * walk on ranks (0: not on ranks), trees per group, rows whose ranks are held at a time, bytes of the one piece of scratch that
+ * this path takes, where in it the word lies that is not 0 after the call if the device declined the ranks; rows per block of the
+ * tiled walk (0: rows and nodes are read through the caches), trees per group, 1 if leaf values come with the trees. */
+int lbk_selftest_predict_plan(lbk_context* ctx, int64_t n_rows, int n_features, int n_outputs, int n_trees, int max_nodes,
+                              int64_t total_nodes, int x_dtype, int transform, int64_t* out);
+
 /* ------------------------------------------------------------------------------------------
  * Weighted gradients of a boosting round in one pass (reference: LBBase._get_weighted_gradient,
  * legateboost/legateboost.py:189-224, with unit sample weights and no subsampling, over

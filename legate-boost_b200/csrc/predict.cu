@@ -33,6 +33,8 @@
 //   * Predictions are accumulated in float64 in tree order (bit-identical to the reference's
 //     tree-by-tree accumulation), transformed and written once.
 // A fallback kernel with the nodes in global memory covers shapes whose tile or trees do not fit.
+#include <algorithm>
+
 #include "predict.cuh"
 
 namespace lbk {
@@ -69,12 +71,16 @@ __device__ inline void MakeNode(Node16& n, double split, int foff)
   n.pad   = 0;
 }
 
+// Kernels that are queued behind the walk on ranks run where it was declined (PredictRanked); null: always.
+__device__ inline bool SkipFor(const int* gate) { return gate != nullptr && *gate == 0; }
+
 // A split node whose children would fall outside the arrays is treated as a leaf, so a walk can
 // never leave the tree whatever the input arrays hold.
 template <typename NodeT>
-__global__ void k_pack_trees(const TreePtrs* __restrict__ trees, int K, int F, NodeT* __restrict__ nodes,
+__global__ void k_pack_trees(const int* __restrict__ gate, const TreePtrs* __restrict__ trees, int K, int F, NodeT* __restrict__ nodes,
                              double* __restrict__ leaves)
 {
+  if (SkipFor(gate)) return;
   const TreePtrs t = trees[blockIdx.x];
   for (int i = threadIdx.x; i < t.max_nodes; i += blockDim.x) {
     int f = t.feature[i];
@@ -112,9 +118,10 @@ static TreeRecord RecordOf(int S, size_t elem, int leaf_values /* of a leaf; 0: 
 // One block packs one tree.  A node whose children would fall outside the input arrays, or whose feature
 // id is outside [0, F), counts as a leaf, so a walk can never leave the arrays.
 template <typename T>
-__global__ void k_pack_complete(const TreePtrs* __restrict__ trees, int K, int F, TreeRecord rec,
+__global__ void k_pack_complete(const int* __restrict__ gate, const TreePtrs* __restrict__ trees, int K, int F, TreeRecord rec,
                                 unsigned char* __restrict__ records, double* __restrict__ leaves_c)
 {
+  if (SkipFor(gate)) return;
   const TreePtrs t   = trees[blockIdx.x];
   const int M = t.max_nodes, S = rec.S;
   unsigned char* out = records + static_cast<int64_t>(blockIdx.x) * rec.bytes;
@@ -241,8 +248,10 @@ struct TiledArgs {
 // its own row's values: 10M x 100 float32, 500 trees of depth 8: 23.2 -> 19.5 ms; 1M x 64 float64, 100 trees: 1117 -> 803
 // us; 100003 x 100, 10 outputs, 50 trees: 224 -> 131 us.
 // kStaged (KR > 0): the leaf values of several outputs are in the records too.
-template <typename T, int TG, int KR, bool kStaged>
-__global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledArgs<T> a)
+// kGated: the launch stands in for the walk on ranks and does nothing where that was not declined.  A resident block then takes tile
+// after tile: a launch that finds nothing to do ends in 2.5 us, where a block per tile would come and go.
+template <typename T, int TG, int KR, bool kStaged, bool kGated = false>
+__global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledArgs<T> a, const int* __restrict__ gate)
 {
   __shared__ __align__(8) unsigned long long s_bar[4];  // full[2], empty[2]
   __shared__ int s_failed;
@@ -255,244 +264,262 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
   const unsigned full0 = static_cast<unsigned>(__cvta_generic_to_shared(&s_bar[0])), empty0 = full0 + 16;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * rb;
-  const int n_groups = (a.n_trees + TG - 1) / TG;
-  if (tid == 0) {
-    s_failed = 0;
-    for (int b = 0; b < 2; ++b) {
-      MbarInit(full0 + 8 * b, 1);
-      MbarInit(empty0 + 8 * b, rb / 32);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncthreads();
-
-  if (warp == rb / 32) {  // the producer: brings group after group into the buffer that every warp is done with
-    if (lane == 0) {
-      int g   = 0;
-      bool ok = true;
-      for (; g < n_groups && ok; ++g) {
-        const int b = a.nbuf == 2 ? g & 1 : 0;
-        if (g >= 2) ok = MbarWait(empty0 + 8 * b, ((g >> 1) - 1) & 1, a.status, &s_failed);
-        if (!ok) break;
-        const unsigned bytes = min(TG, a.n_trees - g * TG) * rec_bytes;
-        MbarExpectTx(full0 + 8 * b, bytes);
-        BulkCopy(tree0 + b * buf_bytes, a.records + static_cast<int64_t>(g) * buf_bytes, bytes, full0 + 8 * b);
+  if (kGated && *gate == 0) return;
+  int64_t tile   = blockIdx.x;
+  auto next_tile = [&]() {
+    __syncthreads();  // (barriers and tile are made anew)
+    tile += gridDim.x;
+    return s_failed == 0 && tile * rb < a.n_rows;
+  };
+  for (;;) {
+    const int64_t row0 = tile * rb;
+    const int n_groups = (a.n_trees + TG - 1) / TG;
+    if (tid == 0) {
+      s_failed = 0;
+      for (int b = 0; b < 2; ++b) {
+        if (kGated && tile != blockIdx.x) {
+          MbarInval(full0 + 8 * b);
+          MbarInval(empty0 + 8 * b);
+        }
+        MbarInit(full0 + 8 * b, 1);
+        MbarInit(empty0 + 8 * b, rb / 32);
       }
-      // nothing is in flight when the block ends, whatever the other warps waited for
-      for (int h = max(g - 2, 0); h < g; ++h) MbarWait(full0 + 8 * (a.nbuf == 2 ? h & 1 : 0), (h >> 1) & 1, a.status, &s_failed);
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
-    if (s_failed != 0) {  // (the other warps have written what they have)
-      const int columns = a.o.transform == LBK_LOGISTIC ? 2 : K;
-      for (int64_t row = row0 + lane; row < row0 + rb && row < a.n_rows; row += 32)
-        for (int k = 0; k < columns; ++k) a.o.pred[row * a.o.ldp + k] = NAN;
-    }
-    return;
-  }
 
-  // Every thread copies its own row into its own column of the tile and reads nothing else of it, with 16-byte loads; the
-  // sectors of a row are reused from L1 by the following loads of the same thread.  Rows that are not all on 16-byte
-  // boundaries: from the row's first whole vector on, value by value before and behind (all value by value, a pass per row
-  // and load: 1M x 75 float32, 100 trees of depth 8: 884 us, now 543; 1M x 127, 50 trees of depth 6: 712 and 406).  In a
-  // function of its own that path takes 687 and 676; inlined, it costs the float64 kernel 0.6 %.
-  if (row0 + tid < a.n_rows) {
-    const T* xr     = a.X + (row0 + tid) * a.ldx;
-    constexpr int V = 16 / sizeof(T);
-    if ((reinterpret_cast<uintptr_t>(a.X) & 15) == 0 && a.ldx % V == 0) {
-      int f = 0;
-#pragma unroll 8
-      for (; f + V <= F; f += V) {
-        const int4 v = *reinterpret_cast<const int4*>(xr + f);
-#pragma unroll
-        for (int i = 0; i < V; ++i) xs[(f + i) * rb + tid] = reinterpret_cast<const T*>(&v)[i];
+    if (warp == rb / 32) {  // the producer: brings group after group into the buffer that every warp is done with
+      if (lane == 0) {
+        int g   = 0;
+        bool ok = true;
+        for (; g < n_groups && ok; ++g) {
+          const int b = a.nbuf == 2 ? g & 1 : 0;
+          if (g >= 2) ok = MbarWait(empty0 + 8 * b, ((g >> 1) - 1) & 1, a.status, &s_failed);
+          if (!ok) break;
+          const unsigned bytes = min(TG, a.n_trees - g * TG) * rec_bytes;
+          MbarExpectTx(full0 + 8 * b, bytes);
+          BulkCopy(tree0 + b * buf_bytes, a.records + static_cast<int64_t>(g) * buf_bytes, bytes, full0 + 8 * b);
+        }
+        // nothing is in flight when the block ends, whatever the other warps waited for
+        for (int h = max(g - 2, 0); h < g; ++h) MbarWait(full0 + 8 * (a.nbuf == 2 ? h & 1 : 0), (h >> 1) & 1, a.status, &s_failed);
       }
-      for (; f < F; ++f) xs[f * rb + tid] = xr[f];
+      __syncthreads();
+      if (s_failed != 0) {  // (the other warps have written what they have)
+        const int columns = a.o.transform == LBK_LOGISTIC ? 2 : K;
+        for (int64_t at = row0; at < a.n_rows; at += static_cast<int64_t>(gridDim.x) * rb) {  // (gated: the block takes no more tiles)
+          for (int64_t row = at + lane; row < at + rb && row < a.n_rows; row += 32)
+            for (int k = 0; k < columns; ++k) a.o.pred[row * a.o.ldp + k] = NAN;
+          if (!kGated) break;
+        }
+      }
+      if (!kGated || !next_tile()) return;
+      continue;
+    }
+
+    // Every thread copies its own row into its own column of the tile and reads nothing else of it, with 16-byte loads; the
+    // sectors of a row are reused from L1 by the following loads of the same thread.  Rows that are not all on 16-byte
+    // boundaries: from the row's first whole vector on, value by value before and behind (all value by value, a pass per row
+    // and load: 1M x 75 float32, 100 trees of depth 8: 884 us, now 543; 1M x 127, 50 trees of depth 6: 712 and 406).  In a
+    // function of its own that path takes 687 and 676; inlined, it costs the float64 kernel 0.6 %.
+    if (row0 + tid < a.n_rows) {
+      const T* xr     = a.X + (row0 + tid) * a.ldx;
+      constexpr int V = 16 / sizeof(T);
+      if ((reinterpret_cast<uintptr_t>(a.X) & 15) == 0 && a.ldx % V == 0) {
+        int f = 0;
+#pragma unroll 8
+        for (; f + V <= F; f += V) {
+          const int4 v = *reinterpret_cast<const int4*>(xr + f);
+#pragma unroll
+          for (int i = 0; i < V; ++i) xs[(f + i) * rb + tid] = reinterpret_cast<const T*>(&v)[i];
+        }
+        for (; f < F; ++f) xs[f * rb + tid] = xr[f];
+      } else {
+        const int head  = min(F, (V - static_cast<int>(reinterpret_cast<uintptr_t>(xr) / sizeof(T) % V)) % V);
+        const int whole = (F - head) / V;
+#pragma unroll
+        for (int f = 0; f < V - 1; ++f)
+          if (f < head) xs[f * rb + tid] = xr[f];
+        const int4* xv = reinterpret_cast<const int4*>(xr + head);
+        T* column      = xs + head * rb + tid;
+#pragma unroll 8
+        for (int v = 0; v < whole; ++v) {
+          const int4 x = xv[v];
+#pragma unroll
+          for (int i = 0; i < V; ++i) column[(v * V + i) * rb] = reinterpret_cast<const T*>(&x)[i];
+        }
+#pragma unroll
+        for (int i = 0; i < V - 1; ++i) {
+          const int f = head + whole * V + i;
+          if (f < F) xs[f * rb + tid] = xr[f];
+        }
+      }
     } else {
-      const int head  = min(F, (V - static_cast<int>(reinterpret_cast<uintptr_t>(xr) / sizeof(T) % V)) % V);
-      const int whole = (F - head) / V;
-#pragma unroll
-      for (int f = 0; f < V - 1; ++f)
-        if (f < head) xs[f * rb + tid] = xr[f];
-      const int4* xv = reinterpret_cast<const int4*>(xr + head);
-      T* column      = xs + head * rb + tid;
-#pragma unroll 8
-      for (int v = 0; v < whole; ++v) {
-        const int4 x = xv[v];
-#pragma unroll
-        for (int i = 0; i < V; ++i) column[(v * V + i) * rb] = reinterpret_cast<const T*>(&x)[i];
-      }
-#pragma unroll
-      for (int i = 0; i < V - 1; ++i) {
-        const int f = head + whole * V + i;
-        if (f < F) xs[f * rb + tid] = xr[f];
-      }
+      // the walks of the missing rows are made too (any value leads to some leaf) and not written
+      for (int f = 0; f < F; ++f) xs[f * rb + tid] = T(0);
     }
-  } else {
-    // the walks of the missing rows are made too (any value leads to some leaf) and not written
-    for (int f = 0; f < F; ++f) xs[f * rb + tid] = T(0);
-  }
-  if (KR < 0)
-    for (int k = 0; k < K; ++k) accs[k * rb + tid] = 0.0;
+    if (KR < 0)
+      for (int k = 0; k < K; ++k) accs[k * rb + tid] = 0.0;
 
-  // KR > 0: the warp's sums are numbered output innermost, lane l holds l, l + 32, ...
-  constexpr int kSums = KR > 0 ? KR : 1;
-  double acc[kSums];
-  int which[kSums];  // of each: lane (row of the warp) + 32 x output
-#pragma unroll
-  for (int i = 0; i < kSums; ++i) {
-    acc[i] = 0.0;
-    const int r = KR > 0 ? (lane + 32 * i) / K : 0;
-    which[i]    = KR > 0 && i < K ? r + 32 * (lane + 32 * i - r * K) : 0;  // (what is beyond K is read and dropped)
-  }
-
-  // The walk works on 32-bit shared addresses; at[j] is that of the split of tree j's current node.
-  constexpr unsigned kT    = sizeof(T);
-  const unsigned xcol_s    = static_cast<unsigned>(__cvta_generic_to_shared(xs + tid));
-  const unsigned pitch     = static_cast<unsigned>(rb * sizeof(T));
-  const unsigned word_off  = a.rec.split_bytes;
-  const unsigned leaf_off  = a.rec.split_bytes + a.rec.word_bytes - (8u << S);
-  constexpr unsigned kMask = kMaxFeature - 1;
-  for (int g = 0; g < n_groups; ++g) {
-    const int b = a.nbuf == 2 ? g & 1 : 0;
-    if (!__all_sync(0xffffffffu, MbarWait(full0 + 8 * b, (g >> 1) & 1, a.status, &s_failed) ? 1 : 0)) break;
-    const int nt = min(TG, a.n_trees - g * TG);
-    unsigned at[TG], base[TG];
-#pragma unroll
-    for (int j = 0; j < TG; ++j) {
-      base[j] = tree0 + b * buf_bytes + j * rec_bytes;
-      at[j]   = base[j] + kT;
-    }
-    // Two levels of all walks at a time: first every split and word, then every x, then the compares, so that
-    // the loads of the independent walks are in flight together (the loads are volatile and keep
-    // their order).  `here(j)` is always true but in the last group.
-    auto walk = [&](auto here) {
-      T split[TG], x[TG];
-      unsigned w[TG];
-      auto first_loads = [&]() {
-#pragma unroll
-        for (int j = 0; j < TG; ++j)
-          if (here(j)) {
-            w[j]     = LdsU32(kT == 4 ? at[j] + word_off : base[j] + word_off + ((at[j] - base[j]) >> 1));
-            split[j] = LdsX(at[j], T());
-          }
-      };
-      auto x_loads = [&]() {
-#pragma unroll
-        for (int j = 0; j < TG; ++j)
-          if (here(j)) x[j] = LdsX(xcol_s + (w[j] & kMask) * pitch, T());
-      };
-      auto descend = [&](int j) {
-        const bool left = x[j] <= split[j];
-        at[j]           = at[j] + at[j] - base[j];
-        if (!left) at[j] += kT;
-        return left;
-      };
-      int l = 0;
-#pragma unroll 1
-      for (; l + 1 < S; l += 2) {
-        first_loads();
-        x_loads();
-#pragma unroll
-        for (int j = 0; j < TG; ++j)
-          if (here(j)) {
-            w[j] >>= descend(j) ? kIdBits : 2 * kIdBits;
-            split[j] = LdsX(at[j], T());
-          }
-        x_loads();
-#pragma unroll
-        for (int j = 0; j < TG; ++j)
-          if (here(j)) descend(j);
-      }
-      if (l < S) {
-        first_loads();
-        x_loads();
-#pragma unroll
-        for (int j = 0; j < TG; ++j)
-          if (here(j)) descend(j);
-      }
-      if (KR == 0) {
-        double v[TG];
-#pragma unroll
-        for (int j = 0; j < TG; ++j)
-          if (here(j)) v[j] = LdsF64(base[j] + leaf_off + (at[j] - base[j]) * (8u / kT));
-#pragma unroll
-        for (int j = 0; j < TG; ++j)
-          if (here(j)) acc[0] += v[j];
-      }
-    };
-    if (nt == TG) walk([](int) { return true; });
-    else walk([&](int j) { return j < nt; });
-    __syncwarp();
-    if (!kStaged && lane == 0) MbarArrive(empty0 + 8 * b);  // this warp is done with the buffer
-    if constexpr (kStaged) {
-      const unsigned values = a.rec.split_bytes + a.rec.word_bytes;
-      auto add = [&](auto here) {
-#pragma unroll
-        for (int j = 0; j < TG; ++j) {
-          if (!here(j)) continue;
-          const unsigned v = base[j] + values + ((at[j] - base[j]) / kT - (1u << S)) * (8u * K);  // where the row's values are
-#pragma unroll
-          for (int i = 0; i < kSums; ++i) {
-            const double x = LdsF64(__shfl_sync(0xffffffffu, v, which[i] & 31) + 8u * (which[i] >> 5));
-            acc[i] += x;
-          }
-        }
-      };
-      if (nt == TG) add([](int) { return true; });
-      else add([&](int j) { return j < nt; });
-      __syncwarp();
-      if (lane == 0) MbarArrive(empty0 + 8 * b);
-    } else if (KR != 0) {
-      const int64_t tree_values = static_cast<int64_t>(K) << S;
-      const double* lf          = a.leaves_c + g * TG * tree_values;
-      auto add = [&](auto here) {
-#pragma unroll
-        for (int j = 0; j < TG; ++j) {
-          if (!here(j)) continue;
-          const int v = (static_cast<int>((at[j] - base[j]) / kT) - (1 << S)) * K;  // the row's first value
-          if (KR > 0) {
-#pragma unroll
-            for (int i = 0; i < kSums; ++i) acc[i] += __ldg(lf + __shfl_sync(0xffffffffu, v, which[i] & 31) + (which[i] >> 5));
-          } else {
-            for (int k = 0; k < K; ++k) accs[k * rb + tid] += lf[v + k];
-          }
-          lf += tree_values;
-        }
-      };
-      if (nt == TG) add([](int) { return true; });
-      else add([&](int j) { return j < nt; });
-    }
-  }
-
-  const PredictOut& o = a.o;
-  const int64_t row   = row0 + tid;
-  if (KR == 0) {
-    const double raw = o.init ? o.init[0] + acc[0] : acc[0];
-    if (row < a.n_rows) FinishRow(&raw, 1, 1, o.pred + row * o.ldp, o.transform);
-  } else if (KR < 0) {
-    if (o.init)
-      for (int k = 0; k < K; ++k) accs[k * rb + tid] = o.init[k] + accs[k * rb + tid];
-    if (row < a.n_rows) FinishRow(accs + tid, rb, K, o.pred + row * o.ldp, o.transform);
-  } else {
-    double* rows = reinterpret_cast<double*>(smem_raw) + static_cast<int64_t>(warp) * 32 * K;  // of the warp, [32][K]
-    if (o.transform != LBK_RAW) {
-      asm volatile("bar.sync 1, %0;\n" ::"r"(rb) : "memory");  // the walks are done: the rows take the place of X
-#pragma unroll
-      for (int i = 0; i < kSums; ++i)
-        if (i < K) rows[lane + 32 * i] = o.init ? o.init[which[i] >> 5] + acc[i] : acc[i];
-      __syncwarp();
-      FinishRow(rows + lane * K, 1, K, rows + lane * K, o.transform);
-      __syncwarp();
-    }
+    // KR > 0: the warp's sums are numbered output innermost, lane l holds l, l + 32, ...
+    constexpr int kSums = KR > 0 ? KR : 1;
+    double acc[kSums];
+    int which[kSums];  // of each: lane (row of the warp) + 32 x output
 #pragma unroll
     for (int i = 0; i < kSums; ++i) {
-      const int64_t r = row0 + warp * 32 + (which[i] & 31);
-      if (i < K && r < a.n_rows)
-        o.pred[r * o.ldp + (which[i] >> 5)] = o.transform != LBK_RAW ? rows[lane + 32 * i] : o.init ? o.init[which[i] >> 5] + acc[i] : acc[i];
+      acc[i] = 0.0;
+      const int r = KR > 0 ? (lane + 32 * i) / K : 0;
+      which[i]    = KR > 0 && i < K ? r + 32 * (lane + 32 * i - r * K) : 0;  // (what is beyond K is read and dropped)
     }
+
+    // The walk works on 32-bit shared addresses; at[j] is that of the split of tree j's current node.
+    constexpr unsigned kT    = sizeof(T);
+    const unsigned xcol_s    = static_cast<unsigned>(__cvta_generic_to_shared(xs + tid));
+    const unsigned pitch     = static_cast<unsigned>(rb * sizeof(T));
+    const unsigned word_off  = a.rec.split_bytes;
+    const unsigned leaf_off  = a.rec.split_bytes + a.rec.word_bytes - (8u << S);
+    constexpr unsigned kMask = kMaxFeature - 1;
+    for (int g = 0; g < n_groups; ++g) {
+      const int b = a.nbuf == 2 ? g & 1 : 0;
+      if (!__all_sync(0xffffffffu, MbarWait(full0 + 8 * b, (g >> 1) & 1, a.status, &s_failed) ? 1 : 0)) break;
+      const int nt = min(TG, a.n_trees - g * TG);
+      unsigned at[TG], base[TG];
+#pragma unroll
+      for (int j = 0; j < TG; ++j) {
+        base[j] = tree0 + b * buf_bytes + j * rec_bytes;
+        at[j]   = base[j] + kT;
+      }
+      // Two levels of all walks at a time: first every split and word, then every x, then the compares, so that
+      // the loads of the independent walks are in flight together (the loads are volatile and keep
+      // their order).  `here(j)` is always true but in the last group.
+      auto walk = [&](auto here) {
+        T split[TG], x[TG];
+        unsigned w[TG];
+        auto first_loads = [&]() {
+#pragma unroll
+          for (int j = 0; j < TG; ++j)
+            if (here(j)) {
+              w[j]     = LdsU32(kT == 4 ? at[j] + word_off : base[j] + word_off + ((at[j] - base[j]) >> 1));
+              split[j] = LdsX(at[j], T());
+            }
+        };
+        auto x_loads = [&]() {
+#pragma unroll
+          for (int j = 0; j < TG; ++j)
+            if (here(j)) x[j] = LdsX(xcol_s + (w[j] & kMask) * pitch, T());
+        };
+        auto descend = [&](int j) {
+          const bool left = x[j] <= split[j];
+          at[j]           = at[j] + at[j] - base[j];
+          if (!left) at[j] += kT;
+          return left;
+        };
+        int l = 0;
+#pragma unroll 1
+        for (; l + 1 < S; l += 2) {
+          first_loads();
+          x_loads();
+#pragma unroll
+          for (int j = 0; j < TG; ++j)
+            if (here(j)) {
+              w[j] >>= descend(j) ? kIdBits : 2 * kIdBits;
+              split[j] = LdsX(at[j], T());
+            }
+          x_loads();
+#pragma unroll
+          for (int j = 0; j < TG; ++j)
+            if (here(j)) descend(j);
+        }
+        if (l < S) {
+          first_loads();
+          x_loads();
+#pragma unroll
+          for (int j = 0; j < TG; ++j)
+            if (here(j)) descend(j);
+        }
+        if (KR == 0) {
+          double v[TG];
+#pragma unroll
+          for (int j = 0; j < TG; ++j)
+            if (here(j)) v[j] = LdsF64(base[j] + leaf_off + (at[j] - base[j]) * (8u / kT));
+#pragma unroll
+          for (int j = 0; j < TG; ++j)
+            if (here(j)) acc[0] += v[j];
+        }
+      };
+      if (nt == TG) walk([](int) { return true; });
+      else walk([&](int j) { return j < nt; });
+      __syncwarp();
+      if (!kStaged && lane == 0) MbarArrive(empty0 + 8 * b);  // this warp is done with the buffer
+      if constexpr (kStaged) {
+        const unsigned values = a.rec.split_bytes + a.rec.word_bytes;
+        auto add = [&](auto here) {
+#pragma unroll
+          for (int j = 0; j < TG; ++j) {
+            if (!here(j)) continue;
+            const unsigned v = base[j] + values + ((at[j] - base[j]) / kT - (1u << S)) * (8u * K);  // where the row's values are
+#pragma unroll
+            for (int i = 0; i < kSums; ++i) {
+              const double x = LdsF64(__shfl_sync(0xffffffffu, v, which[i] & 31) + 8u * (which[i] >> 5));
+              acc[i] += x;
+            }
+          }
+        };
+        if (nt == TG) add([](int) { return true; });
+        else add([&](int j) { return j < nt; });
+        __syncwarp();
+        if (lane == 0) MbarArrive(empty0 + 8 * b);
+      } else if (KR != 0) {
+        const int64_t tree_values = static_cast<int64_t>(K) << S;
+        const double* lf          = a.leaves_c + g * TG * tree_values;
+        auto add = [&](auto here) {
+#pragma unroll
+          for (int j = 0; j < TG; ++j) {
+            if (!here(j)) continue;
+            const int v = (static_cast<int>((at[j] - base[j]) / kT) - (1 << S)) * K;  // the row's first value
+            if (KR > 0) {
+#pragma unroll
+              for (int i = 0; i < kSums; ++i) acc[i] += __ldg(lf + __shfl_sync(0xffffffffu, v, which[i] & 31) + (which[i] >> 5));
+            } else {
+              for (int k = 0; k < K; ++k) accs[k * rb + tid] += lf[v + k];
+            }
+            lf += tree_values;
+          }
+        };
+        if (nt == TG) add([](int) { return true; });
+        else add([&](int j) { return j < nt; });
+      }
+    }
+
+    const PredictOut& o = a.o;
+    const int64_t row   = row0 + tid;
+    if (KR == 0) {
+      const double raw = o.init ? o.init[0] + acc[0] : acc[0];
+      if (row < a.n_rows) FinishRow(&raw, 1, 1, o.pred + row * o.ldp, o.transform);
+    } else if (KR < 0) {
+      if (o.init)
+        for (int k = 0; k < K; ++k) accs[k * rb + tid] = o.init[k] + accs[k * rb + tid];
+      if (row < a.n_rows) FinishRow(accs + tid, rb, K, o.pred + row * o.ldp, o.transform);
+    } else {
+      double* rows = reinterpret_cast<double*>(smem_raw) + static_cast<int64_t>(warp) * 32 * K;  // of the warp, [32][K]
+      if (o.transform != LBK_RAW) {
+        asm volatile("bar.sync 1, %0;\n" ::"r"(rb) : "memory");  // the walks are done: the rows take the place of X
+#pragma unroll
+        for (int i = 0; i < kSums; ++i)
+          if (i < K) rows[lane + 32 * i] = o.init ? o.init[which[i] >> 5] + acc[i] : acc[i];
+        __syncwarp();
+        FinishRow(rows + lane * K, 1, K, rows + lane * K, o.transform);
+        __syncwarp();
+      }
+#pragma unroll
+      for (int i = 0; i < kSums; ++i) {
+        const int64_t r = row0 + warp * 32 + (which[i] & 31);
+        if (i < K && r < a.n_rows)
+          o.pred[r * o.ldp + (which[i] >> 5)] = o.transform != LBK_RAW ? rows[lane + 32 * i] : o.init ? o.init[which[i] >> 5] + acc[i] : acc[i];
+      }
+    }
+    __syncthreads();  // (the producer's copies)
+    if (!kGated || !next_tile()) return;
   }
-  __syncthreads();  // (the producer's copies)
 }
 
 // The raw sums of an ensemble without trees; nothing of X is read.
@@ -504,8 +531,9 @@ __global__ void __launch_bounds__(256) k_predict_nothing(int64_t n_rows, int K, 
 }
 
 // What is left to do after a kernel that wrote the raw sums.
-__global__ void __launch_bounds__(256) k_finish_rows(int64_t n_rows, int K, PredictOut o)
+__global__ void __launch_bounds__(256) k_finish_rows(const int* __restrict__ gate, int64_t n_rows, int K, PredictOut o)
 {
+  if (SkipFor(gate)) return;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (row >= n_rows) return;
   double* p = o.pred + row * o.ldp;
@@ -515,11 +543,12 @@ __global__ void __launch_bounds__(256) k_finish_rows(int64_t n_rows, int K, Pred
 // Fallback: original (uncompleted) trees, nodes and leaves in global memory, X read directly.
 template <typename T>
 __global__ void __launch_bounds__(128)
-  k_predict_global(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int K, int n_trees,
+  k_predict_global(const int* __restrict__ gate, const T* __restrict__ X, int64_t ldx, int64_t n_rows, int K, int n_trees,
                    const TreePtrs* __restrict__ trees, const typename NodeOf<T>::type* __restrict__ nodes,
                    const double* __restrict__ leaves, PredictOut o)
 {
   using NodeT       = typename NodeOf<T>::type;
+  if (SkipFor(gate)) return;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (row >= n_rows) return;
   const T* xr = X + row * ldx;
@@ -555,7 +584,7 @@ __global__ void __launch_bounds__(128)
 constexpr int kTileMinRows         = 64;
 constexpr size_t kTileOneWarpBytes = 2560;
 struct TilePlan {
-  int rb = 0, tg = 0, nbuf = 0;
+  int rb = 0, tg = 0, nbuf = 0, resident = 1;
   unsigned x_bytes = 0;
   size_t smem      = 0;
   int64_t waves    = 0;
@@ -615,7 +644,8 @@ TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, i
     best.rb             = static_cast<int>(((n_rows + waves * slots - 1) / (waves * slots) + 31) / 32 * 32);
     best.x_bytes        = static_cast<unsigned>((x_row * best.rb + 15) / 16 * 16);
     best.smem = best.x_bytes + (K > kRegisterSums ? 8 * static_cast<size_t>(K) * best.rb : 0) + static_cast<size_t>(best.nbuf) * best.tg * best.rec.bytes;
-    best.waves = waves;
+    best.waves    = waves;
+    best.resident = best_res;
     return best;
   };
   if (K == 1) return plan(1);
@@ -626,49 +656,33 @@ TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, i
 }
 
 template <typename T, int TG, int KR>
-void LaunchTiledAs(lbk_context* ctx, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
+void LaunchTiledAs(lbk_context* ctx, const int* gate, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
   auto fn = k_predict_tiled<T, TG, KR, false>;
   if constexpr (KR >= 8)
     if (a.leaves_c == nullptr) fn = k_predict_tiled<T, TG, KR, true>;
+  int64_t grid = (a.n_rows + a.rb - 1) / a.rb;
+  if constexpr (KR == 0)
+    if (gate != nullptr) {
+      fn   = k_predict_tiled<T, TG, 0, false, true>;
+      grid = std::min<int64_t>(grid, static_cast<int64_t>(ctx->sm_count) * plan.resident);
+    }
   // (whatever the size: the limit without it is for the static and the dynamic part together)
   AllowSharedMemory(ctx, fn, kTileStaticBytes);
-  const unsigned grid = static_cast<unsigned>((a.n_rows + a.rb - 1) / a.rb);
-  fn<<<grid, a.rb + 32, plan.smem, stream>>>(a);
+  fn<<<static_cast<unsigned>(grid), a.rb + 32, plan.smem, stream>>>(a, gate);
   LBK_LAUNCH_CHECK();
 }
 
 template <typename T, int TG>
-void LaunchTiled(lbk_context* ctx, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
+void LaunchTiled(lbk_context* ctx, const int* gate, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
-  if (a.K == 1) LaunchTiledAs<T, TG, 0>(ctx, a, plan, stream);
-  else if (a.K <= 2) LaunchTiledAs<T, TG, 2>(ctx, a, plan, stream);
-  else if (a.K <= 4) LaunchTiledAs<T, TG, 4>(ctx, a, plan, stream);
-  else if (a.K <= 8) LaunchTiledAs<T, TG, 8>(ctx, a, plan, stream);
-  else if (a.K <= 12) LaunchTiledAs<T, TG, 12>(ctx, a, plan, stream);
-  else if (a.K <= kRegisterSums) LaunchTiledAs<T, TG, kRegisterSums>(ctx, a, plan, stream);
-  else LaunchTiledAs<T, TG, -1>(ctx, a, plan, stream);
-}
-
-// One output: is it worth finding the ranks of X first (predict_ranked.cu)?
-//
-// What it gives a million rows and tree, and what it costs them for the ranks, in microseconds; what is left pays for the
-// launches that make the tables (40 to 50) and the sorting of a feature's splits (40 per thousand).  Fitted to both
-// paths over 4 to 150 trees of depth 4 to 10 on 8 to 200 features, random splits.  A million rows, tiled and ranked: float32,
-// 100 features, 150 trees of depth 8 873 and 726 us (10M rows, 500 fitted trees: 19.3 and 13.5 ms), 25 trees of depth 4 202 and
-// 324, 64 features, 150 trees of depth 8 622 and 626; float64, 100 features, 150 trees of depth 8 1334 and 830, 10 of depth 4
-// 394 and 380, 30 features, 10 trees of depth 6 135 and 165.  Twenty thousand rows: 20 to 60 and 45 to 130.
-//
-// Not where one feature might have more splits than there are ranks and the average is not far from that either: the rows
-// would be walked through the caches.
-template <typename T>
-bool RankedPays(int64_t n_rows, int F, int K, int n_trees, int S)
-{
-  if (K != 1 || S < 3) return false;
-  const double millions = static_cast<double>(n_rows) * 1e-6, splits = static_cast<double>(n_trees) * ((1 << S) - 1);
-  if (splits > 32764.0 && splits > 8192.0 * F) return false;
-  const double gain = sizeof(T) == 4 ? n_trees * (0.2 * S - 0.6) - 0.7 * F : n_trees * (0.7 * S - 2.3) + 0.3 * F;
-  return millions * gain > (sizeof(T) == 4 ? 40.0 : 50.0) + 0.04 * splits / F;
+  if (a.K == 1) LaunchTiledAs<T, TG, 0>(ctx, gate, a, plan, stream);
+  else if (a.K <= 2) LaunchTiledAs<T, TG, 2>(ctx, gate, a, plan, stream);
+  else if (a.K <= 4) LaunchTiledAs<T, TG, 4>(ctx, gate, a, plan, stream);
+  else if (a.K <= 8) LaunchTiledAs<T, TG, 8>(ctx, gate, a, plan, stream);
+  else if (a.K <= 12) LaunchTiledAs<T, TG, 12>(ctx, gate, a, plan, stream);
+  else if (a.K <= kRegisterSums) LaunchTiledAs<T, TG, kRegisterSums>(ctx, gate, a, plan, stream);
+  else LaunchTiledAs<T, TG, -1>(ctx, gate, a, plan, stream);
 }
 
 }  // namespace
@@ -681,15 +695,15 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   using NodeT = typename NodeOf<T>::type;
   if (n_rows < 1) return;  // an empty shard returns at once (reference: predict.cu:35)
   const PredictOut o{pred, ldp, init, transform};
-  auto finish = [&]() {
+  auto finish = [&](const int* gate) {
     if (transform == LBK_RAW) return;
-    k_finish_rows<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(n_rows, K, o);
+    k_finish_rows<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(gate, n_rows, K, o);
     LBK_LAUNCH_CHECK();
   };
   if (n_trees == 0) {
     k_predict_nothing<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(n_rows, K, o);
     LBK_LAUNCH_CHECK();
-    finish();
+    finish(nullptr);
     return;
   }
   // Few rows: walk the trees in place.  The tiled kernel brings every tree into shared memory per block (of up to
@@ -710,32 +724,55 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   // a walk through M heap-ordered nodes takes at most S = floor(log2(M)) steps
   int S = 0;
   while ((2 << S) <= m_max) ++S;
-  if (RankedPays<T>(n_rows, F, K, n_trees, S) &&
-      PredictRanked<T>(ctx, s, X, ldx, n_rows, F, n_trees, d_trees, S, total_nodes, init, transform, pred, ldp, stream))
-    return;
   const TilePlan plan = S <= 14 && F <= kMaxFeature ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
+  // (what the rows are walked with where the ranks are declined comes first: without room for it the call fails, with or without ranks)
+  NodeT* nodes = nullptr;
+  double *leaves = nullptr, *leaves_c = nullptr;
+  unsigned char* records = nullptr;
   if (plan.rb == 0) {
-    NodeT* nodes   = s.alloc<NodeT>(total_nodes);
-    double* leaves = s.alloc<double>(total_nodes * K);
-    k_pack_trees<NodeT><<<n_trees, 256, 0, stream>>>(d_trees, K, F, nodes, leaves);
+    nodes  = s.alloc<NodeT>(total_nodes);
+    leaves = s.alloc<double>(total_nodes * K);
+  } else {
+    records = static_cast<unsigned char*>(s.alloc_bytes(static_cast<size_t>(n_trees) * plan.rec.bytes));
+    if (plan.rec.leaf_bytes == 0) leaves_c = s.alloc<double>((static_cast<size_t>(n_trees) << S) * K);
+  }
+  const int* gate = nullptr;
+  if (K == 1) {
+    const RankedPlan ranked = PlanRanked<T>(ctx, n_rows, F, n_trees, S, total_nodes);
+    if (ranked.threads > 0)
+      gate = PredictRanked<T>(ctx, s, ranked, X, ldx, n_rows, F, n_trees, d_trees, S, total_nodes, init, transform, pred, ldp, stream);
+  }
+  if (plan.rb == 0) {
+    k_pack_trees<NodeT><<<n_trees, 256, 0, stream>>>(gate, d_trees, K, F, nodes, leaves);
     LBK_LAUNCH_CHECK();
     const unsigned grid = static_cast<unsigned>((n_rows + 127) / 128);
-    k_predict_global<T><<<grid, 128, 0, stream>>>(X, ldx, n_rows, K, n_trees, d_trees, nodes, leaves, o);
+    k_predict_global<T><<<grid, 128, 0, stream>>>(gate, X, ldx, n_rows, K, n_trees, d_trees, nodes, leaves, o);
     LBK_LAUNCH_CHECK();
-    finish();
+    finish(gate);
     return;
   }
-  unsigned char* records = static_cast<unsigned char*>(s.alloc_bytes(static_cast<size_t>(n_trees) * plan.rec.bytes));
-  double* leaves_c       = plan.rec.leaf_bytes > 0 ? nullptr : s.alloc<double>((static_cast<size_t>(n_trees) << S) * K);
-  k_pack_complete<T><<<n_trees, 256, 0, stream>>>(d_trees, K, F, plan.rec, records, leaves_c);
+  k_pack_complete<T><<<n_trees, 256, 0, stream>>>(gate, d_trees, K, F, plan.rec, records, leaves_c);
   LBK_LAUNCH_CHECK();
   const TiledArgs<T> a{X, ldx, n_rows, F, K, n_trees, plan.rb, plan.nbuf, plan.x_bytes, records, plan.rec, leaves_c, o, ctx->d_status};
   switch (plan.tg) {
-    case 8: LaunchTiled<T, 8>(ctx, a, plan, stream); break;
-    case 4: LaunchTiled<T, 4>(ctx, a, plan, stream); break;
-    case 2: LaunchTiled<T, 2>(ctx, a, plan, stream); break;
-    default: LaunchTiled<T, 1>(ctx, a, plan, stream); break;
+    case 8: LaunchTiled<T, 8>(ctx, gate, a, plan, stream); break;
+    case 4: LaunchTiled<T, 4>(ctx, gate, a, plan, stream); break;
+    case 2: LaunchTiled<T, 2>(ctx, gate, a, plan, stream); break;
+    default: LaunchTiled<T, 1>(ctx, gate, a, plan, stream); break;
   }
+}
+
+// How a call would be made: see lbk.h.
+template <typename T>
+static void PlanOfPredict(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, int m_max, int64_t total_nodes, int transform, int64_t* out)
+{
+  int S = 0;
+  while ((2 << S) <= m_max) ++S;
+  const TilePlan tile     = S <= 14 && F <= kMaxFeature ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
+  const RankedPlan ranked = K == 1 ? PlanRanked<T>(ctx, n_rows, F, n_trees, S, total_nodes) : RankedPlan{};
+  const int64_t words[8]  = {ranked.threads, ranked.tg, ranked.piece, static_cast<int64_t>(ranked.bytes), static_cast<int64_t>(ranked.o_words),
+                             tile.rb, tile.tg, tile.rec.leaf_bytes > 0};
+  std::copy(words, words + 8, out);
 }
 
 template void PredictLaunch<float>(lbk_context*, Scratch&, const float*, int64_t, int64_t, int, int, int, const lbk_tree_ref*,
@@ -744,3 +781,15 @@ template void PredictLaunch<double>(lbk_context*, Scratch&, const double*, int64
                                     const lbk_tree_ref*, int, int64_t, const double*, int, double*, int64_t, cudaStream_t);
 
 }  // namespace lbk
+
+extern "C" int lbk_selftest_predict_plan(lbk_context* ctx, int64_t n_rows, int n_features, int n_outputs, int n_trees, int max_nodes,
+                                         int64_t total_nodes, int x_dtype, int transform, int64_t* out)
+{
+  return lbk::Guard(ctx, [&] {
+    LBK_EXPECT(ctx != nullptr && out != nullptr, "null argument");
+    LBK_EXPECT(x_dtype == LBK_F32 || x_dtype == LBK_F64, "X must be float32 or float64");
+    LBK_EXPECT(n_rows >= 1 && n_features >= 1 && n_outputs >= 1 && n_trees >= 1 && max_nodes >= 1 && total_nodes >= 1, "bad shape");
+    (x_dtype == LBK_F32 ? lbk::PlanOfPredict<float> : lbk::PlanOfPredict<double>)(ctx, n_rows, n_features, n_outputs, n_trees, max_nodes, total_nodes,
+                                                                                 transform, out);
+  });
+}

@@ -14,6 +14,10 @@ __device__ inline void MbarInit(unsigned bar, unsigned count)
 {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
 }
+__device__ inline void MbarInval(unsigned bar)
+{
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
+}
 __device__ inline void MbarExpectTx(unsigned bar, unsigned bytes)
 {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");

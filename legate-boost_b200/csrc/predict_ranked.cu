@@ -4,18 +4,26 @@
 // replaced by its rank among them (how many are smaller), and a split by its own: x <= split if and only if rank(x) <=
 // rank(split).  Ranks fit 16 bits, so that a node - rank and feature - is one 4-byte word for float32 and float64 alike, and
 // the values of two rows share a word of shared memory.  That is worth a pass over X which finds the ranks as soon as the
-// ensemble is large enough (RankedPays): the walks are bound by the load/store data pipe of the SM, and a level is two
+// ensemble is large enough (RanksPay): the walks are bound by the load/store data pipe of the SM, and a level is two
 // passes (node, rank) plus bank conflicts, where k_predict_tiled takes two and a half (float32: split, value, half a
-// word of ids) or five (float64).  Measured against that kernel: 10M x 100 float32, 500 trees of depth 8: 19.3 -> 13.5 ms (2.4
-// of it for the ranks); 1M x 64 float64, 100 trees: 807 -> 531 us (170 for the ranks, 30 for the tables).
+// word of ids) or five (float64).  Measured against that kernel: 10M x 100 float32, 500 trees of depth 8: 19.3 -> 13.4 ms (2.4
+// of it for the ranks); 1M x 64 float64, 100 trees: 807 -> 525 us (170 for the ranks, 65 for the tables and records).
 //
 // Launches:
 //   k_rank_count, k_rank_scatter   the ensemble's splits, feature by feature
-//   k_rank_tables                  sorted, and an index by value into them (a block per feature)
-//   k_rank_pack                    the trees' records, completed to one depth as for k_predict_tiled
+//   k_rank_sort                    sorted, up to kSortChunk of a feature by a block; an index by value into them
+//   k_rank_merge                   features of more than that: the chunks as one table with its index
+//   k_rank_pack                    is it worth it, with the tables as they are?  The trees' records, completed to one depth as for
+//                                  k_predict_tiled
 // then for pieces of the rows that bound the memory of their ranks:
 //   k_rank_rows                    X -> ranks, in the order of the walking blocks' tiles
 //   k_predict_ranked               the walks
+//
+// Boosted ensembles put most splits on a few features, which the host does not see.  A feature with more values than ranks, or
+// tables so uneven that they are searched in many turns over the rows, is known when the tables are made: a device word
+// (`declined`) then turns the kernels that follow into nothing, and the path for every other call, queued behind the same
+// word, runs instead.  1M x 100 float32, 500 trees of depth 8 with 25 % of the splits on one feature: 35.4 ms when every block
+// walked X and the trees where they lie, 2.22 now, 2.13 by k_predict_tiled alone (4M rows: 142, 8.22, 8.06).
 //
 // One output.  Sums are made in tree order in float64, as everywhere.
 #include "predict.cuh"
@@ -24,8 +32,10 @@ namespace lbk {
 namespace {
 
 constexpr int kMaxRank      = 32764;  // entries of a feature's table: ranks 1 .. 32765, one more for a NaN, below 2^15
-constexpr int kSortChunk    = 16384;  // values sorted in shared memory at a time
-constexpr int kMaxChunks    = 16;
+constexpr int kSortChunk    = 4096;   // values that a block sorts
+constexpr int kSortThreads  = 1024;
+constexpr int kMaxChunks    = 32;     // of a feature; with more the ranks are declined unseen
+constexpr int kMaxFeatures  = 1024;
 constexpr int kRankThreads  = 512;    // of k_rank_rows
 constexpr int kRankAhead    = 8;      // rows of a lane whose values are on their way together
 constexpr int kRankTileRows = 32;     // rows of a warp per turn: as many of either half of a tile
@@ -57,67 +67,109 @@ __device__ inline bool SplitAt(const TreePtrs& t, int i, int F, int& f, T& cut)
   return true;
 }
 
+// Splits of a tree by feature, in shared memory [kMaxFeatures] (global atomics of every node took 28 us for 500 trees of depth 8).
 template <typename T>
-__global__ void __launch_bounds__(256) k_rank_count(const TreePtrs* __restrict__ trees, int F, int* __restrict__ counts)
+__device__ inline void CountSplits(const TreePtrs& t, int F, int* s_n)
 {
-  const TreePtrs t = trees[blockIdx.x];
+  for (int f = threadIdx.x; f < F; f += blockDim.x) s_n[f] = 0;
+  __syncthreads();
   for (int i = threadIdx.x; i < t.max_nodes; i += blockDim.x) {
     int f;
     T cut;
-    if (SplitAt(t, i, F, f, cut) && cut == cut) atomicAdd(counts + f, 1);
+    if (SplitAt(t, i, F, f, cut) && cut == cut) atomicAdd(s_n + f, 1);
   }
+  __syncthreads();
 }
 
-// off [F + 1]: where each feature's values begin in `lists`
 template <typename T>
-__global__ void __launch_bounds__(256)
-  k_rank_scatter(const TreePtrs* __restrict__ trees, int F, const int* __restrict__ counts, int* __restrict__ cursor, int* __restrict__ off,
-                 T* __restrict__ lists)
+__global__ void __launch_bounds__(256) k_rank_count(const TreePtrs* __restrict__ trees, int F, int* __restrict__ counts)
 {
-  constexpr int kPer = 4;  // (F <= 1024)
-  __shared__ int s_off[256 * kPer], s_wsum[8];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int c[kPer], sum = 0;
-#pragma unroll
-  for (int i = 0; i < kPer; ++i) {
-    const int f = tid * kPer + i;
-    c[i]        = f < F ? counts[f] : 0;
-    sum += c[i];
-  }
+  __shared__ int s_n[kMaxFeatures];
+  CountSplits<T>(trees[blockIdx.x], F, s_n);
+  for (int f = threadIdx.x; f < F; f += blockDim.x)
+    if (s_n[f] != 0) atomicAdd(counts + f, s_n[f]);
+}
+
+// Exclusive prefix sums of four values per thread of a block of 256; returns what is before the thread's first one.
+__device__ inline int BlockPrefix4(const int (&c)[4], int* s_wsum /* [8] */)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int sum = c[0] + c[1] + c[2] + c[3];
   int incl = sum;
   for (int o = 1; o < 32; o <<= 1) {
     const int v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += v;
   }
+  __syncthreads();
   if (lane == 31) s_wsum[warp] = incl;
   __syncthreads();
   int before = incl - sum;
   for (int w = 0; w < warp; ++w) before += s_wsum[w];
+  return before;
+}
+
+__host__ __device__ inline int ChunksOf(int n) { return n > kSortChunk ? (n + kSortChunk - 1) / kSortChunk : 1; }
+
+// off [F + 1]: where each feature's values begin in `lists`; items [*n_items]: (feature, chunk), the chunks of a feature one after
+// the other, at most kMaxChunks of them (more values: *declined).
+template <typename T>
+__global__ void __launch_bounds__(256)
+  k_rank_scatter(const TreePtrs* __restrict__ trees, int F, const int* __restrict__ counts, int* __restrict__ cursor, int* __restrict__ off,
+                 int2* __restrict__ items, int* __restrict__ n_items, int* __restrict__ declined, T* __restrict__ lists)
+{
+  constexpr int kPer = kMaxFeatures / 256;
+  __shared__ int s_n[kMaxFeatures], s_at[kMaxFeatures], s_wsum[8];
+  const int tid = threadIdx.x;
+  int c[kPer], chunks[kPer];
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
     const int f = tid * kPer + i;
-    s_off[f]    = before;
+    c[i]        = f < F ? counts[f] : 0;
+    chunks[i]   = f < F ? ChunksOf(c[i]) : 0;
+  }
+  int before = BlockPrefix4(c, s_wsum);
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int f = tid * kPer + i;
+    s_at[f]     = before;
     if (blockIdx.x == 0 && f < F) off[f] = before;
     before += c[i];
     if (blockIdx.x == 0 && f == F - 1) off[F] = before;
   }
-  __syncthreads();
+  if (blockIdx.x == 0) {
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+      if (chunks[i] > kMaxChunks) {
+        *declined = 1;
+        chunks[i] = 1;
+      }
+    int at = BlockPrefix4(chunks, s_wsum);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      for (int q = 0; q < chunks[i]; ++q) items[at++] = make_int2(tid * kPer + i, q);
+      if (tid * kPer + i == F - 1) *n_items = at;
+    }
+  }
   const TreePtrs t = trees[blockIdx.x];
+  CountSplits<T>(t, F, s_n);
+  for (int f = tid; f < F; f += blockDim.x)
+    if (s_n[f] != 0) s_at[f] += atomicAdd(cursor + f, s_n[f]);
+  __syncthreads();
   for (int i = tid; i < t.max_nodes; i += blockDim.x) {
     int f;
     T cut;
-    if (SplitAt(t, i, F, f, cut) && cut == cut) lists[s_off[f] + atomicAdd(cursor + f, 1)] = cut;
+    if (SplitAt(t, i, F, f, cut) && cut == cut) lists[atomicAdd(s_at + f, 1)] = cut;
   }
 }
 
-// The first index of n sorted values that is not below v (kUpper: that is above v).
-template <bool kUpper, typename T>
-__device__ inline int BoundOf(const T* a, int n, T v)
+// The first index of n sorted values that is not below v.
+template <typename T>
+__device__ inline int LowerBound(const T* a, int n, T v)
 {
   int lo = 0;
   while (n > 0) {
     const int half = n >> 1;
-    if (kUpper ? !(v < a[lo + half]) : a[lo + half] < v) {
+    if (a[lo + half] < v) {
       lo += half + 1;
       n -= half + 1;
     } else {
@@ -127,125 +179,351 @@ __device__ inline int BoundOf(const T* a, int n, T v)
   return lo;
 }
 
-// A block per feature: its values sorted, equal ones once, and the index.  More values than shared memory holds
-// are sorted in chunks (equal values of different chunks stay, which changes no comparison of ranks) and placed by their
-// ranks in the other chunks.  A feature with more values than ranks sets *too_many.
+// How many of each of kAbreast chunks come before v: those below it and, in the chunks before number `upto`, those equal to it.  In steps of
+// falling powers of two; the chunks' loads are on their way together (a lone search is twelve of them, one after the other).
+constexpr int kAbreast = 8;
 template <typename T>
-__global__ void __launch_bounds__(1024)
-  k_rank_tables(const int* __restrict__ off, T* __restrict__ lists, T* __restrict__ cuts, unsigned* __restrict__ lut,
-                RankTable* __restrict__ tables, int* __restrict__ too_many)
+__device__ inline void CountBefore(const T* lists, const int* len, int first, int chunks, int upto, T v, int (&pos)[kAbreast])
 {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* s = reinterpret_cast<T*>(smem_raw);
-  __shared__ int s_wsum[32], s_len[kMaxChunks];
-  const int f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int begin = off[f], n = off[f + 1] - begin;
-  T* list = lists + begin;
-  T* out  = cuts + begin;
-  const int chunks = (n + kSortChunk - 1) / kSortChunk;
-  int m            = 0;
-  bool fits        = chunks <= kMaxChunks;
-  for (int c = 0; c < chunks && fits; ++c) {
-    const int c0 = c * kSortChunk, len = min(kSortChunk, n - c0);
-    int P = 1;
-    while (P < len) P <<= 1;
-    __syncthreads();
-    for (int i = tid; i < P; i += 1024) s[i] = i < len ? list[c0 + i] : static_cast<T>(INFINITY);
-    for (int k = 2; k <= P; k <<= 1) {
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        // (up to 32 apart, values that meet are of one warp)
-        if (j >= 64 || j == k >> 1) __syncthreads();
-        else if (j == 32) __syncthreads();
-        else __syncwarp();
-        for (int e = tid; e < P / 2; e += 1024) {
-          const int i = 2 * e - (e & (j - 1));  // the e-th index without bit j
-          const T a = s[i], b = s[i + j];
-          if ((i & k) == 0 ? b < a : a < b) {
-            s[i]     = b;
-            s[i + j] = a;
-          }
-        }
-      }
+#pragma unroll
+  for (int u = 0; u < kAbreast; ++u) pos[u] = 0;
+#pragma unroll 1
+  for (int h = kSortChunk; h > 0; h >>= 1) {
+    T x[kAbreast];
+#pragma unroll
+    for (int u = 0; u < kAbreast; ++u) {
+      const int n = first + u < chunks ? len[first + u] : 0;
+      x[u]        = pos[u] + h <= n ? lists[(first + u) * kSortChunk + pos[u] + h - 1] : static_cast<T>(NAN);
     }
-    __syncthreads();
-    // equal values once: to the front of the chunk, or straight to the table
-    T* dst   = chunks == 1 ? out : list + c0;
-    int kept = 0;
-    for (int i0 = 0; i0 < len; i0 += 1024) {
-      const int i      = i0 + tid;
-      const bool keep  = i < len && (i == 0 || s[i] != s[i - 1]);
-      const unsigned b = __ballot_sync(0xffffffffu, keep);
-      if (lane == 0) s_wsum[warp] = __popc(b);
-      __syncthreads();
-      int at = kept + __popc(b & ((1u << lane) - 1u)), all = 0;
-      for (int w = 0; w < 32; ++w) {
-        if (w < warp) at += s_wsum[w];
-        all += s_wsum[w];
-      }
-      if (keep) dst[at] = s[i];
-      kept += all;
-      __syncthreads();
-    }
-    if (tid == 0) s_len[c] = kept;
-    m += kept;
+#pragma unroll
+    for (int u = 0; u < kAbreast; ++u)
+      if (x[u] < v || (first + u < upto && x[u] == v)) pos[u] += h;
   }
-  fits = fits && m <= kMaxRank;
-  if (!fits) {
-    if (tid == 0) {
-      *too_many = 1;
-      tables[f] = RankTable{0.f, 0.f, begin, 0, 1};
-    }
-    return;
-  }
-  __syncthreads();
-  if (chunks > 1) {
-    for (int c = 0; c < chunks; ++c) {
-      for (int i = tid; i < s_len[c]; i += 1024) {
-        const T v = list[c * kSortChunk + i];
-        int at    = i;
-        for (int o = 0; o < chunks; ++o)
-          if (o != c)
-            at += o < c ? BoundOf<true>(list + o * kSortChunk, s_len[o], v) : BoundOf<false>(list + o * kSortChunk, s_len[o], v);
-        out[at] = v;
-      }
-    }
-    __syncthreads();
-  }
-  // the index: buckets of equal width between the first and the last finite value
+}
+
+// What the tables are made from and of.
+template <typename T>
+struct RankTables {
+  const int* off;
+  const int2* items;
+  const int* n_items;
+  int* len;           // [items] distinct values of a chunk
+  int* arrived;       // [F] blocks of k_rank_merge that are done with a feature
+  T* lists;           // [values] as scattered; then the sorted chunks
+  T* cuts;            // [values] the tables
+  unsigned* lut;      // [values] of a bucket: its first value, and in the high half how many it has
+  RankTable* tables;  // [F]
+  int* declined;
+};
+
+// Buckets of equal width between the first and the last finite value.
+template <typename T>
+__device__ inline RankTable IndexOf(T first, T last, int off, int m)
+{
   constexpr float kMax = 3.402823466e38f;
-  RankTable t{0.f, 0.f, begin, m, max(m, 1)};
+  RankTable t{0.f, 0.f, off, m, max(m, 1)};
   if (m > 0) {
-    t.lo           = fmaxf(static_cast<float>(out[0]), -kMax);
-    const float hi = fminf(static_cast<float>(out[m - 1]), kMax);
+    t.lo           = fmaxf(static_cast<float>(first), -kMax);
+    const float hi = fminf(static_cast<float>(last), kMax);
     t.scale        = hi > t.lo ? static_cast<float>(t.nb) / (hi - t.lo) : 0.f;
   }
-  int* start = reinterpret_cast<int*>(list);  // first value of every bucket (the values are in `out`)
-  for (int i = tid; i < m; i += 1024) {
-    const int b      = RankBucket(static_cast<float>(out[i]), t.lo, t.scale, t.nb);
-    const int before = i > 0 ? RankBucket(static_cast<float>(out[i - 1]), t.lo, t.scale, t.nb) : -1;
-    for (int q = before + 1; q <= b; ++q) start[q] = i;
-    if (i == m - 1)
-      for (int q = b + 1; q < t.nb; ++q) start[q] = m;
+  return t;
+}
+// The index of a table whose values lie in `out`, by a block.  start [m]: first value of every bucket (the place of the unsorted values).
+template <typename T>
+__device__ inline void MakeIndex(const RankTable& t, const T* out, int* start, unsigned* lut)
+{
+#pragma unroll 4
+  for (int i = threadIdx.x; i < t.m; i += kSortThreads) {
+    const int b = RankBucket(static_cast<float>(__ldcg(out + i)), t.lo, t.scale, t.nb);
+    const int a = i > 0 ? RankBucket(static_cast<float>(__ldcg(out + i - 1)), t.lo, t.scale, t.nb) : -1;
+    for (int q = a + 1; q <= b; ++q) start[q] = i;
+    if (i == t.m - 1)
+      for (int q = b + 1; q < t.nb; ++q) start[q] = t.m;
   }
   __syncthreads();
-  for (int b = tid; b < m; b += 1024) {
-    const int first = start[b], next = b + 1 < m ? start[b + 1] : m;
-    lut[begin + b]  = static_cast<unsigned>(first) | (static_cast<unsigned>(next - first) << 16);
+#pragma unroll 4
+  for (int b = threadIdx.x; b < t.m; b += kSortThreads) {
+    const int first = __ldcg(start + b), next = b + 1 < t.m ? __ldcg(start + b + 1) : t.m;
+    lut[b]          = static_cast<unsigned>(first) | (static_cast<unsigned>(next - first) << 16);
   }
-  if (tid == 0) tables[f] = t;
 }
+
+// The threads' values that are to be kept, in order, to dst + kept; returns kept and how many there are.
+template <typename T>
+__device__ inline int KeepInOrder(bool keep, T v, T* dst, int kept, int* s_wsum /* [kSortThreads / 32] */)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned b = __ballot_sync(0xffffffffu, keep);
+  if (lane == 0) s_wsum[warp] = __popc(b);
+  __syncthreads();
+  const int n = s_wsum[lane];  // (as many warps as lanes)
+  int incl    = n;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  const int before = __shfl_sync(0xffffffffu, incl - n, warp);
+  if (keep) dst[kept + before + __popc(b & ((1u << lane) - 1u))] = v;
+  kept += __shfl_sync(0xffffffffu, incl, 31);
+  __syncthreads();
+  return kept;
+}
+static_assert(kSortThreads == 1024, "KeepInOrder: as many warps as lanes");
+
+template <typename T>
+__device__ inline void ExchangeLanes(T& v, int j, bool up)
+{
+  const T o = __shfl_xor_sync(0xffffffffu, v, j);
+  if (((threadIdx.x & j) == 0) == up ? o < v : v < o) v = o;
+}
+template <typename T>
+__device__ inline void ExchangePair(T& a, T& b, bool up)
+{
+  if (up ? b < a : a < b) {
+    const T t = a;
+    a         = b;
+    b         = t;
+  }
+}
+
+// P values in shared memory (a power of two, 64 or more), by a bitonic network.  A warp takes 64 neighbours and makes the steps that
+// stay among them in registers: of 2048 values 15 steps of 66 go through shared memory (all of them: 22 us, float64).
+template <typename T>
+__device__ inline void SortShared(T* s, int P)
+{
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __syncthreads();
+  for (int q = warp; 64 * q < P; q += kSortThreads / 32) {
+    T a = s[64 * q + lane], b = s[64 * q + 32 + lane];
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        ExchangeLanes(a, j, k == 32 || (lane & k) == 0);
+        ExchangeLanes(b, j, k != 32 && (lane & k) == 0);
+      }
+    const bool up = (q & 1) == 0;
+    ExchangePair(a, b, up);
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+      ExchangeLanes(a, j, up);
+      ExchangeLanes(b, j, up);
+    }
+    s[64 * q + lane]      = a;
+    s[64 * q + 32 + lane] = b;
+  }
+  for (int k = 128; k <= P; k <<= 1) {
+    for (int j = k >> 1; j >= 64; j >>= 1) {
+      __syncthreads();
+      for (int e = tid; e < P / 2; e += kSortThreads) {
+        const int i = 2 * e - (e & (j - 1));  // the e-th index without bit j
+        T a = s[i], b = s[i + j];
+        ExchangePair(a, b, (i & k) == 0);
+        s[i]     = a;
+        s[i + j] = b;
+      }
+    }
+    __syncthreads();
+    for (int q = warp; 64 * q < P; q += kSortThreads / 32) {
+      T a = s[64 * q + lane], b = s[64 * q + 32 + lane];
+      const bool up = (64 * q & k) == 0;
+      ExchangePair(a, b, up);
+#pragma unroll
+      for (int j = 16; j > 0; j >>= 1) {
+        ExchangeLanes(a, j, up);
+        ExchangeLanes(b, j, up);
+      }
+      s[64 * q + lane]      = a;
+      s[64 * q + 32 + lane] = b;
+    }
+  }
+  __syncthreads();
+}
+
+// A block per chunk: its values sorted, equal ones once.  A feature of one chunk has its table then.
+template <typename T>
+__global__ void __launch_bounds__(kSortThreads) k_rank_sort(const RankTables<T> a)
+{
+  __shared__ T s[kSortChunk];
+  __shared__ int s_wsum[kSortThreads / 32];
+  if (*a.declined != 0 || static_cast<int>(blockIdx.x) >= *a.n_items) return;
+  const int2 item = a.items[blockIdx.x];
+  const int f = item.x, tid = threadIdx.x;
+  const int begin = a.off[f], n = a.off[f + 1] - begin, c0 = item.y * kSortChunk, len = min(kSortChunk, n - c0);
+  T* list = a.lists + begin + c0;
+  int P   = 64;
+  while (P < len) P <<= 1;
+  for (int i = tid; i < P; i += kSortThreads) s[i] = i < len ? list[i] : static_cast<T>(INFINITY);
+  SortShared(s, P);
+  const bool alone = ChunksOf(n) == 1;
+  T* dst           = alone ? a.cuts + begin : list;
+  int m            = 0;
+  for (int i0 = 0; i0 < len; i0 += kSortThreads) {
+    const int i     = i0 + tid;
+    const bool keep = i < len && (i == 0 || s[i] != s[i - 1]);
+    m               = KeepInOrder(keep, keep ? s[i] : T(0), dst, m, s_wsum);
+  }
+  if (tid == 0) a.len[blockIdx.x] = m;
+  if (!alone) return;
+  const RankTable t = IndexOf(m > 0 ? s[0] : T(0), m > 0 ? s[len - 1] : T(0), begin, m);
+  MakeIndex(t, dst, reinterpret_cast<int*>(list), a.lut + begin);
+  if (tid == 0) a.tables[f] = t;
+}
+
+// Features of several chunks.  Every value goes to its place among all of them: its own in its chunk, and how many of each other
+// chunk come before it (equal values in the order of the chunks).  The last block that is done with a feature then drops equal values
+// and makes the index.  A feature with more distinct values than ranks sets *declined.
+template <typename T>
+__global__ void __launch_bounds__(kSortThreads) k_rank_merge(const RankTables<T> a)
+{
+  __shared__ int s_len[kMaxChunks], s_wsum[kSortThreads / 32];
+  __shared__ bool s_last;
+  if (__syncthreads_or(*reinterpret_cast<volatile int*>(a.declined)) || static_cast<int>(blockIdx.x) >= *a.n_items) return;  // (all threads or none)
+  const int2 item = a.items[blockIdx.x];
+  const int f = item.x, tid = threadIdx.x;
+  const int begin = a.off[f], chunks = ChunksOf(a.off[f + 1] - begin), first = blockIdx.x - item.y;
+  if (chunks == 1) return;
+  const T* src = a.lists + begin;
+  T* out       = a.cuts + begin;
+  for (int o = tid; o < chunks; o += kSortThreads) s_len[o] = a.len[first + o];
+  __syncthreads();
+  int all = 0;
+  for (int o = 0; o < chunks; ++o) all += s_len[o];
+  // More than there are ranks, and so few of them twice in a chunk (one in 32: values drawn from 65 thousand) that they will not be
+  // few enough once those of several chunks are dropped: declined now, before 50 us of placing and dropping.
+  if (all > kMaxRank && (a.off[f + 1] - begin - all) * 32 < a.off[f + 1] - begin) {
+    if (tid == 0) *a.declined = 1;
+    return;
+  }
+  const int own = blockIdx.y * kSortThreads + tid;  // (a value per thread)
+  if (own < s_len[item.y]) {
+    const T v = src[item.y * kSortChunk + own];
+    int at    = own;
+    for (int o0 = 0; o0 < chunks; o0 += kAbreast) {
+      int pos[kAbreast];
+      CountBefore(src, s_len, o0, chunks, item.y, v, pos);
+#pragma unroll
+      for (int u = 0; u < kAbreast; ++u)
+        if (o0 + u != item.y) at += pos[u];
+    }
+    out[at] = v;
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(a.arrived + f, 1) == chunks * static_cast<int>(gridDim.y) - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // (kept values move to the front, never beyond what has been read; the next ones are on their way)
+  int m   = 0;
+  T ahead = __ldcg(out + min(tid, all - 1)), ahead_before = __ldcg(out + max(min(tid, all - 1) - 1, 0));
+  for (int i0 = 0; i0 < all; i0 += kSortThreads) {
+    const int i     = i0 + tid, next = min(i + kSortThreads, all - 1);
+    const T v       = ahead;
+    const bool keep = i < all && (i == 0 || v != ahead_before);
+    ahead           = __ldcg(out + next);
+    ahead_before    = __ldcg(out + next - 1);
+    m               = KeepInOrder(keep, v, out, m, s_wsum);
+  }
+  if (m > kMaxRank) {
+    if (tid == 0) *a.declined = 1;
+    return;
+  }
+  const RankTable t = IndexOf(__ldcg(out), __ldcg(out + m - 1), begin, m);
+  MakeIndex(t, out, reinterpret_cast<int*>(a.lists + begin), a.lut + begin);
+  if (tid == 0) a.tables[f] = t;
+}
+
+// ---- turns of k_rank_rows, and what they cost ---------------------------------------------------
+// Bytes of shared memory of the tables of `entries` values.
+template <typename T>
+__host__ __device__ inline unsigned TableBytes(int entries)
+{
+  return static_cast<unsigned>((entries + 1) / 2 * 2) * 4u + static_cast<unsigned>(entries) * sizeof(T);
+}
+// The features of a group that a turn from w0 on takes, those up to the result: as many as have room for their tables; a power
+// of two of them but at the end.  begin [width + 1]: entries before each feature.
+template <typename T>
+__host__ __device__ inline int TurnEnd(const int* begin, int w0, int width, unsigned room)
+{
+  int w1 = w0 + 1;
+  while (w1 < width && TableBytes<T>(begin[w1 + 1] - begin[w0]) <= room) ++w1;
+  if (w1 < width) {
+    int n = 1;
+    while (2 * n <= w1 - w0) n *= 2;
+    w1 = w0 + n;
+  }
+  return w1;
+}
+// Shares of k_rank_rows' blocks: those of a last group of fewer than 32 features stand for this many lanes.  (No less than 16: rows of
+// few features are bound by the sectors that an SM can have on their way.)
+__host__ __device__ inline int TailLanes(int F)
+{
+  int lanes = 16;
+  while (lanes < F - 32 * ((F + 31) / 32 - 1)) lanes *= 2;
+  return lanes;
+}
+
+// Microseconds that k_rank_rows takes for group g of F features, as its tables are: of a turn kTurn and kLane per lane that a row
+// takes, per million rows and with all SMs; kGlobal more for a table that is searched where it lies; kFill per entry brought to shared
+// memory.  Fitted to 50 (float32) and 46 (float64) ensembles of 4 to 511 trees of depth 4 to 10 on 8 to 236 features, up to all
+// splits on one of them, and 83 thousand to 1.7 million rows: 7 and 13 % off (rms).
+template <typename T>
+struct RowsCost {
+  static constexpr float kTurn = sizeof(T) == 4 ? 4.f : 3.f, kLane = sizeof(T) == 4 ? 2.1f : 2.8f, kGlobal = 95.f;
+  static constexpr float kFill = sizeof(T) == 4 ? 0.55e-3f : 0.9e-3f, kLaunch = 8.f;
+  __host__ __device__ static float Group(const int* begin, int g, int F, unsigned room, float millions)
+  {
+    const int last = (F + 31) / 32 - 1, width = g < last ? 32 : F - 32 * last, tail = TailLanes(F);
+    float per_million = 0.f, filled = 0.f;
+    for (int w0 = 0, w1; w0 < width; w0 = w1) {
+      w1 = TurnEnd<T>(begin, w0, width, room);
+      int lanes = 1;
+      while (lanes < w1 - w0) lanes *= 2;
+      per_million += kTurn + kLane * static_cast<float>(lanes);
+      const int entries = begin[w1] - begin[w0];
+      if (TableBytes<T>(entries) <= room) filled += static_cast<float>(entries);
+      else per_million += kGlobal;
+    }
+    const float sms = last == 0 ? 1.f : static_cast<float>(32 * last + tail) / static_cast<float>(g == last ? tail : 32);
+    return millions * sms * per_million + kFill * filled + kLaunch;
+  }
+};
 
 // A completed tree of depth S: words [2^S], nodes counted from 1 (the children of i are 2 i and 2 i + 1), then leaf values
 // [2^S].  A word holds the split's rank in its high half (0: nothing passes, a NaN) and, in its low half, where the
 // feature's ranks begin in a walking block's tile, in units of 128 bytes.
 __host__ __device__ inline int RankRecordBytes(int S) { return 12 << S; }
 
+// Every block finds out for itself, from all tables, whether finding the ranks of `millions` of rows stays within `budget` microseconds.
 template <typename T>
 __global__ void __launch_bounds__(256)
-  k_rank_pack(const TreePtrs* __restrict__ trees, int F, int S, int lines, const RankTable* __restrict__ tables,
-              const T* __restrict__ cuts, const unsigned* __restrict__ lut, const int* __restrict__ too_many, unsigned char* __restrict__ records)
+  k_rank_pack(const TreePtrs* __restrict__ trees, int F, int S, int lines, float millions, float budget, unsigned room, const RankTable* __restrict__ tables,
+              const T* __restrict__ cuts, const unsigned* __restrict__ lut, int* __restrict__ declined, unsigned char* __restrict__ records)
 {
-  if (*too_many != 0) return;  // (a feature has no table)
+  // (a feature has no table; or another block has found the same as this one would: all threads or none)
+  if (__syncthreads_or(*reinterpret_cast<volatile int*>(declined))) return;
+  __shared__ int s_begin[8][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float most = 0.f;
+  for (int g = warp; 32 * g < F; g += 8) {
+    const int width = min(32, F - 32 * g);
+    int incl        = lane < width ? tables[32 * g + lane].nb : 0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    __syncwarp();
+    s_begin[warp][lane + 1] = incl;
+    if (lane == 0) s_begin[warp][0] = 0;
+    __syncwarp();
+    most = fmaxf(most, RowsCost<T>::Group(s_begin[warp], g, F, room, millions));
+  }
+  if (__syncthreads_or(most > budget)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *declined = 1;
+    return;
+  }
   const TreePtrs t   = trees[blockIdx.x];
   unsigned char* out = records + static_cast<int64_t>(blockIdx.x) * RankRecordBytes(S);
   unsigned* words    = reinterpret_cast<unsigned*>(out);
@@ -270,7 +548,7 @@ __global__ void __launch_bounds__(256)
         if (cut == cut) {  // (it is in the table)
           const unsigned e = lut[r.off + RankBucket(static_cast<float>(cut), r.lo, r.scale, r.nb)];
           const int first  = static_cast<int>(e & 0xffffu);
-          rank             = 1 + first + BoundOf<false>(cuts + r.off + first, static_cast<int>(e >> 16), cut);
+          rank             = 1 + first + LowerBound(cuts + r.off + first, static_cast<int>(e >> 16), cut);
         }
         w                 = (static_cast<unsigned>(rank) << 16) | static_cast<unsigned>(f * lines);
       }
@@ -289,7 +567,7 @@ struct RankRowsArgs {
   const RankTable* tables;
   const T* cuts;
   const unsigned* lut;
-  const int* too_many;
+  const int* declined;
   unsigned* out;  // [tile][F][threads]
   int tail_blocks;  // blocks for the last group of features
 };
@@ -408,6 +686,43 @@ __device__ __forceinline__ void RankRows(const RankRowsArgs<T>& a, const RankTab
   }
 }
 
+// The tables of features [w0, w1) of a group to shared memory, by a block; eight entries of a thread at a time: places, then loads, then
+// stores.  (A warp per feature, 32 entries at a time: 50 us for one feature of 20 thousand.  Inlined, or with the two arrays as
+// arguments, the float32 loop over the rows comes out 3 % slower: 10M x 100, 500 trees 300 and 310 us a piece.)
+template <typename T>
+__device__ __noinline__ void FillTables(const RankRowsArgs<T>& a, const int* s_begin, const int* s_from, int w0, int w1, unsigned* s_lut, T* s_cuts)
+{
+  constexpr int kFill = 8;
+  const int base = s_begin[w0], entries = s_begin[w1] - base;
+  for (int i0 = threadIdx.x; i0 < entries; i0 += kFill * kRankThreads) {
+    int from[kFill];  // where the entry lies, -1: of a feature without values, whose only bucket is empty
+    unsigned word[kFill];
+    T cut[kFill];
+#pragma unroll
+    for (int u = 0; u < kFill; ++u) {
+      const int i = base + min(i0 + u * kRankThreads, entries - 1);
+      int e       = w0;  // the feature: the last one that begins at or before the entry
+#pragma unroll
+      for (int h = 16; h > 0; h >>= 1)
+        if (e + h < w1 && s_begin[e + h] <= i) e += h;
+      from[u] = s_from[e] >= 0 ? s_from[e] + i - s_begin[e] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < kFill; ++u) {
+      word[u] = from[u] >= 0 ? __ldg(a.lut + from[u]) : 0u;
+      cut[u]  = from[u] >= 0 ? __ldg(a.cuts + from[u]) : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < kFill; ++u) {
+      const int i = i0 + u * kRankThreads;
+      if (i < entries) {
+        s_lut[i]  = word[u];
+        s_cuts[i] = cut[u];
+      }
+    }
+  }
+}
+
 // X -> ranks.  A block serves one group of 32 features and keeps their tables in shared memory; lane = feature, a warp takes
 // kRankTileRows rows of either half of a tile, turns their ranks in shared memory and writes them as words of two rows.  A
 // last group of fewer features puts several rows side by side in a warp.
@@ -423,7 +738,7 @@ __global__ void __launch_bounds__(kRankThreads, 1) k_rank_rows(const RankRowsArg
 {
   constexpr int kWarps = kRankThreads / 32, kPitch = kRankTileRows + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (*a.too_many != 0) return;
+  if (*a.declined != 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // the block's group of features and its share of the rows
   const int groups = (a.F + 31) / 32, last = groups - 1, blocks = gridDim.x;
@@ -434,7 +749,7 @@ __global__ void __launch_bounds__(kRankThreads, 1) k_rank_rows(const RankRowsArg
   const int f0 = 32 * g, width = min(32, a.F - f0);
   unsigned* turn    = reinterpret_cast<unsigned*>(smem_raw) + warp * 32 * kPitch;  // [feature][rows]: low half, high half
   unsigned* s_table = reinterpret_cast<unsigned*>(smem_raw) + kWarps * 32 * kPitch;
-  __shared__ int s_begin[33], s_from[32];  // entries before the tables of the group's features, and where these lie in `cuts`
+  __shared__ int s_begin[33], s_from[32];  // entries before the tables of the group's features, and where these lie
   if (warp == 0) {
     const RankTable r = a.tables[f0 + min(lane, width - 1)];
     const int m       = lane < width ? max(r.m, 1) : 0;
@@ -450,49 +765,35 @@ __global__ void __launch_bounds__(kRankThreads, 1) k_rank_rows(const RankRowsArg
   unsigned dyn_bytes;
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
   const unsigned room = dyn_bytes - kWarps * 32 * kPitch * 4;
-  auto fits = [&](int entries) { return static_cast<unsigned>((entries + 1) / 2 * 2) * 4u + static_cast<unsigned>(entries) * sizeof(T) <= room; };
   for (int w0 = 0, w1; w0 < width; w0 = w1) {
     __syncthreads();  // (the tables before have been read)
-    // features [w0, w1): as many as have room for their tables; a power of two of them but at the end
-    w1 = w0 + 1;
-    while (w1 < width && fits(s_begin[w1 + 1] - s_begin[w0])) ++w1;
-    if (w1 < width) w1 = w0 + (1 << (31 - __clz(w1 - w0)));
+    w1 = TurnEnd<T>(s_begin, w0, width, room);
     const int n = w1 - w0, entries = s_begin[w1] - s_begin[w0];
     int per_row = 1;  // lanes that a row takes
     while (per_row < n) per_row <<= 1;
     const int sub = lane / per_row, subs = 32 / per_row, fl = lane % per_row, f = w0 + min(fl, n - 1);
     const RankTable t = a.tables[f0 + f];
-    if (fits(entries)) {
+    if (TableBytes<T>(entries) <= room) {
       unsigned* s_lut = s_table;
       T* s_cuts       = reinterpret_cast<T*>(s_lut + (entries + 1) / 2 * 2);
-      for (int e = w0 + warp; e < w1; e += kWarps) {
-        const int from = s_from[e], at = s_begin[e] - s_begin[w0], m = s_begin[e + 1] - s_begin[e];
-#pragma unroll 4
-        for (int i = lane; i < m; i += 32) {
-          s_lut[at + i]  = from >= 0 ? a.lut[from + i] : 0u;
-          s_cuts[at + i] = from >= 0 ? a.cuts[from + i] : T(0);
-        }
-      }
+      FillTables(a, s_begin, s_from, w0, w1, s_lut, s_cuts);
       __syncthreads();
       const int at = s_begin[f] - s_begin[w0];
       RankRows<T, true>(a, t, turn, s_lut + at, s_cuts + at, f0 + w0, n, fl, sub, subs, part, parts);
     } else {
-      // (a feature without values: the zero word says that its only bucket is empty)
-      RankRows<T, false>(a, t, turn, t.m > 0 ? a.lut + t.off : reinterpret_cast<const unsigned*>(a.too_many), a.cuts + t.off, f0 + w0, n, fl, sub, subs, part, parts);
+      // (a feature without values has room: no index would say here that its only bucket is empty)
+      RankRows<T, false>(a, t, turn, a.lut + t.off, a.cuts + t.off, f0 + w0, n, fl, sub, subs, part, parts);
     }
   }
 }
 
-template <typename T>
 struct RankedArgs {
-  const T* X;  // the piece's first row; only read where the tables hold too many values
-  int64_t ldx, n_rows;
+  int64_t n_rows;
   int F, n_trees, S;
   int nbuf;
   const unsigned* ranks;
   const unsigned char* records;
-  const TreePtrs* trees;
-  const int* too_many;
+  const int* declined;
   PredictOut o;  // (of the piece's first row)
   int* status;
 };
@@ -506,32 +807,16 @@ struct RankedArgs {
 //
 // Bound by the load/store pipe: 18 to 22 passes per walk of depth 8 (fitted trees; all nodes split), of which five are the
 // 8-byte leaf value, at 20 to 25 clocks; 84 to 93 % of one pass per clock.
-template <typename T, int TG>
-__global__ void __launch_bounds__(kWalkThreads + 32, 1) k_predict_ranked(const RankedArgs<T> a)
+template <int TG>
+__global__ void __launch_bounds__(kWalkThreads + 32, 1) k_predict_ranked(const RankedArgs a)
 {
   __shared__ __align__(8) unsigned long long s_bar[5];  // full[2], empty[2], the tile
   __shared__ int s_failed;
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  if (*a.declined != 0) return;
   const int F = a.F, S = a.S, threads = blockDim.x - 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t row0 = static_cast<int64_t>(blockIdx.x) * 2 * threads;
-  if (*a.too_many != 0) {
-    // (a feature with more distinct splits than ranks: the walks read X and the trees where they lie)
-    for (int64_t row = row0 + tid; row < row0 + 2 * threads && row < a.n_rows; row += blockDim.x) {
-      const T* x = a.X + row * a.ldx;
-      double sum = 0.0;
-      for (int j = 0; j < a.n_trees; ++j) {
-        const TreePtrs t = a.trees[j];
-        int pos = 0, f;
-        T cut;
-        while (SplitAt(t, pos, F, f, cut)) pos = 2 * pos + 1 + (x[f] <= cut ? 0 : 1);
-        sum += t.leaf[pos];
-      }
-      const double raw = a.o.init ? a.o.init[0] + sum : sum;
-      FinishRow(&raw, 1, 1, a.o.pred + row * a.o.ldp, a.o.transform);
-    }
-    return;
-  }
   const unsigned tile_bytes = static_cast<unsigned>(F) * threads * 4;
   const unsigned rec_bytes = RankRecordBytes(S), buf_bytes = TG * rec_bytes;
   const unsigned tile0 = static_cast<unsigned>(__cvta_generic_to_shared(smem_raw)), tree0 = tile0 + tile_bytes;
@@ -674,109 +959,159 @@ __global__ void __launch_bounds__(kWalkThreads + 32, 1) k_predict_ranked(const R
 
 constexpr int kRankedStatic = 256;  // a bound of what k_predict_ranked declares itself
 
-// Threads and trees per group: what is in flight is threads x trees x 2 walks.
-struct RankedPlan {
-  int threads = 0, tg = 0, nbuf = 0;
-  size_t smem = 0;
-};
-RankedPlan PlanRanked(const lbk_context* ctx, int F, int n_trees, int S)
+constexpr size_t kRankBytes = size_t{256} << 20;  // of a piece of the rows
+constexpr int kRankStatic   = 1024;               // of k_rank_rows
+__host__ inline size_t RowsSmem(const lbk_context* ctx) { return static_cast<size_t>(ctx->max_smem_optin) - kRankStatic; }
+__host__ inline unsigned TableRoom(const lbk_context* ctx)
 {
-  RankedPlan best;
-  int best_score = 0;
-  const size_t room = static_cast<size_t>(ctx->max_smem_optin) - kRankedStatic;
-  for (int tg = 4; tg >= 1; tg /= 2) {
-    if (tg > n_trees && tg > 1) continue;
-    const int nbuf     = n_trees > tg ? 2 : 1;
-    const size_t trees = static_cast<size_t>(nbuf) * tg * RankRecordBytes(S);
-    if (trees + static_cast<size_t>(F) * 128 > room) continue;
-    const int threads = static_cast<int>(std::min<size_t>((room - trees) / (static_cast<size_t>(F) * 4), kWalkThreads) / 32 * 32);
-    const int score   = threads * tg;
-    if (score <= best_score) continue;
-    best_score = score;
-    best       = RankedPlan{threads, tg, nbuf, static_cast<size_t>(F) * threads * 4 + trees};
-  }
-  return best;
+  return static_cast<unsigned>(RowsSmem(ctx) - kRankThreads / 32 * 32 * (kRankTileRows + 1) * 4);
 }
 
 }  // namespace
 
-constexpr size_t kRankBytes = size_t{256} << 20;  // of a piece of the rows
+// Is it worth it, as far as the host can tell?  In microseconds: what k_predict_tiled takes, what the walk on ranks takes (whole waves
+// of tiles), and of the difference, less what the tables take, how much there is for finding the ranks.  The device decides with the tables
+// as they are; here the ensemble's splits are spread evenly over the features.  Not for less than 8 % of the tiled kernel's time,
+// and not where a feature is likely to have more splits than there are ranks.
+//
+// The two lines are fitted to the ensembles of RowsCost (9 and 15 % off).  As it is decided here and on the device, the 69 of them that
+// take k_predict_tiled 100 us or more take 0.95 of that on average, 0.54 at best and 1.11 at worst.
+// Microseconds by k_predict_tiled and as it is decided, a million rows, depth 8, none, 25, 40, 80 % of the splits on one feature:
+// float32, 100 features, 500 trees 2136 and 1788 (on ranks), 2128 and 2218, 2119 and 2203, 2065 and 2150 (declined); float64, 64
+// features, 100 trees 810 and 516, 806 and 562, 800 and 626, 779 and 789 (on ranks).  What declining costs is the tables:
+// 300k x 20 float64, 300 trees, 40 % 520 and 576.
+template <typename T>
+static bool RanksPay(const lbk_context* ctx, int64_t n_rows, int F, int n_trees, int S, int threads, double& budget)
+{
+  const double splits = static_cast<double>(n_trees) * ((1 << S) - 1), millions = static_cast<double>(n_rows) * 1e-6;
+  if (splits > kMaxRank && splits > 8192.0 * F) return false;
+  const int64_t wave  = 2 * static_cast<int64_t>(threads) * ctx->sm_count;
+  const double walked = static_cast<double>((n_rows + wave - 1) / wave * wave) * 1e-6;
+  const double tiled  = millions * (sizeof(T) == 4 ? 1.78 * F + n_trees * (0.577 * S - 0.78) : 4.5 * F + n_trees * (1.03 * S - 2.13)) + 10.0;
+  const double walk   = walked * n_trees * (0.34 * S - 0.75 + 0.53 * kWalkThreads / threads) + millions * 0.3 * F + 6.0;
+  budget              = 0.95 * tiled - walk;
+  int begin[33];
+  for (int i = 0; i <= 32; ++i) begin[i] = i * std::max(1, static_cast<int>(splits / F));
+  float even = 0.f;
+  for (int g : {0, (F + 31) / 32 - 1}) even = std::max(even, RowsCost<T>::Group(begin, g, F, TableRoom(ctx), static_cast<float>(millions)));
+  const double tables = 18.0 + 4.8 * S;
+  return budget > even + tables + 0.03 * tiled;
+}
 
 template <typename T>
-bool PredictRanked(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_t n_rows, int F, int n_trees, const lbk_tree_ref* d_trees, int S,
-                   int64_t total_nodes, const double* init, int transform, double* pred, int64_t ldp, cudaStream_t stream)
+RankedPlan PlanRanked(const lbk_context* ctx, int64_t n_rows, int F, int n_trees, int S, int64_t total_nodes)
 {
-  if (S < 3 || S > 12 || F > 1024 || total_nodes > (int64_t{1} << 28)) return false;
-  const RankedPlan plan = PlanRanked(ctx, F, n_trees, S);
-  if (plan.threads < 128) return false;
+  RankedPlan best;
+  if (S < 3 || S > 12 || F > kMaxFeatures || total_nodes > (int64_t{1} << 28)) return best;
+  int best_score = 0;
+  const size_t smem = static_cast<size_t>(ctx->max_smem_optin) - kRankedStatic;
+  for (int tg = 4; tg >= 1; tg /= 2) {
+    if (tg > n_trees && tg > 1) continue;
+    const int nbuf     = n_trees > tg ? 2 : 1;
+    const size_t trees = static_cast<size_t>(nbuf) * tg * RankRecordBytes(S);
+    if (trees + static_cast<size_t>(F) * 128 > smem) continue;
+    const int threads = static_cast<int>(std::min<size_t>((smem - trees) / (static_cast<size_t>(F) * 4), kWalkThreads) / 32 * 32);
+    const int score   = threads * tg;
+    if (score <= best_score) continue;
+    best_score   = score;
+    best.threads = threads;
+    best.tg      = tg;
+    best.nbuf    = nbuf;
+    best.smem    = static_cast<size_t>(F) * threads * 4 + trees;
+  }
+  if (best.threads < 128 || !RanksPay<T>(ctx, n_rows, F, n_trees, S, best.threads, best.budget)) return RankedPlan{};
   // rows are walked in whole waves of tiles
-  const int64_t tile    = 2 * plan.threads;
-  const int64_t wave    = tile * ctx->sm_count;
-  const int64_t waves   = std::max<int64_t>(1, static_cast<int64_t>(kRankBytes / (static_cast<size_t>(wave) * F * 2)));
-  const int64_t piece   = std::min(waves * wave, (n_rows + tile - 1) / tile * tile);
-  // one piece of scratch, so that a call which has no room for it is left as it was: it takes the other path
-  size_t bytes = 0;
+  const int64_t tile  = 2 * best.threads;
+  const int64_t wave  = tile * ctx->sm_count;
+  const int64_t waves = std::max<int64_t>(1, static_cast<int64_t>(kRankBytes / (static_cast<size_t>(wave) * F * 2)));
+  best.piece          = std::min(waves * wave, (n_rows + tile - 1) / tile * tile);
+  best.max_items      = static_cast<int>(F + total_nodes / 2 / kSortChunk);
   auto reserve = [&](size_t n) {
-    const size_t at = bytes;
-    bytes += (n + 255) / 256 * 256;
+    const size_t at = best.bytes;
+    best.bytes += (n + 255) / 256 * 256;
     return at;
   };
-  const size_t nodes = static_cast<size_t>(total_nodes), words_bytes = sizeof(int) * (2 * static_cast<size_t>(F) + 1);
-  const size_t o_words = reserve(words_bytes), o_off = reserve(sizeof(int) * (static_cast<size_t>(F) + 1));
-  const size_t o_lists = reserve(nodes * sizeof(T)), o_cuts = reserve(nodes * sizeof(T)), o_lut = reserve(nodes * sizeof(unsigned));
-  const size_t o_tables = reserve(sizeof(RankTable) * F), o_records = reserve(static_cast<size_t>(n_trees) * RankRecordBytes(S));
-  const size_t o_ranks  = reserve(static_cast<size_t>(piece / 2) * F * sizeof(unsigned));
-  unsigned char* room   = nullptr;
-  try {
-    room = static_cast<unsigned char*>(s.alloc_bytes(bytes));
+  const size_t nodes = static_cast<size_t>(total_nodes), items = static_cast<size_t>(best.max_items);
+  best.o_words   = reserve(sizeof(int) * (3 * static_cast<size_t>(F) + 2));  // declined, items, counts, cursors, blocks that are done
+  best.o_off     = reserve(sizeof(int) * (static_cast<size_t>(F) + 1));
+  best.o_items   = reserve((sizeof(int2) + sizeof(int)) * items);
+  best.o_lists   = reserve(nodes * sizeof(T));
+  best.o_cuts    = reserve(nodes * sizeof(T));
+  best.o_lut     = reserve(nodes * sizeof(unsigned));
+  best.o_tables  = reserve(sizeof(RankTable) * F);
+  best.o_records = reserve(static_cast<size_t>(n_trees) * RankRecordBytes(S));
+  best.o_ranks   = reserve(static_cast<size_t>(best.piece / 2) * F * sizeof(unsigned));
+  return best;
+}
+
+template <typename T>
+const int* PredictRanked(lbk_context* ctx, Scratch& s, const RankedPlan& plan, const T* X, int64_t ldx, int64_t n_rows, int F, int n_trees,
+                         const lbk_tree_ref* d_trees, int S, int64_t total_nodes, const double* init, int transform, double* pred, int64_t ldp, cudaStream_t stream)
+{
+  unsigned char* room = nullptr;
+  try {  // (one piece, so that a call which has no room for it is left as it was)
+    room = static_cast<unsigned char*>(s.alloc_bytes(plan.bytes));
   } catch (const Error& e) {
     if (e.code != LBK_ERR_ALLOC) throw;
-    return false;
+    return nullptr;
   }
-  int* words             = reinterpret_cast<int*>(room + o_words);  // counts, cursors, too many
-  int* too_many          = words + 2 * F;
-  int* off               = reinterpret_cast<int*>(room + o_off);
-  T* lists               = reinterpret_cast<T*>(room + o_lists);
-  T* cuts                = reinterpret_cast<T*>(room + o_cuts);
-  unsigned* lut          = reinterpret_cast<unsigned*>(room + o_lut);
-  RankTable* tables      = reinterpret_cast<RankTable*>(room + o_tables);
-  unsigned char* records = room + o_records;
-  unsigned* ranks        = reinterpret_cast<unsigned*>(room + o_ranks);
-  LBK_CUDA(cudaMemsetAsync(words, 0, words_bytes, stream));
-  k_rank_count<T><<<n_trees, 256, 0, stream>>>(d_trees, F, words);
+  int* words    = reinterpret_cast<int*>(room + plan.o_words);
+  int* declined = words;
+  int* counts   = words + 2;
+  T* cuts       = reinterpret_cast<T*>(room + plan.o_cuts);
+  RankTables<T> t;
+  t.off      = reinterpret_cast<int*>(room + plan.o_off);
+  t.items    = reinterpret_cast<int2*>(room + plan.o_items);
+  t.n_items  = words + 1;
+  t.len      = reinterpret_cast<int*>(room + plan.o_items + sizeof(int2) * plan.max_items);
+  t.arrived  = counts + 2 * F;
+  t.lists    = reinterpret_cast<T*>(room + plan.o_lists);
+  t.cuts     = cuts;
+  t.lut      = reinterpret_cast<unsigned*>(room + plan.o_lut);
+  t.tables   = reinterpret_cast<RankTable*>(room + plan.o_tables);
+  t.declined = declined;
+  unsigned char* records = room + plan.o_records;
+  unsigned* ranks        = reinterpret_cast<unsigned*>(room + plan.o_ranks);
+  const unsigned items   = static_cast<unsigned>(plan.max_items);
+  LBK_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * (3 * static_cast<size_t>(F) + 2), stream));
+  k_rank_count<T><<<n_trees, 256, 0, stream>>>(d_trees, F, counts);
   LBK_LAUNCH_CHECK();
-  k_rank_scatter<T><<<n_trees, 256, 0, stream>>>(d_trees, F, words, words + F, off, lists);
+  k_rank_scatter<T><<<n_trees, 256, 0, stream>>>(d_trees, F, counts, counts + F, const_cast<int*>(t.off), const_cast<int2*>(t.items), words + 1, declined, t.lists);
   LBK_LAUNCH_CHECK();
-  AllowSharedMemory(ctx, k_rank_tables<T>, 1024);
-  k_rank_tables<T><<<F, 1024, kSortChunk * sizeof(T), stream>>>(off, lists, cuts, lut, tables, too_many);
+  k_rank_sort<T><<<items, kSortThreads, 0, stream>>>(t);
   LBK_LAUNCH_CHECK();
-  k_rank_pack<T><<<n_trees, 256, 0, stream>>>(d_trees, F, S, plan.threads / 32, tables, cuts, lut, too_many, records);
+  if (total_nodes / 2 > kSortChunk) {
+    k_rank_merge<T><<<dim3(items, kSortChunk / kSortThreads), kSortThreads, 0, stream>>>(t);
+    LBK_LAUNCH_CHECK();
+  }
+  k_rank_pack<T><<<n_trees, 256, 0, stream>>>(d_trees, F, S, plan.threads / 32, static_cast<float>(n_rows) * 1e-6f, static_cast<float>(plan.budget), TableRoom(ctx), t.tables, cuts, t.lut, declined, records);
   LBK_LAUNCH_CHECK();
-  AllowSharedMemory(ctx, k_rank_rows<T>, 1024);
-  const int groups = (F + 31) / 32;
-  int lanes        = 16;  // (no less: rows of few features are bound by the sectors an SM can have on their way)
-  while (lanes < F - 32 * (groups - 1)) lanes *= 2;
+  AllowSharedMemory(ctx, k_rank_rows<T>, kRankStatic);
+  const int64_t tile    = 2 * plan.threads;
+  const int groups      = (F + 31) / 32;
+  const int lanes       = TailLanes(F);
   const int blocks      = std::max(ctx->sm_count, groups);
   const int tail_blocks = groups == 1 ? blocks
                                       : std::min(blocks - (groups - 1), std::max(1, (blocks * lanes + 16 * (groups - 1) + lanes / 2) / (32 * (groups - 1) + lanes)));
-  auto walk = plan.tg == 4 ? k_predict_ranked<T, 4> : plan.tg == 2 ? k_predict_ranked<T, 2> : k_predict_ranked<T, 1>;
+  auto walk = plan.tg == 4 ? k_predict_ranked<4> : plan.tg == 2 ? k_predict_ranked<2> : k_predict_ranked<1>;
   AllowSharedMemory(ctx, walk, kRankedStatic);
-  const size_t rank_smem = static_cast<size_t>(ctx->max_smem_optin) - 1024;
-  for (int64_t r0 = 0; r0 < n_rows; r0 += piece) {
-    const int64_t rows = std::min(piece, n_rows - r0), tiles = (rows + tile - 1) / tile;
-    RankRowsArgs<T> ra{X + r0 * ldx, ldx, rows, F, plan.threads, tiles, tables, cuts, lut, too_many, ranks, tail_blocks};
-    k_rank_rows<T><<<blocks, kRankThreads, rank_smem, stream>>>(ra);
+  for (int64_t r0 = 0; r0 < n_rows; r0 += plan.piece) {
+    const int64_t rows = std::min(plan.piece, n_rows - r0), tiles = (rows + tile - 1) / tile;
+    RankRowsArgs<T> ra{X + r0 * ldx, ldx, rows, F, plan.threads, tiles, t.tables, cuts, t.lut, declined, ranks, tail_blocks};
+    k_rank_rows<T><<<blocks, kRankThreads, RowsSmem(ctx), stream>>>(ra);
     LBK_LAUNCH_CHECK();
-    RankedArgs<T> wa{X + r0 * ldx, ldx, rows, F, n_trees, S, plan.nbuf, ranks, records, d_trees, too_many, PredictOut{pred + r0 * ldp, ldp, init, transform}, ctx->d_status};
+    RankedArgs wa{rows, F, n_trees, S, plan.nbuf, ranks, records, declined, PredictOut{pred + r0 * ldp, ldp, init, transform}, ctx->d_status};
     walk<<<static_cast<unsigned>(tiles), plan.threads + 32, plan.smem, stream>>>(wa);
     LBK_LAUNCH_CHECK();
   }
-  return true;
+  return declined;
 }
 
-template bool PredictRanked<float>(lbk_context*, Scratch&, const float*, int64_t, int64_t, int, int, const lbk_tree_ref*, int, int64_t,
-                                   const double*, int, double*, int64_t, cudaStream_t);
-template bool PredictRanked<double>(lbk_context*, Scratch&, const double*, int64_t, int64_t, int, int, const lbk_tree_ref*, int, int64_t,
-                                    const double*, int, double*, int64_t, cudaStream_t);
+#define LBK_PREDICT_RANKED(T)                                                                                                                  \
+  template RankedPlan PlanRanked<T>(const lbk_context*, int64_t, int, int, int, int64_t);                                                      \
+  template const int* PredictRanked<T>(lbk_context*, Scratch&, const RankedPlan&, const T*, int64_t, int64_t, int, int, const lbk_tree_ref*,    \
+                                       int, int64_t, const double*, int, double*, int64_t, cudaStream_t);
+LBK_PREDICT_RANKED(float)
+LBK_PREDICT_RANKED(double)
 
 }  // namespace lbk

@@ -20,7 +20,7 @@ EXPORTS = [
     "lbk_version", "lbk_context_create", "lbk_context_destroy", "lbk_last_error", "lbk_context_trim",
     "lbk_context_set_allocator", "lbk_context_pool_bytes", "lbk_context_lent_words",
     "lbk_comm_unique_id", "lbk_comm_init", "lbk_comm_attach_nccl", "lbk_comm_set_callback",
-    "lbk_comm_size", "lbk_owned_features", "lbk_selftest_peer_barrier", "lbk_profile_enable", "lbk_profile_histogram_ms", "lbk_profile_histogram_total", "lbk_build_tree", "lbk_boost_round", "lbk_synchronize", "lbk_sketch_bytes", "lbk_leaf_values", "lbk_update_tree", "lbk_gradient", "lbk_predict", "lbk_split_proposals", "lbk_bin_matrix",
+    "lbk_comm_size", "lbk_owned_features", "lbk_selftest_peer_barrier", "lbk_profile_enable", "lbk_profile_histogram_ms", "lbk_profile_histogram_total", "lbk_build_tree", "lbk_boost_round", "lbk_synchronize", "lbk_sketch_bytes", "lbk_leaf_values", "lbk_update_tree", "lbk_gradient", "lbk_predict", "lbk_selftest_predict_plan", "lbk_split_proposals", "lbk_bin_matrix",
     "lbk_bin_matrix_bytes", "lbk_quantise", "lbk_histogram", "lbk_selftest_histogram", "lbk_histogram_noalloc", "lbk_group_rows",
 ]
 
@@ -141,6 +141,7 @@ def load():
             lib.lbk_boost_round.argtypes = [C.c_void_p, C.POINTER(BoostRoundArgs)]
             lib.lbk_synchronize.argtypes = [C.c_void_p, C.c_void_p]
             lib.lbk_predict.argtypes = [C.c_void_p, C.POINTER(PredictArgs)]
+            lib.lbk_selftest_predict_plan.argtypes = [C.c_void_p, C.c_int64] + [C.c_int] * 4 + [C.c_int64, C.c_int, C.c_int, C.POINTER(C.c_int64)]
             lib.lbk_histogram.argtypes = [C.c_void_p, C.POINTER(HistogramArgs)]
             lib.lbk_selftest_histogram.argtypes = [C.c_void_p, C.POINTER(HistogramArgs)]
             lib.lbk_histogram_noalloc.argtypes = [C.c_int, C.POINTER(HistogramArgs)]

@@ -473,19 +473,54 @@ def _random_trees(rs, T, D, features, odd=False):
     return trees
 
 
-@pytest.mark.parametrize("N,F,T,D,dt,used,what", [
-    (1_000_001, 100, 130, 8, np.float32, None, "odd"),     # a last group of four features, a ragged last tile
-    (1_200_003, 33, 200, 5, np.float32, None, "odd"),    # a last group of one feature; several pieces of rows
-    (300_000, 64, 64, 8, np.float64, None, "odd"),
-    (1_200_001, 9, 70, 10, np.float64, None, "odd"),       # tables of a group in several turns
-    (4_000_000, 1, 60, 4, np.float64, None, ""),         # one feature
-    (300_000, 150, 50, 11, np.float64, None, ""),        # one tree per group
-    (400_000, 20, 100, 8, np.float64, [3], ""),          # all splits on one feature: sorted in chunks, no room for the table
-    (300_000, 20, 150, 8, np.float64, [3], "logistic"),  # ... more of them than there are ranks
+def _predict_plan(lb, table, X, K, transform):
+    """How a prediction is made (lbk_selftest_predict_plan)."""
+    import ctypes
+    from legateboost_b200 import library as L
+
+    ctx, out = L.context(X.device.index), (ctypes.c_int64 * 8)()
+    ctx.check(ctx.lib.lbk_selftest_predict_plan(ctx.handle, X.shape[0], X.shape[1], K, table.n_trees, table.max_nodes, table.total_nodes,
+                                                L.LBK_F32 if X.dtype == torch.float32 else L.LBK_F64, transform, out))
+    return dict(zip(("threads", "group", "piece", "bytes", "word", "tile_rows", "tile_group", "leaves_with_trees"), out))
+
+
+def _predict_and_word(lb, table, X, plan, **kw):
+    """A prediction whose scratch stays here, and the word in it that says whether the device declined the ranks."""
+    ctx, held = lb.library.context(X.device.index), []
+
+    def alloc(user, nbytes, stream):
+        held.append(torch.empty(int(nbytes), dtype=torch.uint8, device="cuda"))
+        return held[-1].data_ptr()
+
+    cbs = lb.library.ALLOC_FN(alloc), lb.library.RELEASE_FN(lambda user, ptr, stream: None)
+    ctx.check(ctx.lib.lbk_context_set_allocator(ctx.handle, cbs[0], cbs[1], None))
+    try:
+        got = table.predict(X, 1, wait=True, **kw)
+        torch.cuda.synchronize()
+    finally:
+        ctx.use_torch_allocator(False)
+    room, = [t for t in held if t.numel() == plan["bytes"]]
+    return got, int(room[plan["word"]: plan["word"] + 4].view(torch.int32))
+
+
+@pytest.mark.parametrize("N,F,T,D,dt,used,what,group,pieces,declined", [
+    (1_000_001, 100, 300, 8, np.float32, None, "odd", 4, 1, False),     # a last group of four features, a ragged last tile
+    (1_600_003, 100, 300, 8, np.float32, None, "odd", 4, 2, False),     # rows in two pieces
+    (1_300_003, 33, 200, 5, np.float64, None, "odd", 4, 1, False),      # a last group of one feature
+    (1_200_001, 9, 70, 10, np.float64, None, "odd", 4, 1, False),       # tables of a group in several turns
+    (4_000_000, 1, 60, 4, np.float64, None, "", 4, 1, False),           # one feature
+    (600_000, 150, 60, 11, np.float64, None, "", 2, 1, False),          # two trees per group
+    (600_000, 150, 60, 12, np.float64, None, "", 1, 1, False),          # one
+    (400_000, 20, 100, 8, np.float64, [3], "", 4, 1, False),            # all splits on one feature, in chunks; no room for the table
+    (400_000, 20, 300, 8, np.float64, [3], "few", 4, 1, False),         # more than there are ranks, of which many are equal
+    (300_000, 20, 300, 8, np.float64, [3], "logistic", 4, 1, True),     # more of them than there are ranks
+    (1_000_001, 100, 300, 8, np.float32, "3", "odd", 4, 1, True),       # one large table: the ranks would cost more than they give
+    (200_000, 330, 300, 8, np.float64, None, "logistic", 4, 1, False),  # rows too wide for the tiled walk
+    (200_000, 330, 300, 8, np.float64, [3], "logistic", 4, 1, True),    # ... which are then read through the caches
 ])
-def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what):
-    """Large ensembles of one output are walked on ranks (RankedPays says so for all of these); a few rows at a time, where
-    the trees are walked where they lie, give the same bits."""
+def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what, group, pieces, declined):
+    """Large ensembles of one output are walked on ranks, if the device does not find their tables too dear; a few rows at a
+    time, where the trees are walked where they lie, give the same bits."""
     from legateboost_b200 import library as L
     from legateboost_b200.tree import TreeTable
 
@@ -496,12 +531,23 @@ def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what):
         for value in (np.nan, np.inf, -np.inf):
             X[rs.randint(N, size=3000), rs.randint(F, size=3000)] = value
         X[-40:] = np.nan
+    if used == "3":  # of three splits two
+        used = np.concatenate([np.arange(F), np.full(2 * F, 3)])
     trees = _random_trees(rs, T, D, np.arange(F) if used is None else used, what == "odd")
+    if what == "few":
+        pool = dev(rs.random(20_000))
+        trees = [(v, f, pool[(s * 20_000).long().clamp(0, 19_999)]) for v, f, s in trees]
     table, transform = TreeTable(trees), L.LOGISTIC if what == "logistic" else L.RAW
     init = dev(np.array([0.25])) if what else None
     dX = dev(X)
-    got = table.predict(dX, 1, init=init, transform=transform, wait=True)
-    picks = [np.arange(5000), np.arange(N - 5000, N), np.sort(rs.choice(N, 8000, replace=False))]
+    plan = _predict_plan(lb, table, dX, 1, transform)
+    assert plan["threads"] > 0 and plan["group"] == group and -(-N // plan["piece"]) == pieces
+    assert (plan["tile_rows"] == 0) == (F > 320)
+    got, word = _predict_and_word(lb, table, dX, plan, init=init, transform=transform)
+    assert (word != 0) == declined
+    assert torch.equal(table.predict(dX, 1, init=init, transform=transform, wait=True), got)
+    edge = min(plan["piece"], N)
+    picks = [np.arange(5000), np.arange(N - 5000, N), np.sort(rs.choice(N, 8000, replace=False)), np.arange(edge - 4000, min(edge + 4000, N))]
     for rows in picks:
         rows = dev(rows)
         few = table.predict(dX[rows].contiguous(), 1, init=init, transform=transform, wait=True)
@@ -516,12 +562,13 @@ def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what):
     assert torch.equal(table.predict(wide[:, 1: F + 1], 1, init=init, transform=transform, wait=True), got)
 
 
-@pytest.mark.parametrize("N,F,K,T,D,dt", [
-    (20_001, 10, 6, 16, 5, np.float32), (30_000, 33, 10, 50, 8, np.float32), (9_000, 65, 16, 17, 6, np.float64),
-    (12_345, 300, 10, 23, 6, np.float32), (20_000, 7, 12, 40, 3, np.float64), (9_999, 20, 10, 20, 9, np.float32),
-    (20_000, 10, 10, 15, 6, np.float32),  # too few trees for tables of leaf values
+@pytest.mark.parametrize("N,F,K,T,D,dt,with_trees", [
+    (20_001, 10, 6, 16, 5, np.float32, True), (100_003, 100, 10, 50, 8, np.float32, True), (9_000, 65, 16, 17, 6, np.float64, True),
+    (12_345, 300, 10, 23, 6, np.float32, True), (20_000, 7, 12, 40, 3, np.float64, True),
+    (30_000, 33, 10, 50, 8, np.float32, False), (9_999, 20, 10, 20, 9, np.float32, False),  # fewer rows in a block than a tree has leaves
+    (20_000, 10, 10, 15, 6, np.float32, False),  # too few trees
 ])
-def test_predict_of_several_outputs_by_tables(lb, oracle, N, F, K, T, D, dt):
+def test_predict_of_several_outputs_by_tables(lb, oracle, N, F, K, T, D, dt, with_trees):
     """Leaf values that come with the trees (and shapes around them): the bits of the walk in place, a few rows at a time."""
     from legateboost_b200 import library as L
     from legateboost_b200.tree import TreeTable
@@ -531,6 +578,7 @@ def test_predict_of_several_outputs_by_tables(lb, oracle, N, F, K, T, D, dt):
     trees = [(dev(rs.normal(size=(t[1].shape[0], K))),) + t[1:] for t in _random_trees(rs, T, D, np.arange(F))]
     table, init = TreeTable(trees), dev(rs.normal(size=K))
     for transform in (L.RAW, L.SOFTMAX):
+        assert _predict_plan(lb, table, X, K, transform)["leaves_with_trees"] == with_trees
         got = table.predict(X, K, init=init, transform=transform, wait=True)
         for rows in (slice(0, 4000), slice(N - 4000, N)):
             assert torch.equal(got[rows], table.predict(X[rows], K, init=init, transform=transform, wait=True))
@@ -539,7 +587,7 @@ def test_predict_of_several_outputs_by_tables(lb, oracle, N, F, K, T, D, dt):
 
 
 def test_predict_without_room_for_ranks(lb):
-    """A caller's allocator that has no 64 MB gets the predictions by the path that needs less."""
+    """A caller's allocator that has no 20 MB gets the predictions by the path that needs less."""
     from legateboost_b200.tree import TreeTable
 
     rs = np.random.RandomState(1)
