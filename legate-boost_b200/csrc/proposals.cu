@@ -64,7 +64,9 @@ __device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals 
   const int S = p.S, S_pad = p.S_pad;
   auto sample = [&](int i) -> T {
     if (i >= S) return static_cast<T>(INFINITY);
-    return p.draft != nullptr ? p.draft[static_cast<int64_t>(f) * S + i] : SampledValue(p, i, f);
+    const T v = p.draft != nullptr ? p.draft[static_cast<int64_t>(f) * S + i] : SampledValue(p, i, f);
+    // (-0 becomes +0: they are equal, and which of them was kept would be up to the threads' timing.  A NaN counts as +inf.)
+    return v == v ? v + T(0) : static_cast<T>(INFINITY);
   };
   const int P     = S_pad < 4 ? 4 : S_pad;  // (whole 16-byte words)
   const uint8_t* mark = nullptr;  // counted: where there is a value
@@ -77,7 +79,6 @@ __device__ inline void SortUniqueBlock(const PrologueArgs<T>& p, int f, T* vals 
     for (int u = 0; u < kPer; ++u) {
       const int i = tid + u * kSortThreads;
       mine[u]     = sample(i);
-      if (mine[u] != mine[u]) mine[u] = static_cast<T>(INFINITY);
       if (i < P) {
         vals[i] = mine[u];
         here[i] = 0;

@@ -166,13 +166,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       eng.discard(static_cast<unsigned long long>(tid));
       const long long row = eng.uniform_int(0, p.dataset_rows - 1) - p.row_offset;
       v = row >= 0 && row < N ? p.X[row * p.ldx + f] : T(0);
+      v = v == v ? v + T(0) : static_cast<T>(INFINITY);  // (-0 becomes +0, or timing would say which of them is kept)
     }
     // sorted by counting, two threads per value
     __syncthreads();
     T* s_sorted = s_cuts + kSmallBins;                              // [256]
     int* s_mark = reinterpret_cast<int*>(s_sorted + kSmallBins);    // [256]
     if (tid < kSmallBins) {
-      s_cuts[tid] = v == v ? v : static_cast<T>(INFINITY);
+      s_cuts[tid] = v;
       s_mark[tid] = 0;
     }
     __syncthreads();

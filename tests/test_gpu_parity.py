@@ -453,6 +453,33 @@ def test_build_tree_level_batching(lb, oracle):
     assert np.array_equal(got["leaf_value"].cpu().numpy(), want.leaf_value)
 
 
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("S", [3, 100, 256, 300, 512, 700, 2048])
+def test_zeros_of_either_sign_among_the_samples(lb, dt, S):
+    """-0 and +0 are one candidate, which is +0 whatever comes first; a NaN among the samples counts as +inf."""
+    from legateboost_b200 import stages
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.RandomState(S)
+    X = (np.round(rs.normal(size=(3000, 5)) * 5) / 5).astype(dt)
+    X[:, 1] = np.where(rs.random(3000) < 0.5, -0.0, X[:, 1])
+    X[:, 2] = np.where(X[:, 2] == 0, -0.0, X[:, 2])
+    X[:, 3] = -0.0
+    X[rs.random(3000) < 0.3, 4] = np.nan
+    want, want_ptr = stages.split_proposals(dev(np.where(np.isnan(X), np.inf, X + 0.0).astype(dt)), S, 7)
+    p, ptr = stages.split_proposals(dev(X), S, 7)
+    words = torch.int32 if dt == np.float32 else torch.int64
+    assert torch.equal(ptr, want_ptr) and torch.equal(p.view(words), want.view(words))
+    X[:, 4] = rs.random(3000)
+    g, h = np.where(X[:, 1:2] > 0, 1.0, -1.0), np.ones((3000, 1))  # (the best split is at zero)
+    for N in (3000, 70_000):  # (the one-launch form and the general one)
+        big = [dev(np.tile(a, (N // 1000, 1))[:N]) for a in (X, g, h)]
+        tree = build_tree_arrays(*big, max_depth=4, split_samples=S, seed=7, row_offset=0, dataset_rows=N)
+        v = tree["split_value"].cpu().numpy()
+        assert not np.signbit(v[v == 0]).any()
+        assert S < 100 or (v[0] == 0 and tree["feature"][0] == 1)
+
+
 def _random_trees(rs, T, D, features, odd=False):
     """Trees of depth <= D on the given features, splits around U(0, 1); with `odd` infinite and NaN ones too."""
     trees = []
