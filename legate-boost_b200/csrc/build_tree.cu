@@ -254,9 +254,10 @@ __global__ void __launch_bounds__(256) k_zero_if(const int* __restrict__ gate, i
 }
 
 // `round`: a boosting round instead of a tree on given gradients (they are those of round->pred, which gets
-// the leaf values added); the call is then asynchronous.
+// the leaf values added); the call is then asynchronous.  held: levels may be held beyond the reference's cache; set while they are and
+// the call, if it fails, may be made again.
 template <typename T>
-void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t stream, const lbk_boost_round_args* round)
+void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t stream, const lbk_boost_round_args* round, bool* held)
 {
   const int F = a.n_features, K = a.n_outputs, D = a.max_depth;
   const int64_t N = a.n_local_rows;
@@ -571,28 +572,14 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   // finds out; where it is so, such a level is derived too, from the level above, which is kept up to kHeldHistogramBytes: half
   // of the rows are summed and half of the histograms read.  Level 7 of 1M x 100, ten classes: 808 -> 324 us for the
   // histograms and 391 -> 302 for scan and search; the launch that finds the other answer 4 us.
-  bool hold = ctx->n_ranks <= 1 && a.trace_hist == nullptr && max_batch > 1;
+  bool hold = held != nullptr && ctx->n_ranks <= 1 && a.trace_hist == nullptr && max_batch > 1 && cdepth < D - 1;
   const int reference_levels = cache_levels;
   while (hold && cache_levels < D - 1 && LevelEnd(cache_levels + 1) * static_cast<int64_t>(K) * B * static_cast<int64_t>(sizeof(GPairI64)) <= kHeldHistogramBytes)
     ++cache_levels;
   const int cache_end_ref = LevelEnd(cdepth);  // extent of the reference's cached histogram
   const size_t node_elems = static_cast<size_t>(K) * B;
-  if (cache == nullptr) {
-    auto allocate = [&]() {
-      const bool last_held = a.trace_hist != nullptr || cache_levels < D - 1 || D <= 1;
-      cache = s.alloc<GPairI64>(static_cast<size_t>(last_held ? LevelEnd(cache_levels) : LevelEnd(D - 2)) * node_elems);
-    };
-    try {
-      allocate();
-    } catch (const Error& e) {  // (no room for more than the reference keeps: nothing is derived beyond it)
-      if (e.code != LBK_ERR_ALLOC || !hold || cache_levels == reference_levels) throw;
-      hold         = false;
-      cache_levels = reference_levels;
-      allocate();
-    }
-  }
-  const int cache_nodes = LevelEnd(cache_levels);
 
+  // What a tree needs whatever its levels are derived from comes first.
   // rows grouped by node, ping-pong; the root's rows are in order and need no list
   int32_t* rows_a = nullptr;
   int32_t* rows_b = D > 1 ? s.alloc<int32_t>(N) : nullptr;
@@ -605,8 +592,17 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   const bool stream_pairs = K <= kMaxStreamedOutputs && D > 0;
   int2* pairs_a = gpair;
   int2* pairs_b = stream_pairs && D > 1 ? s.alloc<int2>(static_cast<size_t>(N) * K) : nullptr;
-
-  SplitParams sp{a.l1_regularization, a.l2_regularization, a.min_split_gain, fset};
+  if (hist_scratch.partial_bytes > 0 && N > 0) hist_scratch.partial = s.alloc_bytes(hist_scratch.partial_bytes);
+  // leaves of the rows, where something wants them: by the kernel that finds them.  A warp adds the outputs of 32 rows: of many outputs
+  // and few rows too little is in flight.  Depth 7, this and the three kernels: 5k x 60, 16 outputs 11.7 and 12.5 us, 40 outputs 17.2
+  // and 12.6, 100 outputs 62 and 14 (with one value of a lane on its way); 200k x 30, 16 outputs 17.6 and 25.4, 40 outputs 27.8 and 43.5.
+  const int64_t pitch  = static_cast<int64_t>((F + kGroup - 1) / kGroup) * kGroup;
+  const bool add_here  = round != nullptr && N > 0 && K <= kLeafOutputs && LeafTiled(bins, pitch * bin_bytes, F, M);
+  const bool make_here = add_here && static_cast<int64_t>(M) * K <= kLeafTable;
+  int32_t* d_leaf      = nullptr;
+  if ((a.out_leaf != nullptr || round != nullptr) && N > 0)
+    d_leaf = a.out_leaf != nullptr && !a.host_buffers ? a.out_leaf
+             : a.out_leaf != nullptr || !add_here     ? s.alloc<int32_t>(static_cast<size_t>(N)) : nullptr;
 
   // raw sums of the built nodes of a level, alternating so that a level can zero the next one's
   GPairI64* built[2]    = {nullptr, nullptr};
@@ -614,15 +610,59 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   auto built_buffer = [&](int which, size_t nodes) {
     if (built_nodes[which] < nodes) {
       if (built[which]) s.free_one(built[which]);
+      built[which]       = nullptr;
+      built_nodes[which] = 0;
       built[which]       = s.alloc<GPairI64>(nodes * node_elems);
       built_nodes[which] = nodes;
     }
     return built[which];
   };
-  bool built_zeroed   = root_zeroed;
   GPairI64* fresh    = nullptr;  // histogram of a batch that lies outside the cache
   size_t fresh_nodes = 0;
-  if (hist_scratch.partial_bytes > 0 && N > 0) hist_scratch.partial = s.alloc_bytes(hist_scratch.partial_bytes);
+  auto fresh_buffer = [&](size_t nodes) {
+    if (fresh_nodes < nodes) {
+      if (fresh) s.free_one(fresh);
+      fresh       = nullptr;
+      fresh_nodes = 0;
+      fresh       = s.alloc<GPairI64>(nodes * node_elems);
+      fresh_nodes = nodes;
+    }
+    return fresh;
+  };
+  auto allocate_cache = [&]() {
+    const bool last_held = a.trace_hist != nullptr || cache_levels < D - 1 || D <= 1;
+    cache = s.alloc<GPairI64>(static_cast<size_t>(last_held ? LevelEnd(cache_levels) : LevelEnd(D - 2)) * node_elems);
+  };
+  // Levels that are derived beyond the reference's cache take more memory than if they were built: the levels held, and a
+  // buffer for all nodes of each of them.  All of that is asked for here; if there is no room, nothing is held.
+  if (hold) {
+    size_t nodes[3] = {0, 0, 0};  // of either built buffer, of a batch
+    for (int depth = 1; depth < D; ++depth) {
+      const int64_t level = int64_t{1} << depth, batch = std::min(level, max_batch & ~int64_t{1});
+      size_t& most        = nodes[depth <= cdepth || LevelBegin(depth) <= LevelEnd(cache_levels) ? depth & 1 : 2];
+      most                = std::max<size_t>(most, depth <= cdepth ? level / 2 : batch);
+    }
+    try {
+      allocate_cache();
+      for (int which : {0, 1}) built_buffer(which, nodes[which]);
+      fresh_buffer(nodes[2]);
+    } catch (const Error& e) {
+      if (e.code != LBK_ERR_ALLOC) throw;
+      for (GPairI64* p : {built[0], built[1], fresh, cache})
+        if (p != nullptr) s.free_one(p);
+      built[0] = built[1] = fresh = cache = nullptr;
+      built_nodes[0] = built_nodes[1] = fresh_nodes = 0;
+      hold         = false;
+      cache_levels = reference_levels;
+    }
+    if (held != nullptr) *held = hold;
+  }
+  if (cache == nullptr) allocate_cache();
+  const int cache_nodes = LevelEnd(cache_levels);
+
+  SplitParams sp{a.l1_regularization, a.l2_regularization, a.min_split_gain, fset};
+
+  bool built_zeroed = root_zeroed;
   // the most recently replaced "cache" of the reference, to decide parent availability
   int ref_hist_begin = 0, ref_hist_end = cache_end_ref;
 
@@ -666,12 +706,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       if (in_cache) {
         if (write_hist || !(derive || may_derive)) level_hist = cache + static_cast<size_t>(nb) * node_elems;
       } else if (!may_derive) {
-        if (fresh_nodes < static_cast<size_t>(n_nodes)) {
-          if (fresh) s.free_one(fresh);
-          fresh       = s.alloc<GPairI64>(static_cast<size_t>(n_nodes) * node_elems);
-          fresh_nodes = n_nodes;
-        }
-        level_hist = fresh;
+        level_hist = fresh_buffer(n_nodes);
       }
       const int n_slots = derive || may_derive ? n_nodes / 2 : n_nodes;  // (all n_nodes of the buffer where may_derive comes to no)
       // With several ranks the level is built into a buffer the other ranks' GPUs can read, and
@@ -782,16 +817,9 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     }
   }
 
-  const int64_t pitch  = static_cast<int64_t>((F + kGroup - 1) / kGroup) * kGroup;
-  // By the kernel that finds the leaves.  A warp adds the outputs of 32 rows: of many outputs and few rows too little is in
-  // flight.  Depth 7, this and the three kernels: 5k x 60, 16 outputs 11.7 and 12.5 us, 40 outputs 17.2 and 12.6, 100 outputs
-  // 62 and 14 (with one value of a lane on its way); 200k x 30, 16 outputs 17.6 and 25.4, 40 outputs 27.8 and 43.5.
-  const bool add_here  = round != nullptr && N > 0 && K <= kLeafOutputs && LeafTiled(bins, pitch * bin_bytes, F, M);
-  const bool make_here = add_here && static_cast<int64_t>(M) * K <= kLeafTable;
+  if (held != nullptr) *held = false;
   if (!make_here) FinishTree(tree, qp, K, a.l1_regularization, a.l2_regularization, hessian, stream);
   if ((a.out_leaf != nullptr || round != nullptr) && N > 0) {
-    int32_t* d_leaf = a.out_leaf != nullptr && !a.host_buffers ? a.out_leaf
-                      : a.out_leaf != nullptr || !add_here     ? s.alloc<int32_t>(static_cast<size_t>(N)) : nullptr;
     LeafRound rnd{};
     if (add_here) {
       rnd = LeafRound{round->pred, K, tree, qp, a.l1_regularization, a.l2_regularization, hessian};
@@ -814,6 +842,20 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
   CheckDeviceStatus(ctx, stream);  // synchronises, as the reference's task does (:1356)
   words.settled();
   if (a.out_total_bins) *a.out_total_bins = sketch_reuse ? head.total_bins : words.get()[0];
+}
+
+// Where what a level allocates for itself finds no room beside the levels that are held, the tree is made again without them: all that it
+// is made from is as it was, and its outputs are written anew.
+template <typename T>
+void BuildTree(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t stream, const lbk_boost_round_args* round)
+{
+  bool held = false;
+  try {
+    BuildTreeImpl<T>(ctx, a, stream, round, &held);
+  } catch (const Error& e) {
+    if (e.code != LBK_ERR_ALLOC || !held) throw;
+    BuildTreeImpl<T>(ctx, a, stream, round, nullptr);
+  }
 }
 
 void CheckTreeArgs(const lbk_build_tree_args& a)
@@ -861,9 +903,9 @@ int lbk_build_tree(lbk_context* ctx, const lbk_build_tree_args* a)
     LBK_EXPECT(a->n_local_rows == 0 || a->ldg >= a->n_outputs, "Expected a dense row major store");
     cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
     if (a->x_dtype == LBK_F32)
-      lbk::BuildTreeImpl<float>(ctx, *a, stream, nullptr);
+      lbk::BuildTree<float>(ctx, *a, stream, nullptr);
     else
-      lbk::BuildTreeImpl<double>(ctx, *a, stream, nullptr);
+      lbk::BuildTree<double>(ctx, *a, stream, nullptr);
   });
 }
 
@@ -880,9 +922,9 @@ int lbk_boost_round(lbk_context* ctx, const lbk_boost_round_args* r)
     lbk::ThrowReportedFault(ctx);
     cudaStream_t stream = static_cast<cudaStream_t>(a.stream);
     if (a.x_dtype == LBK_F32)
-      lbk::BuildTreeImpl<float>(ctx, a, stream, r);
+      lbk::BuildTree<float>(ctx, a, stream, r);
     else
-      lbk::BuildTreeImpl<double>(ctx, a, stream, r);
+      lbk::BuildTree<double>(ctx, a, stream, r);
   });
 }
 

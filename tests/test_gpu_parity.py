@@ -665,7 +665,8 @@ def test_levels_outside_the_cache(lb, oracle, N, F, K, D, zeros):
 
 
 def test_levels_outside_the_cache_without_room_for_more(lb):
-    """A caller's allocator that has room for the reference's cache only gets the tree that is built node by node there."""
+    """A caller's allocator that has no room for more than the reference's cache, in one piece or in all, gets the tree that
+    is built node by node on the levels outside it."""
     from legateboost_b200.tree import build_tree_arrays
 
     rs = np.random.RandomState(4)
@@ -673,29 +674,49 @@ def test_levels_outside_the_cache_without_room_for_more(lb):
     build = lambda: build_tree_arrays(X, g, h, max_depth=10, split_samples=256, seed=5, row_offset=0, dataset_rows=700)
     want = build()
     ctx = lb.library.context(X.device.index)
-    held, refused = {}, []
 
-    def alloc(user, nbytes, stream):
-        if nbytes > 1_000_000_000:
-            refused.append(nbytes)
-            return None
-        t = torch.empty(int(nbytes), dtype=torch.uint8, device="cuda")
-        held[t.data_ptr()] = t
-        return t.data_ptr()
+    def build_within(piece, total, but=-1):
+        """The most that was lent at a time, how often nothing was, and what was asked for; request `but` is refused anyhow."""
+        held, lent, most, refused, asked = {}, [0], [0], [], []
 
-    def release(user, ptr, stream):
-        held.pop(ptr, None)
+        def alloc(user, nbytes, stream):
+            asked.append(nbytes)
+            if nbytes > piece or lent[0] + nbytes > total or len(asked) - 1 == but:
+                refused.append(nbytes)
+                return None
+            t = torch.empty(int(nbytes), dtype=torch.uint8, device="cuda")
+            held[t.data_ptr()] = t
+            lent[0] += nbytes
+            most[0] = max(most[0], lent[0])
+            return t.data_ptr()
 
-    cbs = lb.library.ALLOC_FN(alloc), lb.library.RELEASE_FN(release)
-    ctx.check(ctx.lib.lbk_context_set_allocator(ctx.handle, cbs[0], cbs[1], None))
-    try:
-        got = build()
-        torch.cuda.synchronize()
-    finally:
-        ctx.use_torch_allocator(False)
-    assert len(refused) == 1
-    for name in ("feature", "split_value", "gain", "hessian", "leaf_value"):
-        assert torch.equal(got[name], want[name]), name
+        def release(user, ptr, stream):
+            lent[0] -= held.pop(ptr).numel()
+
+        cbs = lb.library.ALLOC_FN(alloc), lb.library.RELEASE_FN(release)
+        ctx.check(ctx.lib.lbk_context_set_allocator(ctx.handle, cbs[0], cbs[1], None))
+        try:
+            got = build()
+            torch.cuda.synchronize()
+        finally:
+            ctx.use_torch_allocator(False)
+        assert lent[0] == 0
+        for name in ("feature", "split_value", "gain", "hessian", "leaf_value"):
+            assert torch.equal(got[name], want[name]), name
+        return most[0], len(refused), asked
+
+    everything, refusals, asked = build_within(1 << 62, 1 << 62)
+    assert refusals == 0
+    least, refusals, _ = build_within(1_000_000_000, 1 << 62)
+    assert refusals == 1 and least < everything - 1_000_000_000
+    for total in np.linspace(least, everything, 9).astype(np.int64):
+        most, refusals, _ = build_within(1 << 62, int(total))
+        assert (refusals == 0) == (total == everything) and most <= total
+    # every request from the held levels on may be the one that is refused
+    first = next(i for i, n in enumerate(asked) if n > 1_000_000_000)
+    for but in range(first, len(asked)):
+        assert build_within(1 << 62, 1 << 62, but)[1] == 1
+    assert len(asked) - first > 3
 
 
 def test_golden_trees_on_gpu(lb, oracle):
