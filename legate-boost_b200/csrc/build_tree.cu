@@ -245,12 +245,23 @@ constexpr int64_t kHistogramCacheBytes = 1000000000;  // (reference: build_tree.
 // rule the results follow, see BuildTreeImpl).
 constexpr int64_t kHeldHistogramBytes = 2000000000;
 
-// Zeroes n 16-byte words where *gate is not 0.
-__global__ void __launch_bounds__(256) k_zero_if(const int* __restrict__ gate, int4* __restrict__ at, int64_t n)
+// Clears the slots of a batch's nodes where *gate is not 0: those of nodes that exist (parent_feature [n_nodes / 2]: their parents'
+// splits) and are not clear already, which the first `clear` slots are - all of them, or (by_search) those of pairs that exist.
+constexpr int kZeroPiece = 512;  // pairs that a warp clears at a time
+__global__ void __launch_bounds__(256)
+  k_zero_if(const int* __restrict__ gate, int4* __restrict__ at, int64_t slot, int n_nodes, const int32_t* __restrict__ parent_feature, int clear,
+            bool by_search)
 {
   if (*gate == 0) return;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    at[i] = make_int4(0, 0, 0, 0);
+  const int lane = threadIdx.x & 31;
+  const int64_t pieces = (slot + kZeroPiece - 1) / kZeroPiece, items = pieces * n_nodes;
+  for (int64_t item = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / 32; item < items; item += static_cast<int64_t>(gridDim.x) * blockDim.x / 32) {
+    const int j = static_cast<int>(item / pieces);
+    if (parent_feature[j >> 1] < 0 || (j < clear && (!by_search || parent_feature[j] >= 0))) continue;
+    const int64_t from = (item - j * pieces) * kZeroPiece, to = from + kZeroPiece < slot ? from + kZeroPiece : slot;
+    int4* dst = at + j * slot;
+    for (int64_t i = from + lane; i < to; i += 32) dst[i] = make_int4(0, 0, 0, 0);
+  }
 }
 
 // `round`: a boosting round instead of a tree on given gradients (they are those of round->pred, which gets
@@ -717,9 +728,9 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       const int f_end   = owned ? OwnedBegin(ctx->rank + 1, ctx->n_ranks, F) : F;
       // built buffer: when nothing is derived the level histogram itself is the target
       GPairI64* target = derive ? built_buffer(depth & 1, n_slots) : may_derive ? built_buffer(depth & 1, n_nodes) : level_hist;
-      if (may_derive) {  // (what is zero already is so for the pairs whose parent exists)
-        k_zero_if<<<ctx->sm_count * 8, 256, 0, stream>>>(hess_below_one, reinterpret_cast<int4*>(target),
-                                                         static_cast<int64_t>(n_nodes) * static_cast<int64_t>(node_elems));
+      if (may_derive) {
+        k_zero_if<<<ctx->sm_count * 8, 256, 0, stream>>>(hess_below_one, reinterpret_cast<int4*>(target), static_cast<int64_t>(node_elems), n_nodes,
+                                                         tree.feature + (nb - 1) / 2, n_slots, built_zeroed);
         LBK_LAUNCH_CHECK();
       }
       if (a.trace_hist != nullptr && derive)  // (nodes that do not exist read as zeros in a trace)

@@ -659,7 +659,25 @@ def test_levels_outside_the_cache(lb, oracle, N, F, K, D, zeros):
     if zeros:
         h[rs.random(N) < 0.3] = 0.0
     want = oracle.build_tree(X, g, h, max_depth=D, split_samples=256, seed=5, mode="Q")
-    got = build_tree_arrays(dev(X), dev(g), dev(h), max_depth=D, split_samples=256, seed=5, row_offset=0, dataset_rows=N)
+    # (in scratch that holds something: what has to be clear has been cleared)
+    dX, dg, dh = dev(X), dev(g), dev(h)
+    ctx, held = lb.library.context(dX.device.index), {}
+
+    def alloc(user, nbytes, stream):
+        t = torch.full((int(nbytes),), 0x5a, dtype=torch.uint8, device="cuda")
+        held[t.data_ptr()] = t
+        return t.data_ptr()
+
+    def release(user, ptr, stream):
+        held.pop(ptr)
+
+    cbs = lb.library.ALLOC_FN(alloc), lb.library.RELEASE_FN(release)
+    ctx.check(ctx.lib.lbk_context_set_allocator(ctx.handle, cbs[0], cbs[1], None))
+    try:
+        got = build_tree_arrays(dX, dg, dh, max_depth=D, split_samples=256, seed=5, row_offset=0, dataset_rows=N)
+        torch.cuda.synchronize()
+    finally:
+        ctx.use_torch_allocator(False)
     for name in ("feature", "split_value", "node_sums", "gain", "hessian", "leaf_value"):
         assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
 
