@@ -27,12 +27,14 @@ constexpr int kSplitWarps   = kSplitThreads / 32;
 // barrier, and no totals of eight warps to add up, per output and 256 bins.  Microseconds with a block per feature and with
 // a warp: one output, 400 features, 8 units 36 and 27, 128 units 272 and 259; 64 features, 32 units 29 and 24, 16 units 17.7 and 20; 20
 // features, 128 units 36.7 and 27.7, 32 units 15.7 and 20.4; three outputs, 100 features, 32 units 79 and 66, 16 units 46 and
-// 48; ten outputs, 64 units 296 and 287, 32 units 167 and 177.
+// 48; ten outputs, 64 units 296 and 287, 32 units 167 and 177.  A warp's chain is as long as its feature has bins: with more than 256
+// (several outputs: 700) of them on average the line moves up with their number.  One output, 34 features, 256 units of 1000
+// bins 44 and 62, 150 features, 32 and 64 units of 1024 bins 126 and 152, 160 and 150, of 512 bins 69 and 55, 90 and 86.
 constexpr int kWideOutputs = 64;  // (what a block has room for)
-__host__ inline bool ScanIsWide(int64_t units, int n_features, int K)
+__host__ inline bool ScanIsWide(int64_t units, int n_features, int K, int64_t bins_per_feature)
 {
-  const int64_t least = K <= 1 ? 1500 : K < 6 ? 1000 * K : 6000;
-  return K <= kWideOutputs && units * n_features >= least;
+  const int64_t least = K <= 1 ? 1500 : K < 6 ? 1000 * K : 6000, usual = K <= 1 ? 256 : 700;
+  return K <= kWideOutputs && units * n_features * usual >= least * (bins_per_feature > usual ? bins_per_feature : usual);
 }
 
 // What a rank knows about its best split of a node when the features are divided among the ranks:
@@ -494,7 +496,7 @@ void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, co
   const int n_features = lv.f_end - lv.f_begin;
   const int units      = lv.derive ? lv.n_nodes / 2 : lv.n_nodes;
   if (units <= 0) return;
-  const bool wide = ScanIsWide(units, n_features, lv.K);
+  const bool wide = ScanIsWide(units, n_features, lv.K, lv.bin_stride / F);
   // with several outputs a block keeps K terms of two nodes and K running prefixes (of every warp) in shared memory
   const size_t smem = (lv.K > 1 ? sizeof(NodeTerms) * 2 * ((lv.K + 1) / 2 * 2) : 0) + lv.K * sizeof(GPairI64) * (wide ? kSplitWarps : 1);
   // one feature per block (warp) until there are about sixteen blocks per SM, then several

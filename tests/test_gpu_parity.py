@@ -1470,7 +1470,7 @@ def test_many_outputs_at_the_edge_of_default_shared_memory(lb, oracle, K):
 
 @pytest.mark.parametrize("N,F,K,D,S,dt", [
     (40_000, 30, 1, 8, 256, np.float32), (40_000, 33, 1, 8, 100, np.float64),  # a warp per feature on the last levels
-    (9_000, 60, 1, 7, 700, np.float32), (20_000, 101, 3, 7, 256, np.float32), (4_000, 130, 10, 7, 256, np.float32),
+    (9_000, 60, 1, 8, 700, np.float32), (20_000, 101, 3, 7, 256, np.float32), (4_000, 130, 10, 7, 256, np.float32),
     (33_000, 49, 2, 8, 31, np.float32),
 ])
 def test_wide_levels(lb, oracle, N, F, K, D, S, dt):
