@@ -686,13 +686,13 @@ __device__ __forceinline__ void RankRows(const RankRowsArgs<T>& a, const RankTab
   }
 }
 
-// The tables of features [w0, w1) of a group to shared memory, by a block; eight entries of a thread at a time: places, then loads, then
+// The tables of features [w0, w1) of a group to shared memory, by a block; four entries of a thread at a time: places, then loads, then
 // stores.  (A warp per feature, 32 entries at a time: 50 us for one feature of 20 thousand.  Inlined, or with the two arrays as
 // arguments, the float32 loop over the rows comes out 3 % slower: 10M x 100, 500 trees 300 and 310 us a piece.)
 template <typename T>
 __device__ __noinline__ void FillTables(const RankRowsArgs<T>& a, const int* s_begin, const int* s_from, int w0, int w1, unsigned* s_lut, T* s_cuts)
 {
-  constexpr int kFill = 8;
+  constexpr int kFill = 4;
   const int base = s_begin[w0], entries = s_begin[w1] - base;
   for (int i0 = threadIdx.x; i0 < entries; i0 += kFill * kRankThreads) {
     int from[kFill];  // where the entry lies, -1: of a feature without values, whose only bucket is empty
