@@ -421,16 +421,21 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
                    const lbk_tree_ref* d_trees /* device */, int m_max /* nodes of the largest tree */, int64_t total_nodes,
                    const double* init, int transform, double* pred, int64_t ldp, cudaStream_t stream);
 // predict_ranked.cu: one output, more rows and trees than k_predict_tiled is better for.
+struct RankTile {  // of k_predict_tiled: rows that an SM has at a time (0: not tiled), trees that a thread walks together
+  int rows = 0, trees = 0, tree_bytes = 0;
+};
 struct RankedPlan {  // threads == 0: the shape does not fit, or is not worth it
   int threads = 0, tg = 0, nbuf = 0;  // of the walk, and trees per group: what is in flight is threads x trees x 2 walks
   size_t smem   = 0;
   int64_t piece = 0;  // rows whose ranks are held at a time
   double budget = 0;  // microseconds that finding the ranks may take
+  bool sure     = false;  // whatever the splits are, they take no more: the device does not decline
   int max_items = 0;  // pieces of the features' lists of splits
   size_t bytes = 0, o_words = 0, o_off = 0, o_items = 0, o_lists = 0, o_cuts = 0, o_lut = 0, o_tables = 0, o_records = 0, o_ranks = 0;  // scratch
 };
 template <typename T>
-RankedPlan PlanRanked(const lbk_context* ctx, int64_t n_rows, int F, int n_trees, int S, int64_t total_nodes);
+RankedPlan PlanRanked(const lbk_context* ctx, int64_t n_rows, int F, int n_trees, int S, int64_t total_nodes,
+                      const RankTile& tiled);
 // Null: there is no room for it, nothing was done.  Else a device word: where it is not 0 when the stream comes to it, the
 // kernels queued here have done nothing, because the ensemble's splits lie so that the ranks would cost more than they give.
 template <typename T>

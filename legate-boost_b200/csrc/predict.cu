@@ -585,6 +585,7 @@ constexpr int kTileMinRows         = 64;
 constexpr size_t kTileOneWarpBytes = 2560;
 struct TilePlan {
   int rb = 0, tg = 0, nbuf = 0, resident = 1;
+  int sm_rows = 0;  // rows that an SM has at a time
   unsigned x_bytes = 0;
   size_t smem      = 0;
   int64_t waves    = 0;
@@ -630,6 +631,7 @@ TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, i
         const int64_t waves = (n_rows + static_cast<int64_t>(rb) * res * ctx->sm_count - 1) / (static_cast<int64_t>(rb) * res * ctx->sm_count);
         if (leaf_values > 1 && best_score > 0 && waves != best.waves ? waves > best.waves : score < best_score || (score == best_score && tg < best.tg)) continue;
         best_score   = score;
+        best.sm_rows = res * rb;
         best.waves   = waves;
         best_res     = res;
         best.rb      = rb;
@@ -724,7 +726,12 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   // a walk through M heap-ordered nodes takes at most S = floor(log2(M)) steps
   int S = 0;
   while ((2 << S) <= m_max) ++S;
-  const TilePlan plan = S <= 14 && F <= kMaxFeature ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
+  const TilePlan plan     = S <= 14 && F <= kMaxFeature ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
+  const RankedPlan ranked = K == 1 ? PlanRanked<T>(ctx, n_rows, F, n_trees, S, total_nodes, RankTile{plan.sm_rows, plan.tg, plan.rec.bytes}) : RankedPlan{};
+  auto by_ranks = [&]() {
+    return PredictRanked<T>(ctx, s, ranked, X, ldx, n_rows, F, n_trees, d_trees, S, total_nodes, init, transform, pred, ldp, stream);
+  };
+  if (ranked.threads > 0 && ranked.sure && by_ranks() != nullptr) return;
   // (what the rows are walked with where the ranks are declined comes first: without room for it the call fails, with or without ranks)
   NodeT* nodes = nullptr;
   double *leaves = nullptr, *leaves_c = nullptr;
@@ -737,11 +744,7 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
     if (plan.rec.leaf_bytes == 0) leaves_c = s.alloc<double>((static_cast<size_t>(n_trees) << S) * K);
   }
   const int* gate = nullptr;
-  if (K == 1) {
-    const RankedPlan ranked = PlanRanked<T>(ctx, n_rows, F, n_trees, S, total_nodes);
-    if (ranked.threads > 0)
-      gate = PredictRanked<T>(ctx, s, ranked, X, ldx, n_rows, F, n_trees, d_trees, S, total_nodes, init, transform, pred, ldp, stream);
-  }
+  if (ranked.threads > 0 && !ranked.sure) gate = by_ranks();
   if (plan.rb == 0) {
     k_pack_trees<NodeT><<<n_trees, 256, 0, stream>>>(gate, d_trees, K, F, nodes, leaves);
     LBK_LAUNCH_CHECK();
@@ -769,7 +772,7 @@ static void PlanOfPredict(lbk_context* ctx, int64_t n_rows, int F, int K, int n_
   int S = 0;
   while ((2 << S) <= m_max) ++S;
   const TilePlan tile     = S <= 14 && F <= kMaxFeature ? PlanTile<T>(ctx, n_rows, F, K, n_trees, S, transform) : TilePlan{};
-  const RankedPlan ranked = K == 1 ? PlanRanked<T>(ctx, n_rows, F, n_trees, S, total_nodes) : RankedPlan{};
+  const RankedPlan ranked = K == 1 ? PlanRanked<T>(ctx, n_rows, F, n_trees, S, total_nodes, RankTile{tile.sm_rows, tile.tg, tile.rec.bytes}) : RankedPlan{};
   const int64_t words[8]  = {ranked.threads, ranked.tg, ranked.piece, static_cast<int64_t>(ranked.bytes), static_cast<int64_t>(ranked.o_words),
                              tile.rb, tile.tg, tile.rec.leaf_bytes > 0};
   std::copy(words, words + 8, out);

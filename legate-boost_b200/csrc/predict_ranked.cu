@@ -465,23 +465,25 @@ __host__ __device__ inline int TailLanes(int F)
   return lanes;
 }
 
-// Microseconds that k_rank_rows takes for group g of F features, as its tables are: of a turn kTurn and kLane per lane that a row
-// takes, per million rows and with all SMs; kGlobal more for a table that is searched where it lies; kFill per entry brought to shared
-// memory.  Fitted to 50 (float32) and 46 (float64) ensembles of 4 to 511 trees of depth 4 to 10 on 8 to 236 features, up to all
-// splits on one of them, and 83 thousand to 1.7 million rows: 7 and 13 % off (rms).
+// Microseconds that k_rank_rows takes for group g of F features, as its tables are.  Per million rows and with all SMs: kLane of a
+// turn per lane that a row takes (of less than eight the loads of a step are not all used), kGlobal for a table that is
+// searched where it lies, kAgain for every turn but the first where rows have more than one group (what they share of a
+// line is gone by then).  kFill per entry brought to shared memory.  Fitted to 154 (float32) and 145 (float64) ensembles of 4 to
+// 511 trees of depth 3 to 10 on 6 to 236 features, up to all splits on one of them, and 80 thousand to 6 million rows: 9 and 13 %
+// off (rms).
 template <typename T>
 struct RowsCost {
-  static constexpr float kTurn = sizeof(T) == 4 ? 4.f : 3.f, kLane = sizeof(T) == 4 ? 2.1f : 2.8f, kGlobal = 95.f;
-  static constexpr float kFill = sizeof(T) == 4 ? 0.55e-3f : 0.9e-3f, kLaunch = 8.f;
+  static constexpr float kLane = sizeof(T) == 4 ? 2.2f : 2.77f, kGlobal = sizeof(T) == 4 ? 15.f : 22.f, kAgain = sizeof(T) == 4 ? 15.6f : 12.f;
+  static constexpr float kFill = sizeof(T) == 4 ? 0.5e-3f : 0.6e-3f, kLaunch = 8.5f;
   __host__ __device__ static float Group(const int* begin, int g, int F, unsigned room, float millions)
   {
     const int last = (F + 31) / 32 - 1, width = g < last ? 32 : F - 32 * last, tail = TailLanes(F);
     float per_million = 0.f, filled = 0.f;
     for (int w0 = 0, w1; w0 < width; w0 = w1) {
       w1 = TurnEnd<T>(begin, w0, width, room);
-      int lanes = 1;
+      int lanes = 8;
       while (lanes < w1 - w0) lanes *= 2;
-      per_million += kTurn + kLane * static_cast<float>(lanes);
+      per_million += kLane * static_cast<float>(lanes) + (w0 > 0 && last > 0 ? kAgain : 0.f);
       const int entries = begin[w1] - begin[w0];
       if (TableBytes<T>(entries) <= room) filled += static_cast<float>(entries);
       else per_million += kGlobal;
@@ -496,7 +498,8 @@ struct RowsCost {
 // feature's ranks begin in a walking block's tile, in units of 128 bytes.
 __host__ __device__ inline int RankRecordBytes(int S) { return 12 << S; }
 
-// Every block finds out for itself, from all tables, whether finding the ranks of `millions` of rows stays within `budget` microseconds.
+// Every block finds out for itself, from all tables, whether finding the ranks of `millions` of rows stays within `budget` microseconds
+// (millions 0: it does).
 template <typename T>
 __global__ void __launch_bounds__(256)
   k_rank_pack(const TreePtrs* __restrict__ trees, int F, int S, int lines, float millions, float budget, unsigned room, const RankTable* __restrict__ tables,
@@ -507,7 +510,7 @@ __global__ void __launch_bounds__(256)
   __shared__ int s_begin[8][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float most = 0.f;
-  for (int g = warp; 32 * g < F; g += 8) {
+  for (int g = warp; millions > 0.f && 32 * g < F; g += 8) {
     const int width = min(32, F - 32 * g);
     int incl        = lane < width ? tables[32 * g + lane].nb : 0;
     for (int o = 1; o < 32; o <<= 1) {
@@ -971,35 +974,45 @@ __host__ inline unsigned TableRoom(const lbk_context* ctx)
 
 // Is it worth it, as far as the host can tell?  In microseconds: what k_predict_tiled takes, what the walk on ranks takes (whole waves
 // of tiles), and of the difference, less what the tables take, how much there is for finding the ranks.  The device decides with the tables
-// as they are; here the ensemble's splits are spread evenly over the features.  Not for less than 8 % of the tiled kernel's time,
+// as they are; here the ensemble's splits are spread evenly over the features.  Not for less than 4 % of the tiled kernel's time,
 // and not where a feature is likely to have more splits than there are ranks.
 //
-// The two lines are fitted to the ensembles of RowsCost (9 and 15 % off).  As it is decided here and on the device, the 69 of them that
-// take k_predict_tiled 100 us or more take 0.95 of that on average, 0.54 at best and 1.11 at worst.
-// Microseconds by k_predict_tiled and as it is decided, a million rows, depth 8, none, 25, 40, 80 % of the splits on one feature:
-// float32, 100 features, 500 trees 2136 and 1788 (on ranks), 2128 and 2218, 2119 and 2203, 2065 and 2150 (declined); float64, 64
-// features, 100 trees 810 and 516, 806 and 562, 800 and 626, 779 and 789 (on ranks).  What declining costs is the tables:
-// 300k x 20 float64, 300 trees, 40 % 520 and 576.
+// Both are fitted to RowsCost's ensembles (12 and 10 % off).  As it is decided here and on the device, 310 of them take 0.94 of
+// k_predict_tiled's time on average, 0.54 at best and 1.17 at worst (their kernels; with a line of two factors per type, which knew
+// neither the tables nor the tiles, 1.3 without one uneven feature and 19 with).  Microseconds by k_predict_tiled and as it is
+// decided, a million rows, depth 8, none, 25, 40, 80 % of the splits on one feature: float32, 100 features, 500 trees 2136 and 1790 (on ranks),
+// 2121 and 2232, 2108 and 2218, 2060 and 2168 (declined); float64, 64 features, 100 trees 806 and 514, 807 and 562, 800 and 621, 779 and 774
+// (on ranks).  What declining costs is the tables: 300k x 20 float64, 300 trees, 40 % 522 and 588.
 template <typename T>
-static bool RanksPay(const lbk_context* ctx, int64_t n_rows, int F, int n_trees, int S, int threads, double& budget)
+static bool RanksPay(const lbk_context* ctx, int64_t n_rows, int F, int n_trees, int S, const RankTile& tile, RankedPlan& plan)
 {
   const double splits = static_cast<double>(n_trees) * ((1 << S) - 1), millions = static_cast<double>(n_rows) * 1e-6;
-  if (splits > kMaxRank && splits > 8192.0 * F) return false;
-  const int64_t wave  = 2 * static_cast<int64_t>(threads) * ctx->sm_count;
-  const double walked = static_cast<double>((n_rows + wave - 1) / wave * wave) * 1e-6;
-  const double tiled  = millions * (sizeof(T) == 4 ? 1.78 * F + n_trees * (0.577 * S - 0.78) : 4.5 * F + n_trees * (1.03 * S - 2.13)) + 10.0;
-  const double walk   = walked * n_trees * (0.34 * S - 0.75 + 0.53 * kWalkThreads / threads) + millions * 0.3 * F + 6.0;
-  budget              = 0.95 * tiled - walk;
+  if ((splits > kMaxRank && splits > 16384.0 * F) || n_trees * S < 32) return false;
+  const auto waves    = [&](int64_t rows) { return static_cast<double>((n_rows + rows * ctx->sm_count - 1) / (rows * ctx->sm_count)); };
+  const double walked = waves(2 * plan.threads) * 2 * plan.threads * ctx->sm_count * 1e-6;
+  const bool whole    = F * sizeof(T) % 16 == 0;  // (rows of whole vectors)
+  // a tile's rows are staged and its trees brought, then its warps walk: the pipe's passes, and the latency of a step once per wave
+  // and group of trees
+  const double steps = static_cast<double>(n_trees) * S;
+  double tiled       = 3.5 * millions * steps;  // (through the caches, at best)
+  if (tile.rows > 0) {
+    const double n = waves(tile.rows), chain = n * steps / tile.trees, brought = n * n_trees * tile.tree_bytes / 1024.0;
+    tiled = sizeof(T) == 4 ? millions * ((whole ? 0.88 : 1.04) * F + 0.376 * steps) + 0.016 * chain + 0.027 * n * F + 0.005 * brought + 1.3 * n + 9.0
+                           : millions * ((whole ? 2.14 : 2.28) * F + 0.55 * steps) + 0.035 * chain + 0.034 * n * F + 0.003 * brought + 1.3 * n + 7.0;
+  }
+  const double walk = walked * (0.312 * steps + n_trees * (0.55 * kWalkThreads / plan.threads - 0.56)) + millions * 0.31 * F + 6.0;
+  plan.budget       = 0.98 * tiled - walk;
   int begin[33];
   for (int i = 0; i <= 32; ++i) begin[i] = i * std::max(1, static_cast<int>(splits / F));
   float even = 0.f;
   for (int g : {0, (F + 31) / 32 - 1}) even = std::max(even, RowsCost<T>::Group(begin, g, F, TableRoom(ctx), static_cast<float>(millions)));
   const double tables = 18.0 + 4.8 * S;
-  return budget > even + tables + 0.03 * tiled;
+  plan.sure           = splits <= kMaxRank && TableBytes<T>(static_cast<int>(splits) + 32) <= TableRoom(ctx);  // (one turn per group)
+  return plan.budget > even + tables + 0.02 * tiled;
 }
 
 template <typename T>
-RankedPlan PlanRanked(const lbk_context* ctx, int64_t n_rows, int F, int n_trees, int S, int64_t total_nodes)
+RankedPlan PlanRanked(const lbk_context* ctx, int64_t n_rows, int F, int n_trees, int S, int64_t total_nodes, const RankTile& tiled)
 {
   RankedPlan best;
   if (S < 3 || S > 12 || F > kMaxFeatures || total_nodes > (int64_t{1} << 28)) return best;
@@ -1019,7 +1032,7 @@ RankedPlan PlanRanked(const lbk_context* ctx, int64_t n_rows, int F, int n_trees
     best.nbuf    = nbuf;
     best.smem    = static_cast<size_t>(F) * threads * 4 + trees;
   }
-  if (best.threads < 128 || !RanksPay<T>(ctx, n_rows, F, n_trees, S, best.threads, best.budget)) return RankedPlan{};
+  if (best.threads < 128 || !RanksPay<T>(ctx, n_rows, F, n_trees, S, tiled, best)) return RankedPlan{};
   // rows are walked in whole waves of tiles
   const int64_t tile  = 2 * best.threads;
   const int64_t wave  = tile * ctx->sm_count;
@@ -1084,7 +1097,7 @@ const int* PredictRanked(lbk_context* ctx, Scratch& s, const RankedPlan& plan, c
     k_rank_merge<T><<<dim3(items, kSortChunk / kSortThreads), kSortThreads, 0, stream>>>(t);
     LBK_LAUNCH_CHECK();
   }
-  k_rank_pack<T><<<n_trees, 256, 0, stream>>>(d_trees, F, S, plan.threads / 32, static_cast<float>(n_rows) * 1e-6f, static_cast<float>(plan.budget), TableRoom(ctx), t.tables, cuts, t.lut, declined, records);
+  k_rank_pack<T><<<n_trees, 256, 0, stream>>>(d_trees, F, S, plan.threads / 32, plan.sure ? 0.f : static_cast<float>(n_rows) * 1e-6f, static_cast<float>(plan.budget), TableRoom(ctx), t.tables, cuts, t.lut, declined, records);
   LBK_LAUNCH_CHECK();
   AllowSharedMemory(ctx, k_rank_rows<T>, kRankStatic);
   const int64_t tile    = 2 * plan.threads;
@@ -1108,7 +1121,7 @@ const int* PredictRanked(lbk_context* ctx, Scratch& s, const RankedPlan& plan, c
 }
 
 #define LBK_PREDICT_RANKED(T)                                                                                                                  \
-  template RankedPlan PlanRanked<T>(const lbk_context*, int64_t, int, int, int, int64_t);                                                      \
+  template RankedPlan PlanRanked<T>(const lbk_context*, int64_t, int, int, int, int64_t, const RankTile&);                                                    \
   template const int* PredictRanked<T>(lbk_context*, Scratch&, const RankedPlan&, const T*, int64_t, int64_t, int, int, const lbk_tree_ref*,    \
                                        int, int64_t, const double*, int, double*, int64_t, cudaStream_t);
 LBK_PREDICT_RANKED(float)

@@ -531,17 +531,17 @@ def _predict_and_word(lb, table, X, plan, **kw):
 
 
 @pytest.mark.parametrize("N,F,T,D,dt,used,what,group,pieces,declined", [
-    (1_000_001, 100, 300, 8, np.float32, None, "odd", 4, 1, False),     # a last group of four features, a ragged last tile
-    (1_600_003, 100, 300, 8, np.float32, None, "odd", 4, 2, False),     # rows in two pieces
+    (1_000_001, 100, 500, 8, np.float32, None, "odd", 4, 1, False),     # a last group of four features, a ragged last tile
+    (1_600_003, 100, 500, 8, np.float32, None, "odd", 4, 2, False),     # rows in two pieces
     (1_300_003, 33, 200, 5, np.float64, None, "odd", 4, 1, False),      # a last group of one feature
-    (1_200_001, 9, 70, 10, np.float64, None, "odd", 4, 1, False),       # tables of a group in several turns
+    (1_200_001, 9, 100, 10, np.float64, None, "odd", 4, 1, False),       # tables of a group in several turns
     (4_000_000, 1, 60, 4, np.float64, None, "", 4, 1, False),           # one feature
     (600_000, 150, 60, 11, np.float64, None, "", 2, 1, False),          # two trees per group
     (600_000, 150, 60, 12, np.float64, None, "", 1, 1, False),          # one
-    (400_000, 20, 100, 8, np.float64, [3], "", 4, 1, False),            # all splits on one feature, in chunks; no room for the table
+    (800_000, 20, 100, 8, np.float64, [3], "", 4, 1, False),            # all splits on one feature, in chunks; no room for the table
     (400_000, 20, 300, 8, np.float64, [3], "few", 4, 1, False),         # more than there are ranks, of which many are equal
     (300_000, 20, 300, 8, np.float64, [3], "logistic", 4, 1, True),     # more of them than there are ranks
-    (1_000_001, 100, 300, 8, np.float32, "3", "odd", 4, 1, True),       # one large table: the ranks would cost more than they give
+    (1_000_001, 100, 500, 8, np.float32, "3", "odd", 4, 1, True),       # one large table: the ranks would cost more than they give
     (200_000, 330, 300, 8, np.float64, None, "logistic", 4, 1, False),  # rows too wide for the tiled walk
     (200_000, 330, 300, 8, np.float64, [3], "logistic", 4, 1, True),    # ... which are then read through the caches
 ])
@@ -558,8 +558,8 @@ def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what, group, pieces,
         for value in (np.nan, np.inf, -np.inf):
             X[rs.randint(N, size=3000), rs.randint(F, size=3000)] = value
         X[-40:] = np.nan
-    if used == "3":  # of three splits two
-        used = np.concatenate([np.arange(F), np.full(2 * F, 3)])
+    if used == "3":  # of a hundred splits 41
+        used = np.concatenate([np.arange(F), np.full(69, 3)])
     trees = _random_trees(rs, T, D, np.arange(F) if used is None else used, what == "odd")
     if what == "few":
         pool = dev(rs.random(20_000))
