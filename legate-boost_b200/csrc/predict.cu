@@ -4,13 +4,17 @@
 // launch per tree, each re-reading and re-writing pred; rows walk from node 0 while
 // feature[pos] != -1 (at most 100 steps), going left iff (double)x <= split_value[pos].
 //
-// Design for B200: ONE launch for the whole ensemble, everything a step of the walk touches lives
-// in shared memory.  The load/store data pipe of the SM is what bounds it (one pass per clock; a 4-byte load of
+// Three ways, all of one result: a few rows walk the trees where they lie (k_predict_rows); large ensembles of one output are
+// walked on ranks of X (predict_ranked.cu: a pass over X that finds them, and the walks); everything else, and what
+// the device declines to rank, is tiled:
+//
+// Design for B200: one launch for the whole ensemble (after one that packs the trees), everything a step of the walk touches
+// lives in shared memory.  The load/store data pipe of the SM is what bounds it (one pass per clock; a 4-byte load of
 // a warp is one pass, an 8-byte load two, plus one per bank conflict), so the layouts save passes:
 //   * A block owns a tile of rows (one thread per row); every thread stages its own row,
 //     feature-major with a pitch of one element per thread, so thread t only ever touches bank
 //     t mod 32 whatever feature a tree asks for: the x lookups of a walk never conflict.  Every row
-//     of X is read from HBM exactly once (16-byte loads, the rest of a sector comes from L1).
+//     of X is read from HBM once (16-byte loads, the rest of a sector comes from L1).
 //   * The trees are first packed into records: the splits of the heap, then the feature ids of a node and its
 //     two children in one word (10 bits each), then (one output) the bottom level of leaf values.  Two
 //     levels of a walk are two split loads, one feature load and two x loads: 5 passes for float32, where
@@ -245,8 +249,8 @@ struct TiledArgs {
 // KR: outputs whose sums a warp holds in registers (at most KR of them); 0: one output, leaf values in the
 // records; -1: any number of outputs, sums in shared memory.
 // Measured against {split, feature} nodes, a block barrier per group, 256 rows per block and every lane reading
-// its own row's values: 10M x 100 float32, 500 trees of depth 8: 23.2 -> 19.5 ms; 1M x 64 float64, 100 trees: 1117 -> 803
-// us; 100003 x 100, 10 outputs, 50 trees: 224 -> 131 us.
+// its own row's values: 100003 x 100, 10 outputs, 50 trees: 224 -> 131 us (now 107: kStaged); and, since then walked on ranks,
+// 10M x 100 float32, 500 trees of depth 8: 23.2 -> 19.5 ms, 1M x 64 float64, 100 trees: 1117 -> 803 us.
 // kStaged (KR > 0): the leaf values of several outputs are in the records too.
 // kGated: the launch stands in for the walk on ranks and does nothing where that was not declined.  A resident block then takes tile
 // after tile: a launch that finds nothing to do ends in 2.5 us, where a block per tile would come and go.
