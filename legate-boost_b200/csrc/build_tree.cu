@@ -784,6 +784,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       sl.f_end        = f_end;
       sl.derive       = derive || may_derive;
       sl.write_hist   = write_hist;
+      sl.cells        = N * F * K;
       sl.build_all    = lv.build_all;
       ScanSplit<T>(ctx, s, sl, F, row_ptr, cuts, S, qp, sp, tree, split_arrived, owned, stream);
       if (may_derive) {  // the other answer: one of the two launches does nothing

@@ -350,6 +350,7 @@ struct ScanSplitLevel {
   int f_begin, f_end;           // the features scanned and searched (the owned ones with several ranks)
   bool derive;                  // pairs of siblings, one of them built
   bool write_hist;
+  int64_t cells;                // of the matrix: rows x features x outputs
   const int* build_all = nullptr;  // device word (HistLevel): the call does nothing where it says the other of `derive`
 };
 // cuts: the split proposals, feature f's from f * cut_stride on.  arrived: one counter per tree node, zero

@@ -30,12 +30,20 @@ constexpr int kSplitWarps   = kSplitThreads / 32;
 // 48; ten outputs, 64 units 296 and 287, 32 units 167 and 177.  A warp's chain is as long as its feature has bins: with more than 256
 // (several outputs: 700) of them on average the line moves up with their number.  One output, 34 features, 256 units of 1000
 // bins 44 and 62, 150 features, 32 and 64 units of 1024 bins 126 and 152, 160 and 150, of 512 bins 69 and 55, 90 and 86.
+//
+// Units of a level need not exist: nodes of few or of pure rows do not split.  For matrices of which a level takes no more than tens of
+// microseconds anyway (kCountedCells) the kernel counts those that do, 1 to 2 us, and takes the other form if they are too
+// few.  5921 x 206, three classes, 16 units, most of them gone: 33 us with a block per feature, 64 with a warp, 40 with a block and
+// the count; five rounds 1915, 2098 and 1951.
 constexpr int kWideOutputs = 64;  // (what a block has room for)
-__host__ inline bool ScanIsWide(int64_t units, int n_features, int K, int64_t bins_per_feature)
+__host__ inline int64_t WideUnits(int n_features, int K, int64_t bins_per_feature)  // so many and the level is wide
 {
   const int64_t least = K <= 1 ? 1500 : K < 6 ? 1000 * K : 6000, usual = K <= 1 ? 256 : 700;
-  return K <= kWideOutputs && units * n_features * usual >= least * (bins_per_feature > usual ? bins_per_feature : usual);
+  const int64_t bins  = bins_per_feature > usual ? bins_per_feature : usual, one = usual * (n_features > 0 ? n_features : 1);
+  return K <= kWideOutputs ? (least * bins + one - 1) / one : INT64_MAX;
 }
+constexpr int kCountedUnits     = 4096;  // (more units are taken as they are)
+constexpr int64_t kCountedCells = int64_t{1} << 25;  // rows x features x outputs
 
 // What a rank knows about its best split of a node when the features are divided among the ranks:
 // the candidate and the sums left of it; K pairs follow the header.
@@ -83,6 +91,7 @@ struct ScanSplitParams {
   struct SliceBest* slice_best;  // [units][slices][2]
   unsigned int* arrived;
   unsigned char* records;
+  int wide_units;  // (kWide) with fewer units that exist a block takes a feature; 0: they are not counted
 };
 
 // The best candidate of one slice of a unit; with one output also the sums left of it.
@@ -105,7 +114,7 @@ struct SliceBest {
 // asked for before anything is made of the nodes' sums and whose two winners are written by a warp each (200k x 50: 8.7
 // -> 8.2 us a level).  There a thread takes a bin and not a warp a feature: a warp alone on its scheduler gets one
 // instruction in about five clocks, and a feature's instructions were 9 us longer whatever the level held.  On wide levels
-// (ScanIsWide) a warp takes a feature, 32 bins at a time.  Four blocks an SM and not three: 64 features, 8 and 16 units 11.2 and 16.9
+// (WideUnits) a warp takes a feature, 32 bins at a time.  Four blocks an SM and not three: 64 features, 8 and 16 units 11.2 and 16.9
 // us instead of 12.8 and 18.4, for spills that cost the upper levels 0.3.
 template <typename T, bool kManyOutputs, bool kDerive, bool kWide>
 __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
@@ -116,9 +125,10 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
   __shared__ SliceBest s_c[2][kSplitWarps];
   __shared__ SliceBest s_best[2];
   __shared__ bool s_last;
+  __shared__ int s_live[kWide ? kSplitWarps : 1];
   const ScanSplitLevel& lv = p.lv;
   if (lv.build_all != nullptr && (*lv.build_all != 0) == kDerive) return;
-  const int K = lv.K, unit = blockIdx.x, slices = gridDim.y;
+  const int K = lv.K, unit = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int node0 = lv.node_begin + (kDerive ? 2 * unit : unit);
   GPairI64* node_sums = p.tree.node_sums;
@@ -127,8 +137,26 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
   const GPairI64 sum_0 = LoadPair(node_sums + static_cast<int64_t>(node0) * K);
   const GPairI64 sum_1 = kDerive ? LoadPair(node_sums + static_cast<int64_t>(node0 + 1) * K) : GPairI64{0, 0};
   const QuantParams qp = *p.qp;
-  const int f_step = kWide ? kSplitWarps * slices : slices;
-  int f  = lv.f_begin + (kWide ? kSplitWarps * blockIdx.y + warp : blockIdx.y);
+  bool wide  = kWide;
+  int slices = gridDim.y;
+  if constexpr (kWide) {
+    const int units = gridDim.x;
+    if (p.wide_units > 0) {
+      int live = 0;
+      for (int i = tid; i < units; i += kSplitThreads) live += p.tree.feature[(lv.node_begin + (kDerive ? 2 * i : i) - 1) / 2] >= 0 ? 1 : 0;
+      live = __reduce_add_sync(0xffffffffu, live);
+      if (lane == 0) s_live[warp] = live;
+      __syncthreads();
+      live = 0;
+#pragma unroll
+      for (int w = 0; w < kSplitWarps; ++w) live += s_live[w];
+      wide = live >= p.wide_units;
+    }
+    if (wide) slices = min(slices, max((lv.f_end - lv.f_begin + kSplitWarps - 1) / kSplitWarps, 1));
+    if (static_cast<int>(blockIdx.y) >= slices) return;
+  }
+  const int f_step = wide ? kSplitWarps * slices : slices;
+  int f  = lv.f_begin + (wide ? kSplitWarps * blockIdx.y + warp : blockIdx.y);
   int fb = f < lv.f_end ? p.row_ptr[f] : 0, fe = f < lv.f_end ? p.row_ptr[f + 1] : 0;
   if (parent_feature < 0) return;  // the parent did not split: no such node
   // _a: the built node, _b: its sibling (SmallerChildIsLeft)
@@ -178,7 +206,7 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
       }
     }
   };
-  while (kWide && f < lv.f_end) {
+  while (wide && f < lv.f_end) {
     const bool search = p.sp.feature_set == nullptr || p.sp.feature_set[f] != 0;
     GPairI64* carry = s_carry + (kManyOutputs ? warp * K : 0);  // (several outputs: sums of the bins before)
     GPairI64 before{0, 0};
@@ -251,7 +279,7 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
     fb = p.row_ptr[f];
     fe = p.row_ptr[f + 1];
   }
-  while (!kWide && f < lv.f_end) {
+  while (!wide && f < lv.f_end) {
     const bool search = p.sp.feature_set == nullptr || p.sp.feature_set[f] != 0;
     for (int base = fb; base < fe; base += kSplitThreads) {
       const bool in = base + tid < fe;
@@ -496,11 +524,12 @@ void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, co
   const int n_features = lv.f_end - lv.f_begin;
   const int units      = lv.derive ? lv.n_nodes / 2 : lv.n_nodes;
   if (units <= 0) return;
-  const bool wide = ScanIsWide(units, n_features, lv.K, lv.bin_stride / F);
+  const int64_t wide_units = WideUnits(n_features, lv.K, lv.bin_stride / F);
+  const bool wide          = units >= wide_units;
   // with several outputs a block keeps K terms of two nodes and K running prefixes (of every warp) in shared memory
   const size_t smem = (lv.K > 1 ? sizeof(NodeTerms) * 2 * ((lv.K + 1) / 2 * 2) : 0) + lv.K * sizeof(GPairI64) * (wide ? kSplitWarps : 1);
-  // one feature per block (warp) until there are about sixteen blocks per SM, then several
-  int slices     = n_features > 0 ? (wide ? (n_features + kSplitWarps - 1) / kSplitWarps : n_features) : 1;
+  // one feature per block until there are about sixteen blocks per SM, then several
+  int slices     = n_features > 0 ? n_features : 1;
   const int most = (16 * ctx->sm_count + units - 1) / units;
   if (slices > most) slices = most;
   ScanSplitParams<T> p;
@@ -514,6 +543,7 @@ void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, co
   p.slice_best = slices > 1 ? s.alloc<SliceBest>(static_cast<size_t>(units) * slices * 2) : nullptr;
   p.arrived    = arrived;
   p.records    = nullptr;
+  p.wide_units = wide && lv.cells <= kCountedCells && units <= kCountedUnits && lv.node_begin > 0 ? static_cast<int>(wide_units) : 0;
   unsigned char *mine = nullptr, *all = nullptr;
   const size_t rb = SplitRecordBytes(lv.K);
   if (exchange_records) {

@@ -1480,6 +1480,23 @@ def test_wide_levels(lb, oracle, N, F, K, D, S, dt):
             assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
 
 
+@pytest.mark.parametrize("N,F,K,D,S", [(5_921, 206, 3, 7, 256), (25_053, 51, 1, 9, 256), (60_000, 40, 1, 8, 64), (9_001, 300, 1, 7, 300)])
+@pytest.mark.parametrize("pure", [0.0, 0.9])
+def test_wide_levels_of_few_nodes(lb, oracle, N, F, K, D, S, pure):
+    """Levels that are wide by their nodes, of which some or (rows of which most have the same gradient) few exist."""
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.RandomState(D)
+    X = rs.random((N, F)).astype(np.float32)
+    g = rs.normal(size=(N, K))
+    g[X[:, 0] < pure] = -1.0  # (nothing is to be gained below the split that takes these apart)
+    h = np.ones((N, K))
+    want = oracle.build_tree(X, g, h, max_depth=D, split_samples=S, seed=3, mode="Q")
+    got = build_tree_arrays(dev(X), dev(g), dev(h), max_depth=D, split_samples=S, seed=3, row_offset=0, dataset_rows=N)
+    for name in ("feature", "split_value", "node_sums", "gain", "hessian", "leaf_value"):
+        assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
+
+
 @pytest.mark.parametrize("N,F,K,D,dt", [
     (26_001, 20, 1, 6, np.float32), (32_768, 4, 1, 3, np.float64), (32_769, 4, 1, 3, np.float64),  # many rows; one too many
     (3_000, 64, 1, 9, np.float32), (900, 145, 1, 9, np.float64),  # a warp per pair of nodes, in whole and broken turns
