@@ -802,6 +802,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       pl.bins          = bins_t;
       pl.bin_bytes     = bin_bytes;
       pl.bin_pitch     = pitch_t;
+      pl.n_features    = F;
       pl.n_rows        = N;
       pl.row_index_in  = rows_a;
       pl.seg_begin     = seg_a;

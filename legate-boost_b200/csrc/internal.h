@@ -369,6 +369,7 @@ struct PartitionLevel {
   const void* bins;   // feature-major copy of the bin ids: bins[f * bin_pitch + row]
   int bin_bytes;
   int64_t bin_pitch;  // elements per feature
+  int n_features;
   int64_t n_rows;
   const int32_t* row_index_in;  // null: row i is at position i (the root)
   const int32_t* seg_begin;     // [n_nodes]

@@ -21,9 +21,16 @@ namespace lbk {
 namespace {
 
 constexpr int kPartThreads   = 256;
+constexpr int kPartWarps     = kPartThreads / 32;
 constexpr int kPartItems     = 8;
 constexpr int kPartTile      = kPartThreads * kPartItems;  // rows per chunk
 constexpr int kPartBlocks    = 4;    // per SM: as many as are resident
+// Bands of a level (see k_partition): as many as bring the columns of a band's rows to kPartBandBytes of L2, but with
+// kPartBandTurns chunks for every block, because a band is planned anew.  Levels 1 to 8 of 100M x 64: 4.83 ms with one turn,
+// 4.66 with two, 4.67 with four; 10M x 64, six levels: 339, 329 and 322 us; 130 million cells (1M x 128) and fewer have one band.
+constexpr int64_t kPartBandBytes = 24 << 20;
+constexpr int kPartBandTurns     = 4;
+constexpr int kPartMaxLogBands   = 7;
 constexpr int kPartPlanNodes = 1024;  // levels of up to this many nodes are planned inside the kernel
 
 __device__ inline int ChunksOf(const PartitionLevel& p, int j)
@@ -71,111 +78,210 @@ __global__ void __launch_bounds__(1024)
 }
 
 // Persistent blocks, a chunk at a time.  Bound by HBM: per row and level the row id, its pair and the
-// 32-byte sector of its bin in, row id and pair out.  Four blocks of 64 registers a thread are resident on an SM, and no
-// more are launched (six: the two that come later do their third of the chunks on a half-empty SM): 40M x 64, depth 8,
-// seven levels: 1.91 -> 1.60 ms, 10M: 454 -> 414 us; the second level 26 bytes per row at 5.0 TB/s.  512 threads with four rows
-// each: 1.70 ms; five blocks of 48 registers: 2.06 ms; the rows put in order in shared memory and written as
-// whole lines while the next chunk's are on their way: 1.77 ms.  kPlanInside: every block finds the chunks before
-// each node by itself (a scan of at most kPartPlanNodes counts once per block, about a microsecond,
+// byte of its bin in, row id and pair out.  Four blocks of 64 registers a thread are resident on an SM, and no
+// more are launched (six: the two that come later do their third of the chunks on a half-empty SM).  512 threads with four rows
+// each: 1.60 -> 1.70 ms at 40M x 64, depth 8; five blocks of 48 registers: 2.06 ms.  kPlanInside: every block finds the chunks before
+// each node by itself (a scan of at most kPartPlanNodes counts once per block and band, about a microsecond,
 // instead of a launch of its own).
-template <typename BinT, bool kPlanInside>
+//
+// A chunk is a chain of waits (row ids, bins, the claim), and the L1 holds what is on its way: shared memory taken from it costs more
+// than the loads it could hold (row ids and pairs staged there, six blocks, 28 KB of L1: level 8 of 100M x 64 1.26 -> 2.27 ms;
+// three stages of chunks of 1024 rows in a pipeline: 1.44).  So everything stays in registers, and the pairs are asked
+// for after the bins have come, while the room is claimed: level 0 435 -> 400 us, level 1 520 -> 488.
+//
+// Bands.  The rows of a node lie thin in the matrix at depth, so that a 64-byte piece of a column is fetched for one byte.  But
+// many nodes of a level split on the same few features, and their rows use other bytes of the same piece.  The chunks of
+// a level are therefore handed out in bands: band b of n has from every node the b-th n-th of its chunks, in the order
+// of the matrix, so that all nodes pass through the same rows at about the same time and a piece that one of them has
+// fetched is in L2 for the others.  A left child's rows lie in the order of the matrix, a right child's (filled from the end)
+// in the opposite one: its chunks are taken from its end, on every level.  (Upper levels gain nothing from their bands, but
+// keep the rows in order for the ones below: levels 5 to 8 778, 868, 952, 1125 us without, 592, 638, 669, 743 with them.)
+// 100M x 64, nine levels: 6.71 -> 5.07 ms, the last one 1.25 -> 0.74; 30M x 64, seven levels: 1.18 -> 1.08; 20M x 300: 1.08 -> 0.99.
+__device__ inline int BandBegin(int chunks, int band, int log_bands) { return static_cast<int>((static_cast<long long>(chunks) * band) >> log_bands); }
+
+// The whole block: off[j] = the sum of count(0 .. j - 1), off[n] = all of them.
+template <typename Count>
+__device__ inline void PlanInside(int n, Count count, int32_t* off /* [kPartPlanNodes + 1] */, int* wsum /* [kPartWarps] */)
+{
+  constexpr int kPer = kPartPlanNodes / kPartThreads;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int c[kPer], sum = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int j = tid * kPer + i;
+    c[i]        = j < n ? count(j) : 0;
+    sum += c[i];
+  }
+  int incl = sum;
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  if (lane == 31) wsum[warp] = incl;
+  __syncthreads();  // (and whoever still looks for a node of the band before)
+  int before = incl - sum;
+  for (int w = 0; w < warp; ++w) before += wsum[w];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int j = tid * kPer + i;
+    if (j < n) off[j] = before;
+    before += c[i];
+    if (j == n - 1) off[n] = before;
+  }
+  __syncthreads();
+}
+
+__device__ inline int LoadOnce(const int32_t* a)
+{
+  int v;
+  asm volatile("ld.global.cs.s32 %0, [%1];\n" : "=r"(v) : "l"(a));
+  return v;
+}
+__device__ inline int2 LoadOnce(const int2* a)
+{
+  int2 v;
+  asm volatile("ld.global.cs.v2.s32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "l"(a));
+  return v;
+}
+template <bool kL2Only>
+__device__ inline int LoadBin(const uint8_t* a)
+{
+  unsigned short v;
+  if (kL2Only) asm volatile("ld.global.cg.u8 %0, [%1];\n" : "=h"(v) : "l"(a));
+  else asm volatile("ld.global.u8 %0, [%1];\n" : "=h"(v) : "l"(a));
+  return v;
+}
+template <bool kL2Only>
+__device__ inline int LoadBin(const uint16_t* a)
+{
+  unsigned short v;
+  if (kL2Only) asm volatile("ld.global.cg.u16 %0, [%1];\n" : "=h"(v) : "l"(a));
+  else asm volatile("ld.global.u16 %0, [%1];\n" : "=h"(v) : "l"(a));
+  return v;
+}
+
+template <typename BinT, bool kPlanInside, bool kBands>
 __global__ void __launch_bounds__(kPartThreads, kPartBlocks)
-  k_partition(const __grid_constant__ PartitionLevel p, const int32_t* __restrict__ chunk_off_global)
+  k_partition(const __grid_constant__ PartitionLevel p, const int32_t* __restrict__ chunk_off_global, int log_bands)
 {
   __shared__ int32_t s_off[kPlanInside ? kPartPlanNodes + 1 : 1];
-  __shared__ int s_cnt[kPartItems * kPartThreads / 32];  // per (item, warp): lefts | rows << 16, then prefixes
-  __shared__ int s_wsum[kPartThreads / 32];
+  __shared__ int32_t s_count[kBands ? kPartPlanNodes : 1];
+  __shared__ int32_t s_band[kBands ? (1 << kPartMaxLogBands) + 1 : 1];  // chunks before each band
+  __shared__ int s_cnt[kPartItems * kPartWarps];  // per (item, warp): lefts | rows << 16, then prefixes
+  __shared__ int s_wsum[kPartWarps];
   __shared__ int s_base[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n   = p.n_nodes;
-  const int32_t* chunk_off = chunk_off_global;
-  if (kPlanInside) {
-    constexpr int kPer = kPartPlanNodes / kPartThreads;
-    int c[kPer], sum = 0;
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int j = tid * kPer + i;
-      c[i]        = j < n ? ChunksOf(p, j) : 0;
-      sum += c[i];
-    }
-    int incl = sum;
-    for (int off = 1; off < 32; off <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += v;
-    }
-    if (lane == 31) s_wsum[warp] = incl;
+  const int32_t* chunk_off = kPlanInside ? s_off : chunk_off_global;
+  int band = -1, total;
+  if (kBands) {
+    // where every band begins: the nodes are divided among the threads of a band
+    const int bands = 1 << log_bands, parts = kPartThreads >> log_bands;
+    for (int j = tid; j < n; j += kPartThreads) s_count[j] = ChunksOf(p, j);
+    for (int i = tid; i <= bands; i += kPartThreads) s_band[i] = 0;
     __syncthreads();
-    int before = incl - sum;
-    for (int w = 0; w < warp; ++w) before += s_wsum[w];
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int j = tid * kPer + i;
-      if (j < n) s_off[j] = before;
-      before += c[i];
-      if (j == n - 1) s_off[n] = before;
-    }
+    int sum = 0;
+    for (int j = tid >> log_bands; j < n; j += parts) sum += BandBegin(s_count[j], (tid & (bands - 1)) + 1, log_bands);
+    atomicAdd(&s_band[(tid & (bands - 1)) + 1], sum);
     __syncthreads();
-    chunk_off = s_off;
+    total = s_band[bands];
+  } else {
+    if (kPlanInside) PlanInside(n, [&](int j) { return ChunksOf(p, j); }, s_off, s_wsum);
+    total = chunk_off[n];
   }
   // nodes that were not split, or have no rows here, leave two empty segments
   for (int j = blockIdx.x * kPartThreads + tid; j < n; j += gridDim.x * kPartThreads) {
-    if (chunk_off[j + 1] == chunk_off[j]) {
+    if ((kBands ? s_count[j] : chunk_off[j + 1] - chunk_off[j]) == 0) {
       p.seg_begin_out[2 * j] = p.seg_end_out[2 * j] = 0;
       p.seg_begin_out[2 * j + 1] = p.seg_end_out[2 * j + 1] = 0;
     }
   }
-  const int total = chunk_off[n];
-  for (int c = blockIdx.x; c < total; c += gridDim.x) {
+  // The c-th chunk of the level (the whole block asks, in ascending order).
+  struct Chunk {
+    int j, begin, rows;
+  };
+  auto chunk_at = [&](int c) -> Chunk {
+    if (c >= total) return Chunk{0, 0, 0};
+    if (kBands) {
+      int b = max(band, 0);
+      while (c >= s_band[b + 1]) ++b;
+      if (b != band) {
+        band = b;
+        PlanInside(n, [&](int j) { return BandBegin(s_count[j], b + 1, log_bands) - BandBegin(s_count[j], b, log_bands); }, s_off, s_wsum);
+      }
+      c -= s_band[band];
+    }
     int lo = 0, hi = n;  // last node with chunk_off <= c
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
       if (chunk_off[mid] <= c) lo = mid; else hi = mid;
     }
-    const int j    = lo;
-    const int node = p.node_begin + j;
-    const int sb   = p.split_bin[node];
-    const int nb = p.seg_begin[j], ne = p.seg_end[j];
-    const int rb = nb + (c - chunk_off[j]) * kPartTile;
-    const int re = min(ne, rb + kPartTile);
+    int i = c - chunk_off[lo];
+    if (kBands) {
+      i += BandBegin(s_count[lo], band, log_bands);
+      if (lo & 1) i = s_count[lo] - 1 - i;
+    }
+    const int begin = p.seg_begin[lo] + i * kPartTile;
+    return Chunk{lo, begin, min(p.seg_end[lo] - begin, kPartTile)};
+  };
+  const bool move_pairs = p.pairs_in != nullptr && p.K == 1;  // (of several outputs: read where they are written)
+  for (int c = blockIdx.x;; c += gridDim.x) {
+    const Chunk a = chunk_at(c);
+    if (a.rows == 0) break;
+    const int node  = p.node_begin + a.j;
+    const int sb    = p.split_bin[node];
     const BinT* col = static_cast<const BinT*>(p.bins) + static_cast<int64_t>(p.feature[node]) * p.bin_pitch;
-    int rid[kPartItems];
+    // The loads in this order (as volatile statements, so that all of a kind are on their way before one is waited for).
+    int rid[kPartItems], bin[kPartItems];
     int2 pair[kPartItems];
-    unsigned ml[kPartItems], mv[kPartItems];
+    const bool whole = a.rows == kPartTile;
+    auto at = [&](int i) -> int {  // position of the thread's i-th row in the chunk (of the chunk's last row, if it has none)
+      const int e = i * kPartThreads + tid;
+      return whole ? e : min(e, a.rows - 1);
+    };
+    if (p.row_index_in != nullptr) {
+      const int32_t* from = p.row_index_in + a.begin;
+#pragma unroll
+      for (int i = 0; i < kPartItems; ++i) rid[i] = LoadOnce(from + at(i));
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPartItems; ++i) rid[i] = a.begin + at(i);
+    }
+    auto load_pairs = [&]() {
+      const int2* from = p.pairs_in + a.begin;
+#pragma unroll
+      for (int i = 0; i < kPartItems; ++i) pair[i] = LoadOnce(from + at(i));
+    };
+#pragma unroll
+    for (int i = 0; i < kPartItems; ++i) bin[i] = LoadBin<kBands>(col + rid[i]);
+    unsigned ml[kPartItems];
+    // lanes of item i that hold a row
+    auto valid = [&](int i) -> unsigned {
+      const int left = a.rows - i * kPartThreads - warp * 32;
+      return left >= 32 ? 0xffffffffu : left <= 0 ? 0u : (1u << left) - 1u;
+    };
 #pragma unroll
     for (int i = 0; i < kPartItems; ++i) {
-      const int r = rb + i * kPartThreads + tid;
-      rid[i]      = r < re ? (p.row_index_in != nullptr ? __ldcs(p.row_index_in + r) : r) : 0;
+      const unsigned mv = valid(i);
+      ml[i]             = __ballot_sync(0xffffffffu, bin[i] <= sb) & mv;
+      if (lane == 0) s_cnt[i * kPartWarps + warp] = __popc(ml[i]) | (__popc(mv) << 16);
     }
-    if (p.pairs_in != nullptr && p.K == 1) {
-#pragma unroll
-      for (int i = 0; i < kPartItems; ++i) {
-        const int r = rb + i * kPartThreads + tid;
-        if (r < re) pair[i] = __ldcs(p.pairs_in + r);
-      }
-    }
-    int bin[kPartItems];
-#pragma unroll
-    for (int i = 0; i < kPartItems; ++i) bin[i] = rb + i * kPartThreads + tid < re ? static_cast<int>(col[rid[i]]) : 0;
-#pragma unroll
-    for (int i = 0; i < kPartItems; ++i) {
-      const bool in = rb + i * kPartThreads + tid < re;
-      mv[i]         = __ballot_sync(0xffffffffu, in);
-      ml[i]         = __ballot_sync(0xffffffffu, in && bin[i] <= sb);
-      if (lane == 0) s_cnt[i * (kPartThreads / 32) + warp] = __popc(ml[i]) | (__popc(mv[i]) << 16);
-    }
+    if (move_pairs) load_pairs();
     __syncthreads();
     if (warp == 0) {
       // 64 counts, two per lane, in (item, warp) order = row order
-      const int a = s_cnt[2 * lane], b = s_cnt[2 * lane + 1];
-      int incl = a + b;
+      static_assert(kPartItems * kPartWarps == 64, "two counts per lane");
+      const int x = s_cnt[2 * lane], y = s_cnt[2 * lane + 1];
+      int incl = x + y;
       for (int off = 1; off < 32; off <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, incl, off);
         if (lane >= off) incl += v;
       }
-      const int excl      = incl - a - b;
+      const int excl      = incl - x - y;
       s_cnt[2 * lane]     = excl;
-      s_cnt[2 * lane + 1] = excl + a;
+      s_cnt[2 * lane + 1] = excl + x;
       if (lane == 31) {
+        const int nb = p.seg_begin[a.j], ne = p.seg_end[a.j];
         const int lefts = incl & 0xffff, rights = (incl >> 16) - lefts;
         const unsigned long long old =
           atomicAdd(p.cursor + node, static_cast<unsigned long long>(lefts) | (static_cast<unsigned long long>(rights) << 32));
@@ -183,10 +289,10 @@ __global__ void __launch_bounds__(kPartThreads, kPartBlocks)
         s_base[0] = nb + l0;
         s_base[1] = ne - r0 - rights;
         if (l0 + lefts + r0 + rights == ne - nb) {
-          p.seg_begin_out[2 * j]     = nb;
-          p.seg_end_out[2 * j]       = nb + l0 + lefts;
-          p.seg_begin_out[2 * j + 1] = nb + l0 + lefts;
-          p.seg_end_out[2 * j + 1]   = ne;
+          p.seg_begin_out[2 * a.j]     = nb;
+          p.seg_end_out[2 * a.j]       = nb + l0 + lefts;
+          p.seg_begin_out[2 * a.j + 1] = nb + l0 + lefts;
+          p.seg_end_out[2 * a.j + 1]   = ne;
         }
       }
     }
@@ -194,25 +300,29 @@ __global__ void __launch_bounds__(kPartThreads, kPartBlocks)
     const unsigned below = (1u << lane) - 1u;
 #pragma unroll
     for (int i = 0; i < kPartItems; ++i) {
-      const int r = rb + i * kPartThreads + tid;
-      if (r < re) {
-        const int before = s_cnt[i * (kPartThreads / 32) + warp];
+      const int e = i * kPartThreads + tid;
+      if (e < a.rows) {
+        const int before = s_cnt[i * kPartWarps + warp];
         const int lefts = before & 0xffff, rights = (before >> 16) - lefts;
         const int pos = (ml[i] >> lane) & 1u ? s_base[0] + lefts + __popc(ml[i] & below)
-                                             : s_base[1] + rights + __popc(mv[i] & ~ml[i] & below);
+                                             : s_base[1] + rights + __popc(~ml[i] & below);
         p.row_index_out[pos] = rid[i];
-        if (p.pairs_in != nullptr) {
-          if (p.K == 1) {
-            p.pairs_out[pos] = pair[i];
-          } else {
-            for (int k = 0; k < p.K; ++k)
-              p.pairs_out[static_cast<int64_t>(pos) * p.K + k] = p.pairs_in[static_cast<int64_t>(r) * p.K + k];
-          }
+        if (move_pairs) {
+          p.pairs_out[pos] = pair[i];
+        } else if (p.pairs_in != nullptr) {
+          for (int k = 0; k < p.K; ++k)
+            p.pairs_out[static_cast<int64_t>(pos) * p.K + k] = p.pairs_in[static_cast<int64_t>(a.begin + e) * p.K + k];
         }
       }
     }
     __syncthreads();  // s_cnt, s_base are written again
   }
+}
+
+template <typename BinT>
+auto PartitionKernel(bool inside, bool bands)
+{
+  return bands ? k_partition<BinT, true, true> : inside ? k_partition<BinT, true, false> : k_partition<BinT, false, false>;
 }
 
 }  // namespace
@@ -234,9 +344,13 @@ void PartitionRows(lbk_context* ctx, Scratch& s, const PartitionLevel& pl, cudaS
     k_part_plan<<<1, 1024, 0, stream>>>(pl, chunk_off);
     LBK_LAUNCH_CHECK();
   }
-  auto fn = pl.bin_bytes == 1 ? (inside ? k_partition<uint8_t, true> : k_partition<uint8_t, false>)
-                              : (inside ? k_partition<uint16_t, true> : k_partition<uint16_t, false>);
-  fn<<<grid, kPartThreads, 0, stream>>>(pl, chunk_off);
+  int log_bands = 0;
+  if (inside && pl.n_nodes > 1)
+    while (log_bands < kPartMaxLogBands && (pl.n_rows * pl.n_features * pl.bin_bytes) >> log_bands > kPartBandBytes &&
+           (pl.n_rows / kPartTile) >> (log_bands + 1) >= kPartBandTurns * grid)
+      ++log_bands;
+  auto fn = pl.bin_bytes == 1 ? PartitionKernel<uint8_t>(inside, log_bands > 0) : PartitionKernel<uint16_t>(inside, log_bands > 0);
+  fn<<<grid, kPartThreads, 0, stream>>>(pl, chunk_off, log_bands);
   LBK_LAUNCH_CHECK();
 }
 

@@ -312,6 +312,27 @@ def test_scratch_through_the_callers_allocator(lb):
 
 
 @pytest.mark.parametrize("N,F,K,D,S,dtype", [
+    (20_000_003, 3, 1, 7, 256, np.float32),   # four bands, one-byte ids, a ragged last chunk
+    (10_000_001, 4, 1, 6, 600, np.float64),   # two bands, two-byte ids
+    (10_000_001, 5, 2, 5, 64, np.float32),    # two outputs: the pairs are read where they are written
+])
+def test_trees_of_levels_in_bands(lb, oracle, N, F, K, D, S, dtype):
+    """Levels of large matrices are repartitioned in bands of rows, right children from their end: the tree, and with it the
+    sums of every node below, are the oracle's bit for bit."""
+    from legateboost_b200.tree import build_tree_arrays
+
+    rs = np.random.default_rng(N)
+    X = rs.random((N, F), dtype=np.float32).astype(dtype)
+    X[:, 1] = np.round(X[:, 1] * 50)
+    g, h = rs.random((N, K)) - 0.5 + 0.3 * np.sin(9 * X[:, :1]), rs.random((N, K)) + 0.1
+    want = oracle.build_tree(X, g, h, max_depth=D, split_samples=S, seed=3, mode="Q")
+    got = build_tree_arrays(dev(X), dev(g), dev(h), max_depth=D, split_samples=S, seed=3, row_offset=0, dataset_rows=N)
+    assert (want.feature >= 0).sum() > 2 ** (D - 1)
+    for name in ("feature", "split_value", "gain", "leaf_value", "hessian"):
+        assert np.array_equal(got[name].cpu().numpy(), getattr(want, name)), name
+
+
+@pytest.mark.parametrize("N,F,K,D,S,dtype", [
     (50001, 40, 1, 8, 256, np.float32),    # rows of 64 bytes, a last chunk of one row
     (20000, 7, 2, 5, 64, np.float64),      # one group
     (9000, 130, 1, 6, 256, np.float32),    # rows of 160 bytes
