@@ -35,6 +35,7 @@
 //     waits (k_hist_smem); chunks of <= 128 rows skip shared memory.
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "device_utils.cuh"
 #include "internal.h"
@@ -132,6 +133,47 @@ __device__ inline out_t* FeatureBase(const HistParams& p, int f, int seg)
          static_cast<long long>(seg) * p.push_len + (p.row_ptr[f] - lo);
 }
 
+// How the lanes of k_hist_smem share the nt features of a unit: `main` neighbouring bytes a lane and `extra` ones.  Each of the
+// two takes a power of two of features and eight (W = 1: the main ones sixteen) columns of words for each lane of a row, so that
+// fewer features have several copies of their words and a step still updates 32 banks; 2 (main + extra) reductions are issued per
+// batch of rows instead of 32.  Whole numbers use it where a row is one unit: 8M x 40, 4 nodes 200 -> 185 us, 10M x 40, depth 8
+// 2.65 -> 2.62 ms.  Of several units the last one keeps its 16 steps, so that the units' blocks go through the rows at one
+// pace and share the 128-byte lines of a row in L2: with the steps it needs (and blocks dealt by what a unit costs) 8M x 72
+// took 427 -> 528 us and 10M x 200, depth 8, 8.7 -> 9.6 ms, without the dealing 1M x 72, ten outputs, 6.93 -> 7.15 ms.
+// Floating-point reductions are loops where another one of the same word is on its way, and the columns that pad a row all fall
+// into their bin 0: there every unit has the steps it needs, and lanes without a feature leave a step out (HistRows, kMask).
+// 3M x 100 1222 -> 429 us, 3M x 20 341 -> 151, 3M x 64 256 -> 242.
+struct UnitForm {
+  int main, extra;
+};
+__device__ constexpr UnitForm FormOf(bool is_float, int W, bool several_units, int nt)
+{
+  if (W == 1) return {nt > 16 ? 16 : nt > 8 ? 8 : 4, 0};
+  if (nt > 48 || (!is_float && several_units)) return {8, 8};
+  if (!is_float) return {8, 4};
+  if (nt > 32) return {8, nt > 40 ? 4 : nt > 36 ? 2 : 1};
+  return {nt > 16 ? 8 : nt > 8 ? 4 : 2, 0};
+}
+// Feature (relative to the unit's first) of histogram word w of a bin, -1 where the word is a copy of another one.
+__device__ constexpr int FeatureOfWord(int W, UnitForm fm, int w)
+{
+  if (W == 1) {
+    const int q = w >> 4, col = w & 15;
+    return col < fm.main ? fm.main * q + col : -1;
+  }
+  const int half = w >> 5, q = (w >> 3) & 3, col = w & 7;
+  if (col >= (half == 0 ? fm.main : fm.extra)) return -1;
+  if (fm.extra == 8) return 16 * q + 8 * half + col;
+  if (fm.extra == 0) return fm.main * q + col;
+  // 33 to 48 features: lanes 0 and 3 share the first 16 bytes, lanes 1 and 2 have the next 32
+  if (half == 0) {
+    if (fm.extra == 1 && q == 2 && col >= 4) return 24 + (col - 4);
+    return (q == 0 ? 0 : q == 3 ? 8 : 16 * q) + col;
+  }
+  if (fm.extra == 1) return 28 + q;
+  if (fm.extra == 2) return 24 + 2 * q + col;
+  return (q == 0 ? 28 : q == 1 ? 24 : q == 2 ? 40 : 44) + col;
+}
 __device__ inline unsigned SmemAddr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
 
 // largest |grad| and |hess| of a set of quantised pairs (for the stage-level entry point; the
@@ -562,9 +604,10 @@ __global__ void __launch_bounds__(kHistThreads)
 // One update step of a lane: byte J of its 16 bin bytes (already permuted so that step J reads
 // the static byte J), both words of the pair.  `lane_word` is the shared-memory address of the
 // lane's word in bin row 0 of the gradient histogram.
-template <typename A, int W, int J>
-__device__ inline void HistStep(const unsigned (&x)[4], unsigned lane_word, const int2& v)
+template <typename A, int W, int J, bool kMask>
+__device__ inline void HistStep(const unsigned (&x)[4], unsigned lane_word, const int2& v, unsigned steps)
 {
+  if (kMask && (steps >> J & 1u) == 0u) return;
   constexpr int kHistBytes = kSmemBins * kGroup * W * 4;
   if (W == 2) {
     // a bin row is 256 bytes: the offset is (bin << 8) | (lane_word ^ skew), one byte permute and one
@@ -584,59 +627,108 @@ __device__ inline void HistStep(const unsigned (&x)[4], unsigned lane_word, cons
   }
 }
 
+template <typename A, int W, int kFrom, int kTo, bool kMask>
+__device__ inline void HistSteps(const unsigned (&x)[4], unsigned lane_word, const int2& v, unsigned steps)
+{
+  if constexpr (kFrom < kTo) {
+    HistStep<A, W, kFrom, kMask>(x, lane_word, v, steps);
+    HistSteps<A, W, kFrom + 1, kTo, kMask>(x, lane_word, v, steps);
+  }
+}
+
 // The rows [sb, se) of row_index, all of one node, added to the block's private histograms: the
 // main loop of k_hist_smem for one warp.  The warps of the block take the batches of 32 / (2 W)
 // rows in turn.  Every load of the loop is unconditional: batch numbers beyond the warp's last one
-// are clamped to it (the rows are fetched again and dropped), lanes whose feature group does not
-// exist read the group that does and add zero pairs, and the last, partial batch of the range is
+// are clamped to it (the rows are fetched again and dropped), and the last, partial batch of the range is
 // handled after the loop.  In flight per warp: the rows of the next two batches and the row ids of
 // the two after; the loop is unrolled three times so that the three row buffers rotate by name.
-// The row's bin bytes come with a plain load that bypasses L1 and asks L2 for the whole 128-byte
-// line (the other half of the row is wanted soon by the block that builds the neighbouring
-// groups).  kOrder: kPairsByPosition - the pairs are stored in row_index order and read as a stream;
+// The row's bin bytes come with a plain load that bypasses L1 and, where a row is longer than a unit's 64 bytes (kLine),
+// asks L2 for the whole 128-byte line (the other half of the row is wanted soon by the block that builds the neighbouring
+// groups).  A row of 64 bytes has its neighbour in the other half: asking for 128 brought 132 bytes a row from DRAM where a node
+// has one row in 64, now 79 (100M x 64, depth 10: 26.2 -> 25.2 ms).  kOrder: kPairsByPosition - the pairs are stored in row_index order and read as a stream;
 // kPairsByRow - they are gathered by row id; kRowsInOrder - there is no row_index, row i is at position i.
+//
+// kMain, kExtra: the form of the unit (UnitForm).  Of 33 to 48 features (kExtra 1, 2, 4) the 16-byte loads are not as the steps
+// want them: lane 3 takes the upper half of lane 0's piece, and a word or two go from lane 1 (and 2) to the others by shuffle,
+// cheaper than a second load, which would touch the row's line again.
 enum RowOrder { kPairsByRow, kPairsByPosition, kRowsInOrder };
-template <typename A, int W, RowOrder kOrder>
-__device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, int g0, int groups, int k, int warp,
-                                         int lane, unsigned lane_word)
+template <typename A, int W, RowOrder kOrder, int kMain, int kExtra, bool kLine, bool kMask>
+__device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, int g0, int k, int warp, int lane, unsigned lane_word)
 {
   using in_t = typename A::in_t;
   constexpr int kWarps        = kHistThreads * W / 32;
   constexpr int kLanesPerRow  = 2 * W;
   constexpr int kRowsPerBatch = 32 / kLanesPerRow;
+  constexpr int kLoad         = kExtra != 0 ? 16 : kMain;  // bytes of a lane's load
+  constexpr bool kShared      = kExtra == 1 || kExtra == 2 || kExtra == 4;
   const unsigned rslot = lane / kLanesPerRow, q = lane % kLanesPerRow;
   const unsigned wsel = rslot >> 2, bsel = rslot & 3;
   const unsigned perm = bsel == 0 ? 0x3210u : bsel == 1 ? 0x2301u : bsel == 2 ? 0x1032u : 0x0123u;
   const unsigned sel0 = perm + ((wsel & 1) ? 0x4444u : 0u), sel1 = perm + ((wsel & 1) ? 0u : 0x4444u);
-  const bool lane_on  = static_cast<int>(q >> 1) < groups;  // the group this lane's 16 bytes belong to exists
-  const unsigned q_eff = lane_on ? q : (q & 1u);
-  const int pair_mask  = lane_on ? -1 : 0;
-  const int64_t pitch  = static_cast<int64_t>(p.G) * kGroup;
-  const unsigned char* gb = static_cast<const unsigned char*>(p.bins) + g0 * kGroup + q_eff * 16;
+  const unsigned sel2 = (rslot & 1) ? 0x4401u : 0x4410u;  // two bytes
+  const unsigned from = kShared && q == 3 ? 0u : q;       // the lane's piece of the row
+  const int64_t pitch = static_cast<int64_t>(p.G) * kGroup;
+  const unsigned char* gb = static_cast<const unsigned char*>(p.bins) + g0 * kGroup + from * kLoad;
+  unsigned steps = 0u;  // kMask: those in which the lane has a feature
+  if (kMask) {
+#pragma unroll 1
+    for (int j = 0; j < 16; ++j) {
+      const int n = W == 1 || j < 8 ? kMain : kExtra, col = (static_cast<int>(rslot) ^ j) & (n - 1);
+      const int w = W == 1 ? 16 * static_cast<int>(q) + col : 32 * (j >> 3) + 8 * static_cast<int>(q) + col;
+      if (n > 0 && g0 * kGroup + FeatureOfWord(W, UnitForm{kMain, kExtra}, w) < p.F) steps |= 1u << j;
+    }
+  }
   const in_t* gpair    = static_cast<const in_t*>(p.gpair);
   const int pos0       = sb + static_cast<int>(rslot);  // the lane's row of batch 0, as a position in row_index
   const int32_t* rp    = p.row_index + pos0;            // + batch * kRowsPerBatch
 
   // rid: the row; pos: its position in row_index (only used for pairs stored by position)
   auto load = [&](int rid, int pos, int4& w, int2& v) {
-    const int4* ap = reinterpret_cast<const int4*>(gb + static_cast<int64_t>(rid) * pitch);
-    asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.s32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
-                 : "l"(ap));
+    const unsigned char* ap = gb + static_cast<int64_t>(rid) * pitch;
+    if (kLoad == 16 && kLine) {
+      asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "l"(ap));
+    } else if (kLoad == 16) {
+      asm volatile("ld.global.nc.L1::no_allocate.L2::64B.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "l"(ap));
+    } else if (kLoad == 8) {
+      asm volatile("ld.global.nc.L1::no_allocate.L2::64B.v2.s32 {%0,%1}, [%2];" : "=r"(w.x), "=r"(w.y) : "l"(ap));
+    } else if (kLoad == 4) {
+      asm volatile("ld.global.nc.L1::no_allocate.L2::64B.s32 %0, [%1];" : "=r"(w.x) : "l"(ap));
+    } else {
+      asm volatile("{.reg .u16 t; ld.global.nc.L1::no_allocate.L2::64B.u16 t, [%1]; cvt.u32.u16 %0, t;}" : "=r"(w.x) : "l"(ap));
+    }
     if (kOrder != kPairsByRow) v = __ldcs(reinterpret_cast<const int2*>(gpair + static_cast<int64_t>(pos) * p.K + k));
     else v = __ldcg(reinterpret_cast<const int2*>(gpair + static_cast<int64_t>(rid) * p.K + k));
-    if (W == 2) {
-      v.x &= pair_mask;
-      v.y &= pair_mask;
-    }
   };
   auto consume = [&](const int4& w, const int2& v) {
-    unsigned x[4];
-    if (W == 2) {
+    unsigned x[4] = {};
+    if (kShared) {
+      const int l1 = lane - static_cast<int>(q) + 1;  // the row's lane 1
+      int m0 = q == 3 ? w.z : w.x, m1 = q == 3 ? w.w : w.y;
+      if (kExtra == 4) {
+        const int other = __shfl_sync(0xffffffffu, w.w, q == 3 ? l1 + 1 : l1);
+        x[2]            = __byte_perm(q == 1 || q == 2 ? w.z : other, 0, perm);
+      } else {
+        const int s6 = __shfl_sync(0xffffffffu, w.z, l1), s7 = __shfl_sync(0xffffffffu, w.w, l1);
+        if (kExtra == 1) {
+          x[2] = __byte_perm(s7, 0, 0x4440u | q);
+          if (q == 2) m1 = s6;
+        } else {
+          x[2] = __byte_perm(s6, s7, (sel2 & 0xffu) + 0x22u * q);
+        }
+      }
+      x[0] = __byte_perm(m0, m1, sel0);
+      x[1] = __byte_perm(m0, m1, sel1);
+    } else if (kMain == 2) {
+      x[0] = __byte_perm(w.x, 0, sel2);
+    } else if (kMain == 4) {
+      x[0] = __byte_perm(w.x, 0, perm);
+    } else if (kMain == 8) {
       x[0] = __byte_perm(w.x, w.y, sel0);
       x[1] = __byte_perm(w.x, w.y, sel1);
-      x[2] = __byte_perm(w.z, w.w, sel0);
-      x[3] = __byte_perm(w.z, w.w, sel1);
+      if (kExtra == 8) {
+        x[2] = __byte_perm(w.z, w.w, sel0);
+        x[3] = __byte_perm(w.z, w.w, sel1);
+      }
     } else {
       const unsigned a0 = (wsel & 2) ? w.z : w.x, a1 = (wsel & 2) ? w.w : w.y;
       const unsigned b0 = (wsel & 2) ? w.x : w.z, b1 = (wsel & 2) ? w.y : w.w;
@@ -645,22 +737,8 @@ __device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, in
       x[2] = __byte_perm(b0, b1, sel0);
       x[3] = __byte_perm(b0, b1, sel1);
     }
-    HistStep<A, W, 0>(x, lane_word, v);
-    HistStep<A, W, 1>(x, lane_word, v);
-    HistStep<A, W, 2>(x, lane_word, v);
-    HistStep<A, W, 3>(x, lane_word, v);
-    HistStep<A, W, 4>(x, lane_word, v);
-    HistStep<A, W, 5>(x, lane_word, v);
-    HistStep<A, W, 6>(x, lane_word, v);
-    HistStep<A, W, 7>(x, lane_word, v);
-    HistStep<A, W, 8>(x, lane_word, v);
-    HistStep<A, W, 9>(x, lane_word, v);
-    HistStep<A, W, 10>(x, lane_word, v);
-    HistStep<A, W, 11>(x, lane_word, v);
-    HistStep<A, W, 12>(x, lane_word, v);
-    HistStep<A, W, 13>(x, lane_word, v);
-    HistStep<A, W, 14>(x, lane_word, v);
-    HistStep<A, W, 15>(x, lane_word, v);
+    HistSteps<A, W, 0, kMain, kMask>(x, lane_word, v, steps);
+    HistSteps<A, W, 8, 8 + kExtra, kMask>(x, lane_word, v, steps);
   };
 
   const int n_here  = se - sb;
@@ -756,7 +834,7 @@ __device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, in
 // adds one to the counter of its group of four; the last one to arrive adds the others' slots to its own sums and goes on
 // as one member of the next level, until one block holds the node's total and writes the histogram.  Nobody waits for
 // anybody: whoever arrives first leaves.  (lbk_selftest_histogram takes it with local histograms.)
-template <bool kFloat, int W, RowOrder kOrder>
+template <bool kFloat, int W, RowOrder kOrder, bool kLine>
 __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
   k_hist_smem(const HistParams p)
 {
@@ -773,8 +851,8 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
   constexpr int kStageWords   = kFlushBins * 32;  // per warp
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned int s_ticket;
-  __shared__ int s_rp[kCols + 1];  // row_ptr of the unit's features (clamped at F)
-  __shared__ typename Acc<kFloat>::out_t* s_base[kCols];  // where bin 0 of each of them goes, for the piece at hand
+  __shared__ int s_nb[kCols];  // bins of the feature of each word (0: no feature, or a copy of another word)
+  __shared__ typename Acc<kFloat>::out_t* s_base[kCols];  // where its bin 0 goes, for the piece at hand
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned base = SmemAddr(smem_raw);
@@ -817,8 +895,6 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
   const int64_t pitch   = static_cast<int64_t>(p.G) * kGroup;  // bins are row-major, rows padded to whole groups
   // chunks that merge through slots never flush in the middle: they stay below the safe count
   const int cap_rows    = rows_safe >= (1 << 30) ? (1 << 30) : (rows_safe & ~(kTileRows - 1));
-  // feature (relative to the unit's first) of histogram word w
-  auto feature_of_word = [](int w) -> int { return W == 1 ? w : 16 * ((w >> 3) & 3) + 8 * (w >> 5) + (w & 7); };
 
   const unsigned rslot    = lane / kLanesPerRow, q = lane % kLanesPerRow;
   const unsigned wsel     = rslot >> 2, bsel = rslot & 3;
@@ -847,11 +923,13 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
       DirectRows<uint8_t, A>(p, pc.rb, pc.re, g0 * kGroup, groups, k, seg, warp, kWarps, lane);
       return;
     }
-    __syncthreads();  // whoever still reads the histogram or s_rp of the piece before
-    for (int i = tid; i <= kCols; i += kThreads) {
-      const int f = g0 * kGroup + i;
-      s_rp[i]     = p.row_ptr[min(p.F, f)];
-      if (i < kCols) s_base[i] = f < p.F ? FeatureBase<out_t>(p, f, seg) : nullptr;
+    __syncthreads();  // whoever still reads the histogram or s_nb of the piece before
+    const UnitForm form = kLine && !kFloat ? UnitForm{8, 8} : FormOf(kFloat, W, kLine, min(kCols, p.F - g0 * kGroup));
+    for (int i = tid; i < kCols; i += kThreads) {
+      const int r = FeatureOfWord(W, form, i), f = g0 * kGroup + r;
+      const bool is = r >= 0 && f < p.F;
+      s_nb[i]       = is ? p.row_ptr[f + 1] - p.row_ptr[f] : 0;
+      s_base[i]     = is ? FeatureBase<out_t>(p, f, seg) : nullptr;
     }
     zero();
     __syncthreads();
@@ -862,8 +940,10 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
       smem_t* stage      = stage_all + warp * kStageWords;
       const int n_btiles = (mb + kFlushBins - 1) / kFlushBins;
       const int a = lane / kFlushBins, b = lane % kFlushBins;
-      for (int t = warp; t < n_btiles * W; t += kWarps) {
+      const int halves   = W == 2 && (!kFloat || form.extra != 0) ? 2 : 1;
+      for (int t = warp; t < n_btiles * halves; t += kWarps) {
         const int half = t / n_btiles, bin0 = (t - half * n_btiles) * kFlushBins;
+        const int own  = half == 0 ? form.main : form.extra;  // columns that are not copies
         smem_t gv[kFlushBins];
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
@@ -871,7 +951,10 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
 #pragma unroll
           for (int bb = 0; bb < kFlushBins; ++bb) {
             const int bin = bin0 + bb;
-            stage[bb * 32 + ((lane + kWordsPer * bb) & 31)] = bin < mb ? src[bin * kCols] : smem_t(0);
+            smem_t v      = bin < mb ? src[bin * kCols] : smem_t(0);
+            if (!kLine || kFloat)
+              for (int d = own; d < (W == 1 ? 16 : 8); d <<= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+            stage[bb * 32 + ((lane + kWordsPer * bb) & 31)] = v;
           }
           __syncwarp();
           if (pass == 0) {
@@ -888,16 +971,16 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
                 for (int part = 0; part < 2; ++part) {
                   const int from  = part * 16 + (lane >> 1);
                   const smem_t vg = __shfl_sync(0xffffffffu, gv[i], from), vh = __shfl_sync(0xffffffffu, hv, from);
-                  const int f     = feature_of_word(half * 32 + kWordsPer * i + from / kFlushBins);
+                  const int f     = half * 32 + kWordsPer * i + from / kFlushBins;
                   const int bin   = bin0 + from % kFlushBins;
                   const smem_t v  = (lane & 1) ? vh : vg;
-                  if (bin < s_rp[f + 1] - s_rp[f] && v != smem_t(0)) A::add_word(s_base[f] + bin, lane & 1, v);
+                  if (bin < s_nb[f] && v != smem_t(0)) A::add_word(s_base[f] + bin, lane & 1, v);
                 }
                 continue;
               }
-              const int f   = feature_of_word(half * 32 + kWordsPer * i + a);
+              const int f   = half * 32 + kWordsPer * i + a;
               const int bin = bin0 + b;
-              if (bin < s_rp[f + 1] - s_rp[f] && A::nonzero(gv[i], hv)) A::store_global(s_base[f] + bin, gv[i], hv);
+              if (bin < s_nb[f] && A::nonzero(gv[i], hv)) A::store_global(s_base[f] + bin, gv[i], hv);
             }
           }
           __syncwarp();
@@ -917,7 +1000,29 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
         zero();
         __syncthreads();
       }
-      HistRows<A, W, kOrder>(p, sb, se, g0, groups, k, warp, lane, lane_word);
+      auto rows = [&](auto main, auto extra, auto mask) {
+        HistRows<A, W, kOrder, decltype(main)::value, decltype(extra)::value, kLine, decltype(mask)::value>(p, sb, se, g0, k, warp, lane, lane_word);
+      };
+      using std::false_type;
+      using std::integral_constant;
+      using mask           = integral_constant<bool, kFloat>;
+      const int form_steps = form.main + form.extra;
+      const bool no_mask   = !kFloat || p.F - g0 * kGroup >= kCols;  // (of 16 steps)
+      if constexpr (W == 1) {
+        if (form_steps == 16 && no_mask) rows(integral_constant<int, 16>{}, integral_constant<int, 0>{}, false_type{});
+        else if (kFloat && form_steps == 16) rows(integral_constant<int, 16>{}, integral_constant<int, 0>{}, mask{});
+        else if (form_steps == 8) rows(integral_constant<int, 8>{}, integral_constant<int, 0>{}, mask{});
+        else rows(integral_constant<int, 4>{}, integral_constant<int, 0>{}, mask{});
+      } else {
+        if ((kLine && !kFloat) || (form_steps == 16 && no_mask)) rows(integral_constant<int, 8>{}, integral_constant<int, 8>{}, false_type{});
+        else if (kFloat && form_steps == 16) rows(integral_constant<int, 8>{}, integral_constant<int, 8>{}, mask{});
+        else if (!kFloat || form_steps == 12) rows(integral_constant<int, 8>{}, integral_constant<int, 4>{}, mask{});
+        else if (form_steps == 10) rows(integral_constant<int, 8>{}, integral_constant<int, 2>{}, mask{});
+        else if (form_steps == 9) rows(integral_constant<int, 8>{}, integral_constant<int, 1>{}, mask{});
+        else if (form_steps == 8) rows(integral_constant<int, 8>{}, integral_constant<int, 0>{}, mask{});
+        else if (form_steps == 4) rows(integral_constant<int, 4>{}, integral_constant<int, 0>{}, mask{});
+        else rows(integral_constant<int, 2>{}, integral_constant<int, 0>{}, mask{});
+      }
     }
     __syncthreads();
     if (!tree) {
@@ -1270,11 +1375,17 @@ RowOrder OrderOf(const HistParams& p)
   return p.row_index == nullptr ? kRowsInOrder : p.pairs_by_position != 0 ? kPairsByPosition : kPairsByRow;
 }
 
-template <bool kFloat, int W>
+template <bool kFloat, int W, bool kLine>
 void (*SmemKernel(RowOrder order))(HistParams)
 {
-  return order == kPairsByRow ? k_hist_smem<kFloat, W, kPairsByRow>
-                              : order == kPairsByPosition ? k_hist_smem<kFloat, W, kPairsByPosition> : k_hist_smem<kFloat, W, kRowsInOrder>;
+  return order == kPairsByRow         ? k_hist_smem<kFloat, W, kPairsByRow, kLine>
+         : order == kPairsByPosition ? k_hist_smem<kFloat, W, kPairsByPosition, kLine>
+                                     : k_hist_smem<kFloat, W, kRowsInOrder, kLine>;
+}
+template <bool kFloat>
+void (*SmemKernel(int n_groups, RowOrder order))(HistParams)
+{
+  return n_groups > 2 ? SmemKernel<kFloat, 2, true>(order) : n_groups == 2 ? SmemKernel<kFloat, 2, false>(order) : SmemKernel<kFloat, 1, false>(order);
 }
 
 HistLaunch PickHistKernel(int bin_bytes, int mb, bool float_mode, RowOrder order, int F, int K, int64_t n_rows, int n_nodes, bool derive, int sm_count, int ranks, bool aligned)
@@ -1304,8 +1415,7 @@ HistLaunch PickHistKernel(int bin_bytes, int mb, bool float_mode, RowOrder order
     else h.fn = k_hist_tile<uint16_t, 2048, 1024, 1>;
   } else if (h.smem_path) {
     h.smem = HistSmemBytes(h.width);
-    h.fn = h.width == 2 ? (float_mode ? SmemKernel<true, 2>(order) : SmemKernel<false, 2>(order))
-                        : (float_mode ? SmemKernel<true, 1>(order) : SmemKernel<false, 1>(order));
+    h.fn   = float_mode ? SmemKernel<true>(n_groups, order) : SmemKernel<false>(n_groups, order);
   } else if (bin_bytes == 1) {
     h.fn = float_mode ? k_hist_direct<uint8_t, true> : k_hist_direct<uint8_t, false>;
   } else {

@@ -1001,6 +1001,33 @@ def test_full_size_histogram_exact(lb):
     assert torch.equal(stages.histogram(bins, row_ptr, gpair, row_index, seg, bench.HIST_FEATURES, mode=0), hist)
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("F", [1, 4, 5, 8, 9, 16, 17, 31, 32, 33, 36, 37, 40, 41, 48, 49, 63, 64, 65, 66, 72, 73, 80, 81, 96, 97, 100, 101, 105, 112, 113, 129])
+def test_histogram_of_every_unit_form(lb, F, mode):
+    """Units of fewer than 64 features have fewer steps and copies of their words: every number of features at which the
+    form changes, against an independent histogram.  The pairs are small whole numbers, whose float32 sums are exact as well."""
+    from legateboost_b200 import stages
+
+    N, n_nodes = 17_000_000 // F + 77, 300
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(F)
+    bins = torch.zeros((N, (F + 31) // 32 * 32), dtype=torch.uint8, device="cuda")
+    bins[:, :F] = torch.randint(0, 256, (N, F), dtype=torch.uint8, device="cuda", generator=gen)
+    node = (torch.rand(N, device="cuda", generator=gen) ** 3 * n_nodes).to(torch.int32) + (n_nodes - 1)
+    pairs = torch.randint(-5, 6, (N, 1, 2), dtype=torch.int32, device="cuda", generator=gen)
+    row_index, seg = stages.group_rows(node, n_nodes - 1, n_nodes)
+    row_ptr = torch.arange(F + 1, dtype=torch.int32, device="cuda") * 256
+    want = _torch_histogram(bins, pairs, node, n_nodes - 1, n_nodes, F, 256)
+    cast = torch.float32 if mode else torch.int32
+    for by_position in (False, True):
+        given = pairs[row_index.long()].contiguous() if by_position else pairs
+        max_abs = torch.tensor([5, 5], dtype=torch.int32, device="cuda") if mode == 0 else None
+        for merge_tree in (False, True):
+            got = stages.histogram(bins, row_ptr, given.to(cast), row_index, seg, F, mode=mode, max_abs=max_abs,
+                                   pairs_by_position=by_position, merge_tree=merge_tree)
+            assert torch.equal(got, want.to(got.dtype)), (by_position, merge_tree)
+
+
 @pytest.mark.parametrize("merge_tree", [False, True])
 @pytest.mark.parametrize("N,F,K,weights,mode,qmax", [
     (1_500_000, 64, 1, [0.80, 0.0, 0.15, 0.05], 0, 300),    # one node in about 120 pieces (a deep merge tree)
