@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   __syncthreads();
 
   const double l1 = p.l1, reg = fmax(1e-5, p.l2), msg = p.msg;
+  const bool plain = GainsArePlain(qp, l1, reg);
   for (int depth = 0; depth < D; ++depth) {
     const int begin = (1 << depth) - 1, nodes = 1 << depth;
     const bool derive = depth > 0, write_hist = depth < D - 1;
@@ -503,7 +504,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
               if (gb < -1e299) ok_b = 0u;
             }
             if (__any_sync(0xffffffffu, ok_a | ok_b))
-              AddGains(va, ok_a, s_terms[static_cast<int64_t>(n.ja) * K + k], ga, vb, ok_b, s_terms[static_cast<int64_t>(n.jb) * K + k], gb, qp, l1, reg, msg);
+              AddGains(va, ok_a, s_terms[static_cast<int64_t>(n.ja) * K + k], ga, vb, ok_b, s_terms[static_cast<int64_t>(n.jb) * K + k], gb, qp, l1, reg, msg, plain);
             if (k < K - 1) {
               if (in) {
                 gains[b]              = ok_a ? ga : -1e300;
@@ -585,7 +586,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                   if (ga < -1e299) ok_a = 0u;
                   if (gb < -1e299) ok_b = 0u;
                 }
-                if (__any_sync(0xffffffffu, ok_a | ok_b)) AddGains(va, ok_a, ta, ga, vb, ok_b, tb, gb, qp, l1, reg, msg);
+                if (__any_sync(0xffffffffu, ok_a | ok_b)) AddGains(va, ok_a, ta, ga, vb, ok_b, tb, gb, qp, l1, reg, msg, plain);
                 if (k < K - 1) {
                   if (in) {
                     gains[b]              = ok_a ? ga : -1e300;

@@ -114,7 +114,8 @@ struct SliceBest {
 // asked for before anything is made of the nodes' sums and whose two winners are written by a warp each (200k x 50: 8.7
 // -> 8.2 us a level).  There a thread takes a bin and not a warp a feature: a warp alone on its scheduler gets one
 // instruction in about five clocks, and a feature's instructions were 9 us longer whatever the level held.  On wide levels
-// (WideUnits) a warp takes a feature, 32 bins at a time.  Four blocks an SM and not three: 64 features, 8 and 16 units 11.2 and 16.9
+// (WideUnits) a warp takes a feature, 32 bins at a time.  Without the tests that GainsArePlain makes needless: 1M x 100, ten outputs,
+// levels 1 to 7 422 -> 396 us and 294 -> 250 for the last one; 1M x 64, depth 9 192 -> 178; 200k x 50, six levels 67 -> 64.  Four blocks an SM and not three: 64 features, 8 and 16 units 11.2 and 16.9
 // us instead of 12.8 and 18.4, for spills that cost the upper levels 0.3.
 template <typename T, bool kManyOutputs, bool kDerive, bool kWide>
 __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
   const GPairI64 sum_a = left_built ? sum_0 : sum_1, sum_b = left_built ? sum_1 : sum_0;
   const bool eval_a = sum_a.hess > 0, eval_b = kDerive && sum_b.hess > 0;
   const double l1 = p.sp.l1, reg = fmax(1e-5, p.sp.l2), msg = p.sp.min_split_gain;
+  const bool plain    = GainsArePlain(qp, l1, reg);
   const int64_t Bs    = lv.bin_stride;
   const GPairI64* src = lv.built + static_cast<int64_t>(unit) * K * Bs;
   GPairI64* dst_a     = lv.level_hist + static_cast<int64_t>(ja) * K * Bs;
@@ -266,9 +268,9 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
           }
         }
         if (kDerive) {
-          if (__any_sync(0xffffffffu, ok_a | ok_b)) AddGains(va, ok_a, ta, gain_a, vb, ok_b, tb, gain_b, qp, l1, reg, msg);
+          if (__any_sync(0xffffffffu, ok_a | ok_b)) AddGains(va, ok_a, ta, gain_a, vb, ok_b, tb, gain_b, qp, l1, reg, msg, plain);
         } else if (__any_sync(0xffffffffu, ok_a)) {
-          ok_a = AddGain(va, ok_a, ta, qp, l1, reg, msg, gain_a);
+          ok_a = AddGain(va, ok_a, ta, qp, l1, reg, msg, plain, gain_a);
         }
       }
       keep_best(ok_a, gain_a, base + lane, va, best_a, left_a);
@@ -355,9 +357,9 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
           }
         }
         if (kDerive) {
-          if (__any_sync(0xffffffffu, ok_a | ok_b)) AddGains(va, ok_a, ta, gain_a, vb, ok_b, tb, gain_b, qp, l1, reg, msg);
+          if (__any_sync(0xffffffffu, ok_a | ok_b)) AddGains(va, ok_a, ta, gain_a, vb, ok_b, tb, gain_b, qp, l1, reg, msg, plain);
         } else if (__any_sync(0xffffffffu, ok_a)) {
-          ok_a = AddGain(va, ok_a, ta, qp, l1, reg, msg, gain_a);
+          ok_a = AddGain(va, ok_a, ta, qp, l1, reg, msg, plain, gain_a);
         }
       }
       keep_best(ok_a, gain_a, base + tid, va, best_a, left_a);

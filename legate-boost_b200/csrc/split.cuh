@@ -70,17 +70,37 @@ __device__ inline double LeafNumerator(double g, double l1)
   return z * z;
 }
 
+// Without an l1 term, and with scales and a regulariser of moderate size, the numerator is a square and every division of a gain
+// is plain whatever the bin (DivisionIsPlain; sums are whole numbers below 2^52, so a square is zero or at least inv_g^2, a
+// divisor at least reg), but for a divisor whose mantissa is all ones, of which the low word is looked at.  Of the 408
+// instructions a warp took for 32 bins of an output of two nodes the tests of the general form were a fifth.
+__device__ inline bool GainsArePlain(const QuantParams& qp, double l1, double reg)
+{
+  return l1 == 0.0 && qp.inv_g >= 0x1p-250 && qp.inv_g < 0x1p198 && qp.inv_h >= 0.0 && qp.inv_h < 0x1p340 && reg >= 0x1p-400 && reg < 0x1p400;
+}
+__device__ inline bool LowWordOnes(double d) { return __double2loint(d) == -1; }
+
 // The gain of one output at a lane's bin, added to `gain` where `ok`; returns whether both sides have a positive hessian
-// too (sums are below 2^51, so their differences are exact in float64).  All lanes of a warp call it.
+// too (sums are below 2^51, so their differences are exact in float64).  All lanes of a warp call it.  plain: GainsArePlain.
 __device__ inline unsigned AddGain(const GPairI64& left, unsigned ok, const NodeTerms& n, const QuantParams& qp, double l1,
-                                   double reg, double msg, double& gain)
+                                   double reg, double msg, bool plain, double& gain)
 {
   const double lg = WholeToDouble(left.grad), lh = WholeToDouble(left.hess);
   const double rg = n.g - lg, rh = n.h - lh;
   if (lh <= 0.0 || rh <= 0.0) ok = 0u;
-  double a = LeafNumerator(lg * qp.inv_g, l1), b = LeafNumerator(rg * qp.inv_g, l1);
+  double a = lg * qp.inv_g, b = rg * qp.inv_g;
   const double da = lh * qp.inv_h + reg, db = rh * qp.inv_h + reg;
-  if (__all_sync(0xffffffffu, ok == 0u || (DivisionIsPlain(a, da) && DivisionIsPlain(b, db)))) {
+  bool all_plain;
+  if (plain) {
+    a         = a * a;
+    b         = b * b;
+    all_plain = !__any_sync(0xffffffffu, LowWordOnes(da) || LowWordOnes(db));
+  } else {
+    a         = LeafNumerator(a, l1);
+    b         = LeafNumerator(b, l1);
+    all_plain = __all_sync(0xffffffffu, ok == 0u || (DivisionIsPlain(a, da) && DivisionIsPlain(b, db)));
+  }
+  if (all_plain) {
     a = DividePlain(a, da);
     b = DividePlain(b, db);
   } else if (ok != 0u) {
@@ -94,17 +114,30 @@ __device__ inline unsigned AddGain(const GPairI64& left, unsigned ok, const Node
 // The same for a node and its sibling: the four divisions of a lane are under way together (one after the other's vote they
 // take twice as long, and a lone chain is what small levels wait for).
 __device__ inline void AddGains(const GPairI64& left_a, unsigned& ok_a, const NodeTerms& a, double& gain_a, const GPairI64& left_b, unsigned& ok_b,
-                                const NodeTerms& b, double& gain_b, const QuantParams& qp, double l1, double reg, double msg)
+                                const NodeTerms& b, double& gain_b, const QuantParams& qp, double l1, double reg, double msg, bool plain)
 {
   const double alg = WholeToDouble(left_a.grad), alh = WholeToDouble(left_a.hess), arg = a.g - alg, arh = a.h - alh;
   const double blg = WholeToDouble(left_b.grad), blh = WholeToDouble(left_b.hess), brg = b.g - blg, brh = b.h - blh;
   if (alh <= 0.0 || arh <= 0.0) ok_a = 0u;
   if (blh <= 0.0 || brh <= 0.0) ok_b = 0u;
-  double n0 = LeafNumerator(alg * qp.inv_g, l1), n1 = LeafNumerator(arg * qp.inv_g, l1);
-  double n2 = LeafNumerator(blg * qp.inv_g, l1), n3 = LeafNumerator(brg * qp.inv_g, l1);
+  double n0 = alg * qp.inv_g, n1 = arg * qp.inv_g, n2 = blg * qp.inv_g, n3 = brg * qp.inv_g;
   const double d0 = alh * qp.inv_h + reg, d1 = arh * qp.inv_h + reg, d2 = blh * qp.inv_h + reg, d3 = brh * qp.inv_h + reg;
-  if (__all_sync(0xffffffffu, (ok_a == 0u || (DivisionIsPlain(n0, d0) && DivisionIsPlain(n1, d1))) &&
-                                (ok_b == 0u || (DivisionIsPlain(n2, d2) && DivisionIsPlain(n3, d3))))) {
+  bool all_plain;
+  if (plain) {
+    n0        = n0 * n0;
+    n1        = n1 * n1;
+    n2        = n2 * n2;
+    n3        = n3 * n3;
+    all_plain = !__any_sync(0xffffffffu, LowWordOnes(d0) || LowWordOnes(d1) || LowWordOnes(d2) || LowWordOnes(d3));
+  } else {
+    n0        = LeafNumerator(n0, l1);
+    n1        = LeafNumerator(n1, l1);
+    n2        = LeafNumerator(n2, l1);
+    n3        = LeafNumerator(n3, l1);
+    all_plain = __all_sync(0xffffffffu, (ok_a == 0u || (DivisionIsPlain(n0, d0) && DivisionIsPlain(n1, d1))) &&
+                                          (ok_b == 0u || (DivisionIsPlain(n2, d2) && DivisionIsPlain(n3, d3))));
+  }
+  if (all_plain) {
     n0 = DividePlain(n0, d0);
     n1 = DividePlain(n1, d1);
     n2 = DividePlain(n2, d2);
