@@ -1,4 +1,5 @@
-"""Builds liblbk.so (the CUDA kernels and their C ABI) in-tree with nvcc for sm_100a."""
+"""Builds liblbk.so (the CUDA kernels and their C ABI) in-tree with nvcc for sm_100a, and held_arrays.so, a small module
+of the Python package."""
 import os
 import subprocess
 import sys
@@ -8,6 +9,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB = os.path.join(HERE, "liblbk.so")
+MODULE = os.path.join(HERE, "held_arrays.so")
 SOURCES = ["context.cu", "proposals.cu", "quantise.cu", "histogram.cu", "split.cu", "partition.cu",
            "predict.cu", "predict_ranked.cu", "update_tree.cu", "objective.cu", "exchange.cu", "small_tree.cu", "build_tree.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -38,7 +40,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+            raise RuntimeError("the build failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
         return r.stderr
 
     if jobs:
@@ -48,6 +50,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
                     print(out)
     if jobs or not os.path.exists(LIB):
         run([NVCC, "-shared", "-o", LIB] + objs + ["-lcudart", "-ldl"])
+    source = os.path.join(CSRC, "held_arrays.cpp")
+    if force or not _newer(MODULE, [source]):
+        import sysconfig
+
+        from torch.utils import cpp_extension
+
+        # (torch has loaded the libraries it names before it is imported)
+        run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", source, "-o", MODULE]
+            + ["-I" + d for d in cpp_extension.include_paths() + [sysconfig.get_paths()["include"]]]
+            + ["-L" + d for d in cpp_extension.library_paths()] + ["-ltorch_python", "-ltorch_cpu", "-lc10"])
     return LIB
 
 

@@ -251,10 +251,12 @@ struct TiledArgs {
 // Measured against {split, feature} nodes, a block barrier per group, 256 rows per block and every lane reading
 // its own row's values: 100003 x 100, 10 outputs, 50 trees: 224 -> 131 us (now 107: kStaged); and, since then walked on ranks,
 // 10M x 100 float32, 500 trees of depth 8: 23.2 -> 19.5 ms, 1M x 64 float64, 100 trees: 1117 -> 803 us.
-// kStaged (KR > 0): the leaf values of several outputs are in the records too.
+// kStaged (KR > 0): the leaf values of several outputs are in the records too; 2: of an even number, and a lane has the sums of two
+// neighbouring outputs, whose values are one 16-byte load.  Per tree and 32 rows of ten outputs that is 35 passes instead of 55
+// (with 12 values loaded for 10), of about 80 with the walks.
 // kGated: the launch stands in for the walk on ranks and does nothing where that was not declined.  A resident block then takes tile
 // after tile: a launch that finds nothing to do ends in 2.5 us, where a block per tile would come and go.
-template <typename T, int TG, int KR, bool kStaged, bool kGated = false>
+template <typename T, int TG, int KR, int kStaged, bool kGated = false>
 __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledArgs<T> a, const int* __restrict__ gate)
 {
   __shared__ __align__(8) unsigned long long s_bar[4];  // full[2], empty[2]
@@ -364,15 +366,18 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
     if (KR < 0)
       for (int k = 0; k < K; ++k) accs[k * rb + tid] = 0.0;
 
-    // KR > 0: the warp's sums are numbered output innermost, lane l holds l, l + 32, ...
-    constexpr int kSums = KR > 0 ? KR : 1;
+    // KR > 0: the warp's sums (kStaged 2: pairs of them) are numbered output innermost, lane l holds l, l + 32, ...
+    constexpr int kWide  = kStaged == 2 ? 2 : 1;
+    constexpr int kSums  = KR > 0 ? KR : 1, kSlots = kSums / kWide;
+    const int slots      = K / kWide;  // of the warp's, per row
     double acc[kSums];
-    int which[kSums];  // of each: lane (row of the warp) + 32 x output
+    int which[kSlots];  // of each slot: lane (row of the warp) + 32 x output (pair)
 #pragma unroll
-    for (int i = 0; i < kSums; ++i) {
-      acc[i] = 0.0;
-      const int r = KR > 0 ? (lane + 32 * i) / K : 0;
-      which[i]    = KR > 0 && i < K ? r + 32 * (lane + 32 * i - r * K) : 0;  // (what is beyond K is read and dropped)
+    for (int i = 0; i < kSums; ++i) acc[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < kSlots; ++i) {
+      const int r = KR > 0 ? (lane + 32 * i) / slots : 0;
+      which[i]    = KR > 0 && i < slots ? r + 32 * (lane + 32 * i - r * slots) : 0;  // (what is beyond is dropped)
     }
 
     // The walk works on 32-bit shared addresses; at[j] is that of the split of tree j's current node.
@@ -453,18 +458,26 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
       if (nt == TG) walk([](int) { return true; });
       else walk([&](int j) { return j < nt; });
       __syncwarp();
-      if (!kStaged && lane == 0) MbarArrive(empty0 + 8 * b);  // this warp is done with the buffer
-      if constexpr (kStaged) {
+      if (kStaged == 0 && lane == 0) MbarArrive(empty0 + 8 * b);  // this warp is done with the buffer
+      if constexpr (kStaged != 0) {
         const unsigned values = a.rec.split_bytes + a.rec.word_bytes;
         auto add = [&](auto here) {
 #pragma unroll
           for (int j = 0; j < TG; ++j) {
             if (!here(j)) continue;
             const unsigned v = base[j] + values + ((at[j] - base[j]) / kT - (1u << S)) * (8u * K);  // where the row's values are
+            if constexpr (kStaged == 2) {
+              double2 x[kSlots];
 #pragma unroll
-            for (int i = 0; i < kSums; ++i) {
-              const double x = LdsF64(__shfl_sync(0xffffffffu, v, which[i] & 31) + 8u * (which[i] >> 5));
-              acc[i] += x;
+              for (int i = 0; i < kSlots; ++i) x[i] = LdsF64x2(__shfl_sync(0xffffffffu, v, which[i] & 31) + 16u * (which[i] >> 5));
+#pragma unroll
+              for (int i = 0; i < kSlots; ++i) {
+                acc[2 * i] += x[i].x;
+                acc[2 * i + 1] += x[i].y;
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < kSlots; ++i) acc[i] += LdsF64(__shfl_sync(0xffffffffu, v, which[i] & 31) + 8u * (which[i] >> 5));
             }
           }
         };
@@ -508,17 +521,29 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
       if (o.transform != LBK_RAW) {
         asm volatile("bar.sync 1, %0;\n" ::"r"(rb) : "memory");  // the walks are done: the rows take the place of X
 #pragma unroll
-        for (int i = 0; i < kSums; ++i)
-          if (i < K) rows[lane + 32 * i] = o.init ? o.init[which[i] >> 5] + acc[i] : acc[i];
+        for (int i = 0; i < kSlots; ++i)
+          if (i < slots) {
+#pragma unroll
+            for (int e = 0; e < kWide; ++e) {
+              const double sum                  = acc[kWide * i + e];
+              rows[kWide * (lane + 32 * i) + e] = o.init ? o.init[kWide * (which[i] >> 5) + e] + sum : sum;
+            }
+          }
         __syncwarp();
         FinishRow(rows + lane * K, 1, K, rows + lane * K, o.transform);
         __syncwarp();
       }
 #pragma unroll
-      for (int i = 0; i < kSums; ++i) {
+      for (int i = 0; i < kSlots; ++i) {
         const int64_t r = row0 + warp * 32 + (which[i] & 31);
-        if (i < K && r < a.n_rows)
-          o.pred[r * o.ldp + (which[i] >> 5)] = o.transform != LBK_RAW ? rows[lane + 32 * i] : o.init ? o.init[which[i] >> 5] + acc[i] : acc[i];
+        if (i < slots && r < a.n_rows) {
+#pragma unroll
+          for (int e = 0; e < kWide; ++e) {
+            const int k = kWide * (which[i] >> 5) + e;
+            const double sum = acc[kWide * i + e];
+            o.pred[r * o.ldp + k] = o.transform != LBK_RAW ? rows[kWide * (lane + 32 * i) + e] : o.init ? o.init[k] + sum : sum;
+          }
+        }
       }
     }
     __syncthreads();  // (the producer's copies)
@@ -664,13 +689,13 @@ TilePlan PlanTile(lbk_context* ctx, int64_t n_rows, int F, int K, int n_trees, i
 template <typename T, int TG, int KR>
 void LaunchTiledAs(lbk_context* ctx, const int* gate, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
-  auto fn = k_predict_tiled<T, TG, KR, false>;
+  auto fn = k_predict_tiled<T, TG, KR, 0>;
   if constexpr (KR >= 8)
-    if (a.leaves_c == nullptr) fn = k_predict_tiled<T, TG, KR, true>;
+    if (a.leaves_c == nullptr) fn = a.K % 2 == 0 ? k_predict_tiled<T, TG, KR, 2> : k_predict_tiled<T, TG, KR, 1>;
   int64_t grid = (a.n_rows + a.rb - 1) / a.rb;
   if constexpr (KR == 0)
     if (gate != nullptr) {
-      fn   = k_predict_tiled<T, TG, 0, false, true>;
+      fn   = k_predict_tiled<T, TG, 0, 0, true>;
       grid = std::min<int64_t>(grid, static_cast<int64_t>(ctx->sm_count) * plan.resident);
     }
   // (whatever the size: the limit without it is for the static and the dynamic part together)

@@ -82,6 +82,14 @@ __device__ inline double LdsF64(unsigned addr)
   return v;
 }
 
+// (on a 16-byte boundary)
+__device__ inline double2 LdsF64x2(unsigned addr)
+{
+  double2 v;
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "r"(addr));
+  return v;
+}
+
 __device__ inline void MakeSplit(float& s, double split) { s = __double2float_rd(split); }
 __device__ inline void MakeSplit(double& s, double split) { s = split; }
 

@@ -10,6 +10,7 @@ rank passes its own contiguous block of rows and all ranks get the same tree.
 import copy
 import ctypes as C
 import warnings
+from array import array
 from itertools import accumulate, chain
 from operator import attrgetter, is_
 from typing import Any, Callable, List, Sequence, Union
@@ -141,6 +142,14 @@ def build_tree_arrays(X, g, h, *, max_depth, split_samples, seed, l1=0.0, l2=1.0
     return out
 
 
+try:
+    from .held_arrays import holds as _holds
+except ImportError as e:  # importing works anywhere
+    _missing = "held_arrays.so is missing or of another build: build it with `python legate-boost_b200/build.py` (%s)" % e
+
+    def _holds(models, source, addresses):
+        raise RuntimeError(_missing)
+
 _ARRAYS = attrgetter("leaf_value", "feature", "split_value")
 _ARRAY_TYPES = (torch.float64, torch.int32, torch.float64)
 
@@ -152,7 +161,7 @@ class TreeTable:
 
     def __init__(self, arrays):
         # (few calls per tensor: an ensemble's first prediction waits for them)
-        self.source = list(chain.from_iterable(arrays))
+        self.source = tuple(chain.from_iterable(arrays))
         keep = list(self.source)
         for i, t in enumerate(keep):
             want = _ARRAY_TYPES[i % 3]
@@ -172,8 +181,8 @@ class TreeTable:
             raise ValueError("the trees of an ensemble must have arrays of one shape per node")
         # converted copies would not follow later changes of the originals: such a table is not kept
         self.reusable = all(map(is_, keep, self.source))
-        self.addresses = list(map(torch.Tensor.data_ptr, self.source))
-        at = self.addresses if self.reusable else list(map(torch.Tensor.data_ptr, keep))
+        at = list(map(torch.Tensor.data_ptr, keep))
+        self.addresses = array("q", at).tobytes()
         rows = np.array((at[0::3], at[1::3], at[2::3], [m | (e - m) << 32 for m, e in zip(nodes, ends)]), dtype=np.int64).T.copy()
         self.keep, self.total_nodes, self.max_nodes, self.n_trees = keep, ends[-1], max(nodes), len(nodes)
         self.table = torch.from_numpy(rows).to(device)
@@ -183,10 +192,7 @@ class TreeTable:
     def matches(self, models) -> bool:
         """Whether these models still hold the very tensors the table was made from, and these still lie
         where they did (``t.data = ...`` or ``t.set_(...)`` moves a tensor)."""
-        if not self.reusable or len(models) != self.n_trees:
-            return False
-        arrays = list(chain.from_iterable(map(_ARRAYS, models)))
-        return all(map(is_, arrays, self.source)) and list(map(torch.Tensor.data_ptr, arrays)) == self.addresses
+        return self.reusable and _holds(models if type(models) is list else list(models), self.source, self.addresses)
 
     def _hold(self, X, init, stream):
         """The call is queued, and what it reads may have been allocated on another stream: given up by its owner, it

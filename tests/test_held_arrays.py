@@ -1,0 +1,68 @@
+"""The check that a kept table of addresses still belongs to an ensemble's tensors (CPU)."""
+from array import array
+
+import pytest
+import torch
+
+import legateboost_b200 as lb  # noqa: F401
+from legateboost_b200.tree import _holds
+
+
+class Model:
+    def __init__(self):
+        self.leaf_value, self.feature, self.split_value = torch.zeros(7, 1), torch.zeros(7, dtype=torch.int32), torch.zeros(7)
+
+
+def _table(models):
+    source = tuple(t for m in models for t in (m.leaf_value, m.feature, m.split_value))
+    return source, array("q", [t.data_ptr() for t in source]).tobytes()
+
+
+def test_holds_the_same_tensors_where_they_were():
+    models = [Model() for _ in range(5)]
+    source, at = _table(models)
+    assert _holds(models, source, at) and _holds(list(models), source, at) and _holds([], (), b"")
+    models[3].leaf_value.fill_(2.0)  # contents do not matter
+    assert _holds(models, source, at)
+    assert not _holds(models[:4], source, at) and not _holds(models + [Model()], source, at)
+    assert not _holds([models[1], models[0]] + models[2:], source, at)
+
+
+@pytest.mark.parametrize("name", ["leaf_value", "feature", "split_value"])
+def test_another_or_a_moved_tensor_is_seen(name):
+    models = [Model() for _ in range(3)]
+    source, at = _table(models)
+    was = getattr(models[2], name)
+    setattr(models[2], name, was.clone())
+    assert not _holds(models, source, at)
+    setattr(models[2], name, None)
+    assert not _holds(models, source, at)
+    setattr(models[2], name, was)
+    assert _holds(models, source, at)
+    was.data = was.clone()  # the same object elsewhere
+    assert not _holds(models, source, at)
+
+
+def test_errors_are_python_errors():
+    models = [Model()]
+    source, at = _table(models)
+    with pytest.raises(TypeError):
+        _holds(models, list(source), at)
+    with pytest.raises(ValueError):
+        _holds(models, source, at[:-1])
+    del models[0].feature
+    with pytest.raises(AttributeError):
+        _holds(models, source, at)
+
+    class Odd(Model):  # an attribute that changes the list while it is walked
+        @property
+        def feature(self):
+            models.clear()
+            return None
+
+        @feature.setter
+        def feature(self, value):
+            pass
+
+    models[:] = [Odd(), Model()]
+    assert not _holds(models, source + source, at + at)
