@@ -252,8 +252,10 @@ struct TiledArgs {
 // its own row's values: 100003 x 100, 10 outputs, 50 trees: 224 -> 131 us (now 107: kStaged); and, since then walked on ranks,
 // 10M x 100 float32, 500 trees of depth 8: 23.2 -> 19.5 ms, 1M x 64 float64, 100 trees: 1117 -> 803 us.
 // kStaged (KR > 0): the leaf values of several outputs are in the records too; 2: of an even number, and a lane has the sums of two
-// neighbouring outputs, whose values are one 16-byte load.  Per tree and 32 rows of ten outputs that is 35 passes instead of 55
-// (with 12 values loaded for 10), of about 80 with the walks.
+// neighbouring outputs, whose values are one 16-byte load.  Per tree and 32 rows of ten outputs that is 30 passes instead of 55
+// (as 8-byte loads, 12 values for 10), of about 80 with the walks: 100 features, ten outputs, 50 trees of depth 8, 1M rows 1141 -> 946 us,
+// 100003 rows 97 -> 92 (two waves that wait for the trees' 300 MB); 300k x 20, 100 trees of depth 6 303 -> 256; sixteen
+// outputs, 200003 x 30 170 -> 160.  Three outputs with three sums instead of four: 2M x 50, 100 trees of depth 7 1229 -> 1153.
 // kGated: the launch stands in for the walk on ranks and does nothing where that was not declined.  A resident block then takes tile
 // after tile: a launch that finds nothing to do ends in 2.5 us, where a block per tile would come and go.
 template <typename T, int TG, int KR, int kStaged, bool kGated = false>
@@ -709,8 +711,10 @@ void LaunchTiled(lbk_context* ctx, const int* gate, const TiledArgs<T>& a, const
 {
   if (a.K == 1) LaunchTiledAs<T, TG, 0>(ctx, gate, a, plan, stream);
   else if (a.K <= 2) LaunchTiledAs<T, TG, 2>(ctx, gate, a, plan, stream);
-  else if (a.K <= 4) LaunchTiledAs<T, TG, 4>(ctx, gate, a, plan, stream);
+  else if (a.K == 3) LaunchTiledAs<T, TG, 3>(ctx, gate, a, plan, stream);
+  else if (a.K == 4) LaunchTiledAs<T, TG, 4>(ctx, gate, a, plan, stream);
   else if (a.K <= 8) LaunchTiledAs<T, TG, 8>(ctx, gate, a, plan, stream);
+  else if (a.K <= 10) LaunchTiledAs<T, TG, 10>(ctx, gate, a, plan, stream);
   else if (a.K <= 12) LaunchTiledAs<T, TG, 12>(ctx, gate, a, plan, stream);
   else if (a.K <= kRegisterSums) LaunchTiledAs<T, TG, kRegisterSums>(ctx, gate, a, plan, stream);
   else LaunchTiledAs<T, TG, -1>(ctx, gate, a, plan, stream);

@@ -634,6 +634,27 @@ def test_predict_of_several_outputs_by_tables(lb, oracle, N, F, K, T, D, dt, wit
     assert np.array_equal(table.predict(X, K, wait=True)[:300].cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("K", [6, 7, 8, 9, 10, 11, 12, 14, 15, 16])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_predict_of_even_and_odd_outputs(lb, oracle, K, dt):
+    """Leaf values that come with the trees, of an even number of outputs two at a time: the bits of the oracle's sums."""
+    from legateboost_b200 import library as L
+    from legateboost_b200.tree import TreeTable
+
+    N, F, T, D = 9_003, 11, 17, 5
+    rs = np.random.RandomState(K)
+    X = rs.random((N, F)).astype(dt)
+    trees = [(dev(rs.normal(size=(t[1].shape[0], K))),) + t[1:] for t in _random_trees(rs, T, D, np.arange(F))]
+    table, init = TreeTable(trees), dev(rs.normal(size=K))
+    assert _predict_plan(lb, table, dev(X), K, L.RAW)["leaves_with_trees"]
+    want = oracle.predict(X, [tuple(a.cpu().numpy() for a in t) for t in trees])
+    assert np.array_equal(table.predict(dev(X), K, wait=True).cpu().numpy(), want)
+    softmax = table.predict(dev(X), K, init=init, transform=L.SOFTMAX, wait=True).cpu().numpy()
+    raw = want + init.cpu().numpy()
+    e = np.exp(raw - raw.max(axis=1, keepdims=True))
+    assert np.allclose(softmax, e / e.sum(axis=1, keepdims=True), rtol=1e-13, atol=0)  # (a few roundings of exp and a sum)
+
+
 def test_predict_without_room_for_ranks(lb):
     """A caller's allocator that has no 20 MB gets the predictions by the path that needs less."""
     from legateboost_b200.tree import TreeTable
