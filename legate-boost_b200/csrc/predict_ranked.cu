@@ -575,6 +575,8 @@ struct RankRowsArgs {
   int tail_blocks;  // blocks for the last group of features
 };
 
+constexpr int kMaxSteps = 4, kPad = 1 << (kMaxSteps - 2);
+
 // c = *at where n >= h, else as it was: a load without a branch.
 __device__ inline void LoadSharedIf(float& c, int n, int h, unsigned at)
 {
@@ -585,8 +587,9 @@ __device__ inline void LoadSharedIf(double& c, int n, int h, unsigned at)
   asm volatile("{\n.reg .pred p;\nsetp.ge.s32 p, %1, %2;\n@p ld.shared.f64 %0, [%3];\n}\n" : "+d"(c) : "r"(n), "r"(h), "r"(at));
 }
 
-// The rows of a block of k_rank_rows.  lut, cuts: the lane's feature's table, in shared memory (kInside) or in global.
-template <typename T, bool kInside>
+// The rows of a block of k_rank_rows.  lut, cuts: the lane's feature's table, in shared memory (kInside) or in global.  kSteps: no bucket
+// has 2^kSteps values or more, and kPad infinities follow the table; 0: any.
+template <typename T, bool kInside, int kSteps>
 __device__ __forceinline__ void RankRows(const RankRowsArgs<T>& a, const RankTable& t, unsigned* turn, const unsigned* lut, const T* cuts, int f0,
                                          int width, int fl, int sub, int subs, int part, int parts)
 {
@@ -609,6 +612,7 @@ __device__ __forceinline__ void RankRows(const RankRowsArgs<T>& a, const RankTab
     i.t0   = (w - i.tile * per_tile) * kRankTileRows;
     return i;
   };
+  const unsigned below_first = cuts_at - kSize;
   // the rows of a step of an item; those behind the last one are the last one again
   auto load = [&](const Item& i, int st, T (&x)[kRankAhead]) {
     const int half = st >= steps ? 1 : 0;
@@ -640,23 +644,20 @@ __device__ __forceinline__ void RankRows(const RankRowsArgs<T>& a, const RankTab
       // at: where the value is that x is compared with next, an address or an index
       unsigned at[kRankAhead];
       int n[kRankAhead];
-      int most = 0;
 #pragma unroll
       for (int u = 0; u < kRankAhead; ++u) {
         const int b      = RankBucket(static_cast<float>(x[u]), t.lo, t.scale, t.nb);
         const unsigned e = kInside ? LdsU32(lut_at + 4u * b) : __ldg(lut + b);
-        at[u]            = kInside ? cuts_at + (e & 0xffffu) * kSize : e & 0xffffu;
+        at[u]            = kInside ? (e & 0xffffu) * kSize : e & 0xffffu;
         n[u]             = static_cast<int>(e >> 16);
-        most             = max(most, n[u]);
       }
-      most = __reduce_max_sync(0xffffffffu, most);
       // how many of the bucket's values are below x, in steps of falling powers of two: all rows' values are asked for before
       // the first is compared
       auto descend = [&](int h) {
         T cut[kRankAhead];
 #pragma unroll
         for (int u = 0; u < kRankAhead; ++u) {
-          cut[u] = static_cast<T>(INFINITY);
+          cut[u] = kSteps > 0 ? x[u] : static_cast<T>(INFINITY);
           if (kInside) LoadSharedIf(cut[u], n[u], h, at[u] + (h - 1) * kSize);
           else if (n[u] >= h) cut[u] = __ldg(cuts + at[u] + (h - 1));
         }
@@ -664,20 +665,32 @@ __device__ __forceinline__ void RankRows(const RankRowsArgs<T>& a, const RankTab
         for (int u = 0; u < kRankAhead; ++u)
           if (cut[u] < x[u]) {
             at[u] += kInside ? h * kSize : h;
-            n[u] -= h;
+            if (kSteps == 0) n[u] -= h;
           }
       };
-      for (int h = most >= 8 ? 1 << (31 - __clz(most)) : 0; h >= 8; h >>= 1) descend(h);
-      if (most >= 4) descend(4);
-      if (most >= 2) descend(2);
-      if (most >= 1) descend(1);
+      if (kSteps > 0) {
+        // (what a step looks at beyond the bucket is not below x: a value of another one or an infinity)
+        if (kSteps > 3) descend(8);
+        descend(4);
+        descend(2);
+        descend(1);
+      } else {
+        int most = 0;
+#pragma unroll
+        for (int u = 0; u < kRankAhead; ++u) most = max(most, n[u]);
+        most = __reduce_max_sync(0xffffffffu, most);
+        for (int h = most >= 8 ? 1 << (31 - __clz(most)) : 0; h >= 8; h >>= 1) descend(h);
+        if (most >= 4) descend(4);
+        if (most >= 2) descend(2);
+        if (most >= 1) descend(1);
+      }
       if (fl < width) {
         const int half = st >= steps ? 1 : 0, r0 = (st - half * steps) * step_rows + sub;
         uint16_t* mine = reinterpret_cast<uint16_t*>(turn) + 2 * (fl * kPitch + r0) + half;
 #pragma unroll
         for (int u = 0; u < kRankAhead; ++u)
           if (step_rows <= kRankTileRows || r0 + u * subs < kRankTileRows)
-            mine[2 * u * subs] = static_cast<uint16_t>(x[u] == x[u] ? 1 + (kInside ? (at[u] - cuts_at) / kSize : at[u]) : t.m + 2);
+            mine[2 * u * subs] = static_cast<uint16_t>(x[u] == x[u] ? (kInside ? (at[u] - below_first) / kSize : 1 + at[u]) : t.m + 2);
       }
     }
     __syncwarp();
@@ -691,14 +704,23 @@ __device__ __forceinline__ void RankRows(const RankRowsArgs<T>& a, const RankTab
 
 // The tables of features [w0, w1) of a group to shared memory, by a block; four entries of a thread at a time: places, then loads, then
 // stores.  (A warp per feature, 32 entries at a time: 50 us for one feature of 20 thousand.  Inlined, or with the two arrays as
-// arguments, the float32 loop over the rows comes out 3 % slower: 10M x 100, 500 trees 300 and 310 us a piece.)
+// arguments, the float32 loop over the rows comes out 3 % slower: 10M x 100, 500 trees 300 and 310 us a piece.)  A word of a table:
+// the address of the bucket's first value in units of values, and in the high half how many there are.  `pad` infinities
+// follow the values of a feature.  Returns the values of the fullest bucket of the thread's.
 template <typename T>
-__device__ __noinline__ void FillTables(const RankRowsArgs<T>& a, const int* s_begin, const int* s_from, int w0, int w1, unsigned* s_lut, T* s_cuts)
+__device__ __noinline__ unsigned FillTables(const RankRowsArgs<T>& a, const int* s_begin, const int* s_from, int w0, int w1, int pad, unsigned* s_lut, T* s_cuts)
 {
   constexpr int kFill = 4;
   const int base = s_begin[w0], entries = s_begin[w1] - base;
+  const unsigned cuts_at = static_cast<unsigned>(__cvta_generic_to_shared(s_cuts)) / sizeof(T);
+  unsigned fullest = 0;
+  for (int i = threadIdx.x; i < (w1 - w0) * pad; i += kRankThreads) {
+    const int e = i / pad;
+    s_cuts[s_begin[w0 + e + 1] - base + e * pad + i - e * pad] = static_cast<T>(INFINITY);
+  }
   for (int i0 = threadIdx.x; i0 < entries; i0 += kFill * kRankThreads) {
     int from[kFill];  // where the entry lies, -1: of a feature without values, whose only bucket is empty
+    int first[kFill], to[kFill];  // in s_cuts: the feature's first value, and the entry's
     unsigned word[kFill];
     T cut[kFill];
 #pragma unroll
@@ -708,7 +730,9 @@ __device__ __noinline__ void FillTables(const RankRowsArgs<T>& a, const int* s_b
 #pragma unroll
       for (int h = 16; h > 0; h >>= 1)
         if (e + h < w1 && s_begin[e + h] <= i) e += h;
-      from[u] = s_from[e] >= 0 ? s_from[e] + i - s_begin[e] : -1;
+      from[u]  = s_from[e] >= 0 ? s_from[e] + i - s_begin[e] : -1;
+      first[u] = s_begin[e] - base + (e - w0) * pad;
+      to[u]    = first[u] + i - s_begin[e];
     }
 #pragma unroll
     for (int u = 0; u < kFill; ++u) {
@@ -719,11 +743,14 @@ __device__ __noinline__ void FillTables(const RankRowsArgs<T>& a, const int* s_b
     for (int u = 0; u < kFill; ++u) {
       const int i = i0 + u * kRankThreads;
       if (i < entries) {
-        s_lut[i]  = word[u];
-        s_cuts[i] = cut[u];
+        const unsigned n = word[u] >> 16;
+        s_lut[i]         = word[u] + cuts_at + first[u];
+        s_cuts[to[u]]    = cut[u];
+        fullest          = max(fullest, n);
       }
     }
   }
+  return fullest;
 }
 
 // X -> ranks.  A block serves one group of 32 features and keeps their tables in shared memory; lane = feature, a warp takes
@@ -733,7 +760,9 @@ __device__ __noinline__ void FillTables(const RankRowsArgs<T>& a, const int* s_b
 // Bound by the load/store pipe and the latency of its lookups: per 32 values a load of X, the bucket and about three steps of
 // a search, each with the conflicts of 32 lanes on random banks, and the turn: twelve to sixteen passes and about 65
 // instructions; 1.2M x 96 float32 238 us, x 64 float64 224.  (The values of a step asked for under branches, one row after
-// the other: 700 us.)  Where the tables of a
+// the other: 700 us.)  Where no bucket of a turn has 16 values (8) the search takes four (three) steps without counting
+// what is left of the bucket; only tables whose values crowd together take as many as their fullest bucket wants.  300003 x 130
+// float32, 300 trees of depth 7 384 -> 366 us, 1M x 64 float64, 100 trees 533 -> 524.  Where the tables of a
 // group do not fit (20 thousand values of float32) its features are taken in several turns over the rows; a feature
 // that has no room alone is searched where its table lies.
 template <typename T>
@@ -779,13 +808,16 @@ __global__ void __launch_bounds__(kRankThreads, 1) k_rank_rows(const RankRowsArg
     if (TableBytes<T>(entries) <= room) {
       unsigned* s_lut = s_table;
       T* s_cuts       = reinterpret_cast<T*>(s_lut + (entries + 1) / 2 * 2);
-      FillTables(a, s_begin, s_from, w0, w1, s_lut, s_cuts);
-      __syncthreads();
-      const int at = s_begin[f] - s_begin[w0];
-      RankRows<T, true>(a, t, turn, s_lut + at, s_cuts + at, f0 + w0, n, fl, sub, subs, part, parts);
+      const int pad   = TableBytes<T>(entries) + n * kPad * static_cast<unsigned>(sizeof(T)) <= room ? kPad : 0;
+      const unsigned fullest = FillTables(a, s_begin, s_from, w0, w1, pad, s_lut, s_cuts);
+      const int beyond = __syncthreads_or(fullest >= 16) != 0 || pad == 0 ? 2 : __syncthreads_or(fullest >= 8) != 0 ? 1 : 0;
+      const int at = s_begin[f] - s_begin[w0], cut = at + (f - w0) * pad;
+      if (beyond == 0) RankRows<T, true, 3>(a, t, turn, s_lut + at, s_cuts + cut, f0 + w0, n, fl, sub, subs, part, parts);
+      else if (beyond == 1) RankRows<T, true, 4>(a, t, turn, s_lut + at, s_cuts + cut, f0 + w0, n, fl, sub, subs, part, parts);
+      else RankRows<T, true, 0>(a, t, turn, s_lut + at, s_cuts + cut, f0 + w0, n, fl, sub, subs, part, parts);
     } else {
       // (a feature without values has room: no index would say here that its only bucket is empty)
-      RankRows<T, false>(a, t, turn, a.lut + t.off, a.cuts + t.off, f0 + w0, n, fl, sub, subs, part, parts);
+      RankRows<T, false, 0>(a, t, turn, a.lut + t.off, a.cuts + t.off, f0 + w0, n, fl, sub, subs, part, parts);
     }
   }
 }

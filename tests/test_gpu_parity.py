@@ -610,6 +610,41 @@ def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what, group, pieces,
     assert torch.equal(table.predict(wide[:, 1: F + 1], 1, init=init, transform=transform, wait=True), got)
 
 
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("what,used", [("even", None), ("any", None), ("seven", None), ("fifteen", None), ("sixteen", None), ("sixty", None), ("one", [3])])
+def test_ranks_from_buckets_of_any_size(lb, what, used, dt):
+    """Splits evenly apart, by chance, and crowded in buckets of up to so many (one: nearly all of a feature's): the steps of the
+    search are another number each time.  A few rows at a time, where trees are walked where they lie, give the same bits."""
+    from legateboost_b200 import library as L
+    from legateboost_b200.tree import TreeTable
+
+    N, F, T, D = (1_000_003, 60, 300, 8) if dt is np.float32 else (800_011, 20, 70, 8)
+    rs = np.random.RandomState(len(what))
+    trees, crowd = [], dict(seven=7, fifteen=15, sixteen=17, sixty=60).get(what)
+    for v, f, s in _random_trees(rs, T, D, np.arange(F) if used is None else used):
+        s = s.cpu().numpy()
+        if what == "even":
+            s = np.round(s * 700) / 700
+        elif crowd is not None:  # clusters a good deal further apart than a bucket is wide, in a small part of one each
+            s = np.floor(s * 40) / 40 + np.floor(rs.random(s.shape) * crowd) * 2e-6
+        elif what == "one":
+            s = np.where(rs.random(s.shape) < 0.002, np.sign(s - 0.5) * 1e4, 0.5 + s * 0.02)
+        trees.append((v, f, dev(s.astype(dt).astype(np.float64))))
+    table = TreeTable(trees)
+    X = np.random.default_rng(len(what)).random((N, F), dtype=dt)
+    splits = np.concatenate([t[2].cpu().numpy() for t in trees]).astype(dt)
+    X[::2] = splits[rs.randint(len(splits), size=X[::2].shape)]  # ties
+    X[rs.randint(N, size=500), rs.randint(F, size=500)] = np.nan
+    X[rs.randint(N, size=500), rs.randint(F, size=500)] = np.inf
+    dX = dev(X)
+    plan = _predict_plan(lb, table, dX, 1, L.RAW)
+    assert plan["threads"] > 0
+    got, _ = _predict_and_word(lb, table, dX, plan)
+    for rows in (np.arange(8000), np.arange(N - 8000, N), np.sort(rs.choice(N, 8000, replace=False))):
+        rows = dev(rows)
+        assert torch.equal(got[rows], table.predict(dX[rows].contiguous(), 1, wait=True))
+
+
 @pytest.mark.parametrize("N,F,K,T,D,dt,with_trees", [
     (20_001, 10, 6, 16, 5, np.float32, True), (100_003, 100, 10, 50, 8, np.float32, True), (9_000, 65, 16, 17, 6, np.float64, True),
     (12_345, 300, 10, 23, 6, np.float32, True), (20_000, 7, 12, 40, 3, np.float64, True),
