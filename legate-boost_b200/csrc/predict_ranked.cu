@@ -229,22 +229,26 @@ __device__ inline RankTable IndexOf(T first, T last, int off, int m)
   }
   return t;
 }
-// The index of a table whose values lie in `out`, by a block.  start [m]: first value of every bucket (the place of the unsorted values).
-template <typename T>
-__device__ inline void MakeIndex(const RankTable& t, const T* out, int* start, unsigned* lut)
+// (memory of the block, or what other blocks may have written)
+__device__ inline float ValueAt(const float* p) { return __isShared(p) ? *p : __ldcg(p); }
+__device__ inline double ValueAt(const double* p) { return __isShared(p) ? *p : __ldcg(p); }
+
+// The index of a table whose values lie in `out`, by a block.  start [m]: scratch, first value of every bucket.
+template <typename T, typename Start>
+__device__ inline void MakeIndex(const RankTable& t, const T* out, Start* start, unsigned* lut)
 {
 #pragma unroll 4
   for (int i = threadIdx.x; i < t.m; i += kSortThreads) {
-    const int b = RankBucket(static_cast<float>(__ldcg(out + i)), t.lo, t.scale, t.nb);
-    const int a = i > 0 ? RankBucket(static_cast<float>(__ldcg(out + i - 1)), t.lo, t.scale, t.nb) : -1;
-    for (int q = a + 1; q <= b; ++q) start[q] = i;
+    const int b = RankBucket(static_cast<float>(ValueAt(out + i)), t.lo, t.scale, t.nb);
+    const int a = i > 0 ? RankBucket(static_cast<float>(ValueAt(out + i - 1)), t.lo, t.scale, t.nb) : -1;
+    for (int q = a + 1; q <= b; ++q) start[q] = static_cast<Start>(i);
     if (i == t.m - 1)
-      for (int q = b + 1; q < t.nb; ++q) start[q] = t.m;
+      for (int q = b + 1; q < t.nb; ++q) start[q] = static_cast<Start>(t.m);
   }
   __syncthreads();
 #pragma unroll 4
   for (int b = threadIdx.x; b < t.m; b += kSortThreads) {
-    const int first = __ldcg(start + b), next = b + 1 < t.m ? __ldcg(start + b + 1) : t.m;
+    const int first = static_cast<int>(start[b]), next = b + 1 < t.m ? static_cast<int>(start[b + 1]) : t.m;
     lut[b]          = static_cast<unsigned>(first) | (static_cast<unsigned>(next - first) << 16);
   }
 }
@@ -341,12 +345,114 @@ __device__ inline void SortShared(T* s, int P)
   __syncthreads();
 }
 
+// The values of a chunk in order, by as many buckets of equal width: counted, scattered, and those of a bucket put in order by a thread.
+// False, with the values in another order, where more than kSortBucket share a bucket and are not all equal (columns of few
+// values have splits that are).  start: scratch.  k_rank_sort of 64 features of 170 to 2000 float64 values: 29 us by the
+// network, 15; of 100 features, float32, 27 and 15.
+constexpr int kSortBucket = 24;
+template <typename T>
+__device__ inline bool SortByBuckets(T* s, unsigned* start /* [kSortChunk / 2]: two of 16 bits */, int* s_wsum, float2* s_range /* [32] */, int len)
+{
+  constexpr int kPer = kSortChunk / kSortThreads;
+  static_assert(kPer == 4, "two words of counts a thread");
+  constexpr float kMax = 3.402823466e38f;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  T v[kPer];
+  float lo = kMax, hi = -kMax;
+  reinterpret_cast<uint2*>(start)[tid] = make_uint2(0u, 0u);
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int i = tid + u * kSortThreads;
+    v[u]        = i < len ? s[i] : T(0);
+    if (i < len) {
+      const float x = fminf(fmaxf(static_cast<float>(v[u]), -kMax), kMax);
+      lo            = fminf(lo, x);
+      hi            = fmaxf(hi, x);
+    }
+  }
+  auto range_of_warp = [&]() {
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+  };
+  range_of_warp();
+  if (lane == 0) s_range[warp] = make_float2(lo, hi);
+  __syncthreads();
+  lo = s_range[lane].x;
+  hi = s_range[lane].y;
+  range_of_warp();
+  const float scale = hi > lo ? static_cast<float>(len) / (hi - lo) : 0.f;
+  int bucket[kPer], before[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    bucket[u] = RankBucket(static_cast<float>(v[u]), lo, scale, len);
+    before[u] = 0;
+    if (tid + u * kSortThreads < len) {
+      const int shift = 16 * (bucket[u] & 1);
+      before[u]       = static_cast<int>(atomicAdd(start + (bucket[u] >> 1), 1u << shift) >> shift & 0xffffu);
+    }
+  }
+  __syncthreads();
+  // counts become first places
+  const uint2 c  = reinterpret_cast<uint2*>(start)[tid];
+  const int n[4] = {static_cast<int>(c.x & 0xffffu), static_cast<int>(c.x >> 16), static_cast<int>(c.y & 0xffffu), static_cast<int>(c.y >> 16)};
+  int incl       = n[0] + n[1] + n[2] + n[3];
+  const int own  = incl;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  if (lane == 31) s_wsum[warp] = incl;
+  __syncthreads();
+  int sums = s_wsum[lane];
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, sums, o);
+    if (lane >= o) sums += x;
+  }
+  const int below_warp = __shfl_sync(0xffffffffu, sums, max(warp - 1, 0));
+  int at[5];
+  at[0] = incl - own + (warp > 0 ? below_warp : 0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) at[k + 1] = at[k] + n[k];
+  reinterpret_cast<uint2*>(start)[tid] = make_uint2(at[0] | at[1] << 16, at[2] | at[3] << 16);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kPer; ++u)
+    if (tid + u * kSortThreads < len) {
+      bucket[u] = static_cast<int>(start[bucket[u] >> 1] >> (16 * (bucket[u] & 1)) & 0xffffu);  // (its first place)
+      s[bucket[u] + before[u]] = v[u];
+    }
+  __syncthreads();
+  bool crowded = false;
+#pragma unroll
+  for (int u = 0; u < kPer; ++u)
+    if (tid + u * kSortThreads < len && before[u] >= kSortBucket) crowded = crowded || s[bucket[u]] != v[u];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (n[k] > kSortBucket)
+      for (int i = 1; i < kSortBucket; ++i) crowded = crowded || s[at[k] + i] != s[at[k]];
+  if (__syncthreads_or(crowded)) return false;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    for (int i = at[k] + 1; n[k] <= kSortBucket && i < at[k + 1]; ++i) {
+      const T x = s[i];
+      int j     = i;
+      for (; j > at[k] && x < s[j - 1]; --j) s[j] = s[j - 1];
+      s[j] = x;
+    }
+  __syncthreads();
+  return true;
+}
+
 // A block per chunk: its values sorted, equal ones once.  A feature of one chunk has its table then.
 template <typename T>
 __global__ void __launch_bounds__(kSortThreads) k_rank_sort(const RankTables<T> a)
 {
   __shared__ T s[kSortChunk];
+  __shared__ __align__(8) unsigned s_start[kSortChunk / 2];
   __shared__ int s_wsum[kSortThreads / 32];
+  __shared__ float2 s_range[kSortThreads / 32];
   if (*a.declined != 0 || static_cast<int>(blockIdx.x) >= *a.n_items) return;
   const int2 item = a.items[blockIdx.x];
   const int f = item.x, tid = threadIdx.x;
@@ -355,19 +461,22 @@ __global__ void __launch_bounds__(kSortThreads) k_rank_sort(const RankTables<T> 
   int P   = 64;
   while (P < len) P <<= 1;
   for (int i = tid; i < P; i += kSortThreads) s[i] = i < len ? list[i] : static_cast<T>(INFINITY);
-  SortShared(s, P);
-  const bool alone = ChunksOf(n) == 1;
-  T* dst           = alone ? a.cuts + begin : list;
-  int m            = 0;
+  __syncthreads();
+  if (!SortByBuckets(s, s_start, s_wsum, s_range, len)) SortShared(s, P);
+  // (kept values move to the front, never beyond what has been read)
+  int m = 0;
   for (int i0 = 0; i0 < len; i0 += kSortThreads) {
     const int i     = i0 + tid;
     const bool keep = i < len && (i == 0 || s[i] != s[i - 1]);
-    m               = KeepInOrder(keep, keep ? s[i] : T(0), dst, m, s_wsum);
+    m               = KeepInOrder(keep, keep ? s[i] : T(0), s, m, s_wsum);
   }
+  const bool alone = ChunksOf(n) == 1;
+  T* dst           = alone ? a.cuts + begin : list;
+  for (int i = tid; i < m; i += kSortThreads) dst[i] = s[i];
   if (tid == 0) a.len[blockIdx.x] = m;
   if (!alone) return;
-  const RankTable t = IndexOf(m > 0 ? s[0] : T(0), m > 0 ? s[len - 1] : T(0), begin, m);
-  MakeIndex(t, dst, reinterpret_cast<int*>(list), a.lut + begin);
+  const RankTable t = IndexOf(m > 0 ? s[0] : T(0), m > 0 ? s[m - 1] : T(0), begin, m);
+  MakeIndex(t, s, reinterpret_cast<uint16_t*>(s_start), a.lut + begin);
   if (tid == 0) a.tables[f] = t;
 }
 
