@@ -133,31 +133,35 @@ __global__ void k_pack_complete(const int* __restrict__ gate, const TreePtrs* __
   unsigned* words    = reinterpret_cast<unsigned*>(out + rec.split_bytes);
   double* leaves     = rec.leaf_bytes > 0 ? reinterpret_cast<double*>(out + rec.split_bytes + rec.word_bytes)
                                           : leaves_c + (static_cast<int64_t>(blockIdx.x) << S) * K;
-  auto splits_here = [&](int a) {
-    if (a >= M || 2 * a + 2 >= M) return false;
-    const int f = t.feature[a];
-    return f >= 0 && f < F;
-  };
-  // first leaf on the path root -> i, or -1
-  auto cover_of = [&](int i) {
-    const int L = 31 - __clz(i + 1);
+  // the features of the nodes above the bottom level, kNoSplit: none; then the paths are followed in shared memory (through the
+  // arrays, a load behind the other: 50 trees of depth 8, ten outputs 9.9 us, now 9.4, of which most are the values; a thread per value 12.2)
+  extern __shared__ uint16_t s_feature[];
+  constexpr int kNoSplit = 0xffff;
+  for (int a = threadIdx.x; a < (1 << S) - 1; a += blockDim.x) {
+    const int f  = 2 * a + 2 < M ? t.feature[a] : -1;
+    s_feature[a] = static_cast<uint16_t>(f >= 0 && f < F ? f : kNoSplit);
+  }
+  __syncthreads();
+  auto splits_here = [&](int a) { return s_feature[a] != kNoSplit; };
+  // first leaf on the path root -> i (of level L), or -1
+  auto cover_of = [&](int i, int L) {
     for (int l = 0; l <= L; ++l) {
       const int a = ((i + 1) >> (L - l)) - 1;
-      if (!splits_here(a)) return a;
+      if (l == S || !splits_here(a)) return a;
     }
     return -1;
   };
   const int total = (2 << S) - 1;  // nodes of the complete tree
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
-    const int L = 31 - __clz(i + 1), cover = cover_of(i);
+    const int L = 31 - __clz(i + 1), cover = cover_of(i, L);
     if (L < S) {
       // (a pass-through node sends a NaN to the right: the same leaf value is there)
       MakeSplit(splits[i + 1], cover >= 0 ? static_cast<double>(INFINITY) : t.split[i]);
       if ((L & 1) == 0) {
-        unsigned w = cover >= 0 ? 0u : static_cast<unsigned>(t.feature[i]);
+        unsigned w = cover >= 0 ? 0u : static_cast<unsigned>(s_feature[i]);
         if (cover < 0 && L + 1 < S) {
-          if (splits_here(2 * i + 1)) w |= static_cast<unsigned>(t.feature[2 * i + 1]) << kIdBits;
-          if (splits_here(2 * i + 2)) w |= static_cast<unsigned>(t.feature[2 * i + 2]) << (2 * kIdBits);
+          if (splits_here(2 * i + 1)) w |= static_cast<unsigned>(s_feature[2 * i + 1]) << kIdBits;
+          if (splits_here(2 * i + 2)) w |= static_cast<unsigned>(s_feature[2 * i + 2]) << (2 * kIdBits);
         }
         words[i + 1] = w;
       }
@@ -787,7 +791,7 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
     finish(gate);
     return;
   }
-  k_pack_complete<T><<<n_trees, 256, 0, stream>>>(gate, d_trees, K, F, plan.rec, records, leaves_c);
+  k_pack_complete<T><<<n_trees, 256, sizeof(uint16_t) << S, stream>>>(gate, d_trees, K, F, plan.rec, records, leaves_c);
   LBK_LAUNCH_CHECK();
   const TiledArgs<T> a{X, ldx, n_rows, F, K, n_trees, plan.rb, plan.nbuf, plan.x_bytes, records, plan.rec, leaves_c, o, ctx->d_status};
   switch (plan.tg) {
