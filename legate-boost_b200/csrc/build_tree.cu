@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32, kForm == 0 ? 6 : 5)
                       const int32_t* __restrict__ split_bin, int max_depth, int n_nodes, int32_t* __restrict__ leaf,
                       const __grid_constant__ LeafRound rnd)
 {
+  AfterTheKernelBefore();
   constexpr bool kRound = kForm != 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned* s_node = reinterpret_cast<unsigned*>(smem_raw);
@@ -145,6 +146,7 @@ __global__ void __launch_bounds__(256)
   k_leaf_of_row(const BinT* __restrict__ bins, int64_t pitch, int64_t n_rows, const int32_t* __restrict__ feature,
                 const int32_t* __restrict__ split_bin, int max_depth, int32_t* __restrict__ leaf)
 {
+  AfterTheKernelBefore();
   const int64_t row = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (row >= n_rows) return;
   const BinT* b = bins + row * pitch;
@@ -177,12 +179,12 @@ void LeafOfRow(lbk_context* ctx, const void* bins, int64_t pitch, int64_t N, int
     const int64_t chunks = (N + 31) / 32;
     int64_t blocks       = static_cast<int64_t>(ctx->sm_count) * (per_sm > 0 ? per_sm : 1);
     blocks               = std::min<int64_t>(blocks, (chunks + kLeafWarps - 1) / kLeafWarps);
-    fn<<<static_cast<unsigned>(std::max<int64_t>(blocks, 1)), kLeafWarps * 32, smem, stream>>>(
+    LaunchChained(fn, static_cast<unsigned>(std::max<int64_t>(blocks, 1)), kLeafWarps * 32, smem, stream,
       static_cast<const BinT*>(bins), static_cast<int>(pitch_bytes), N, feature, split_bin, D, M, leaf,
       rnd != nullptr ? *rnd : LeafRound{});
   } else {
     const unsigned blocks = static_cast<unsigned>((N + 255) / 256);
-    k_leaf_of_row<BinT><<<blocks, 256, 0, stream>>>(static_cast<const BinT*>(bins), pitch, N, feature, split_bin, D, leaf);
+    LaunchChained(k_leaf_of_row<BinT>, blocks, 256, 0, stream, static_cast<const BinT*>(bins), pitch, N, feature, split_bin, D, leaf);
   }
   LBK_LAUNCH_CHECK();
 }
@@ -192,6 +194,7 @@ __global__ void __launch_bounds__(256)
   k_gather_rows(const double* __restrict__ table, const int32_t* __restrict__ index, int64_t n, int K,
                 double* __restrict__ out)
 {
+  AfterTheKernelBefore();
   const int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (e >= n * K) return;
   const int64_t i = e / K;
@@ -229,6 +232,7 @@ __global__ void __launch_bounds__(256)
   k_add_leaf_values(const double* __restrict__ table, const int32_t* __restrict__ leaf, int64_t n, int K,
                     double* __restrict__ pred)
 {
+  AfterTheKernelBefore();
   const int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (e >= n * K) return;
   const int64_t i = K == 1 ? e : e / K;
@@ -252,6 +256,7 @@ __global__ void __launch_bounds__(256)
   k_zero_if(const int* __restrict__ gate, int4* __restrict__ at, int64_t slot, int n_nodes, const int32_t* __restrict__ parent_feature, int clear,
             bool by_search)
 {
+  AfterTheKernelBefore();
   if (*gate == 0) return;
   const int lane = threadIdx.x & 31;
   const int64_t pieces = (slot + kZeroPiece - 1) / kZeroPiece, items = pieces * n_nodes;
@@ -367,7 +372,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     t.info_host = a.out_total_bins != nullptr ? words.get() : nullptr;
     SmallTree<T>(ctx, s, t, stream);
     if (round != nullptr && !fused) {
-      k_add_leaf_values<<<static_cast<unsigned>((N * K + 255) / 256), 256, 0, stream>>>(leaf_value, leaf, N, K, round->pred);
+      LaunchChained(k_add_leaf_values, static_cast<unsigned>((N * K + 255) / 256), 256, 0, stream, leaf_value, leaf, N, K, round->pred);
       LBK_LAUNCH_CHECK();
     }
     if (a.trace_node_sums && !keep_sums)
@@ -729,7 +734,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
       // built buffer: when nothing is derived the level histogram itself is the target
       GPairI64* target = derive ? built_buffer(depth & 1, n_slots) : may_derive ? built_buffer(depth & 1, n_nodes) : level_hist;
       if (may_derive) {
-        k_zero_if<<<ctx->sm_count * 8, 256, 0, stream>>>(hess_below_one, reinterpret_cast<int4*>(target), static_cast<int64_t>(node_elems), n_nodes,
+        LaunchChained(k_zero_if, ctx->sm_count * 8, 256, 0, stream, hess_below_one, reinterpret_cast<int4*>(target), static_cast<int64_t>(node_elems), n_nodes,
                                                          tree.feature + (nb - 1) / 2, n_slots, built_zeroed);
         LBK_LAUNCH_CHECK();
       }
@@ -844,7 +849,7 @@ void BuildTreeImpl(lbk_context* ctx, const lbk_build_tree_args& a, cudaStream_t 
     if (a.host_buffers && a.out_leaf)
       LBK_CUDA(cudaMemcpyAsync(a.out_leaf, d_leaf, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, stream));
     if (round != nullptr && !add_here) {
-      k_add_leaf_values<<<static_cast<unsigned>((N * K + 255) / 256), 256, 0, stream>>>(leaf_value, d_leaf, N, K, round->pred);
+      LaunchChained(k_add_leaf_values, static_cast<unsigned>((N * K + 255) / 256), 256, 0, stream, leaf_value, d_leaf, N, K, round->pred);
       LBK_LAUNCH_CHECK();
     }
   }
@@ -1220,7 +1225,7 @@ int lbk_leaf_values(lbk_context* ctx, const double* leaf_value, const int32_t* l
     const int64_t total  = n_rows * n_outputs;
     const int64_t blocks = (total + 255) / 256;
     LBK_EXPECT(blocks <= 2147483647ll, "too many elements for one launch");
-    lbk::k_gather_rows<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(leaf_value, leaf, n_rows, n_outputs, out);
+    lbk::LaunchChained(lbk::k_gather_rows, static_cast<unsigned>(blocks), 256, 0, stream, leaf_value, leaf, n_rows, n_outputs, out);
     LBK_LAUNCH_CHECK();
   });
 }

@@ -180,6 +180,7 @@ __device__ inline unsigned SmemAddr(const void* p) { return static_cast<unsigned
 // tree builder gets them from the quantiser)
 __global__ void k_max_abs(const int2* __restrict__ gpair, int64_t n, int* __restrict__ max_abs)
 {
+  AfterTheKernelBefore();
   int mg = 0, mh = 0;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -271,6 +272,7 @@ __global__ void __launch_bounds__(1024)
   k_hist_plan(const __grid_constant__ HistParams p, int GK, int resident, int min_chunk, bool whole_turns, int32_t* __restrict__ chunk_off,
               int32_t* __restrict__ wpre, int32_t* __restrict__ plan)
 {
+  AfterTheKernelBefore();
   __shared__ long long red[32];
   __shared__ long long wsum[32];
   __shared__ long long carry;
@@ -584,6 +586,7 @@ template <typename BinT, bool kFloat>
 __global__ void __launch_bounds__(kHistThreads)
   k_hist_direct(const HistParams p)
 {
+  AfterTheKernelBefore();
   using A = Acc<kFloat>;
   __shared__ unsigned int s_ticket;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -849,6 +852,7 @@ __global__ void __launch_bounds__(kHistThreads * W, W == 1 ? 2 : 1)
   constexpr int kLanesPerRow  = 2 * W;
   constexpr int kRowsPerBatch = 32 / kLanesPerRow;
   constexpr int kStageWords   = kFlushBins * 32;  // per warp
+  AfterTheKernelBefore();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned int s_ticket;
   __shared__ int s_nb[kCols];  // bins of the feature of each word (0: no feature, or a copy of another word)
@@ -1172,6 +1176,7 @@ template <typename BinT, int kBins, int kThreads, int kCopies>
 __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 6 : 1)
   k_hist_tile(const HistParams p)
 {
+  AfterTheKernelBefore();
   using A = Acc<false>;
   constexpr int kRow = kTileFeatures * kCopies;  // words of a bin
   extern __shared__ __align__(128) int s_hist[];  // [2][kBins][copies][8]
@@ -1560,7 +1565,7 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
     LBK_CUDA(cudaMemsetAsync(m, 0, 2 * sizeof(int), stream));
     const int64_t n = lv.n_rows * lv.K;
     if (n > 0) {
-      k_max_abs<<<ctx->sm_count * 8, 256, 0, stream>>>(lv.gpair, n, m);
+      LaunchChained(k_max_abs, ctx->sm_count * 8, 256, 0, stream, lv.gpair, n, m);
       LBK_LAUNCH_CHECK();
     }
     max_abs = m;
@@ -1601,7 +1606,7 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
     int32_t* wpre      = hl.smem_path ? s.alloc<int32_t>(static_cast<size_t>(lv.n_nodes) + 1) : nullptr;
     int32_t* plan      = s.alloc<int32_t>(8);
     p.ticket           = reinterpret_cast<unsigned int*>(plan + 2);
-    k_hist_plan<<<1, 1024, 0, stream>>>(p, units, hl.tile ? p.tile_items : hl.grid, hl.tile ? kTileMinRows : kMinChunk, hl.copies != 1, chunk_off, wpre, plan);
+    LaunchChained(k_hist_plan, 1, 1024, 0, stream, p, units, hl.tile ? p.tile_items : hl.grid, hl.tile ? kTileMinRows : kMinChunk, hl.copies != 1, chunk_off, wpre, plan);
     LBK_LAUNCH_CHECK();
     p.chunk_off = chunk_off;
     p.wpre      = wpre;
@@ -1614,8 +1619,7 @@ void BuildHistogram(lbk_context* ctx, Scratch& s, const HistLevel& lv, cudaStrea
     ev = NextProfileEvents(ctx);
     LBK_CUDA(cudaEventRecord(ev.first, stream));
   }
-  hl.fn<<<hl.grid, hl.threads, hl.smem, stream>>>(p);
-  LBK_LAUNCH_CHECK();
+  LaunchChained(hl.fn, hl.grid, hl.threads, hl.smem, stream, p);
   if (ctx->profile) LBK_CUDA(cudaEventRecord(ev.second, stream));
   // stream ordered: the slots go back to the pool once the kernel has run
   if (own.partial) s.free_one(own.partial);
@@ -1833,7 +1837,7 @@ extern "C" int lbk_histogram_noalloc(int device, const lbk_histogram_args* a)
     } else if (!float_mode) {
       const int64_t n = a->n_rows * K;
       if (n > 0) {
-        k_max_abs<<<sm_count * 8, 256, 0, stream>>>(static_cast<const int2*>(p.gpair), n, max_abs);
+        LaunchChained(k_max_abs, sm_count * 8, 256, 0, stream, static_cast<const int2*>(p.gpair), n, max_abs);
         LBK_LAUNCH_CHECK();
       }
     }
@@ -1853,9 +1857,9 @@ extern "C" int lbk_histogram_noalloc(int device, const lbk_histogram_args* a)
     p.n_arrive          = 0;
     p.tile_items        = sm_count * kTileItemsPerSm;
     const int units     = (hl.tile ? (F + kTileFeatures - 1) / kTileFeatures : (p.G + hl.width - 1) / hl.width) * K;
-    k_hist_plan<<<1, 1024, 0, stream>>>(p, units, hl.tile ? p.tile_items : hl.grid, hl.tile ? kTileMinRows : kMinChunk, hl.copies != 1, chunk_off, nullptr, plan);
+    LaunchChained(k_hist_plan, 1, 1024, 0, stream, p, units, hl.tile ? p.tile_items : hl.grid, hl.tile ? kTileMinRows : kMinChunk, hl.copies != 1, chunk_off, nullptr, plan);
     LBK_LAUNCH_CHECK();
-    hl.fn<<<hl.grid, hl.threads, hl.smem, stream>>>(p);
+    LaunchChained(hl.fn, hl.grid, hl.threads, hl.smem, stream, p);
     LBK_LAUNCH_CHECK();
     LBK_CUDA(cudaStreamSynchronize(stream));
   });

@@ -18,6 +18,7 @@ __global__ void __launch_bounds__(256)
   k_gradient_squared_error(const double* __restrict__ raw, const double* __restrict__ y, int64_t n, double lr,
                            double* __restrict__ g, double* __restrict__ h)
 {
+  AfterTheKernelBefore();
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   const double2 v = GradientSquaredError(raw[i], y[i], lr);
@@ -29,6 +30,7 @@ __global__ void __launch_bounds__(256)
   k_gradient_logloss_binary(const double* __restrict__ raw, const double* __restrict__ y, int64_t n, double lr,
                             double* __restrict__ g, double* __restrict__ h)
 {
+  AfterTheKernelBefore();
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   const double2 v = GradientLogistic(raw[i], y[i], lr);
@@ -47,6 +49,7 @@ __global__ void __launch_bounds__(kSoftmaxThreads)
   k_gradient_softmax(const double* __restrict__ raw, const double* __restrict__ label, int64_t n_rows, int K, int rows, double lr,
                      double* __restrict__ g, double* __restrict__ h)
 {
+  AfterTheKernelBefore();
   extern __shared__ double s_e[];
   const int pitch    = K | 1;
   double* s_div      = s_e + rows * pitch;
@@ -86,6 +89,7 @@ __global__ void __launch_bounds__(256)
   k_gradient_softmax_wide(const double* __restrict__ raw, const double* __restrict__ label, int64_t n_rows, int K, double lr,
                           double* __restrict__ g, double* __restrict__ h)
 {
+  AfterTheKernelBefore();
   const int64_t row = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (row >= n_rows) return;
   const double* r = raw + row * K;
@@ -109,16 +113,16 @@ void Gradient(int objective, const double* raw_pred, const double* y, int64_t n_
   if (n_rows == 0) return;
   const int64_t n = n_rows * n_outputs;
   if (objective == LBK_SQUARED_ERROR) {
-    k_gradient_squared_error<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(raw_pred, y, n, learning_rate, g, h);
+    LaunchChained(k_gradient_squared_error, static_cast<unsigned>((n + 255) / 256), 256, 0, stream, raw_pred, y, n, learning_rate, g, h);
   } else if (n_outputs == 1) {
-    k_gradient_logloss_binary<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(raw_pred, y, n, learning_rate, g, h);
+    LaunchChained(k_gradient_logloss_binary, static_cast<unsigned>((n + 255) / 256), 256, 0, stream, raw_pred, y, n, learning_rate, g, h);
   } else {
     const int rows = static_cast<int>(std::min<size_t>(kSoftmaxThreads, 48 * 1024 / SoftmaxRowBytes(n_outputs)) / 32 * 32);
     if (rows > 0)
-      k_gradient_softmax<<<static_cast<unsigned>((n_rows + rows - 1) / rows), kSoftmaxThreads, rows * SoftmaxRowBytes(n_outputs), stream>>>(
+      LaunchChained(k_gradient_softmax, static_cast<unsigned>((n_rows + rows - 1) / rows), kSoftmaxThreads, rows * SoftmaxRowBytes(n_outputs), stream,
         raw_pred, y, n_rows, n_outputs, rows, learning_rate, g, h);
     else
-      k_gradient_softmax_wide<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(raw_pred, y, n_rows, n_outputs,
+      LaunchChained(k_gradient_softmax_wide, static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream, raw_pred, y, n_rows, n_outputs,
                                                                                              learning_rate, g, h);
   }
   LBK_LAUNCH_CHECK();

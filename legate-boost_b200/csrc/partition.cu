@@ -43,6 +43,7 @@ __device__ inline int ChunksOf(const PartitionLevel& p, int j)
 __global__ void __launch_bounds__(1024)
   k_part_plan(const __grid_constant__ PartitionLevel p, int32_t* __restrict__ chunk_off)
 {
+  AfterTheKernelBefore();
   __shared__ int carry, wsum[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {
@@ -164,6 +165,7 @@ template <typename BinT, bool kPlanInside, bool kBands>
 __global__ void __launch_bounds__(kPartThreads, kPartBlocks)
   k_partition(const __grid_constant__ PartitionLevel p, const int32_t* __restrict__ chunk_off_global, int log_bands)
 {
+  AfterTheKernelBefore();
   __shared__ int32_t s_off[kPlanInside ? kPartPlanNodes + 1 : 1];
   __shared__ int32_t s_count[kBands ? kPartPlanNodes : 1];
   __shared__ int32_t s_band[kBands ? (1 << kPartMaxLogBands) + 1 : 1];  // chunks before each band
@@ -341,7 +343,7 @@ void PartitionRows(lbk_context* ctx, Scratch& s, const PartitionLevel& pl, cudaS
   int32_t* chunk_off       = nullptr;
   if (!inside) {
     chunk_off = s.alloc<int32_t>(static_cast<size_t>(pl.n_nodes) + 1);
-    k_part_plan<<<1, 1024, 0, stream>>>(pl, chunk_off);
+    LaunchChained(k_part_plan, 1, 1024, 0, stream, pl, chunk_off);
     LBK_LAUNCH_CHECK();
   }
   int log_bands = 0;
@@ -350,8 +352,7 @@ void PartitionRows(lbk_context* ctx, Scratch& s, const PartitionLevel& pl, cudaS
            (pl.n_rows / kPartTile) >> (log_bands + 1) >= kPartBandTurns * grid)
       ++log_bands;
   auto fn = pl.bin_bytes == 1 ? PartitionKernel<uint8_t>(inside, log_bands > 0) : PartitionKernel<uint16_t>(inside, log_bands > 0);
-  fn<<<grid, kPartThreads, 0, stream>>>(pl, chunk_off, log_bands);
-  LBK_LAUNCH_CHECK();
+  LaunchChained(fn, grid, kPartThreads, 0, stream, pl, chunk_off, log_bands);
 }
 
 }  // namespace lbk

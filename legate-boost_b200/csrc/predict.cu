@@ -84,6 +84,7 @@ template <typename NodeT>
 __global__ void k_pack_trees(const int* __restrict__ gate, const TreePtrs* __restrict__ trees, int K, int F, NodeT* __restrict__ nodes,
                              double* __restrict__ leaves)
 {
+  AfterTheKernelBefore();
   if (SkipFor(gate)) return;
   const TreePtrs t = trees[blockIdx.x];
   for (int i = threadIdx.x; i < t.max_nodes; i += blockDim.x) {
@@ -125,6 +126,7 @@ template <typename T>
 __global__ void k_pack_complete(const int* __restrict__ gate, const TreePtrs* __restrict__ trees, int K, int F, TreeRecord rec,
                                 unsigned char* __restrict__ records, double* __restrict__ leaves_c)
 {
+  AfterTheKernelBefore();
   if (SkipFor(gate)) return;
   const TreePtrs t   = trees[blockIdx.x];
   const int M = t.max_nodes, S = rec.S;
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(kRowsThreads)
   k_predict_rows(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, int K, int n_trees, int rows_per_block,
                  const TreePtrs* __restrict__ trees, PredictOut o)
 {
+  AfterTheKernelBefore();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // [rows][trees] values (K == 1) or addresses of the leaves' values | [rows][K] sums | [rows][F] X
   double* vals        = reinterpret_cast<double*>(smem_raw);
@@ -265,6 +268,7 @@ struct TiledArgs {
 template <typename T, int TG, int KR, int kStaged, bool kGated = false>
 __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledArgs<T> a, const int* __restrict__ gate)
 {
+  AfterTheKernelBefore();
   __shared__ __align__(8) unsigned long long s_bar[4];  // full[2], empty[2]
   __shared__ int s_failed;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -560,6 +564,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_predict_tiled(const TiledAr
 // The raw sums of an ensemble without trees; nothing of X is read.
 __global__ void __launch_bounds__(256) k_predict_nothing(int64_t n_rows, int K, PredictOut o)
 {
+  AfterTheKernelBefore();
   const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (row >= n_rows) return;
   for (int k = 0; k < K; ++k) o.pred[row * o.ldp + k] = o.init ? o.init[k] : 0.0;
@@ -568,6 +573,7 @@ __global__ void __launch_bounds__(256) k_predict_nothing(int64_t n_rows, int K, 
 // What is left to do after a kernel that wrote the raw sums.
 __global__ void __launch_bounds__(256) k_finish_rows(const int* __restrict__ gate, int64_t n_rows, int K, PredictOut o)
 {
+  AfterTheKernelBefore();
   if (SkipFor(gate)) return;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (row >= n_rows) return;
@@ -582,6 +588,7 @@ __global__ void __launch_bounds__(128)
                    const TreePtrs* __restrict__ trees, const typename NodeOf<T>::type* __restrict__ nodes,
                    const double* __restrict__ leaves, PredictOut o)
 {
+  AfterTheKernelBefore();
   using NodeT       = typename NodeOf<T>::type;
   if (SkipFor(gate)) return;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -706,7 +713,7 @@ void LaunchTiledAs(lbk_context* ctx, const int* gate, const TiledArgs<T>& a, con
     }
   // (whatever the size: the limit without it is for the static and the dynamic part together)
   AllowSharedMemory(ctx, fn, kTileStaticBytes);
-  fn<<<static_cast<unsigned>(grid), a.rb + 32, plan.smem, stream>>>(a, gate);
+  LaunchChained(fn, static_cast<unsigned>(grid), a.rb + 32, plan.smem, stream, a, gate);
   LBK_LAUNCH_CHECK();
 }
 
@@ -736,11 +743,11 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   const PredictOut o{pred, ldp, init, transform};
   auto finish = [&](const int* gate) {
     if (transform == LBK_RAW) return;
-    k_finish_rows<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(gate, n_rows, K, o);
+    LaunchChained(k_finish_rows, static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream, gate, n_rows, K, o);
     LBK_LAUNCH_CHECK();
   };
   if (n_trees == 0) {
-    k_predict_nothing<<<static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream>>>(n_rows, K, o);
+    LaunchChained(k_predict_nothing, static_cast<unsigned>((n_rows + 255) / 256), 256, 0, stream, n_rows, K, o);
     LBK_LAUNCH_CHECK();
     finish(nullptr);
     return;
@@ -755,7 +762,7 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
     while (r > 1 && need(r) > 48 * 1024) r /= 2;
     if (n_rows <= kRowsMax && need(r) <= 48 * 1024) {
       const unsigned grid = static_cast<unsigned>((n_rows + r - 1) / r);
-      k_predict_rows<T><<<grid, kRowsThreads, need(r), stream>>>(X, ldx, n_rows, F, K, n_trees, r, d_trees, o);
+      LaunchChained(k_predict_rows<T>, grid, kRowsThreads, need(r), stream, X, ldx, n_rows, F, K, n_trees, r, d_trees, o);
       LBK_LAUNCH_CHECK();
       return;
     }
@@ -783,15 +790,15 @@ void PredictLaunch(lbk_context* ctx, Scratch& s, const T* X, int64_t ldx, int64_
   const int* gate = nullptr;
   if (ranked.threads > 0 && !ranked.sure) gate = by_ranks();
   if (plan.rb == 0) {
-    k_pack_trees<NodeT><<<n_trees, 256, 0, stream>>>(gate, d_trees, K, F, nodes, leaves);
+    LaunchChained(k_pack_trees<NodeT>, n_trees, 256, 0, stream, gate, d_trees, K, F, nodes, leaves);
     LBK_LAUNCH_CHECK();
     const unsigned grid = static_cast<unsigned>((n_rows + 127) / 128);
-    k_predict_global<T><<<grid, 128, 0, stream>>>(gate, X, ldx, n_rows, K, n_trees, d_trees, nodes, leaves, o);
+    LaunchChained(k_predict_global<T>, grid, 128, 0, stream, gate, X, ldx, n_rows, K, n_trees, d_trees, nodes, leaves, o);
     LBK_LAUNCH_CHECK();
     finish(gate);
     return;
   }
-  k_pack_complete<T><<<n_trees, 256, sizeof(uint16_t) << S, stream>>>(gate, d_trees, K, F, plan.rec, records, leaves_c);
+  LaunchChained(k_pack_complete<T>, n_trees, 256, sizeof(uint16_t) << S, stream, gate, d_trees, K, F, plan.rec, records, leaves_c);
   LBK_LAUNCH_CHECK();
   const TiledArgs<T> a{X, ldx, n_rows, F, K, n_trees, plan.rb, plan.nbuf, plan.x_bytes, records, plan.rec, leaves_c, o, ctx->d_status};
   switch (plan.tg) {

@@ -84,6 +84,7 @@ __device__ inline void CountSplits(const TreePtrs& t, int F, int* s_n)
 template <typename T>
 __global__ void __launch_bounds__(256) k_rank_count(const TreePtrs* __restrict__ trees, int F, int* __restrict__ counts)
 {
+  AfterTheKernelBefore();
   __shared__ int s_n[kMaxFeatures];
   CountSplits<T>(trees[blockIdx.x], F, s_n);
   for (int f = threadIdx.x; f < F; f += blockDim.x)
@@ -117,6 +118,7 @@ __global__ void __launch_bounds__(256)
   k_rank_scatter(const TreePtrs* __restrict__ trees, int F, const int* __restrict__ counts, int* __restrict__ cursor, int* __restrict__ off,
                  int2* __restrict__ items, int* __restrict__ n_items, int* __restrict__ declined, T* __restrict__ lists)
 {
+  AfterTheKernelBefore();
   constexpr int kPer = kMaxFeatures / 256;
   __shared__ int s_n[kMaxFeatures], s_at[kMaxFeatures], s_wsum[8];
   const int tid = threadIdx.x;
@@ -449,6 +451,7 @@ __device__ inline bool SortByBuckets(T* s, unsigned* start /* [kSortChunk / 2]: 
 template <typename T>
 __global__ void __launch_bounds__(kSortThreads) k_rank_sort(const RankTables<T> a)
 {
+  AfterTheKernelBefore();
   __shared__ T s[kSortChunk];
   __shared__ __align__(8) unsigned s_start[kSortChunk / 2];
   __shared__ int s_wsum[kSortThreads / 32];
@@ -486,6 +489,7 @@ __global__ void __launch_bounds__(kSortThreads) k_rank_sort(const RankTables<T> 
 template <typename T>
 __global__ void __launch_bounds__(kSortThreads) k_rank_merge(const RankTables<T> a)
 {
+  AfterTheKernelBefore();
   __shared__ int s_len[kMaxChunks], s_wsum[kSortThreads / 32];
   __shared__ bool s_last;
   if (__syncthreads_or(*reinterpret_cast<volatile int*>(a.declined)) || static_cast<int>(blockIdx.x) >= *a.n_items) return;  // (all threads or none)
@@ -614,6 +618,7 @@ __global__ void __launch_bounds__(256)
   k_rank_pack(const TreePtrs* __restrict__ trees, int F, int S, int lines, float millions, float budget, unsigned room, const RankTable* __restrict__ tables,
               const T* __restrict__ cuts, const unsigned* __restrict__ lut, int* __restrict__ declined, unsigned char* __restrict__ records)
 {
+  AfterTheKernelBefore();
   // (a feature has no table; or another block has found the same as this one would: all threads or none)
   if (__syncthreads_or(*reinterpret_cast<volatile int*>(declined))) return;
   __shared__ int s_begin[8][33];
@@ -886,6 +891,7 @@ __device__ __noinline__ unsigned FillTables(const RankRowsArgs<T>& a, const int*
 template <typename T>
 __global__ void __launch_bounds__(kRankThreads, 1) k_rank_rows(const RankRowsArgs<T> a)
 {
+  AfterTheKernelBefore();
   constexpr int kWarps = kRankThreads / 32, kPitch = kRankTileRows + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (*a.declined != 0) return;
@@ -963,6 +969,7 @@ struct RankedArgs {
 template <int TG>
 __global__ void __launch_bounds__(kWalkThreads + 32, 1) k_predict_ranked(const RankedArgs a)
 {
+  AfterTheKernelBefore();
   __shared__ __align__(8) unsigned long long s_bar[5];  // full[2], empty[2], the tile
   __shared__ int s_failed;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1237,17 +1244,17 @@ const int* PredictRanked(lbk_context* ctx, Scratch& s, const RankedPlan& plan, c
   unsigned* ranks        = reinterpret_cast<unsigned*>(room + plan.o_ranks);
   const unsigned items   = static_cast<unsigned>(plan.max_items);
   LBK_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * (3 * static_cast<size_t>(F) + 2), stream));
-  k_rank_count<T><<<n_trees, 256, 0, stream>>>(d_trees, F, counts);
+  LaunchChained(k_rank_count<T>, n_trees, 256, 0, stream, d_trees, F, counts);
   LBK_LAUNCH_CHECK();
-  k_rank_scatter<T><<<n_trees, 256, 0, stream>>>(d_trees, F, counts, counts + F, const_cast<int*>(t.off), const_cast<int2*>(t.items), words + 1, declined, t.lists);
+  LaunchChained(k_rank_scatter<T>, n_trees, 256, 0, stream, d_trees, F, counts, counts + F, const_cast<int*>(t.off), const_cast<int2*>(t.items), words + 1, declined, t.lists);
   LBK_LAUNCH_CHECK();
-  k_rank_sort<T><<<items, kSortThreads, 0, stream>>>(t);
+  LaunchChained(k_rank_sort<T>, items, kSortThreads, 0, stream, t);
   LBK_LAUNCH_CHECK();
   if (total_nodes / 2 > kSortChunk) {
-    k_rank_merge<T><<<dim3(items, kSortChunk / kSortThreads), kSortThreads, 0, stream>>>(t);
+    LaunchChained(k_rank_merge<T>, dim3(items, kSortChunk / kSortThreads), kSortThreads, 0, stream, t);
     LBK_LAUNCH_CHECK();
   }
-  k_rank_pack<T><<<n_trees, 256, sizeof(uint16_t) << S, stream>>>(d_trees, F, S, plan.threads / 32, plan.sure ? 0.f : static_cast<float>(n_rows) * 1e-6f, static_cast<float>(plan.budget), TableRoom(ctx), t.tables, cuts, t.lut, declined, records);
+  LaunchChained(k_rank_pack<T>, n_trees, 256, sizeof(uint16_t) << S, stream, d_trees, F, S, plan.threads / 32, plan.sure ? 0.f : static_cast<float>(n_rows) * 1e-6f, static_cast<float>(plan.budget), TableRoom(ctx), t.tables, cuts, t.lut, declined, records);
   LBK_LAUNCH_CHECK();
   AllowSharedMemory(ctx, k_rank_rows<T>, kRankStatic);
   const int64_t tile    = 2 * plan.threads;
@@ -1261,10 +1268,10 @@ const int* PredictRanked(lbk_context* ctx, Scratch& s, const RankedPlan& plan, c
   for (int64_t r0 = 0; r0 < n_rows; r0 += plan.piece) {
     const int64_t rows = std::min(plan.piece, n_rows - r0), tiles = (rows + tile - 1) / tile;
     RankRowsArgs<T> ra{X + r0 * ldx, ldx, rows, F, plan.threads, tiles, t.tables, cuts, t.lut, declined, ranks, tail_blocks};
-    k_rank_rows<T><<<blocks, kRankThreads, RowsSmem(ctx), stream>>>(ra);
+    LaunchChained(k_rank_rows<T>, blocks, kRankThreads, RowsSmem(ctx), stream, ra);
     LBK_LAUNCH_CHECK();
     RankedArgs wa{rows, F, n_trees, S, plan.nbuf, ranks, records, declined, PredictOut{pred + r0 * ldp, ldp, init, transform}, ctx->d_status};
-    walk<<<static_cast<unsigned>(tiles), plan.threads + 32, plan.smem, stream>>>(wa);
+    LaunchChained(walk, static_cast<unsigned>(tiles), plan.threads + 32, plan.smem, stream, wa);
     LBK_LAUNCH_CHECK();
   }
   return declined;

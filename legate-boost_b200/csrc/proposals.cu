@@ -148,6 +148,7 @@ template <typename T>
 __global__ void __launch_bounds__(kSortThreads)
   k_prologue(const __grid_constant__ PrologueArgs<T> p)
 {
+  AfterTheKernelBefore();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_cnt[kSortThreads / 32 + 1];
   __shared__ double s_sum[2 * kSumThreads / 32];
@@ -184,6 +185,7 @@ __global__ void __launch_bounds__(1024)
                     int32_t* info_host, double* part_g, double* part_h, int64_t n_parts, double* sums,
                     QuantParams* params)
 {
+  AfterTheKernelBefore();
   __shared__ int warp_sums[32];
   __shared__ int carry_s;
   __shared__ int max_s;
@@ -269,6 +271,7 @@ template <typename T>
 __global__ void k_write_proposals(const T* __restrict__ cuts, int S, const int32_t* __restrict__ row_ptr,
                                   T* __restrict__ proposals)
 {
+  AfterTheKernelBefore();
   const int f     = blockIdx.x;
   const int begin = row_ptr[f], end = row_ptr[f + 1];
   for (int j = threadIdx.x; j < end - begin; j += blockDim.x) proposals[begin + j] = cuts[static_cast<int64_t>(f) * S + j];
@@ -428,6 +431,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
   k_bin_smem(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const T* __restrict__ proposals,
              int64_t cut_stride, const int32_t* __restrict__ row_ptr, BinT* __restrict__ bins, BinT* __restrict__ bins_t, int64_t pitch_t)
 {
+  AfterTheKernelBefore();
   constexpr int P = 1 << kLog2P;
   constexpr bool kTile = kCopyT && sizeof(BinT) == 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -608,6 +612,7 @@ __global__ void __launch_bounds__(kLutThreads, 1)
             int64_t cut_stride, const int32_t* __restrict__ row_ptr, uint8_t* __restrict__ bins, uint8_t* __restrict__ bins_t, int64_t pitch_t,
             int* __restrict__ status)
 {
+  AfterTheKernelBefore();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_n[kGroup];
   __shared__ float2 s_map[kGroup];
@@ -815,6 +820,7 @@ __global__ void __launch_bounds__(kWideThreads, 2)
   k_bin_wide(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const T* __restrict__ proposals, int64_t cut_stride,
              const int32_t* __restrict__ row_ptr, int pitch, uint16_t* __restrict__ bins, uint16_t* __restrict__ bins_t, int64_t pitch_t)
 {
+  AfterTheKernelBefore();
   using Table             = WideTable<T, kLog2P>;
   constexpr int P         = Table::P;
   constexpr int kFeatures = Table::kFeatures;
@@ -887,6 +893,7 @@ __global__ void __launch_bounds__(256)
   k_bin_global(const T* __restrict__ X, int64_t ldx, int64_t n_rows, int F, const T* __restrict__ proposals,
                int64_t cut_stride, const int32_t* __restrict__ row_ptr, BinT* __restrict__ bins, BinT* __restrict__ bins_t, int64_t pitch_t)
 {
+  AfterTheKernelBefore();
   const int g    = blockIdx.y;
   const int f0   = g * kGroup;
   const int lane = threadIdx.x & 31;
@@ -956,11 +963,11 @@ void Prologue(lbk_context* ctx, Scratch& s, PrologueArgs<T> p, int32_t* row_ptr,
   p.fill_blocks = static_cast<int>(std::min<int64_t>((fill + 4 * kSortThreads - 1) / (4 * kSortThreads), ctx->sm_count * 4));
   const int64_t blocks = p.sort_blocks + p.sum_blocks + p.fill_blocks;
   if (blocks > 0) {
-    k_prologue<T><<<static_cast<unsigned>(blocks), kSortThreads, SortSmem<T>(p.S_pad), stream>>>(p);
+    LaunchChained(k_prologue<T>, static_cast<unsigned>(blocks), kSortThreads, SortSmem<T>(p.S_pad), stream, p);
     LBK_LAUNCH_CHECK();
   }
   const bool one_rank = ctx->n_ranks <= 1;
-  k_prologue_finish<<<1, 1024, 0, stream>>>(p.counts, p.F, row_ptr, info, info_host, p.part_g, p.part_h, p.sum_blocks, sums,
+  LaunchChained(k_prologue_finish, 1, 1024, 0, stream, p.counts, p.F, row_ptr, info, info_host, p.part_g, p.part_h, p.sum_blocks, sums,
                                             one_rank ? params : nullptr);
   LBK_LAUNCH_CHECK();
   if (!one_rank && sums != nullptr) {
@@ -988,7 +995,7 @@ ProposalInfo SplitProposals(lbk_context* ctx, Scratch& s, const T* X, int64_t ld
   p.counts       = s.alloc<int32_t>(F);
   int32_t* info  = s.alloc<int32_t>(2);
   Prologue<T>(ctx, s, p, row_ptr, info, nullptr, nullptr, nullptr, stream);
-  k_write_proposals<T><<<F, 128, 0, stream>>>(p.cuts, S, row_ptr, proposals);
+  LaunchChained(k_write_proposals<T>, F, 128, 0, stream, p.cuts, S, row_ptr, proposals);
   LBK_LAUNCH_CHECK();
   int32_t h[2] = {0, 0};
   LBK_CUDA(cudaMemcpyAsync(h, info, sizeof(h), cudaMemcpyDeviceToHost, stream));
@@ -1030,7 +1037,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       LBK_CUDA(cudaFuncSetAttribute(fn_, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))); \
     int per_sm_ = 0;                                                                                      \
     LBK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_, fn_, 256, smem));                    \
-    fn_<<<make_grid(per_sm_, kSmemFillRows), 256, smem, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr,                 \
+    LaunchChained(fn_, make_grid(per_sm_, kSmemFillRows), 256, smem, stream, X, ldx, n_rows, F, proposals, cut_stride, row_ptr,                 \
                                                    static_cast<BinT*>(bins), static_cast<BinT*>(bins_t), pitch_t); \
   } while (0)
 #define LBK_BIN_SMEM(BinT, L)                                                                             \
@@ -1045,7 +1052,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       else if (log2p == 8) LBK_BIN_SMEM(BinT, 8);                                                         \
       else LBK_BIN_SMEM(BinT, 9);                                                                         \
     } else {                                                                                              \
-      k_bin_global<T, BinT><<<make_grid(8, 0), 256, 0, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr,     \
+      LaunchChained(k_bin_global<T, BinT>, make_grid(8, 0), 256, 0, stream, X, ldx, n_rows, F, proposals, cut_stride, row_ptr,     \
                                                        static_cast<BinT*>(bins), static_cast<BinT*>(bins_t), \
                                                        pitch_t);                                          \
     }                                                                                                     \
@@ -1055,7 +1062,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
     if (bin_bytes == 1 && log2p == 8 && (reinterpret_cast<uintptr_t>(bins) & 3) == 0) {
       auto fn = bins_t != nullptr ? k_bin_lut<true> : k_bin_lut<false>;
       LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLutEnd)));
-      fn<<<make_grid(1, kLutFillRows), kLutThreads, kLutEnd, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, static_cast<uint8_t*>(bins),
+      LaunchChained(fn, make_grid(1, kLutFillRows), kLutThreads, kLutEnd, stream, X, ldx, n_rows, F, proposals, cut_stride, row_ptr, static_cast<uint8_t*>(bins),
                                                   static_cast<uint8_t*>(bins_t), pitch_t, status);
       LBK_LAUNCH_CHECK();
       return;
@@ -1071,7 +1078,7 @@ void BinMatrix(const T* X, int64_t ldx, int64_t n_rows, int F, const T* proposal
       LBK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Table::kSmem)));
       // (two blocks per SM, spread over the tables that hold features)
       const dim3 grid(blocks_of((F + kFeatures - 1) / kFeatures, 2, kSmemFillRows), G * kGroup / kFeatures);
-      fn<<<grid, kWideThreads, Table::kSmem, stream>>>(X, ldx, n_rows, F, proposals, cut_stride, row_ptr, G * kGroup,
+      LaunchChained(fn, grid, kWideThreads, Table::kSmem, stream, X, ldx, n_rows, F, proposals, cut_stride, row_ptr, G * kGroup,
                                                  static_cast<uint16_t*>(bins), static_cast<uint16_t*>(bins_t), pitch_t);
     };
     auto by_copy = [&](auto log2p_) {

@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(256)
              int2* __restrict__ gpair, GPairI64* __restrict__ root_sums, int* __restrict__ max_abs,
              int* __restrict__ hess_below_one)
 {
+  AfterTheKernelBefore();
   extern __shared__ unsigned long long s_sum[];  // [K][2]
   __shared__ int s_max[2];
   const QuantParams qp = *qp_ptr;
@@ -102,7 +103,7 @@ void Quantise(lbk_context* ctx, const double* g, const double* h, int64_t ldg, c
     const size_t smem = sizeof(unsigned long long) * 2 * K;
     LBK_EXPECT(smem <= 48 * 1024, "too many outputs for the quantiser's block sums");
     if (smem > 40 * 1024) AllowSharedMemory(ctx, k_quantise, 1024);  // (the limit without it counts the static part too)
-    k_quantise<<<static_cast<unsigned>(blocks), 256, smem, stream>>>(g, h, ldg, form, row_offset, n_local, K,
+    LaunchChained(k_quantise, static_cast<unsigned>(blocks), 256, smem, stream, g, h, ldg, form, row_offset, n_local, K,
                                                                   static_cast<long long>(seed), params, gpair, root_sums, max_abs,
                                                                   hess_below_one);
     LBK_LAUNCH_CHECK();

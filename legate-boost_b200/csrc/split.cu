@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kSplitThreads, kManyOutputs || kWide ? 3 : 4)
   __shared__ SliceBest s_best[2];
   __shared__ bool s_last;
   __shared__ int s_live[kWide ? kSplitWarps : 1];
+  AfterTheKernelBefore();
   const ScanSplitLevel& lv = p.lv;
   if (lv.build_all != nullptr && (*lv.build_all != 0) == kDerive) return;
   const int K = lv.K, unit = blockIdx.x;
@@ -509,6 +510,7 @@ __global__ void __launch_bounds__(256)
   k_finish_tree(TreeArrays tree, const QuantParams* __restrict__ qp_ptr, int K, int64_t n, double l1, double l2,
                 double* __restrict__ hessian)
 {
+  AfterTheKernelBefore();
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   const double2 v    = FinishedNode(tree, *qp_ptr, K, i, l1, l2);
@@ -559,8 +561,7 @@ void ScanSplit(lbk_context* ctx, Scratch& s, const ScanSplitLevel& lv, int F, co
                      : (lv.derive ? (wide ? k_scan_split<T, false, true, true> : k_scan_split<T, false, true, false>)
                                   : (wide ? k_scan_split<T, false, false, true> : k_scan_split<T, false, false, false>));
   if (smem > 40 * 1024) AllowSharedMemory(ctx, fn, 2048);  // (the limit without it counts the static part too)
-  fn<<<dim3(units, slices), kSplitThreads, smem, stream>>>(p);
-  LBK_LAUNCH_CHECK();
+  LaunchChained(fn, dim3(units, slices), kSplitThreads, smem, stream, p);
   if (exchange_records) {
     // every rank has searched its own features: the candidates of all ranks meet on every rank
     if (!AllGatherBytes(ctx, mine, all, rb * lv.n_nodes, stream))
@@ -578,7 +579,7 @@ void FinishTree(const TreeArrays& tree, const QuantParams* qp, int K, double l1,
                 cudaStream_t stream)
 {
   const int64_t n = static_cast<int64_t>(tree.max_nodes) * K;
-  k_finish_tree<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(tree, qp, K, n, l1, l2, hessian);
+  LaunchChained(k_finish_tree, static_cast<unsigned>((n + 255) / 256), 256, 0, stream, tree, qp, K, n, l1, l2, hessian);
   LBK_LAUNCH_CHECK();
 }
 

@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(kUpdThreads)
                 const double* __restrict__ h, int64_t ldg, int F, int K, int max_nodes, const int32_t* __restrict__ feature,
                 const double* __restrict__ split_value, double* __restrict__ sums /* [max_nodes][K][2] */)
 {
+  AfterTheKernelBefore();
   extern __shared__ double s_sums[];
   const int words = max_nodes * K * 2;
   if (kSmem) {
@@ -71,6 +72,7 @@ __global__ void __launch_bounds__(kUpdThreads)
 __global__ void __launch_bounds__(1024)
   k_update_ascend(double* __restrict__ sums, int K, int max_nodes, int F, const int32_t* __restrict__ feature)
 {
+  AfterTheKernelBefore();
   int top = 0;
   while ((2 << top) - 1 <= max_nodes) ++top;  // levels 0..top-1 are complete; level `top` may be cut
   for (int level = top; level >= 0; --level) {
@@ -91,6 +93,7 @@ __global__ void __launch_bounds__(1024)
 __global__ void k_update_finish(const double* __restrict__ sums, int64_t n, double l1, double l2,
                                 double* __restrict__ leaf_value, double* __restrict__ hessian)
 {
+  AfterTheKernelBefore();
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   const double G = sums[2 * i], H = sums[2 * i + 1];
@@ -116,20 +119,20 @@ void UpdateTreeImpl(lbk_context* ctx, const lbk_update_tree_args& a, cudaStream_
     if (smem <= static_cast<size_t>(kUpdSmemBytes)) {
       if (smem > 48 * 1024)
         LBK_CUDA(cudaFuncSetAttribute(k_update_ends<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdSmemBytes));
-      k_update_ends<T, true><<<static_cast<unsigned>(blocks), kUpdThreads, smem, stream>>>(
+      LaunchChained(k_update_ends<T, true>, static_cast<unsigned>(blocks), kUpdThreads, smem, stream,
         X, a.ldx, N, a.g, a.h, a.ldg, a.n_features, K, M, a.feature, a.split_value, sums);
     } else {
-      k_update_ends<T, false><<<static_cast<unsigned>(blocks), kUpdThreads, 0, stream>>>(
+      LaunchChained(k_update_ends<T, false>, static_cast<unsigned>(blocks), kUpdThreads, 0, stream,
         X, a.ldx, N, a.g, a.h, a.ldg, a.n_features, K, M, a.feature, a.split_value, sums);
     }
     LBK_LAUNCH_CHECK();
   }
-  k_update_ascend<<<1, 1024, 0, stream>>>(sums, K, M, a.n_features, a.feature);
+  LaunchChained(k_update_ascend, 1, 1024, 0, stream, sums, K, M, a.n_features, a.feature);
   LBK_LAUNCH_CHECK();
   // the reference reduces gradients and hessians with one all-reduce each; they are interleaved here
   AllReduce(ctx, sums, static_cast<size_t>(words), LBK_F64, LBK_SUM, stream);
   const int64_t n = static_cast<int64_t>(M) * K;
-  k_update_finish<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(sums, n, a.l1_regularization,
+  LaunchChained(k_update_finish, static_cast<unsigned>((n + 255) / 256), 256, 0, stream, sums, n, a.l1_regularization,
                                                                              a.l2_regularization, a.leaf_value, a.hessian);
   LBK_LAUNCH_CHECK();
   CheckDeviceStatus(ctx, stream);

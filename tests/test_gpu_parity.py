@@ -690,6 +690,36 @@ def test_predict_of_even_and_odd_outputs(lb, oracle, K, dt):
     assert np.allclose(softmax, e / e.sum(axis=1, keepdims=True), rtol=1e-13, atol=0)  # (a few roundings of exp and a sum)
 
 
+@pytest.mark.parametrize("N,F,K,T,D,dt", [(16, 30, 1, 100, 6, np.float32), (20_001, 40, 10, 20, 6, np.float32), (900_001, 30, 1, 100, 8, np.float64)])
+def test_chained_launches_under_capture_and_on_two_streams(lb, N, F, K, T, D, dt):
+    """Kernels that may begin as the one before them ends see all that it wrote: in a captured graph, replayed on changing inputs,
+    and in calls on two streams at a time."""
+    from legateboost_b200.tree import TreeTable
+
+    rs = np.random.RandomState(N % 89)
+    trees = [(dev(rs.normal(size=(t[1].shape[0], K))),) + t[1:] for t in _random_trees(rs, T, D, np.arange(F))]
+    table = TreeTable(trees)
+    inputs = [dev(rs.random((N, F)).astype(dt)) for _ in range(3)]
+    want = [table.predict(X, K, wait=True) for X in inputs]
+    X, streams = inputs[0].clone(), [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[0]):
+        got = table.predict(X * 1, K)
+    for given, expected in zip(inputs[::-1], want[::-1]):
+        X.copy_(given)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, expected)
+    out = []
+    for turn in range(6):
+        with torch.cuda.stream(streams[turn % 2]):
+            out.append(table.predict(inputs[turn % 3] * 1, K))
+    torch.cuda.synchronize()
+    for turn in range(6):
+        assert torch.equal(out[turn], want[turn % 3])
+
+
 def test_predict_without_room_for_ranks(lb):
     """A caller's allocator that has no 20 MB gets the predictions by the path that needs less."""
     from legateboost_b200.tree import TreeTable
