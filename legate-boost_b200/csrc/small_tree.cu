@@ -749,9 +749,11 @@ struct SmallPlan {
 // Is this form faster than the general path?  A block passes over all rows for every feature, output and chunk of pairs of
 // nodes that it has, and takes the pairs in turns; the general path pays for launches, whatever they do, and a little for
 // bins and rows.  Fitted to 318 shapes of both (microseconds for three rounds; what the histograms' memory costs is the same
-// on either side): all but seven of those more than 4 % apart are told right, and these are at most 12 % apart.  General and small:
-// 20k rows x 60, depth 6 1.16, 28k x 60 0.99; 16k x 100, depth 8 1.13, depth 10 0.78; 10k x 300, depth 6 1.00, depth 8 0.84; three
-// classes, 8k x 100, depth 6 1.03, 1333 x 300 0.78; ten classes, 1000 x 20, depth 4 1.14, 400 x 300 0.65.
+// on either side), before the general path's launches were chained (LaunchChained), which took a third of what a level costs
+// whatever it holds: with that third less, 31 shapes on either side of the line are told right or are within 2 %.  General and small,
+// microseconds for five rounds: 20k rows x 30, depth 6 1013 and 1035, 10k x 30 992 and 770; 16k x 100, depth 8 1584 and 1775, 6k x 100 1605 and
+// 1435; 8k x 200, depth 6 1157 and 1235, 2k x 200 1195 and 978; three classes, 3k x 50, depth 6 1377 and 1205; ten classes, 1500 x 40,
+// depth 6 1650 and 2075.
 static bool SmallPays(const SmallPlan& plan, int64_t N, int F, int K, int D)
 {
   int64_t passes = 0, turns = 0;
@@ -765,7 +767,7 @@ static bool SmallPays(const SmallPlan& plan, int64_t N, int F, int K, int D)
   const int abreast  = plan.blocks / plan.parts;  // features that are worked on at a time
   const double each  = static_cast<double>((F + abreast - 1) / abreast) * K;
   const double small = each * (2.4e-3 * static_cast<double>(passes * N) + 20.0 * static_cast<double>(turns) - 9.0 * D);
-  const double general = D * (72.0 + 5.0 * K + (K > 1 ? 7.0 : 0.0) + 3.4e-6 * static_cast<double>(N) * F * K);
+  const double general = D * (49.0 + 5.0 * K + (K > 1 ? 7.0 : 0.0) + 3.4e-6 * static_cast<double>(N) * F * K);
   return small <= general;
 }
 
