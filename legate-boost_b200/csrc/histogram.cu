@@ -38,6 +38,7 @@
 #include <type_traits>
 
 #include "device_utils.cuh"
+#include "hist_units.h"
 #include "internal.h"
 
 namespace lbk {
@@ -133,47 +134,6 @@ __device__ inline out_t* FeatureBase(const HistParams& p, int f, int seg)
          static_cast<long long>(seg) * p.push_len + (p.row_ptr[f] - lo);
 }
 
-// How the lanes of k_hist_smem share the nt features of a unit: `main` neighbouring bytes a lane and `extra` ones.  Each of the
-// two takes a power of two of features and eight (W = 1: the main ones sixteen) columns of words for each lane of a row, so that
-// fewer features have several copies of their words and a step still updates 32 banks; 2 (main + extra) reductions are issued per
-// batch of rows instead of 32.  Whole numbers use it where a row is one unit: 8M x 40, 4 nodes 200 -> 185 us, 10M x 40, depth 8
-// 2.65 -> 2.62 ms.  Of several units the last one keeps its 16 steps, so that the units' blocks go through the rows at one
-// pace and share the 128-byte lines of a row in L2: with the steps it needs (and blocks dealt by what a unit costs) 8M x 72
-// took 427 -> 528 us and 10M x 200, depth 8, 8.7 -> 9.6 ms, without the dealing 1M x 72, ten outputs, 6.93 -> 7.15 ms.
-// Floating-point reductions are loops where another one of the same word is on its way, and the columns that pad a row all fall
-// into their bin 0: there every unit has the steps it needs, and lanes without a feature leave a step out (HistRows, kMask).
-// 3M x 100 1222 -> 429 us, 3M x 20 341 -> 151, 3M x 64 256 -> 242.
-struct UnitForm {
-  int main, extra;
-};
-__device__ constexpr UnitForm FormOf(bool is_float, int W, bool several_units, int nt)
-{
-  if (W == 1) return {nt > 16 ? 16 : nt > 8 ? 8 : 4, 0};
-  if (nt > 48 || (!is_float && several_units)) return {8, 8};
-  if (!is_float) return {8, 4};
-  if (nt > 32) return {8, nt > 40 ? 4 : nt > 36 ? 2 : 1};
-  return {nt > 16 ? 8 : nt > 8 ? 4 : 2, 0};
-}
-// Feature (relative to the unit's first) of histogram word w of a bin, -1 where the word is a copy of another one.
-__device__ constexpr int FeatureOfWord(int W, UnitForm fm, int w)
-{
-  if (W == 1) {
-    const int q = w >> 4, col = w & 15;
-    return col < fm.main ? fm.main * q + col : -1;
-  }
-  const int half = w >> 5, q = (w >> 3) & 3, col = w & 7;
-  if (col >= (half == 0 ? fm.main : fm.extra)) return -1;
-  if (fm.extra == 8) return 16 * q + 8 * half + col;
-  if (fm.extra == 0) return fm.main * q + col;
-  // 33 to 48 features: lanes 0 and 3 share the first 16 bytes, lanes 1 and 2 have the next 32
-  if (half == 0) {
-    if (fm.extra == 1 && q == 2 && col >= 4) return 24 + (col - 4);
-    return (q == 0 ? 0 : q == 3 ? 8 : 16 * q) + col;
-  }
-  if (fm.extra == 1) return 28 + q;
-  if (fm.extra == 2) return 24 + 2 * q + col;
-  return (q == 0 ? 28 : q == 1 ? 24 : q == 2 ? 40 : 44) + col;
-}
 __device__ inline unsigned SmemAddr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
 
 // largest |grad| and |hess| of a set of quantised pairs (for the stage-level entry point; the
@@ -662,14 +622,15 @@ __device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, in
   constexpr int kWarps        = kHistThreads * W / 32;
   constexpr int kLanesPerRow  = 2 * W;
   constexpr int kRowsPerBatch = 32 / kLanesPerRow;
-  constexpr int kLoad         = kExtra != 0 ? 16 : kMain;  // bytes of a lane's load
+  constexpr UnitForm kForm{kMain, kExtra};
+  constexpr int kLoad         = LaneBytes(kForm);  // bytes of a lane's load
   constexpr bool kShared      = kExtra == 1 || kExtra == 2 || kExtra == 4;
   const unsigned rslot = lane / kLanesPerRow, q = lane % kLanesPerRow;
   const unsigned wsel = rslot >> 2, bsel = rslot & 3;
   const unsigned perm = bsel == 0 ? 0x3210u : bsel == 1 ? 0x2301u : bsel == 2 ? 0x1032u : 0x0123u;
   const unsigned sel0 = perm + ((wsel & 1) ? 0x4444u : 0u), sel1 = perm + ((wsel & 1) ? 0u : 0x4444u);
   const unsigned sel2 = (rslot & 1) ? 0x4401u : 0x4410u;  // two bytes
-  const unsigned from = kShared && q == 3 ? 0u : q;       // the lane's piece of the row
+  const int from      = PieceOfLane(W, kForm, kLine ? min(W, p.G - g0) : W, static_cast<int>(q));  // the lane's piece of the row
   const int64_t pitch = static_cast<int64_t>(p.G) * kGroup;
   const unsigned char* gb = static_cast<const unsigned char*>(p.bins) + g0 * kGroup + from * kLoad;
   unsigned steps = 0u;  // kMask: those in which the lane has a feature
@@ -678,7 +639,7 @@ __device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, in
     for (int j = 0; j < 16; ++j) {
       const int n = W == 1 || j < 8 ? kMain : kExtra, col = (static_cast<int>(rslot) ^ j) & (n - 1);
       const int w = W == 1 ? 16 * static_cast<int>(q) + col : 32 * (j >> 3) + 8 * static_cast<int>(q) + col;
-      if (n > 0 && g0 * kGroup + FeatureOfWord(W, UnitForm{kMain, kExtra}, w) < p.F) steps |= 1u << j;
+      if (n > 0 && g0 * kGroup + FeatureOfWord(W, kForm, w) < p.F) steps |= 1u << j;
     }
   }
   const in_t* gpair    = static_cast<const in_t*>(p.gpair);
