@@ -60,7 +60,9 @@ void LaunchChained(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStr
   cfg.stream           = stream;
   cfg.attrs            = attr;
   cfg.numAttrs         = 1;
-  LBK_CUDA(cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...));
+  const cudaError_t launched = cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+  if (launched != cudaSuccess) cudaGetLastError();  // (left with the runtime, it would be the answer to the next launch, whoever's)
+  LBK_CUDA(launched);
 }
 
 // 16-byte (grad, hess) pairs

@@ -1021,6 +1021,21 @@ def test_classifier_multiclass(lb):
     assert (m.predict(dev(X)).cpu().numpy() == y).mean() > 0.5
 
 
+def test_a_refused_launch_is_the_error_of_its_own_call(lb):
+    """More feature groups than a grid is high: the runtime refuses the launch on the host.  The calls that come after it, of
+    this library and of torch, do not find that error waiting."""
+    from legateboost_b200 import stages
+
+    F = 32 * 65535 + 1
+    row_ptr, proposals = torch.arange(F + 1, dtype=torch.int32, device="cuda"), torch.full((F,), np.inf, device="cuda")
+    with pytest.raises(lb.library.LbkError, match="invalid"):
+        stages.bin_matrix(torch.zeros((1, F), device="cuda"), proposals, row_ptr)
+    assert torch.equal(torch.arange(5, device="cuda") + 1, dev(np.arange(1, 6)))
+    F = 40
+    bins = stages.bin_matrix(torch.zeros((3, F), device="cuda"), proposals[:F], row_ptr[: F + 1])
+    assert bins.shape == (3, 64) and not bins.any()
+
+
 def test_bad_arguments_are_errors(lb):
     from legateboost_b200.tree import build_tree_arrays
 
