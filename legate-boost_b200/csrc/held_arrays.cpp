@@ -69,11 +69,17 @@ PyMethodDef g_methods[] = {
   {"holds", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(Holds)), METH_FASTCALL,
    "Whether the models hold the source's tensors, at these addresses."},
   {nullptr, nullptr, 0, nullptr}};
-PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "held_arrays", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+// LBK_MODULE: the module's name, which tells the torch it is compiled for (build.py)
+#define LBK_TEXT_(x) #x
+#define LBK_TEXT(x) LBK_TEXT_(x)
+#define LBK_JOIN_(a, b) a##b
+#define LBK_JOIN(a, b) LBK_JOIN_(a, b)
+
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, LBK_TEXT(LBK_MODULE), nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_held_arrays()
+PyMODINIT_FUNC LBK_JOIN(PyInit_, LBK_MODULE)()
 {
   const char* names[3] = {"leaf_value", "feature", "split_value"};
   for (int i = 0; i < 3; ++i) {

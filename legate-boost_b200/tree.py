@@ -11,6 +11,7 @@ import copy
 import ctypes as C
 import warnings
 from array import array
+from importlib import import_module
 from itertools import accumulate, chain
 from operator import attrgetter, is_
 from typing import Any, Callable, List, Sequence, Union
@@ -19,6 +20,7 @@ import numpy as np
 import torch
 
 from . import library as L
+from .build import module_name
 
 
 def _dtype_code(t: torch.Tensor) -> int:
@@ -143,9 +145,9 @@ def build_tree_arrays(X, g, h, *, max_depth, split_samples, seed, l1=0.0, l2=1.0
 
 
 try:
-    from .held_arrays import holds as _holds
+    _holds = import_module("." + module_name(), __package__).holds
 except ImportError as e:  # importing works anywhere
-    _missing = "held_arrays.so is missing or of another build: build it with `python legate-boost_b200/build.py` (%s)" % e
+    _missing = "the extension module %s is missing: build it with `python legate-boost_b200/build.py` (%s)" % (module_name(), e)
 
     def _holds(models, source, addresses):
         raise RuntimeError(_missing)

@@ -1,4 +1,5 @@
 """The check that a kept table of addresses still belongs to an ensemble's tensors (CPU)."""
+import os
 from array import array
 
 import pytest
@@ -66,3 +67,16 @@ def test_errors_are_python_errors():
 
     models[:] = [Odd(), Model()]
     assert not _holds(models, source + source, at + at)
+
+
+def test_another_torch_or_python_has_a_module_of_its_own():
+    """What is compiled in are the layouts of one torch and one Python: a module of another pair neither counts as built nor is
+    ever loaded."""
+    import sysconfig
+
+    from legateboost_b200 import build
+
+    assert _holds.__module__ == "legateboost_b200." + build.module_name()
+    other = build.module_path("0.1.0+none")
+    assert build.module_path() != other and not os.path.exists(other) and os.path.exists(build.module_path())
+    assert build.module_path().endswith(sysconfig.get_config_var("EXT_SUFFIX")) and build.module_name("0.1.0+none").isidentifier()
