@@ -144,16 +144,22 @@ def build_tree_arrays(X, g, h, *, max_depth, split_samples, seed, l1=0.0, l2=1.0
     return out
 
 
-try:
-    _holds = import_module("." + module_name(), __package__).holds
-except ImportError as e:  # importing works anywhere
-    _missing = "the extension module %s is missing: build it with `python legate-boost_b200/build.py` (%s)" % (module_name(), e)
-
-    def _holds(models, source, addresses):
-        raise RuntimeError(_missing)
-
 _ARRAYS = attrgetter("leaf_value", "feature", "split_value")
 _ARRAY_TYPES = (torch.float64, torch.int32, torch.float64)
+
+
+def _holds_in_python(models, source, addresses):
+    """``holds`` of csrc/held_arrays.cpp: whether the models hold the source's tensors (three each), at these addresses."""
+    if 3 * len(models) != len(source):
+        return False
+    arrays = tuple(chain.from_iterable(map(_ARRAYS, models)))
+    return all(map(is_, arrays, source)) and array("q", list(map(torch.Tensor.data_ptr, arrays))).tobytes() == addresses
+
+
+try:
+    _holds = import_module("." + module_name(), __package__).holds
+except ImportError:  # not built, or for another torch or Python: the same answer, for 100 trees 23 us later
+    _holds = _holds_in_python
 
 
 class TreeTable:

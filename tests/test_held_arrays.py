@@ -1,12 +1,16 @@
 """The check that a kept table of addresses still belongs to an ensemble's tensors (CPU)."""
 import os
+import subprocess
+import sys
 from array import array
 
 import pytest
 import torch
 
 import legateboost_b200 as lb  # noqa: F401
-from legateboost_b200.tree import _holds
+from legateboost_b200.tree import _holds, _holds_in_python
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 class Model:
@@ -80,3 +84,56 @@ def test_another_torch_or_python_has_a_module_of_its_own():
     other = build.module_path("0.1.0+none")
     assert build.module_path() != other and not os.path.exists(other) and os.path.exists(build.module_path())
     assert build.module_path().endswith(sysconfig.get_config_var("EXT_SUFFIX")) and build.module_name("0.1.0+none").isidentifier()
+
+
+@pytest.mark.parametrize("n", [1, 4])
+def test_the_python_way_gives_the_same_answers(n):
+    def changed(models, what):
+        last = models[-1]
+        if what == "shorter":
+            return models[:-1]
+        if what == "longer":
+            return models + [Model()]
+        if what == "order":
+            return models[::-1]
+        if what == "none":
+            last.feature = None
+        elif what == "other":
+            last.split_value = last.split_value.clone()
+        elif what == "moved":
+            last.leaf_value.data = last.leaf_value.clone()
+        elif what == "filled":
+            last.leaf_value.fill_(3.0)
+        return models
+
+    for what in ("same", "shorter", "longer", "order", "none", "other", "moved", "filled"):
+        models = [Model() for _ in range(n)]
+        source, at = _table(models)
+        models = changed(models, what)
+        answer = _holds_in_python(models, source, at)
+        assert answer == _holds(models, source, at) == (what in ("same", "filled") or (what == "order" and n == 1)), what
+    with pytest.raises(AttributeError):
+        _holds_in_python([object()], source[:3], at[:24])
+
+
+def test_without_the_module_tables_are_checked_all_the_same():
+    """The module makes the check faster; without it (not built, or built for another torch) predictions work as with it."""
+    program = """
+import importlib.util, sys
+spec = importlib.util.spec_from_file_location("lbk_build", sys.argv[1])
+build = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(build)
+sys.modules["legateboost_b200." + build.module_name()] = None  # importing it is an ImportError
+import torch
+from legateboost_b200 import tree
+assert tree._holds is tree._holds_in_python
+class Model:
+    def __init__(self):
+        self.leaf_value, self.feature, self.split_value = torch.zeros(7, 1, dtype=torch.float64), -torch.ones(7, dtype=torch.int32), torch.zeros(7, dtype=torch.float64)
+models = [Model() for _ in range(3)]
+table = tree.TreeTable([(m.leaf_value, m.feature, m.split_value) for m in models])
+assert table.matches(models) and table.matches(tuple(models)) and not table.matches(models[:2])
+models[1].feature = models[1].feature.clone()
+assert not table.matches(models)
+"""
+    subprocess.run([sys.executable, "-c", program, os.path.join(ROOT, "legate-boost_b200", "build.py")], check=True, cwd=ROOT)
