@@ -189,9 +189,10 @@ class TreeTable:
             raise ValueError("the trees of an ensemble must have arrays of one shape per node")
         # converted copies would not follow later changes of the originals: such a table is not kept
         self.reusable = all(map(is_, keep, self.source))
-        at = list(map(torch.Tensor.data_ptr, keep))
-        self.addresses = array("q", at).tobytes()
-        rows = np.array((at[0::3], at[1::3], at[2::3], [m | (e - m) << 32 for m, e in zip(nodes, ends)]), dtype=np.int64).T.copy()
+        at = np.fromiter(map(torch.Tensor.data_ptr, keep), np.int64, len(keep))
+        self.addresses = at.tobytes()
+        rows = np.empty((len(nodes), 4), dtype=np.int64)
+        rows[:, :3], rows[:, 3] = at.reshape(-1, 3), [m | (e - m) << 32 for m, e in zip(nodes, ends)]
         self.keep, self.total_nodes, self.max_nodes, self.n_trees = keep, ends[-1], max(nodes), len(nodes)
         self.table = torch.from_numpy(rows).to(device)
         self.device = device
