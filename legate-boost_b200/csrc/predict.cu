@@ -40,6 +40,7 @@
 #include <algorithm>
 
 #include "predict.cuh"
+#include "predict_sums.h"
 
 namespace lbk {
 namespace {
@@ -262,7 +263,7 @@ struct TiledArgs {
 // neighbouring outputs, whose values are one 16-byte load.  Per tree and 32 rows of ten outputs that is 30 passes instead of 55
 // (as 8-byte loads, 12 values for 10), of about 80 with the walks: 100 features, ten outputs, 50 trees of depth 8, 1M rows 1141 -> 946 us,
 // 100003 rows 97 -> 92 (two waves that wait for the trees' 300 MB); 300k x 20, 100 trees of depth 6 303 -> 256; sixteen
-// outputs, 200003 x 30 170 -> 160.  Three outputs with three sums instead of four: 2M x 50, 100 trees of depth 7 1229 -> 1153.
+// outputs, 200003 x 30 170 -> 160.  Three outputs with three sums instead of four: 2M x 50, 100 trees of depth 7 1229 -> 1153 (which numbers: predict_sums.h).
 // kGated: the launch stands in for the walk on ranks and does nothing where that was not declined.  A resident block then takes tile
 // after tile: a launch that finds nothing to do ends in 2.5 us, where a block per tile would come and go.
 template <typename T, int TG, int KR, int kStaged, bool kGated = false>
@@ -633,7 +634,6 @@ struct TilePlan {
   int64_t waves    = 0;
   TreeRecord rec{};
 };
-constexpr int kRegisterSums    = 16;   // outputs whose sums a warp keeps in registers
 constexpr int kStagedOutputs   = 6;    // from which leaf values may come with the records (PlanTile), ...
 constexpr int kStagedTrees     = 16;   // ... and trees: of fewer the rows are most of the work, which more blocks an SM overlap
 constexpr int kTileStaticBytes = 256;  // (a bound of what the kernel declares)
@@ -703,8 +703,10 @@ template <typename T, int TG, int KR>
 void LaunchTiledAs(lbk_context* ctx, const int* gate, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
   auto fn = k_predict_tiled<T, TG, KR, 0>;
-  if constexpr (KR >= 8)
-    if (a.leaves_c == nullptr) fn = a.K % 2 == 0 ? k_predict_tiled<T, TG, KR, 2> : k_predict_tiled<T, TG, KR, 1>;
+  if constexpr (KR >= kStagedOutputs)
+    if (a.leaves_c == nullptr) fn = k_predict_tiled<T, TG, KR, 2>;
+  if constexpr (KR > kStagedOutputs)
+    if (a.leaves_c == nullptr && a.K % 2 != 0) fn = k_predict_tiled<T, TG, KR, 1>;
   int64_t grid = (a.n_rows + a.rb - 1) / a.rb;
   if constexpr (KR == 0)
     if (gate != nullptr) {
@@ -720,15 +722,19 @@ void LaunchTiledAs(lbk_context* ctx, const int* gate, const TiledArgs<T>& a, con
 template <typename T, int TG>
 void LaunchTiled(lbk_context* ctx, const int* gate, const TiledArgs<T>& a, const TilePlan& plan, cudaStream_t stream)
 {
-  if (a.K == 1) LaunchTiledAs<T, TG, 0>(ctx, gate, a, plan, stream);
-  else if (a.K <= 2) LaunchTiledAs<T, TG, 2>(ctx, gate, a, plan, stream);
-  else if (a.K == 3) LaunchTiledAs<T, TG, 3>(ctx, gate, a, plan, stream);
-  else if (a.K == 4) LaunchTiledAs<T, TG, 4>(ctx, gate, a, plan, stream);
-  else if (a.K <= 8) LaunchTiledAs<T, TG, 8>(ctx, gate, a, plan, stream);
-  else if (a.K <= 10) LaunchTiledAs<T, TG, 10>(ctx, gate, a, plan, stream);
-  else if (a.K <= 12) LaunchTiledAs<T, TG, 12>(ctx, gate, a, plan, stream);
-  else if (a.K <= kRegisterSums) LaunchTiledAs<T, TG, kRegisterSums>(ctx, gate, a, plan, stream);
-  else LaunchTiledAs<T, TG, -1>(ctx, gate, a, plan, stream);
+  switch (SumsOf(a.K)) {
+    case 0: LaunchTiledAs<T, TG, 0>(ctx, gate, a, plan, stream); break;
+    case 2: LaunchTiledAs<T, TG, 2>(ctx, gate, a, plan, stream); break;
+    case 3: LaunchTiledAs<T, TG, 3>(ctx, gate, a, plan, stream); break;
+    case 4: LaunchTiledAs<T, TG, 4>(ctx, gate, a, plan, stream); break;
+    case 6: LaunchTiledAs<T, TG, 6>(ctx, gate, a, plan, stream); break;
+    case 8: LaunchTiledAs<T, TG, 8>(ctx, gate, a, plan, stream); break;
+    case 10: LaunchTiledAs<T, TG, 10>(ctx, gate, a, plan, stream); break;
+    case 12: LaunchTiledAs<T, TG, 12>(ctx, gate, a, plan, stream); break;
+    case 14: LaunchTiledAs<T, TG, 14>(ctx, gate, a, plan, stream); break;
+    case 16: LaunchTiledAs<T, TG, 16>(ctx, gate, a, plan, stream); break;
+    default: LaunchTiledAs<T, TG, -1>(ctx, gate, a, plan, stream); break;
+  }
 }
 
 }  // namespace

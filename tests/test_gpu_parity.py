@@ -690,6 +690,24 @@ def test_predict_of_even_and_odd_outputs(lb, oracle, K, dt):
     assert np.allclose(softmax, e / e.sum(axis=1, keepdims=True), rtol=1e-13, atol=0)  # (a few roundings of exp and a sum)
 
 
+@pytest.mark.parametrize("K", [2, 3, 4, 5, 6, 7, 8, 9, 11, 12, 13, 14, 15, 16, 17])
+@pytest.mark.parametrize("T", [5, 16])
+def test_predict_of_any_number_of_outputs(lb, oracle, K, T):
+    """As many sums as outputs, or one more, with the leaf values apart (few trees, few outputs) or with the trees: the oracle's bits."""
+    from legateboost_b200 import library as L
+    from legateboost_b200.tree import TreeTable
+
+    N, F, D = 9_001, 12, 6
+    rs = np.random.RandomState(100 * T + K)
+    X = rs.random((N, F)).astype(np.float32)
+    trees = [(dev(rs.normal(size=(t[1].shape[0], K))),) + t[1:] for t in _random_trees(rs, T, D, np.arange(F))]
+    table = TreeTable(trees)
+    plan = _predict_plan(lb, table, dev(X), K, L.RAW)
+    assert plan["tile_rows"] > 0 and plan["leaves_with_trees"] == (T >= 16 and 6 <= K <= 16)
+    want = oracle.predict(X, [tuple(a.cpu().numpy() for a in t) for t in trees])
+    assert np.array_equal(table.predict(dev(X), K, wait=True).cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("N,F,K,T,D,dt", [(16, 30, 1, 100, 6, np.float32), (20_001, 40, 10, 20, 6, np.float32), (900_001, 30, 1, 100, 8, np.float64)])
 def test_chained_launches_under_capture_and_on_two_streams(lb, N, F, K, T, D, dt):
     """Kernels that may begin as the one before them ends see all that it wrote: in a captured graph, replayed on changing inputs,
