@@ -610,15 +610,55 @@ def test_predict_by_ranks(lb, oracle, N, F, T, D, dt, used, what, group, pieces,
     assert torch.equal(table.predict(wide[:, 1: F + 1], 1, init=init, transform=transform, wait=True), got)
 
 
+def _rank_searches(trees, F, dt):
+    """How k_rank_rows finds the ranks of the turns over an ensemble's features: in 3 or 4 steps, by as many as its fullest bucket
+    wants ("counted"), or in a table that has no room in shared memory ("where it lies").  Restated from its tables and turns."""
+    room = torch.cuda.get_device_properties(0).shared_memory_per_block_optin - 1024 - 16 * 32 * 33 * 4
+    f = np.concatenate([t[1].cpu().numpy()[: len(t[1]) // 2] for t in trees])
+    s = np.concatenate([t[2].cpu().numpy()[: len(t[2]) // 2] for t in trees])
+    fullest, entries = [], []
+    for i in range(F):
+        v = np.unique(s[f == i]).astype(np.float32 if dt is np.float32 else np.float64)
+        entries.append(max(len(v), 1))
+        fullest.append(0)
+        if len(v):
+            lo, hi = np.float32(v[0]), np.float32(v[-1])
+            scale = np.float32(len(v)) / (hi - lo) if hi > lo else np.float32(0)
+            fullest[-1] = np.bincount(np.minimum(((v.astype(np.float32) - lo) * scale).astype(np.int64), len(v) - 1)).max()
+
+    def table(a, b, pad=0):
+        n = sum(entries[a:b])
+        return (n + 1) // 2 * 8 + (n + pad * (b - a)) * np.dtype(dt).itemsize
+
+    found = set()
+    for g in range(0, F, 32):
+        a, end = g, min(g + 32, F)
+        while a < end:
+            b = a + 1
+            while b < end and table(a, b + 1) <= room:
+                b += 1
+            if b < end:
+                b = a + 2 ** int(np.log2(b - a))
+            most = max(fullest[a:b])
+            if most > 0:
+                found.add("where it lies" if table(a, b) > room else "counted" if most >= 16 or table(a, b, 4) > room else 4 if most >= 8 else 3)
+            a = b
+    return found
+
+
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
-@pytest.mark.parametrize("what,used", [("even", None), ("any", None), ("seven", None), ("fifteen", None), ("sixteen", None), ("sixty", None), ("one", [3])])
-def test_ranks_from_buckets_of_any_size(lb, what, used, dt):
+@pytest.mark.parametrize("what,used,searches", [
+    ("even", None, (3, 3)), ("any", None, (3, 3)), ("seven", None, (3, 3)), ("fifteen", None, (4, 4)), ("sixteen", None, ("counted", 4)),
+    ("sixty", None, ("counted", "counted")), ("one", [3], ("where it lies", "counted"))])
+def test_ranks_from_buckets_of_any_size(lb, what, used, searches, dt):
     """Splits evenly apart, by chance, and crowded in buckets of up to so many (one: nearly all of a feature's): the steps of the
-    search are another number each time.  A few rows at a time, where trees are walked where they lie, give the same bits."""
+    search are another number each time (float32, float64).  A few rows at a time, where trees are walked where they lie, give the same bits."""
     from legateboost_b200 import library as L
     from legateboost_b200.tree import TreeTable
 
     N, F, T, D = (1_000_003, 60, 300, 8) if dt is np.float32 else (800_011, 20, 70, 8)
+    if used is not None and dt is np.float32:  # (of two groups of features the ranks are found too dear)
+        F, T = 20, 200
     rs = np.random.RandomState(len(what))
     trees, crowd = [], dict(seven=7, fifteen=15, sixteen=17, sixty=60).get(what)
     for v, f, s in _random_trees(rs, T, D, np.arange(F) if used is None else used):
@@ -630,6 +670,7 @@ def test_ranks_from_buckets_of_any_size(lb, what, used, dt):
         elif what == "one":
             s = np.where(rs.random(s.shape) < 0.002, np.sign(s - 0.5) * 1e4, 0.5 + s * 0.02)
         trees.append((v, f, dev(s.astype(dt).astype(np.float64))))
+    assert _rank_searches(trees, F, dt) == {searches[0 if dt is np.float32 else 1]}
     table = TreeTable(trees)
     X = np.random.default_rng(len(what)).random((N, F), dtype=dt)
     splits = np.concatenate([t[2].cpu().numpy() for t in trees]).astype(dt)
@@ -639,7 +680,8 @@ def test_ranks_from_buckets_of_any_size(lb, what, used, dt):
     dX = dev(X)
     plan = _predict_plan(lb, table, dX, 1, L.RAW)
     assert plan["threads"] > 0
-    got, _ = _predict_and_word(lb, table, dX, plan)
+    got, word = _predict_and_word(lb, table, dX, plan)
+    assert word == 0  # (the ranks were found and walked on: not declined)
     for rows in (np.arange(8000), np.arange(N - 8000, N), np.sort(rs.choice(N, 8000, replace=False))):
         rows = dev(rows)
         assert torch.equal(got[rows], table.predict(dX[rows].contiguous(), 1, wait=True))
