@@ -169,8 +169,8 @@ class TreeTable:
 
     def __init__(self, arrays):
         # (few calls per tensor: an ensemble's first prediction waits for them)
-        self.source = tuple(chain.from_iterable(arrays))
-        keep = list(self.source)
+        keep = list(chain.from_iterable(arrays))
+        self.source = tuple(keep)
         for i, t in enumerate(keep):
             want = _ARRAY_TYPES[i % 3]
             if t.dtype is not want or not t.is_contiguous():
