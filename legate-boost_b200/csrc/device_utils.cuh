@@ -10,10 +10,10 @@
 
 namespace lbk {
 
-// Stores a fault code into the context's status word (mapped host memory).
 // First statement of a kernel that LaunchChained (internal.h) launches; nothing to wait for where it was launched otherwise.
 __device__ inline void AfterTheKernelBefore() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
+// Stores a fault code into the context's status word (mapped host memory).
 __device__ inline void ReportFault(int* status, int code)
 {
   *reinterpret_cast<volatile int*>(status) = code;

@@ -564,8 +564,8 @@ __global__ void __launch_bounds__(kHistThreads)
   }
 }
 
-// One update step of a lane: byte J of its 16 bin bytes (already permuted so that step J reads
-// the static byte J), both words of the pair.  `lane_word` is the shared-memory address of the
+// One update step of a lane: byte J of its bin bytes (already permuted so that step J reads
+// the static byte J; at most 16, with places for eight main and eight extra ones), both words of the pair.  `lane_word` is the shared-memory address of the
 // lane's word in bin row 0 of the gradient histogram.
 template <typename A, int W, int J, bool kMask>
 __device__ inline void HistStep(const unsigned (&x)[4], unsigned lane_word, const int2& v, unsigned steps)
@@ -774,17 +774,20 @@ __device__ __forceinline__ void HistRows(const HistParams& p, int sb, int se, in
 // hessian histogram behind it, so that an update needs no base register; then the staging area of the
 // flush and the plan.  Every warp runs its own pipeline over batches of 32 / (2 W) rows (no block barrier
 // inside).  2 W lanes own one row of the batch and load its bin bytes straight from global memory
-// into registers, 16 bytes per lane.  In step j of 16 the lanes of row slot r handle byte (j xor r)
-// of their 16, and the histogram words of a bin are laid out so that the 32 lanes of a warp always
-// update 32 different banks, whatever the bins:
+// into registers.  Units of all their features, and those of several units of whole numbers, take 16 bytes per lane: in step j of 16
+// the lanes of row slot r handle byte (j xor r) of their 16, and the histogram words of a bin are laid out so that the 32 lanes of a
+// warp always update 32 different banks, whatever the bins:
 //   W = 1 (r < 16, quarter q < 2):  word = 16 q + byte                   (bank = word)
 //   W = 2 (r < 8,  quarter q < 4):  word = 32 (byte / 8) + 8 q + byte % 8 (bank = 8 q + byte % 8)
+// Other units load fewer bytes per lane and take fewer steps, and words that no feature needs are copies of other ones, so that the
+// banks stay different (UnitForm, FeatureOfWord and PieceOfLane, hist_units.h).
 // The bytes are permuted once per batch (a word swap and one byte permute per word) so that step
 // j reads the static byte j.  Per 32 updates that leaves the two reductions on the pipe.
 //
 // Flush: a warp takes a tile of 4 bins x 32 words, turns it in its staging area (a skewed 4 x 32
 // array, conflict free both ways) and writes, per word, the 4 bins of a feature as 64 contiguous
-// bytes of the output.
+// bytes of the output.  Copies of a word are added up on the way into the staging area, by shuffle, and the words without a feature are left out;
+// an image that goes into a slot of a merge tree (below) is the words as they are, copies apart.
 //
 // The pieces of a node that reaches over range boundaries add their sums to its histogram with 64-bit atomics. An
 // instruction of the warp covers 16 whole (grad, hess) pairs, so that every sector is touched once: 148 blocks adding 256 KB

@@ -27,7 +27,8 @@ constexpr int kPartTile      = kPartThreads * kPartItems;  // rows per chunk
 constexpr int kPartBlocks    = 4;    // per SM: as many as are resident
 // Bands of a level (see k_partition): as many as bring the columns of a band's rows to kPartBandBytes of L2, but with
 // kPartBandTurns chunks for every block, because a band is planned anew.  Levels 1 to 8 of 100M x 64: 4.83 ms with one turn,
-// 4.66 with two, 4.67 with four; 10M x 64, six levels: 339, 329 and 322 us; 130 million cells (1M x 128) and fewer have one band.
+// 4.66 with two, 4.67 with four; 10M x 64, six levels: 339, 329 and 322 us.  So a level has bands where its bins are more than
+// 24 MB and its rows at least eight chunks for every block (9.7 million rows on 148 SMs), whatever the number of features.
 constexpr int64_t kPartBandBytes = 24 << 20;
 constexpr int kPartBandTurns     = 4;
 constexpr int kPartMaxLogBands   = 7;

@@ -262,7 +262,8 @@ struct TiledArgs {
 // kStaged (KR > 0): the leaf values of several outputs are in the records too; 2: of an even number, and a lane has the sums of two
 // neighbouring outputs, whose values are one 16-byte load.  Per tree and 32 rows of ten outputs that is 30 passes instead of 55
 // (as 8-byte loads, 12 values for 10), of about 80 with the walks: 100 features, ten outputs, 50 trees of depth 8, 1M rows 1141 -> 946 us,
-// 100003 rows 97 -> 92 (two waves that wait for the trees' 300 MB); 300k x 20, 100 trees of depth 6 303 -> 256; sixteen
+// 100003 rows 97 -> 92 (what is left is the latency of the walks in flight, eleven warps with two trees each: ncu has the load/store pipe
+// at 56 %, the issue slots at 25 and L2 at 15, and an instruction of a warp every eleven cycles); 300k x 20, 100 trees of depth 6 303 -> 256; sixteen
 // outputs, 200003 x 30 170 -> 160.  Three outputs with three sums instead of four: 2M x 50, 100 trees of depth 7 1229 -> 1153 (which numbers: predict_sums.h).
 // kGated: the launch stands in for the walk on ranks and does nothing where that was not declined.  A resident block then takes tile
 // after tile: a launch that finds nothing to do ends in 2.5 us, where a block per tile would come and go.
