@@ -649,7 +649,7 @@ def _rank_searches(trees, F, dt):
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 @pytest.mark.parametrize("what,used,searches", [
     ("even", None, (3, 3)), ("any", None, (3, 3)), ("seven", None, (3, 3)), ("fifteen", None, (4, 4)), ("sixteen", None, ("counted", 4)),
-    ("sixty", None, ("counted", "counted")), ("one", [3], ("where it lies", "counted"))])
+    ("sixty", None, ("counted", "counted")), ("skewed", None, ("counted", "counted")), ("one", [3], ("where it lies", "counted"))])
 def test_ranks_from_buckets_of_any_size(lb, what, used, searches, dt):
     """Splits evenly apart, by chance, and crowded in buckets of up to so many (one: nearly all of a feature's): the steps of the
     search are another number each time (float32, float64).  A few rows at a time, where trees are walked where they lie, give the same bits."""
@@ -667,6 +667,8 @@ def test_ranks_from_buckets_of_any_size(lb, what, used, searches, dt):
             s = np.round(s * 700) / 700
         elif crowd is not None:  # clusters a good deal further apart than a bucket is wide, in a small part of one each
             s = np.floor(s * 40) / 40 + np.floor(rs.random(s.shape) * crowd) * 2e-6
+        elif what == "skewed":  # many buckets side by side that are nearly too full to be put in order one by one
+            s = np.exp(4 * s)
         elif what == "one":
             s = np.where(rs.random(s.shape) < 0.002, np.sign(s - 0.5) * 1e4, 0.5 + s * 0.02)
         trees.append((v, f, dev(s.astype(dt).astype(np.float64))))
